@@ -316,6 +316,343 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attention_kernel(const __grid_
     trace_end(a.tr);
 }
 
+// ------------------------------------------------------------------------------------------------
+// fp16 caches, head sizes 64 / 128, up to four query heads per key/value head: the same job on mma.sync.
+//
+// What bounds it: the cache's bytes.  The FMA kernel above spends ~480 instructions per 8 tokens and warp (a 31-shuffle
+// reduction of the scores, four f32 conversions and shuffled weights per token) and keeps 7 warps per SM busy: 91 us at 32 rows
+// of 1500 to 3000 tokens (8 kv heads of 128), 3.3 TB/s.  Here a warp takes 16 tokens at a time through 32 MMAs: 56 us,
+// 5.4 TB/s, and the distance to a 64-bit result went from 4.5e-7 to 3.0e-7.
+//
+// Nothing is rounded to 16 bits: keys and values ARE fp16, and an f32 query (or softmax weight) is the exact sum of three fp16
+// numbers, q = q1 + q2 + q3 (11 bits each).  One 16-row MMA tile holds the splits of all four heads -- row h: q1 of head h,
+// row 4 + h: q2, row 8 + h: q3 -- so the three products cost no extra instruction, and summing three accumulator rows gives
+// the f32 product.  (The factors 2^6 on the queries and 2^12 on the weights keep the small parts out of fp16's subnormals.)
+// MMA accumulators are short-lived: 4 steps of K for a score, one step of 16 tokens for an output; both are then added to f32
+// registers with rounded adds, since a long MMA chain truncates.
+//
+// A warp walks its own 16-token half pages (w, w + 4, ...) through a private ring of cp.async stages, chunks of 16 bytes
+// XOR-swizzled by the token so ldmatrix is free of conflicts: no barrier between warps until the final merge.  Tokens past the
+// context are zero-filled.  Where an infinity or NaN shows up in a warp's sums (an fp16 cache overflowed: inf - inf between
+// splits is not what an f32 product gives) the warp takes its tokens again in plain f32.
+// ------------------------------------------------------------------------------------------------
+#define AM_TOK 16
+#define AM_Q_UP 64.0f                     // 2^6 on the queries
+#define AM_P_UP 12.0f                     // 2^12 on the weights (added to the exponent)
+
+DL_DEVINL void am_cp16(uint32_t dst, const void* src, bool live) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(live ? 16 : 0) : "memory");
+}
+DL_DEVINL void am_ldm(uint32_t (&r)[4], uint32_t a) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+}
+DL_DEVINL void am_ldm_trans(uint32_t (&r)[4], uint32_t a) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+}
+DL_DEVINL void am_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+DL_DEVINL float am_exp2(float x) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+DL_DEVINL uint32_t am_pack(__half a, __half b) { __half2 h = __halves2half2(a, b); return *reinterpret_cast<uint32_t*>(&h); }
+// the two fp16 parts of v that this lane's rows hold: row g (first part for g < 4, second for g >= 4) and row g + 8 (third / none)
+DL_DEVINL void am_split(float v, bool lower, __half& top, __half& bot) {
+    const __half h1 = __float2half_rn(v);
+    const float r1 = v - __half2float(h1);
+    const __half h2 = __float2half_rn(r1);
+    top = lower ? h1 : h2;
+    bot = lower ? __float2half_rn(r1 - __half2float(h2)) : __ushort_as_half(0);
+}
+
+template <int HS>
+__global__ void __launch_bounds__(ATT_WARPS * 32, 2) attention_mma_kernel(const __grid_constant__ AttArgs a) {
+    constexpr int ROWB = HS * 2, CH = ROWB / 16;               // bytes / 16-byte chunks of a token's line
+    constexpr int HALF = AM_TOK * ROWB;                        // K (or V) of a half page
+    constexpr int ST = HS == 128 ? 3 : 6;                      // ring stages per warp (24 KB)
+    constexpr int KS = HS / 16, NT = HS / 8;
+    extern __shared__ __align__(128) uint8_t smem[];
+    trace_begin(a.tr);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int sp = blockIdx.x, kvh = blockIdx.y, m = blockIdx.z;
+    const int G = a.n_heads / a.n_kv_heads;
+    pdl_launch_dependents();
+    pdl_wait();     // q, pos, block tables and the KV cache all come from earlier kernels
+    if (a.row_skip != nullptr && a.row_skip[m] != 0) { trace_end(a.tr); return; }      // uniform for the CTA
+    const int T = a.pos[m] + 1;
+    const int n_pages = (T + ATT_PAGE - 1) / ATT_PAGE;
+    const int n_eff = (n_pages <= ATT_MIN_SPLIT_PAGES) ? 1 : min(a.n_splits, (n_pages + 7) / 8);      // as in attention_kernel
+    if (sp >= n_eff) { trace_end(a.tr); return; }
+    const int pps = (n_pages + n_eff - 1) / n_eff;
+    const int pg0 = sp * pps, pg1 = min(n_pages, pg0 + pps);
+    const int t_end = min(T, pg1 * ATT_PAGE);
+    const int n_hp = max(0, (t_end - pg0 * ATT_PAGE + AM_TOK - 1) / AM_TOK);       // half pages of this CTA; warp w takes w, w + 4, ...
+    const int* bt = a.block_table + (size_t)a.slot[m] * a.max_pages;
+    const int n_my = (n_hp - warp + ATT_WARPS - 1) / ATT_WARPS;
+
+    float* w_acc = reinterpret_cast<float*>(smem);             // [WARPS][4][HS], after the ring is done with
+    float* w_ml = w_acc + ATT_WARPS * 4 * HS;                  // [WARPS][4][2]
+    int* s_last = reinterpret_cast<int*>(w_ml + ATT_WARPS * 4 * 2);
+    const uint32_t ring = smem_u32(smem) + warp * (ST * 2 * HALF);
+    const int g = lane >> 2, qd = lane & 3, head = g & 3;
+    const bool lower = g < 4;
+
+    // this warp's half page i: page pg0 + (w + 4 i) / 2; the lanes hold the next 32 page numbers
+    auto page_at = [&](int i) { const int p = pg0 + ((warp + ATT_WARPS * i) >> 1); return i < n_my ? bt[p] : 0; };
+    int my_page = page_at(lane);
+    const uint8_t* kc = reinterpret_cast<const uint8_t*>(a.k_cache);
+    const uint8_t* vc = reinterpret_cast<const uint8_t*>(a.v_cache);
+    auto load = [&](int i, int st, int page) {
+        const int hp = warp + ATT_WARPS * i;
+        const int left = t_end - pg0 * ATT_PAGE - hp * AM_TOK;           // live tokens from this half page on
+        const size_t off = (((size_t)page * a.n_kv_heads + kvh) * ATT_PAGE + (hp & 1) * AM_TOK) * (size_t)ROWB;
+        const uint32_t dst = ring + st * (2 * HALF);
+#pragma unroll
+        for (int j = 0; j < AM_TOK * CH / 32; ++j) {
+            const int idx = j * 32 + lane, t = idx / CH, c = idx % CH;
+            const uint32_t d = dst + t * ROWB + ((c ^ (t & 7)) << 4);
+            am_cp16(d, kc + off + (size_t)idx * 16, t < left);
+            am_cp16(d + HALF, vc + off + (size_t)idx * 16, t < left);
+        }
+    };
+
+    // queries: three fp16 parts per head in the A fragments, pre-scaled by log2(e) / sqrt(HS) and 2^6
+    uint32_t qf[KS][4];
+    {
+        const float scale = rsqrtf((float)HS) * 1.44269504088896341f * AM_Q_UP;
+        const float* q = a.q + (size_t)m * a.n_heads * HS + (size_t)(kvh * G + (head < G ? head : 0)) * HS + qd * 2;
+#pragma unroll
+        for (int k = 0; k < KS; ++k)
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                float2 x = *reinterpret_cast<const float2*>(q + k * 16 + u * 8);
+                if (head >= G) x = make_float2(0.f, 0.f);
+                __half t0, b0, t1, b1;
+                am_split(x.x * scale, lower, t0, b0);
+                am_split(x.y * scale, lower, t1, b1);
+                qf[k][2 * u] = am_pack(t0, t1);
+                qf[k][2 * u + 1] = am_pack(b0, b1);
+            }
+    }
+    float o[NT][4];
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[n][e] = 0.f;
+    float run_m = -INFINITY, run_l = 0.f;                      // of head g % 4; run_l: this lane's own tokens
+
+#pragma unroll
+    for (int i = 0; i < ST - 1; ++i) {
+        const int page = __shfl_sync(0xffffffffu, my_page, i);
+        if (i < n_my) load(i, i, page);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    int st = 0;
+    for (int i = 0; i < n_my; ++i) {
+        {
+            const int nx = i + ST - 1;
+            if ((nx & 31) == 0) my_page = page_at(nx + lane);
+            const int page = __shfl_sync(0xffffffffu, my_page, nx & 31);
+            if (nx < n_my) load(nx, st == 0 ? ST - 1 : st - 1, page);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        }
+        asm volatile("cp.async.wait_group %0;" ::"n"(ST - 1) : "memory");
+        __syncwarp();
+        const uint32_t kb = ring + st * (2 * HALF), vb = kb + HALF;
+        // scores of 16 tokens: n-tile j = tokens 8 j ..; two short chains over K, then rounded adds
+        float c[2][2][4];
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int u = 0; u < 2; ++u)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) c[j][u][e] = 0.f;
+        {
+            const int t = (lane & 7) + ((lane >> 4) << 3), c1 = (lane >> 3) & 1;
+            const uint32_t base = kb + t * ROWB;
+#pragma unroll
+            for (int k = 0; k < KS; ++k) {
+                uint32_t b[4];
+                am_ldm(b, base + (((2 * k + c1) ^ (t & 7)) << 4));
+                am_mma(c[0][k & 1], qf[k][0], qf[k][1], qf[k][2], qf[k][3], b[0], b[1]);
+                am_mma(c[1][k & 1], qf[k][0], qf[k][1], qf[k][2], qf[k][3], b[2], b[3]);
+            }
+        }
+        const int left = t_end - pg0 * ATT_PAGE - (warp + ATT_WARPS * i) * AM_TOK;
+        float s[4];
+        float mx = -INFINITY;
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                float v = (c[j][0][e] + c[j][1][e]) + (c[j][0][e + 2] + c[j][1][e + 2]);      // rows g and g + 8
+                v += __shfl_xor_sync(0xffffffffu, v, 16);                                     // row g +- 4
+                v = (j * 8 + qd * 2 + e < left) ? v * (1.f / AM_Q_UP) : -INFINITY;
+                s[j * 2 + e] = v;
+                mx = fmaxf(mx, v);
+            }
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+        const float m_new = fmaxf(run_m, mx), m_use = m_new == -INFINITY ? 0.f : m_new;
+        const float corr = am_exp2(run_m - m_use);
+        run_m = m_new;
+        uint32_t pa[4];
+        float ps = 0.f;
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            __half t0, b0, t1, b1;
+            const float p0 = am_exp2(s[2 * j] - m_use + AM_P_UP), p1 = am_exp2(s[2 * j + 1] - m_use + AM_P_UP);
+            ps += p0 + p1;
+            am_split(p0, lower, t0, b0);
+            am_split(p1, lower, t1, b1);
+            pa[2 * j] = am_pack(t0, t1);
+            pa[2 * j + 1] = am_pack(b0, b1);
+        }
+        run_l = fmaf(run_l, corr, ps);
+        {
+            const int t = (lane & 7) + (((lane >> 3) & 1) << 3), c1 = lane >> 4;
+            const uint32_t base = vb + t * ROWB;
+#pragma unroll
+            for (int n = 0; n < NT; n += 2) {
+                uint32_t b[4];
+                am_ldm_trans(b, base + (((n + c1) ^ (t & 7)) << 4));
+                float x[4] = {0.f, 0.f, 0.f, 0.f}, y[4] = {0.f, 0.f, 0.f, 0.f};
+                am_mma(x, pa[0], pa[1], pa[2], pa[3], b[0], b[1]);
+                am_mma(y, pa[0], pa[1], pa[2], pa[3], b[2], b[3]);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    o[n][e] = fmaf(o[n][e], corr, x[e]);
+                    o[n + 1][e] = fmaf(o[n + 1][e], corr, y[e]);
+                }
+            }
+        }
+        __syncwarp();
+        st = st == ST - 1 ? 0 : st + 1;
+    }
+    run_l += __shfl_xor_sync(0xffffffffu, run_l, 1);
+    run_l += __shfl_xor_sync(0xffffffffu, run_l, 2);
+    // row h + row 8 + h, then row 4 + h: lanes of g < 4 hold head g
+    bool bad = !(fabsf(run_l) < INFINITY);
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            float v = o[n][e] + o[n][e + 2];
+            v += __shfl_xor_sync(0xffffffffu, v, 16);
+            o[n][e] = v;
+            bad |= !(fabsf(v) < INFINITY);
+        }
+    bad = __any_sync(0xffffffffu, bad);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();                                           // the ring is done with
+    if (!bad) {
+        if (lower) {
+            float* w = w_acc + (warp * 4 + g) * HS + qd * 2;
+#pragma unroll
+            for (int n = 0; n < NT; ++n) *reinterpret_cast<float2*>(w + n * 8) = make_float2(o[n][0], o[n][1]);
+            if (qd == 0) { w_ml[(warp * 4 + g) * 2] = run_m; w_ml[(warp * 4 + g) * 2 + 1] = run_l; }
+        }
+    } else {
+        // infinities or NaN among this warp's tokens: plain f32, one head at a time, lanes along the head's dimensions
+        constexpr int DPL = HS / 32;
+        const float scale = rsqrtf((float)HS) * 1.44269504088896341f;
+        for (int h = 0; h < G; ++h) {
+            float q[DPL], acc[DPL], M = -INFINITY, Ls = 0.f;
+#pragma unroll
+            for (int d = 0; d < DPL; ++d) { q[d] = a.q[((size_t)m * a.n_heads + kvh * G + h) * HS + lane * DPL + d] * scale; acc[d] = 0.f; }
+            for (int i = 0; i < n_my; ++i) {
+                const int hp = warp + ATT_WARPS * i, page = bt[pg0 + (hp >> 1)];
+                const int n_tok = min(AM_TOK, t_end - pg0 * ATT_PAGE - hp * AM_TOK);
+                for (int t = 0; t < n_tok; ++t) {
+                    const size_t at = (((size_t)page * a.n_kv_heads + kvh) * ATT_PAGE + (hp & 1) * AM_TOK + t) * HS + lane * DPL;
+                    float v = 0.f;
+#pragma unroll
+                    for (int d = 0; d < DPL; ++d) v = fmaf(q[d], __half2float(reinterpret_cast<const __half*>(a.k_cache)[at + d]), v);
+                    v = warp_sum(v);
+                    const float mn = fmaxf(M, v), mu = mn == -INFINITY ? 0.f : mn;
+                    const float cr = am_exp2(M - mu), p = am_exp2(v - mu + AM_P_UP);
+                    M = mn;
+                    Ls = fmaf(Ls, cr, p);
+#pragma unroll
+                    for (int d = 0; d < DPL; ++d) acc[d] = fmaf(acc[d], cr, p * __half2float(reinterpret_cast<const __half*>(a.v_cache)[at + d]));
+                }
+            }
+#pragma unroll
+            for (int d = 0; d < DPL; ++d) w_acc[(warp * 4 + h) * HS + lane * DPL + d] = acc[d];
+            if (lane == 0) { w_ml[(warp * 4 + h) * 2] = M; w_ml[(warp * 4 + h) * 2 + 1] = Ls; }
+        }
+    }
+    __syncthreads();
+
+    // the four warps' shares: thread d < HS owns head dim d (maxima are in units of log2)
+    const bool single = (n_eff == 1);
+    if (tid < HS) {
+        for (int h = 0; h < G; h++) {
+            float Mx = -INFINITY;
+#pragma unroll
+            for (int w = 0; w < ATT_WARPS; w++) Mx = fmaxf(Mx, w_ml[(w * 4 + h) * 2]);
+            const float Mu = (Mx == -INFINITY) ? 0.0f : Mx;
+            float Ls = 0.0f, O = 0.0f;
+#pragma unroll
+            for (int w = 0; w < ATT_WARPS; w++) {
+                const float e = am_exp2(w_ml[(w * 4 + h) * 2] - Mu);
+                Ls += w_ml[(w * 4 + h) * 2 + 1] * e;
+                O += w_acc[(w * 4 + h) * HS + tid] * e;
+            }
+            const int hd = kvh * G + h;
+            if (single) {
+                const float y = (Ls > 0.0f) ? O / Ls : 0.0f;
+                if (a.y_out != nullptr) a.y_out[(size_t)m * a.n_heads * HS + (size_t)hd * HS + tid] = y;
+                if (a.xq_out != nullptr || a.xh_out != nullptr) q80_block_store(y, lane, m, (hd * HS + tid) >> 5, a.out_mcap, a.xq_out, a.xh_out);
+            } else {
+                const size_t pidx = ((size_t)m * a.n_heads + hd) * a.n_splits + sp;
+                a.part_o[pidx * HS + tid] = O;
+                if (tid == 0) { a.part_ml[pidx * 2] = Mx; a.part_ml[pidx * 2 + 1] = Ls; }
+            }
+        }
+    }
+    if (single) { trace_end(a.tr); return; }
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) {
+        const unsigned prev = atomicAdd(&a.counters[m * a.n_kv_heads + kvh], 1u);
+        *s_last = (prev == (unsigned)n_eff - 1u) ? 1 : 0;
+        if (*s_last) a.counters[m * a.n_kv_heads + kvh] = 0u;
+    }
+    __syncthreads();
+    if (!*s_last) { trace_end(a.tr); return; }
+    __threadfence();
+    // warp h merges head h: lane s holds split s's (max, sum), every lane sums its dims over the splits
+    if (warp < G) {
+        constexpr int DPL = HS / 32;
+        const int hd = kvh * G + warp;
+        const size_t base = ((size_t)m * a.n_heads + hd) * a.n_splits;
+        float ms = -INFINITY, ls = 0.0f;
+        if (lane < n_eff) { ms = __ldcg(&a.part_ml[(base + lane) * 2]); ls = __ldcg(&a.part_ml[(base + lane) * 2 + 1]); }
+        const float Mx = warp_max(ms);
+        const float Mu = (Mx == -INFINITY) ? 0.0f : Mx;
+        const float e = (lane < n_eff) ? am_exp2(ms - Mu) : 0.0f;
+        const float Ls = warp_sum(ls * e);
+        float O[DPL];
+#pragma unroll
+        for (int d = 0; d < DPL; d++) O[d] = 0.0f;
+#pragma unroll 4
+        for (int s2 = 0; s2 < n_eff; s2++) {
+            const float es = __shfl_sync(0xffffffffu, e, s2);
+#pragma unroll
+            for (int d = 0; d < DPL; d++) O[d] += __ldcg(&a.part_o[(base + s2) * HS + d * 32 + lane]) * es;
+        }
+        const float inv = (Ls > 0.0f) ? 1.0f / Ls : 0.0f;
+#pragma unroll
+        for (int d = 0; d < DPL; d++) {          // 32 dims at a time: one Q80 block
+            const float y = O[d] * inv;
+            if (a.y_out != nullptr) a.y_out[(size_t)m * a.n_heads * HS + (size_t)hd * HS + d * 32 + lane] = y;
+            if (a.xq_out != nullptr || a.xh_out != nullptr) q80_block_store(y, lane, m, (hd * HS) / 32 + d, a.out_mcap, a.xq_out, a.xh_out);
+        }
+    }
+    trace_end(a.tr);
+}
+
 extern void dl_set_error(const char* fmt, ...);
 
 static size_t att_smem_bytes(int HS, int NCH, int esize) {
@@ -346,6 +683,33 @@ static int launch_att(const AttArgs& a, int pdl, cudaStream_t stream) {
         cfg.numAttrs = 1;
     }
     cudaError_t e = cudaLaunchKernelEx(&cfg, attention_kernel<HS, NCH, KV>, a);
+    if (e != cudaSuccess) { dl_set_error("attention launch: %s", cudaGetErrorString(e)); return -(int)e; }
+    return 0;
+}
+
+template <int HS>
+static int launch_att_mma(const AttArgs& a, int pdl, cudaStream_t stream) {
+    constexpr int smem = ATT_WARPS * 24 * 1024;
+    static_assert(ATT_WARPS * 4 * (HS + 2) * 4 + 4 <= smem, "the merge fits the ring");
+    static bool attr_set = false;
+    if (!attr_set) {
+        cudaError_t e = cudaFuncSetAttribute(attention_mma_kernel<HS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) { dl_set_error("attention smem attr: %s", cudaGetErrorString(e)); return -(int)e; }
+        attr_set = true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(a.n_splits, a.n_kv_heads, a.M);
+    cfg.blockDim = dim3(ATT_WARPS * 32);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    if (pdl) {
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+    }
+    cudaError_t e = cudaLaunchKernelEx(&cfg, attention_mma_kernel<HS>, a);
     if (e != cudaSuccess) { dl_set_error("attention launch: %s", cudaGetErrorString(e)); return -(int)e; }
     return 0;
 }
@@ -390,8 +754,11 @@ extern "C" int dl_attention(const float* q, int M, int n_heads, int n_kv_heads, 
         if (head_size == 64) return launch_att_nch<64, float>(a, G, pdl, st);
         if (head_size == 32) return launch_att_nch<32, float>(a, G, pdl, st);
     } else {
-        if (head_size == 128) return launch_att_nch<128, __half>(a, G, pdl, st);
-        if (head_size == 64) return launch_att_nch<64, __half>(a, G, pdl, st);
+        // up to four query heads per key/value head fill one MMA tile with their three parts; the queries are read as pairs and the
+        // cache in 16-byte pieces (PyTorch's allocations are aligned to 512 bytes, a caller's offset may not be)
+        const bool mma = G <= 4 && ((uintptr_t)q & 7) == 0 && (((uintptr_t)k_cache | (uintptr_t)v_cache) & 15) == 0;
+        if (head_size == 128) return mma ? launch_att_mma<128>(a, pdl, st) : launch_att_nch<128, __half>(a, G, pdl, st);
+        if (head_size == 64) return mma ? launch_att_mma<64>(a, pdl, st) : launch_att_nch<64, __half>(a, G, pdl, st);
         if (head_size == 32) return launch_att_nch<32, __half>(a, G, pdl, st);
     }
     dl_set_error("dl_attention: unsupported head_size %d", head_size);
