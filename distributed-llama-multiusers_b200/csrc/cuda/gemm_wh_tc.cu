@@ -366,6 +366,225 @@ __global__ void __launch_bounds__(512) q40t_to_wh_kernel(const uint8_t* __restri
 extern void dl_set_error(const char* fmt, ...);
 extern "C" int dl_device_sm_count();
 
+// ------------------------------------------------------------------------------------------------
+// Few activation rows (batched decoding of dense-weight models): y[m][r] for M <= WS_MAX_NT rows, epilogues of DL_EPI_DENSE.
+//
+// What bounds it: the weights' bytes.  The 256 x 256 pair tiles above give a 4096-wide output 16 of the 74 pairs, and 28672
+// columns 112 tiles in two waves: norm, gate|up and down of 4096 x 14336 in bf16 at 32 rows took 184 us, 1.9 TB/s
+// (now 86: 47 and 35 us for the products, 5.0 and 3.3 TB/s).  Here the OUTPUT
+// COLUMNS are dealt to all SMs in groups of 8 (one core-matrix row group of the weight image, 2 KB per k tile), so every SM
+// streams the same number of bytes to within 8 rows; a CTA walks the whole K (or its share of a cluster's) once through a
+// ring of bulk copies, MMA M = 128 with the rows past its share reading whatever lies behind (those accumulator lanes are
+// never looked at), and drains once.
+//
+// K split: each cluster of S CTAs reads all activations, (SMs / S) M K against N K of weights, and walks K / S; the shares meet in
+// distributed shared memory, each CTA summing and finishing its part of the activation rows in rank order (ws_split: when).
+// ------------------------------------------------------------------------------------------------
+#define WS_MAX_NT 128
+#define WS_THREADS 352
+#define WS_MAX_ROWS 256                // output columns per CTA: two accumulators of 128 lanes
+#define WS_PIECE 4                     // row groups (2 KB each) per bulk copy
+#define WS_SMEM (208 * 1024)           // ring + what the last stage's MMA reads behind it
+
+struct WsArgs {
+    const uint8_t* wh;
+    const uint8_t* xh;
+    int d_real, R8, KT, ncap, M, NT, S, NS, nacc, stage, tmem_cols, bf16;
+    DlEpilogue epi;
+};
+
+__global__ void __launch_bounds__(WS_THREADS, 1) gemm_wh_rows_kernel(const __grid_constant__ WsArgs a) {
+    extern __shared__ __align__(1024) uint8_t smem[];
+    __shared__ uint64_t full[16], empty[16], acc_full;
+    __shared__ uint32_t tmem_holder;
+    const unsigned long long t0 = globaltimer_ns();
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int S = a.S, KT = a.KT, NT = a.NT;
+    const int crank = S > 1 ? (int)cg::this_cluster().block_rank() : 0;
+    const int c = blockIdx.x / S, n = gridDim.x / S;
+    const int g0 = (int)((long long)a.R8 * c / n), g1 = (int)((long long)a.R8 * (c + 1) / n), ng = g1 - g0;      // this CTA's row groups
+    const int kt0 = KT * crank / S, nk = KT * (crank + 1) / S - kt0;
+    const int nb = (a.M + 7) >> 3;                               // live row groups of the activations
+    const int a_bytes = ng * 2048, b_off = a.stage - NT * 256;   // stage: weights, then activations
+
+    const int nacc = min(a.nacc, nk), acc_step = a.tmem_cols >> 1, tile_step = acc_step >> 1;      // accumulators = issuing warps; columns from one to the next
+    if (tid == 0) {
+        for (int s = 0; s < a.NS; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+        mbar_init(&acc_full, nacc);
+        mbar_fence_init();
+    }
+    if (warp == 1) tmem_alloc(&tmem_holder, a.tmem_cols);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_holder;
+    pdl_launch_dependents();
+
+    if (warp == 0) {
+        // lane = one bulk copy per stage: pieces of the weights' row groups (cut at the image's 128-row tiles), then of the activations
+        const uint8_t* src = nullptr;
+        size_t step = 0;
+        uint32_t bytes = 0, dst = 0;
+        int l = 0;
+        for (int g = g0; g < g1; l++) {
+            const int len = min(min(WS_PIECE, g1 - g), 16 - (g & 15));
+            if (l == lane) {
+                src = a.wh + ((size_t)(g >> 4) * KT + kt0) * WH_TILE_BYTES + (size_t)(g & 15) * 2048;
+                step = WH_TILE_BYTES;
+                bytes = len * 2048;
+                dst = (g - g0) * 2048;
+            }
+            g += len;
+        }
+        const bool is_w = bytes != 0;
+        for (int g = 0; g < nb; g += WS_PIECE, l++) {
+            if (l == lane) {
+                src = a.xh + ((size_t)kt0 * (a.ncap >> 3) + g) * 2048;
+                step = (size_t)(a.ncap >> 3) * 2048;
+                bytes = min(WS_PIECE, nb - g) * 2048;
+                dst = b_off + g * 2048;
+            }
+        }
+        if (!is_w && bytes) pdl_wait();                          // weights do not depend on the previous kernel
+        for (int i = 0; i < nk; i++) {
+            const int s = i % a.NS;
+            if (i >= a.NS) wt_wait(&empty[s], ((i / a.NS) & 1) ^ 1, t0);
+            if (lane == 0) mbar_arrive_expect_tx(&full[s], a_bytes + nb * 2048);
+            if (bytes) bulk_g2s(smem + (size_t)s * a.stage + dst, src + (size_t)i * step, bytes, &full[s]);
+        }
+    } else if (warp <= nacc) {
+        // up to two warps issue in turn, each into accumulators of its own (the drain adds them): a k tile costs its issuing thread ~570 clk of
+        // waits and issue, more than the bytes of a narrow share take to arrive
+        const int mw = warp - 1;
+        const uint32_t idesc = umma_idesc_f16_f32(128, NT) | (a.bf16 ? ((1u << 7) | (1u << 10)) : 0u);
+        const uint32_t desc_hi = (2048u >> 4) | (1u << 14);      // SBO 2048 B, descriptor version 1
+        const int tiles = ng > 16 ? 2 : 1;
+        for (int i = mw; i < nk; i += nacc) {
+            const int s = i % a.NS;
+            wt_wait(&full[s], (i / a.NS) & 1, t0);
+            tc_fence_after();
+            if (elect_one()) {
+                const uint32_t sa = smem_u32(smem + (size_t)s * a.stage);
+                const uint32_t b_lo = (((sa + b_off) & 0x3FFFFu) >> 4) | ((128u >> 4) << 16);
+                for (int t = 0; t < tiles; t++) {
+                    const uint32_t a_lo = (((sa + t * WH_TILE_BYTES) & 0x3FFFFu) >> 4) | ((128u >> 4) << 16);
+#pragma unroll
+                    for (int j = 0; j < 8; j++) {
+                        uint64_t da, db;
+                        asm("mov.b64 %0, {%1, %2};" : "=l"(da) : "r"(a_lo + j * 16), "r"(desc_hi));
+                        asm("mov.b64 %0, {%1, %2};" : "=l"(db) : "r"(b_lo + j * 16), "r"(desc_hi));
+                        umma_f16_ss(tmem + mw * acc_step + t * tile_step, da, db, idesc, (i > mw || j > 0) ? 1u : 0u);
+                    }
+                }
+                umma_commit(&empty[s]);
+                if (i + nacc >= nk) umma_commit(&acc_full);
+            }
+            __syncwarp();
+        }
+    }
+    // accumulators -> shared memory [m][rows] in the ring's place (every copy has landed and every MMA is done)
+    wt_wait(&acc_full, 0, t0);
+    tc_fence_after();
+    float* out_s = reinterpret_cast<float*>(smem);
+    const int rows = ng * 8;
+    if (warp >= 3) {
+        const int q = warp & 3, half = (warp - 3) >> 2;           // TMEM lane quarter; the other four warps take every other 8 columns
+        for (int t = 0; t * 128 < rows; t++) {
+            const int r = t * 128 + q * 32 + lane;
+            if (t * 128 + q * 32 >= rows) break;
+            for (int m = half * 8; m < a.M; m += 16) {
+                const uint32_t at = tmem + ((uint32_t)(q * 32) << 16) + t * tile_step + m;
+                uint32_t v[8], w[8];
+                tmem_ld_32x32b_x8(at, v);
+                if (nacc > 1) tmem_ld_32x32b_x8(at + acc_step, w);
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 8; j++)
+                    if (r < rows && m + j < a.M) out_s[(m + j) * rows + r] = __uint_as_float(v[j]) + (nacc > 1 ? __uint_as_float(w[j]) : 0.f);
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem, a.tmem_cols); }
+    int m0 = 0, m1 = a.M;
+    if (S > 1) {
+        cg::cluster_group cluster = cg::this_cluster();
+        cluster.sync();
+        m0 = a.M * crank / S;
+        m1 = a.M * (crank + 1) / S;
+        for (int i = m0 * rows + tid; i < m1 * rows; i += WS_THREADS) {
+            float v = 0.f;
+            for (int k = 0; k < S; k++) v += cluster.map_shared_rank(out_s, k)[i];
+            out_s[i] = v;                                          // nobody else reads these rows
+        }
+        cluster.sync();                                            // no peer still reads this CTA's memory when it leaves
+    }
+    pdl_wait();
+    const bool pair = a.epi.dense_op == DL_DENSE_GLU_CLAMP || a.epi.dense_op == DL_DENSE_GLU_SILU || a.epi.dense_op == DL_DENSE_GLU_GELU;
+    const int na = pair ? rows >> 1 : rows, step = na ? max(1, WS_THREADS / na) : 1;      // threads along the columns, several rows at a time
+    for (int t = tid; t < na * step; t += WS_THREADS)
+        epilogue_rows(a.epi, out_s + m0 * rows, rows, rows, g0 * 8, a.d_real, m1 - m0, m0, t % na, t / na, step);
+}
+
+// CTAs per cluster that share K: shares of fewer than 5 row groups (40 columns) leave an SM more activations than weights to read and
+// too many k tiles to walk; a pair halves both (32 rows, us with 1 / 2 / 4: 4096 x 14336 45 / 35 / 44, 2048 x 8192 36 / 19 / 29, 128 x 2048
+// 11 / 10 / 10; but 6144 x 2048 at 100 rows 21 / 21 / 41, 16384 x 2048 19 / 25 / 41, 28672 x 4096 47 / 60 / 82)
+static int ws_split(int R8, int KT, int n_sms) { return R8 < 5 * n_sms && KT >= 2 ? 2 : 1; }
+
+static int gemm_wh_rows_launch(const uint8_t* wh, int d, int n, const uint8_t* xh, int ncap, int M, const DlEpilogue* epi, int bf16,
+                               int pdl, cudaStream_t stream, int n_sms) {
+    WsArgs a;
+    a.wh = wh; a.xh = xh; a.d_real = d; a.R8 = (d + 7) / 8; a.KT = n / 128; a.ncap = ncap; a.M = M;
+    a.NT = (M + 15) / 16 * 16;
+    a.bf16 = bf16; a.epi = *epi;
+    a.S = ws_split(a.R8, a.KT, n_sms);
+    const int slots = n_sms / a.S;
+    int clusters = a.R8 < slots ? a.R8 : slots;
+    clusters *= (a.R8 + clusters * (WS_MAX_ROWS / 8) - 1) / (clusters * (WS_MAX_ROWS / 8));      // more columns than one wave holds
+    const int ng = (a.R8 + clusters - 1) / clusters;
+    a.stage = ng * 2048 + a.NT * 256;
+    // an MMA reads 128 (256) rows of weights from the start of its stage whatever the CTA's share is
+    const int over = (ng > 16 ? 2 : 1) * WH_TILE_BYTES > a.stage ? (ng > 16 ? 2 : 1) * WH_TILE_BYTES - a.stage : 0;
+    a.NS = (WS_SMEM - over) / a.stage;
+    if (a.NS > 16) a.NS = 16;
+    // A stage must belong to ONE issuer: with an odd count its uses would alternate between the two, and an issuer that runs ahead
+    // would take the parity of the use before last for its own.  Odd counts are those of wide shares, whose bytes cover one issuer.
+    a.nacc = a.NS % 2 == 0 ? 2 : 1;
+    a.tmem_cols = 32;
+    while (a.tmem_cols < 4 * a.NT) a.tmem_cols *= 2;            // two issuers x two tiles
+    static bool attr_set = false;
+    if (!attr_set) {
+        cudaError_t e = cudaFuncSetAttribute(gemm_wh_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, WS_SMEM);
+        if (e != cudaSuccess) { dl_set_error("gemm wh rows smem attr: %s", cudaGetErrorString(e)); return -(int)e; }
+        attr_set = true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(clusters * a.S));
+    cfg.blockDim = dim3(WS_THREADS);
+    cfg.dynamicSmemBytes = WS_SMEM;
+    cfg.stream = stream;
+    cudaLaunchAttribute attrs[2];
+    int na = 0;
+    if (a.S > 1) {
+        attrs[na].id = cudaLaunchAttributeClusterDimension;
+        attrs[na].val.clusterDim.x = a.S;
+        attrs[na].val.clusterDim.y = 1;
+        attrs[na].val.clusterDim.z = 1;
+        na++;
+    }
+    if (pdl) {
+        attrs[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attrs[na].val.programmaticStreamSerializationAllowed = 1;
+        na++;
+    }
+    cfg.attrs = attrs;
+    cfg.numAttrs = na;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_wh_rows_kernel, a);
+    if (e != cudaSuccess) { dl_set_error("gemm wh rows launch: %s", cudaGetErrorString(e)); return -(int)e; }
+    return 0;
+}
+
 static int g_wh_dbg = 0, g_wh_pf_dist = 0, g_wh_pf_mask = 0, g_wh_piece = 16384;      // bytes per bulk copy: 16 KB pieces (4 / 8 KB measured: no gain)
 extern "C" void dl_debug_set_wh_piece(int b) { if (b == 4096 || b == 8192 || b == 16384) g_wh_piece = b; }
 extern "C" void dl_debug_set_wh_mode(int m) { g_wh_dbg = m; }
@@ -389,6 +608,9 @@ static int gemm_wh_launch(const uint8_t* wh, int d, int n, const uint8_t* xh, in
     if (n % 128 != 0) { dl_set_error("dl_gemm_wh_tc: n=%d not a multiple of 128", n); return -1; }
     if (M < 1 || ncap % 8 != 0 || ncap < M) { dl_set_error("dl_gemm_wh_tc: bad M=%d / ncap=%d", M, ncap); return -1; }
     if (epi->kind == DL_EPI_SILU_MUL && d % 64 != 0) { dl_set_error("dl_gemm_wh_tc: silu epilogue needs d%%64==0"); return -1; }
+    // few rows: all SMs stream equal shares of the weights (force_cg bit 0 keeps the tiles below, for comparisons)
+    if (epi->kind == DL_EPI_DENSE && grp == nullptr && M <= WS_MAX_NT && !(force_cg & 1))
+        return gemm_wh_rows_launch(wh, d, n, xh, ncap, M, epi, (force_cg & 2) ? 1 : 0, pdl, (cudaStream_t)stream, dl_device_sm_count());
     WhArgs a;
     a.wh = wh; a.xh = xh; a.d_real = d;
     a.row_tiles = (d + 127) / 128;

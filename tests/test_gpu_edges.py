@@ -43,3 +43,37 @@ def test_decode_attention_half_pages(heads, kv, hs, n_splits):
     got = y.cpu().double().view(M, heads, hs)
     assert torch.isfinite(got).all()
     assert (got - want).abs().max() <= 2e-6 * want.abs().max()
+
+
+@pytest.mark.parametrize("M,N,K_", [(1, 8, 128), (7, 200, 128), (32, 1000, 384), (33, 6000, 256), (64, 40, 1024), (100, 2056, 512), (127, 7000, 128),
+                                    (128, 40008, 128), (128, 5888, 640)])
+def test_dense_rows_shares(M, N, K_):
+    """Few-row products: shares that end inside a 128-column tile, one and two accumulators, odd and even ring depths, one k tile, more
+    columns than one wave of CTAs holds, clusters that split K.  bf16 products are exact in f32; a tensor-core chain of K / 16 steps
+    truncates, each step by at most 2^-22 of the largest partial sum: 1e-5 relative covers K = 1024 several times over."""
+    g = torch.Generator(device="cuda").manual_seed(N + M)
+    w = (torch.randn(N, K_, generator=g, device="cuda") * K_ ** -0.5).bfloat16()
+    x, ncap = torch.randn(M, K_, generator=g, device="cuda"), (M + 7) // 8 * 8
+    bias, aux = torch.randn(N, generator=g, device="cuda"), torch.randn(M, N, generator=g, device="cuda")
+    xh = torch.zeros(L().xh_bytes(K_, ncap), dtype=torch.uint8, device="cuda")
+    L().xh_from_rows(x, M, K_, ncap, xh)
+    wh, z = L().make_wh(w), x.bfloat16().double() @ w.double().t()
+
+    def close(y, want):
+        assert (y.double() - want).norm() <= 1e-5 * want.norm() + 1e-12
+
+    y = torch.full((M + 2, N + 3), 7.0, device="cuda")
+    L().dense_tc(wh, N, K_, xh, ncap, y, M, bias=bias)
+    close(y[:M, :N], z + bias.double())
+    assert (y[M:] == 7).all() and (y[:, N:] == 7).all()          # nothing past the rows and columns asked for
+    L().dense_tc(wh, N, K_, xh, ncap, y, M, epi=L().DENSE_SIGMOID_MUL, aux=aux)
+    close(y[:M, :N], aux.double() * z.sigmoid())
+    half = torch.zeros(M, N // 2, device="cuda")
+    L().dense_tc(wh, N, K_, xh, ncap, half, M, epi=L().DENSE_GLU_GELU)
+    close(half, torch.nn.functional.gelu(z[:, 0::2], approximate="tanh") * z[:, 1::2])
+    if N % 256 == 0:
+        img, direct = (torch.zeros(L().xh_bytes(N // 2, ncap), dtype=torch.uint8, device="cuda") for _ in range(2))
+        L().dense_tc(wh, N, K_, xh, ncap, half, M, epi=L().DENSE_GLU_GELU, image=(img, ncap))
+        L().xh_from_rows(half, M, N // 2, ncap, direct)
+        live = lambda t: t.view(-1, ncap // 8, 16, 8, 16).permute(1, 3, 0, 2, 4).reshape(ncap, -1)[:M]
+        assert torch.equal(live(img), live(direct))
