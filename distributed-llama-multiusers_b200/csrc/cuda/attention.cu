@@ -321,8 +321,8 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attention_kernel(const __grid_
 //
 // What bounds it: the cache's bytes.  The FMA kernel above spends ~480 instructions per 8 tokens and warp (a 31-shuffle
 // reduction of the scores, four f32 conversions and shuffled weights per token) and keeps 7 warps per SM busy: 91 us at 32 rows
-// of 1500 to 3000 tokens (8 kv heads of 128), 3.3 TB/s.  Here a warp takes 16 tokens at a time through 32 MMAs: 56 us,
-// 5.4 TB/s, and the distance to a 64-bit result went from 4.5e-7 to 3.0e-7.
+// of 1500 to 3000 tokens (8 kv heads of 128), 3.3 TB/s.  Here a warp takes 16 tokens at a time through 32 MMAs: 54 us,
+// 5.5 TB/s, and the distance to a 64-bit result went from 4.5e-7 to 3.0e-7.
 //
 // Nothing is rounded to 16 bits: keys and values ARE fp16, and an f32 query (or softmax weight) is the exact sum of three fp16
 // numbers, q = q1 + q2 + q3 (11 bits each).  One 16-row MMA tile holds the splits of all four heads -- row h: q1 of head h,
@@ -366,10 +366,10 @@ DL_DEVINL void am_split(float v, bool lower, __half& top, __half& bot) {
 }
 
 template <int HS>
-__global__ void __launch_bounds__(ATT_WARPS * 32, 2) attention_mma_kernel(const __grid_constant__ AttArgs a) {
+__global__ void __launch_bounds__(ATT_WARPS * 32, 3) attention_mma_kernel(const __grid_constant__ AttArgs a) {
     constexpr int ROWB = HS * 2, CH = ROWB / 16;               // bytes / 16-byte chunks of a token's line
     constexpr int HALF = AM_TOK * ROWB;                        // K (or V) of a half page
-    constexpr int ST = HS == 128 ? 3 : 6;                      // ring stages per warp (24 KB)
+    constexpr int ST = HS == 128 ? 2 : 4;                      // ring stages per warp (16 KB)
     constexpr int KS = HS / 16, NT = HS / 8;
     extern __shared__ __align__(128) uint8_t smem[];
     trace_begin(a.tr);
@@ -397,6 +397,14 @@ __global__ void __launch_bounds__(ATT_WARPS * 32, 2) attention_mma_kernel(const 
     const int g = lane >> 2, qd = lane & 3, head = g & 3;
     const bool lower = g < 4;
 
+    float2 qr[KS][2];
+    {
+        const float* q = a.q + (size_t)m * a.n_heads * HS + (size_t)(kvh * G + (head < G ? head : 0)) * HS + qd * 2;
+#pragma unroll
+        for (int k = 0; k < KS; ++k)
+#pragma unroll
+            for (int u = 0; u < 2; ++u) qr[k][u] = *reinterpret_cast<const float2*>(q + k * 16 + u * 8);
+    }
     // this warp's half page i: page pg0 + (w + 4 i) / 2; the lanes hold the next 32 page numbers
     auto page_at = [&](int i) { const int p = pg0 + ((warp + ATT_WARPS * i) >> 1); return i < n_my ? bt[p] : 0; };
     int my_page = page_at(lane);
@@ -416,24 +424,25 @@ __global__ void __launch_bounds__(ATT_WARPS * 32, 2) attention_mma_kernel(const 
         }
     };
 
+#pragma unroll
+    for (int i = 0; i < ST - 1; ++i) {
+        const int page = __shfl_sync(0xffffffffu, my_page, i);
+        if (i < n_my) load(i, i, page);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
     // queries: three fp16 parts per head in the A fragments, pre-scaled by log2(e) / sqrt(HS) and 2^6
     uint32_t qf[KS][4];
-    {
-        const float scale = rsqrtf((float)HS) * 1.44269504088896341f * AM_Q_UP;
-        const float* q = a.q + (size_t)m * a.n_heads * HS + (size_t)(kvh * G + (head < G ? head : 0)) * HS + qd * 2;
+    const float scale = rsqrtf((float)HS) * 1.44269504088896341f * AM_Q_UP;
 #pragma unroll
-        for (int k = 0; k < KS; ++k)
+    for (int k = 0; k < KS; ++k)
 #pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                float2 x = *reinterpret_cast<const float2*>(q + k * 16 + u * 8);
-                if (head >= G) x = make_float2(0.f, 0.f);
-                __half t0, b0, t1, b1;
-                am_split(x.x * scale, lower, t0, b0);
-                am_split(x.y * scale, lower, t1, b1);
-                qf[k][2 * u] = am_pack(t0, t1);
-                qf[k][2 * u + 1] = am_pack(b0, b1);
-            }
-    }
+        for (int u = 0; u < 2; ++u) {
+            __half t0, b0, t1, b1;
+            am_split(head < G ? qr[k][u].x * scale : 0.f, lower, t0, b0);
+            am_split(head < G ? qr[k][u].y * scale : 0.f, lower, t1, b1);
+            qf[k][2 * u] = am_pack(t0, t1);
+            qf[k][2 * u + 1] = am_pack(b0, b1);
+        }
     float o[NT][4];
 #pragma unroll
     for (int n = 0; n < NT; ++n)
@@ -441,12 +450,6 @@ __global__ void __launch_bounds__(ATT_WARPS * 32, 2) attention_mma_kernel(const 
         for (int e = 0; e < 4; ++e) o[n][e] = 0.f;
     float run_m = -INFINITY, run_l = 0.f;                      // of head g % 4; run_l: this lane's own tokens
 
-#pragma unroll
-    for (int i = 0; i < ST - 1; ++i) {
-        const int page = __shfl_sync(0xffffffffu, my_page, i);
-        if (i < n_my) load(i, i, page);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    }
     int st = 0;
     for (int i = 0; i < n_my; ++i) {
         {
@@ -689,7 +692,7 @@ static int launch_att(const AttArgs& a, int pdl, cudaStream_t stream) {
 
 template <int HS>
 static int launch_att_mma(const AttArgs& a, int pdl, cudaStream_t stream) {
-    constexpr int smem = ATT_WARPS * 24 * 1024;
+    constexpr int smem = ATT_WARPS * 16 * 1024;
     static_assert(ATT_WARPS * 4 * (HS + 2) * 4 + 4 <= smem, "the merge fits the ring");
     static bool attr_set = false;
     if (!attr_set) {
