@@ -77,3 +77,27 @@ def test_dense_rows_shares(M, N, K_):
         L().xh_from_rows(half, M, N // 2, ncap, direct)
         live = lambda t: t.view(-1, ncap // 8, 16, 8, 16).permute(1, 3, 0, 2, 4).reshape(ncap, -1)[:M]
         assert torch.equal(live(img), live(direct))
+
+
+@pytest.mark.parametrize("M", [1, 2, 3, 8])
+def test_gemv_extreme_nibbles(M):
+    """The largest products of a block (nibbles 0 and 15, activations of +-127) through the integer-to-float step, and every sign mixed:
+    integers below 2^20 times one scale are exact in f32, a row of 4 such blocks to its last additions (4 * 2^-24)."""
+    d, n = 256, 512
+    g = torch.Generator().manual_seed(M)
+    nib = torch.randint(0, 16, (d, n // 32, 32), generator=g, dtype=torch.uint8)
+    nib[0::4], nib[1::4] = 15, 0
+    nib[2::4, :, ::2], nib[2::4, :, 1::2] = 15, 0
+    scale = torch.full((d, n // 32, 1), 0.5).half()
+    raw = torch.cat([scale.view(torch.uint8), nib[:, :, :16] | (nib[:, :, 16:] << 4)], dim=2)
+    x = torch.where(torch.rand(M, n, generator=g) < 0.5, -1.0, 1.0)
+    x[0], x[M - 1, ::2] = 1.0, -1.0
+    k = K()
+    xq = k.alloc_xq(n, M, "cuda")
+    k.quant_q80(x.cuda(), M, n, M, xq_out=xq)
+    y = torch.zeros(M, d, device="cuda")
+    k.gemv_q40(k.make_q40t(raw.reshape(-1).cuda(), d, n), d, n, xq, M, k.epi_store([y.data_ptr()], d))
+    w = (nib.double() - 8).reshape(d, n) * 0.5
+    xd = x.double().sign() * 127 * float(torch.tensor(1 / 127).half())
+    want = xd @ w.t()
+    assert (y.cpu().double() - want).abs().max() <= 2.0 ** -21 * want.abs().max()
