@@ -41,6 +41,7 @@ struct TcArgs {
     int d_real, d_pad, KT, ncap, M, NT, S;
     int NSA, NSB, nsb_log;
     int nstg;              // A stages in TMEM (64 columns each), at columns [512 - 64*nstg, 512)
+    int pair;              // 1: this CTA multiplies row tiles 2c and 2c + 1 side by side (item i = row tile i & 1, k-tile i >> 1; one accumulator each)
     int nacc;              // MMA-issuing warps = independent TMEM accumulators (1, 2 or 4; nacc*NT <= 256), summed by the epilogue
     int LA, LB;            // issuing lanes per ring; each divides its stage count so a stage has ONE owner lane
     int n_epi_ctas;
@@ -75,12 +76,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_q40_tc_kernel(const __grid
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int S = a.S;
     const int crank = (S > 1) ? (int)cg::this_cluster().block_rank() : 0;
-    const int rt = blockIdx.x / S;
+    const int P = a.pair ? 2 : 1;
+    const int rt = (int)(blockIdx.x / S) * P;      // first row tile
     const int m0 = blockIdx.y * NT;
     const int Mt = min(NT, a.M - m0);
     const int kt0 = (a.KT * crank) / S, kt1 = (a.KT * (crank + 1)) / S;
     const int nk = kt1 - kt0;
-    const int nacc = (a.nacc <= nk) ? a.nacc : (nk >= 2 ? 2 : 1);      // accumulators in use = MMA-issuing warps (power of two)
+    const int n_it = nk * P;               // items: weight tiles of this CTA
+    const int nacc = a.pair ? 2 : (a.nacc <= nk) ? a.nacc : (nk >= 2 ? 2 : 1);      // accumulators in use = MMA-issuing warps (power of two)
 
     if (tid == 0) {
         for (int s = 0; s < 16; s++) {
@@ -89,7 +92,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_q40_tc_kernel(const __grid
         }
         for (int s = 0; s < 8; s++) {
             mbar_init(&fullB[s], 1);
-            mbar_init(&emptyB[s], 1);
+            mbar_init(&emptyB[s], P);
             mbar_init(&fullH[s], 4);
             mbar_init(&emptyH[s], 1);
         }
@@ -117,27 +120,29 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_q40_tc_kernel(const __grid
         const uint8_t* xb = a.xh + (size_t)kt0 * (a.ncap >> 3) * XH_ROWGROUP_BYTES + (size_t)(m0 >> 3) * XH_ROWGROUP_BYTES;
         const size_t x_kt_stride = (size_t)(a.ncap >> 3) * XH_ROWGROUP_BYTES;
         const uint64_t pol = l2_policy_evict_first();
+        const int n_role = role_a ? n_it : nk;
         int i = role_a ? lane : (role_b ? lane - 4 : nk);
         const int step = role_a ? a.LA : a.LB;
+        auto tile_of = [&](int it) { return wt + (P == 2 ? (size_t)(it & 1) * a.KT + (it >> 1) : (size_t)it) * Q40T_TILE_BYTES; };
         if (role_a) {
             // weights do not depend on the previous kernel: fill the whole ring before the PDL wait
-            for (; i < nk && i < a.NSA; i += step) {
+            for (; i < n_it && i < a.NSA; i += step) {
                 if (!(a.dbg_mode & 4)) TC_DBG(0, i);
                 mbar_arrive_expect_tx(&fullA[i], Q40T_TILE_BYTES);
-                bulk_g2s_hint(ringA + i * Q40T_TILE_BYTES, wt + (size_t)i * Q40T_TILE_BYTES, Q40T_TILE_BYTES, &fullA[i], pol);
+                bulk_g2s_hint(ringA + i * Q40T_TILE_BYTES, tile_of(i), Q40T_TILE_BYTES, &fullA[i], pol);
             }
         }
         __syncwarp();
         pdl_wait();
-        while (__any_sync(0xffffffffu, i < nk)) {
+        while (__any_sync(0xffffffffu, i < n_role)) {
             bool issued = false;
-            if (i < nk) {
+            if (i < n_role) {
                 if (role_a) {
                     const int sa = i % a.NSA;
                     if (mbar_test_wait(&emptyA[sa], ((i / a.NSA) & 1) ^ 1)) {      // i >= NSA here
                         if (!(a.dbg_mode & 4)) TC_DBG(0, i);
                         mbar_arrive_expect_tx(&fullA[sa], Q40T_TILE_BYTES);
-                        bulk_g2s_hint(ringA + sa * Q40T_TILE_BYTES, wt + (size_t)i * Q40T_TILE_BYTES, Q40T_TILE_BYTES, &fullA[sa], pol);
+                        bulk_g2s_hint(ringA + sa * Q40T_TILE_BYTES, tile_of(i), Q40T_TILE_BYTES, &fullA[sa], pol);
                         i += step;
                         issued = true;
                     }
@@ -177,8 +182,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_q40_tc_kernel(const __grid
         const uint32_t a_col0 = TC_TMEM_COLS - nstg * TC_A_STAGE_COLS;
         if (mw < nacc) {
             int sh = mw, ph = 0;      // A stage of k-tile i = i % nstg, phase parity = (i / nstg) & 1
-            for (int i = mw; i < nk; i += nacc) {
-                const int sb = i & nsb_mask, pb = (i >> nsb_log) & 1;
+            for (int i = mw; i < n_it; i += nacc) {
+                const int k = a.pair ? i >> 1 : i;
+                const int sb = k & nsb_mask, pb = (k >> nsb_log) & 1;
                 if (det && stamp) TC_DBG(0, i);
                 mbar_wait_sleep(&fullH[sh], ph, mma_sleep);
                 if (stamp) TC_DBG(det ? 1 : 5, i);
@@ -199,7 +205,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_q40_tc_kernel(const __grid
                     if (det && mw == 0) TC_DBG(4, i);
                     umma_commit(&emptyH[sh]);          // implicit tcgen05.fence::before_thread_sync
                     umma_commit(&emptyB[sb]);
-                    if (i + nacc >= nk) umma_commit(accum_full);      // this warp's last k-tile
+                    if (i + nacc >= n_it) umma_commit(accum_full);      // this warp's last k-tile
                     if (det && mw == 0) TC_DBG(6, i);
                 }
                 __syncwarp();
@@ -230,7 +236,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_q40_tc_kernel(const __grid
         const int nsa = a.NSA;
         int sh = g, ph = 0;      // A stage of k-tile i = i % nstg (g < 4 <= nstg), phase parity = (i / nstg) & 1
         int sa = g, pa = 0;      // raw ring stage i % NSA and its phase parity
-        for (int i = g; i < nk; i += TC_GROUPS) {
+        for (int i = g; i < n_it; i += TC_GROUPS) {
             mbar_wait_sleep(&fullA[sa], pa, 32);
             if (stamp) TC_DBG(1, i);
             const uint8_t* raw = ringA + sa * Q40T_TILE_BYTES;
@@ -302,58 +308,75 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_q40_tc_kernel(const __grid
         if (tid == 64) TC_DBG(2, 63);
     }
     const int n_chunks = (Mt + TC_EPI_CHUNK - 1) / TC_EPI_CHUNK;
-    for (int ch = 0; ch < n_chunks; ch++) {
-        const int mc = min(TC_EPI_CHUNK, Mt - ch * TC_EPI_CHUNK);
-        if (is_epi) {
-            const uint32_t taddr = tmem_base + ((uint32_t)(eq * 32) << 16) + (uint32_t)(ch * TC_EPI_CHUNK);
-            const int ncol = min(TC_EPI_CHUNK, NT - ch * TC_EPI_CHUNK);
-            const int c0 = eg * 8;
-            if (c0 < ncol) {
-                uint32_t v[8];
-                tmem_ld_32x32b_x8(taddr + c0, v);
+    // columns [8 eg, 8 eg + 8) of chunk ch of row tile rt + h -> dst[column][128] (with one row tile: the sum over the accumulators)
+    auto drain = [&](int h, int ch, float* dst) {
+        const uint32_t taddr = tmem_base + ((uint32_t)(eq * 32) << 16) + (uint32_t)(h * NT + ch * TC_EPI_CHUNK);
+        const int ncol = min(TC_EPI_CHUNK, NT - ch * TC_EPI_CHUNK);
+        const int c0 = eg * 8;
+        if (c0 < ncol) {
+            uint32_t v[8];
+            tmem_ld_32x32b_x8(taddr + c0, v);
+            tmem_ld_wait();
+            float f[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++) f[j] = __uint_as_float(v[j]);
+            for (int ac = 1; ac < nacc && !a.pair; ac++) {
+                tmem_ld_32x32b_x8(taddr + c0 + ac * NT, v);
                 tmem_ld_wait();
-                float f[8];
 #pragma unroll
-                for (int j = 0; j < 8; j++) f[j] = __uint_as_float(v[j]);
-                for (int ac = 1; ac < nacc; ac++) {
-                    tmem_ld_32x32b_x8(taddr + c0 + ac * NT, v);
-                    tmem_ld_wait();
-#pragma unroll
-                    for (int j = 0; j < 8; j++) f[j] += __uint_as_float(v[j]);
-                }
-#pragma unroll
-                for (int j = 0; j < 8; j++) out_s[(c0 + j) * 128 + etid] = f[j];
+                for (int j = 0; j < 8; j++) f[j] += __uint_as_float(v[j]);
             }
+#pragma unroll
+            for (int j = 0; j < 8; j++) dst[(c0 + j) * 128 + etid] = f[j];
         }
-        if (S > 1) {
-            // split-K: every rank publishes its partial chunk, the leader sums them over DSMEM and runs the
-            // epilogue; all threads of the cluster take part in both syncs
-            cg::cluster_group cluster = cg::this_cluster();
-            tc_fence_before();
-            cluster.sync();
-            if (crank == 0) {
-                for (int idx = tid; idx < mc * 128; idx += TC_THREADS) {
-                    float v = out_s[idx];
-                    for (int c = 1; c < S; c++) v += cluster.map_shared_rank(out_s, c)[idx];
-                    out_s[idx] = v;
-                }
-            }
-            cluster.sync();
-            if (crank == 0 && is_epi) {
-                pdl_wait();
-                epilogue_rows(a.epi, out_s, 128, 128, rt * 128, a.d_real, mc, m0 + ch * TC_EPI_CHUNK, etid, eg, TC_GROUPS);
-                if (ch + 1 < n_chunks) asm volatile("bar.sync 1, 512;");      // out_s is rewritten by the next chunk
-            }
-        } else if (is_epi) {
-            if (tid == 64 && ch == 0) TC_DBG(4, 63);
-            asm volatile("bar.sync 1, 512;");
+    };
+    if (S > 1) {
+        // split-K: every rank publishes its partial tile(s) in the rings' place, then sums and finishes ITS share of the activation rows
+        // over DSMEM, in rank order.  (One rank finishing all rows chunk by chunk took two cluster barriers and S - 1 remote reads of
+        // 16 KB per 32 rows.)
+        float* all_s = reinterpret_cast<float*>(smem);               // [P][NT][128]
+        cg::cluster_group cluster = cg::this_cluster();
+        if (is_epi) {
+            for (int h = 0; h < P; h++)
+                for (int ch = 0; ch < n_chunks; ch++) drain(h, ch, all_s + ((size_t)h * NT + ch * TC_EPI_CHUNK) * 128);
+        }
+        tc_fence_before();
+        cluster.sync();
+        if (is_epi) {
+            const int ms = Mt * crank / S, me = Mt * (crank + 1) / S;
             pdl_wait();
-            if (tid == 64 && ch == 0) TC_DBG(5, 63);
-            epilogue_rows(a.epi, out_s, 128, 128, rt * 128, a.d_real, mc, m0 + ch * TC_EPI_CHUNK, etid, eg, TC_GROUPS);
-            if (tid == 64 && ch == 0) TC_DBG(6, 63);
-            asm volatile("bar.sync 1, 512;");
-            if (tid == 64 && ch == 0) TC_DBG(7, 63);
+            for (int h = 0; h < P; h++)
+                for (int mb = ms; mb < me; mb += TC_EPI_CHUNK) {
+                    const int mc = min(TC_EPI_CHUNK, me - mb);
+                    const size_t base = ((size_t)h * NT + mb) * 128;
+                    for (int idx = tid - 64; idx < mc * 32; idx += TC_DEQ_WARPS * 32) {
+                        float4 v = *reinterpret_cast<const float4*>(cluster.map_shared_rank(all_s, 0) + base + idx * 4);
+                        for (int c = 1; c < S; c++) {
+                            const float4 x = *reinterpret_cast<const float4*>(cluster.map_shared_rank(all_s, c) + base + idx * 4);
+                            v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
+                        }
+                        reinterpret_cast<float4*>(out_s)[idx] = v;
+                    }
+                    asm volatile("bar.sync 1, 512;" ::: "memory");
+                    epilogue_rows(a.epi, out_s, 128, 128, (rt + h) * 128, a.d_real, mc, m0 + mb, etid, eg, TC_GROUPS);
+                    asm volatile("bar.sync 1, 512;" ::: "memory");      // out_s is rewritten by the next round
+                }
         }
+        cluster.sync();      // nobody leaves while a peer may still read its share
+    } else if (is_epi) {
+        for (int h = 0; h < P; h++)
+            for (int ch = 0; ch < n_chunks; ch++) {
+                const int mc = min(TC_EPI_CHUNK, Mt - ch * TC_EPI_CHUNK);
+                drain(h, ch, out_s);
+                if (tid == 64 && ch == 0) TC_DBG(4, 63);
+                asm volatile("bar.sync 1, 512;" ::: "memory");
+                pdl_wait();
+                if (tid == 64 && ch == 0) TC_DBG(5, 63);
+                epilogue_rows(a.epi, out_s, 128, 128, (rt + h) * 128, a.d_real, mc, m0 + ch * TC_EPI_CHUNK, etid, eg, TC_GROUPS);
+                if (tid == 64 && ch == 0) TC_DBG(6, 63);
+                asm volatile("bar.sync 1, 512;" ::: "memory");
+                if (tid == 64 && ch == 0) TC_DBG(7, 63);
+            }
     }
     tc_fence_before();
     __syncthreads();
@@ -361,7 +384,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_q40_tc_kernel(const __grid
         tc_fence_after();
         tmem_dealloc(tmem_base, TC_TMEM_COLS);
     }
-    if (crank == 0) epilogue_complete(a.epi, tid, a.n_epi_ctas, sflag);
+    epilogue_complete(a.epi, tid, a.n_epi_ctas, sflag);
     if (threadIdx.x == 0) TC_DBG(3, 63);
     trace_end(a.tr);
 }
@@ -405,7 +428,7 @@ extern "C" int dl_gemm_q40_tc(const uint8_t* w_q40t, int d, int n, const uint8_t
     if (a.NSA < TC_GROUPS || a.NSA > 16) { dl_set_error("dl_gemm_q40_tc: bad NSA=%d", a.NSA); return -1; }
     // nacc must divide nstg: then successive phases of an A stage are consumed by the SAME issuing warp (and
     // written after a retire that is ordered behind the previous one), so a parity wait can never be lapped
-    a.nacc = (a.NT <= 128) ? 2 : 1;
+    a.nacc = (a.NT <= 128) ? 2 : 1;                        // (also the two row tiles of a pair)
     a.nstg = (a.NT <= 64) ? 6 : 4;
     if (a.nacc * a.NT + a.nstg * TC_A_STAGE_COLS > TC_TMEM_COLS || a.nstg < TC_GROUPS || a.nstg > 8 || a.nstg % a.nacc != 0 || (a.nacc != 1 && a.nacc != 2 && a.nacc != 4)) {
         dl_set_error("dl_gemm_q40_tc: bad TMEM plan nacc=%d nstg=%d NT=%d", a.nacc, a.nstg, a.NT);
@@ -414,7 +437,11 @@ extern "C" int dl_gemm_q40_tc(const uint8_t* w_q40t, int d, int n, const uint8_t
     a.nsb_log = (a.NSB == 8) ? 3 : (a.NSB == 4) ? 2 : 1;
     a.LA = (a.NSA % 4 == 0) ? 4 : (a.NSA % 3 == 0) ? 3 : (a.NSA % 2 == 0) ? 2 : 1;
     a.LB = (a.NSB % 4 == 0) ? 4 : (a.NSB % 3 == 0) ? 3 : (a.NSB % 2 == 0) ? 2 : 1;
-    a.n_epi_ctas = (a.d_pad / 128) * ((M + a.NT - 1) / a.NT);
+    // more row tiles than SMs and one activation tile: two row tiles per CTA share the activations (at 128 rows those are 32 KB per k-tile
+    // beside 9 KB of weights) and the second wave's start and end disappear
+    a.pair = M <= a.NT && a.NT <= 128 && a.S == 1 && row_tiles % 2 == 0 && row_tiles > n_sms;
+    const int cta_rows = row_tiles / (a.pair ? 2 : 1);
+    a.n_epi_ctas = cta_rows * a.S * ((M + a.NT - 1) / a.NT);
     a.epi = *epi;
     a.tr = dl_trace_next(TR_TC);
     a.dbg = g_tc_dbg;
@@ -428,7 +455,7 @@ extern "C" int dl_gemm_q40_tc(const uint8_t* w_q40t, int d, int n, const uint8_t
         max_set = smem;
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)((a.d_pad / 128) * a.S), (unsigned)((M + a.NT - 1) / a.NT));
+    cfg.gridDim = dim3((unsigned)(cta_rows * a.S), (unsigned)((M + a.NT - 1) / a.NT));
     cfg.blockDim = dim3(TC_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = (cudaStream_t)stream;

@@ -101,3 +101,30 @@ def test_gemv_extreme_nibbles(M):
     xd = x.double().sign() * 127 * float(torch.tensor(1 / 127).half())
     want = xd @ w.t()
     assert (y.cpu().double() - want).abs().max() <= 2.0 ** -21 * want.abs().max()
+
+
+@pytest.mark.parametrize("d,n,k_split,rows", [(19200, 256, 1, [4, 17, 33, 100, 128]), (19072, 384, 1, [5, 64]), (384, 1024, 2, [4, 33, 128]), (256, 1024, 4, [6, 100]),
+                                              (256, 1152, 8, [5, 16, 65])])
+def test_q40_tc_pairs_and_shares(d, n, k_split, rows):
+    """Row tiles side by side (more even row tiles than SMs; an odd number stays alone) and K shares whose ranks finish part of the rows
+    each (also ranks left without a row).  Bound: the operands are taken as the kernel rounds them, f32 accumulation of n <= 1152 terms: 1e-5."""
+    k = K()
+    g = torch.Generator(device="cuda").manual_seed(d + n)
+    nib = torch.randint(0, 16, (d, n // 32, 32), generator=g, device="cuda", dtype=torch.uint8)
+    scale = (0.01 + 0.01 * torch.rand(d, n // 32, 1, generator=g, device="cuda")).half()
+    raw = torch.cat([scale.view(torch.uint8), nib[:, :, :16] | (nib[:, :, 16:] << 4)], dim=2)
+    w = ((nib.half() - 8) * scale).double().reshape(d, n)
+    q40t = k.make_q40t(raw.reshape(-1), d, n)
+    for M in rows:
+        x = torch.randn(M, n, generator=g, device="cuda")
+        ncap = 16 if M <= 16 else 32 if M <= 32 else 64 if M <= 64 else 128
+        xh = k.alloc_xh(n, ncap, "cuda")
+        k.quant_q80(x, M, n, ncap, xh_out=xh)
+        blocks = x.view(M, n // 32, 32)
+        s = blocks.abs().amax(dim=2, keepdim=True) / 127
+        xq = ((blocks * (1 / s)).round() * s.half().float()).half().double().view(M, n)
+        y = torch.full((M + 1, d), 3.0, device="cuda")
+        k.gemm_q40_tc(q40t, d, n, xh, ncap, M, k.epi_store([y.data_ptr()], d), k_split)
+        want = xq @ w.t()
+        assert (y[:M].double() - want).norm() <= 1e-5 * want.norm()
+        assert (y[M] == 3).all()
