@@ -20,141 +20,189 @@
 #include "gated_common.cuh"
 
 #define GT_TB 8                   // tokens staged per barrier pair of the token-by-token kernel
-#define GT_COLS 32                // columns of S per CTA of the token-by-token kernel
+#define GT_GROUPS 32              // column groups of S per CTA of the token-by-token kernel (of 1 or 2 columns)
 
 // ------------------------------------------------------------------------------------------------
 // token by token: a CTA owns GT_COLS columns of one head's S; thread (column, dq) keeps the rows d with (d / 4) % 4 == dq of its
 // column (NR registers; rows in groups of four so that q, k and f leave shared memory as 16-byte words), the four threads
 // of a column are neighbouring lanes and sum their shares of y by two shuffles.  In the head form column `vdim` is n: its
-// value is 1 for every token and its output is den.  Ahead form: the bonus term is one number per token (bs).  Delta form:
-// the column's share of S^T k is summed over the four lanes before the update.
+// value is 1 for every token and its output is den.
+//
+// Decoding (a row per sequence) is bound by the state's bytes, read and written once: what counts is how many of them an SM has in
+// flight.  The addresses of a thread's rows were kept from load to store, two registers each, so three CTAs fitted an SM (28.8 us for 32
+// sequences x 16 heads of 128 x 128, 2.4 TB/s); formed again at the end, and with two columns per thread in 8-byte pieces, four CTAs
+// hold twice the bytes each: 18.6 us, 3.6 TB/s (one column and seven CTAs 20.0, four columns and two CTAs 20.6).
 // ------------------------------------------------------------------------------------------------
-template <int NR, int MODE>
-__global__ void __launch_bounds__(GT_COLS * 4, NR <= 32 ? 3 : 1) gated_scan_kernel(DlMambaBatch b, DlGatedArgs a) {
+template <int NR, int MODE, int CW>
+__global__ void __launch_bounds__(GT_GROUPS * 4, NR * CW <= 32 ? 6 : NR * CW <= 64 && NR <= 32 ? 4 : 1) gated_scan_kernel(DlMambaBatch b, DlGatedArgs a) {
     constexpr int DP = NR * 4;
     constexpr bool CH = MODE != GATED_HEAD;
     extern __shared__ __align__(16) float sm[];
-    const int n = blockIdx.x, h = blockIdx.y, dq = threadIdx.x & 3, c = blockIdx.z * GT_COLS + (threadIdx.x >> 2);
+    const int n = blockIdx.x, h = blockIdx.y, dq = threadIdx.x & 3, c = (blockIdx.z * GT_GROUPS + (threadIdx.x >> 2)) * CW;
     const int D = a.dim, V = a.vdim, H = a.n_heads, hk = gated_k_head(a, h);
     float* qs = sm;                             // [GT_TB][DP]
     float* ks = qs + GT_TB * DP;                // [GT_TB][DP]
     float* fs = ks + GT_TB * DP;                // per channel: [GT_TB][DP]; head form: [GT_TB] decays
-    float* bs = fs + GT_TB * DP;                // ahead form: [GT_TB] sums of q bonus k; delta form: [GT_TB] sigmoid(beta)
+    float* bs = fs + GT_TB * DP;                // ahead form: [GT_TB][DP / 32] sums of q bonus k; delta form: [GT_TB][..] sigmoid(beta)
     const size_t sh = (size_t)b.seq_slot[n] * H + h;
     const bool fresh = b.seq_pos0[n] == 0, is_n = !CH && c == V, live = c < V || is_n;
     float* Sg = is_n ? a.n_state + sh * D : a.state + sh * D * V + c;       // row d at Sg[d * step]
     const size_t step = is_n ? 1 : V;
-    float s[NR];
+    float s[CW][NR];
 #pragma unroll
     for (int i = 0; i < NR; ++i) {
         const int d = (i >> 2) * 16 + dq * 4 + (i & 3);
-        s[i] = (live && !fresh && d < D) ? Sg[d * step] : 0.f;
+        const bool have = live && !fresh && d < D;
+        if (CW == 2) {
+            const float2 v = have ? *reinterpret_cast<const float2*>(Sg + d * step) : make_float2(0.f, 0.f);
+            s[0][i] = v.x; s[CW - 1][i] = v.y;
+        } else {
+            s[0][i] = have ? Sg[d * step] : 0.f;
+        }
     }
     const int r0 = b.seq_start[n], r1 = b.seq_start[n + 1];
     for (int rb = r0; rb < r1; rb += GT_TB) {
         const int nt = min(GT_TB, r1 - rb);
         __syncthreads();
-        for (int t = threadIdx.x / 32; t < nt; t += GT_COLS * 4 / 32) {
+        // all threads stage, a warp 32 channels of one token (DP is a multiple of 32)
+#pragma unroll 1
+        for (int i = threadIdx.x; i < nt * DP; i += GT_GROUPS * 4) {
+            const int t = i / DP, d = i - t * DP;
             const size_t row = b.seq_rows[rb + t];
-            const float put = CH ? 0.f : a.put[row * H + h];
-            float bonus = 0.f;
-            for (int d = threadIdx.x & 31; d < DP; d += 32) {
-                float q = 0.f, k = 0.f, f = 0.f;
-                if (d < D) {
-                    q = gated_q(a, row, hk * D + d);
-                    if (CH) gated_fk(a, row, h, hk, d, f, k);
-                    else k = put * a.k[row * a.ldk + h * D + d];
-                    if (MODE == GATED_AHEAD) bonus = fmaf(q * a.bonus[h * D + d], k, bonus);
-                }
-                qs[t * DP + d] = q;
-                ks[t * DP + d] = k;
-                if (CH) fs[t * DP + d] = f;
+            float q = 0.f, k = 0.f, f = 0.f, bonus = 0.f;
+            if (d < D) {
+                q = gated_q(a, row, hk * D + d);
+                if (CH) gated_fk(a, row, h, hk, d, f, k);
+                else k = a.put[row * H + h] * a.k[row * a.ldk + h * D + d];
+                if (MODE == GATED_AHEAD) bonus = q * a.bonus[h * D + d] * k;
             }
-            if (MODE == GATED_AHEAD) bonus = warp_sum(bonus);
-            if ((threadIdx.x & 31) == 0) {
+            qs[i] = q;
+            ks[i] = k;
+            if (CH) fs[i] = f;
+            if (MODE == GATED_AHEAD) {
+                bonus = warp_sum(bonus);
+                if ((threadIdx.x & 31) == 0) bs[t * (DP / 32) + d / 32] = bonus;
+            }
+            if (d == 0) {
                 if (!CH) fs[t] = expf(a.log_keep[row * H + h]);
-                if (MODE == GATED_AHEAD) bs[t] = bonus;
-                if (MODE == GATED_DELTA) bs[t] = sigmoid_f(a.beta[row * a.ld_beta + h]);
+                if (MODE == GATED_DELTA) bs[t * (DP / 32)] = sigmoid_f(a.beta[row * a.ld_beta + h]);
             }
         }
         __syncthreads();
         for (int t = 0; t < nt; ++t) {
             const size_t row = b.seq_rows[rb + t];
-            float v = c < V ? a.v[row * a.ldv + h * V + c] : 1.f;
+            float v[CW];
+#pragma unroll
+            for (int w = 0; w < CW; ++w) v[w] = c < V ? a.v[row * a.ldv + h * V + c + w] : 1.f;
             const float keep = CH ? 0.f : fs[t];
-            float y0 = 0.f, y1 = 0.f;
             if (MODE == GATED_DELTA) {          // v becomes u, the state is decayed already
-                float d0 = 0.f, d1 = 0.f;
+                float d0[CW], d1[CW];
+#pragma unroll
+                for (int w = 0; w < CW; ++w) d0[w] = d1[w] = 0.f;
 #pragma unroll
                 for (int i = 0; i < NR; i += 4) {
                     const int at = t * DP + i * 4 + dq * 4;
                     const float4 k = *reinterpret_cast<const float4*>(ks + at), f = *reinterpret_cast<const float4*>(fs + at);
-                    s[i] *= f.x;         d0 = fmaf(s[i], k.x, d0);
-                    s[i + 1] *= f.y;     d1 = fmaf(s[i + 1], k.y, d1);
-                    s[i + 2] *= f.z;     d0 = fmaf(s[i + 2], k.z, d0);
-                    s[i + 3] *= f.w;     d1 = fmaf(s[i + 3], k.w, d1);
+#pragma unroll
+                    for (int w = 0; w < CW; ++w) {
+                        s[w][i] *= f.x;         d0[w] = fmaf(s[w][i], k.x, d0[w]);
+                        s[w][i + 1] *= f.y;     d1[w] = fmaf(s[w][i + 1], k.y, d1[w]);
+                        s[w][i + 2] *= f.z;     d0[w] = fmaf(s[w][i + 2], k.z, d0[w]);
+                        s[w][i + 3] *= f.w;     d1[w] = fmaf(s[w][i + 3], k.w, d1[w]);
+                    }
                 }
-                d0 += d1;
-                d0 += __shfl_xor_sync(0xffffffffu, d0, 1);
-                d0 += __shfl_xor_sync(0xffffffffu, d0, 2);
-                v = bs[t] * (v - d0);
+#pragma unroll
+                for (int w = 0; w < CW; ++w) {
+                    d0[w] += d1[w];
+                    d0[w] += __shfl_xor_sync(0xffffffffu, d0[w], 1);
+                    d0[w] += __shfl_xor_sync(0xffffffffu, d0[w], 2);
+                    v[w] = bs[t * (DP / 32)] * (v[w] - d0[w]);
+                }
             }
+            float bonus = 0.f;
+            if (MODE == GATED_AHEAD)
+                for (int u = 0; u < DP / 32; ++u) bonus += bs[t * (DP / 32) + u];
+            float y0[CW], y1[CW];
+#pragma unroll
+            for (int w = 0; w < CW; ++w) y0[w] = y1[w] = 0.f;
 #pragma unroll
             for (int i = 0; i < NR; i += 4) {
                 const int at = t * DP + i * 4 + dq * 4;
                 const float4 q = *reinterpret_cast<const float4*>(qs + at), k = *reinterpret_cast<const float4*>(ks + at);
                 float4 f = make_float4(keep, keep, keep, keep);
-                if (MODE == GATED_DELTA) {
-                    s[i] = fmaf(k.x, v, s[i]);               y0 = fmaf(s[i], q.x, y0);
-                    s[i + 1] = fmaf(k.y, v, s[i + 1]);       y1 = fmaf(s[i + 1], q.y, y1);
-                    s[i + 2] = fmaf(k.z, v, s[i + 2]);       y0 = fmaf(s[i + 2], q.z, y0);
-                    s[i + 3] = fmaf(k.w, v, s[i + 3]);       y1 = fmaf(s[i + 3], q.w, y1);
-                    continue;
+                if (CH && MODE != GATED_DELTA) f = *reinterpret_cast<const float4*>(fs + at);
+#pragma unroll
+                for (int w = 0; w < CW; ++w) {
+                    if (MODE == GATED_DELTA) {
+                        s[w][i] = fmaf(k.x, v[w], s[w][i]);               y0[w] = fmaf(s[w][i], q.x, y0[w]);
+                        s[w][i + 1] = fmaf(k.y, v[w], s[w][i + 1]);       y1[w] = fmaf(s[w][i + 1], q.y, y1[w]);
+                        s[w][i + 2] = fmaf(k.z, v[w], s[w][i + 2]);       y0[w] = fmaf(s[w][i + 2], q.z, y0[w]);
+                        s[w][i + 3] = fmaf(k.w, v[w], s[w][i + 3]);       y1[w] = fmaf(s[w][i + 3], q.w, y1[w]);
+                    } else if (MODE == GATED_AHEAD) {
+                        y0[w] = fmaf(s[w][i], q.x, y0[w]);                s[w][i] = fmaf(f.x, s[w][i], k.x * v[w]);
+                        y1[w] = fmaf(s[w][i + 1], q.y, y1[w]);            s[w][i + 1] = fmaf(f.y, s[w][i + 1], k.y * v[w]);
+                        y0[w] = fmaf(s[w][i + 2], q.z, y0[w]);            s[w][i + 2] = fmaf(f.z, s[w][i + 2], k.z * v[w]);
+                        y1[w] = fmaf(s[w][i + 3], q.w, y1[w]);            s[w][i + 3] = fmaf(f.w, s[w][i + 3], k.w * v[w]);
+                    } else {
+                        s[w][i] = fmaf(f.x, s[w][i], k.x * v[w]);             y0[w] = fmaf(s[w][i], q.x, y0[w]);
+                        s[w][i + 1] = fmaf(f.y, s[w][i + 1], k.y * v[w]);     y1[w] = fmaf(s[w][i + 1], q.y, y1[w]);
+                        s[w][i + 2] = fmaf(f.z, s[w][i + 2], k.z * v[w]);     y0[w] = fmaf(s[w][i + 2], q.z, y0[w]);
+                        s[w][i + 3] = fmaf(f.w, s[w][i + 3], k.w * v[w]);     y1[w] = fmaf(s[w][i + 3], q.w, y1[w]);
+                    }
                 }
-                if (CH) f = *reinterpret_cast<const float4*>(fs + at);
-                if (MODE == GATED_AHEAD) {
-                    y0 = fmaf(s[i], q.x, y0);                s[i] = fmaf(f.x, s[i], k.x * v);
-                    y1 = fmaf(s[i + 1], q.y, y1);            s[i + 1] = fmaf(f.y, s[i + 1], k.y * v);
-                    y0 = fmaf(s[i + 2], q.z, y0);            s[i + 2] = fmaf(f.z, s[i + 2], k.z * v);
-                    y1 = fmaf(s[i + 3], q.w, y1);            s[i + 3] = fmaf(f.w, s[i + 3], k.w * v);
-                    continue;
-                }
-                s[i] = fmaf(f.x, s[i], k.x * v);             y0 = fmaf(s[i], q.x, y0);
-                s[i + 1] = fmaf(f.y, s[i + 1], k.y * v);     y1 = fmaf(s[i + 1], q.y, y1);
-                s[i + 2] = fmaf(f.z, s[i + 2], k.z * v);     y0 = fmaf(s[i + 2], q.z, y0);
-                s[i + 3] = fmaf(f.w, s[i + 3], k.w * v);     y1 = fmaf(s[i + 3], q.w, y1);
             }
-            float y = y0 + y1;
-            y += __shfl_xor_sync(0xffffffffu, y, 1);
-            y += __shfl_xor_sync(0xffffffffu, y, 2);
-            if (MODE == GATED_AHEAD) y = fmaf(bs[t], v, y);
-            if (live && dq == 0) {
-                if (is_n) a.den[row * H + h] = y;
-                else a.y[row * a.ld_y + h * V + c] = y;
+#pragma unroll
+            for (int w = 0; w < CW; ++w) {
+                float y = y0[w] + y1[w];
+                y += __shfl_xor_sync(0xffffffffu, y, 1);
+                y += __shfl_xor_sync(0xffffffffu, y, 2);
+                if (MODE == GATED_AHEAD) y = fmaf(bonus, v[w], y);
+                if (live && dq == w % 4) {
+                    if (is_n) a.den[row * H + h] = y;
+                    else a.y[row * a.ld_y + h * V + c + w] = y;
+                }
             }
         }
     }
     if (live) {
+        asm volatile("" : "+l"(Sg));            // the rows' addresses are formed again: kept, they would take two registers each
 #pragma unroll
         for (int i = 0; i < NR; ++i) {
             const int d = (i >> 2) * 16 + dq * 4 + (i & 3);
-            if (d < D) Sg[d * step] = s[i];
+            if (d >= D) continue;
+            if (CW == 2) *reinterpret_cast<float2*>(Sg + d * step) = make_float2(s[0][i], s[CW - 1][i]);
+            else Sg[d * step] = s[0][i];
         }
     }
 }
 
 extern "C" int dl_gated_scan_supported(int dim, int vdim) { return dim >= 1 && dim <= 512 && vdim >= 1 ? 0 : -1; }
 
-template <int NR, int MODE>
-static int launch_gated_mode(const DlMambaBatch& b, int n_seq, const DlGatedArgs& a, cudaStream_t st) {
+template <int NR, int MODE, int CW>
+static int launch_gated_cols(const DlMambaBatch& b, int n_seq, const DlGatedArgs& a, cudaStream_t st) {
     constexpr bool CH = MODE != GATED_HEAD;
-    const size_t smem = ((size_t)(CH ? 3 : 2) * GT_TB * NR * 4 + GT_TB) * sizeof(float);
+    const size_t smem = ((size_t)(CH ? 3 : 2) * GT_TB * NR * 4 + GT_TB * (NR * 4 / 32)) * sizeof(float);
     if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(gated_scan_kernel<NR, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = cudaFuncSetAttribute(gated_scan_kernel<NR, MODE, CW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) { dl_set_error("dl_gated_scan: shared memory attribute: %s", cudaGetErrorString(e)); return -(int)e; }
     }
-    gated_scan_kernel<NR, MODE><<<dim3(n_seq, a.n_heads, (a.vdim + (CH ? 0 : 1) + GT_COLS - 1) / GT_COLS), GT_COLS * 4, smem, st>>>(b, a);
+    constexpr int cols = GT_GROUPS * CW;
+    gated_scan_kernel<NR, MODE, CW><<<dim3(n_seq, a.n_heads, (a.vdim + (CH ? 0 : 1) + cols - 1) / cols), GT_GROUPS * 4, smem, st>>>(b, a);
     return 0;
+}
+// Two columns per thread while the CTAs still fill the chip.  (A head's n is a column of its own, and more than 32 rows per thread leave
+// no registers for a second column.)
+static bool gated_two_columns(int n_seq, const DlGatedArgs& a, int n_sms) {
+    constexpr int cols = GT_GROUPS * 2;
+    return a.dim <= 128 && a.vdim % 2 == 0 && a.vdim >= cols && ((uintptr_t)a.state & 7) == 0 &&
+           (long long)n_seq * a.n_heads * ((a.vdim + cols - 1) / cols) >= n_sms;
+}
+template <int NR, int MODE>
+static int launch_gated_mode(const DlMambaBatch& b, int n_seq, const DlGatedArgs& a, cudaStream_t st) {
+    if constexpr (NR <= 32 && MODE != GATED_HEAD) {
+        if (gated_two_columns(n_seq, a, dl_device_sm_count())) return launch_gated_cols<NR, MODE, 2>(b, n_seq, a, st);
+    }
+    return launch_gated_cols<NR, MODE, 1>(b, n_seq, a, st);
 }
 template <int NR>
 static int launch_gated(const DlMambaBatch& b, int n_seq, const DlGatedArgs& a, cudaStream_t st) {

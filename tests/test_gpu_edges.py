@@ -128,3 +128,47 @@ def test_q40_tc_pairs_and_shares(d, n, k_split, rows):
         want = xq @ w.t()
         assert (y[:M].double() - want).norm() <= 1e-5 * want.norm()
         assert (y[M] == 3).all()
+
+
+@pytest.mark.parametrize("dim,vdim,form", [(48, 66, "lower"), (128, 128, "keys"), (64, 64, "ahead"), (20, 130, "delta"), (128, 64, "delta")])
+def test_gated_scan_two_columns(dim, vdim, form):
+    """Token by token with two columns per thread (160 CTAs and more): widths that end inside a CTA's 64 columns, head sizes that end inside
+    a group of 16 rows, several rows per sequence, fresh and continued sequences.  f32 chains of at most 128 terms: 1e-5."""
+    lib, H, S, per = L(), 4, 40, 3
+    g = torch.Generator(device="cuda").manual_seed(dim * 1000 + vdim)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    M = S * per
+    q, v, f, fb = rnd(M, H * dim), rnd(M, H * vdim), rnd(M, H * dim), rnd(H * dim)
+    key, state = rnd(M, H * dim) * dim ** -0.5, rnd(S, H, dim, vdim)
+    i32 = lambda t: torch.tensor(t, dtype=torch.int32, device="cuda")
+    start = [0 if s % 3 == 0 else 7 for s in range(S)]
+    slots = list(range(S))[::-1]
+    keep = dict(pos=i32([start[m // per] + m % per for m in range(M)]), row_seq=i32([m // per for m in range(M)]), seq_start=i32([s * per for s in range(S + 1)]),
+                seq_rows=i32(list(range(M))), seq_slot=i32(slots), seq_pos0=i32(start))
+    lower, beta, bonus = torch.rand(H * dim, generator=g, device="cuda"), rnd(M, H), rnd(H * dim)
+    kw = dict(f=f, f_bias=fb)
+    if form == "lower":
+        kw.update(lower=lower, gate=lib.GATE_LOWER)
+    else:
+        kw.update(k=key, gate=lib.GATE_ROOT_SIGMOID, tau=4.0)
+        kw.update({"ahead": dict(bonus=bonus), "delta": dict(beta=beta)}.get(form, {}))
+    y, st = torch.zeros(M, H * vdim, device="cuda"), state.clone()
+    lib.gated_scan(lib.mamba_batch(**keep), S, q, v, y, st, H, dim, vdim, **kw)
+    z = (f + fb).double().view(S, per, H, dim)
+    gate = lower.double().view(H, dim) + (1 - lower.double().view(H, dim)) * z.sigmoid() if form == "lower" else z.sigmoid() ** 0.25
+    kk = (1 - gate) if form == "lower" else key.double().view(S, per, H, dim)
+    qq, vv = q.double().view(S, per, H, dim), v.double().view(S, per, H, vdim)
+    cur = state.double()[slots] * torch.tensor([p != 0 for p in start], device="cuda").view(S, 1, 1, 1)
+    for t in range(per):
+        if form == "ahead":
+            out = torch.einsum("shd,shdv->shv", qq[:, t], cur) + (qq[:, t] * bonus.double().view(H, dim) * kk[:, t]).sum(-1, keepdim=True) * vv[:, t]
+        cur = gate[:, t, :, :, None] * cur
+        u = vv[:, t]
+        if form == "delta":
+            u = beta.double().view(S, per, H, 1)[:, t].sigmoid() * (u - torch.einsum("shd,shdv->shv", kk[:, t], cur))
+        cur = cur + kk[:, t, :, :, None] * u[:, :, None, :]
+        if form != "ahead":
+            out = torch.einsum("shd,shdv->shv", qq[:, t], cur)
+        got = y.view(S, per, H, vdim)[:, t].double()
+        assert (got - out).norm() <= 1e-5 * out.norm()
+    assert (st.double()[slots] - cur).norm() <= 1e-5 * cur.norm()
