@@ -136,10 +136,11 @@ extern "C" int dl_embedding(const float* table, const int* tokens, float* x, int
 
 // ------------------------------------------------------------------------------------------------
 // reduce (merge-add of the peers' partial sums) + residual + RMSNorm + Q80 cast
-// one CTA per activation row; dim <= 16384
+// one CTA per activation row, or per 8 of them; dim <= 16384
 // ------------------------------------------------------------------------------------------------
 #define RNQ_THREADS 512
 #define RNQ_MAX_PER_THREAD 32     // dim <= 512*32 = 16384
+#define RNQ_WIDE_ROWS 512         // from here on 8 rows per CTA
 
 struct RnqArgs {
     const float* x_in;
@@ -160,13 +161,23 @@ struct RnqArgs {
     unsigned long long* tr;
 };
 
+// Four lanes hold a 32-block: lane c its elements 4c .. 4c + 3 and 16 + 4c .. 16 + 4c + 3, which are one 16-byte chunk of the XH image.  A
+// warp is 8 such blocks: of 8 rows side by side (ROWS = 8, many rows: a chunk of the 8 rows is one whole 128-byte line of the image), or
+// 8 neighbouring blocks of one row (ROWS = 1: a CTA per row).  The merged row stays in registers between the two passes.
+// What bounds it: bytes (x, partial sums, image) for many rows, latency for few.  One thread per block, 128 bytes apart, as it was:
+// a feed-forward block of 2048 rows of 4096 took 846 us with it and 832 with this; 32 rows are as fast either way.
+template <int ROWS>
 __global__ void __launch_bounds__(RNQ_THREADS) reduce_norm_quant_kernel(const __grid_constant__ RnqArgs a) {
     trace_begin(a.tr);
-    __shared__ float s_part[RNQ_THREADS / 32];
-    __shared__ float s_inv;
+    constexpr int NW = RNQ_THREADS / 32, KEEP = ROWS == 8 ? 8 : 4;
+    __shared__ float s_part[NW][8];
     pdl_launch_dependents();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, c = lane & 3;
+    const int r = ROWS == 8 ? lane >> 2 : 0, m = blockIdx.x * ROWS + r;
+    const int nb = a.dim >> 5;
+    const bool live = m < a.M;
+    auto block_of = [&](int u) { return ROWS == 8 ? warp + u * NW : (warp + u * NW) * 8 + (lane >> 2); };
     pdl_wait();
-    const int m = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (a.flags != nullptr && a.n_src > 0) {
         if (tid < a.n_src) {
             const uint32_t epoch = ld_volatile_u32(a.step_counter) * a.flag_mul + a.flag_add;
@@ -179,123 +190,131 @@ __global__ void __launch_bounds__(RNQ_THREADS) reduce_norm_quant_kernel(const __
     const size_t rowb = (size_t)a.dim + (a.dim >> 4);
     const size_t src_rows = (size_t)a.src_stride / a.dim;
     const uint32_t ll_epoch = ll ? ld_volatile_u32(a.step_counter) * a.flag_mul + a.flag_add : 0u;
-    // pass 1: merged residual (float4, coalesced) -> x_out, sum of squares
-    constexpr int nwarps = RNQ_THREADS / 32;
     const size_t row = (size_t)m * a.dim;
-    float ss = 0.0f;
-    for (int i4 = tid; i4 < a.dim / 4; i4 += RNQ_THREADS) {
-        float4 v = reinterpret_cast<const float4*>(a.x_in + row)[i4];
-        for (int s = 0; s < a.n_src; s++) {
-            float4 p;
-            if (wire) {
-                const uint8_t* wr = reinterpret_cast<const uint8_t*>(a.partials) + ((size_t)s * src_rows + m) * rowb;
-                const int q4 = *reinterpret_cast<const int*>(wr + 4 * i4);
-                const float d = __half2float(*reinterpret_cast<const __half*>(wr + a.dim + ((i4 >> 3) << 1)));
-                p = make_float4((float)(int8_t)(q4 & 0xff) * d, (float)(int8_t)((q4 >> 8) & 0xff) * d,
-                                (float)(int8_t)((q4 >> 16) & 0xff) * d, (float)(q4 >> 24) * d);
-            } else {
-                p = part_load4(a.partials, (size_t)s * a.src_stride + row + 4 * (size_t)i4, ll, ll_epoch);
-            }
-            v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w;
-        }
-        if (a.x_out != nullptr) reinterpret_cast<float4*>(a.x_out + row)[i4] = v;
-        ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
-    }
-    ss = warp_sum(ss);
-    if (lane == 0) s_part[warp] = ss;
-    __syncthreads();
-    if (warp == 0) {
-        float t = (lane < nwarps) ? s_part[lane] : 0.0f;
-        t = warp_sum(t);
-        if (lane == 0) s_inv = 1.0f / sqrtf(t / (float)a.dim + a.eps);
-    }
-    __syncthreads();
-    const float inv = (a.norm_w != nullptr) ? s_inv : 1.0f;
-    // pass 2: one thread per 32-block (independent 16-byte loads, no shuffles)
-    for (int b = tid; b < a.dim / 32; b += RNQ_THREADS) {
-        const size_t e = row + (size_t)b * 32;
-        float4 v[8];
+    auto merged = [&](int b, float4 (&v)[2]) {
 #pragma unroll
-        for (int j = 0; j < 8; j++) v[j] = reinterpret_cast<const float4*>(a.x_in + e)[j];
-        for (int s = 0; s < a.n_src; s++) {
-            if (wire) {
-                const uint8_t* wr = reinterpret_cast<const uint8_t*>(a.partials) + ((size_t)s * src_rows + m) * rowb;
-                const uint4 qa = *reinterpret_cast<const uint4*>(wr + b * 32), qb = *reinterpret_cast<const uint4*>(wr + b * 32 + 16);
-                const float d = __half2float(*reinterpret_cast<const __half*>(wr + a.dim + (b << 1)));
-                const uint32_t w8[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
-#pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    const int q4 = (int)w8[j];
-                    v[j].x += (float)(int8_t)(q4 & 0xff) * d; v[j].y += (float)(int8_t)((q4 >> 8) & 0xff) * d;
-                    v[j].z += (float)(int8_t)((q4 >> 16) & 0xff) * d; v[j].w += (float)(q4 >> 24) * d;
+        for (int h = 0; h < 2; h++) {
+            const int e = b * 32 + h * 16 + c * 4;
+            v[h] = *reinterpret_cast<const float4*>(a.x_in + row + e);
+            for (int s = 0; s < a.n_src; s++) {
+                float4 p;
+                if (wire) {
+                    const uint8_t* wr = reinterpret_cast<const uint8_t*>(a.partials) + ((size_t)s * src_rows + m) * rowb;
+                    const int q4 = *reinterpret_cast<const int*>(wr + e);
+                    const float d = __half2float(*reinterpret_cast<const __half*>(wr + a.dim + (b << 1)));
+                    p = make_float4((float)(int8_t)(q4 & 0xff) * d, (float)(int8_t)((q4 >> 8) & 0xff) * d,
+                                    (float)(int8_t)((q4 >> 16) & 0xff) * d, (float)(q4 >> 24) * d);
+                } else {
+                    p = part_load4(a.partials, (size_t)s * a.src_stride + row + e, ll, ll_epoch);
                 }
-                continue;
-            }
-            const size_t pe = (size_t)s * a.src_stride + e;
-#pragma unroll
-            for (int j = 0; j < 8; j++) {
-                const float4 t = part_load4(a.partials, pe + 4 * j, ll, ll_epoch);
-                v[j].x += t.x; v[j].y += t.y; v[j].z += t.z; v[j].w += t.w;
+                v[h].x += p.x; v[h].y += p.y; v[h].z += p.z; v[h].w += p.w;
             }
         }
+    };
+    // pass 1: merged residual -> x_out, sum of squares
+    float4 keep[KEEP][2];
+    float ss = 0.0f;
+    auto first = [&](int b, float4 (&v)[2]) {
+        merged(b, v);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            if (a.x_out != nullptr) *reinterpret_cast<float4*>(a.x_out + row + b * 32 + h * 16 + c * 4) = v[h];
+            ss += v[h].x * v[h].x + v[h].y * v[h].y + v[h].z * v[h].z + v[h].w * v[h].w;
+        }
+    };
+#pragma unroll
+    for (int u = 0; u < KEEP; u++)
+        if (live && block_of(u) < nb) first(block_of(u), keep[u]);
+    for (int u = KEEP; live && block_of(u) < nb; u++) {
+        float4 v[2];
+        first(block_of(u), v);
+    }
+    float inv = 1.0f;
+    if (a.norm_w != nullptr) {
+        ss += __shfl_xor_sync(0xffffffffu, ss, 1);
+        ss += __shfl_xor_sync(0xffffffffu, ss, 2);
+        if (c == 0) s_part[warp][lane >> 2] = ss;
+        __syncthreads();
+        float t = 0.0f;
+        if (ROWS == 8) {              // lane (r, c) sums the warps c, c + 4, ... of row r
+#pragma unroll
+            for (int w = 0; w < NW; w += 4) t += s_part[w + c][r];
+            t += __shfl_xor_sync(0xffffffffu, t, 1);
+            t += __shfl_xor_sync(0xffffffffu, t, 2);
+        } else {
+#pragma unroll
+            for (int w = 0; w < NW * 8; w += 32) t += (&s_part[0][0])[w + lane];
+            t = warp_sum(t);
+        }
+        inv = 1.0f / sqrtf(t / (float)a.dim + a.eps);
+    }
+    // pass 2: norm, Q80
+    auto second = [&](int b, bool on, float4 (&v)[2]) {
         float amax = 0.0f;
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-            if (a.norm_w != nullptr) {
-                const float4 w4 = reinterpret_cast<const float4*>(a.norm_w + (size_t)b * 32)[j];
-                v[j].x = w4.x * (inv * v[j].x); v[j].y = w4.y * (inv * v[j].y);
-                v[j].z = w4.z * (inv * v[j].z); v[j].w = w4.w * (inv * v[j].w);
+        for (int h = 0; h < 2; h++) {
+            if (a.norm_w != nullptr && on) {
+                const float4 w4 = *reinterpret_cast<const float4*>(a.norm_w + b * 32 + h * 16 + c * 4);
+                v[h].x = w4.x * (inv * v[h].x); v[h].y = w4.y * (inv * v[h].y);
+                v[h].z = w4.z * (inv * v[h].z); v[h].w = w4.w * (inv * v[h].w);
             }
-            amax = fmaxf(amax, fmaxf(fmaxf(fabsf(v[j].x), fabsf(v[j].y)), fmaxf(fabsf(v[j].z), fabsf(v[j].w))));
+            amax = fmaxf(amax, fmaxf(fmaxf(fabsf(v[h].x), fabsf(v[h].y)), fmaxf(fabsf(v[h].z), fabsf(v[h].w))));
+            if (a.y_out != nullptr && on) *reinterpret_cast<float4*>(a.y_out + row + b * 32 + h * 16 + c * 4) = v[h];
         }
-        if (a.y_out != nullptr) {
-#pragma unroll
-            for (int j = 0; j < 8; j++) reinterpret_cast<float4*>(a.y_out + e)[j] = v[j];
-        }
-        if (a.xq_out == nullptr && a.xh_out == nullptr) continue;
+        if (a.xq_out == nullptr && a.xh_out == nullptr) return;
+        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
         const float d = amax / 127.0f;
         const float id = (d != 0.0f) ? (1.0f / d) : 0.0f;
         const float df = __half2float(__float2half_rn(d));
-        int q[32];
-        int sumq = 0;
+        int q[2][4];
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-            q[4 * j + 0] = __float2int_rn(v[j].x * id); q[4 * j + 1] = __float2int_rn(v[j].y * id);
-            q[4 * j + 2] = __float2int_rn(v[j].z * id); q[4 * j + 3] = __float2int_rn(v[j].w * id);
-            sumq += q[4 * j] + q[4 * j + 1] + q[4 * j + 2] + q[4 * j + 3];
+        for (int h = 0; h < 2; h++) {
+            q[h][0] = __float2int_rn(v[h].x * id); q[h][1] = __float2int_rn(v[h].y * id);
+            q[h][2] = __float2int_rn(v[h].z * id); q[h][3] = __float2int_rn(v[h].w * id);
         }
         const int kt = b >> 2, kb = b & 3;
         if (a.xq_out != nullptr) {
-            uint8_t* rowp = a.xq_out + ((size_t)kt * a.mcap + m) * XQ_ROW_BYTES;
-            uint32_t pk[8];
+            int sumq = q[0][0] + q[0][1] + q[0][2] + q[0][3] + q[1][0] + q[1][1] + q[1][2] + q[1][3];
+            sumq += __shfl_xor_sync(0xffffffffu, sumq, 1);
+            sumq += __shfl_xor_sync(0xffffffffu, sumq, 2);
+            if (on) {
+                uint8_t* rowp = a.xq_out + ((size_t)kt * a.mcap + m) * XQ_ROW_BYTES;
 #pragma unroll
-            for (int j = 0; j < 8; j++)
-                pk[j] = (uint32_t)(q[4 * j] & 0xff) | ((uint32_t)(q[4 * j + 1] & 0xff) << 8) |
-                        ((uint32_t)(q[4 * j + 2] & 0xff) << 16) | ((uint32_t)(q[4 * j + 3] & 0xff) << 24);
-            uint4* qd = reinterpret_cast<uint4*>(rowp + kb * 32);
-            qd[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-            qd[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
-            reinterpret_cast<float*>(rowp + 128)[kb] = df;
-            reinterpret_cast<int*>(rowp + 144)[kb] = 8 * sumq;
-        }
-        if (a.xh_out != nullptr) {
-            // chunk w holds elements [4w, 4w+2, 4w+1, 4w+3, 4w+16, 4w+18, 4w+17, 4w+19] (see xh_slot)
-            uint8_t* base = a.xh_out + (size_t)kt * (size_t)(a.mcap >> 3) * XH_ROWGROUP_BYTES +
-                            (size_t)(m >> 3) * XH_ROWGROUP_BYTES + (size_t)(kb * 4) * 128 + (size_t)(m & 7) * 16;
-            const float dfh = fminf(df, 515.0f);       // fp16 operand: saturate (|x| > 65405) instead of producing inf
-#pragma unroll
-            for (int w = 0; w < 4; w++) {
-                const int o = 4 * w;
-                __half2 h0 = __floats2half2_rn((float)q[o] * dfh, (float)q[o + 2] * dfh);
-                __half2 h1 = __floats2half2_rn((float)q[o + 1] * dfh, (float)q[o + 3] * dfh);
-                __half2 h2 = __floats2half2_rn((float)q[o + 16] * dfh, (float)q[o + 18] * dfh);
-                __half2 h3 = __floats2half2_rn((float)q[o + 17] * dfh, (float)q[o + 19] * dfh);
-                uint4 u;
-                u.x = *reinterpret_cast<uint32_t*>(&h0); u.y = *reinterpret_cast<uint32_t*>(&h1);
-                u.z = *reinterpret_cast<uint32_t*>(&h2); u.w = *reinterpret_cast<uint32_t*>(&h3);
-                *reinterpret_cast<uint4*>(base + w * 128) = u;
+                for (int h = 0; h < 2; h++)
+                    *reinterpret_cast<uint32_t*>(rowp + kb * 32 + h * 16 + c * 4) = (uint32_t)(q[h][0] & 0xff) | ((uint32_t)(q[h][1] & 0xff) << 8) |
+                                                                                    ((uint32_t)(q[h][2] & 0xff) << 16) | ((uint32_t)(q[h][3] & 0xff) << 24);
+                if (c == 0) {
+                    reinterpret_cast<float*>(rowp + 128)[kb] = df;
+                    reinterpret_cast<int*>(rowp + 144)[kb] = 8 * sumq;
+                }
             }
         }
+        if (a.xh_out != nullptr && on) {
+            // chunk c holds elements [4c, 4c+2, 4c+1, 4c+3, 4c+16, 4c+18, 4c+17, 4c+19] (see xh_slot)
+            const float dfh = fminf(df, 515.0f);       // fp16 operand: saturate (|x| > 65405) instead of producing inf
+            uint32_t w[4];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                __half2 h0 = __floats2half2_rn((float)q[h][0] * dfh, (float)q[h][2] * dfh), h1 = __floats2half2_rn((float)q[h][1] * dfh, (float)q[h][3] * dfh);
+                w[2 * h] = *reinterpret_cast<uint32_t*>(&h0);
+                w[2 * h + 1] = *reinterpret_cast<uint32_t*>(&h1);
+            }
+            *reinterpret_cast<uint4*>(a.xh_out + ((size_t)kt * (size_t)(a.mcap >> 3) + (size_t)(m >> 3)) * XH_ROWGROUP_BYTES + (size_t)(kb * 4 + c) * 128 +
+                                      (size_t)(m & 7) * 16) = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+    };
+#pragma unroll
+    for (int u = 0; u < KEEP; u++) {
+        const bool on = live && block_of(u) < nb;
+        if (!on) keep[u][0] = keep[u][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (__any_sync(0xffffffffu, on)) second(block_of(u), on, keep[u]);
+    }
+    for (int u = KEEP; ROWS == 8 ? block_of(u) < nb : (warp + u * NW) * 8 < nb; u++) {
+        const bool on = live && block_of(u) < nb;
+        float4 v[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
+        if (on) merged(block_of(u), v);
+        second(block_of(u), on, v);
     }
     trace_end(a.tr);
 }
@@ -313,7 +332,8 @@ extern "C" int dl_reduce_norm_quant(const float* x_in, float* x_out, const float
     a.xq_out = xq_out; a.xh_out = xh_out; a.y_out = y_out;
     a.tr = dl_trace_next(TR_RNQ);
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(M);
+    const bool wide = M >= RNQ_WIDE_ROWS;
+    cfg.gridDim = dim3(wide ? (M + 7) / 8 : M);
     cfg.blockDim = dim3(RNQ_THREADS);
     cfg.stream = (cudaStream_t)stream;
     cudaLaunchAttribute attr[1];
@@ -323,7 +343,7 @@ extern "C" int dl_reduce_norm_quant(const float* x_in, float* x_out, const float
         cfg.attrs = attr;
         cfg.numAttrs = 1;
     }
-    cudaError_t e = cudaLaunchKernelEx(&cfg, reduce_norm_quant_kernel, a);
+    cudaError_t e = wide ? cudaLaunchKernelEx(&cfg, reduce_norm_quant_kernel<8>, a) : cudaLaunchKernelEx(&cfg, reduce_norm_quant_kernel<1>, a);
     if (e != cudaSuccess) { dl_set_error("dl_reduce_norm_quant: %s", cudaGetErrorString(e)); return -(int)e; }
     return 0;
 }

@@ -172,3 +172,30 @@ def test_gated_scan_two_columns(dim, vdim, form):
         got = y.view(S, per, H, vdim)[:, t].double()
         assert (got - out).norm() <= 1e-5 * out.norm()
     assert (st.double()[slots] - cur).norm() <= 1e-5 * cur.norm()
+
+
+@pytest.mark.parametrize("M,dim", [(1, 32), (3, 2080), (511, 256), (513, 4096), (600, 4128), (515, 96)])
+def test_norm_q80_rows_per_cta(M, dim):
+    """Norm and Q80 cast with a CTA per row and per 8 rows: rows and blocks that leave lanes without work, rows longer than the registers
+    hold.  The cast agrees with the norm's own output to one step of the block (a sum in another order may move a value across a half)."""
+    from test_gpu_kernels import _decode_xh
+    k = K()
+    g = torch.Generator(device="cuda").manual_seed(M + dim)
+    x, part, w = (torch.randn(*s, generator=g, device="cuda") for s in ((M, dim), (M, dim), (dim,)))
+    ncap, kp = (M + 7) // 8 * 8, (dim + 127) // 128 * 128
+    xq, xh = k.alloc_xq(kp, ncap, "cuda"), k.alloc_xh(kp, ncap, "cuda")
+    x_out, y = torch.zeros(M, dim, device="cuda"), torch.zeros(M, dim, device="cuda")
+    k.reduce_norm_quant(x, x_out, part.data_ptr(), 1, M * dim, None, None, 0, 0, w, 1e-5, dim, M, ncap, xq, xh, y_out=y)
+    s = x.double() + part.double()
+    want = w.double() * s / (s.square().mean(dim=1, keepdim=True) + 1e-5).sqrt()
+    assert (x_out.double() - s).abs().max() <= 1e-6 * s.abs().max()
+    assert (y.double() - want).norm() <= 1e-6 * want.norm()
+    step = want.view(M, dim // 32, 32).abs().amax(dim=2, keepdim=True) / 127
+    raw = xq.view(kp // 128, ncap, 160)[:, :M]
+    q = raw[:, :, :128].view(torch.int8).double().view(kp // 128, M, 4, 32)
+    d = raw[:, :, 128:144].contiguous().view(torch.float32).double().view(kp // 128, M, 4, 1)
+    for got in ((q * d).permute(1, 0, 2, 3).reshape(M, kp // 32, 32)[:, :dim // 32], torch.from_numpy(_decode_xh(xh, kp, ncap, M)).cuda().double().view(M, kp // 32, 32)[:, :dim // 32]):
+        assert ((got - want.view(M, dim // 32, 32)).abs() <= 1.01 * step + 1e-9).all()
+    sums = raw[:, :, 144:160].contiguous().view(torch.int32).view(kp // 128, M, 4)
+    live = sums.permute(1, 0, 2).reshape(M, kp // 32)[:, :dim // 32]
+    assert (live == 8 * q.sum(dim=3).long().permute(1, 0, 2).reshape(M, kp // 32)[:, :dim // 32]).all()
