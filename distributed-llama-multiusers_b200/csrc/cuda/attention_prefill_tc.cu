@@ -24,6 +24,13 @@
 // (The first version copied K/V with cp.async in 16-byte pieces into un-swizzled core matrices: 4096 LDGSTS per step
 // cost 3500 clk of issue time, three times the MMAs -- scripts/trace_attention_tc.py.)
 // TMEM columns: S0 [0,128) S1 [128,256) P0 [256,320) P1 [320,384) O [384,512).
+//
+// The second instance (LINES) serves layer-list models: bf16 cache lines [key 128 | value 128], tiles of up to rq consecutive positions
+// of one sequence whose query heads of one key/value head stack on the MMA's rows (row = position * rep + head), so two neighbouring
+// tiles of 64 stacked rows fill the 128 lanes; window or chunk masks (only the steps that a tile sees are walked), soft cap, distance
+// bias, sink, gate; f32 output.  mma.sync with its 64-row tiles took 142 us for 2000 rows of 16 heads on 4 under a window of 1024
+// (88 TFLOP/s); 52 us here.
+//
 // Reference semantics: multiheadAtt_F32 (src/nn/nn-cpu-ops.cpp:749-784), softmax in f32, output cast as OP_CAST
 // (src/llm.cpp:296-301).  KV cache: fp16 pages [page][kv_head][32][128].
 #include <cuda.h>
@@ -57,14 +64,19 @@ struct PtArgs {
     unsigned long long* tr;
 };
 
+struct PtLineArgs {
+    DlWindowAttnArgs w;
+    const int* tile_rows;      // [n_tiles][rq], -1 where a tile has fewer rows
+    int n_tiles, rq, rep;
+};
+template <bool LINES> struct PtKernelArgs { typedef PtArgs T; };
+template <> struct PtKernelArgs<true> { typedef PtLineArgs T; };
+
 DL_DEVINL void pt_wait(uint64_t* bar, uint32_t parity, unsigned long long t0) {
     unsigned n = 0;
     while (!mbar_try_wait(bar, parity)) {
         if ((++n & 0x3FFu) == 0 && globaltimer_ns() - t0 > PT_DEADLINE_NS) __trap();
     }
-}
-DL_DEVINL void pt_cp_async16(uint32_t smem_dst, const void* gsrc) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_dst), "l"(gsrc) : "memory");
 }
 DL_DEVINL void tmem_ld_32x32b_x32(uint32_t taddr, uint32_t (&v)[32]) {
     asm volatile(
@@ -87,23 +99,31 @@ DL_DEVINL void tmem_st_32x32b_x32(uint32_t taddr, const uint32_t (&v)[32]) {
         "r"(v[31])
         : "memory");
 }
-// instruction descriptor, kind::f16: A fp16 K-major (or TMEM), B fp16 with selectable major-ness, D f32
-DL_DEVINL uint32_t pt_idesc(int M, int N, int b_mn_major) {
+// instruction descriptor, kind::f16: A fp16 / bf16 K-major (or TMEM), B alike with selectable major-ness, D f32
+DL_DEVINL uint32_t pt_idesc(int M, int N, int b_mn_major, bool bf16) {
     uint32_t d = 0;
     d |= 1u << 4;                                  // D = f32
+    if (bf16) d |= (1u << 7) | (1u << 10);         // A and B = bf16
     d |= (uint32_t)(b_mn_major & 1) << 16;         // b_major: 0 = K, 1 = MN
     d |= (uint32_t)(N >> 3) << 17;
     d |= (uint32_t)(M >> 4) << 24;
     return d;
 }
-#define PT_STAMP(slot, j) do { if (a.stamps && blockIdx.x == 0 && blockIdx.y == 0 && (j) < 64) a.stamps[(j) * 8 + (slot)] = clock64(); } while (0)
+#define PT_STAMP(slot, j) do { if constexpr (!LINES) { if (a.stamps && blockIdx.x == 0 && blockIdx.y == 0 && (j) < 64) a.stamps[(j) * 8 + (slot)] = clock64(); } } while (0)
+#define PT_DBG(bit) (pt_dbg(a) & (bit))
+DL_DEVINL int pt_dbg(const PtArgs& a) { return a.dbg; }
+DL_DEVINL int pt_dbg(const PtLineArgs&) { return 0; }
 
 DL_DEVINL float pt_ex2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-DL_DEVINL uint32_t pt_pack_half2(float lo, float hi) {
+template <bool LINES> DL_DEVINL uint32_t pt_pack2(float lo, float hi) {
+    if (LINES) {
+        __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+        return *reinterpret_cast<uint32_t*>(&h);
+    }
     __half2 h = __floats2half2_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&h);
 }
@@ -120,7 +140,7 @@ DL_DEVINL float pt_ex2_poly(float x) {
 }
 
 // 32 scores (masked ones are -inf) -> exp2(s * sc - ref) as 16 packed fp16 pairs into TMEM; returns their sum
-DL_DEVINL float pt_probs(const uint32_t (&v)[32], float sc, float ref, uint32_t taddr) {
+template <bool LINES> DL_DEVINL float pt_probs(const uint32_t (&v)[32], float sc, float ref, uint32_t taddr) {
     uint32_t pk[16];
     float sum = 0.0f;
 #pragma unroll
@@ -129,16 +149,17 @@ DL_DEVINL float pt_probs(const uint32_t (&v)[32], float sc, float ref, uint32_t 
         const float xb = fmaf(__uint_as_float(v[e + 1]), sc, -ref);
         const float pb = (e & 2) ? pt_ex2_poly(xb) : pt_ex2(xb);
         sum += pa + pb;
-        pk[e >> 1] = pt_pack_half2(pa, pb);
+        pk[e >> 1] = pt_pack2<LINES>(pa, pb);
     }
     tmem_st_32x32b_x16(taddr, pk);
     return sum;
 }
 
-__global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(const __grid_constant__ PtArgs a, const __grid_constant__ CUtensorMap kmap,
-                                                                                const __grid_constant__ CUtensorMap vmap) {
+template <bool LINES>
+__global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(const __grid_constant__ typename PtKernelArgs<LINES>::T a,
+                                                                             const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap) {
     extern __shared__ __align__(1024) uint8_t smem[];
-    trace_begin(a.tr);
+    if constexpr (!LINES) trace_begin(a.tr);
     const unsigned long long t0 = globaltimer_ns();
     uint8_t* q_s = smem;                                        // Q tile, K-major core matrices
     uint8_t* k_s = smem + PT_TILE_BYTES;                        // [3] K tiles (tokens x head dim, K-major)
@@ -158,32 +179,68 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
     float* mx_s = reinterpret_cast<float*>(bars + 24);          // [2 step parities][2 halves][128 rows] row maxima (and row sums at the end)
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int head = blockIdx.y;
-    const int kvh = head / (a.n_heads / a.n_kv_heads);
+    int kvh, n_rows, r_first, p0, last_pos, seq_end, first_page, j0, j1, max_pages, n_kv, begin = 0, head = 0;
+    const int *bt, *rows_of = nullptr;
     pdl_launch_dependents();
-    pdl_wait();                                                  // q, this chunk's KV rows and meta come from earlier kernels
-    // which (segment, 128-row tile) is this CTA?  Large tiles (late rows: long histories) are handed out first.
-    int tile = blockIdx.x, begin = 0, end = 0;
-    {
-        const int n_seg = min(a.meta[0], PT_MAX_SEG);
-        int i = 0;
-        for (; i < n_seg; i++) {
-            begin = a.meta[1 + 2 * i];
-            end = a.meta[2 + 2 * i];
-            const int nt = (end - begin + PT_ROWS - 1) / PT_ROWS;
-            if (tile < nt) { tile = nt - 1 - tile; break; }
-            tile -= nt;
+    if constexpr (!LINES) {
+        head = blockIdx.y;
+        kvh = head / (a.n_heads / a.n_kv_heads);
+        pdl_wait();                                              // q, this chunk's KV rows and meta come from earlier kernels
+        // which (segment, 128-row tile) is this CTA?  Large tiles (late rows: long histories) are handed out first.
+        int tile = blockIdx.x, end = 0;
+        {
+            const int n_seg = min(a.meta[0], PT_MAX_SEG);
+            int i = 0;
+            for (; i < n_seg; i++) {
+                begin = a.meta[1 + 2 * i];
+                end = a.meta[2 + 2 * i];
+                const int nt = (end - begin + PT_ROWS - 1) / PT_ROWS;
+                if (tile < nt) { tile = nt - 1 - tile; break; }
+                tile -= nt;
+            }
+            if (i == n_seg) { trace_end(a.tr); return; }
         }
-        if (i == n_seg) { trace_end(a.tr); return; }
+        n_rows = end - begin;
+        r_first = tile * PT_ROWS;
+        p0 = a.pos[begin];
+        bt = a.block_table + (size_t)a.slot[begin] * a.max_pages;
+        last_pos = p0 + r_first + min(PT_ROWS, n_rows - r_first) - 1;
+        seq_end = p0 + n_rows;                                   // tokens of this sequence that exist
+        first_page = j0 = 0;
+        j1 = last_pos / PT_KV + 1;
+        n_kv = a.n_kv_heads;
+    } else {
+        // (launched behind a kernel that writes other rows of the same output and reads the same inputs: nothing to wait for here)
+        const DlWindowAttnArgs& w = a.w;
+        kvh = blockIdx.y;
+        const int t = (int)gridDim.x - 1 - (int)blockIdx.x;      // late tiles (long histories) first
+        auto count = [&](int u) { int n = 0; if (u < a.n_tiles) while (n < a.rq && a.tile_rows[(size_t)u * a.rq + n] >= 0) ++n; return n; };
+        const int e = t & ~1;                                    // an even tile takes its neighbour along where that continues its sequence
+        const int ne = count(e), no = count(e + 1);
+        bool both = ne == a.rq && no > 0;
+        if (both) {
+            const int me = a.tile_rows[(size_t)e * a.rq], mo = a.tile_rows[(size_t)(e + 1) * a.rq];
+            both = w.slot[me] == w.slot[mo] && w.pos[mo] == w.pos[me] + ne;
+        }
+        if ((t & 1) && both) return;
+        const int run = (t & 1) ? no : both ? ne + no : ne;
+        if (run * a.rep <= 16) return;                           // a decoding tile belongs to the other kernel
+        rows_of = a.tile_rows + (size_t)t * a.rq;
+        const int m0 = rows_of[0], p_first = w.pos[m0];
+        n_rows = run * a.rep;
+        r_first = 0;
+        p0 = p_first;
+        last_pos = p_first + run - 1;
+        seq_end = last_pos + 1;                                  // what lies behind was not written yet, or is of no use here
+        bt = w.block_table + (size_t)w.slot[m0] * w.max_pages;
+        int lo = w.window > 0 ? max(0, p_first - w.window + 1) : 0;
+        if (w.chunk > 0) lo = max(lo, p_first / w.chunk * w.chunk);
+        first_page = lo / 32;                                    // pages ahead of it are not touched
+        j0 = lo / PT_KV;
+        j1 = last_pos / PT_KV + 1;
+        n_kv = w.kv_heads;
     }
-    const int n_rows = end - begin;
-    const int r_first = tile * PT_ROWS;
-    const int rows_here = min(PT_ROWS, n_rows - r_first);
-    const int p0 = a.pos[begin];
-    const int* bt = a.block_table + (size_t)a.slot[begin] * a.max_pages;
-    const int last_pos = p0 + r_first + rows_here - 1;
-    const int seq_end = p0 + n_rows;                             // tokens of this sequence that exist
-    const int n_tiles = last_pos / PT_KV + 1;
+    const int n_tiles = j1 - j0;                                 // steps of 128 tokens, the first one at token j0 * 128
 
     if (tid == 0) {
         for (int s = 0; s < PT_STAGES; s++) {
@@ -214,7 +271,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
     const uint32_t desc_hi = (1024u >> 4) | (1u << 14) | (2u << 29);
     if (warp == 0) {
         // ------------------------------------ S = Q K^T issuer ------------------------------------
-        const uint32_t idesc_s = pt_idesc(PT_ROWS, PT_KV, 0);
+        const uint32_t idesc_s = pt_idesc(PT_ROWS, PT_KV, 0, LINES);
         auto lo_k = [](const void* p) { return ((smem_u32(p) & 0x3FFFFu) >> 4) | (1u << 16); };
         pt_wait(q_full, 0, t0);
         for (int j = 0; j < n_tiles; j++) {
@@ -230,7 +287,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
                     uint64_t da, db;
                     asm("mov.b64 %0, {%1, %2};" : "=l"(da) : "r"(a_lo + off), "r"(desc_hi));
                     asm("mov.b64 %0, {%1, %2};" : "=l"(db) : "r"(b_lo + off), "r"(desc_hi));
-                    if (!(a.dbg & 4)) umma_f16_ss(T_S + (j & 1) * 128, da, db, idesc_s, k > 0 ? 1u : 0u);
+                    if (!PT_DBG(4)) umma_f16_ss(T_S + (j & 1) * 128, da, db, idesc_s, k > 0 ? 1u : 0u);
                 }
                 umma_commit(&s_full[j & 1]);
                 umma_commit(&k_empty[j % PT_STAGES]);
@@ -240,14 +297,21 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
         }
     } else if (warp == 6) {
         // ------------------------------------ O += P V issuer ------------------------------------
-        const uint32_t idesc_pv = pt_idesc(PT_ROWS, PT_HS, 1);
+        const uint32_t idesc_pv = pt_idesc(PT_ROWS, PT_HS, 1, LINES);
         for (int i = 0; i < n_tiles; i++) {
             uint8_t* vz = v_s + (i % PT_STAGES) * PT_TILE_BYTES;
-            if ((i + 1) * PT_KV > seq_end) {
+            if (LINES && i == 0 && first_page * 32 > j0 * PT_KV) {      // tokens of pages that this tile does not touch
+                pt_wait(&v_full[0], 0, t0);
+                for (int idx = lane; idx < (first_page * 32 - j0 * PT_KV) * 16; idx += 32)
+                    *reinterpret_cast<uint4*>(vz + ((idx >> 3) & 1) * 16384 + (idx >> 4) * 128 + (idx & 7) * 16) = make_uint4(0, 0, 0, 0);
+                fence_proxy_async_smem();
+                __syncwarp();
+            }
+            if ((j0 + i + 1) * PT_KV > seq_end) {
                 // the step that contains the end of the sequence: rows past it were never written (or not copied at all);
                 // their scores are masked, but a zero probability times a non-finite V would poison the product -> zero them
                 pt_wait(&v_full[i % PT_STAGES], (i / PT_STAGES) & 1, t0);
-                const int r0 = max(0, seq_end - i * PT_KV);
+                const int r0 = max(0, seq_end - (j0 + i) * PT_KV);
                 for (int idx = r0 * 16 + lane; idx < PT_KV * 16; idx += 32) {      // 16 pieces of 16 B per token row (two halves)
                     const int r = idx >> 4, c = idx & 15;
                     *reinterpret_cast<uint4*>(vz + (c >> 3) * 16384 + r * 128 + (c & 7) * 16) = make_uint4(0, 0, 0, 0);
@@ -265,7 +329,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
                 for (int k = 0; k < 8; k++) {      // 16 tokens per MMA: 8 TMEM columns of P, two 8-token groups (2048 B) of V
                     uint64_t db;
                     asm("mov.b64 %0, {%1, %2};" : "=l"(db) : "r"(b_lo + k * 128), "r"(desc_hi));
-                    if (!(a.dbg & 4)) umma_f16_ts(T_O, T_P + (i & 1) * 64 + k * 8, db, idesc_pv, (i > 0 || k > 0) ? 1u : 0u);
+                    if (!PT_DBG(4)) umma_f16_ts(T_O, T_P + (i & 1) * 64 + k * 8, db, idesc_pv, (i > 0 || k > 0) ? 1u : 0u);
                 }
                 umma_commit(&o_full[i & 1]);
                 umma_commit(&v_empty[i % PT_STAGES]);
@@ -278,23 +342,48 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
         // (128 x 128 exp2) is fixed, but with two warps per scheduler the loads, maxima, packs and stores overlap it
         const int quarter = warp & 3, row = quarter * 32 + lane, hf = warp >= 8 ? 1 : 0;
         const int r_abs = r_first + row;
+        const int r_live = min(r_abs, n_rows - 1);
+        int m_row = 0, h_row = 0;                                // LINES: this row's batch row and head
         {
-            const float* qg = a.q + (size_t)(begin + min(r_abs, n_rows - 1)) * a.n_heads * PT_HS + head * PT_HS + hf * 64;
+            const float* qg;
+            if constexpr (LINES) {
+                m_row = rows_of[r_live / a.rep];
+                h_row = kvh * a.rep + r_live % a.rep;
+                qg = a.w.q + (size_t)m_row * a.w.ldq + h_row * PT_HS + hf * 64;
+            } else {
+                qg = a.q + (size_t)(begin + r_live) * a.n_heads * PT_HS + head * PT_HS + hf * 64;
+            }
             uint8_t* qd = q_s + hf * 16384 + row * 128;
 #pragma unroll 4
             for (int c = 0; c < 8; c++) {       // 16-byte piece c of this half of the row -> swizzled slot c ^ (row & 7)
                 const float4 x = reinterpret_cast<const float4*>(qg)[2 * c], y = reinterpret_cast<const float4*>(qg)[2 * c + 1];
                 uint4 u;
-                u.x = pt_pack_half2(x.x, x.y); u.y = pt_pack_half2(x.z, x.w);
-                u.z = pt_pack_half2(y.x, y.y); u.w = pt_pack_half2(y.z, y.w);
+                u.x = pt_pack2<LINES>(x.x, x.y); u.y = pt_pack2<LINES>(x.z, x.w);
+                u.z = pt_pack2<LINES>(y.x, y.y); u.w = pt_pack2<LINES>(y.z, y.w);
                 *reinterpret_cast<uint4*>(qd + ((c ^ (row & 7)) << 4)) = u;
             }
             fence_proxy_async_smem();
             mbar_arrive(q_full);
         }
-        const int pos_r = p0 + r_abs;
+        int pos_r, lb = 0;                                       // last and first visible position of this row
+        float sc, c1 = 0.f, cap_k = 0.f, slope = 0.f;
+        bool shaped = false;                                     // scores leave the accumulator through a cap or a bias
+        if constexpr (LINES) {
+            const DlWindowAttnArgs& w = a.w;
+            pos_r = p0 + r_live / a.rep;
+            if (w.window > 0) lb = max(0, pos_r - w.window + 1);
+            if (w.chunk > 0) lb = max(lb, pos_r / w.chunk * w.chunk);
+            shaped = w.softcap > 0.f || w.slope != nullptr;
+            sc = 1.4426950408889634f * w.scale;
+            c1 = w.softcap > 0.f ? sc * 2.f / w.softcap : sc;
+            cap_k = w.softcap * 1.4426950408889634f;
+            if (w.slope != nullptr) slope = w.slope[h_row] * 1.4426950408889634f;
+            if (shaped) sc = 1.f;
+        } else {
+            pos_r = p0 + r_abs;
+            sc = 1.4426950408889634f * rsqrtf((float)PT_HS);     // scores in the log2 domain
+        }
         const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
-        const float sc = 1.4426950408889634f * rsqrtf((float)PT_HS);      // scores in the log2 domain
         float m_used = -INFINITY, l = 0.0f;
         uint32_t v0[32], v1[32];
         for (int j = 0; j < n_tiles; j++) {
@@ -302,16 +391,32 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
             if (tid == 32) PT_STAMP(3, j);
             tc_fence_after();
             const uint32_t t_s = T_S + lane_base + (j & 1) * 128 + hf * 64;
-            const int tok0 = j * PT_KV + hf * 64;
-            if (a.dbg & 1) { tc_fence_before(); mbar_arrive(&s_empty[j & 1]); mbar_arrive(&p_full[j & 1]); continue; }
+            const int tok0 = (j0 + j) * PT_KV + hf * 64;
+            if PT_DBG(1) { tc_fence_before(); mbar_arrive(&s_empty[j & 1]); mbar_arrive(&p_full[j & 1]); continue; }
             tmem_ld_32x32b_x32(t_s, v0);
             tmem_ld_32x32b_x32(t_s + 32, v1);
             tmem_ld_wait();
             tc_fence_before();
             mbar_arrive(&s_empty[j & 1]);                    // the scores of step j+2 may overwrite the buffer now
             const int lim = pos_r - tok0;                    // columns e <= lim of this half are visible to this row
+            const int low = LINES ? lb - tok0 : 0;           // and e >= low
+            if constexpr (LINES) {
+                if (shaped) {
+#pragma unroll
+                    for (int e = 0; e < 64; e++) {
+                        float x = __uint_as_float(e < 32 ? v0[e & 31] : v1[e & 31]) * c1;
+                        if (cap_k > 0.f) {                   // cap tanh(s / cap) in base 2, as the mma.sync kernel forms it
+                            float r;
+                            asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(pt_ex2(x) + 1.f));
+                            x = fmaf(-2.f * cap_k, r, cap_k);
+                        }
+                        x = fmaf(-slope, (float)(lim - e), x);
+                        if (e < 32) v0[e & 31] = __float_as_uint(x); else v1[e & 31] = __float_as_uint(x);
+                    }
+                }
+            }
             float ma = -INFINITY, mb = -INFINITY;
-            if (lim >= 63) {
+            if (lim >= 63 && (!LINES || low <= 0)) {
 #pragma unroll
                 for (int e = 0; e < 32; e += 2) {
                     ma = fmaxf(ma, fmaxf(__uint_as_float(v0[e]), __uint_as_float(v1[e])));
@@ -320,8 +425,8 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
             } else {
 #pragma unroll
                 for (int e = 0; e < 32; e++) {
-                    if (e > lim) v0[e] = 0xff800000u;        // -inf
-                    if (e + 32 > lim) v1[e] = 0xff800000u;
+                    if (e > lim || (LINES && e < low)) v0[e] = 0xff800000u;        // -inf
+                    if (e + 32 > lim || (LINES && e + 32 < low)) v1[e] = 0xff800000u;
                     ma = fmaxf(ma, fmaxf(__uint_as_float(v0[e]), __uint_as_float(v1[e])));
                 }
             }
@@ -360,8 +465,8 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
                 pt_wait(&o_full[j & 1], ((j - 2) >> 1) & 1, t0);
                 tc_fence_after();
             }
-            l += pt_probs(v0, sc, ref, t_p);
-            l += pt_probs(v1, sc, ref, t_p + 16);
+            l += pt_probs<LINES>(v0, sc, ref, t_p);
+            l += pt_probs<LINES>(v1, sc, ref, t_p + 16);
             tmem_st_wait();
             tc_fence_before();
             mbar_arrive(&p_full[j & 1]);
@@ -376,7 +481,13 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
         mx_s[(fs + hf) * PT_ROWS + row] = l;
         asm volatile("bar.sync 2, 256;" ::: "memory");
         l += mx_s[(fs + (hf ^ 1)) * PT_ROWS + row];
-        const float inv = l > 0.0f ? 1.0f / l : 0.0f;
+        float inv;
+        if constexpr (LINES) {
+            if (a.w.sink) l += pt_ex2(a.w.sink[h_row] * 1.4426950408889634f - m_used);
+            inv = (a.w.gate ? 1.f / (1.f + expf(-a.w.gate[(size_t)m_row * a.w.ld_gate + h_row])) : 1.f) / l;
+        } else {
+            inv = l > 0.0f ? 1.0f / l : 0.0f;
+        }
 #pragma unroll 1
         for (int ch = 0; ch < 2; ch++) {
             tmem_ld_32x32b_x32(T_O + lane_base + hf * 64 + ch * 32, v0);
@@ -388,12 +499,18 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
         for (int rr = 0; rr < 32; rr++) {
             const int rc = r_first + quarter * 32 + rr;
             if (rc >= n_rows) break;
+            if constexpr (LINES) {
+                float* dst = a.w.out + (size_t)__shfl_sync(0xffffffffu, m_row, rr) * a.w.ldo + __shfl_sync(0xffffffffu, h_row, rr) * PT_HS + hf * 64 + lane;
+                dst[0] = out_s[(quarter * 32 + rr) * PT_OUT_LD + hf * 64 + lane];
+                dst[32] = out_s[(quarter * 32 + rr) * PT_OUT_LD + hf * 64 + 32 + lane];
+            } else {
             const int m = begin + rc;
 #pragma unroll
             for (int b = 0; b < 2; b++) {
                 const float val = out_s[(quarter * 32 + rr) * PT_OUT_LD + hf * 64 + b * 32 + lane];
                 q80_block_store(val, lane, m, (head * PT_HS) / 32 + hf * 2 + b, a.out_mcap, a.xq_out, a.xh_out);
                 if (a.y_out != nullptr) a.y_out[(size_t)m * a.n_heads * PT_HS + head * PT_HS + hf * 64 + b * 32 + lane] = val;
+            }
             }
         }
     } else if (warp == 5 || warp == 7) {
@@ -405,32 +522,35 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
             uint64_t* empty = is_k ? k_empty : v_empty;
             uint8_t* ring = is_k ? k_s : v_s;
             const int total_pages = (seq_end + 31) / 32;
+            auto page_of = [&](int p) { return p >= first_page && p < total_pages ? bt[p] : 0; };
             // the page ids of a step are fetched one step ahead, so the table reads (dependent global loads) overlap the
             // wait for a free stage instead of delaying the copies
             int pg[4], pg_next[4];
 #pragma unroll
-            for (int p4 = 0; p4 < 4; p4++) pg_next[p4] = (p4 < total_pages) ? bt[p4] : 0;
+            for (int p4 = 0; p4 < 4; p4++) pg_next[p4] = page_of(4 * j0 + p4);
             for (int j = 0; j < n_tiles; j++) {
                 const int st = j % PT_STAGES;
 #pragma unroll
                 for (int p4 = 0; p4 < 4; p4++) {
                     pg[p4] = pg_next[p4];
-                    pg_next[p4] = (4 * (j + 1) + p4 < total_pages) ? bt[4 * (j + 1) + p4] : 0;
+                    pg_next[p4] = page_of(4 * (j0 + j + 1) + p4);
                 }
                 if (j >= PT_STAGES) pt_wait(&empty[st], ((j / PT_STAGES) & 1) ^ 1, t0);
                 if (is_k) PT_STAMP(6, j);
-                const int n_pg = (a.dbg & 2) ? 0 : min(4, (seq_end - j * PT_KV + 31) / 32);      // pages of this step that exist
-                mbar_arrive_expect_tx(&full[st], (uint32_t)n_pg * 2u * 4096u);
+                const int n_pg = PT_DBG(2) ? 0 : min(4, (seq_end - (j0 + j) * PT_KV + 31) / 32);      // pages of this step that exist
+                const int p_lo = LINES ? max(0, first_page - 4 * (j0 + j)) : 0;                 // ... and are looked at (at most the first step starts later)
+                mbar_arrive_expect_tx(&full[st], (uint32_t)max(0, n_pg - p_lo) * 2u * 4096u);
                 const uint32_t dst = smem_u32(ring + st * PT_TILE_BYTES), bar = smem_u32(&full[st]);
 #pragma unroll
                 for (int p4 = 0; p4 < 4; p4++) {
                     if (p4 >= n_pg) break;
-                    const int y = (pg[p4] * a.n_kv_heads + kvh) * 32;      // first row of the page in the [rows][128] view
+                    if (LINES && p4 < p_lo) continue;
+                    const int y = (pg[p4] * n_kv + kvh) * 32;      // first row of the page in the [rows][128] view
 #pragma unroll
                     for (int h = 0; h < 2; h++)
                         asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
                                          dst + h * 16384 + p4 * 4096),
-                                     "l"(map), "r"(h * 64), "r"(y), "r"(bar)
+                                     "l"(map), "r"((LINES && !is_k ? PT_HS : 0) + h * 64), "r"(y), "r"(bar)
                                      : "memory");
                 }
                 if (is_k) PT_STAMP(7, j);
@@ -443,7 +563,8 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
         tc_fence_after();
         tmem_dealloc(tmem_base, 512);
     }
-    trace_end(a.tr);
+    if constexpr (LINES) pdl_wait();                             // what follows this grid follows the one ahead of it too
+    else trace_end(a.tr);
 }
 
 extern void dl_set_error(const char* fmt, ...);
@@ -456,9 +577,9 @@ typedef CUresult (*PtEncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-// [rows][128] fp16 view of a KV cache on THIS GPU (rows = pages x kv heads x 32), box = 64 columns x 32 rows (one page of
+// [rows][width] fp16 or bf16 view of a KV cache on THIS GPU (rows = pages x kv heads x 32), box = 64 columns x 32 rows (one page of
 // one head, half of the head dimension), 128-byte swizzle: the image tcgen05.mma reads as a swizzled K- or MN-major tile
-static int pt_make_map(CUtensorMap* m, const void* base, long long rows) {
+static int pt_make_map(CUtensorMap* m, const void* base, long long rows, int width, bool bf16) {
     static PtEncodeTiled enc = nullptr;
     if (enc == nullptr) {
         void* fn = nullptr;
@@ -469,10 +590,10 @@ static int pt_make_map(CUtensorMap* m, const void* base, long long rows) {
         }
         enc = (PtEncodeTiled)fn;
     }
-    const cuuint64_t dims[2] = {PT_HS, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {PT_HS * 2};
+    const cuuint64_t dims[2] = {(cuuint64_t)width, (cuuint64_t)rows};
+    const cuuint64_t strides[1] = {(cuuint64_t)width * 2};
     const cuuint32_t box[2] = {64, 32}, es[2] = {1, 1};
-    const CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    const CUresult r = enc(m, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
                            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) { dl_set_error("attention_prefill_tc: cuTensorMapEncodeTiled failed (%d)", (int)r); return -1; }
     return 0;
@@ -494,11 +615,11 @@ extern "C" int dl_attention_prefill_tc(const float* q, int M, int n_heads, int n
     a.tr = dl_trace_next(TR_ATT);
     alignas(64) CUtensorMap kmap, vmap;
     const long long rows = (long long)n_cache_pages * n_kv_heads * 32;
-    if (pt_make_map(&kmap, k_cache, rows) != 0 || pt_make_map(&vmap, v_cache, rows) != 0) return -1;
+    if (pt_make_map(&kmap, k_cache, rows, PT_HS, false) != 0 || pt_make_map(&vmap, v_cache, rows, PT_HS, false) != 0) return -1;
     const size_t smem = (1 + 2 * PT_STAGES) * PT_TILE_BYTES + 24 * 8 + 4 * PT_ROWS * 4;
     static bool set = false;
     if (!set) {
-        cudaError_t e = cudaFuncSetAttribute(attention_prefill_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = cudaFuncSetAttribute(attention_prefill_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) { dl_set_error("attention_prefill_tc smem attr: %s", cudaGetErrorString(e)); return -(int)e; }
         set = true;
     }
@@ -514,7 +635,43 @@ extern "C" int dl_attention_prefill_tc(const float* q, int M, int n_heads, int n
         cfg.attrs = attr;
         cfg.numAttrs = 1;
     }
-    cudaError_t e = cudaLaunchKernelEx(&cfg, attention_prefill_tc_kernel, a, kmap, vmap);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, attention_prefill_tc_kernel<false>, a, kmap, vmap);
     if (e != cudaSuccess) { dl_set_error("attention_prefill_tc launch: %s", cudaGetErrorString(e)); return -(int)e; }
+    return 0;
+}
+
+// 0 if the kernel's LINES instance takes these sizes: bf16 lines of a key and a value of 128, full tiles of 64 stacked rows
+int dl_window_prefill_tc_supported(const DlWindowAttnArgs& a, int rq) {
+    const int rep = a.kv_heads > 0 ? a.heads / a.kv_heads : 0;
+    return a.dim == PT_HS && a.vdim == PT_HS && a.page_size == 32 && rep > 0 && rq * rep == PT_ROWS / 2 &&
+                   ((uintptr_t)a.cache & 15) == 0 ? 0 : -1;
+}
+
+// The tiles of more than 16 stacked rows; launched behind the kernel that takes the others (programmatic launch: they run side by side).
+int dl_window_prefill_tc(const DlWindowAttnArgs& w, const int* tile_rows, int n_tiles, int rq, cudaStream_t stream) {
+    PtLineArgs a;
+    a.w = w; a.tile_rows = tile_rows; a.n_tiles = n_tiles; a.rq = rq; a.rep = w.heads / w.kv_heads;
+    alignas(64) CUtensorMap map;
+    // the cache's page count is not known here; every copy reads a page that the block table names
+    if (pt_make_map(&map, w.cache, 1ll << 31, 2 * PT_HS, true) != 0) return -1;
+    const size_t smem = (1 + 2 * PT_STAGES) * PT_TILE_BYTES + 24 * 8 + 4 * PT_ROWS * 4;
+    static bool set = false;
+    if (!set) {
+        cudaError_t e = cudaFuncSetAttribute(attention_prefill_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) { dl_set_error("window_prefill_tc smem attr: %s", cudaGetErrorString(e)); return -(int)e; }
+        set = true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)n_tiles, (unsigned)w.kv_heads);
+    cfg.blockDim = dim3(PT_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, attention_prefill_tc_kernel<true>, a, map, map);
+    if (e != cudaSuccess) { dl_set_error("window_prefill_tc launch: %s", cudaGetErrorString(e)); return -(int)e; }
     return 0;
 }

@@ -367,9 +367,186 @@ __host__ __device__ __forceinline__ int wm_line_stride(int LD) {      // bf16 el
     return s;
 }
 
+// A decoding tile: all its stacked rows fit ONE 16-row MMA tile, so the four warps share the tokens instead of the rows.  A warp
+// takes every fourth half page (16 tokens) through a buffer of its own -- no barrier between warps until the merge in shared memory;
+// 16 warps per SM keep ~100 KB in flight.  As a quarter-full row tile (one warp of four multiplying, a barrier per page) 32 rows over
+// 1000 to 2000 positions of 4 key/value heads took 58.5 us with the merge; 40.1 now.
+template <int DK>
+__device__ __forceinline__ void window_small_tile(const DlWindowAttnArgs& a, const int* s_row, int n_rows, int tile, int g, int n_splits, int pg_lo, int pg_hi, int lo,
+                                                  int p_first, int slot, __nv_bfloat16* smem, float* __restrict__ partial) {
+    constexpr int D = 16 * DK, NV = D / 8, QS = D + 8;
+    const int RD = a.rope_dims, LD = D + (a.vdim > 0 ? a.vdim : RD), LDS = wm_line_stride(LD), rep = a.heads / a.kv_heads;
+    const bool own_v = a.vdim > 0, capped = a.softcap > 0.f, biased = a.slope != nullptr;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3, mat = lane >> 3, rr = lane & 7;
+    const float c1 = capped ? a.scale * 2.f / a.softcap * WM_LOG2E : a.scale * WM_LOG2E, capK = a.softcap * WM_LOG2E;
+    __nv_bfloat16* kv = smem + (size_t)warp * 16 * LDS;                              // this warp's half page; behind the four: the queries
+    __nv_bfloat16* q_s = smem + (size_t)4 * 16 * LDS;
+    for (int idx = threadIdx.x; idx < 16 * (D / 4); idx += 128) {
+        const int sr = idx / (D / 4), c4 = idx - sr * (D / 4), r = sr / rep;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (r < n_rows) v = *reinterpret_cast<const float4*>(a.q + (size_t)s_row[r] * a.ldq + (size_t)(g * rep + sr % rep) * D + c4 * 4);
+        uint2 pk;
+        pk.x = pack_bf16(v.x, v.y);
+        pk.y = pack_bf16(v.z, v.w);
+        *reinterpret_cast<uint2*>(q_s + (size_t)sr * QS + c4 * 4) = pk;
+    }
+    __syncthreads();
+    uint32_t qf[DK][4];
+#pragma unroll
+    for (int kk = 0; kk < DK; ++kk) ldmatrix_x4(qf[kk], q_s + (size_t)((mat & 1) * 8 + rr) * QS + kk * 16 + (mat >> 1) * 8);
+    int pos_[2], cs_[2];
+    bool ok_[2];
+    float sl_[2], m_[2] = {-INFINITY, -INFINITY}, l_[2] = {0.f, 0.f};
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const int s = gid + u * 8, r = s / rep;
+        ok_[u] = r < n_rows;
+        pos_[u] = p_first + r;
+        cs_[u] = a.chunk > 0 ? pos_[u] / a.chunk * a.chunk : 0;
+        sl_[u] = biased ? a.slope[g * rep + s % rep] * WM_LOG2E : 0.f;
+    }
+    float o[NV][4];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) { o[v][0] = o[v][1] = o[v][2] = o[v][3] = 0.f; }
+    const int p_last = p_first + n_rows - 1, parts = LD / 8, cs_last = a.chunk > 0 ? p_last / a.chunk * a.chunk : 0;
+    for (int hp = 2 * pg_lo + warp; hp <= 2 * pg_hi + 1; hp += 4) {
+        const int first = hp * 16;
+        if (first > p_last) break;
+        if (first + 15 < lo) continue;
+        const int page = a.block_table[(size_t)slot * a.max_pages + (hp >> 1)];
+        const __nv_bfloat16* src = (const __nv_bfloat16*)a.cache + (((size_t)page * a.kv_heads + g) * WA_PAGE + (hp & 1) * 16) * LD;
+        __syncwarp();                                          // every lane is done with the last half page
+        if (parts == 32) {                                     // key and value of 128: a line per instruction
+#pragma unroll
+            for (int j = 0; j < 16; ++j) cp_async16(kv + j * LDS + lane * 8, src + j * 256 + lane * 8);
+        } else {
+            for (int c = lane; c < 16 * parts; c += 32) {
+                const int j = c / parts, part = c - j * parts;
+                cp_async16(kv + (size_t)j * LDS + part * 8, src + (size_t)c * 8);
+            }
+        }
+        cp_async_wait_all();
+        __syncwarp();
+        float sc[2][4];
+#pragma unroll
+        for (int n = 0; n < 2; ++n) sc[n][0] = sc[n][1] = sc[n][2] = sc[n][3] = 0.f;
+#pragma unroll
+        for (int kk = 0; kk < DK; ++kk) {
+            uint32_t b[4];
+            ldmatrix_x4(b, kv + (size_t)((mat >> 1) * 8 + rr) * LDS + kk * 16 + (mat & 1) * 8);
+            mma_bf16(sc[0], qf[kk], b[0], b[1]);
+            mma_bf16(sc[1], qf[kk], b[2], b[3]);
+        }
+        float mx[2] = {-INFINITY, -INFINITY};
+        // (stacked rows without a position are never stored)
+        const bool whole = first + 15 <= p_first && (a.window == 0 || p_last - first < a.window) && first >= cs_last;
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                float s2 = sc[n][e] * c1;
+                if (capped) s2 = fmaf(-2.f * capK, fast_rcp(fast_ex2(s2) + 1.f), capK);
+                sc[n][e] = s2;
+            }
+        if (biased || !whole) {
+#pragma unroll
+            for (int n = 0; n < 2; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int u = e >> 1, j = first + n * 8 + tig * 2 + (e & 1);
+                    const float s2 = fmaf(-sl_[u], (float)(pos_[u] - j), sc[n][e]);
+                    const bool vis = ok_[u] && j <= pos_[u] && (a.window == 0 || pos_[u] - j < a.window) && j >= cs_[u];
+                    sc[n][e] = vis ? s2 : -INFINITY;
+                }
+        }
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) mx[e >> 1] = fmaxf(mx[e >> 1], sc[n][e]);
+        float al[2], ref[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            mx[u] = fmaxf(mx[u], __shfl_xor_sync(0xffffffffu, mx[u], 1));
+            mx[u] = fmaxf(mx[u], __shfl_xor_sync(0xffffffffu, mx[u], 2));
+            const float mn = fmaxf(m_[u], mx[u]);
+            al[u] = m_[u] == -INFINITY ? 0.f : fast_ex2(m_[u] - mn);
+            ref[u] = mn == -INFINITY ? 0.f : mn;
+            m_[u] = mn;
+            l_[u] *= al[u];
+        }
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                sc[n][e] = fast_ex2(sc[n][e] - ref[e >> 1]);
+                l_[e >> 1] += sc[n][e];
+            }
+        if (__any_sync(0xffffffffu, al[0] != 1.f || al[1] != 1.f)) {
+#pragma unroll
+            for (int v = 0; v < NV; ++v) { o[v][0] *= al[0]; o[v][1] *= al[0]; o[v][2] *= al[1]; o[v][3] *= al[1]; }
+        }
+        uint32_t pa[4];
+        pa[0] = pack_bf16(sc[0][0], sc[0][1]);
+        pa[1] = pack_bf16(sc[0][2], sc[0][3]);
+        pa[2] = pack_bf16(sc[1][0], sc[1][1]);
+        pa[3] = pack_bf16(sc[1][2], sc[1][3]);
+#pragma unroll
+        for (int vp = 0; vp < NV / 2; ++vp) {
+            const int vt = 2 * vp + (mat >> 1);
+            const int col = (own_v || vt * 8 < RD) ? D + vt * 8 : vt * 8;
+            uint32_t b[4];
+            ldmatrix_x4_trans(b, kv + (size_t)((mat & 1) * 8 + rr) * LDS + col);
+            mma_bf16(o[2 * vp], pa, b[0], b[1]);
+            mma_bf16(o[2 * vp + 1], pa, b[2], b[3]);
+        }
+    }
+    // the warps' shares meet in the buffers' place: [warp][16][D], maxima and sums behind
+    __syncthreads();
+    float* acc = reinterpret_cast<float*>(smem);
+    float* ml = acc + 4 * 16 * D;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        l_[u] += __shfl_xor_sync(0xffffffffu, l_[u], 1);
+        l_[u] += __shfl_xor_sync(0xffffffffu, l_[u], 2);
+        float* dst = acc + (size_t)(warp * 16 + gid + u * 8) * D;
+        if (ok_[u]) {
+#pragma unroll
+            for (int v = 0; v < NV; ++v) *reinterpret_cast<float2*>(dst + v * 8 + tig * 2) = make_float2(o[v][2 * u], o[v][2 * u + 1]);
+            if (tig == 0) { ml[(warp * 16 + gid + u * 8) * 2] = m_[u]; ml[(warp * 16 + gid + u * 8) * 2 + 1] = l_[u]; }
+        }
+    }
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < n_rows * rep * (D / 4); idx += 128) {
+        const int sr = idx / (D / 4), c4 = idx - sr * (D / 4), r = sr / rep, h = g * rep + sr % rep;
+        float mx = -INFINITY, l = 0.f;
+#pragma unroll
+        for (int w = 0; w < 4; ++w) mx = fmaxf(mx, ml[(w * 16 + sr) * 2]);
+        float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+            const float mw = ml[(w * 16 + sr) * 2], e = mw == -INFINITY ? 0.f : fast_ex2(mw - mx);
+            const float4 v = *reinterpret_cast<const float4*>(acc + (size_t)(w * 16 + sr) * D + c4 * 4);
+            l = fmaf(e, ml[(w * 16 + sr) * 2 + 1], l);
+            t.x = fmaf(e, v.x, t.x); t.y = fmaf(e, v.y, t.y); t.z = fmaf(e, v.z, t.z); t.w = fmaf(e, v.w, t.w);
+        }
+        if (n_splits > 1) {
+            float* dst = partial + ((((size_t)tile * a.kv_heads + g) * n_splits + blockIdx.z) * WM_ROWS + sr) * (D + 2);
+            *reinterpret_cast<float2*>(dst + c4 * 4) = make_float2(t.x, t.y);
+            *reinterpret_cast<float2*>(dst + c4 * 4 + 2) = make_float2(t.z, t.w);
+            if (c4 == 0) { dst[D] = mx * WM_LN2; dst[D + 1] = l; }
+            continue;
+        }
+        if (a.sink) l += fast_ex2(a.sink[h] * WM_LOG2E - mx);
+        const float inv = (a.gate ? sigmoid_f(a.gate[(size_t)s_row[r] * a.ld_gate + h]) : 1.f) / l;
+        float* dst = a.out + (size_t)s_row[r] * a.ldo + (size_t)h * D + c4 * 4;
+        *reinterpret_cast<float2*>(dst) = make_float2(t.x * inv, t.y * inv);
+        *reinterpret_cast<float2*>(dst + 2) = make_float2(t.z * inv, t.w * inv);
+    }
+}
+
 template <int DK>
 __global__ void __launch_bounds__(128, 4) window_attention_mma_kernel(DlWindowAttnArgs a, const int* __restrict__ tile_rows, int rq,
-                                                                   int n_splits, float* __restrict__ partial) {
+                                                                   int n_splits, float* __restrict__ partial, int only_small, int max_small) {
     constexpr int D = 16 * DK, NV = D / 8;
     extern __shared__ __align__(16) uint8_t smraw[];
     __shared__ int s_row[WM_ROWS];
@@ -380,6 +557,7 @@ __global__ void __launch_bounds__(128, 4) window_attention_mma_kernel(DlWindowAt
     __nv_bfloat16* q_s = kv_s + (size_t)2 * WA_PAGE * LDS;                          // [WM_ROWS][QS]: the stacked queries
     const int tile = blockIdx.x, g = blockIdx.y, rep = a.heads / a.kv_heads;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");      // the merge (its CTAs wait for this grid's end), or the tiles of many rows
     if (threadIdx.x < rq) s_row[threadIdx.x] = tile_rows[(size_t)tile * rq + threadIdx.x];
     __syncthreads();
     int n_rows = 0;
@@ -390,10 +568,26 @@ __global__ void __launch_bounds__(128, 4) window_attention_mma_kernel(DlWindowAt
     if (a.chunk > 0) lo = max(lo, p_first / a.chunk * a.chunk);
     int pg_lo = lo / WA_PAGE, pg_hi = p_last / WA_PAGE;
     if (n_splits > 1) {                  // this CTA's share of the tile's pages (possibly none)
-        const int per = (pg_hi - pg_lo + n_splits) / n_splits;
+        // a decoding tile needs no more shares than fill the SMs: a warp of a share of 5 pages spends more on its start and its part of the
+        // merge than on its two or three half pages
+        const int shares = n_rows * rep <= 16 ? min(n_splits, max_small) : n_splits;
+        const int per = (pg_hi - pg_lo + shares) / shares;
         pg_lo += (int)blockIdx.z * per;
         pg_hi = min(pg_hi, pg_lo + per - 1);
     }
+    if (n_rows * rep <= 16) {            // decoding: one 16-row tile, the warps share the tokens
+        if (pg_lo > pg_hi) {             // a share without pages (of several): it weighs nothing
+            if (threadIdx.x < n_rows * rep) {
+                float* dst = partial + ((((size_t)tile * a.kv_heads + g) * n_splits + blockIdx.z) * WM_ROWS + threadIdx.x) * (D + 2) + D;
+                dst[0] = -INFINITY;
+                dst[1] = 0.f;
+            }
+            return;
+        }
+        window_small_tile<DK>(a, s_row, n_rows, tile, g, n_splits, pg_lo, pg_hi, lo, p_first, slot, kv_s, partial);
+        return;
+    }
+    if (only_small) return;              // attention_prefill_tc.cu takes the others
     const bool active = warp * 16 < n_rows * rep;
     const bool capped = a.softcap > 0.f, biased = a.slope != nullptr;
     const float c1 = capped ? a.scale * 2.f / a.softcap * WM_LOG2E : a.scale * WM_LOG2E;
@@ -559,8 +753,9 @@ __global__ void __launch_bounds__(128) window_merge_kernel(DlWindowAttnArgs a, c
                                                            const float* __restrict__ partial) {
     __shared__ float w_s[WM_ROWS * WM_MAX_SPLITS];
     const int tile = blockIdx.x, g = blockIdx.y, r = blockIdx.z, D = a.dim, rep = a.heads / a.kv_heads;
-    const int m = tile_rows[(size_t)tile * rq + r];
+    const int m = tile_rows[(size_t)tile * rq + r];                           // not written by the kernel that this launch runs ahead of
     if (m < 0) return;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const float* base = partial + ((size_t)tile * a.kv_heads + g) * n_splits * WM_ROWS * (D + 2);
     for (int hg = threadIdx.x >> 5; hg < rep; hg += blockDim.x >> 5) {        // a warp per head, a lane per share
         const int k = threadIdx.x & 31;
@@ -576,18 +771,22 @@ __global__ void __launch_bounds__(128) window_merge_kernel(DlWindowAttnArgs a, c
     for (int idx = threadIdx.x; idx < rep * D; idx += blockDim.x) {
         const int hg = idx / D, c = idx - hg * D;
         const float* p = base + (size_t)(r * rep + hg) * (D + 2) + c;
-        float acc = 0.f;                      // a share without pages left zeros and weighs 0: sixteen shares are in flight at once
+        float acc = 0.f;                      // a share without pages weighs 0, whatever it left: sixteen shares are in flight at once
         for (int k0 = 0; k0 < n_splits; k0 += 16) {
             float v[16];
 #pragma unroll
             for (int k = 0; k < 16; ++k) v[k] = k0 + k < n_splits ? p[(size_t)(k0 + k) * WM_ROWS * (D + 2)] : 0.f;
 #pragma unroll
             for (int k = 0; k < 16; ++k)
-                if (k0 + k < n_splits) acc = fmaf(w_s[hg * n_splits + k0 + k], v[k], acc);
+                if (k0 + k < n_splits && w_s[hg * n_splits + k0 + k] != 0.f) acc = fmaf(w_s[hg * n_splits + k0 + k], v[k], acc);
         }
         a.out[(size_t)m * a.ldo + (size_t)(g * rep + hg) * D + c] = acc;
     }
 }
+
+// attention_prefill_tc.cu
+int dl_window_prefill_tc_supported(const DlWindowAttnArgs& a, int rq);
+int dl_window_prefill_tc(const DlWindowAttnArgs& a, const int* tile_rows, int n_tiles, int rq, cudaStream_t stream);
 
 // rows of one sequence per tile: as many positions as fit 64 stacked (position, head) pairs
 extern "C" int dl_window_tc_rows(int heads, int kv_heads) {
@@ -624,19 +823,39 @@ extern "C" int dl_window_attention_tc(const DlWindowAttnArgs* args, const int* t
     if (n_tiles < 1) return 0;
     if (n_splits < 1 || n_splits > WM_MAX_SPLITS || (n_splits > 1 && partial == nullptr)) { dl_set_error("dl_window_attention_tc: n_splits %d without scratch", n_splits); return -1; }
     const size_t smem = ((size_t)2 * WA_PAGE * wm_line_stride(a.dim + (a.vdim > 0 ? a.vdim : a.rope_dims)) + (size_t)WM_ROWS * (a.dim + 8)) * sizeof(__nv_bfloat16);
+    // tiles enough for the chip without sharing pages are prompt portions (or very many users, whose tiles stay here): tcgen05, 128 stacked rows
+    const bool tc5 = n_splits == 1 && dl_window_prefill_tc_supported(a, rq) == 0;
+    const int max_small = (3 * dl_device_sm_count() + n_tiles * a.kv_heads - 1) / (n_tiles * a.kv_heads);
     dim3 grid(n_tiles, a.kv_heads, n_splits);
     cudaStream_t st = (cudaStream_t)stream;
     switch (a.dim / 16) {
 #define WM_CASE(DK_)                                                                                                      \
     case DK_:                                                                                                             \
         if (smem > 48 * 1024) cudaFuncSetAttribute(window_attention_mma_kernel<DK_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-        window_attention_mma_kernel<DK_><<<grid, 128, smem, st>>>(a, tile_rows, rq, n_splits, partial);                  \
+        window_attention_mma_kernel<DK_><<<grid, 128, smem, st>>>(a, tile_rows, rq, n_splits, partial, tc5 ? 1 : 0, max_small);                  \
         break;
         WM_CASE(1) WM_CASE(2) WM_CASE(3) WM_CASE(4) WM_CASE(6) WM_CASE(8)
 #undef WM_CASE
         default: dl_set_error("dl_window_attention_tc: dim %d", a.dim); return -1;
     }
-    if (n_splits > 1) window_merge_kernel<<<dim3(n_tiles, a.kv_heads, rq), 128, 0, st>>>(a, tile_rows, rq, n_splits, partial);
+    if (tc5) {
+        LAYER_CHECK_LAUNCH("dl_window_attention_tc");
+        const int rc = dl_window_prefill_tc(a, tile_rows, n_tiles, rq, st);
+        if (rc != 0) return rc;
+    }
+    if (n_splits > 1) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(n_tiles, a.kv_heads, rq);
+        cfg.blockDim = dim3(128);
+        cfg.stream = st;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        cudaError_t e = cudaLaunchKernelEx(&cfg, window_merge_kernel, a, tile_rows, rq, n_splits, (const float*)partial);
+        if (e != cudaSuccess) { dl_set_error("window merge launch: %s", cudaGetErrorString(e)); return -(int)e; }
+    }
     LAYER_CHECK_LAUNCH("dl_window_attention_tc");
     return 0;
 }

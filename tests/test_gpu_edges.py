@@ -199,3 +199,44 @@ def test_norm_q80_rows_per_cta(M, dim):
     sums = raw[:, :, 144:160].contiguous().view(torch.int32).view(kp // 128, M, 4)
     live = sums.permute(1, 0, 2).reshape(M, kp // 32)[:, :dim // 32]
     assert (live == 8 * q.sum(dim=3).long().permute(1, 0, 2).reshape(M, kp // 32)[:, :dim // 32]).all()
+
+
+@pytest.mark.parametrize("window,chunk,softcap,extra", [(0, 0, 0.0, False), (50, 0, 0.0, True), (130, 0, 30.0, True), (0, 64, 0.0, False), (1, 0, 0.0, False)])
+def test_window_prompt_tiles(window, chunk, softcap, extra):
+    """Tiles of many rows (tcgen05, two neighbours on 128 lanes where the second continues the first) beside decoding tiles, in one call: pairs
+    that fit and that do not, a last tile of few rows, windows that start inside a page, pages ahead of a window full of NaN and never
+    touched.  Bound: queries and weights are rounded to bf16 (2^-9 each), so about 2e-3 of a row; 8e-3."""
+    heads, kv, dim, pages = 8, 2, 128, 12
+    g = torch.Generator().manual_seed(window + chunk)
+    runs = [(100, 37), (211, 1), (0, 20), (300, 16), (64, 16), (0, 3), (31, 64)]             # (first position, rows) per sequence
+    M, S = sum(n for _, n in runs), len(runs)
+    cache = torch.randn(S * pages, kv, 32, 2 * dim, generator=g).bfloat16()
+    bt = torch.randperm(S * pages, generator=g).int().view(S, pages)
+    pos, slot, tiles = [], [], []
+    for s, (p0, n) in enumerate(runs):
+        rows = list(range(len(pos), len(pos) + n))
+        pos += list(range(p0, p0 + n))
+        slot += [s] * n
+        tiles += [rows[i:i + 16] for i in range(0, n, 16)]
+        lo = max(0, p0 - window + 1) if window else p0 // chunk * chunk if chunk else 0
+        cache[bt[s, :lo // 32].long()] = float("nan")
+        cache[bt[s, (p0 + n + 31) // 32:].long()] = float("nan")
+    q, sink, slope, gate = torch.randn(M, heads * dim, generator=g), torch.randn(heads, generator=g), torch.rand(heads, generator=g) * 0.1, torch.randn(M, heads, generator=g)
+    opt = dict(sink=sink.cuda(), slope=slope.cuda(), gate=gate.cuda()) if extra else {}
+    out = torch.zeros(M, heads * dim, device="cuda")
+    L().window_attention_tiles(q.cuda(), out, heads, kv, dim, 0, 0.2, softcap, window, torch.tensor(pos, dtype=torch.int32, device="cuda"),
+                               torch.tensor(slot, dtype=torch.int32, device="cuda"), bt.cuda(), cache.cuda(), tiles, vdim=dim, chunk=chunk, **opt)
+    got = out.cpu().double().view(M, heads, dim)
+    for m in range(M):
+        p = pos[m]
+        lo = max(p - window + 1 if window else 0, p // chunk * chunk if chunk else 0, 0)
+        line = cache[bt[slot[m]].long()].transpose(1, 2).reshape(-1, kv, 2 * dim)[lo:p + 1].double().repeat_interleave(heads // kv, dim=1)
+        s = torch.einsum("hd,thd->ht", q[m].bfloat16().double().view(heads, dim), line[..., :dim]) * 0.2
+        if softcap:
+            s = softcap * (s / softcap).tanh()
+        if extra:
+            s = torch.cat([s - slope.double()[:, None] * (p - torch.arange(lo, p + 1))[None], sink.double()[:, None]], dim=1)
+        want = torch.einsum("ht,thd->hd", s.softmax(dim=1)[:, :p + 1 - lo], line[..., dim:])
+        if extra:
+            want = want * gate[m].double().sigmoid()[:, None]
+        assert (got[m] - want).norm() <= 8e-3 * want.norm(), (m, p)
