@@ -155,6 +155,48 @@ template <bool LINES> DL_DEVINL float pt_probs(const uint32_t (&v)[32], float sc
     return sum;
 }
 
+// One thread's 32 consecutive outputs of row m (a Q80 block) into the slabs of the next matmul: the block's maximum is in the thread's own
+// registers.  (A warp per block, lane = element, took a five-step shuffle reduction for each of a warp's 64 blocks, one behind the other:
+// 25 k clk of a CTA that multiplies for 31 k; 4096 rows of 32 heads took 331 us, 210 now; into f32
+// rows, which take the same path without the cast, 4001 rows 266 -> 229.)
+DL_DEVINL void pt_q80_block(const float (&v)[32], int m, int kblock, int mcap, uint8_t* xq, uint8_t* xh) {
+    float amax = 0.f;
+#pragma unroll
+    for (int e = 0; e < 32; e++) amax = fmaxf(amax, fabsf(v[e]));
+    const float d = amax / 127.0f;
+    const float id = (d != 0.0f) ? (1.0f / d) : 0.0f;
+    const float df = __half2float(__float2half_rn(d));
+    const int kt = kblock >> 2, kb = kblock & 3;
+    int q[32];
+#pragma unroll
+    for (int e = 0; e < 32; e++) q[e] = __float2int_rn(v[e] * id);
+    if (xq != nullptr) {
+        uint8_t* row = xq + ((size_t)kt * mcap + m) * XQ_ROW_BYTES;
+        int sumq = 0;
+#pragma unroll
+        for (int e = 0; e < 32; e += 4) {
+            sumq += q[e] + q[e + 1] + q[e + 2] + q[e + 3];
+            *reinterpret_cast<uint32_t*>(row + kb * 32 + e) =
+                (uint32_t)(q[e] & 0xff) | ((uint32_t)(q[e + 1] & 0xff) << 8) | ((uint32_t)(q[e + 2] & 0xff) << 16) | ((uint32_t)(q[e + 3] & 0xff) << 24);
+        }
+        reinterpret_cast<float*>(row + 128)[kb] = df;
+        reinterpret_cast<int*>(row + 144)[kb] = 8 * sumq;
+    }
+    if (xh != nullptr) {
+        const float dfh = fminf(df, 515.0f);       // fp16 operand: saturate (|x| > 65405) instead of producing inf
+        uint8_t* base = xh + ((size_t)kt * (size_t)(mcap >> 3) + (size_t)(m >> 3)) * XH_ROWGROUP_BYTES + (size_t)(kb * 4) * 128 + (size_t)(m & 7) * 16;
+#pragma unroll
+        for (int w = 0; w < 4; w++) {              // chunk w: elements 4w, 4w+2, 4w+1, 4w+3, then the same + 16 (see xh_slot)
+            uint4 u;
+            u.x = pt_pack2<false>((float)q[4 * w] * dfh, (float)q[4 * w + 2] * dfh);
+            u.y = pt_pack2<false>((float)q[4 * w + 1] * dfh, (float)q[4 * w + 3] * dfh);
+            u.z = pt_pack2<false>((float)q[4 * w + 16] * dfh, (float)q[4 * w + 18] * dfh);
+            u.w = pt_pack2<false>((float)q[4 * w + 17] * dfh, (float)q[4 * w + 19] * dfh);
+            *reinterpret_cast<uint4*>(base + w * 128) = u;
+        }
+    }
+}
+
 template <bool LINES>
 __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(const __grid_constant__ typename PtKernelArgs<LINES>::T a,
                                                                              const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap) {
@@ -488,29 +530,36 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
         } else {
             inv = l > 0.0f ? 1.0f / l : 0.0f;
         }
+        bool rows_out = true;                                    // f32 rows wanted: through shared memory, lanes along a row
+        if constexpr (!LINES) rows_out = a.y_out != nullptr;
 #pragma unroll 1
         for (int ch = 0; ch < 2; ch++) {
             tmem_ld_32x32b_x32(T_O + lane_base + hf * 64 + ch * 32, v0);
             tmem_ld_wait();
+            float v[32];
 #pragma unroll
-            for (int e = 0; e < 32; e++) out_s[row * PT_OUT_LD + hf * 64 + ch * 32 + e] = __uint_as_float(v0[e]) * inv;
-        }
-        __syncwarp();                                            // a warp only re-reads the 32 rows x 64 columns it wrote
-        for (int rr = 0; rr < 32; rr++) {
-            const int rc = r_first + quarter * 32 + rr;
-            if (rc >= n_rows) break;
-            if constexpr (LINES) {
-                float* dst = a.w.out + (size_t)__shfl_sync(0xffffffffu, m_row, rr) * a.w.ldo + __shfl_sync(0xffffffffu, h_row, rr) * PT_HS + hf * 64 + lane;
-                dst[0] = out_s[(quarter * 32 + rr) * PT_OUT_LD + hf * 64 + lane];
-                dst[32] = out_s[(quarter * 32 + rr) * PT_OUT_LD + hf * 64 + 32 + lane];
-            } else {
-            const int m = begin + rc;
-#pragma unroll
-            for (int b = 0; b < 2; b++) {
-                const float val = out_s[(quarter * 32 + rr) * PT_OUT_LD + hf * 64 + b * 32 + lane];
-                q80_block_store(val, lane, m, (head * PT_HS) / 32 + hf * 2 + b, a.out_mcap, a.xq_out, a.xh_out);
-                if (a.y_out != nullptr) a.y_out[(size_t)m * a.n_heads * PT_HS + head * PT_HS + hf * 64 + b * 32 + lane] = val;
+            for (int e = 0; e < 32; e++) v[e] = __uint_as_float(v0[e]) * inv;
+            if constexpr (!LINES) {
+                if (r_abs < n_rows && (a.xq_out != nullptr || a.xh_out != nullptr))
+                    pt_q80_block(v, begin + r_abs, (head * PT_HS) / 32 + hf * 2 + ch, a.out_mcap, a.xq_out, a.xh_out);
             }
+            if (rows_out) {
+#pragma unroll
+                for (int e = 0; e < 32; e++) out_s[row * PT_OUT_LD + hf * 64 + ch * 32 + e] = v[e];
+            }
+        }
+        if (rows_out) {
+            __syncwarp();                                        // a warp only re-reads the 32 rows x 64 columns it wrote
+#pragma unroll 4
+            for (int rr = 0; rr < 32; rr++) {
+                const int rc = r_first + quarter * 32 + rr;
+                if (rc >= n_rows) break;
+                float* dst;
+                if constexpr (LINES) dst = a.w.out + (size_t)__shfl_sync(0xffffffffu, m_row, rr) * a.w.ldo + __shfl_sync(0xffffffffu, h_row, rr) * PT_HS;
+                else dst = a.y_out + (size_t)(begin + rc) * a.n_heads * PT_HS + head * PT_HS;
+                const float* src = out_s + (quarter * 32 + rr) * PT_OUT_LD + hf * 64 + lane;
+                dst[hf * 64 + lane] = src[0];
+                dst[hf * 64 + 32 + lane] = src[32];
             }
         }
     } else if (warp == 5 || warp == 7) {
