@@ -103,17 +103,22 @@ __global__ void __launch_bounds__(GV_WARPS * 32) dense_gemv_kernel(DlDenseArgs a
     }
 }
 
-// vectorised variant: K % 8 == 0, rows 16-byte aligned (checked on the host)
+// Vectorised variant: K % 8 == 0, rows 16-byte aligned (checked on the host).  One warp per output column (PAIR: per gated unit, its gate
+// row and its up row), 8 weights per lane and load, a batch of U loads in flight while the last one is multiplied.
+// What bounds it: the weights' bytes, which takes many loads in flight and few instructions per weight -- so the CTA's eight warps share
+// the activations in shared memory, rounded once (each warp loaded, and rounded, all of them for itself: 8192 inputs x 2048 columns
+// took 15.2 us, 2.2 TB/s; 10.2 us now, 3.3 TB/s) -- and the latency of a chain of small kernels: programmatic launch, with the start of
+// every weight row on its way into L2 before the previous kernel is waited for.  A lane's products are added in the old order.
 template <typename WT> struct WVec;
 template <> struct WVec<float> {
-    static __device__ __forceinline__ void load8(const float* p, float* o) {
-        const float4 u = *reinterpret_cast<const float4*>(p), v = *reinterpret_cast<const float4*>(p + 4);
-        o[0] = u.x; o[1] = u.y; o[2] = u.z; o[3] = u.w; o[4] = v.x; o[5] = v.y; o[6] = v.z; o[7] = v.w;
-    }
+    float4 u, v;
+    __device__ __forceinline__ void load(const float* p) { u = *reinterpret_cast<const float4*>(p); v = *reinterpret_cast<const float4*>(p + 4); }
+    __device__ __forceinline__ void get(float* o) const { o[0] = u.x; o[1] = u.y; o[2] = u.z; o[3] = u.w; o[4] = v.x; o[5] = v.y; o[6] = v.z; o[7] = v.w; }
 };
 template <> struct WVec<__nv_bfloat16> {
-    static __device__ __forceinline__ void load8(const __nv_bfloat16* p, float* o) {
-        const uint4 u = *reinterpret_cast<const uint4*>(p);
+    uint4 u;
+    __device__ __forceinline__ void load(const __nv_bfloat16* p) { u = *reinterpret_cast<const uint4*>(p); }
+    __device__ __forceinline__ void get(float* o) const {
         const uint32_t r[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -123,43 +128,253 @@ template <> struct WVec<__nv_bfloat16> {
     }
 };
 
-template <typename WT, int MT, bool RX>
+template <typename WT, int MT, bool RX, bool PAIR>
 __global__ void __launch_bounds__(GV_WARPS * 32) dense_gemv_vec_kernel(DlDenseArgs a) {
+    constexpr int XC = 8192 / MT;                                            // inputs staged at a time, per row
+    constexpr int U = (sizeof(WT) == 2 ? (MT == 8 ? 4 : 8) : 4) / (PAIR ? 2 : 1);
+    static_assert(XC % (256 * U) == 0, "batches end with the staged inputs");
+    __shared__ __align__(16) float xs[MT * XC];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n = blockIdx.x * GV_WARPS + warp;
     const int b = blockIdx.z;
-    if (n >= a.N) return;
-    const WT* w = (const WT*)a.W + (size_t)b * a.w_bs + (size_t)n * a.ldw;
+    const bool on = PAIR ? 2 * n + 1 < a.N : n < a.N;
+    const WT* w0 = (const WT*)a.W + (size_t)b * a.w_bs + (size_t)(PAIR ? 2 * n : n) * a.ldw;
+    const WT* w1 = w0 + a.ldw;
     const float* x = a.X + (size_t)b * a.x_bs;
-    float acc[MT];
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (on && lane < (PAIR ? 2 : 1)) {
+        const uint32_t bytes = min((uint32_t)(a.K * sizeof(WT)), 4096u);     // a multiple of 16: K % 8 == 0
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(lane ? w1 : w0), "r"(bytes) : "memory");
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    float g[MT], h[MT];
 #pragma unroll
-    for (int m = 0; m < MT; ++m) acc[m] = 0.f;
-    for (int k = lane * 8; k < a.K; k += 256) {
-        float wv[8];
-        WVec<WT>::load8(w + k, wv);
+    for (int m = 0; m < MT; ++m) g[m] = h[m] = 0.f;
+    WVec<WT> cur[PAIR ? 2 : 1][U], nxt[PAIR ? 2 : 1][U];
+    auto fetch = [&](WVec<WT> (&v)[PAIR ? 2 : 1][U], int k0) {
 #pragma unroll
-        for (int m = 0; m < MT; ++m) {
-            if (m < a.M) {
-                float xv[8];
-                WVec<float>::load8(x + (size_t)m * a.ldx + k, xv);
+        for (int u = 0; u < U; ++u) {
+            const int k = k0 + u * 256 + lane * 8;
+            if (on && k < a.K) {
+                v[0][u].load(w0 + k);
+                if (PAIR) v[PAIR ? 1 : 0][u].load(w1 + k);
+            }
+        }
+    };
+    fetch(cur, 0);
+    for (int c0 = 0; c0 < a.K; c0 += XC) {
+        const int kc = min(XC, a.K - c0);
+        if (c0) __syncthreads();
 #pragma unroll
-                for (int i = 0; i < 8; ++i) acc[m] = fmaf(RX ? round_bf16(xv[i]) : xv[i], wv[i], acc[m]);
+        for (int m = 0; m < MT; ++m)
+            if (m < a.M)
+                for (int i = threadIdx.x * 4; i < kc; i += GV_WARPS * 128) {
+                    float4 v = *reinterpret_cast<const float4*>(x + (size_t)m * a.ldx + c0 + i);
+                    if (RX) { v.x = round_bf16(v.x); v.y = round_bf16(v.y); v.z = round_bf16(v.z); v.w = round_bf16(v.w); }
+                    // a block of 256 inputs as the first and the second four of every lane's eight: 16-byte reads without bank conflicts
+                    *reinterpret_cast<float4*>(xs + m * XC + (i & ~255) + (i & 4) * 32 + ((i & 255) >> 3) * 4) = v;
+                }
+        __syncthreads();
+        for (int k0 = 0; k0 < kc; k0 += 256 * U) {
+            fetch(nxt, c0 + k0 + 256 * U);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int k = k0 + u * 256 + lane * 8;
+                if (k < kc) {
+                    float wg[8], wu[8];
+                    cur[0][u].get(wg);
+                    if (PAIR) cur[PAIR ? 1 : 0][u].get(wu);
+#pragma unroll
+                    for (int m = 0; m < MT; ++m) {
+                        if (m < a.M) {
+                            const float4 p = *reinterpret_cast<const float4*>(xs + m * XC + k0 + u * 256 + lane * 4), q = *reinterpret_cast<const float4*>(xs + m * XC + k0 + u * 256 + 128 + lane * 4);
+                            const float xv[8] = {p.x, p.y, p.z, p.w, q.x, q.y, q.z, q.w};
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) {
+                                g[m] = fmaf(xv[i], wg[i], g[m]);
+                                if (PAIR) h[m] = fmaf(xv[i], wu[i], h[m]);
+                            }
+                        }
+                    }
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                cur[0][u] = nxt[0][u];
+                if (PAIR) cur[PAIR ? 1 : 0][u] = nxt[PAIR ? 1 : 0][u];
             }
         }
     }
+    if (!on) return;
 #pragma unroll
-    for (int m = 0; m < MT; ++m) acc[m] = warp_sum(acc[m]);
+    for (int m = 0; m < MT; ++m) {
+        g[m] = warp_sum(g[m]);
+        if (PAIR) h[m] = warp_sum(h[m]);
+    }
     if (lane == 0) {
 #pragma unroll
         for (int m = 0; m < MT; ++m) {
-            if (m < a.M) dense_store(a, b, m, n, acc[m]);
+            if (m < a.M) {
+                if (PAIR) dense_store_pair(a, b, m, n, g[m], h[m]);
+                else dense_store(a, b, m, n, g[m]);
+            }
         }
     }
 }
 
+// ------------------------------------------------------------------------------------------------
+// 3 to 32 rows, bf16 weights, activations rounded to bf16 (K % 8 == 0, aligned rows): mma.sync with the weights as the 16-row operand, so
+// the products of 8 activation rows cost one instruction per 16 x 16 weights.
+//
+// What bounds it: the weights' bytes.  On CUDA cores every row adds 8 FMAs per 16 bytes of weights and lane, and from 9 rows the tiles
+// below (16 K steps of scalar loads) left the weights behind entirely: gate|up + down of 4096 x 14336 took 441 us at 8 rows and
+// 3150 us at 16; 118 and 153 us here.  (Two rows are faster one by one: 2048 x 8192, 39.5 us there, 43.3 here.)
+//
+// Weights go from global memory straight into the A fragments: a lane's 16 bytes are 8 consecutive inputs of row g, and the four pairs
+// fill k slots of two MMAs; the activations' 16 bytes of the same inputs fill the same slots, so no shuffle and no shared memory for the
+// weights.  A CTA owns 16 C columns; its eight warps split K, each staging its own activations (bf16, 128 inputs at a time), and meet in
+// shared memory at the end, summed in warp order.  An MMA chain truncates, so it is 4 steps long and ends in a rounded f32 add.
+// ------------------------------------------------------------------------------------------------
+#define DM_STEP 128                    // inputs staged at a time by a warp
+#define DM_LD (DM_STEP + 8)            // row stride of the staged activations (bf16): 16-byte reads of 8 rows without conflicts
+
+__device__ __forceinline__ void dense_mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+template <int NT, int C>               // 8 NT rows, 16 C columns per CTA
+__global__ void __launch_bounds__(256) dense_mma_kernel(DlDenseArgs a) {
+    extern __shared__ __align__(16) uint8_t dm_smem[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int b = blockIdx.z, n0 = blockIdx.x * 16 * C;
+    const __nv_bfloat16* W = (const __nv_bfloat16*)a.W + (size_t)b * a.w_bs;
+    const float* X = a.X + (size_t)b * a.x_bs;
+    __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(dm_smem) + (size_t)warp * NT * 8 * DM_LD;
+    // this warp's inputs: whole steps of DM_STEP, contiguous
+    const int steps = (a.K + DM_STEP - 1) / DM_STEP;
+    const int s0 = steps * warp / 8, s1 = steps * (warp + 1) / 8;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (s1 > s0 && lane < 16) {          // the start of this warp's weights is on its way into L2 while the previous kernel ends
+        const uint32_t bytes = min((uint32_t)(min(a.K, s1 * DM_STEP) - s0 * DM_STEP) * 2u, 2048u);
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+            if (n0 + c * 16 + lane < a.N)
+                asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(W + (size_t)(n0 + c * 16 + lane) * a.ldw + s0 * DM_STEP), "r"(bytes) : "memory");
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    float acc[C][NT][4];
+#pragma unroll
+    for (int c = 0; c < C; ++c)
+#pragma unroll
+        for (int n = 0; n < NT; ++n) acc[c][n][0] = acc[c][n][1] = acc[c][n][2] = acc[c][n][3] = 0.f;
+    const uint4 zero = make_uint4(0, 0, 0, 0);
+    // a lane's weights of half a step: [two 32-input pieces][C][rows g and g + 8]
+    auto fetch = [&](uint4 (&w)[2][C][2], int k0) {
+#pragma unroll
+        for (int p = 0; p < 2; ++p)
+#pragma unroll
+            for (int c = 0; c < C; ++c)
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const int k = k0 + p * 32 + t * 8, n = n0 + c * 16 + u * 8 + g;
+                    w[p][c][u] = k < a.K && n < a.N ? *reinterpret_cast<const uint4*>(W + (size_t)n * a.ldw + k) : zero;
+                }
+    };
+    uint4 cur[2][C][2], nxt[2][C][2];
+    if (s1 > s0) fetch(cur, s0 * DM_STEP);
+    for (int s = s0; s < s1; ++s) {
+        const int k0 = s * DM_STEP;
+        __syncwarp();
+#pragma unroll 4
+        for (int m = 0; m < NT * 8; ++m) {          // a row's 128 inputs by the whole warp
+            const int k = k0 + lane * 4;
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (m < a.M && k < a.K) v = *reinterpret_cast<const float4*>(X + (size_t)m * a.ldx + k);
+            __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+            *reinterpret_cast<uint2*>(xs + m * DM_LD + lane * 4) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+        }
+        __syncwarp();
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {                // halves of 64 inputs: four MMAs to a chain
+            if (h == 0 || s + 1 < s1) fetch(nxt, k0 + (h + 1) * 64);
+            uint4 x[2][NT];
+#pragma unroll
+            for (int p = 0; p < 2; ++p)
+#pragma unroll
+                for (int n = 0; n < NT; ++n) x[p][n] = *reinterpret_cast<const uint4*>(xs + (n * 8 + g) * DM_LD + h * 64 + p * 32 + t * 8);
+#pragma unroll
+            for (int c = 0; c < C; ++c)
+#pragma unroll
+                for (int n = 0; n < NT; ++n) {
+                    float d[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                    for (int p = 0; p < 2; ++p) {
+                        dense_mma_bf16(d, cur[p][c][0].x, cur[p][c][1].x, cur[p][c][0].y, cur[p][c][1].y, x[p][n].x, x[p][n].y);
+                        dense_mma_bf16(d, cur[p][c][0].z, cur[p][c][1].z, cur[p][c][0].w, cur[p][c][1].w, x[p][n].z, x[p][n].w);
+                    }
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) acc[c][n][e] += d[e];
+                }
+#pragma unroll
+            for (int p = 0; p < 2; ++p)
+#pragma unroll
+                for (int c = 0; c < C; ++c) { cur[p][c][0] = nxt[p][c][0]; cur[p][c][1] = nxt[p][c][1]; }
+        }
+    }
+    // [warp][row m][16 C columns], in the activations' place
+    __syncthreads();
+    float* red = reinterpret_cast<float*>(dm_smem);
+    constexpr int COLS = 16 * C, PER = NT * 8 * COLS;
+#pragma unroll
+    for (int c = 0; c < C; ++c)
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) red[warp * PER + (n * 8 + t * 2 + (e & 1)) * COLS + c * 16 + (e >> 1) * 8 + g] = acc[c][n][e];
+    __syncthreads();
+    const bool pair = a.epi == DL_DENSE_GLU_GELU;
+    for (int i = threadIdx.x * 2; i < a.M * COLS; i += 512) {          // two neighbouring columns of a row
+        const int m = i / COLS, n = n0 + (i - m * COLS);
+        float2 v = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int w = 0; w < 8; ++w) {
+            const float2 p = *reinterpret_cast<const float2*>(red + w * PER + i);
+            v.x += p.x;
+            v.y += p.y;
+        }
+        if (pair) {
+            if (n + 1 < a.N) dense_store_pair(a, b, m, n >> 1, v.x, v.y);
+        } else {
+            if (n < a.N) dense_store(a, b, m, n, v.x);
+            if (n + 1 < a.N) dense_store(a, b, m, n + 1, v.y);
+        }
+    }
+}
+
+template <int NT, int C>
+static void launch_dense_mma_t(const DlDenseArgs& a, cudaStream_t st) {
+    constexpr int smem = NT * 8 * 8 * (DM_LD * 2 > 16 * C * 4 ? DM_LD * 2 : 16 * C * 4);
+    static bool set = false;
+    if (!set && smem > 48 * 1024) {
+        cudaFuncSetAttribute(dense_mma_kernel<NT, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        set = true;
+    }
+    launch_after(dense_mma_kernel<NT, C>, dim3((a.N + 16 * C - 1) / (16 * C), 1, a.batch), 256, st, a, smem);
+}
+// columns per CTA: as many as leave the chip a CTA per SM (they share the staged activations)
+template <int NT>
+static void launch_dense_mma(const DlDenseArgs& a, cudaStream_t st, int n_sms) {
+    const long long groups = (long long)(a.N + 15) / 16 * a.batch;
+    if (NT <= 2 && groups >= 4ll * n_sms) launch_dense_mma_t<NT <= 2 ? NT : 1, 4>(a, st);      // (4 x 4 accumulator tiles do not fit the registers)
+    else if (groups >= 2ll * n_sms) launch_dense_mma_t<NT, 2>(a, st);
+    else launch_dense_mma_t<NT, 1>(a, st);
+}
+
 // paired columns (GLU): one warp per value, its gate row and its up row side by side
 template <typename WT, int MT, bool RX>
-__global__ void __launch_bounds__(GV_WARPS * 32) dense_gemv_pair_kernel(DlDenseArgs a, int vec) {
+__global__ void __launch_bounds__(GV_WARPS * 32) dense_gemv_pair_kernel(DlDenseArgs a) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int j = blockIdx.x * GV_WARPS + warp;
     const int b = blockIdx.z;
@@ -170,37 +385,15 @@ __global__ void __launch_bounds__(GV_WARPS * 32) dense_gemv_pair_kernel(DlDenseA
     float g[MT], u[MT];
 #pragma unroll
     for (int m = 0; m < MT; ++m) g[m] = u[m] = 0.f;
-    if (vec) {
-#pragma unroll 2
-        for (int k = lane * 8; k < a.K; k += 256) {
-            float wg[8], wu[8];
-            WVec<WT>::load8(w0 + k, wg);
-            WVec<WT>::load8(w1 + k, wu);
+    for (int k = lane; k < a.K; k += 32) {
+        const float wg = ld_f(w0 + k), wu = ld_f(w1 + k);
 #pragma unroll
-            for (int m = 0; m < MT; ++m) {
-                if (m < a.M) {
-                    float xv[8];
-                    WVec<float>::load8(x + (size_t)m * a.ldx + k, xv);
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        const float v = RX ? round_bf16(xv[i]) : xv[i];
-                        g[m] = fmaf(v, wg[i], g[m]);
-                        u[m] = fmaf(v, wu[i], u[m]);
-                    }
-                }
-            }
-        }
-    } else {
-        for (int k = lane; k < a.K; k += 32) {
-            const float wg = ld_f(w0 + k), wu = ld_f(w1 + k);
-#pragma unroll
-            for (int m = 0; m < MT; ++m) {
-                if (m < a.M) {
-                    float v = x[(size_t)m * a.ldx + k];
-                    if (RX) v = round_bf16(v);
-                    g[m] = fmaf(v, wg, g[m]);
-                    u[m] = fmaf(v, wu, u[m]);
-                }
+        for (int m = 0; m < MT; ++m) {
+            if (m < a.M) {
+                float v = x[(size_t)m * a.ldx + k];
+                if (RX) v = round_bf16(v);
+                g[m] = fmaf(v, wg, g[m]);
+                u[m] = fmaf(v, wu, u[m]);
             }
         }
     }
@@ -283,20 +476,41 @@ __global__ void __launch_bounds__(256) dense_tile_kernel(DlDenseArgs a) {
 
 template <typename WT, bool RX>
 static void launch_dense(const DlDenseArgs& a, cudaStream_t st) {
+    const bool vec = a.K % 8 == 0 && a.ldw % 8 == 0 && a.w_bs % 8 == 0 && a.ldx % 4 == 0 && a.x_bs % 4 == 0 &&
+                     ((uintptr_t)a.W & 15) == 0 && ((uintptr_t)a.X & 15) == 0;
+    if constexpr (sizeof(WT) == 2 && RX) {
+        if (vec && a.M >= 3 && a.M <= 32) {
+            const int n_sms = dl_device_sm_count();
+            if (a.M <= 8) launch_dense_mma<1>(a, st, n_sms);
+            else if (a.M <= 16) launch_dense_mma<2>(a, st, n_sms);
+            else launch_dense_mma<4>(a, st, n_sms);
+            return;
+        }
+    }
     if (a.M <= 8) {
-        const bool vec = a.K % 8 == 0 && a.ldw % 8 == 0 && a.w_bs % 8 == 0 && a.ldx % 4 == 0 && a.x_bs % 4 == 0 &&
-                         ((uintptr_t)a.W & 15) == 0 && ((uintptr_t)a.X & 15) == 0;
         const bool pair = a.epi == DL_DENSE_GLU_GELU;
         dim3 grid(((pair ? a.N / 2 : a.N) + GV_WARPS - 1) / GV_WARPS, 1, a.batch);
         const int mt = a.M <= 1 ? 1 : a.M <= 2 ? 2 : a.M <= 4 ? 4 : 8;
 #define GV_CASE(MT_)                                                                                   \
     case MT_:                                                                                          \
-        if (pair) dense_gemv_pair_kernel<WT, MT_, RX><<<grid, GV_WARPS * 32, 0, st>>>(a, vec ? 1 : 0);  \
-        else if (vec) dense_gemv_vec_kernel<WT, MT_, RX><<<grid, GV_WARPS * 32, 0, st>>>(a);                \
+        if (vec && pair) launch_after(dense_gemv_vec_kernel<WT, MT_, RX, true>, grid, GV_WARPS * 32, st, a);        \
+        else if (vec) launch_after(dense_gemv_vec_kernel<WT, MT_, RX, false>, grid, GV_WARPS * 32, st, a);          \
+        else if (pair) dense_gemv_pair_kernel<WT, MT_, RX><<<grid, GV_WARPS * 32, 0, st>>>(a);                      \
         else dense_gemv_kernel<WT, MT_, RX><<<grid, GV_WARPS * 32, 0, st>>>(a);                        \
         break;
         switch (mt) { GV_CASE(1) GV_CASE(2) GV_CASE(4) GV_CASE(8) }
 #undef GV_CASE
+    } else if (vec && a.M <= 32) {
+        // up to four rounds of 8 rows: each streams the weights at their own pace, which the tiles below (a scalar load per weight, most of 64
+        // rows empty) do not (gate|up + down of 4096 x 14336 in f32 at 16 rows: 3460 us there, 630 here)
+        for (int m0 = 0; m0 < a.M; m0 += 8) {
+            DlDenseArgs r = a;
+            r.M = a.M - m0 < 8 ? a.M - m0 : 8;
+            r.X += (size_t)m0 * a.ldx;
+            r.Y += (size_t)m0 * a.ldy;
+            if (a.aux) r.aux += (size_t)m0 * a.ld_aux;
+            launch_dense<WT, RX>(r, st);
+        }
     } else {
         dim3 grid((a.N + GT_BN - 1) / GT_BN, (a.M + GT_BM - 1) / GT_BM, a.batch);
         dense_tile_kernel<WT, RX><<<grid, 256, 0, st>>>(a);

@@ -445,7 +445,10 @@ __global__ void __launch_bounds__(WS_THREADS, 1) gemm_wh_rows_kernel(const __gri
                 dst = b_off + g * 2048;
             }
         }
-        if (!is_w && bytes) pdl_wait();                          // weights do not depend on the previous kernel
+        // the weights' first stages are on their way into L2 while the previous kernel ends (a hint: a kernel that still writes them is waited for)
+        for (int i = 0; is_w && i < min(nk, a.NS); i++)
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src + (size_t)i * step), "r"(bytes) : "memory");
+        pdl_wait();
         for (int i = 0; i < nk; i++) {
             const int s = i % a.NS;
             if (i >= a.NS) wt_wait(&empty[s], ((i / a.NS) & 1) ^ 1, t0);
@@ -533,7 +536,7 @@ __global__ void __launch_bounds__(WS_THREADS, 1) gemm_wh_rows_kernel(const __gri
 static int ws_split(int R8, int KT, int n_sms) { return R8 < 5 * n_sms && KT >= 2 ? 2 : 1; }
 
 static int gemm_wh_rows_launch(const uint8_t* wh, int d, int n, const uint8_t* xh, int ncap, int M, const DlEpilogue* epi, int bf16,
-                               int pdl, cudaStream_t stream, int n_sms) {
+                               cudaStream_t stream, int n_sms) {
     WsArgs a;
     a.wh = wh; a.xh = xh; a.d_real = d; a.R8 = (d + 7) / 8; a.KT = n / 128; a.ncap = ncap; a.M = M;
     a.NT = (M + 15) / 16 * 16;
@@ -573,11 +576,9 @@ static int gemm_wh_rows_launch(const uint8_t* wh, int d, int n, const uint8_t* x
         attrs[na].val.clusterDim.z = 1;
         na++;
     }
-    if (pdl) {
-        attrs[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attrs[na].val.programmaticStreamSerializationAllowed = 1;
-        na++;
-    }
+    attrs[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // it waits by itself before it reads what others wrote
+    attrs[na].val.programmaticStreamSerializationAllowed = 1;
+    na++;
     cfg.attrs = attrs;
     cfg.numAttrs = na;
     cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_wh_rows_kernel, a);
@@ -610,7 +611,7 @@ static int gemm_wh_launch(const uint8_t* wh, int d, int n, const uint8_t* xh, in
     if (epi->kind == DL_EPI_SILU_MUL && d % 64 != 0) { dl_set_error("dl_gemm_wh_tc: silu epilogue needs d%%64==0"); return -1; }
     // few rows: all SMs stream equal shares of the weights (force_cg bit 0 keeps the tiles below, for comparisons)
     if (epi->kind == DL_EPI_DENSE && grp == nullptr && M <= WS_MAX_NT && !(force_cg & 1))
-        return gemm_wh_rows_launch(wh, d, n, xh, ncap, M, epi, (force_cg & 2) ? 1 : 0, pdl, (cudaStream_t)stream, dl_device_sm_count());
+        return gemm_wh_rows_launch(wh, d, n, xh, ncap, M, epi, (force_cg & 2) ? 1 : 0, (cudaStream_t)stream, dl_device_sm_count());
     WhArgs a;
     a.wh = wh; a.xh = xh; a.d_real = d;
     a.row_tiles = (d + 127) / 128;

@@ -23,6 +23,23 @@ extern void dl_set_error(const char* fmt, ...);
         }                                                                               \
     } while (0)
 
+// Programmatic launch: the kernel may start while the one ahead of it in the stream still runs.  It must call griddepcontrol.wait before it
+// touches anything that an earlier kernel writes or reads; its own dependents start no earlier than it says launch_dependents.
+template <typename A>
+static inline void launch_after(void (*kernel)(A), dim3 grid, int threads, cudaStream_t st, const A& args, size_t smem = 0) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, args);          // an error is the caller's next cudaGetLastError
+}
+
 template <typename T> __device__ __forceinline__ float ld_f(const T* p);
 template <> __device__ __forceinline__ float ld_f<float>(const float* p) { return *p; }
 template <> __device__ __forceinline__ float ld_f<__nv_bfloat16>(const __nv_bfloat16* p) { return __bfloat162float(*p); }

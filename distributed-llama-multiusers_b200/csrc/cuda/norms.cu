@@ -220,6 +220,8 @@ __device__ __forceinline__ void rs_put(float* h, uint8_t* xh, int ncap, int m, l
 
 template <int NG>
 __global__ void __launch_bounds__(RS_THREADS) residual_step_vec_kernel(DlResidualArgs a) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     __shared__ float red[2 * (RS_THREADS / 32)];
     const int m = blockIdx.x, dim = a.dim, n4 = dim >> 2, tid = threadIdx.x;
     const size_t src = a.rows ? a.rows[m] : m;
@@ -339,10 +341,10 @@ extern "C" int dl_residual_step(const DlResidualArgs* args, void* stream) {
                      al(a.w1, 0) && al(a.w2, 0) && al(a.b1, 0) && al(a.b2, 0) && al(a.h1, a.ldh) && al(a.h2, a.ldh);
     if (vec) {
         cudaStream_t st = (cudaStream_t)stream;
-        if (a.dim <= 4 * RS_THREADS) residual_step_vec_kernel<1><<<a.M, RS_THREADS, 0, st>>>(a);
-        else if (a.dim <= 8 * RS_THREADS) residual_step_vec_kernel<2><<<a.M, RS_THREADS, 0, st>>>(a);
-        else if (a.dim <= 16 * RS_THREADS) residual_step_vec_kernel<4><<<a.M, RS_THREADS, 0, st>>>(a);
-        else residual_step_vec_kernel<8><<<a.M, RS_THREADS, 0, st>>>(a);
+        if (a.dim <= 4 * RS_THREADS) launch_after(residual_step_vec_kernel<1>, dim3(a.M), RS_THREADS, st, a);
+        else if (a.dim <= 8 * RS_THREADS) launch_after(residual_step_vec_kernel<2>, dim3(a.M), RS_THREADS, st, a);
+        else if (a.dim <= 16 * RS_THREADS) launch_after(residual_step_vec_kernel<4>, dim3(a.M), RS_THREADS, st, a);
+        else launch_after(residual_step_vec_kernel<8>, dim3(a.M), RS_THREADS, st, a);
         LAYER_CHECK_LAUNCH("dl_residual_step");
         return 0;
     }

@@ -240,3 +240,25 @@ def test_window_prompt_tiles(window, chunk, softcap, extra):
         if extra:
             want = want * gate[m].double().sigmoid()[:, None]
         assert (got[m] - want).norm() <= 8e-3 * want.norm(), (m, p)
+
+
+@pytest.mark.parametrize("M,N,K_,dtype,round_x", [(1, 24, 8, "bf16", True), (2, 40, 136, "bf16", True), (8, 1000, 264, "bf16", True), (9, 5008, 128, "bf16", True),
+                                                  (16, 10000, 392, "bf16", True), (17, 48, 1160, "bf16", True), (32, 2064, 256, "bf16", True), (1, 9, 8200, "f32", False),
+                                                  (4, 64, 2056, "f32", False), (8, 24, 1032, "bf16", False), (31, 33, 72, "f32", False)])
+def test_dense_few_rows(M, N, K_, dtype, round_x):
+    """Few-row products straight from the weight rows: one row, the MMA form's row and column tiles and their remainders, K that ends inside
+    a staged step and inside a batch of loads, both weight types, paired columns and an output gate.  f32 sums of K terms: 3e-6."""
+    g = torch.Generator(device="cuda").manual_seed(M * 1000 + N)
+    w = (torch.randn(N, K_, generator=g, device="cuda") * K_ ** -0.5).to(torch.bfloat16 if dtype == "bf16" else torch.float32)
+    x, aux, bias = torch.randn(M, K_ + 4, generator=g, device="cuda")[:, :K_], torch.randn(M, N, generator=g, device="cuda"), torch.randn(N, generator=g, device="cuda")
+    z = (x.bfloat16() if round_x else x).double() @ w.double().t()
+    close = lambda y, want: (y.double() - want).norm() <= 3e-6 * want.norm() + 1e-12
+    y = torch.full((M + 1, N + 2), 5.0, device="cuda")
+    L().dense(w, x, y, M, round_x, bias=bias)
+    assert close(y[:M, :N], z + bias.double()) and (y[M] == 5).all() and (y[:, N:] == 5).all()
+    L().dense(w, x, y, M, round_x, epi=L().DENSE_SIGMOID_MUL, aux=aux)
+    assert close(y[:M, :N], aux.double() * z.sigmoid())
+    if N % 2 == 0:
+        half = torch.zeros(M, N // 2, device="cuda")
+        L().dense(w, x, half, M, round_x, epi=L().DENSE_GLU_GELU)
+        assert close(half, torch.nn.functional.gelu(z[:, 0::2], approximate="tanh") * z[:, 1::2])
