@@ -129,17 +129,20 @@ template <bool LINES> DL_DEVINL uint32_t pt_pack2(float lo, float hi) {
 }
 
 // exp2 on the FMA pipe (Cody-Waite split + degree-3 polynomial, relative error 8e-5 -- the result is rounded to fp16,
-// 5e-4, right after): the softmax is bound by the 16 MUFU results per clock and SM (128 x 128 exp2 per step = 1024 clk,
-// as long as the MMAs of the step), so every fourth element takes this path instead
-DL_DEVINL float pt_ex2_poly(float x) {
+// 5e-4, right after; LINES, whose other kernels form it in full: degree 5, 2e-7): the softmax is bound by the 16 MUFU results
+// per clock and SM (128 x 128 exp2 per step = 1024 clk, as long as the MMAs of the step), so every fourth element takes this
+// path instead
+template <bool LINES> DL_DEVINL float pt_ex2_poly(float x) {
     const float xc = fmaxf(x, -126.0f);
     const float t = xc + 12582912.0f;              // 1.5 * 2^23: round(x) lands in the low mantissa bits
     const float f = xc - (t - 12582912.0f);        // [-0.5, 0.5]
-    const float p = fmaf(fmaf(fmaf(0.0550886838f, f, 0.242604051f), f, 0.693276242f), f, 0.99992894f);
+    const float p = LINES ? fmaf(fmaf(fmaf(fmaf(fmaf(1.32764725e-3f, f, 9.67554096e-3f), f, 0.0555071309f), f, 0.240221202f), f, 0.693146944f), f, 1.00000012f)
+                          : fmaf(fmaf(fmaf(0.0550886838f, f, 0.242604051f), f, 0.693276242f), f, 0.99992894f);
     return __int_as_float(__float_as_int(p) + (__float_as_int(t) << 23));
 }
 
-// 32 scores (masked ones are -inf) -> exp2(s * sc - ref) as 16 packed fp16 pairs into TMEM; returns their sum
+// 32 scores (masked ones are -inf) -> exp2(s * sc - ref) as 16 packed fp16 (LINES: bf16) pairs into TMEM; returns their sum.  LINES: the
+// sum of the ROUNDED probabilities, so that a row's weights add up to one
 template <bool LINES> DL_DEVINL float pt_probs(const uint32_t (&v)[32], float sc, float ref, uint32_t taddr) {
     uint32_t pk[16];
     float sum = 0.0f;
@@ -147,9 +150,10 @@ template <bool LINES> DL_DEVINL float pt_probs(const uint32_t (&v)[32], float sc
     for (int e = 0; e < 32; e += 2) {
         const float pa = pt_ex2(fmaf(__uint_as_float(v[e]), sc, -ref));
         const float xb = fmaf(__uint_as_float(v[e + 1]), sc, -ref);
-        const float pb = (e & 2) ? pt_ex2_poly(xb) : pt_ex2(xb);
-        sum += pa + pb;
+        const float pb = (e & 2) ? pt_ex2_poly<LINES>(xb) : pt_ex2(xb);
         pk[e >> 1] = pt_pack2<LINES>(pa, pb);
+        if (LINES) sum += __uint_as_float(pk[e >> 1] << 16) + __uint_as_float(pk[e >> 1] & 0xffff0000u);
+        else sum += pa + pb;
     }
     tmem_st_32x32b_x16(taddr, pk);
     return sum;
@@ -480,7 +484,10 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
             mx = fmaxf(mx, mx_s[((j & 1) * 2 + (hf ^ 1)) * PT_ROWS + row]);
             if (tid == 32) PT_STAMP(4, j);
             mx *= sc;
-            const bool need = mx > m_used + 8.0f;
+            // the reference may lag the maximum by 2^8 where probabilities are fp16 (11 bits).  LINES has bf16 ones: with the maximum itself as the
+            // reference a row's largest probability is 1 and exact, otherwise its rounding (2^-9) is the largest share of the error (2000 tokens
+            // under a window of 256, against 64 bits: 2.30e-3 lagging, 2.17e-3 here, 2.15e-3 in the mma.sync kernel; 47.2 and 47.5 us)
+            const bool need = mx > m_used + (LINES ? 0.0f : 8.0f);
             if (__any_sync(0xffffffffu, need)) {
                 const float m_new = need ? mx : m_used;
                 const float alpha = need ? pt_ex2(m_used - m_new) : 1.0f;
