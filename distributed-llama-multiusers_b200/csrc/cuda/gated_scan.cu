@@ -230,9 +230,9 @@ extern "C" int dl_gated_scan(const DlMambaBatch* batch, int n_seq, const DlGated
 // Scratch: states [slots][H][D][V] | decay of the whole chunk [slots][H][D] (head form: entry 0 of D) | n sums [slots][H][D].
 // ------------------------------------------------------------------------------------------------
 // pass 1: a chunk's own sum of (decay to the chunk's end * k_j) v_j^T, and the decay of the whole chunk
-// RT x 4 NC elements of S per thread: tiles of 16 RT rows and 64 NC columns
+// RT x 4 NC elements of S per thread: tiles of 16 RT rows and 64 NC columns.  Two tokens of a key or value column lie side by side
 template <bool CH, int RT, int NC>
-__global__ void __launch_bounds__(GC_THREADS) gated_chunk_state_kernel(DlMambaBatch b, DlGatedArgs a, GatedScratch sc) {
+__global__ void __launch_bounds__(GC_THREADS, RT * NC <= 4 ? 4 : 2) gated_chunk_state_kernel(DlMambaBatch b, DlGatedArgs a, GatedScratch sc) {
     extern __shared__ __align__(16) float sm[];
     __shared__ int rows[GC];
     __shared__ float w_s[GC];
@@ -254,28 +254,49 @@ __global__ void __launch_bounds__(GC_THREADS) gated_chunk_state_kernel(DlMambaBa
         if (threadIdx.x == 0) sc.dec[((size_t)ci * H + h) * D] = expf((float)(g + l_s[0]));
     }
     if (!CH) __syncthreads();
-    if (CH) gated_stage_rows<false, false>(a, rows, len, h, hk, D8, D8, nullptr, ks, vt);
-    for (int j = warp; !CH && j < GC; j += GC_THREADS / 32) {
-        const size_t row = rows[j];
+    if (CH) gated_stage_rows<false, false, true>(a, rows, len, h, hk, D8, D8, nullptr, ks, vt);
+    for (int j = 2 * warp; !CH && j < GC; j += GC_THREADS / 16) {
+        const size_t row0 = rows[j], row1 = rows[j + 1];
 #pragma unroll 4
-        for (int d = lane; d < D8; d += 32) ks[j * D8 + d] = j < len && d < D ? w_s[j] * a.k[row * a.ldk + h * D + d] : 0.f;
+        for (int d = lane; d < D8; d += 32)
+            *reinterpret_cast<float2*>(ks + j * D8 + 2 * d) = make_float2(j < len && d < D ? w_s[j] * a.k[row0 * a.ldk + h * D + d] : 0.f,
+                                                                         j + 1 < len && d < D ? w_s[j + 1] * a.k[row1 * a.ldk + h * D + d] : 0.f);
     }
     __syncthreads();
     if (CH) {
-        for (int d = threadIdx.x; d < D; d += GC_THREADS) {
+        // the late and the early half of the rows by a thread each: the early one first forms the late rows' decay
+        for (int t = threadIdx.x; t < 2 * D; t += GC_THREADS) {
+            const int late = t < D, d = late ? t : t - D;
             float p = 1.f;
+            if (!late)
 #pragma unroll 8
-            for (int j = GC - 1; j >= 0; --j) {
-                ks[j * D8 + d] *= p;
-                p *= vt[j * D8 + d];
+                for (int j = GC - 2; j >= GC / 2; j -= 2) {
+                    const float2 f = *reinterpret_cast<const float2*>(vt + j * D8 + 2 * d);
+                    p *= f.y;
+                    p *= f.x;
+                }
+            const int top = late ? GC : GC / 2;
+#pragma unroll 8
+            for (int j = top - 2; j >= top - GC / 2; j -= 2) {
+                const float2 f = *reinterpret_cast<const float2*>(vt + j * D8 + 2 * d);
+                float2 k = *reinterpret_cast<const float2*>(ks + j * D8 + 2 * d);
+                k.y *= p;
+                p *= f.y;
+                k.x *= p;
+                p *= f.x;
+                *reinterpret_cast<float2*>(ks + j * D8 + 2 * d) = k;
             }
-            sc.dec[((size_t)ci * H + h) * D + d] = p;
+            if (!late) sc.dec[((size_t)ci * H + h) * D + d] = p;
         }
     } else {
         for (int d = threadIdx.x; d < D; d += GC_THREADS) {
             float s = 0.f;
 #pragma unroll 8
-            for (int j = 0; j < GC; ++j) s += ks[j * D8 + d];
+            for (int j = 0; j < GC; j += 2) {
+                const float2 k = *reinterpret_cast<const float2*>(ks + j * D8 + 2 * d);
+                s += k.x;
+                s += k.y;
+            }
             sc.ns[((size_t)ci * H + h) * D + d] = s;
         }
     }
@@ -283,40 +304,40 @@ __global__ void __launch_bounds__(GC_THREADS) gated_chunk_state_kernel(DlMambaBa
     const int tb = threadIdx.x >> 4, cb = threadIdx.x & 15;
     for (int c0 = 0; c0 < V; c0 += 64 * NC) {
         __syncthreads();
-        gated_stage_v<64 * NC>(a, rows, len, h, c0, vt);
+        gated_stage_v<64 * NC, true>(a, rows, len, h, c0, vt);
         __syncthreads();
         for (int d0 = 0; d0 < D; d0 += 16 * RT) {
-            const int dt = d0 + tb * RT;         // this thread: RT rows of S, columns cb * 4 .. + 3 (and 64 + cb * 4 .. + 3) of the tile
+            const int dt = d0 + tb * RT;         // this thread: RT rows of S, columns 32 u + cb * 2 and + 1 of the tile
             if (dt >= D8) continue;
-            float acc[RT][4 * NC];
+            pair_f acc[RT][4 * NC];              // the sums over even and odd tokens
 #pragma unroll
             for (int r = 0; r < RT; ++r)
 #pragma unroll
-                for (int u = 0; u < 4 * NC; ++u) acc[r][u] = 0.f;
-#pragma unroll 2
-            for (int j = 0; j < len; ++j) {
-                float kk[RT], vv[4 * NC];
+                for (int u = 0; u < 4 * NC; ++u) acc[r][u] = 0;
+#pragma unroll 1
+            for (int j = 0; j < len; j += 2) {   // rows beyond the chunk are zeros
+                pair_f kk[RT];
 #pragma unroll
-                for (int r = 0; r < RT; r += 4) {
-                    const float4 k = *reinterpret_cast<const float4*>(ks + j * D8 + dt + r);
-                    kk[r] = k.x; kk[r + 1] = k.y; kk[r + 2] = k.z; kk[r + 3] = k.w;
+                for (int r = 0; r < RT; r += 2) {
+                    const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(ks + j * D8 + (dt + r) * 2);
+                    kk[r] = k.x; kk[r + 1] = k.y;
                 }
 #pragma unroll
-                for (int u = 0; u < NC; ++u) {
-                    const float4 v = *reinterpret_cast<const float4*>(vt + j * 64 * NC + u * 64 + cb * 4);
-                    vv[4 * u] = v.x; vv[4 * u + 1] = v.y; vv[4 * u + 2] = v.z; vv[4 * u + 3] = v.w;
+                for (int u = 0; u < 2 * NC; ++u) {
+                    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(vt + j * 64 * NC + (u * 32 + cb * 2) * 2);
+#pragma unroll
+                    for (int r = 0; r < RT; ++r) {
+                        acc[r][2 * u] = fma2(kk[r], v.x, acc[r][2 * u]);
+                        acc[r][2 * u + 1] = fma2(kk[r], v.y, acc[r][2 * u + 1]);
+                    }
                 }
-#pragma unroll
-                for (int r = 0; r < RT; ++r)
-#pragma unroll
-                    for (int u = 0; u < 4 * NC; ++u) acc[r][u] = fmaf(kk[r], vv[u], acc[r][u]);
             }
 #pragma unroll
             for (int r = 0; r < RT; ++r)
 #pragma unroll
                 for (int u = 0; u < 4 * NC; ++u) {
-                    const int d = dt + r, cc = c0 + (u >> 2) * 64 + cb * 4 + (u & 3);
-                    if (d < D && cc < V) out[(size_t)d * V + cc] = acc[r][u];
+                    const int d = dt + r, cc = c0 + (u >> 1) * 32 + cb * 2 + (u & 1);
+                    if (d < D && cc < V) out[(size_t)d * V + cc] = pair_sum(acc[r][u]);
                 }
         }
     }
@@ -355,10 +376,18 @@ __global__ void __launch_bounds__(256) gated_chunk_prefix_kernel(DlMambaBatch b,
     *Sg = R;
 }
 
+// Passes 1 and 3 are bound by the instructions that their 16 warps per SM issue (shared memory holds two CTAs of the output kernel): f32
+// multiply-adds throughout, whole running products for the diagonal sub-blocks, and the gates' exponentials, formed in both.  So two
+// neighbours along the contraction are one operand (fma2: two multiply-adds an issue), the diagonal takes two columns and two
+// channels at a time, and a warp's eight rows form their gates side by side: 2000 rows x 16 heads of 128 x 128 240.7 -> 180 us, pass 1
+// 75 -> 63, pass 3 153 -> 103.  Twice the warps at half the registers (a column of the diagonal and half of the tile each): 206,
+// three CTAs of pass 1 on an SM (80 registers, spilled): 205.  Narrow tiles leave shared memory for more CTAs and do with fewer registers:
+// three of pass 3 (80) and four of pass 1 (64), 2000 rows x 32 heads of 64 x 64 136 -> 123 us (head form 156 -> 128; before 175 and 150).
+//
 // pass 3: the outputs of a chunk.  Shared memory: Q [GC][DP] | K [GC][DP], later tiles of V and of the carried state
 // [GC][64 NC] | F [GC][DP] (channel form), later the scores A [GC][GC_AS] | block decays [4][DP].
 template <int MODE, int NC>
-__global__ void __launch_bounds__(GC_THREADS, 2) gated_chunk_out_kernel(DlMambaBatch b, DlGatedArgs a, GatedScratch sc) {
+__global__ void __launch_bounds__(GC_THREADS, NC == 1 ? 3 : 2) gated_chunk_out_kernel(DlMambaBatch b, DlGatedArgs a, GatedScratch sc) {
     constexpr bool CH = MODE != GATED_HEAD;
     extern __shared__ __align__(16) float sm[];
     __shared__ int rows[GC];
@@ -448,47 +477,47 @@ __global__ void __launch_bounds__(GC_THREADS, 2) gated_chunk_out_kernel(DlMambaB
     constexpr int VW = 64 * NC;
     for (int c0 = 0; c0 < V; c0 += VW) {
         const int cw = min(VW, V - c0);
-        float acc[4][4 * NC];
+        // acc: rows tb * 4 + r, columns 32 (u / 2) + cb * 2 + (u & 1), the sums over even and odd k
+        pair_f acc[4][4 * NC];
 #pragma unroll
         for (int r = 0; r < 4; ++r)
 #pragma unroll
-            for (int u = 0; u < 4 * NC; ++u) acc[r][u] = 0.f;
+            for (int u = 0; u < 4 * NC; ++u) acc[r][u] = 0;
         __syncthreads();
-        gated_stage_v<VW>(a, rows, len, h, c0, W);
+        gated_stage_v<VW, true>(a, rows, len, h, c0, W);
         __syncthreads();
         auto tile_mac = [&](const float* X, int ldx, int kn) {           // acc += X[rows][0 .. kn) . W[0 .. kn)[columns], kn a multiple of 4
             for (int k = 0; k < kn; k += 4) {
-                float4 x[4];
+                ulonglong2 x[4];
 #pragma unroll
-                for (int r = 0; r < 4; ++r) x[r] = *reinterpret_cast<const float4*>(X + (tb * 4 + r) * ldx + k);
+                for (int r = 0; r < 4; ++r) x[r] = *reinterpret_cast<const ulonglong2*>(X + (tb * 4 + r) * ldx + k);
 #pragma unroll
-                for (int kk = 0; kk < 4; ++kk) {
-                    float wv[4 * NC];
+                for (int kk = 0; kk < 4; kk += 2)
 #pragma unroll
-                    for (int u = 0; u < NC; ++u) {
-                        const float4 w = *reinterpret_cast<const float4*>(W + (k + kk) * VW + u * 64 + cb * 4);
-                        wv[4 * u] = w.x; wv[4 * u + 1] = w.y; wv[4 * u + 2] = w.z; wv[4 * u + 3] = w.w;
+                    for (int u = 0; u < 2 * NC; ++u) {
+                        const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(W + (k + kk) * VW + (u * 32 + cb * 2) * 2);
+#pragma unroll
+                        for (int r = 0; r < 4; ++r) {
+                            const pair_f xv = kk == 0 ? x[r].x : x[r].y;
+                            acc[r][2 * u] = fma2(xv, w.x, acc[r][2 * u]);
+                            acc[r][2 * u + 1] = fma2(xv, w.y, acc[r][2 * u + 1]);
+                        }
                     }
-#pragma unroll
-                    for (int r = 0; r < 4; ++r) {
-                        const float xv = kk == 0 ? x[r].x : kk == 1 ? x[r].y : kk == 2 ? x[r].z : x[r].w;
-#pragma unroll
-                        for (int u = 0; u < 4 * NC; ++u) acc[r][u] = fmaf(xv, wv[u], acc[r][u]);
-                    }
-                }
             }
         };
         if (tb * 4 < len) tile_mac(A, GC_AS, tb * 4 + 4);
         for (int d0 = 0; d0 < D; d0 += GC) {
             const int dn = min(GC, D - d0), dn4 = (dn + 3) & ~3;
             __syncthreads();
-#pragma unroll 4
-            for (int d = warp; d < dn4; d += GC_THREADS / 32) {
-                float p[VW / 32];
+#pragma unroll 2
+            for (int d = 2 * warp; d < dn4; d += GC_THREADS / 16) {
+                float p[2][VW / 32];
 #pragma unroll
-                for (int u = 0; u < VW / 32; ++u) p[u] = (d < dn && lane + 32 * u < cw) ? P[(size_t)(d0 + d) * V + c0 + lane + 32 * u] : 0.f;
+                for (int u = 0; u < VW / 32; ++u)
 #pragma unroll
-                for (int u = 0; u < VW / 32; ++u) W[d * VW + lane + 32 * u] = p[u];
+                    for (int w = 0; w < 2; ++w) p[w][u] = (d + w < dn && lane + 32 * u < cw) ? P[(size_t)(d0 + d + w) * V + c0 + lane + 32 * u] : 0.f;
+#pragma unroll
+                for (int u = 0; u < VW / 32; ++u) *reinterpret_cast<float2*>(W + d * VW + (lane + 32 * u) * 2) = make_float2(p[0][u], p[1][u]);
             }
             __syncthreads();
             if (tb * 4 < len) tile_mac(Q + d0, DP, dn4);
@@ -500,8 +529,8 @@ __global__ void __launch_bounds__(GC_THREADS, 2) gated_chunk_out_kernel(DlMambaB
             float* y = a.y + (size_t)rows[i] * a.ld_y + (size_t)h * V + c0;
 #pragma unroll
             for (int u = 0; u < 4 * NC; ++u) {
-                const int cc = (u >> 2) * 64 + cb * 4 + (u & 3);
-                if (cc < cw) y[cc] = acc[r][u];
+                const int cc = (u >> 1) * 32 + cb * 2 + (u & 1);
+                if (cc < cw) y[cc] = pair_sum(acc[r][u]);
             }
         }
     }
@@ -555,7 +584,7 @@ static int launch_gated_chunked(const DlMambaBatch& b, int n_seq, int max_chunks
     constexpr bool CH = MODE != GATED_HEAD;
     const bool narrow = gated_nc(a.vdim) == 1, low = a.dim <= 64;
     int rc = narrow ? (low ? launch_gated_state<CH, 4, 1>(b, n_seq, max_chunks, a, sc, st) : launch_gated_state<CH, 8, 1>(b, n_seq, max_chunks, a, sc, st))
-                    : (low ? launch_gated_state<CH, 4, 2>(b, n_seq, max_chunks, a, sc, st) : launch_gated_state<CH, 8, 2>(b, n_seq, max_chunks, a, sc, st));
+                    : launch_gated_state<CH, 4, 2>(b, n_seq, max_chunks, a, sc, st);
     if (rc != 0) return rc;
     gated_chunk_prefix_kernel<CH><<<dim3(n_seq, a.n_heads, (a.dim * (a.vdim + (CH ? 0 : 1)) + 255) / 256), 256, 0, st>>>(b, a, sc);
     return narrow ? launch_gated_out<MODE, 1>(b, n_seq, max_chunks, a, sc, st) : launch_gated_out<MODE, 2>(b, n_seq, max_chunks, a, sc, st);

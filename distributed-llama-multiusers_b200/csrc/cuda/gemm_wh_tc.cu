@@ -371,7 +371,7 @@ extern "C" int dl_device_sm_count();
 //
 // What bounds it: the weights' bytes.  The 256 x 256 pair tiles above give a 4096-wide output 16 of the 74 pairs, and 28672
 // columns 112 tiles in two waves: norm, gate|up and down of 4096 x 14336 in bf16 at 32 rows took 184 us, 1.9 TB/s
-// (now 86: 47 and 35 us for the products, 5.0 and 3.3 TB/s).  Here the OUTPUT
+// (here 86: 47 and 35 us for the products, 5.0 and 3.3 TB/s; 79.5 with the launches chained).  Here the OUTPUT
 // COLUMNS are dealt to all SMs in groups of 8 (one core-matrix row group of the weight image, 2 KB per k tile), so every SM
 // streams the same number of bytes to within 8 rows; a CTA walks the whole K (or its share of a cluster's) once through a
 // ring of bulk copies, MMA M = 128 with the rows past its share reading whatever lies behind (those accumulator lanes are
