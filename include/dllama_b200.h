@@ -320,7 +320,7 @@ int dl_peer_barrier(uint32_t* const* flags_on_peers /*host array*/, uint32_t* my
 
 /* ==== layer-list models: dense bf16 / f32 weights, latent attention, Mamba-2 ===================
  * Built into libdllama_b200_layers.so (dense.cu, norms.cu, latent_attention.cu, mamba2.cu, hyper.cu, window_attention.cu,
- * talk_attention.cu, lightning.cu, moe.cu, plus the shared prep.cu, sampler.cu and gemm_wh_tc.cu).  Activations between kernels are f32; `wtype` / `ctype`: 0 = f32, 1 = bf16. */
+ * talk_attention.cu, lightning.cu, moe.cu, plus the shared prep.cu, sampler.cu, gemm_wh_tc.cu and attention_prefill_tc.cu).  Activations between kernels are f32; `wtype` / `ctype`: 0 = f32, 1 = bf16. */
 
 /* Y[b][m][n] = epi( sum_k X[b][m][k] * W[b][n][k] ),  b < batch (element strides *_bs).  round_x: the activation
  * operand is rounded to bf16 on load (bf16 mode).  DL_DENSE_SIGMOID_MUL: aux[m][n] * sigmoid(.);
