@@ -338,7 +338,8 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attention_kernel(const __grid_
 // ------------------------------------------------------------------------------------------------
 #define AM_TOK 16
 #define AM_Q_UP 64.0f                     // 2^6 on the queries
-#define AM_P_UP 12.0f                     // 2^12 on the weights (added to the exponent)
+#define AM_P_UP 4096.0f                   // 2^12 on the weights (a factor: added to the exponent ahead of exp2 it rounded the difference to 2^-21,
+                                          // 2.8e-7 against 64 bits at 180 tokens instead of the FMA kernel's 1.6e-7)
 
 DL_DEVINL void am_cp16(uint32_t dst, const void* src, bool live) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(live ? 16 : 0) : "memory");
@@ -504,7 +505,7 @@ __global__ void __launch_bounds__(ATT_WARPS * 32, 3) attention_mma_kernel(const 
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
             __half t0, b0, t1, b1;
-            const float p0 = am_exp2(s[2 * j] - m_use + AM_P_UP), p1 = am_exp2(s[2 * j + 1] - m_use + AM_P_UP);
+            const float p0 = am_exp2(s[2 * j] - m_use) * AM_P_UP, p1 = am_exp2(s[2 * j + 1] - m_use) * AM_P_UP;
             ps += p0 + p1;
             am_split(p0, lower, t0, b0);
             am_split(p1, lower, t1, b1);
@@ -573,7 +574,7 @@ __global__ void __launch_bounds__(ATT_WARPS * 32, 3) attention_mma_kernel(const 
                     for (int d = 0; d < DPL; ++d) v = fmaf(q[d], __half2float(reinterpret_cast<const __half*>(a.k_cache)[at + d]), v);
                     v = warp_sum(v);
                     const float mn = fmaxf(M, v), mu = mn == -INFINITY ? 0.f : mn;
-                    const float cr = am_exp2(M - mu), p = am_exp2(v - mu + AM_P_UP);
+                    const float cr = am_exp2(M - mu), p = am_exp2(v - mu) * AM_P_UP;
                     M = mn;
                     Ls = fmaf(Ls, cr, p);
 #pragma unroll
