@@ -342,27 +342,35 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_q40_tc_kernel(const __grid
         }
         tc_fence_before();
         cluster.sync();
+        // a rank tells its peers that it has read their shares as soon as it has, ahead of its own epilogue: the barrier at the end then
+        // costs nothing (with the epilogue's loads and stores ahead of it a 4-row step of width 2048 took 236 us, now 230)
+        auto read_all = [] { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); };
+        const int ms = Mt * crank / S, me = Mt * (crank + 1) / S;
+        if (!is_epi || ms >= me) read_all();
         if (is_epi) {
-            const int ms = Mt * crank / S, me = Mt * (crank + 1) / S;
             pdl_wait();
             for (int h = 0; h < P; h++)
                 for (int mb = ms; mb < me; mb += TC_EPI_CHUNK) {
                     const int mc = min(TC_EPI_CHUNK, me - mb);
                     const size_t base = ((size_t)h * NT + mb) * 128;
                     for (int idx = tid - 64; idx < mc * 32; idx += TC_DEQ_WARPS * 32) {
-                        float4 v = *reinterpret_cast<const float4*>(cluster.map_shared_rank(all_s, 0) + base + idx * 4);
-                        for (int c = 1; c < S; c++) {
-                            const float4 x = *reinterpret_cast<const float4*>(cluster.map_shared_rank(all_s, c) + base + idx * 4);
-                            v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
-                        }
+                        float4 x[8];                            // S <= 8: the ranks' shares in flight together, summed in rank order
+#pragma unroll
+                        for (int c = 0; c < 8; c++)
+                            if (c < S) x[c] = *reinterpret_cast<const float4*>(cluster.map_shared_rank(all_s, c) + base + idx * 4);
+                        float4 v = x[0];
+#pragma unroll
+                        for (int c = 1; c < 8; c++)
+                            if (c < S) { v.x += x[c].x; v.y += x[c].y; v.z += x[c].z; v.w += x[c].w; }
                         reinterpret_cast<float4*>(out_s)[idx] = v;
                     }
                     asm volatile("bar.sync 1, 512;" ::: "memory");
+                    if (h == P - 1 && mb + TC_EPI_CHUNK >= me) read_all();
                     epilogue_rows(a.epi, out_s, 128, 128, (rt + h) * 128, a.d_real, mc, m0 + mb, etid, eg, TC_GROUPS);
                     asm volatile("bar.sync 1, 512;" ::: "memory");      // out_s is rewritten by the next round
                 }
         }
-        cluster.sync();      // nobody leaves while a peer may still read its share
+        asm volatile("barrier.cluster.wait.acquire;" ::: "memory");     // nobody leaves while a peer may still read its share
     } else if (is_epi) {
         for (int h = 0; h < P; h++)
             for (int ch = 0; ch < n_chunks; ch++) {
