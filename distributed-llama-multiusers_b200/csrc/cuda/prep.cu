@@ -140,7 +140,9 @@ extern "C" int dl_embedding(const float* table, const int* tokens, float* x, int
 // ------------------------------------------------------------------------------------------------
 #define RNQ_THREADS 512
 #define RNQ_MAX_PER_THREAD 32     // dim <= 512*32 = 16384
-#define RNQ_WIDE_ROWS 512         // from here on 8 rows per CTA
+// From here on 8 rows per CTA: 148 CTAs, one for every SM.  Below, fewer cannot pull as much (width 4096, the kernel alone: 512 rows 6.7 us with a
+// row per CTA, 10.2 with 8; norm and feed-forward at 1024 rows 427 and 430); above, whole lines of the image count (2048 rows 783 and 769).
+#define RNQ_WIDE_ROWS 1184
 
 struct RnqArgs {
     const float* x_in;
