@@ -256,8 +256,12 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
         j1 = last_pos / PT_KV + 1;
         n_kv = a.n_kv_heads;
     } else {
-        // (launched behind a kernel that writes other rows of the same output and reads the same inputs: nothing to wait for here)
+        // (launched behind a kernel that writes other rows of the same output and reads the same inputs: nothing to wait for here.  What
+        // follows this grid must follow that one too, so this grid may not end ahead of it: a CTA with work waits when it is done, and the
+        // first CTA waits even without -- one is enough, a grid ends with its last CTA, and all of the idle ones would keep an SM each
+        // from those with work)
         const DlWindowAttnArgs& w = a.w;
+        const bool first_cta = blockIdx.x == 0 && blockIdx.y == 0;
         kvh = blockIdx.y;
         const int t = (int)gridDim.x - 1 - (int)blockIdx.x;      // late tiles (long histories) first
         auto count = [&](int u) { int n = 0; if (u < a.n_tiles) while (n < a.rq && a.tile_rows[(size_t)u * a.rq + n] >= 0) ++n; return n; };
@@ -268,9 +272,11 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
             const int me = a.tile_rows[(size_t)e * a.rq], mo = a.tile_rows[(size_t)(e + 1) * a.rq];
             both = w.slot[me] == w.slot[mo] && w.pos[mo] == w.pos[me] + ne;
         }
-        if ((t & 1) && both) return;
-        const int run = (t & 1) ? no : both ? ne + no : ne;
-        if (run * a.rep <= 16) return;                           // a decoding tile belongs to the other kernel
+        const int run = (t & 1) ? (both ? 0 : no) : both ? ne + no : ne;
+        if (run * a.rep <= 16) {                                 // taken along by its neighbour, or a decoding tile, which belongs to the other kernel
+            if (first_cta) pdl_wait();
+            return;
+        }
         rows_of = a.tile_rows + (size_t)t * a.rq;
         const int m0 = rows_of[0], p_first = w.pos[m0];
         n_rows = run * a.rep;

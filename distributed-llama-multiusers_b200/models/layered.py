@@ -569,6 +569,8 @@ class WindowAttentionMixer:
         tile = attn_tc and self.own_v and L.talk_tc_supported(H, G, d, dv, self.key_heads, eng.wdtype, self.value_heads)
         if attn_tc and not (tile and self.head_gate) and dv == d and self.talk is None and L.window_tc_supported(H, G, d, 0 if self.own_v else self.rope_dims, eng.wdtype):
             self.tc_rq = L.window_tc_rows(H, G)
+            # batches of decoding rows alone: tiles of 16 stacked rows, so that no grid for taller ones is launched beside them
+            self.tc_rq_small = 16 // (H // G)
         elif tile:
             # values wider or narrower than the keys, head-mixed scores, head gates: the tile kernel of talk_attention.cu
             # tiles of 128 stacked (row, head) pairs for long portions, of 16 for decoding, 64 where those do not fit

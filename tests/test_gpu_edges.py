@@ -262,3 +262,60 @@ def test_dense_few_rows(M, N, K_, dtype, round_x):
         half = torch.zeros(M, N // 2, device="cuda")
         L().dense(w, x, half, M, round_x, epi=L().DENSE_GLU_GELU)
         assert close(half, torch.nn.functional.gelu(z[:, 0::2], approximate="tanh") * z[:, 1::2])
+
+
+def _one_row_tiles(contexts, heads, kv, seed):
+    """Decoding rows of sequences of these lengths on 128 / 128 bf16 lines: call(out) runs the attention, n_splits == 1."""
+    M, dim = len(contexts), 128
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    need = [(t + 31) // 32 for t in contexts]
+    bt = torch.zeros(M, max(need), dtype=torch.int32)
+    perm = torch.randperm(sum(need), generator=torch.Generator().manual_seed(seed)).int()
+    for m in range(M):
+        bt[m, :need[m]] = perm[sum(need[:m]):sum(need[:m + 1])]
+    cache = torch.randn(sum(need), kv, 32, 2 * dim, generator=g, device="cuda").bfloat16()
+    q = torch.randn(M, heads * dim, generator=g, device="cuda")
+    rq = L().window_tc_rows(heads, kv)
+    tiles = torch.full((M, rq), -1, dtype=torch.int32)
+    tiles[:, 0] = torch.arange(M, dtype=torch.int32)
+    pos, slot = torch.tensor([t - 1 for t in contexts], dtype=torch.int32, device="cuda"), torch.arange(M, dtype=torch.int32, device="cuda")
+    bt, tiles = bt.cuda(), tiles.cuda()
+    return lambda out: L().window_attention_tc(q, out, heads, kv, dim, 0, dim ** -0.5, 0.0, 0, pos, slot, bt, cache, tiles, M, rq, vdim=dim)
+
+
+@pytest.mark.parametrize("M,heads,kv,graph", [(80, 16, 4, False), (40, 32, 8, True)])
+def test_window_decode_is_whole_before_what_follows(M, heads, kv, graph):
+    """Many decoding rows without page shares, one context much longer than the others, and behind them a programmatically launched product
+    that reads the output (a gate on it, then its image): the same bits as with a synchronisation in between."""
+    width, N = heads * 128, 256
+    attend = _one_row_tiles([4000] + [1] * (M - 1), heads, kv, M)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    w, w2 = (L().make_wh((torch.randn(n, k, generator=g, device="cuda") * k ** -0.5).bfloat16()) for n, k in ((width, N), (N, width)))
+    x, ncap = torch.randn(M, N, generator=g, device="cuda"), (M + 7) // 8 * 8
+    xh, oh = (torch.zeros(L().xh_bytes(k, ncap), dtype=torch.uint8, device="cuda") for k in (N, width))
+    L().xh_from_rows(x, M, N, ncap, xh)
+    out, gated, y = (torch.zeros(M, k, device="cuda") for k in (width, width, N))
+
+    def step(between=lambda: None):
+        attend(out)
+        between()
+        L().dense_tc(w, width, N, xh, ncap, gated, M, epi=L().DENSE_SIGMOID_MUL, aux=out)
+        L().xh_from_rows(out, M, width, ncap, oh)
+        L().dense_tc(w2, N, width, oh, ncap, y, M)
+
+    step(torch.cuda.synchronize)
+    want = [t.clone() for t in (out, gated, y)]
+    run = step
+    if graph:
+        cg, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.graph(cg, stream=side):
+            step()
+        run = cg.replay
+    for _ in range(20):
+        for t in (out, gated, y):
+            t.zero_()
+        run()
+        torch.cuda.synchronize()
+        for t, ref in zip((out, gated, y), want):
+            assert torch.equal(t, ref)
