@@ -35,6 +35,7 @@
 // (src/llm.cpp:296-301).  KV cache: fp16 pages [page][kv_head][32][128].
 #include <cuda.h>
 #include "epilogue.cuh"
+#include "window_tiles.cuh"
 
 #define PT_HS 128
 #define PT_ROWS 128
@@ -256,7 +257,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
         j1 = last_pos / PT_KV + 1;
         n_kv = a.n_kv_heads;
     } else {
-        // (launched behind a kernel that writes other rows of the same output and reads the same inputs: nothing to wait for here.  What
+        // (launched behind a kernel that writes the rows of other tiles and reads the same inputs: nothing to wait for here.  What
         // follows this grid must follow that one too, so this grid may not end ahead of it: a CTA with work waits when it is done, and the
         // first CTA waits even without -- one is enough, a grid ends with its last CTA, and all of the idle ones would keep an SM each
         // from those with work)
@@ -264,14 +265,9 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
         const bool first_cta = blockIdx.x == 0 && blockIdx.y == 0;
         kvh = blockIdx.y;
         const int t = (int)gridDim.x - 1 - (int)blockIdx.x;      // late tiles (long histories) first
-        auto count = [&](int u) { int n = 0; if (u < a.n_tiles) while (n < a.rq && a.tile_rows[(size_t)u * a.rq + n] >= 0) ++n; return n; };
         const int e = t & ~1;                                    // an even tile takes its neighbour along where that continues its sequence
-        const int ne = count(e), no = count(e + 1);
-        bool both = ne == a.rq && no > 0;
-        if (both) {
-            const int me = a.tile_rows[(size_t)e * a.rq], mo = a.tile_rows[(size_t)(e + 1) * a.rq];
-            both = w.slot[me] == w.slot[mo] && w.pos[mo] == w.pos[me] + ne;
-        }
+        const int ne = window_tile_count(a.tile_rows, a.n_tiles, a.rq, e), no = window_tile_count(a.tile_rows, a.n_tiles, a.rq, e + 1);
+        const bool both = window_tiles_join(w, a.tile_rows, a.rq, e, ne, no);
         const int run = (t & 1) ? (both ? 0 : no) : both ? ne + no : ne;
         if (run * a.rep <= 16) {                                 // taken along by its neighbour, or a decoding tile, which belongs to the other kernel
             if (first_cta) pdl_wait();

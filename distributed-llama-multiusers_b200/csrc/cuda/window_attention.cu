@@ -23,6 +23,7 @@
 // (row, key/value head), all query heads of the group share each staged page; pages outside the window are never
 // touched); the tensor-core kernel for prompt portions (bf16 cache) further down.
 #include "mma_common.cuh"
+#include "window_tiles.cuh"
 #include "../../../include/dllama_b200.h"
 
 #define WA_PAGE 32
@@ -576,6 +577,8 @@ __global__ void __launch_bounds__(128, 4) window_attention_mma_kernel(DlWindowAt
         pg_hi = min(pg_hi, pg_lo + per - 1);
     }
     if (n_rows * rep <= 16) {            // decoding: one 16-row tile, the warps share the tokens
+        if (only_small && (tile & 1) && window_tiles_join(a, tile_rows, rq, tile - 1, window_tile_count(tile_rows, gridDim.x, rq, tile - 1), n_rows))
+            return;                      // the end of a prompt: attention_prefill_tc.cu takes it along with the full tile ahead of it
         if (pg_lo > pg_hi) {             // a share without pages (of several): it weighs nothing
             if (threadIdx.x < n_rows * rep) {
                 float* dst = partial + ((((size_t)tile * a.kv_heads + g) * n_splits + blockIdx.z) * WM_ROWS + threadIdx.x) * (D + 2) + D;
