@@ -28,8 +28,12 @@
 // The second instance (LINES) serves layer-list models: bf16 cache lines [key 128 | value 128], tiles of up to rq consecutive positions
 // of one sequence whose query heads of one key/value head stack on the MMA's rows (row = position * rep + head), so two neighbouring
 // tiles of 64 stacked rows fill the 128 lanes; window or chunk masks (only the steps that a tile sees are walked), soft cap, distance
-// bias, sink, gate; f32 output.  mma.sync with its 64-row tiles took 142 us for 2000 rows of 16 heads on 4 under a window of 1024
-// (88 TFLOP/s); 52 us here.
+// bias, sink, gate; f32 output.  Probabilities are two bf16 numbers each, the second the first one's remainder, and P V two MMAs: rounded to
+// one (2^-9) they are the larger share of the error, and how large depends on how often a row's maximum, whose probability is exact, moves
+// -- every 32 tokens in the mma.sync kernel, every 128 here (2000 tokens under a window of 1024, against 64 bits: 1.929e-3 with one number,
+// 1.926e-3 there, 1.50e-3 with two; 1300 tokens: 2.19e-3, 2.17e-3, 1.64e-3; the time is the same).  The remainders lie in the score buffer that they
+// came from, so S of step j + 2 waits for P V of step j.  mma.sync with its 64-row tiles took 142 us for 2000 rows of 16 heads on 4 under a window of 1024
+// (88 TFLOP/s); 55 us here.
 //
 // Reference semantics: multiheadAtt_F32 (src/nn/nn-cpu-ops.cpp:749-784), softmax in f32, output cast as OP_CAST
 // (src/llm.cpp:296-301).  KV cache: fp16 pages [page][kv_head][32][128].
@@ -142,21 +146,22 @@ template <bool LINES> DL_DEVINL float pt_ex2_poly(float x) {
     return __int_as_float(__float_as_int(p) + (__float_as_int(t) << 23));
 }
 
-// 32 scores (masked ones are -inf) -> exp2(s * sc - ref) as 16 packed fp16 (LINES: bf16) pairs into TMEM; returns their sum.  LINES: the
-// sum of the ROUNDED probabilities, so that a row's weights add up to one
-template <bool LINES> DL_DEVINL float pt_probs(const uint32_t (&v)[32], float sc, float ref, uint32_t taddr) {
-    uint32_t pk[16];
+// 32 scores (masked ones are -inf) -> exp2(s * sc - ref) as 16 packed fp16 pairs into TMEM; returns their sum.  LINES: as bf16 and, at
+// taddr_lo, the bf16 remainder of each, 17 bits together
+template <bool LINES> DL_DEVINL float pt_probs(const uint32_t (&v)[32], float sc, float ref, uint32_t taddr, uint32_t taddr_lo) {
+    uint32_t pk[16], lo[LINES ? 16 : 1];
     float sum = 0.0f;
 #pragma unroll
     for (int e = 0; e < 32; e += 2) {
         const float pa = pt_ex2(fmaf(__uint_as_float(v[e]), sc, -ref));
         const float xb = fmaf(__uint_as_float(v[e + 1]), sc, -ref);
         const float pb = (e & 2) ? pt_ex2_poly<LINES>(xb) : pt_ex2(xb);
+        sum += pa + pb;
         pk[e >> 1] = pt_pack2<LINES>(pa, pb);
-        if (LINES) sum += __uint_as_float(pk[e >> 1] << 16) + __uint_as_float(pk[e >> 1] & 0xffff0000u);
-        else sum += pa + pb;
+        if constexpr (LINES) lo[e >> 1] = pt_pack2<LINES>(pa - __uint_as_float(pk[e >> 1] << 16), pb - __uint_as_float(pk[e >> 1] & 0xffff0000u));
     }
     tmem_st_32x32b_x16(taddr, pk);
+    if constexpr (LINES) tmem_st_32x32b_x16(taddr_lo, lo);
     return sum;
 }
 
@@ -325,7 +330,8 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
         for (int j = 0; j < n_tiles; j++) {
             pt_wait(&k_full[j % PT_STAGES], (j / PT_STAGES) & 1, t0);
             if (lane == 0) PT_STAMP(0, j);
-            if (j >= 2) pt_wait(&s_empty[j & 1], ((j - 2) >> 1) & 1, t0);     // softmax(j-2) has this score buffer in registers
+            // softmax(j-2) has this score buffer in registers; LINES: P V(j-2) has read the remainders that lay in it
+            if (j >= 2) pt_wait(LINES ? &o_full[j & 1] : &s_empty[j & 1], ((j - 2) >> 1) & 1, t0);
             tc_fence_after();
             if (elect_one()) {
                 const uint32_t a_lo = lo_k(q_s), b_lo = lo_k(k_s + (j % PT_STAGES) * PT_TILE_BYTES);
@@ -378,6 +384,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
                     uint64_t db;
                     asm("mov.b64 %0, {%1, %2};" : "=l"(db) : "r"(b_lo + k * 128), "r"(desc_hi));
                     if (!PT_DBG(4)) umma_f16_ts(T_O, T_P + (i & 1) * 64 + k * 8, db, idesc_pv, (i > 0 || k > 0) ? 1u : 0u);
+                    if constexpr (LINES) umma_f16_ts(T_O, T_S + (i & 1) * 128 + k * 8, db, idesc_pv, 1u);
                 }
                 umma_commit(&o_full[i & 1]);
                 umma_commit(&v_empty[i % PT_STAGES]);
@@ -484,12 +491,10 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
             mx_s[((j & 1) * 2 + hf) * PT_ROWS + row] = mx;
             asm volatile("bar.sync 2, 256;" ::: "memory");
             mx = fmaxf(mx, mx_s[((j & 1) * 2 + (hf ^ 1)) * PT_ROWS + row]);
+            if constexpr (LINES) tc_fence_after();           // both halves have read their scores: the remainders take their place
             if (tid == 32) PT_STAMP(4, j);
             mx *= sc;
-            // the reference may lag the maximum by 2^8 where probabilities are fp16 (11 bits).  LINES has bf16 ones: with the maximum itself as the
-            // reference a row's largest probability is 1 and exact, otherwise its rounding (2^-9) is the largest share of the error (2000 tokens
-            // under a window of 256, against 64 bits: 2.30e-3 lagging, 2.17e-3 here, 2.15e-3 in the mma.sync kernel; 47.2 and 47.5 us)
-            const bool need = mx > m_used + (LINES ? 0.0f : 8.0f);
+            const bool need = mx > m_used + 8.0f;            // the reference may lag the maximum by 2^8
             if (__any_sync(0xffffffffu, need)) {
                 const float m_new = need ? mx : m_used;
                 const float alpha = need ? pt_ex2(m_used - m_new) : 1.0f;
@@ -516,8 +521,9 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
                 pt_wait(&o_full[j & 1], ((j - 2) >> 1) & 1, t0);
                 tc_fence_after();
             }
-            l += pt_probs<LINES>(v0, sc, ref, t_p);
-            l += pt_probs<LINES>(v1, sc, ref, t_p + 16);
+            const uint32_t t_lo = T_S + lane_base + (j & 1) * 128 + hf * 32;
+            l += pt_probs<LINES>(v0, sc, ref, t_p, t_lo);
+            l += pt_probs<LINES>(v1, sc, ref, t_p + 16, t_lo + 16);
             tmem_st_wait();
             tc_fence_before();
             mbar_arrive(&p_full[j & 1]);

@@ -321,12 +321,14 @@ def test_window_decode_is_whole_before_what_follows(M, heads, kv, graph):
             assert torch.equal(t, ref)
 
 
-def _prompt(rows, heads, kv, n_tokens=None, scale=None, keys=None, seed=5, **opt):
+def _prompt(rows, heads, kv, scale=None, keys=None, seed=5, **opt):
     """A prompt of `rows` positions in one sequence on 128 / 128 bf16 lines, no page shares: call() runs it and returns the output rows."""
     dim, pages = 128, (rows + 31) // 32
     g = torch.Generator(device="cuda").manual_seed(seed)
     cache = torch.randn(128, kv, 32, 2 * dim, generator=g, device="cuda").bfloat16()
     q = torch.randn(4096, heads * dim, generator=g, device="cuda")[:rows]
+    if opt.get("bf16_queries"):
+        q = q.bfloat16().float()
     if keys is not None:
         keys(cache)
     bt = torch.arange(pages, dtype=torch.int32, device="cuda").view(1, pages)
@@ -353,3 +355,28 @@ def test_window_prompt_tiles_have_one_owner(rows):
     want = _prompt((rows + 31) // 32 * 32, 16, 4)()[:rows]
     for _ in range(50):
         assert torch.equal(call(), want)
+
+
+def _window_want(call, heads, kv, scale, softcap, window, rows):
+    """Output of these rows of a _prompt in 64 bits, from queries as they are."""
+    line = call.cache.double().transpose(1, 2).reshape(-1, kv, 256)
+    k, v = (line[..., o:o + 128].repeat_interleave(heads // kv, dim=1) for o in (0, 128))
+    at = torch.arange(k.shape[0], device="cuda")
+    out = []
+    for m in rows:
+        seen = (at <= m) & ((m - at < window) if window else torch.ones_like(at, dtype=torch.bool))
+        s = torch.einsum("hd,thd->ht", call.q[m].double().view(heads, 128), k[seen]) * scale
+        if softcap:
+            s = softcap * (s / softcap).tanh()
+        out.append(torch.einsum("ht,thd->hd", s.softmax(dim=1), v[seen]).reshape(-1))
+    return torch.stack(out)
+
+
+@pytest.mark.parametrize("window,softcap,rows", [(0, 0.0, 1333), (256, 0.0, 2000), (1000, 50.0, 2000)])
+def test_window_prompt_probabilities(window, softcap, rows):
+    """Queries that bf16 holds, so that the probabilities are all that is rounded: two bf16 numbers each, 2^-17, and a tensor-core chain of at most
+    16 steps of 16 tokens that truncates by 2^-24 of the running sum each: 5e-5 covers both several times, one bf16 number (1e-3) misses it."""
+    call = _prompt(rows, 16, 4, softcap=softcap, window=window, bf16_queries=True)
+    got, some = call().double(), [0, 1, 127, 128, 129, 700, rows - 20, rows - 1]
+    want = _window_want(call, 16, 4, 128 ** -0.5, softcap, window, some)
+    assert (got[some] - want).norm() <= 5e-5 * want.norm()
