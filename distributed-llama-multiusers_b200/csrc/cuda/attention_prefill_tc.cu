@@ -422,13 +422,13 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
         }
         int pos_r, lb = 0;                                       // last and first visible position of this row
         float sc, c1 = 0.f, cap_k = 0.f, slope = 0.f;
-        bool shaped = false;                                     // scores leave the accumulator through a cap or a bias
+        bool shaped = false;                                     // scores leave the accumulator through a cap, a bias or a factor that is not positive
         if constexpr (LINES) {
             const DlWindowAttnArgs& w = a.w;
             pos_r = p0 + r_live / a.rep;
             if (w.window > 0) lb = max(0, pos_r - w.window + 1);
             if (w.chunk > 0) lb = max(lb, pos_r / w.chunk * w.chunk);
-            shaped = w.softcap > 0.f || w.slope != nullptr;
+            shaped = w.softcap > 0.f || w.slope != nullptr || !(w.scale > 0.f);      // (a factor that keeps no order meets the scores ahead of mask and maximum)
             sc = 1.4426950408889634f * w.scale;
             c1 = w.softcap > 0.f ? sc * 2.f / w.softcap : sc;
             cap_k = w.softcap * 1.4426950408889634f;

@@ -380,3 +380,13 @@ def test_window_prompt_probabilities(window, softcap, rows):
     got, some = call().double(), [0, 1, 127, 128, 129, 700, rows - 20, rows - 1]
     want = _window_want(call, 16, 4, 128 ** -0.5, softcap, window, some)
     assert (got[some] - want).norm() <= 5e-5 * want.norm()
+
+
+@pytest.mark.parametrize("scale", [-0.2, 0.0])
+def test_window_prompt_factor_without_order(scale):
+    """A score factor that is negative (the smallest product takes the weight) or zero (all positions alike)."""
+    rows = 700
+    call = _prompt(rows, 16, 4, scale=scale, window=300)
+    got, some = call().double(), [0, 1, 299, 300, 511, rows - 1]
+    want = _window_want(call, 16, 4, scale, 0.0, 300, some)
+    assert (got[some] - want).norm() <= 8e-3 * want.norm()
