@@ -138,11 +138,14 @@ template <bool LINES> DL_DEVINL uint32_t pt_pack2(float lo, float hi) {
 // per clock and SM (128 x 128 exp2 per step = 1024 clk, as long as the MMAs of the step), so every fourth element takes this
 // path instead
 template <bool LINES> DL_DEVINL float pt_ex2_poly(float x) {
-    const float xc = fmaxf(x, -126.0f);
+    float xc;                                      // LINES: a NaN stays one, as in the mma.sync kernel
+    if (LINES) asm("max.NaN.f32 %0, %1, %2;" : "=f"(xc) : "f"(x), "f"(-126.0f));
+    else xc = fmaxf(x, -126.0f);
     const float t = xc + 12582912.0f;              // 1.5 * 2^23: round(x) lands in the low mantissa bits
     const float f = xc - (t - 12582912.0f);        // [-0.5, 0.5]
     const float p = LINES ? fmaf(fmaf(fmaf(fmaf(fmaf(1.32764725e-3f, f, 9.67554096e-3f), f, 0.0555071309f), f, 0.240221202f), f, 0.693146944f), f, 1.00000012f)
                           : fmaf(fmaf(fmaf(0.0550886838f, f, 0.242604051f), f, 0.693276242f), f, 0.99992894f);
+    if (LINES) return p * __int_as_float((__float_as_int(t) << 23) + 0x3f800000);
     return __int_as_float(__float_as_int(p) + (__float_as_int(t) << 23));
 }
 

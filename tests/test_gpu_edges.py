@@ -390,3 +390,20 @@ def test_window_prompt_factor_without_order(scale):
     got, some = call().double(), [0, 1, 299, 300, 511, rows - 1]
     want = _window_want(call, 16, 4, scale, 0.0, 300, some)
     assert (got[some] - want).norm() <= 8e-3 * want.norm()
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+def test_window_prompt_non_finite_keys(value):
+    """A key that is not finite, at each place of a group of four: the rows that see it have no finite result (as on the mma.sync kernel), the
+    others are as without it."""
+    rows, window = 700, 150
+    clean = _prompt(rows, 16, 4, window=window)()
+    for at in (40, 41, 42, 43, 330):
+        def spoil(cache):
+            cache[at // 32, :, at % 32, :128] = value
+        out = _prompt(rows, 16, 4, window=window, keys=spoil)()
+        seen = torch.zeros(rows, dtype=torch.bool, device="cuda")
+        seen[at:at + window] = True
+        assert torch.equal(out[~seen], clean[~seen])
+        bad = ~torch.isfinite(out[seen].view(-1, 128)).all(dim=1)
+        assert bad.all() if value != value else bad.view(-1, 16).any(dim=1).float().mean() > 0.9
