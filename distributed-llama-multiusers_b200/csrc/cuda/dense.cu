@@ -1,9 +1,10 @@
 // Dense (unquantised) weights: embedding gather and  Y[M][N] = epi(X[M][K] . W[N][K]^T)  for bf16 or f32 weights,
-// f32 activations, f32 accumulation.  Two kernels: a weight-streaming one for up to 8 rows (decode: every weight
-// byte is read once, lanes stride K) and a shared-memory tiled one for more rows.  Both take a batch dimension
+// f32 activations, f32 accumulation.  Up to 8 rows a warp per output column streams its weight row (activations staged for
+// the CTA, or direct: dense_rows_staged), up to 32 in rounds of 8 or, in bf16 mode from 3 rows on, on mma.sync; more rows, or few columns and inputs
+// (dense_in_rounds), take a shared-memory tiled kernel.  All take a batch dimension
 // (grid.z) with element strides, which is how per-head products (a head's slice of a weight against a head's slice
 // of the activations) run as one launch.  In bf16 mode (`round_x`) the activation operand is rounded to bf16 on
-// load, so products are exact in f32 and only the accumulation order differs from a tensor-core product.
+// load, so products are exact in f32 and only the accumulation differs between the kernels.
 //
 // Epilogues (what other models of this library fuse into their matmul kernels too): plain store, relu(.)^2,
 // aux * sigmoid(.) (an output gate), cap * tanh(. / cap) (logit soft-capping), . * sigmoid(.) (SiLU), aux * (.) (the second
@@ -103,7 +104,7 @@ __global__ void __launch_bounds__(GV_WARPS * 32) dense_gemv_kernel(DlDenseArgs a
     }
 }
 
-// Vectorised variant: K % 8 == 0, rows 16-byte aligned (checked on the host).  One warp per output column (PAIR: per gated unit, its gate
+// Staged variant: K % 8 == 0, rows 16-byte aligned (checked on the host).  One warp per output column (PAIR: per gated unit, its gate
 // row and its up row), 8 weights per lane and load, a batch of U loads in flight while the last one is multiplied.
 // What bounds it: the weights' bytes, which takes many loads in flight and few instructions per weight -- so the CTA's eight warps share
 // the activations in shared memory, rounded once (each warp loaded, and rounded, all of them for itself: 8192 inputs x 2048 columns
@@ -127,6 +128,60 @@ template <> struct WVec<__nv_bfloat16> {
         }
     }
 };
+
+// Short weight rows, or very many of them: each warp loads the activations for itself, in a quarter of the staged kernel's registers, so that
+// the SMs hold four times the warps and a row's few loads need no barrier ahead of them (dense_rows_staged: where the line lies).  The same
+// products in the same order.
+template <typename WT, int MT, bool RX, bool PAIR>
+__global__ void __launch_bounds__(GV_WARPS * 32) dense_gemv_direct_kernel(DlDenseArgs a) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n = blockIdx.x * GV_WARPS + warp;
+    const int b = blockIdx.z;
+    if (PAIR ? 2 * n + 1 >= a.N : n >= a.N) return;
+    const WT* w0 = (const WT*)a.W + (size_t)b * a.w_bs + (size_t)(PAIR ? 2 * n : n) * a.ldw;
+    const WT* w1 = w0 + a.ldw;
+    const float* x = a.X + (size_t)b * a.x_bs;
+    float g[MT], h[MT];
+#pragma unroll
+    for (int m = 0; m < MT; ++m) g[m] = h[m] = 0.f;
+    for (int k = lane * 8; k < a.K; k += 256) {
+        WVec<WT> v0, v1;
+        float wg[8], wu[8];
+        v0.load(w0 + k);
+        if (PAIR) v1.load(w1 + k);
+        v0.get(wg);
+        if (PAIR) v1.get(wu);
+#pragma unroll
+        for (int m = 0; m < MT; ++m) {
+            if (m < a.M) {
+                WVec<float> xm;
+                float xv[8];
+                xm.load(x + (size_t)m * a.ldx + k);
+                xm.get(xv);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const float v = RX ? round_bf16(xv[i]) : xv[i];
+                    g[m] = fmaf(v, wg[i], g[m]);
+                    if (PAIR) h[m] = fmaf(v, wu[i], h[m]);
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+        g[m] = warp_sum(g[m]);
+        if (PAIR) h[m] = warp_sum(h[m]);
+    }
+    if (lane == 0) {
+#pragma unroll
+        for (int m = 0; m < MT; ++m) {
+            if (m < a.M) {
+                if (PAIR) dense_store_pair(a, b, m, n, g[m], h[m]);
+                else dense_store(a, b, m, n, g[m]);
+            }
+        }
+    }
+}
 
 template <typename WT, int MT, bool RX, bool PAIR>
 __global__ void __launch_bounds__(GV_WARPS * 32) dense_gemv_vec_kernel(DlDenseArgs a) {
@@ -474,13 +529,63 @@ __global__ void __launch_bounds__(256) dense_tile_kernel(DlDenseArgs a) {
     }
 }
 
+// Bytes of weights per warp from which the staged kernel is the faster one.  Its CTAs take half an SM's registers: one wave of them streams
+// more than the direct kernel from short rows on; every further wave waits for its activations again, where the direct kernel's many warps
+// hide each other's start (us, direct and staged, cold weights: one row of bf16, 2048 x 2048 5.8 and 3.4, 8192 x 4096 17.9 and 16.3, 8192 x 512 5.2 and 7.1,
+// 32768 x 2048 27.6 and 34.5, 65536 x 4096 93 and 98; two rows 8192 x 4096 22.4 and 23.4, 32768 x 8192 161 and 145; f32, one row 512 x 512 2.1 and
+// 2.1, four rows 2048 x 256 3.3 and 3.9, 2048 x 2048 9.2 and 7.7, 32768 x 4096 162 and 170; pairs of 8192 x 2048 in bf16 15.8 and 15.0,
+// of 32768 x 2048 43 and 45).  Waves are of 2 CTAs an SM: one, up to eight, more.
+static bool dense_rows_staged(const DlDenseArgs& a, int wsize, int mt, bool pair, long long ctas, int n_sms) {
+    static const int kb[4][3] = {{1, 8, 32}, {4, 16, 16}, {8, 32, 32}, {2, 16, 16}}, kb_pair[4][3] = {{1, 8, 32}, {4, 8, 16}, {4, 16, 16}, {1, 8, 8}};
+    const int r = mt == 1 ? 0 : mt == 2 ? 1 : mt == 4 ? 2 : 3, w = ctas <= 2ll * n_sms ? 0 : ctas <= 16ll * n_sms ? 1 : 2;
+    const int least = mt == 2 && w == 0 && wsize == 2 ? 1 : (pair ? kb_pair : kb)[r][w];
+    return (long long)a.K * wsize * (pair ? 2 : 1) >= least * 1024ll;
+}
+
+template <typename WT, int MT, bool RX>
+static void launch_dense_rows(const DlDenseArgs& a, cudaStream_t st, bool vec) {
+    const bool pair = a.epi == DL_DENSE_GLU_GELU;
+    const dim3 grid(((pair ? a.N / 2 : a.N) + GV_WARPS - 1) / GV_WARPS, 1, a.batch);
+    if (!vec) {
+        if (pair) dense_gemv_pair_kernel<WT, MT, RX><<<grid, GV_WARPS * 32, 0, st>>>(a);
+        else dense_gemv_kernel<WT, MT, RX><<<grid, GV_WARPS * 32, 0, st>>>(a);
+        return;
+    }
+    if constexpr (MT <= 2 || sizeof(WT) != 2 || !RX) {       // (more rows of these run on dense_mma_kernel, or 3 and 4 direct)
+        if (dense_rows_staged(a, sizeof(WT), MT, pair, (long long)grid.x * a.batch, dl_device_sm_count())) {
+            if (pair) launch_after(dense_gemv_vec_kernel<WT, MT, RX, true>, grid, GV_WARPS * 32, st, a);
+            else launch_after(dense_gemv_vec_kernel<WT, MT, RX, false>, grid, GV_WARPS * 32, st, a);
+            return;
+        }
+    }
+    if constexpr (MT <= 4 || sizeof(WT) != 2 || !RX) {
+        if (pair) dense_gemv_direct_kernel<WT, MT, RX, true><<<grid, GV_WARPS * 32, 0, st>>>(a);
+        else dense_gemv_direct_kernel<WT, MT, RX, false><<<grid, GV_WARPS * 32, 0, st>>>(a);
+    }
+}
+
+// 9 to 32 rows in rounds of 8, each of which streams the weights at their own pace, or in the tiles above (a scalar load per weight, most of 64
+// rows empty, but one launch)?  In f32, us by tile and by rounds: gate|up + down of 4096 x 14336 at 16 rows 3460 and 630, 2048 x 64 at 32 rows
+// 10.9 and 21.9, 8192 x 128 22 and 64, 16 x 2048 x 512 at 16 rows 133 and 160, at 9 133 and 104.  Both go by what these sweeps (64 to 8192 inputs, 64 to 131072
+// columns) fit, in ns: a round by its CTAs and their inputs, or by the length of one; the tiles by their steps of K, side by side on the SMs or in turn.
+static bool dense_in_rounds(const DlDenseArgs& a, int n_sms) {
+    const bool pair = a.epi == DL_DENSE_GLU_GELU;
+    const long long rounds = (a.M + 7) / 8, ctas = ((pair ? a.N / 2 : a.N) + GV_WARPS - 1) / GV_WARPS * (long long)a.batch;
+    const long long tiles = (a.N + GT_BN - 1) / GT_BN * (long long)a.batch, deep = tiles > n_sms ? tiles * 60 / n_sms : 60;
+    const long long by_ctas = ctas * (6 + (pair ? 34ll : 17ll) * a.K / 1000);
+    return rounds * (by_ctas > 4500 ? by_ctas : 4500) <= 5000 + a.K * (35 + deep);
+}
+
 template <typename WT, bool RX>
 static void launch_dense(const DlDenseArgs& a, cudaStream_t st) {
     const bool vec = a.K % 8 == 0 && a.ldw % 8 == 0 && a.w_bs % 8 == 0 && a.ldx % 4 == 0 && a.x_bs % 4 == 0 &&
                      ((uintptr_t)a.W & 15) == 0 && ((uintptr_t)a.X & 15) == 0;
+    const int n_sms = dl_device_sm_count();
     if constexpr (sizeof(WT) == 2 && RX) {
-        if (vec && a.M >= 3 && a.M <= 32) {
-            const int n_sms = dl_device_sm_count();
+        // with few steps of K most warps of an mma CTA idle: of very many columns, 3 and 4 rows go direct (us, direct and mma: 16 x 8192 x 256,
+        // 3 rows 51 and 75, 4 rows 60 and 75, 8 rows 115 and 78; 16 x 2048 x 512, 3 rows 21.9 and 21.5; 8192 x 256, 3 rows 5.7 and 3.8)
+        const bool direct = a.M <= 4 && a.K <= (a.M == 3 ? 512 : 256) && (long long)a.N * a.batch >= 128ll * n_sms;
+        if (vec && a.M >= 3 && a.M <= 32 && !direct) {
             if (a.M <= 8) launch_dense_mma<1>(a, st, n_sms);
             else if (a.M <= 16) launch_dense_mma<2>(a, st, n_sms);
             else launch_dense_mma<4>(a, st, n_sms);
@@ -488,21 +593,11 @@ static void launch_dense(const DlDenseArgs& a, cudaStream_t st) {
         }
     }
     if (a.M <= 8) {
-        const bool pair = a.epi == DL_DENSE_GLU_GELU;
-        dim3 grid(((pair ? a.N / 2 : a.N) + GV_WARPS - 1) / GV_WARPS, 1, a.batch);
-        const int mt = a.M <= 1 ? 1 : a.M <= 2 ? 2 : a.M <= 4 ? 4 : 8;
-#define GV_CASE(MT_)                                                                                   \
-    case MT_:                                                                                          \
-        if (vec && pair) launch_after(dense_gemv_vec_kernel<WT, MT_, RX, true>, grid, GV_WARPS * 32, st, a);        \
-        else if (vec) launch_after(dense_gemv_vec_kernel<WT, MT_, RX, false>, grid, GV_WARPS * 32, st, a);          \
-        else if (pair) dense_gemv_pair_kernel<WT, MT_, RX><<<grid, GV_WARPS * 32, 0, st>>>(a);                      \
-        else dense_gemv_kernel<WT, MT_, RX><<<grid, GV_WARPS * 32, 0, st>>>(a);                        \
-        break;
-        switch (mt) { GV_CASE(1) GV_CASE(2) GV_CASE(4) GV_CASE(8) }
-#undef GV_CASE
-    } else if (vec && a.M <= 32) {
-        // up to four rounds of 8 rows: each streams the weights at their own pace, which the tiles below (a scalar load per weight, most of 64
-        // rows empty) do not (gate|up + down of 4096 x 14336 in f32 at 16 rows: 3460 us there, 630 here)
+        if (a.M <= 1) launch_dense_rows<WT, 1, RX>(a, st, vec);
+        else if (a.M <= 2) launch_dense_rows<WT, 2, RX>(a, st, vec);
+        else if (a.M <= 4) launch_dense_rows<WT, 4, RX>(a, st, vec);
+        else launch_dense_rows<WT, 8, RX>(a, st, vec);
+    } else if (vec && a.M <= 32 && dense_in_rounds(a, n_sms)) {
         for (int m0 = 0; m0 < a.M; m0 += 8) {
             DlDenseArgs r = a;
             r.M = a.M - m0 < 8 ? a.M - m0 : 8;

@@ -16,6 +16,11 @@ def L():
     return layers
 
 
+def lib():
+    from dllama_b200.ops import lib
+    return lib
+
+
 @pytest.mark.parametrize("heads,kv,hs,n_splits", [(4, 1, 128, 1), (3, 1, 128, 4), (4, 2, 64, 1), (8, 2, 64, 3), (2, 2, 128, 2)])
 def test_decode_attention_half_pages(heads, kv, hs, n_splits):
     """Contexts around the borders of half pages, of the warps' turns and of the split rule (24 pages); an infinite key that a head's
@@ -407,3 +412,26 @@ def test_window_prompt_non_finite_keys(value):
         assert torch.equal(out[~seen], clean[~seen])
         bad = ~torch.isfinite(out[seen].view(-1, 128)).all(dim=1)
         assert bad.all() if value != value else bad.view(-1, 16).any(dim=1).float().mean() > 0.9
+
+
+@pytest.mark.parametrize("M,N,K_,batch,dtype", [(1, 40, 2048, 1, "bf16"), (1, 30000, 256, 1, "bf16"), (2, 24, 512, 3, "bf16"), (2, 9000, 128, 2, "f32"), (3, 20000, 264, 1, "bf16"),
+                                                (4, 1000, 256, 24, "bf16"), (4, 64, 4096, 1, "f32"), (8, 3000, 72, 8, "f32"), (32, 64, 64, 1, "f32"), (16, 2000, 64, 16, "f32"),
+                                                (25, 100, 520, 1, "f32")])
+def test_dense_rows_by_shape(M, N, K_, batch, dtype):
+    """Few rows on every side of the rules that choose between staged and direct rows, mma, rounds and tiles, plain and in pairs, one product and a
+    batch of them.  f32 sums of K terms: 3e-6."""
+    g = torch.Generator(device="cuda").manual_seed(M * 1000 + N)
+    w = (torch.randn(batch, N, K_, generator=g, device="cuda") * K_ ** -0.5).to(torch.bfloat16 if dtype == "bf16" else torch.float32)
+    x = torch.randn(M, batch * K_, generator=g, device="cuda")
+    z = torch.einsum("mbk,bnk->mbn", (x.bfloat16() if dtype == "bf16" else x).double().view(M, batch, K_), w.double())
+    for pair in (False, True):
+        width = N // 2 if pair else N
+        want = torch.nn.functional.gelu(z[..., 0::2], approximate="tanh") * z[..., 1::2] if pair else z
+        y = torch.zeros(M, batch * width, device="cuda")
+        a = lib().DlDenseArgs()
+        a.W, a.wtype, a.ldw, a.w_bs = w.data_ptr(), 1 if dtype == "bf16" else 0, K_, N * K_
+        a.X, a.ldx, a.x_bs, a.Y, a.ldy, a.y_bs = x.data_ptr(), batch * K_, K_, y.data_ptr(), batch * width, width
+        a.M, a.N, a.K, a.batch, a.round_x, a.epi = M, N, K_, batch, 1 if dtype == "bf16" else 0, L().DENSE_GLU_GELU if pair else 0
+        L().check_layers(L().layers_lib().dl_dense(a, torch.cuda.current_stream().cuda_stream), "dl_dense")
+        got = y.double().view(M, batch, width)
+        assert (got - want).norm() <= 3e-6 * want.norm()
