@@ -397,7 +397,6 @@ __global__ void __launch_bounds__(WS_THREADS, 1) gemm_wh_rows_kernel(const __gri
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ uint64_t full[16], empty[16], acc_full;
     __shared__ uint32_t tmem_holder;
-    const unsigned long long t0 = globaltimer_ns();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int S = a.S, KT = a.KT, NT = a.NT;
     const int crank = S > 1 ? (int)cg::this_cluster().block_rank() : 0;
@@ -419,6 +418,9 @@ __global__ void __launch_bounds__(WS_THREADS, 1) gemm_wh_rows_kernel(const __gri
     tc_fence_after();
     const uint32_t tmem = tmem_holder;
     pdl_launch_dependents();
+    // the waits' deadline runs from the end of the kernel ahead: this one may start long before it
+    if (warp != 0) pdl_wait();
+    unsigned long long t0 = globaltimer_ns();
 
     if (warp == 0) {
         // lane = one bulk copy per stage: pieces of the weights' row groups (cut at the image's 128-row tiles), then of the activations
@@ -449,6 +451,7 @@ __global__ void __launch_bounds__(WS_THREADS, 1) gemm_wh_rows_kernel(const __gri
         for (int i = 0; is_w && i < min(nk, a.NS); i++)
             asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src + (size_t)i * step), "r"(bytes) : "memory");
         pdl_wait();
+        t0 = globaltimer_ns();
         for (int i = 0; i < nk; i++) {
             const int s = i % a.NS;
             if (i >= a.NS) wt_wait(&empty[s], ((i / a.NS) & 1) ^ 1, t0);
@@ -523,7 +526,6 @@ __global__ void __launch_bounds__(WS_THREADS, 1) gemm_wh_rows_kernel(const __gri
         }
         cluster.sync();                                            // no peer still reads this CTA's memory when it leaves
     }
-    pdl_wait();
     const bool pair = a.epi.dense_op == DL_DENSE_GLU_CLAMP || a.epi.dense_op == DL_DENSE_GLU_SILU || a.epi.dense_op == DL_DENSE_GLU_GELU;
     const int na = pair ? rows >> 1 : rows, step = na ? max(1, WS_THREADS / na) : 1;      // threads along the columns, several rows at a time
     for (int t = tid; t < na * step; t += WS_THREADS)
