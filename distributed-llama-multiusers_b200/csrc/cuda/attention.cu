@@ -322,14 +322,16 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attention_kernel(const __grid_
 // What bounds it: the cache's bytes.  The FMA kernel above spends ~480 instructions per 8 tokens and warp (a 31-shuffle
 // reduction of the scores, four f32 conversions and shuffled weights per token) and keeps 7 warps per SM busy: 91 us at 32 rows
 // of 1500 to 3000 tokens (8 kv heads of 128), 3.3 TB/s.  Here a warp takes 16 tokens at a time through 32 MMAs: 54 us,
-// 5.5 TB/s, and the distance to a 64-bit result went from 4.5e-7 to 3.0e-7.
+// 5.5 TB/s, and the distance to a 64-bit result went from 4.5e-7 to 2.1e-7.
 //
-// Nothing is rounded to 16 bits: keys and values ARE fp16, and an f32 query (or softmax weight) is the exact sum of three fp16
-// numbers, q = q1 + q2 + q3 (11 bits each).  One 16-row MMA tile holds the splits of all four heads -- row h: q1 of head h,
-// row 4 + h: q2, row 8 + h: q3 -- so the three products cost no extra instruction, and summing three accumulator rows gives
-// the f32 product.  (The factors 2^6 on the queries and 2^12 on the weights keep the small parts out of fp16's subnormals.)
-// MMA accumulators are short-lived: 4 steps of K for a score, one step of 16 tokens for an output; both are then added to f32
-// registers with rounded adds, since a long MMA chain truncates.
+// Nothing is rounded to 16 bits: keys and values ARE fp16, and an f32 query (or softmax weight) is taken as three fp16 numbers,
+// q = q1 + 2^-11 q2 + 2^-22 q3 (11 bits each).  The second and third hold the remainders at a scale of their own, so that they do not fall into
+// fp16's subnormals ahead of the first: the sum is exact from 2^-23 of the scaled value on and off by 2^-47 at most below, 2^-53 of a score per
+// unit of key and 2^-62 of the largest weight.  One 16-row MMA tile holds the parts of all four heads -- row h: q1 of head h,
+// row 4 + h: q2, row 8 + h: q3 -- so the three products cost no extra instruction, and summing three accumulator rows, at their scales, gives the
+// f32 product.  An MMA truncates what it adds, so its chains are short: a quarter of K for a score (two MMAs at most), the quarters added in
+// pairs in f32, and 16 tokens for an output.  32 heads of 128 on 8, against 64 bits, the FMA kernel / this one / with chains of four:
+// 32 tokens 1.23e-7 / 1.23e-7 / 1.41e-7, 60 tokens 1.36e-7 / 1.38e-7 / 1.58e-7, 180 tokens 1.66e-7 / 1.55e-7 / 1.88e-7, 3000 tokens 3.29e-7 / 1.92e-7 / 2.19e-7.
 //
 // A warp walks its own 16-token half pages (w, w + 4, ...) through a private ring of cp.async stages, chunks of 16 bytes
 // XOR-swizzled by the token so ldmatrix is free of conflicts: no barrier between warps until the final merge.  Tokens past the
@@ -337,9 +339,9 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attention_kernel(const __grid_
 // splits is not what an f32 product gives) the warp takes its tokens again in plain f32.
 // ------------------------------------------------------------------------------------------------
 #define AM_TOK 16
-#define AM_Q_UP 64.0f                     // 2^6 on the queries
-#define AM_P_UP 4096.0f                   // 2^12 on the weights (a factor: added to the exponent ahead of exp2 it rounded the difference to 2^-21,
-                                          // 2.8e-7 against 64 bits at 180 tokens instead of the FMA kernel's 1.6e-7)
+#define AM_Q_UP 64.0f                     // 2^6 on the queries: fp16 holds them up to 8000 (beyond, an infinity: the plain f32 form)
+#define AM_P_UP 32768.0f                  // 2^15 on the weights, as high as fp16 goes (a factor: added to the exponent ahead of exp2 it rounds the difference)
+#define AM_PART 0x1p-11f                  // from one part to the next
 
 DL_DEVINL void am_cp16(uint32_t dst, const void* src, bool live) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(live ? 16 : 0) : "memory");
@@ -357,13 +359,16 @@ DL_DEVINL void am_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint
 }
 DL_DEVINL float am_exp2(float x) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
 DL_DEVINL uint32_t am_pack(__half a, __half b) { __half2 h = __halves2half2(a, b); return *reinterpret_cast<uint32_t*>(&h); }
-// the two fp16 parts of v that this lane's rows hold: row g (first part for g < 4, second for g >= 4) and row g + 8 (third / none)
-DL_DEVINL void am_split(float v, bool lower, __half& top, __half& bot) {
-    const __half h1 = __float2half_rn(v);
-    const float r1 = v - __half2float(h1);
-    const __half h2 = __float2half_rn(r1);
+// the fp16 parts of v0 and v1 that this lane's rows hold: row g (first part for g < 4, second for g >= 4) and row g + 8 (third / none)
+DL_DEVINL void am_split(float v0, float v1, bool lower, uint32_t& top, uint32_t& bot) {
+    const uint32_t h1 = am_pack(__float2half_rn(v0), __float2half_rn(v1));
+    const float2 f1 = __half22float2(*reinterpret_cast<const __half2*>(&h1));
+    const float r0 = (v0 - f1.x) * (1.f / AM_PART), r1 = (v1 - f1.y) * (1.f / AM_PART);
+    const uint32_t h2 = am_pack(__float2half_rn(r0), __float2half_rn(r1));
+    const float2 f2 = __half22float2(*reinterpret_cast<const __half2*>(&h2));
+    const uint32_t h3 = am_pack(__float2half_rn((r0 - f2.x) * (1.f / AM_PART)), __float2half_rn((r1 - f2.y) * (1.f / AM_PART)));
     top = lower ? h1 : h2;
-    bot = lower ? __float2half_rn(r1 - __half2float(h2)) : __ushort_as_half(0);
+    bot = lower ? h3 : 0u;
 }
 
 template <int HS>
@@ -438,11 +443,7 @@ __global__ void __launch_bounds__(ATT_WARPS * 32, 3) attention_mma_kernel(const 
     for (int k = 0; k < KS; ++k)
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
-            __half t0, b0, t1, b1;
-            am_split(head < G ? qr[k][u].x * scale : 0.f, lower, t0, b0);
-            am_split(head < G ? qr[k][u].y * scale : 0.f, lower, t1, b1);
-            qf[k][2 * u] = am_pack(t0, t1);
-            qf[k][2 * u + 1] = am_pack(b0, b1);
+            am_split(head < G ? qr[k][u].x * scale : 0.f, head < G ? qr[k][u].y * scale : 0.f, lower, qf[k][2 * u], qf[k][2 * u + 1]);
         }
     float o[NT][4];
 #pragma unroll
@@ -450,6 +451,7 @@ __global__ void __launch_bounds__(ATT_WARPS * 32, 3) attention_mma_kernel(const 
 #pragma unroll
         for (int e = 0; e < 4; ++e) o[n][e] = 0.f;
     float run_m = -INFINITY, run_l = 0.f;                      // of head g % 4; run_l: this lane's own tokens
+    const float s_up = (lower ? 1.f : AM_PART) / AM_Q_UP;      // row g's part of a score
 
     int st = 0;
     for (int i = 0; i < n_my; ++i) {
@@ -463,23 +465,31 @@ __global__ void __launch_bounds__(ATT_WARPS * 32, 3) attention_mma_kernel(const 
         asm volatile("cp.async.wait_group %0;" ::"n"(ST - 1) : "memory");
         __syncwarp();
         const uint32_t kb = ring + st * (2 * HALF), vb = kb + HALF;
-        // scores of 16 tokens: n-tile j = tokens 8 j ..; two short chains over K, then rounded adds
-        float c[2][2][4];
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-            for (int u = 0; u < 2; ++u)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) c[j][u][e] = 0.f;
+        // scores of 16 tokens: n-tile j = tokens 8 j ..; quarters of K, added in pairs
+        float c[2][4];
         {
             const int t = (lane & 7) + ((lane >> 4) << 3), c1 = (lane >> 3) & 1;
             const uint32_t base = kb + t * ROWB;
+            float x[2][2][4];
 #pragma unroll
             for (int k = 0; k < KS; ++k) {
+                const int u = k / (KS / 4);                    // quarter
+                if (k % (KS / 4) == 0) {
+#pragma unroll
+                    for (int j = 0; j < 2; ++j)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) x[u & 1][j][e] = 0.f;
+                }
                 uint32_t b[4];
                 am_ldm(b, base + (((2 * k + c1) ^ (t & 7)) << 4));
-                am_mma(c[0][k & 1], qf[k][0], qf[k][1], qf[k][2], qf[k][3], b[0], b[1]);
-                am_mma(c[1][k & 1], qf[k][0], qf[k][1], qf[k][2], qf[k][3], b[2], b[3]);
+                am_mma(x[u & 1][0], qf[k][0], qf[k][1], qf[k][2], qf[k][3], b[0], b[1]);
+                am_mma(x[u & 1][1], qf[k][0], qf[k][1], qf[k][2], qf[k][3], b[2], b[3]);
+                if (k == KS / 2 - 1 || k == KS - 1) {
+#pragma unroll
+                    for (int j = 0; j < 2; ++j)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) c[j][e] = k < KS / 2 ? x[0][j][e] + x[1][j][e] : c[j][e] + (x[0][j][e] + x[1][j][e]);
+                }
             }
         }
         const int left = t_end - pg0 * ATT_PAGE - (warp + ATT_WARPS * i) * AM_TOK;
@@ -489,9 +499,9 @@ __global__ void __launch_bounds__(ATT_WARPS * 32, 3) attention_mma_kernel(const 
         for (int j = 0; j < 2; ++j)
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-                float v = (c[j][0][e] + c[j][1][e]) + (c[j][0][e + 2] + c[j][1][e + 2]);      // rows g and g + 8
+                float v = fmaf(c[j][e + 2], AM_PART * AM_PART / AM_Q_UP, c[j][e] * s_up);     // rows g and g + 8
                 v += __shfl_xor_sync(0xffffffffu, v, 16);                                     // row g +- 4
-                v = (j * 8 + qd * 2 + e < left) ? v * (1.f / AM_Q_UP) : -INFINITY;
+                v = (j * 8 + qd * 2 + e < left) ? v : -INFINITY;
                 s[j * 2 + e] = v;
                 mx = fmaxf(mx, v);
             }
@@ -504,13 +514,9 @@ __global__ void __launch_bounds__(ATT_WARPS * 32, 3) attention_mma_kernel(const 
         float ps = 0.f;
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
-            __half t0, b0, t1, b1;
             const float p0 = am_exp2(s[2 * j] - m_use) * AM_P_UP, p1 = am_exp2(s[2 * j + 1] - m_use) * AM_P_UP;
             ps += p0 + p1;
-            am_split(p0, lower, t0, b0);
-            am_split(p1, lower, t1, b1);
-            pa[2 * j] = am_pack(t0, t1);
-            pa[2 * j + 1] = am_pack(b0, b1);
+            am_split(p0, p1, lower, pa[2 * j], pa[2 * j + 1]);
         }
         run_l = fmaf(run_l, corr, ps);
         {
@@ -535,13 +541,13 @@ __global__ void __launch_bounds__(ATT_WARPS * 32, 3) attention_mma_kernel(const 
     }
     run_l += __shfl_xor_sync(0xffffffffu, run_l, 1);
     run_l += __shfl_xor_sync(0xffffffffu, run_l, 2);
-    // row h + row 8 + h, then row 4 + h: lanes of g < 4 hold head g
+    // row h + 2^-22 row 8 + h, then 2^-11 row 4 + h: lanes of g < 4 hold head g
     bool bad = !(fabsf(run_l) < INFINITY);
 #pragma unroll
     for (int n = 0; n < NT; ++n)
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-            float v = o[n][e] + o[n][e + 2];
+            float v = fmaf(o[n][e + 2], AM_PART * AM_PART, lower ? o[n][e] : o[n][e] * AM_PART);
             v += __shfl_xor_sync(0xffffffffu, v, 16);
             o[n][e] = v;
             bad |= !(fabsf(v) < INFINITY);

@@ -435,3 +435,45 @@ def test_dense_rows_by_shape(M, N, K_, batch, dtype):
         L().check_layers(L().layers_lib().dl_dense(a, torch.cuda.current_stream().cuda_stream), "dl_dense")
         got = y.double().view(M, batch, width)
         assert (got - want).norm() <= 3e-6 * want.norm()
+
+
+def _decode_one(q, k, v, kv_heads):
+    """One row of decode attention over these keys and values [tokens][kv][hs] and its result in 64 bits."""
+    heads, hs, T = q.shape[0], q.shape[1], k.shape[0]
+    pages = (T + 31) // 32
+    kc, vc = (torch.zeros(pages * 32, kv_heads, hs, dtype=torch.float16) for _ in range(2))
+    kc[:T], vc[:T] = k.half(), v.half()
+    paged = [c.view(pages, 32, kv_heads, hs).transpose(1, 2).contiguous().cuda() for c in (kc, vc)]
+    y = torch.zeros(1, heads * hs, device="cuda")
+    scratch = torch.zeros(K().attention_scratch_bytes(1, heads, hs, 2), dtype=torch.uint8, device="cuda")
+    K().attention(q.reshape(1, -1).cuda(), 1, heads, kv_heads, hs, *paged, torch.tensor([T - 1], dtype=torch.int32, device="cuda"),
+                  torch.zeros(1, dtype=torch.int32, device="cuda"), torch.arange(pages, dtype=torch.int32, device="cuda").view(1, -1), pages, 2, scratch,
+                  None, None, 1, y)
+    kk, vv = (c[:T].double().repeat_interleave(heads // kv_heads, dim=1) for c in (kc, vc))
+    p = (torch.einsum("hd,thd->ht", q.double(), kk) * hs ** -0.5).softmax(dim=1)
+    return y.cpu().double().view(heads, hs), torch.einsum("ht,thd->hd", p, vv)
+
+
+@pytest.mark.parametrize("hs", [64, 128])
+@pytest.mark.parametrize("q_size,k_size", [(1.0, 1.0), (1e-3, 1e3), (1e-4, 1e4), (1e-5, 1e4), (2000.0, 1e-3)])
+def test_decode_attention_small_queries(hs, q_size, k_size):
+    """Queries far from 1 against keys that make up for it: f32 products keep 24 bits of each.  Bound: a score's terms add up to at most 20 here, so
+    its f32 sum is within a few 2^-24 of that, 2e-6, as the softmax and its sums are."""
+    g = torch.Generator().manual_seed(hs)
+    q, k, v = torch.randn(4, hs, generator=g) * q_size, torch.randn(300, 1, hs, generator=g) * k_size, torch.randn(300, 1, hs, generator=g)
+    got, want = _decode_one(q, k, v, 1)
+    assert (got - want).norm() <= 2e-6 * want.norm()
+
+
+@pytest.mark.parametrize("hs", [64, 128])
+@pytest.mark.parametrize("below", [13, 20, 30])
+def test_decode_attention_small_weights(hs, below):
+    """One token takes the weight and has no value; the others are 2^-below of it and make up the output.  f32 weights keep 24 bits each; a score
+    near -below in units of log2 is rounded to 2^-24 of itself, 2e-6 for 30, which is the largest share: 6e-6."""
+    g = torch.Generator().manual_seed(below)
+    q, k, v = torch.zeros(4, hs), torch.zeros(200, 1, hs), torch.randn(200, 1, hs, generator=g) * 1000
+    q[:, 0] = hs ** 0.5 * 0.6931471805599453
+    k[:, 0, 0] = -(below + torch.rand(200, generator=g))
+    k[7], v[7] = 0, 0
+    got, want = _decode_one(q, k, v, 1)
+    assert (got - want).norm() <= 6e-6 * want.norm()
