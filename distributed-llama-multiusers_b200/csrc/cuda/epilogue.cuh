@@ -58,6 +58,8 @@ DL_DEVINL float act_gelu(float x) {
 // rows.  A caller with several thread groups per tile passes (m_first, m_step) so group k handles
 // rows k, k+step, ...; everything a row needs from global memory (position, KV page) is fetched
 // once per warp by lane m and broadcast with shuffles, so the per-row loop has no dependent loads.
+// DL_EPI_DENSE has no shuffles and no lane per row, so with that kind alone `rows` may be any multiple
+// of 8 and M any number (gemm_wh_rows_kernel: up to 256 and 128).
 DL_DEVINL void epilogue_rows(const DlEpilogue& e, const float* out_s, int out_ld, int rows, int grow0, int d_real,
                              int M, int m0, int tid, int m_first = 0, int m_step = 1) {
     const int lane = tid & 31;

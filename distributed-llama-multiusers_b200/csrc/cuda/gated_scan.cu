@@ -23,10 +23,10 @@
 #define GT_GROUPS 32              // column groups of S per CTA of the token-by-token kernel (of 1 or 2 columns)
 
 // ------------------------------------------------------------------------------------------------
-// token by token: a CTA owns GT_COLS columns of one head's S; thread (column, dq) keeps the rows d with (d / 4) % 4 == dq of its
-// column (NR registers; rows in groups of four so that q, k and f leave shared memory as 16-byte words), the four threads
-// of a column are neighbouring lanes and sum their shares of y by two shuffles.  In the head form column `vdim` is n: its
-// value is 1 for every token and its output is den.
+// token by token: a CTA owns GT_GROUPS groups of CW columns (one or two: gated_two_columns) of one head's S; thread (group, dq) keeps the
+// rows d with (d / 4) % 4 == dq of its columns (NR registers each; rows in groups of four so that q, k and f leave shared memory as
+// 16-byte words), the four threads of a group are neighbouring lanes and sum their shares of y by two shuffles.  In the head form
+// column `vdim` is n: its value is 1 for every token and its output is den.
 //
 // Decoding (a row per sequence) is bound by the state's bytes, read and written once: what counts is how many of them an SM has in
 // flight.  The addresses of a thread's rows were kept from load to store, two registers each, so three CTAs fitted an SM (28.8 us for 32

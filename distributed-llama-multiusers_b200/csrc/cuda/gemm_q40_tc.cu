@@ -331,15 +331,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_q40_tc_kernel(const __grid
         }
     };
     if (S > 1) {
-        // split-K: every rank publishes its partial tile(s) in the rings' place, then sums and finishes ITS share of the activation rows
-        // over DSMEM, in rank order.  (One rank finishing all rows chunk by chunk took two cluster barriers and S - 1 remote reads of
-        // 16 KB per 32 rows.)
-        float* all_s = reinterpret_cast<float*>(smem);               // [P][NT][128]
+        // split-K (of a single row tile: pairs are for more row tiles than SMs): every rank publishes its partial tile in the rings' place, then
+        // sums and finishes ITS share of the activation rows over DSMEM, in rank order.  (One rank finishing all rows chunk by chunk took two
+        // cluster barriers and S - 1 remote reads of 16 KB per 32 rows.)
+        float* all_s = reinterpret_cast<float*>(smem);               // [NT][128]
         cg::cluster_group cluster = cg::this_cluster();
-        if (is_epi) {
-            for (int h = 0; h < P; h++)
-                for (int ch = 0; ch < n_chunks; ch++) drain(h, ch, all_s + ((size_t)h * NT + ch * TC_EPI_CHUNK) * 128);
-        }
+        if (is_epi)
+            for (int ch = 0; ch < n_chunks; ch++) drain(0, ch, all_s + (size_t)ch * TC_EPI_CHUNK * 128);
         tc_fence_before();
         cluster.sync();
         // a rank tells its peers that it has read their shares as soon as it has, ahead of its own epilogue: the barrier at the end then
@@ -349,26 +347,24 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_q40_tc_kernel(const __grid
         if (!is_epi || ms >= me) read_all();
         if (is_epi) {
             pdl_wait();
-            for (int h = 0; h < P; h++)
-                for (int mb = ms; mb < me; mb += TC_EPI_CHUNK) {
-                    const int mc = min(TC_EPI_CHUNK, me - mb);
-                    const size_t base = ((size_t)h * NT + mb) * 128;
-                    for (int idx = tid - 64; idx < mc * 32; idx += TC_DEQ_WARPS * 32) {
-                        float4 x[8];                            // S <= 8: the ranks' shares in flight together, summed in rank order
+            for (int mb = ms; mb < me; mb += TC_EPI_CHUNK) {
+                const int mc = min(TC_EPI_CHUNK, me - mb);
+                for (int idx = tid - 64; idx < mc * 32; idx += TC_DEQ_WARPS * 32) {
+                    float4 x[8];                            // S <= 8: the ranks' shares in flight together, summed in rank order
 #pragma unroll
-                        for (int c = 0; c < 8; c++)
-                            if (c < S) x[c] = *reinterpret_cast<const float4*>(cluster.map_shared_rank(all_s, c) + base + idx * 4);
-                        float4 v = x[0];
+                    for (int c = 0; c < 8; c++)
+                        if (c < S) x[c] = *reinterpret_cast<const float4*>(cluster.map_shared_rank(all_s, c) + (size_t)mb * 128 + idx * 4);
+                    float4 v = x[0];
 #pragma unroll
-                        for (int c = 1; c < 8; c++)
-                            if (c < S) { v.x += x[c].x; v.y += x[c].y; v.z += x[c].z; v.w += x[c].w; }
-                        reinterpret_cast<float4*>(out_s)[idx] = v;
-                    }
-                    asm volatile("bar.sync 1, 512;" ::: "memory");
-                    if (h == P - 1 && mb + TC_EPI_CHUNK >= me) read_all();
-                    epilogue_rows(a.epi, out_s, 128, 128, (rt + h) * 128, a.d_real, mc, m0 + mb, etid, eg, TC_GROUPS);
-                    asm volatile("bar.sync 1, 512;" ::: "memory");      // out_s is rewritten by the next round
+                    for (int c = 1; c < 8; c++)
+                        if (c < S) { v.x += x[c].x; v.y += x[c].y; v.z += x[c].z; v.w += x[c].w; }
+                    reinterpret_cast<float4*>(out_s)[idx] = v;
                 }
+                asm volatile("bar.sync 1, 512;" ::: "memory");
+                if (mb + TC_EPI_CHUNK >= me) read_all();
+                epilogue_rows(a.epi, out_s, 128, 128, rt * 128, a.d_real, mc, m0 + mb, etid, eg, TC_GROUPS);
+                asm volatile("bar.sync 1, 512;" ::: "memory");      // out_s is rewritten by the next round
+            }
         }
         asm volatile("barrier.cluster.wait.acquire;" ::: "memory");     // nobody leaves while a peer may still read its share
     } else if (is_epi) {
