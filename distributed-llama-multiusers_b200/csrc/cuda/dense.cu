@@ -283,16 +283,27 @@ __global__ void __launch_bounds__(GV_WARPS * 32) dense_gemv_vec_kernel(DlDenseAr
 //
 // What bounds it: the weights' bytes.  On CUDA cores every row adds 8 FMAs per 16 bytes of weights and lane, and from 9 rows the tiles
 // below (16 K steps of scalar loads) left the weights behind entirely: gate|up + down of 4096 x 14336 took 441 us at 8 rows and
-// 3150 us at 16; 118 and 153 us here.  (Two rows are faster one by one: 2048 x 8192, 39.5 us there, 43.3 here.)
+// 3150 us at 16; 118 and 145 us here.  (Two rows are faster one by one: 2048 x 8192, 39.5 us there, 43.3 here.)
 //
 // Weights go from global memory straight into the A fragments: a lane's 16 bytes are 8 consecutive inputs of row g, and the four pairs
 // fill k slots of two MMAs; the activations' 16 bytes of the same inputs fill the same slots, so no shuffle and no shared memory for the
 // weights.  A CTA owns 16 C columns; its eight warps split K, each staging its own activations (bf16, 128 inputs at a time), and meet in
-// shared memory at the end, summed in warp order.  An MMA chain truncates, so it is 4 steps long and ends in a rounded f32 add.
+// shared memory at the end, summed in warp order.
+//
+// An MMA truncates its sum, so none is chained to another: four are added in pairs, rounded, and the last sum keeps its rounding errors
+// (two-sum).  8 rows against 64 bits, 2^-24 = 6.0e-8 (one column per warp in f32 FMAs / chains of four / now): normal operands, 256 inputs
+// 5.6e-8 / 7.4e-8 / 6.1e-8, 512 inputs 6.3e-8 / 8.3e-8 / 5.8e-8, 2048 7.9e-8 / 9.4e-8 / 6.4e-8, 14336 1.6e-7 / 1.2e-7 / 1.1e-7; operands of one
+// sign, 512 inputs 3.3e-8 / 8.2e-8 / 3.3e-8, 2048 3.2e-8 / 8.5e-8 / 2.9e-8.  No slower: norm, gate|up and down of 4096 x 14336 at 8, 16 and 31 rows
+// 118.1, 153.3 and 244.7 us with the chains, 117.9, 145.2 and 237.8 now.
 // ------------------------------------------------------------------------------------------------
 #define DM_STEP 128                    // inputs staged at a time by a warp
 #define DM_LD (DM_STEP + 8)            // row stride of the staged activations (bf16): 16-byte reads of 8 rows without conflicts
 
+__device__ __forceinline__ void dense_two_sum(float& s, float& err, float x) {      // s + x, its rounding error (Knuth) added to err
+    const float t = s + x, b = t - s;
+    err += (s - (t - b)) + (x - b);
+    s = t;
+}
 __device__ __forceinline__ void dense_mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
@@ -352,7 +363,7 @@ __global__ void __launch_bounds__(256) dense_mma_kernel(DlDenseArgs a) {
         }
         __syncwarp();
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {                // halves of 64 inputs: four MMAs to a chain
+        for (int h = 0; h < 2; ++h) {                // halves of 64 inputs: four MMAs, added in pairs
             if (h == 0 || s + 1 < s1) fetch(nxt, k0 + (h + 1) * 64);
             uint4 x[2][NT];
 #pragma unroll
@@ -363,14 +374,16 @@ __global__ void __launch_bounds__(256) dense_mma_kernel(DlDenseArgs a) {
             for (int c = 0; c < C; ++c)
 #pragma unroll
                 for (int n = 0; n < NT; ++n) {
-                    float d[4] = {0.f, 0.f, 0.f, 0.f};
+                    float d[4][4];
 #pragma unroll
                     for (int p = 0; p < 2; ++p) {
-                        dense_mma_bf16(d, cur[p][c][0].x, cur[p][c][1].x, cur[p][c][0].y, cur[p][c][1].y, x[p][n].x, x[p][n].y);
-                        dense_mma_bf16(d, cur[p][c][0].z, cur[p][c][1].z, cur[p][c][0].w, cur[p][c][1].w, x[p][n].z, x[p][n].w);
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) d[2 * p][e] = d[2 * p + 1][e] = 0.f;
+                        dense_mma_bf16(d[2 * p], cur[p][c][0].x, cur[p][c][1].x, cur[p][c][0].y, cur[p][c][1].y, x[p][n].x, x[p][n].y);
+                        dense_mma_bf16(d[2 * p + 1], cur[p][c][0].z, cur[p][c][1].z, cur[p][c][0].w, cur[p][c][1].w, x[p][n].z, x[p][n].w);
                     }
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) acc[c][n][e] += d[e];
+                    for (int e = 0; e < 4; ++e) acc[c][n][e] += (d[0][e] + d[1][e]) + (d[2][e] + d[3][e]);
                 }
 #pragma unroll
             for (int p = 0; p < 2; ++p)
@@ -392,13 +405,15 @@ __global__ void __launch_bounds__(256) dense_mma_kernel(DlDenseArgs a) {
     const bool pair = a.epi == DL_DENSE_GLU_GELU;
     for (int i = threadIdx.x * 2; i < a.M * COLS; i += 512) {          // two neighbouring columns of a row
         const int m = i / COLS, n = n0 + (i - m * COLS);
-        float2 v = make_float2(0.f, 0.f);
+        float2 v = make_float2(0.f, 0.f), e = v;
 #pragma unroll
         for (int w = 0; w < 8; ++w) {
             const float2 p = *reinterpret_cast<const float2*>(red + w * PER + i);
-            v.x += p.x;
-            v.y += p.y;
+            dense_two_sum(v.x, e.x, p.x);
+            dense_two_sum(v.y, e.y, p.y);
         }
+        if (fabsf(e.x) < INFINITY) v.x += e.x;      // (of an infinite sum it is NaN)
+        if (fabsf(e.y) < INFINITY) v.y += e.y;
         if (pair) {
             if (n + 1 < a.N) dense_store_pair(a, b, m, n >> 1, v.x, v.y);
         } else {

@@ -437,6 +437,20 @@ def test_dense_rows_by_shape(M, N, K_, batch, dtype):
         assert (got - want).norm() <= 3e-6 * want.norm()
 
 
+@pytest.mark.parametrize("M,N,K_", [(3, 2048, 512), (8, 100, 2048), (16, 4096, 520), (31, 200, 8200)])
+def test_dense_mma_rounds_once(M, N, K_):
+    """Products of numbers of one sign, which nothing cancels: off by no more than one rounding to f32 (half a unit in the last place, 2^-24;
+    truncated sums chained to each other were off by 8e-8 to 9e-8).  An infinite sum stays infinite."""
+    g = torch.Generator(device="cuda").manual_seed(M * 1000 + N)
+    w, x = torch.randn(N, K_, generator=g, device="cuda").abs().bfloat16(), torch.randn(M, K_, generator=g, device="cuda").abs()
+    want, y = x.bfloat16().double() @ w.double().t(), torch.zeros(M, N, device="cuda")
+    L().dense(w, x, y, M, True)
+    assert (y - want).norm() <= 2.0 ** -24 * want.norm()
+    over, w[0], x[1, 5] = torch.zeros(M, N, device="cuda"), 0.5, float("inf")
+    L().dense(w, x, over, M, True)
+    assert over[1, 0] == float("inf") and not torch.isfinite(over[1]).any() and torch.equal(over[2, 1:], y[2, 1:])
+
+
 def _decode_one(q, k, v, kv_heads):
     """One row of decode attention over these keys and values [tokens][kv][hs] and its result in 64 bits."""
     heads, hs, T = q.shape[0], q.shape[1], k.shape[0]
