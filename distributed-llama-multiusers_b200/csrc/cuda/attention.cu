@@ -321,17 +321,19 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attention_kernel(const __grid_
 //
 // What bounds it: the cache's bytes.  The FMA kernel above spends ~480 instructions per 8 tokens and warp (a 31-shuffle
 // reduction of the scores, four f32 conversions and shuffled weights per token) and keeps 7 warps per SM busy: 91 us at 32 rows
-// of 1500 to 3000 tokens (8 kv heads of 128), 3.3 TB/s.  Here a warp takes 16 tokens at a time through 32 MMAs: 54 us,
-// 5.5 TB/s, and the distance to a 64-bit result went from 4.5e-7 to 2.1e-7.
+// of 1500 to 3000 tokens (8 kv heads of 128), 3.3 TB/s.  Here a warp takes 16 tokens at a time through 32 MMAs: 53 us,
+// 5.6 TB/s, and the distance to a 64-bit result went from 4.4e-7 to 1.9e-7.
 //
 // Nothing is rounded to 16 bits: keys and values ARE fp16, and an f32 query (or softmax weight) is taken as three fp16 numbers,
-// q = q1 + 2^-11 q2 + 2^-22 q3 (11 bits each).  The second and third hold the remainders at a scale of their own, so that they do not fall into
-// fp16's subnormals ahead of the first: the sum is exact from 2^-23 of the scaled value on and off by 2^-47 at most below, 2^-53 of a score per
-// unit of key and 2^-62 of the largest weight.  One 16-row MMA tile holds the parts of all four heads -- row h: q1 of head h,
-// row 4 + h: q2, row 8 + h: q3 -- so the three products cost no extra instruction, and summing three accumulator rows, at their scales, gives the
-// f32 product.  An MMA truncates what it adds, so its chains are short: a quarter of K for a score (two MMAs at most), the quarters added in
-// pairs in f32, and 16 tokens for an output.  32 heads of 128 on 8, against 64 bits, the FMA kernel / this one / with chains of four:
-// 32 tokens 1.23e-7 / 1.23e-7 / 1.41e-7, 60 tokens 1.36e-7 / 1.38e-7 / 1.58e-7, 180 tokens 1.66e-7 / 1.55e-7 / 1.88e-7, 3000 tokens 3.29e-7 / 1.92e-7 / 2.19e-7.
+// q = q1 + 2^-7 q2 + 2^-14 q3, of 8 bits each.  The second and third hold the remainders at a scale of their own, so that they do not fall into
+// fp16's subnormals ahead of the first: the sum is exact from 2^-15 of the scaled value on and off by 2^-39 at most below, 2^-45 of a score per
+// unit of key and 2^-54 of the largest weight.  One 16-row MMA tile holds the parts of all four heads -- row h: q1 of head h,
+// row 4 + h: q2, row 12 + h: q3 -- so the three products cost no extra instruction, and summing three accumulator rows, the small ones first,
+// gives the f32 product.  An MMA truncates what it adds.  So parts have 8 bits and not the 11 that fp16 holds: a product with an fp16 number
+// then has 19, and a sum of 16 of them loses little or nothing; and chains are short: a quarter of K for a score (two MMAs at most), the
+// quarters added in pairs in f32, and 16 tokens for an output.  32 heads of 128 on 8, against 64 bits, the FMA kernel / parts of 11 bits /
+// this one: up to 40 tokens 1.26e-7 / 1.30e-7 / 1.19e-7, up to 400 2.06e-7 / 1.66e-7 / 1.54e-7, up to 3000 3.34e-7 / 1.95e-7 / 1.84e-7; 32 rows of 1500 to
+// 3000 tokens 54.1 us with parts of 11 bits, 53.2 now.
 //
 // A warp walks its own 16-token half pages (w, w + 4, ...) through a private ring of cp.async stages, chunks of 16 bytes
 // XOR-swizzled by the token so ldmatrix is free of conflicts: no barrier between warps until the final merge.  Tokens past the
@@ -341,7 +343,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attention_kernel(const __grid_
 #define AM_TOK 16
 #define AM_Q_UP 64.0f                     // 2^6 on the queries: fp16 holds them up to 8000 (beyond, an infinity: the plain f32 form)
 #define AM_P_UP 32768.0f                  // 2^15 on the weights, as high as fp16 goes (a factor: added to the exponent ahead of exp2 it rounds the difference)
-#define AM_PART 0x1p-11f                  // from one part to the next
+#define AM_PART 0x1p-7f                   // from one part to the next
 
 DL_DEVINL void am_cp16(uint32_t dst, const void* src, bool live) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(live ? 16 : 0) : "memory");
@@ -359,16 +361,17 @@ DL_DEVINL void am_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint
 }
 DL_DEVINL float am_exp2(float x) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
 DL_DEVINL uint32_t am_pack(__half a, __half b) { __half2 h = __halves2half2(a, b); return *reinterpret_cast<uint32_t*>(&h); }
-// the fp16 parts of v0 and v1 that this lane's rows hold: row g (first part for g < 4, second for g >= 4) and row g + 8 (third / none)
+// the fp16 parts of v0 and v1 that this lane's rows hold: row g (first part for g < 4, second for g >= 4) and row g + 8 (none / third)
+DL_DEVINL float am_top8(float v) { return __uint_as_float(__float_as_uint(v) & 0xFFFF0000u); }      // 8 significant bits
 DL_DEVINL void am_split(float v0, float v1, bool lower, uint32_t& top, uint32_t& bot) {
-    const uint32_t h1 = am_pack(__float2half_rn(v0), __float2half_rn(v1));
+    const uint32_t h1 = am_pack(__float2half_rn(am_top8(v0)), __float2half_rn(am_top8(v1)));
     const float2 f1 = __half22float2(*reinterpret_cast<const __half2*>(&h1));
     const float r0 = (v0 - f1.x) * (1.f / AM_PART), r1 = (v1 - f1.y) * (1.f / AM_PART);
-    const uint32_t h2 = am_pack(__float2half_rn(r0), __float2half_rn(r1));
+    const uint32_t h2 = am_pack(__float2half_rn(am_top8(r0)), __float2half_rn(am_top8(r1)));
     const float2 f2 = __half22float2(*reinterpret_cast<const __half2*>(&h2));
     const uint32_t h3 = am_pack(__float2half_rn((r0 - f2.x) * (1.f / AM_PART)), __float2half_rn((r1 - f2.y) * (1.f / AM_PART)));
     top = lower ? h1 : h2;
-    bot = lower ? h3 : 0u;
+    bot = lower ? 0u : h3;
 }
 
 template <int HS>
@@ -541,7 +544,7 @@ __global__ void __launch_bounds__(ATT_WARPS * 32, 3) attention_mma_kernel(const 
     }
     run_l += __shfl_xor_sync(0xffffffffu, run_l, 1);
     run_l += __shfl_xor_sync(0xffffffffu, run_l, 2);
-    // row h + 2^-22 row 8 + h, then 2^-11 row 4 + h: lanes of g < 4 hold head g
+    // 2^-7 row 4 + h + 2^-14 row 12 + h, then row h: lanes of g < 4 hold head g
     bool bad = !(fabsf(run_l) < INFINITY);
 #pragma unroll
     for (int n = 0; n < NT; ++n)

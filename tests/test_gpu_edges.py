@@ -480,6 +480,27 @@ def test_decode_attention_small_queries(hs, q_size, k_size):
 
 
 @pytest.mark.parametrize("hs", [64, 128])
+@pytest.mark.parametrize("tokens", [16, 40, 300])
+def test_decode_attention_as_exact_as_f32(hs, tokens):
+    """128 rows over as many tokens each: no further from 64 bits than the f32 arithmetic that a cache of f32 takes on the same numbers."""
+    M, heads, kv, pages = 128, 32, 8, (tokens + 31) // 32
+    g = torch.Generator(device="cuda").manual_seed(hs + tokens)
+    q = torch.randn(M, heads * hs, generator=g, device="cuda")
+    k, v = (torch.randn(M * pages, kv, 32, hs, generator=g, device="cuda").half() for _ in range(2))
+    bt, slot = torch.arange(M * pages, dtype=torch.int32, device="cuda").view(M, pages), torch.arange(M, dtype=torch.int32, device="cuda")
+    scratch = torch.zeros(K().attention_scratch_bytes(M, heads, hs, 1), dtype=torch.uint8, device="cuda")
+    kk, vv = (c.double().view(M, pages, kv, 32, hs).transpose(2, 3).reshape(M, -1, kv, hs)[:, :tokens].repeat_interleave(heads // kv, dim=2) for c in (k, v))
+    want = torch.einsum("mht,mthd->mhd", (torch.einsum("mhd,mthd->mht", q.double().view(M, heads, hs), kk) * hs ** -0.5).softmax(dim=2), vv).reshape(M, -1)
+    off = []
+    for cast in (torch.half, torch.float):
+        y = torch.zeros(M, heads * hs, device="cuda")
+        K().attention(q, M, heads, kv, hs, k.to(cast), v.to(cast), torch.full((M,), tokens - 1, dtype=torch.int32, device="cuda"), slot, bt, pages, 1, scratch,
+                      None, None, M, y)
+        off.append(float((y - want).norm() / want.norm()))
+    assert off[0] <= off[1], off
+
+
+@pytest.mark.parametrize("hs", [64, 128])
 @pytest.mark.parametrize("below", [13, 20, 30])
 def test_decode_attention_small_weights(hs, below):
     """One token takes the weight and has no value; the others are 2^-below of it and make up the output.  f32 weights keep 24 bits each; a score
