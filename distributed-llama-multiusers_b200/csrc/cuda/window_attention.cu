@@ -579,11 +579,11 @@ __global__ void __launch_bounds__(128, 4) window_attention_mma_kernel(DlWindowAt
     if (n_rows * rep <= 16) {            // decoding: one 16-row tile, the warps share the tokens
         if (only_small && (tile & 1) && window_tiles_join(a, tile_rows, rq, tile - 1, window_tile_count(tile_rows, gridDim.x, rq, tile - 1), n_rows))
             return;                      // the end of a prompt: attention_prefill_tc.cu takes it along with the full tile ahead of it
-        if (pg_lo > pg_hi) {             // a share without pages (of several): it weighs nothing
+        if (pg_lo > pg_hi) {             // a share without pages (of several): the merge leaves it out by its sum
             if (threadIdx.x < n_rows * rep) {
                 float* dst = partial + ((((size_t)tile * a.kv_heads + g) * n_splits + blockIdx.z) * WM_ROWS + threadIdx.x) * (D + 2) + D;
                 dst[0] = -INFINITY;
-                dst[1] = 0.f;
+                dst[1] = -1.f;
             }
             return;
         }
@@ -763,25 +763,25 @@ __global__ void __launch_bounds__(128) window_merge_kernel(DlWindowAttnArgs a, c
     for (int hg = threadIdx.x >> 5; hg < rep; hg += blockDim.x >> 5) {        // a warp per head, a lane per share
         const int k = threadIdx.x & 31;
         const float* p = base + ((size_t)k * WM_ROWS + r * rep + hg) * (D + 2) + D;
-        const float mk = k < n_splits ? p[0] : -INFINITY, lk = k < n_splits ? p[1] : 0.f;
+        const float mk = k < n_splits ? p[0] : -INFINITY, lk = k < n_splits ? p[1] : -1.f;
         const float sink = a.sink ? a.sink[g * rep + hg] : 0.f, gate = a.gate ? sigmoid_f(a.gate[(size_t)m * a.ld_gate + g * rep + hg]) : 1.f;
         const float mx = warp_max(mk), e = mk == -INFINITY ? 0.f : expf(mk - mx);
-        float l = warp_sum(lk * e);
+        float l = warp_sum(lk < 0.f ? 0.f : lk * e);
         if (a.sink) l += expf(sink - mx);
-        if (k < n_splits) w_s[hg * n_splits + k] = e * (gate / l);
+        if (k < n_splits) w_s[hg * n_splits + k] = lk < 0.f ? -1.f : e * (gate / l);
     }
     __syncthreads();
     for (int idx = threadIdx.x; idx < rep * D; idx += blockDim.x) {
         const int hg = idx / D, c = idx - hg * D;
         const float* p = base + (size_t)(r * rep + hg) * (D + 2) + c;
-        float acc = 0.f;                      // a share without pages weighs 0, whatever it left: sixteen shares are in flight at once
+        float acc = 0.f;                      // sixteen shares are in flight at once; those without pages (-1) have left nothing to read
         for (int k0 = 0; k0 < n_splits; k0 += 16) {
             float v[16];
 #pragma unroll
             for (int k = 0; k < 16; ++k) v[k] = k0 + k < n_splits ? p[(size_t)(k0 + k) * WM_ROWS * (D + 2)] : 0.f;
 #pragma unroll
             for (int k = 0; k < 16; ++k)
-                if (k0 + k < n_splits && w_s[hg * n_splits + k0 + k] != 0.f) acc = fmaf(w_s[hg * n_splits + k0 + k], v[k], acc);
+                if (k0 + k < n_splits && !(w_s[hg * n_splits + k0 + k] < 0.f)) acc = fmaf(w_s[hg * n_splits + k0 + k], v[k], acc);
         }
         a.out[(size_t)m * a.ldo + (size_t)(g * rep + hg) * D + c] = acc;
     }

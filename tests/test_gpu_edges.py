@@ -512,3 +512,29 @@ def test_decode_attention_small_weights(hs, below):
     k[7], v[7] = 0, 0
     got, want = _decode_one(q, k, v, 1)
     assert (got - want).norm() <= 6e-6 * want.norm()
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+def test_window_decode_non_finite_values_far_below(value):
+    """A value that is not finite, under a weight that a share's merge rounds to zero, on shares with and without pages: the column that it stands in is not
+    finite (0 times it), and no other column changes."""
+    heads, kv, dim, tokens, n_splits = 8, 2, 128, 300, 16
+    g = torch.Generator(device="cuda").manual_seed(5)
+    pages = (tokens + 31) // 32
+    cache = torch.randn(pages, kv, 32, 2 * dim, generator=g, device="cuda").bfloat16()
+    q = torch.ones(1, heads * dim, device="cuda")
+    cache[0, :, :, :dim] = -2.0                    # the first page: scores of -256, the others' some 10
+    rq = L().window_tc_rows(heads, kv)
+    tiles = torch.full((1, rq), -1, dtype=torch.int32, device="cuda")
+    tiles[0, 0] = 0
+    pos, slot, bt = (torch.tensor(v, dtype=torch.int32, device="cuda") for v in ([tokens - 1], [0], [list(range(pages))]))
+    partial, outs = torch.full((kv * n_splits * 64 * (dim + 2),), float("nan"), device="cuda"), []
+    for bad in (False, True):
+        if bad:
+            cache[0, 1, 7, dim + 3] = value
+        outs.append(torch.zeros(1, heads * dim, device="cuda"))
+        L().window_attention_tc(q, outs[-1], heads, kv, dim, 0, 1.0, 0.0, 0, pos, slot, bt, cache, tiles, 1, rq, n_splits, partial, vdim=dim)
+    clean, out = (o.view(kv, heads // kv, dim) for o in outs)
+    assert torch.isfinite(clean).all() and not torch.isfinite(out[1, :, 3]).any()
+    out[1, :, 3] = clean[1, :, 3]
+    assert torch.equal(out, clean)
