@@ -140,8 +140,11 @@ extern "C" int dl_embedding(const float* table, const int* tokens, float* x, int
 // ------------------------------------------------------------------------------------------------
 #define RNQ_THREADS 512
 #define RNQ_MAX_PER_THREAD 32     // dim <= 512*32 = 16384
-// From here on 8 rows per CTA: 148 CTAs, one for every SM.  Below, fewer cannot pull as much (width 4096, the kernel alone: 512 rows 6.7 us with a
-// row per CTA, 10.2 with 8; norm and feed-forward at 1024 rows 427 and 430); above, whole lines of the image count (2048 rows 783 and 769).
+// From here on 8 rows per CTA, which takes a whole SM: 148 CTAs, one for every SM.  Below, fewer cannot pull as much (512 rows of 4096, the
+// kernel alone: 6.7 us with a row per CTA, 10.2 with 8).  Above it goes by waves of 1184 rows: whole lines of the image win in full ones and a
+// barely begun one loses (norm and feed-forward, us with a row per CTA and with 8: width 2048, 1184 rows 271 and 267, 1300 310 and 314, 1536
+// 314 and 314, 2048 352 and 347; width 4096 567 and 561..566, 644 and 653, 657 and 661, 802..805 and 797..801; the kernel alone, 4096 wide,
+// 1300 rows 18.5 and 26.6, 2048 25.4 and 26.7, 2368 28.8 and 26.8).
 #define RNQ_WIDE_ROWS 1184
 
 struct RnqArgs {
@@ -166,8 +169,8 @@ struct RnqArgs {
 // Four lanes hold a 32-block: lane c its elements 4c .. 4c + 3 and 16 + 4c .. 16 + 4c + 3, which are one 16-byte chunk of the XH image.  A
 // warp is 8 such blocks: of 8 rows side by side (ROWS = 8, many rows: a chunk of the 8 rows is one whole 128-byte line of the image), or
 // 8 neighbouring blocks of one row (ROWS = 1: a CTA per row).  The merged row stays in registers between the two passes.
-// What bounds it: bytes (x, partial sums, image) for many rows, latency for few.  One thread per block, 128 bytes apart, as it was:
-// a feed-forward block of 2048 rows of 4096 took 846 us with it and 832 with this; 32 rows are as fast either way.
+// What bounds it: bytes (x, partial sums, image) for many rows, latency for few.  With one thread per block, 128 bytes apart, 2048 rows of
+// 4096 took 55.4 us alone, 512 rows 18.3; 25.4 (26.7 with 8 rows per CTA) and 9.3 with this.  32 rows are as fast either way (9 us).
 template <int ROWS>
 __global__ void __launch_bounds__(RNQ_THREADS) reduce_norm_quant_kernel(const __grid_constant__ RnqArgs a) {
     trace_begin(a.tr);

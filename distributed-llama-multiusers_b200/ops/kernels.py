@@ -361,8 +361,10 @@ def choose_tc_split(d: int, n: int, M: int, n_sms: int) -> int:
     row_tiles = (d + 127) // 128
     nt = 16 if M <= 16 else 32 if M <= 32 else 64 if M <= 64 else 128
     m_tiles = (M + nt - 1) // nt
-    # wide tiles reduce one 32-row chunk at a time over DSMEM (two cluster syncs per chunk): only worth it when
-    # every CTA still keeps a long k-loop (measured: w2 with 112 k-tiles gains 1.5x at S=4, qkv/wo with 32 lose)
+    # from 33 rows on a share keeps a long k-loop.  The line was drawn when one rank summed and finished all rows, two cluster barriers per
+    # 32 of them (4096 x 4096 at 64 rows: 18.4 us whole, 15.8 / 20.0 in 2 / 4 shares).  Every rank finishes rows of its own now and shorter
+    # shares would pay too (18.4, 14.4 / 12.8; 6144 x 4096 18.5 and 16.2 in 2), eight of them not (2048 x 2048 12.3 whole, 10.2 in 4, 16.9 in 8),
+    # so the line costs time where it forbids a split, and none where it allows one (4096 x 14336 45.2 whole, 20.6 in 4)
     min_kt = 1 if M <= 32 else 24
     S = 1
     while row_tiles * m_tiles * S * 2 <= n_sms and S < 8 and (n // 128) // (S * 2) >= min_kt:
