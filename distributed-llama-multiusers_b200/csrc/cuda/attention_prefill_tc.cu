@@ -39,16 +39,18 @@
 // (src/llm.cpp:296-301).  KV cache: fp16 pages [page][kv_head][32][128].
 #include <cuda.h>
 #include "epilogue.cuh"
+#include "f32_pairs.cuh"
 #include "window_tiles.cuh"
 
 #define PT_HS 128
 #define PT_ROWS 128
 #define PT_KV 128                      // tokens per step
-#define PT_THREADS 384
+#define PT_THREADS 512
 #define PT_MAX_SEG 8
 #define PT_TILE_BYTES 32768            // 128 x 128 fp16
-#define PT_STAGES 3                    // KV tiles in flight (K + V: 64 KB each)
-#define PT_OUT_LD 129
+#define PT_STAGES 2                    // K tiles and V tiles in flight
+#define PT_OUT_LD 20
+#define PT_SHARE_STEPS 4
 #define PT_DEADLINE_NS 4000000000ull
 
 struct PtArgs {
@@ -64,8 +66,6 @@ struct PtArgs {
     uint8_t* xh_out;
     int out_mcap;
     float* y_out;
-    long long* stamps;         // debug: clock64 stamps of CTA (0, 0), [tile][8]
-    int dbg;                   // timing experiments (results invalid): 1 = no softmax arithmetic, 2 = no KV copies, 4 = no MMAs
     unsigned long long* tr;
 };
 
@@ -73,16 +73,12 @@ struct PtLineArgs {
     DlWindowAttnArgs w;
     const int* tile_rows;      // [n_tiles][rq], -1 where a tile has fewer rows
     int n_tiles, rq, rep;
+    int group;                 // list tiles that one CTA may take: 2 or 4
+    float* partial;            // [n_tiles][kv_heads][grid.z][64][130] where grid.z > 1: sums, reference maximum, sum of weights
 };
 template <bool LINES> struct PtKernelArgs { typedef PtArgs T; };
 template <> struct PtKernelArgs<true> { typedef PtLineArgs T; };
 
-DL_DEVINL void pt_wait(uint64_t* bar, uint32_t parity, unsigned long long t0) {
-    unsigned n = 0;
-    while (!mbar_try_wait(bar, parity)) {
-        if ((++n & 0x3FFu) == 0 && globaltimer_ns() - t0 > PT_DEADLINE_NS) __trap();
-    }
-}
 DL_DEVINL void tmem_ld_32x32b_x32(uint32_t taddr, uint32_t (&v)[32]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, "
@@ -114,11 +110,6 @@ DL_DEVINL uint32_t pt_idesc(int M, int N, int b_mn_major, bool bf16) {
     d |= (uint32_t)(M >> 4) << 24;
     return d;
 }
-#define PT_STAMP(slot, j) do { if constexpr (!LINES) { if (a.stamps && blockIdx.x == 0 && blockIdx.y == 0 && (j) < 64) a.stamps[(j) * 8 + (slot)] = clock64(); } } while (0)
-#define PT_DBG(bit) (pt_dbg(a) & (bit))
-DL_DEVINL int pt_dbg(const PtArgs& a) { return a.dbg; }
-DL_DEVINL int pt_dbg(const PtLineArgs&) { return 0; }
-
 DL_DEVINL float pt_ex2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -137,35 +128,53 @@ template <bool LINES> DL_DEVINL uint32_t pt_pack2(float lo, float hi) {
 // 5e-4, right after; LINES, whose other kernels form it in full: degree 5, 2e-7): the softmax is bound by the 16 MUFU results
 // per clock and SM (128 x 128 exp2 per step = 1024 clk, as long as the MMAs of the step), so every fourth element takes this
 // path instead
-template <bool LINES> DL_DEVINL float pt_ex2_poly(float x) {
-    float xc;                                      // LINES: a NaN stays one, as in the mma.sync kernel
-    if (LINES) asm("max.NaN.f32 %0, %1, %2;" : "=f"(xc) : "f"(x), "f"(-126.0f));
-    else xc = fmaxf(x, -126.0f);
-    const float t = xc + 12582912.0f;              // 1.5 * 2^23: round(x) lands in the low mantissa bits
-    const float f = xc - (t - 12582912.0f);        // [-0.5, 0.5]
-    const float p = LINES ? fmaf(fmaf(fmaf(fmaf(fmaf(1.32764725e-3f, f, 9.67554096e-3f), f, 0.0555071309f), f, 0.240221202f), f, 0.693146944f), f, 1.00000012f)
-                          : fmaf(fmaf(fmaf(0.0550886838f, f, 0.242604051f), f, 0.693276242f), f, 0.99992894f);
-    if (LINES) return p * __int_as_float((__float_as_int(t) << 23) + 0x3f800000);
-    return __int_as_float(__float_as_int(p) + (__float_as_int(t) << 23));
+template <bool LINES> DL_DEVINL pair_f pt_ex2_poly(pair_f x) {
+    float lo, hi;                                  // LINES: a NaN stays one, as in the mma.sync kernel
+    pair_get(x, lo, hi);
+    if (LINES) {
+        asm("max.NaN.f32 %0, %0, %1;" : "+f"(lo) : "f"(-126.0f));
+        asm("max.NaN.f32 %0, %0, %1;" : "+f"(hi) : "f"(-126.0f));
+    } else {
+        lo = fmaxf(lo, -126.0f);
+        hi = fmaxf(hi, -126.0f);
+    }
+    auto both = [](float c) { return pair_of(c, c); };
+    const pair_f xc = pair_of(lo, hi), t = add2(xc, both(12582912.0f));                 // 1.5 * 2^23: round(x) lands in the low mantissa bits
+    const pair_f f = fma2(add2(t, both(-12582912.0f)), both(-1.0f), xc);                // [-0.5, 0.5]
+    float tl, th, pl, ph;
+    pair_get(t, tl, th);
+    if (LINES) {
+        const pair_f p = fma2(fma2(fma2(fma2(fma2(both(1.32764725e-3f), f, both(9.67554096e-3f)), f, both(0.0555071309f)), f, both(0.240221202f)), f, both(0.693146944f)), f, both(1.00000012f));
+        return mul2(p, pair_of(__int_as_float((__float_as_int(tl) << 23) + 0x3f800000), __int_as_float((__float_as_int(th) << 23) + 0x3f800000)));
+    }
+    pair_get(fma2(fma2(fma2(both(0.0550886838f), f, both(0.242604051f)), f, both(0.693276242f)), f, both(0.99992894f)), pl, ph);
+    return pair_of(__int_as_float(__float_as_int(pl) + (__float_as_int(tl) << 23)), __int_as_float(__float_as_int(ph) + (__float_as_int(th) << 23)));
 }
 
-// 32 scores (masked ones are -inf) -> exp2(s * sc - ref) as 16 packed fp16 pairs into TMEM; returns their sum.  LINES: as bf16 and, at
+// 32 scores (masked ones are -inf) -> exp2(s * sc - ref) as 16 packed fp16 pairs into TMEM; their sum is added to `sum`.  LINES: as bf16 and, at
 // taddr_lo, the bf16 remainder of each, 17 bits together
-template <bool LINES> DL_DEVINL float pt_probs(const uint32_t (&v)[32], float sc, float ref, uint32_t taddr, uint32_t taddr_lo) {
+template <bool LINES> DL_DEVINL void pt_probs(const uint32_t (&v)[32], float sc, float ref, uint32_t taddr, uint32_t taddr_lo, pair_f& sum) {
     uint32_t pk[16], lo[LINES ? 16 : 1];
-    float sum = 0.0f;
+    const pair_f sc2 = pair_of(sc, sc), ref2 = pair_of(-ref, -ref);
 #pragma unroll
     for (int e = 0; e < 32; e += 2) {
-        const float pa = pt_ex2(fmaf(__uint_as_float(v[e]), sc, -ref));
-        const float xb = fmaf(__uint_as_float(v[e + 1]), sc, -ref);
-        const float pb = (e & 2) ? pt_ex2_poly<LINES>(xb) : pt_ex2(xb);
-        sum += pa + pb;
+        pair_f p = fma2(pair_of(__uint_as_float(v[e]), __uint_as_float(v[e + 1])), sc2, ref2);
+        float pa, pb;
+        if ((e & 6) == 6) {
+            p = pt_ex2_poly<LINES>(p);
+            pair_get(p, pa, pb);
+        } else {
+            pair_get(p, pa, pb);
+            pa = pt_ex2(pa);
+            pb = pt_ex2(pb);
+            p = pair_of(pa, pb);
+        }
+        sum = add2(sum, p);
         pk[e >> 1] = pt_pack2<LINES>(pa, pb);
         if constexpr (LINES) lo[e >> 1] = pt_pack2<LINES>(pa - __uint_as_float(pk[e >> 1] << 16), pb - __uint_as_float(pk[e >> 1] & 0xffff0000u));
     }
     tmem_st_32x32b_x16(taddr, pk);
     if constexpr (LINES) tmem_st_32x32b_x16(taddr_lo, lo);
-    return sum;
 }
 
 // One thread's 32 consecutive outputs of row m (a Q80 block) into the slabs of the next matmul: the block's maximum is in the thread's own
@@ -210,422 +219,574 @@ DL_DEVINL void pt_q80_block(const float (&v)[32], int m, int kblock, int mcap, u
     }
 }
 
+// What a CTA works on: two query tiles of up to 128 (stacked) rows that meet the same keys and values, and the steps that they see.
+struct PtItem {
+    int kvh, p0, slot, seq_end;            // key/value head; position of the first row of the segment (or run); tokens of the sequence that exist
+    int first_page, j0, J;                 // pages ahead of first_page are not touched; steps of 128 tokens, the first one at token j0 * 128
+    int ja[2], jb[2];                      // steps [ja, jb) of these are tile t's (none: the tile is not there)
+    int row0[2], rows, head[2];            // first row of tile t, rows of the segment (or run), the tile's head
+    int begin;                             // batch row of the segment's first row; LINES: entry of tile_rows where the run starts
+};
+
+// A wait that gives up after PT_DEADLINE_NS: the flag ends the other waits, too, and every output of the CTA becomes a NaN
+struct PtWaits {
+    volatile int* gave_up;
+    unsigned long long t0;
+    DL_DEVINL void operator()(uint64_t* bar, uint32_t parity) const {
+        unsigned n = 0;
+        while (!mbar_try_wait(bar, parity)) {
+            if ((++n & 0x3FFu) == 0) {
+                if (*gave_up) return;
+                if (globaltimer_ns() - t0 > PT_DEADLINE_NS) { *gave_up = 1; return; }
+            }
+        }
+    }
+};
+
+// Llama path: the items of a batch are (128-row tile of a segment, query head), late tiles (long histories) first: two heads of one key/value head
+// side by side, or two tiles of one head where the heads come alone; single tiles while there are SMs for all of them.  Item `idx` of the
+// order that all roles of all CTAs walk; false behind the last one.
+DL_DEVINL bool pt_item(const PtArgs& a, const int (*seg)[4], int n_seg, int idx, PtItem& it) {
+    const int rep = a.n_heads / a.n_kv_heads;
+    int tiles = 0;
+    for (int i = 0; i < n_seg; i++) tiles += (seg[i][1] + PT_ROWS - 1) / PT_ROWS;
+    const bool single = tiles * a.n_heads <= (int)gridDim.x, by_heads = !single && rep % 2 == 0, by_rows = !single && !by_heads;
+    const int cols = by_heads ? a.n_heads / 2 : a.n_heads;
+    for (int i = 0; i < n_seg; i++) {
+        const int nt = (seg[i][1] + PT_ROWS - 1) / PT_ROWS, groups = by_rows ? (nt + 1) / 2 : nt;
+        if (idx >= groups * cols) { idx -= groups * cols; continue; }
+        const int group = groups - 1 - idx / cols, col = idx % cols;
+        it.begin = seg[i][0]; it.rows = seg[i][1]; it.p0 = seg[i][2]; it.slot = seg[i][3];
+        it.seq_end = it.p0 + it.rows;
+        it.first_page = it.j0 = it.J = 0;
+#pragma unroll
+        for (int t = 0; t < 2; t++) {
+            it.row0[t] = (by_rows ? 2 * group + t : group) * PT_ROWS;
+            it.head[t] = by_heads ? 2 * col + t : col;
+            const bool there = it.row0[t] < it.rows && (t == 0 || !single);
+            it.ja[t] = 0;
+            it.jb[t] = there ? (it.p0 + min(it.row0[t] + PT_ROWS, it.rows) - 1) / PT_KV + 1 : 0;
+            it.J = max(it.J, it.jb[t]);
+        }
+        it.kvh = it.head[0] / rep;
+        return true;
+    }
+    return false;
+}
+
+// Layer-list models: the run of list tiles that this CTA owns and the share of its steps; false where there is nothing to do.  (By whole warps)
+DL_DEVINL bool pt_run(const PtLineArgs& a, PtItem& it, int& shares) {
+    const DlWindowAttnArgs& w = a.w;
+    const int t = (int)gridDim.x - 1 - (int)blockIdx.x, lane = threadIdx.x & 31;          // late tiles (long histories) first
+    // the tile ahead, this one and the three behind: rows of each, and where the first one is (a lane per tile)
+    int cnt[5] = {0, 0, 0, 0, 0}, m = 0, mine = 0;
+#pragma unroll
+    for (int u = 0; u < 5; u++) {
+        const int tu = t - 1 + u;
+        for (int r0 = 0; r0 < a.rq && tu >= 0 && tu < a.n_tiles; r0 += 32) {
+            const int row = r0 + lane < a.rq ? a.tile_rows[(size_t)tu * a.rq + r0 + lane] : -1;
+            cnt[u] += __popc(__ballot_sync(0xffffffffu, row >= 0));
+            const int first = __shfl_sync(0xffffffffu, row, 0);
+            if (r0 == 0 && lane == u) { m = first; mine = first >= 0; }
+        }
+    }
+    const int pos = mine ? w.pos[m] : 0, slot = mine ? w.slot[m] : 0;
+    bool joined[5];                                              // tile u - 1 is full and u continues its sequence (window_tiles_join)
+#pragma unroll
+    for (int u = 1; u < 5; u++) {
+        const bool follows = __shfl_sync(0xffffffffu, pos, u - 1) + a.rq == __shfl_sync(0xffffffffu, pos, u) && __shfl_sync(0xffffffffu, slot, u - 1) == __shfl_sync(0xffffffffu, slot, u);
+        joined[u] = follows && cnt[u - 1] == a.rq && cnt[u] > 0 && ((t - 1 + u) & (a.group - 1)) != 0;
+    }
+    if (cnt[1] == 0 || joined[1]) return false;
+    int run = cnt[1];
+#pragma unroll
+    for (int u = 2; u < 5; u++) {
+        if (!joined[u]) break;
+        run += cnt[u];
+    }
+    if (run * a.rep <= 16) return false;                         // a decoding tile, which belongs to the other kernel
+    it.begin = t * a.rq;
+    it.rows = run * a.rep;
+    it.p0 = __shfl_sync(0xffffffffu, pos, 1);
+    it.slot = __shfl_sync(0xffffffffu, slot, 1);
+    it.seq_end = it.p0 + run;                                    // what lies behind was not written yet, or is of no use here
+    it.kvh = blockIdx.y;
+    int lo[2], j[2];
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+        it.row0[u] = u * PT_ROWS;
+        it.head[u] = 0;
+        const int p = it.p0 + u * PT_ROWS / a.rep, last = it.p0 + min((u + 1) * PT_ROWS / a.rep, run) - 1;
+        lo[u] = w.window > 0 ? max(0, p - w.window + 1) : 0;
+        if (w.chunk > 0) lo[u] = max(lo[u], p / w.chunk * w.chunk);
+        j[u] = it.row0[u] < it.rows ? last / PT_KV + 1 : 0;
+    }
+    it.first_page = lo[0] / 32;                                  // (tile 1 starts no earlier)
+    it.j0 = lo[0] / PT_KV;
+    it.J = max(j[0], j[1]) - it.j0;
+    // shares of the steps by grid.z: no more than leave each PT_SHARE_STEPS, so that a short run is done without a merge
+    shares = max(1, min((int)gridDim.z, it.J / PT_SHARE_STEPS));
+    const int per = (it.J + shares - 1) / shares, z0 = min(it.J, (int)blockIdx.z * per), z1 = min(it.J, z0 + per);
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+        it.ja[u] = max(lo[u] / PT_KV - it.j0 - z0, 0);
+        it.jb[u] = max(min(j[u] - it.j0 - z0, z1 - z0), it.ja[u]);
+    }
+    it.j0 += z0;
+    it.J = z1 - z0;
+    it.first_page = max(it.first_page, it.j0 * (PT_KV / 32));
+    return (int)blockIdx.z < shares || shares > 1;               // (a share without steps says so in its partial sums)
+}
+
+// Queries of 32 rows into the tile's K-major, swizzled image: lane i holds the address of row r0 + i; N rows are in flight, a row a load
+template <bool LINES, int N, typename Ready>
+DL_DEVINL void pt_load_rows(const float* mine, uint8_t* tile, int r0, Ready ready) {
+    const int lane = threadIdx.x & 31;
+    uint8_t* qd = tile + r0 * 128 + (lane >> 4) * 16384 + (lane & 1) * 8;
+#pragma unroll 1
+    for (int i = 0; i < 32; i += N) {
+        float4 x[N];
+#pragma unroll
+        for (int u = 0; u < N; u++)
+            x[u] = reinterpret_cast<const float4*>(__shfl_sync(0xffffffffu, (unsigned long long)(uintptr_t)mine, i + u))[lane];
+        if (i == 0) ready();
+#pragma unroll
+        for (int u = 0; u < N; u++)              // 16-byte piece c of a half row -> swizzled slot c ^ (row & 7)
+            *reinterpret_cast<uint2*>(qd + (i + u) * 128 + ((((lane >> 1) & 7) ^ (u & 7)) << 4)) = make_uint2(pt_pack2<LINES>(x[u].x, x[u].y), pt_pack2<LINES>(x[u].z, x[u].w));
+    }
+    fence_proxy_async_smem();
+}
+
 template <bool LINES>
 __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(const __grid_constant__ typename PtKernelArgs<LINES>::T a,
                                                                              const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap) {
     extern __shared__ __align__(1024) uint8_t smem[];
+    __shared__ int seg[PT_MAX_SEG][4], n_seg_s, gave_up_s;
     if constexpr (!LINES) trace_begin(a.tr);
-    const unsigned long long t0 = globaltimer_ns();
-    uint8_t* q_s = smem;                                        // Q tile, K-major core matrices
-    uint8_t* k_s = smem + PT_TILE_BYTES;                        // [3] K tiles (tokens x head dim, K-major)
-    uint8_t* v_s = k_s + PT_STAGES * PT_TILE_BYTES;             // [3] V tiles (tokens x head dim, MN-major for P V)
-    float* out_s = reinterpret_cast<float*>(k_s);               // [128][129] f32, reuses the KV stages after the loop
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + (1 + 2 * PT_STAGES) * PT_TILE_BYTES);
-    uint64_t* k_full = bars;             // [3] transaction bytes of the step's K copies
-    uint64_t* k_empty = bars + 3;        // [3] the scores that read the stage are complete
-    uint64_t* v_full = bars + 6;         // [3] transaction bytes of the step's V copies
-    uint64_t* v_empty = bars + 9;        // [3] P V of the step has retired
-    uint64_t* q_full = bars + 12;
-    uint64_t* s_full = bars + 13;        // [2] scores complete
-    uint64_t* p_full = bars + 15;        // [2] probabilities written (and the score buffer read)
-    uint64_t* o_full = bars + 17;        // [2] P V of tile j complete (barrier j & 1)
-    uint64_t* s_empty = bars + 19;       // [2] the score buffer has been read into registers
-    uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 21);
-    float* mx_s = reinterpret_cast<float*>(bars + 24);          // [2 step parities][2 halves][128 rows] row maxima (and row sums at the end)
+    uint8_t* q_s = smem;                                        // [2] query tiles
+    uint8_t* k_s = q_s + 2 * PT_TILE_BYTES;                     // [2] K tiles (tokens x head dim, K-major)
+    uint8_t* v_s = k_s + PT_STAGES * PT_TILE_BYTES;             // [2] V tiles (tokens x head dim, MN-major for P V)
+    float* out_s = reinterpret_cast<float*>(v_s + PT_STAGES * PT_TILE_BYTES);      // [8 warps][32][PT_OUT_LD] f32: rows on their way out
+    uint64_t* bars = reinterpret_cast<uint64_t*>(out_s + 8 * 32 * PT_OUT_LD);
+    uint64_t* k_full = bars;             // [2] transaction bytes of the step's K copies
+    uint64_t* k_empty = bars + 2;        // [2] the scores that read the stage are complete (both tiles')
+    uint64_t* v_full = bars + 4;         // [2] transaction bytes of the step's V copies
+    uint64_t* v_empty = bars + 6;        // [2] P V of the step has retired (both tiles')
+    uint64_t* q_full = bars + 8;         // [2] the tile's queries are there
+    uint64_t* q_empty = bars + 10;       // [2] the tile's last scores are complete
+    uint64_t* s_full = bars + 12;        // [2] scores complete
+    uint64_t* p_full = bars + 14;        // [2] probabilities written
+    uint64_t* o_full = bars + 16;        // [2] P V complete
+    uint64_t* s_empty = bars + 18;       // the scores have been read into registers (one buffer for both tiles)
+    uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 19);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    int kvh, n_rows, r_first, p0, last_pos, seq_end, first_page, j0, j1, max_pages, n_kv, begin = 0, head = 0;
-    const int *bt, *rows_of = nullptr;
     pdl_launch_dependents();
-    if constexpr (!LINES) {
-        head = blockIdx.y;
-        kvh = head / (a.n_heads / a.n_kv_heads);
-        pdl_wait();                                              // q, this chunk's KV rows and meta come from earlier kernels
-        // which (segment, 128-row tile) is this CTA?  Large tiles (late rows: long histories) are handed out first.
-        int tile = blockIdx.x, end = 0;
-        {
-            const int n_seg = min(a.meta[0], PT_MAX_SEG);
-            int i = 0;
-            for (; i < n_seg; i++) {
-                begin = a.meta[1 + 2 * i];
-                end = a.meta[2 + 2 * i];
-                const int nt = (end - begin + PT_ROWS - 1) / PT_ROWS;
-                if (tile < nt) { tile = nt - 1 - tile; break; }
-                tile -= nt;
-            }
-            if (i == n_seg) { trace_end(a.tr); return; }
+    if (tid == 0) {
+        gave_up_s = 0;
+        for (int s = 0; s < 2; s++) {
+            mbar_init(&k_full[s], 1);
+            mbar_init(&k_empty[s], 1);
+            mbar_init(&v_full[s], 1);
+            mbar_init(&v_empty[s], 1);
+            mbar_init(&q_full[s], 128);
+            mbar_init(&q_empty[s], 1);
+            mbar_init(&s_full[s], 1);
+            mbar_init(&p_full[s], 128);
+            mbar_init(&o_full[s], 1);
         }
-        n_rows = end - begin;
-        r_first = tile * PT_ROWS;
-        p0 = a.pos[begin];
-        bt = a.block_table + (size_t)a.slot[begin] * a.max_pages;
-        last_pos = p0 + r_first + min(PT_ROWS, n_rows - r_first) - 1;
-        seq_end = p0 + n_rows;                                   // tokens of this sequence that exist
-        first_page = j0 = 0;
-        j1 = last_pos / PT_KV + 1;
-        n_kv = a.n_kv_heads;
+        mbar_init(s_empty, 128);
+        mbar_fence_init();
+    }
+    int n_seg = 0, shares = 1;
+    PtItem one;                                                  // LINES: a CTA has one item
+    if constexpr (!LINES) {
+        pdl_wait();                                              // q, this chunk's KV rows and meta come from earlier kernels
+        if (warp == 1) {
+            const int ns = min(a.meta[0], PT_MAX_SEG);
+            if (lane == 0) n_seg_s = ns;
+            if (lane < ns) {
+                const int b = a.meta[1 + 2 * lane], e = a.meta[2 + 2 * lane];
+                seg[lane][0] = b;
+                seg[lane][1] = e - b;
+                seg[lane][2] = e > b ? a.pos[b] : 0;
+                seg[lane][3] = e > b ? a.slot[b] : 0;
+            }
+        }
     } else {
         // (launched behind a kernel that writes the rows of other tiles and reads the same inputs: nothing to wait for here.  What
         // follows this grid must follow that one too, so this grid may not end ahead of it: a CTA with work waits when it is done, and the
         // first CTA waits even without -- one is enough, a grid ends with its last CTA, and all of the idle ones would keep an SM each
         // from those with work)
-        const DlWindowAttnArgs& w = a.w;
-        const bool first_cta = blockIdx.x == 0 && blockIdx.y == 0;
-        kvh = blockIdx.y;
-        const int t = (int)gridDim.x - 1 - (int)blockIdx.x;      // late tiles (long histories) first
-        const int e = t & ~1;                                    // an even tile takes its neighbour along where that continues its sequence
-        const int ne = window_tile_count(a.tile_rows, a.n_tiles, a.rq, e), no = window_tile_count(a.tile_rows, a.n_tiles, a.rq, e + 1);
-        const bool both = window_tiles_join(w, a.tile_rows, a.rq, e, ne, no);
-        const int run = (t & 1) ? (both ? 0 : no) : both ? ne + no : ne;
-        if (run * a.rep <= 16) {                                 // taken along by its neighbour, or a decoding tile, which belongs to the other kernel
-            if (first_cta) pdl_wait();
+        if (!pt_run(a, one, shares)) {
+            if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) pdl_wait();
             return;
         }
-        rows_of = a.tile_rows + (size_t)t * a.rq;
-        const int m0 = rows_of[0], p_first = w.pos[m0];
-        n_rows = run * a.rep;
-        r_first = 0;
-        p0 = p_first;
-        last_pos = p_first + run - 1;
-        seq_end = last_pos + 1;                                  // what lies behind was not written yet, or is of no use here
-        bt = w.block_table + (size_t)w.slot[m0] * w.max_pages;
-        int lo = w.window > 0 ? max(0, p_first - w.window + 1) : 0;
-        if (w.chunk > 0) lo = max(lo, p_first / w.chunk * w.chunk);
-        first_page = lo / 32;                                    // pages ahead of it are not touched
-        j0 = lo / PT_KV;
-        j1 = last_pos / PT_KV + 1;
-        n_kv = w.kv_heads;
-    }
-    const int n_tiles = j1 - j0;                                 // steps of 128 tokens, the first one at token j0 * 128
-
-    if (tid == 0) {
-        for (int s = 0; s < PT_STAGES; s++) {
-            mbar_init(&k_full[s], 1);
-            mbar_init(&k_empty[s], 1);
-            mbar_init(&v_full[s], 1);
-            mbar_init(&v_empty[s], 1);
-        }
-        for (int s = 0; s < 2; s++) {
-            mbar_init(&s_full[s], 1);
-            mbar_init(&s_empty[s], 256);
-            mbar_init(&p_full[s], 256);
-            mbar_init(&o_full[s], 1);
-        }
-        mbar_init(q_full, 256);
-        mbar_fence_init();
     }
     if (warp == 0) tmem_alloc(tmem_holder, 512);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    const PtWaits wait = {&gave_up_s, globaltimer_ns()};
+    if constexpr (!LINES) n_seg = n_seg_s;
+    // the items of this CTA, in the same order for every role; rounds run back and forth over the CTAs, so that a long item goes with a short one
+    auto item_at = [&](int round, PtItem& it) {
+        if constexpr (LINES) {
+            it = one;
+            return round == 0;
+        } else {
+            const int G = gridDim.x, b = blockIdx.x;
+            return pt_item(a, seg, n_seg, round * G + ((round & 1) ? G - 1 - b : b), it);
+        }
+    };
     const uint32_t tmem_base = *tmem_holder;
-    const uint32_t T_S = tmem_base, T_P = tmem_base + 256, T_O = tmem_base + 384;
+    // TMEM columns: outputs at 256 + 128 t.  One buffer of scores at 0, taken in turn, and probabilities at 128 + 64 t; LINES, whose
+    // probabilities need 128 columns: scores, then probabilities, at 128 t
+    const auto t_s = [&](int t) { return tmem_base + (LINES ? t * 128 : 0); };
+    const auto t_p = [&](int t) { return tmem_base + (LINES ? t * 128 : 128 + t * 64); };
+    auto row_of = [&](const PtItem& it, int t, int row) -> const float* {      // the queries of a tile's row (rows that are not there: of the last one)
+        const int r = min((t ? it.row0[1] : it.row0[0]) + row, it.rows - 1);
+        if constexpr (LINES) return a.w.q + (size_t)a.tile_rows[it.begin + r / a.rep] * a.w.ldq + (it.kvh * a.rep + r % a.rep) * PT_HS;
+        else return a.q + (size_t)(it.begin + r) * a.n_heads * PT_HS + (t ? it.head[1] : it.head[0]) * PT_HS;
+    };
 
     // 128-byte-swizzled operands: rows of 128 B (64 halfs), 8-row groups 1024 B apart; the head dimension is split in
     // two such half tiles 16 KB apart.  K-major (Q, K): LBO unused (1), SBO 1024.  MN-major (V as B of P V): LBO =
     // distance between the two 64-wide halves of N (16 KB), SBO = distance between 8-token groups (1024 B).
-    const uint32_t desc_hi = (1024u >> 4) | (1u << 14) | (2u << 29);
-    if (warp == 0) {
-        // ------------------------------------ S = Q K^T issuer ------------------------------------
-        const uint32_t idesc_s = pt_idesc(PT_ROWS, PT_KV, 0, LINES);
-        auto lo_k = [](const void* p) { return ((smem_u32(p) & 0x3FFFFu) >> 4) | (1u << 16); };
-        pt_wait(q_full, 0, t0);
-        for (int j = 0; j < n_tiles; j++) {
-            pt_wait(&k_full[j % PT_STAGES], (j / PT_STAGES) & 1, t0);
-            if (lane == 0) PT_STAMP(0, j);
-            // softmax(j-2) has this score buffer in registers; LINES: P V(j-2) has read the remainders that lay in it
-            if (j >= 2) pt_wait(LINES ? &o_full[j & 1] : &s_empty[j & 1], ((j - 2) >> 1) & 1, t0);
-            tc_fence_after();
-            if (elect_one()) {
-                const uint32_t a_lo = lo_k(q_s), b_lo = lo_k(k_s + (j % PT_STAGES) * PT_TILE_BYTES);
-#pragma unroll
-                for (int k = 0; k < 8; k++) {      // K = 16 per MMA: 32 B inside the swizzled row, the second half tile after four
-                    const uint32_t off = (uint32_t)((k >> 2) * (16384 >> 4) + (k & 3) * 2);
-                    uint64_t da, db;
-                    asm("mov.b64 %0, {%1, %2};" : "=l"(da) : "r"(a_lo + off), "r"(desc_hi));
-                    asm("mov.b64 %0, {%1, %2};" : "=l"(db) : "r"(b_lo + off), "r"(desc_hi));
-                    if (!PT_DBG(4)) umma_f16_ss(T_S + (j & 1) * 128, da, db, idesc_s, k > 0 ? 1u : 0u);
-                }
-                umma_commit(&s_full[j & 1]);
-                umma_commit(&k_empty[j % PT_STAGES]);
+    if (warp < 8) {
+        // ---------------- softmax: warps 0-3 tile 0, warps 4-7 tile 1; a thread per query row (= TMEM lane) ----------------
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 192;");
+        const int t = warp >> 2, quarter = warp & 3, row = quarter * 32 + lane;
+        const uint32_t lane_base = (uint32_t)(quarter * 32) << 16, T_S = t_s(t) + lane_base, T_P = t_p(t) + lane_base, T_O = tmem_base + lane_base + 256 + t * 128;
+        float* stage = out_s + (size_t)warp * 32 * PT_OUT_LD;
+        uint32_t ns = 0;                                         // steps of this tile so far
+        PtItem it;
+        for (int round = 0; item_at(round, it); round++) {
+            const int ja = t ? it.ja[1] : it.ja[0], jb = t ? it.jb[1] : it.jb[0], row0 = t ? it.row0[1] : it.row0[0], head = t ? it.head[1] : it.head[0];
+            const int r_abs = row0 + row, r_live = min(r_abs, it.rows - 1);
+            if (!LINES && jb == 0) continue;
+            if (round == 0 && jb > ja) {                         // the first queries (the others: warps 12-15, ahead of time)
+                pt_load_rows<LINES, 32>(row_of(it, t, row), q_s + t * PT_TILE_BYTES, quarter * 32, [] {});
+                mbar_arrive(&q_full[t]);
             }
-            __syncwarp();
-            if (lane == 0) PT_STAMP(1, j);
-        }
-    } else if (warp == 6) {
-        // ------------------------------------ O += P V issuer ------------------------------------
-        const uint32_t idesc_pv = pt_idesc(PT_ROWS, PT_HS, 1, LINES);
-        for (int i = 0; i < n_tiles; i++) {
-            uint8_t* vz = v_s + (i % PT_STAGES) * PT_TILE_BYTES;
-            if (LINES && i == 0 && first_page * 32 > j0 * PT_KV) {      // tokens of pages that this tile does not touch
-                pt_wait(&v_full[0], 0, t0);
-                for (int idx = lane; idx < (first_page * 32 - j0 * PT_KV) * 16; idx += 32)
-                    *reinterpret_cast<uint4*>(vz + ((idx >> 3) & 1) * 16384 + (idx >> 4) * 128 + (idx & 7) * 16) = make_uint4(0, 0, 0, 0);
-                fence_proxy_async_smem();
-                __syncwarp();
-            }
-            if ((j0 + i + 1) * PT_KV > seq_end) {
-                // the step that contains the end of the sequence: rows past it were never written (or not copied at all);
-                // their scores are masked, but a zero probability times a non-finite V would poison the product -> zero them
-                pt_wait(&v_full[i % PT_STAGES], (i / PT_STAGES) & 1, t0);
-                const int r0 = max(0, seq_end - (j0 + i) * PT_KV);
-                for (int idx = r0 * 16 + lane; idx < PT_KV * 16; idx += 32) {      // 16 pieces of 16 B per token row (two halves)
-                    const int r = idx >> 4, c = idx & 15;
-                    *reinterpret_cast<uint4*>(vz + (c >> 3) * 16384 + r * 128 + (c & 7) * 16) = make_uint4(0, 0, 0, 0);
-                }
-                fence_proxy_async_smem();
-                __syncwarp();
-            }
-            pt_wait(&v_full[i % PT_STAGES], (i / PT_STAGES) & 1, t0);
-            pt_wait(&p_full[i & 1], (i >> 1) & 1, t0);
-            if (lane == 0) PT_STAMP(2, i);
-            tc_fence_after();
-            if (elect_one()) {
-                const uint32_t b_lo = ((smem_u32(vz) & 0x3FFFFu) >> 4) | ((16384u >> 4) << 16);
-#pragma unroll
-                for (int k = 0; k < 8; k++) {      // 16 tokens per MMA: 8 TMEM columns of P, two 8-token groups (2048 B) of V
-                    uint64_t db;
-                    asm("mov.b64 %0, {%1, %2};" : "=l"(db) : "r"(b_lo + k * 128), "r"(desc_hi));
-                    if (!PT_DBG(4)) umma_f16_ts(T_O, T_P + (i & 1) * 64 + k * 8, db, idesc_pv, (i > 0 || k > 0) ? 1u : 0u);
-                    if constexpr (LINES) umma_f16_ts(T_O, T_S + (i & 1) * 128 + k * 8, db, idesc_pv, 1u);
-                }
-                umma_commit(&o_full[i & 1]);
-                umma_commit(&v_empty[i % PT_STAGES]);
-            }
-            __syncwarp();
-        }
-    } else if (warp <= 4 || warp >= 8) {
-        // ---------------- softmax: two threads per query row (= TMEM lane), 64 score columns each ----------------
-        // warps 1-4 take columns [0, 64) of their lane quarter, warps 8-11 columns [64, 128): the MUFU work of a step
-        // (128 x 128 exp2) is fixed, but with two warps per scheduler the loads, maxima, packs and stores overlap it
-        const int quarter = warp & 3, row = quarter * 32 + lane, hf = warp >= 8 ? 1 : 0;
-        const int r_abs = r_first + row;
-        const int r_live = min(r_abs, n_rows - 1);
-        int m_row = 0, h_row = 0;                                // LINES: this row's batch row and head
-        {
-            const float* qg;
+            int pos_r, lb = 0, m_row = 0, h_row = 0;             // last and first visible position of this row; LINES: its batch row and head
+            float sc, c1 = 0.f, cap_k = 0.f, slope = 0.f;
+            bool shaped = false;                                 // scores leave the accumulator through a cap, a bias or a factor that is not positive
             if constexpr (LINES) {
-                m_row = rows_of[r_live / a.rep];
-                h_row = kvh * a.rep + r_live % a.rep;
-                qg = a.w.q + (size_t)m_row * a.w.ldq + h_row * PT_HS + hf * 64;
+                const DlWindowAttnArgs& w = a.w;
+                m_row = a.tile_rows[it.begin + r_live / a.rep];
+                h_row = it.kvh * a.rep + r_live % a.rep;
+                pos_r = it.p0 + r_live / a.rep;
+                if (w.window > 0) lb = max(0, pos_r - w.window + 1);
+                if (w.chunk > 0) lb = max(lb, pos_r / w.chunk * w.chunk);
+                shaped = w.softcap > 0.f || w.slope != nullptr || !(w.scale > 0.f);      // (a factor that keeps no order meets the scores ahead of mask and maximum)
+                sc = 1.4426950408889634f * w.scale;
+                c1 = w.softcap > 0.f ? sc * 2.f / w.softcap : sc;
+                cap_k = w.softcap * 1.4426950408889634f;
+                if (w.slope != nullptr) slope = w.slope[h_row] * 1.4426950408889634f;
+                if (shaped) sc = 1.f;
             } else {
-                qg = a.q + (size_t)(begin + r_live) * a.n_heads * PT_HS + head * PT_HS + hf * 64;
+                pos_r = it.p0 + r_abs;
+                sc = 1.4426950408889634f * rsqrtf((float)PT_HS);     // scores in the log2 domain
             }
-            uint8_t* qd = q_s + hf * 16384 + row * 128;
-#pragma unroll 4
-            for (int c = 0; c < 8; c++) {       // 16-byte piece c of this half of the row -> swizzled slot c ^ (row & 7)
-                const float4 x = reinterpret_cast<const float4*>(qg)[2 * c], y = reinterpret_cast<const float4*>(qg)[2 * c + 1];
-                uint4 u;
-                u.x = pt_pack2<LINES>(x.x, x.y); u.y = pt_pack2<LINES>(x.z, x.w);
-                u.z = pt_pack2<LINES>(y.x, y.y); u.w = pt_pack2<LINES>(y.z, y.w);
-                *reinterpret_cast<uint4*>(qd + ((c ^ (row & 7)) << 4)) = u;
-            }
-            fence_proxy_async_smem();
-            mbar_arrive(q_full);
-        }
-        int pos_r, lb = 0;                                       // last and first visible position of this row
-        float sc, c1 = 0.f, cap_k = 0.f, slope = 0.f;
-        bool shaped = false;                                     // scores leave the accumulator through a cap, a bias or a factor that is not positive
-        if constexpr (LINES) {
-            const DlWindowAttnArgs& w = a.w;
-            pos_r = p0 + r_live / a.rep;
-            if (w.window > 0) lb = max(0, pos_r - w.window + 1);
-            if (w.chunk > 0) lb = max(lb, pos_r / w.chunk * w.chunk);
-            shaped = w.softcap > 0.f || w.slope != nullptr || !(w.scale > 0.f);      // (a factor that keeps no order meets the scores ahead of mask and maximum)
-            sc = 1.4426950408889634f * w.scale;
-            c1 = w.softcap > 0.f ? sc * 2.f / w.softcap : sc;
-            cap_k = w.softcap * 1.4426950408889634f;
-            if (w.slope != nullptr) slope = w.slope[h_row] * 1.4426950408889634f;
-            if (shaped) sc = 1.f;
-        } else {
-            pos_r = p0 + r_abs;
-            sc = 1.4426950408889634f * rsqrtf((float)PT_HS);     // scores in the log2 domain
-        }
-        const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
-        float m_used = -INFINITY, l = 0.0f;
-        uint32_t v0[32], v1[32];
-        for (int j = 0; j < n_tiles; j++) {
-            pt_wait(&s_full[j & 1], (j >> 1) & 1, t0);
-            if (tid == 32) PT_STAMP(3, j);
-            tc_fence_after();
-            const uint32_t t_s = T_S + lane_base + (j & 1) * 128 + hf * 64;
-            const int tok0 = (j0 + j) * PT_KV + hf * 64;
-            if PT_DBG(1) { tc_fence_before(); mbar_arrive(&s_empty[j & 1]); mbar_arrive(&p_full[j & 1]); continue; }
-            tmem_ld_32x32b_x32(t_s, v0);
-            tmem_ld_32x32b_x32(t_s + 32, v1);
-            tmem_ld_wait();
-            tc_fence_before();
-            mbar_arrive(&s_empty[j & 1]);                    // the scores of step j+2 may overwrite the buffer now
-            const int lim = pos_r - tok0;                    // columns e <= lim of this half are visible to this row
-            const int low = LINES ? lb - tok0 : 0;           // and e >= low
-            if constexpr (LINES) {
-                if (shaped) {
-#pragma unroll
-                    for (int e = 0; e < 64; e++) {
-                        float x = __uint_as_float(e < 32 ? v0[e & 31] : v1[e & 31]) * c1;
-                        if (cap_k > 0.f) {                   // cap tanh(s / cap) in base 2, as the mma.sync kernel forms it
-                            float r;
-                            asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(pt_ex2(x) + 1.f));
-                            x = fmaf(-2.f * cap_k, r, cap_k);
-                        }
-                        x = fmaf(-slope, (float)(lim - e), x);
-                        if (e < 32) v0[e & 31] = __float_as_uint(x); else v1[e & 31] = __float_as_uint(x);
-                    }
-                }
-            }
-            float ma = -INFINITY, mb = -INFINITY;
-            if (lim >= 63 && (!LINES || low <= 0)) {
-#pragma unroll
-                for (int e = 0; e < 32; e += 2) {
-                    ma = fmaxf(ma, fmaxf(__uint_as_float(v0[e]), __uint_as_float(v1[e])));
-                    mb = fmaxf(mb, fmaxf(__uint_as_float(v0[e + 1]), __uint_as_float(v1[e + 1])));
-                }
-            } else {
-#pragma unroll
-                for (int e = 0; e < 32; e++) {
-                    if (e > lim || (LINES && e < low)) v0[e] = 0xff800000u;        // -inf
-                    if (e + 32 > lim || (LINES && e + 32 < low)) v1[e] = 0xff800000u;
-                    ma = fmaxf(ma, fmaxf(__uint_as_float(v0[e]), __uint_as_float(v1[e])));
-                }
-            }
-            // row maximum over both halves: exchange through shared memory (slot of step parity: the next write to it
-            // comes two steps later, after everybody has passed the barrier of the step in between)
-            float mx = fmaxf(ma, mb);
-            mx_s[((j & 1) * 2 + hf) * PT_ROWS + row] = mx;
-            asm volatile("bar.sync 2, 256;" ::: "memory");
-            mx = fmaxf(mx, mx_s[((j & 1) * 2 + (hf ^ 1)) * PT_ROWS + row]);
-            if constexpr (LINES) tc_fence_after();           // both halves have read their scores: the remainders take their place
-            if (tid == 32) PT_STAMP(4, j);
-            mx *= sc;
-            const bool need = mx > m_used + 8.0f;            // the reference may lag the maximum by 2^8
-            if (__any_sync(0xffffffffu, need)) {
-                const float m_new = need ? mx : m_used;
-                const float alpha = need ? pt_ex2(m_used - m_new) : 1.0f;
-                if (j > 0) {      // the accumulated output moves to the new reference (rare after the first tiles)
-                    pt_wait(&o_full[(j - 1) & 1], ((j - 1) >> 1) & 1, t0);
-                    tc_fence_after();
-                    uint32_t w[32];
-#pragma unroll 1
-                    for (int ch = 0; ch < 2; ch++) {
-                        tmem_ld_32x32b_x32(T_O + lane_base + hf * 64 + ch * 32, w);
-                        tmem_ld_wait();
-#pragma unroll
-                        for (int e = 0; e < 32; e++) w[e] = __float_as_uint(__uint_as_float(w[e]) * alpha);
-                        tmem_st_32x32b_x32(T_O + lane_base + hf * 64 + ch * 32, w);
-                    }
-                    tmem_st_wait();
-                }
-                l *= alpha;
-                m_used = m_new;
-            }
-            const float ref = (m_used == -INFINITY) ? 0.0f : m_used;
-            const uint32_t t_p = T_P + lane_base + (j & 1) * 64 + hf * 32;
-            if (j >= 2) {      // P V(j-2) has consumed this probability buffer (long done; the wait keeps it a guarantee)
-                pt_wait(&o_full[j & 1], ((j - 2) >> 1) & 1, t0);
+            float m_used = -INFINITY, l = 0.0f;
+            for (int j = ja; j < jb; j++, ns++) {
+                uint32_t v[4][32];
+                wait(&s_full[t], ns & 1);                        // LINES: also P V of the step before is complete
                 tc_fence_after();
-            }
-            const uint32_t t_lo = T_S + lane_base + (j & 1) * 128 + hf * 32;
-            l += pt_probs<LINES>(v0, sc, ref, t_p, t_lo);
-            l += pt_probs<LINES>(v1, sc, ref, t_p + 16, t_lo + 16);
-            tmem_st_wait();
-            tc_fence_before();
-            mbar_arrive(&p_full[j & 1]);
-            if (tid == 32) PT_STAMP(5, j);
-        }
-        // ---- finish: O / l -> shared memory -> Q80 cast into the slabs of the wo matmul ----
-        pt_wait(&o_full[(n_tiles - 1) & 1], ((n_tiles - 1) >> 1) & 1, t0);
-        tc_fence_after();
-        // the two halves of the row sum, through the exchange slots the LAST step did not use (their previous readers
-        // have all passed that step's barrier)
-        const int fs = (n_tiles & 1) * 2;
-        mx_s[(fs + hf) * PT_ROWS + row] = l;
-        asm volatile("bar.sync 2, 256;" ::: "memory");
-        l += mx_s[(fs + (hf ^ 1)) * PT_ROWS + row];
-        float inv;
-        if constexpr (LINES) {
-            if (a.w.sink) l += pt_ex2(a.w.sink[h_row] * 1.4426950408889634f - m_used);
-            inv = (a.w.gate ? 1.f / (1.f + expf(-a.w.gate[(size_t)m_row * a.w.ld_gate + h_row])) : 1.f) / l;
-        } else {
-            inv = l > 0.0f ? 1.0f / l : 0.0f;
-        }
-        bool rows_out = true;                                    // f32 rows wanted: through shared memory, lanes along a row
-        if constexpr (!LINES) rows_out = a.y_out != nullptr;
+#pragma unroll
+                for (int c = 0; c < 4; c++) tmem_ld_32x32b_x32(T_S + c * 32, v[c]);
+                tmem_ld_wait();
+                if constexpr (!LINES) {                          // the other tile's scores may take the place
+                    tc_fence_before();
+                    mbar_arrive(s_empty);
+                }
+                const int tok0 = (it.j0 + j) * PT_KV;
+                const int lim = pos_r - tok0, low = LINES ? lb - tok0 : 0;      // columns low <= e <= lim are visible to this row
+                if constexpr (LINES) {
+                    if (shaped) {
+#pragma unroll
+                        for (int e = 0; e < PT_KV; e++) {
+                            float x = __uint_as_float(v[e >> 5][e & 31]) * c1;
+                            if (cap_k > 0.f) {                   // cap tanh(s / cap) in base 2, as the mma.sync kernel forms it
+                                float r;
+                                asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(pt_ex2(x) + 1.f));
+                                x = fmaf(-2.f * cap_k, r, cap_k);
+                            }
+                            v[e >> 5][e & 31] = __float_as_uint(fmaf(-slope, (float)(lim - e), x));
+                        }
+                    }
+                }
+                if (lim < PT_KV - 1 || (LINES && low > 0)) {
+#pragma unroll
+                    for (int e = 0; e < PT_KV; e++)
+                        if (e > lim || (LINES && e < low)) v[e >> 5][e & 31] = 0xff800000u;        // -inf
+                }
+                float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+                for (int e = 0; e < 32; e += 2)
+#pragma unroll
+                    for (int c = 0; c < 4; c++) mx4[c] = fmaxf(mx4[c], fmaxf(__uint_as_float(v[c][e]), __uint_as_float(v[c][e + 1])));
+                const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * sc;
+                const bool need = mx > m_used + 8.0f;            // the reference may lag the maximum by 2^8
+                if (!LINES && j > ja) {                          // P V of the step before is done with the probabilities
+                    wait(&o_full[t], (ns - 1) & 1);
+                    tc_fence_after();
+                }
+                if (__any_sync(0xffffffffu, need)) {
+                    const float m_new = need ? mx : m_used;
+                    const float alpha = need ? pt_ex2(m_used - m_new) : 1.0f;
+                    if (j > ja) {      // the accumulated output moves to the new reference (rare after the first steps)
+                        uint32_t w[32];
 #pragma unroll 1
-        for (int ch = 0; ch < 2; ch++) {
-            tmem_ld_32x32b_x32(T_O + lane_base + hf * 64 + ch * 32, v0);
-            tmem_ld_wait();
-            float v[32];
+                        for (int ch = 0; ch < 4; ch++) {
+                            tmem_ld_32x32b_x32(T_O + ch * 32, w);
+                            tmem_ld_wait();
 #pragma unroll
-            for (int e = 0; e < 32; e++) v[e] = __uint_as_float(v0[e]) * inv;
-            if constexpr (!LINES) {
-                if (r_abs < n_rows && (a.xq_out != nullptr || a.xh_out != nullptr))
-                    pt_q80_block(v, begin + r_abs, (head * PT_HS) / 32 + hf * 2 + ch, a.out_mcap, a.xq_out, a.xh_out);
-            }
-            if (rows_out) {
-#pragma unroll
-                for (int e = 0; e < 32; e++) out_s[row * PT_OUT_LD + hf * 64 + ch * 32 + e] = v[e];
-            }
-        }
-        if (rows_out) {
-            __syncwarp();                                        // a warp only re-reads the 32 rows x 64 columns it wrote
-#pragma unroll 4
-            for (int rr = 0; rr < 32; rr++) {
-                const int rc = r_first + quarter * 32 + rr;
-                if (rc >= n_rows) break;
-                float* dst;
-                if constexpr (LINES) dst = a.w.out + (size_t)__shfl_sync(0xffffffffu, m_row, rr) * a.w.ldo + __shfl_sync(0xffffffffu, h_row, rr) * PT_HS;
-                else dst = a.y_out + (size_t)(begin + rc) * a.n_heads * PT_HS + head * PT_HS;
-                const float* src = out_s + (quarter * 32 + rr) * PT_OUT_LD + hf * 64 + lane;
-                dst[hf * 64 + lane] = src[0];
-                dst[hf * 64 + 32 + lane] = src[32];
-            }
-        }
-    } else if (warp == 5 || warp == 7) {
-        // ------------------------------------ K producer (warp 5) / V producer (warp 7), one lane each ------------------------------------
-        if (lane == 0) {
-            const bool is_k = warp == 5;
-            const uint64_t map = is_k ? reinterpret_cast<uint64_t>(&kmap) : reinterpret_cast<uint64_t>(&vmap);
-            uint64_t* full = is_k ? k_full : v_full;
-            uint64_t* empty = is_k ? k_empty : v_empty;
-            uint8_t* ring = is_k ? k_s : v_s;
-            const int total_pages = (seq_end + 31) / 32;
-            auto page_of = [&](int p) { return p >= first_page && p < total_pages ? bt[p] : 0; };
-            // the page ids of a step are fetched one step ahead, so the table reads (dependent global loads) overlap the
-            // wait for a free stage instead of delaying the copies
-            int pg[4], pg_next[4];
-#pragma unroll
-            for (int p4 = 0; p4 < 4; p4++) pg_next[p4] = page_of(4 * j0 + p4);
-            for (int j = 0; j < n_tiles; j++) {
-                const int st = j % PT_STAGES;
-#pragma unroll
-                for (int p4 = 0; p4 < 4; p4++) {
-                    pg[p4] = pg_next[p4];
-                    pg_next[p4] = page_of(4 * (j0 + j + 1) + p4);
+                            for (int e = 0; e < 32; e++) w[e] = __float_as_uint(__uint_as_float(w[e]) * alpha);
+                            tmem_st_32x32b_x32(T_O + ch * 32, w);
+                        }
+                    }
+                    l *= alpha;
+                    m_used = m_new;
                 }
-                if (j >= PT_STAGES) pt_wait(&empty[st], ((j / PT_STAGES) & 1) ^ 1, t0);
-                if (is_k) PT_STAMP(6, j);
-                const int n_pg = PT_DBG(2) ? 0 : min(4, (seq_end - (j0 + j) * PT_KV + 31) / 32);      // pages of this step that exist
-                const int p_lo = LINES ? max(0, first_page - 4 * (j0 + j)) : 0;                 // ... and are looked at (at most the first step starts later)
-                mbar_arrive_expect_tx(&full[st], (uint32_t)max(0, n_pg - p_lo) * 2u * 4096u);
-                const uint32_t dst = smem_u32(ring + st * PT_TILE_BYTES), bar = smem_u32(&full[st]);
+                const float ref = (m_used == -INFINITY) ? 0.0f : m_used;
+                pair_f sum = 0;
 #pragma unroll
-                for (int p4 = 0; p4 < 4; p4++) {
-                    if (p4 >= n_pg) break;
-                    if (LINES && p4 < p_lo) continue;
-                    const int y = (pg[p4] * n_kv + kvh) * 32;      // first row of the page in the [rows][128] view
-#pragma unroll
-                    for (int h = 0; h < 2; h++)
-                        asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-                                         dst + h * 16384 + p4 * 4096),
-                                     "l"(map), "r"((LINES && !is_k ? PT_HS : 0) + h * 64), "r"(y), "r"(bar)
-                                     : "memory");
+                for (int c = 0; c < 4; c++) pt_probs<LINES>(v[c], sc, ref, T_P + c * 16, T_P + 64 + c * 16, sum);
+                l += pair_sum(sum);
+                tmem_st_wait();
+                tc_fence_before();
+                mbar_arrive(&p_full[t]);
+            }
+            // ---- finish: O / l -> f32 rows, partial sums, or the Q80 cast into the slabs of the wo matmul ----
+            float inv;
+            if constexpr (LINES) {
+                if (shares == 1 && a.w.sink) l += pt_ex2(a.w.sink[h_row] * 1.4426950408889634f - m_used);
+                inv = shares > 1 ? 1.f : (a.w.gate ? 1.f / (1.f + expf(-a.w.gate[(size_t)m_row * a.w.ld_gate + h_row])) : 1.f) / l;
+            } else {
+                inv = l > 0.0f ? 1.0f / l : 0.0f;
+            }
+            float* out = nullptr;                                // this thread's row; null: none
+            bool vec = true;                                     // 16-byte rows
+            if constexpr (LINES) {
+                if (row0 >= it.rows) continue;
+                out = a.w.out + (size_t)m_row * a.w.ldo + h_row * PT_HS;
+                vec = ((uintptr_t)a.w.out & 15) == 0 && (a.w.ldo & 3) == 0;
+                if (gridDim.z > 1) {                             // a stacked row's slot among the list tile's partial sums
+                    const int u = it.begin / a.rq + r_live / (PT_ROWS / 2);
+                    float* part = a.partial + ((((size_t)u * a.w.kv_heads + it.kvh) * gridDim.z + blockIdx.z) * (PT_ROWS / 2) + r_live % (PT_ROWS / 2)) * (PT_HS + 2);
+                    if (r_abs < it.rows) {                       // (-2: no merge, -1: nothing in this share)
+                        part[PT_HS] = m_used * 0.6931471805599453f;
+                        part[PT_HS + 1] = shares == 1 ? -2.f : jb > ja ? l : -1.f;
+                    }
+                    if (shares > 1) { out = part; vec = false; }
                 }
-                if (is_k) PT_STAMP(7, j);
+                if (jb == ja) continue;
+            } else if (a.y_out != nullptr) {
+                out = a.y_out + (size_t)(it.begin + r_live) * a.n_heads * PT_HS + head * PT_HS;
+                vec = ((uintptr_t)a.y_out & 15) == 0;
+            }
+            wait(&o_full[t], (ns - 1) & 1);
+            tc_fence_after();
+            if (gave_up_s) inv = __int_as_float(0x7fffffff);
+            const int live = it.rows - (row0 + quarter * 32);      // rows of this warp that are there
+#pragma unroll 1
+            for (int ch = 0; ch < 4; ch++) {
+                uint32_t o[32];
+                float f[32];
+                tmem_ld_32x32b_x32(T_O + ch * 32, o);
+                tmem_ld_wait();
+#pragma unroll
+                for (int e = 0; e < 32; e++) f[e] = __uint_as_float(o[e]) * inv;
+                if constexpr (!LINES) {
+                    if (r_abs < it.rows && (a.xq_out != nullptr || a.xh_out != nullptr))
+                        pt_q80_block(f, it.begin + r_abs, head * (PT_HS / 32) + ch, a.out_mcap, a.xq_out, a.xh_out);
+                    if (out == nullptr) continue;
+                }
+#pragma unroll
+                for (int h = 0; h < 2; h++) {                    // 16 columns of the warp's rows, then as many lanes along a row
+                    __syncwarp();
+#pragma unroll
+                    for (int e = 0; e < 16; e += 4) *reinterpret_cast<float4*>(stage + lane * PT_OUT_LD + e) = make_float4(f[h * 16 + e], f[h * 16 + e + 1], f[h * 16 + e + 2], f[h * 16 + e + 3]);
+                    __syncwarp();
+#pragma unroll
+                    for (int rr = 0; rr < 32; rr += 8) {
+                        const int r = rr + (lane >> 2);
+                        float* dst = reinterpret_cast<float*>(__shfl_sync(0xffffffffu, (unsigned long long)(uintptr_t)out, r)) + ch * 32 + h * 16 + (lane & 3) * 4;
+                        const float4 x = *reinterpret_cast<const float4*>(stage + r * PT_OUT_LD + (lane & 3) * 4);
+                        if (r >= live) continue;
+                        if (vec) *reinterpret_cast<float4*>(dst) = x;
+                        else { dst[0] = x.x; dst[1] = x.y; dst[2] = x.z; dst[3] = x.w; }
+                    }
+                }
+            }
+            tc_fence_before();                                   // the next item's P V may write the output (behind p_full)
+        }
+    } else {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+        const uint32_t desc_hi = (1024u >> 4) | (1u << 14) | (2u << 29);
+        if (warp == 8) {
+            // ---------------- MMAs, all by one thread: what it issues runs in that order ----------------
+            const uint32_t idesc_s = pt_idesc(PT_ROWS, PT_KV, 0, LINES), idesc_pv = pt_idesc(PT_ROWS, PT_HS, 1, LINES);
+            uint32_t g = 0, n_s = 0, ns[2] = {0, 0}, nq[2] = {0, 0};      // steps, scores, steps of a tile, items of a tile so far
+            PtItem it;
+            for (int round = 0; item_at(round, it); round++) {
+                auto on = [&](int t, int j) { return j >= it.ja[t] && j < it.jb[t]; };
+                auto scores = [&](int t, int j) {                // S = Q K^T of a step
+                    if (!on(t, j)) {
+                        if (LINES && t == 1 && j < it.J) {       // (a step that only tile 0 sees)
+                            if (elect_one()) umma_commit(&k_empty[(g + j) & 1]);
+                            __syncwarp();
+                        }
+                        return;
+                    }
+                    wait(&k_full[(g + j) & 1], ((g + j) >> 1) & 1);
+                    if (j == it.ja[t]) wait(&q_full[t], nq[t]++ & 1);
+                    if (!LINES && n_s > 0) wait(s_empty, (n_s - 1) & 1);
+                    n_s++;
+                    tc_fence_after();
+                    if (elect_one()) {
+                        const uint32_t a_lo = ((smem_u32(q_s + t * PT_TILE_BYTES) & 0x3FFFFu) >> 4) | (1u << 16);
+                        const uint32_t b_lo = ((smem_u32(k_s + ((g + j) & 1) * PT_TILE_BYTES) & 0x3FFFFu) >> 4) | (1u << 16);
+#pragma unroll
+                        for (int k = 0; k < 8; k++) {      // K = 16 per MMA: 32 B inside the swizzled row, the second half tile after four
+                            const uint32_t off = (uint32_t)((k >> 2) * (16384 >> 4) + (k & 3) * 2);
+                            uint64_t da, db;
+                            asm("mov.b64 %0, {%1, %2};" : "=l"(da) : "r"(a_lo + off), "r"(desc_hi));
+                            asm("mov.b64 %0, {%1, %2};" : "=l"(db) : "r"(b_lo + off), "r"(desc_hi));
+                            umma_f16_ss(t_s(t), da, db, idesc_s, k > 0 ? 1u : 0u);
+                        }
+                        umma_commit(&s_full[t]);
+                        if (t == 1 || (!LINES && !on(1, j))) umma_commit(&k_empty[(g + j) & 1]);
+                        if (j + 1 == it.jb[t]) umma_commit(&q_empty[t]);
+                    }
+                    __syncwarp();
+                };
+                auto outputs = [&](int t, int j) {               // O += P V of a step
+                    const int st = (g + j) & 1;
+                    if (on(t, j)) {
+                        wait(&p_full[t], ns[t]++ & 1);
+                        tc_fence_after();
+                    }
+                    if (elect_one()) {
+                        if (on(t, j)) {
+                            const uint32_t b_lo = ((smem_u32(v_s + st * PT_TILE_BYTES) & 0x3FFFFu) >> 4) | ((16384u >> 4) << 16), T_O = tmem_base + 256 + t * 128;
+#pragma unroll
+                            for (int k = 0; k < 8; k++) {      // 16 tokens per MMA: 8 TMEM columns of P, two 8-token groups (2048 B) of V
+                                uint64_t db;
+                                asm("mov.b64 %0, {%1, %2};" : "=l"(db) : "r"(b_lo + k * 128), "r"(desc_hi));
+                                umma_f16_ts(T_O, t_p(t) + k * 8, db, idesc_pv, (j > it.ja[t] || k > 0) ? 1u : 0u);
+                                if constexpr (LINES) umma_f16_ts(T_O, t_p(t) + 64 + k * 8, db, idesc_pv, 1u);
+                            }
+                            umma_commit(&o_full[t]);
+                        }
+                        if (t == 1) umma_commit(&v_empty[st]);
+                    }
+                    __syncwarp();
+                };
+                scores(0, 0);
+                scores(1, 0);
+                if (!LINES) scores(0, 1);
+                for (int j = 0; j < it.J; j++) {
+                    const int st = (g + j) & 1;
+                    wait(&v_full[st], ((g + j) >> 1) & 1);
+                    // tokens that were not copied, or never written: their scores are masked, but a zero probability times a non-finite V would
+                    // poison the product -> zero them
+                    const int tok0 = (it.j0 + j) * PT_KV;
+                    if ((LINES && it.first_page * 32 > tok0) || tok0 + PT_KV > it.seq_end) {
+                        uint8_t* vz = v_s + st * PT_TILE_BYTES;
+                        const int z0 = LINES ? max(0, it.first_page * 32 - tok0) : 0, z1 = min(PT_KV, it.seq_end - tok0);
+                        for (int idx = lane; idx < PT_KV * 16; idx += 32) {      // 16 pieces of 16 B per token row (two halves)
+                            const int r = idx >> 4, c = idx & 15;
+                            if (r < z0 || r >= z1) *reinterpret_cast<uint4*>(vz + (c >> 3) * 16384 + r * 128 + (c & 7) * 16) = make_uint4(0, 0, 0, 0);
+                        }
+                        fence_proxy_async_smem();
+                        __syncwarp();
+                    }
+                    // probabilities that take the place of their scores: a tile's next scores behind its P V.  Else the other tile's, or its own
+                    // next but one: they wait in the buffer when the softmax threads come for them
+                    outputs(0, j);
+                    scores(LINES ? 0 : 1, j + 1);
+                    outputs(1, j);
+                    scores(LINES ? 1 : 0, j + (LINES ? 1 : 2));
+                }
+                g += it.J;
+            }
+        } else if (warp == 10 || warp == 11) {
+            // ---------------- K producer (warp 10) / V producer (warp 11), one lane each ----------------
+            if (lane == 0) {
+                const bool is_k = warp == 10;
+                const uint64_t map = is_k ? reinterpret_cast<uint64_t>(&kmap) : reinterpret_cast<uint64_t>(&vmap);
+                uint64_t* full = is_k ? k_full : v_full;
+                uint64_t* empty = is_k ? k_empty : v_empty;
+                uint8_t* ring = is_k ? k_s : v_s;
+                int n_kv, max_pages;
+                const int* table;
+                if constexpr (LINES) { n_kv = a.w.kv_heads; max_pages = a.w.max_pages; table = a.w.block_table; }
+                else { n_kv = a.n_kv_heads; max_pages = a.max_pages; table = a.block_table; }
+                uint32_t g = 0;
+                PtItem it;
+                for (int round = 0; item_at(round, it); round++) {
+                    const int* bt = table + (size_t)it.slot * max_pages;
+                    const int total_pages = (it.seq_end + 31) / 32;
+                    auto page_of = [&](int p) { return p >= it.first_page && p < total_pages ? bt[p] : 0; };
+                    // the page ids of a step are fetched one step ahead, so the table reads (dependent global loads) overlap the
+                    // wait for a free stage instead of delaying the copies
+                    int pg[4], pg_next[4];
+#pragma unroll
+                    for (int p4 = 0; p4 < 4; p4++) pg_next[p4] = page_of(4 * it.j0 + p4);
+                    for (int j = 0; j < it.J; j++, g++) {
+                        const int st = g & 1;
+#pragma unroll
+                        for (int p4 = 0; p4 < 4; p4++) {
+                            pg[p4] = pg_next[p4];
+                            pg_next[p4] = page_of(4 * (it.j0 + j + 1) + p4);
+                        }
+                        if (g >= PT_STAGES) wait(&empty[st], ((g >> 1) & 1) ^ 1);
+                        if (gave_up_s) break;                    // no more copies into a CTA that ends
+                        const int n_pg = min(4, total_pages - 4 * (it.j0 + j));                          // pages of this step that exist
+                        const int p_lo = LINES ? max(0, it.first_page - 4 * (it.j0 + j)) : 0;            // ... and are looked at (at most the first step starts later)
+                        mbar_arrive_expect_tx(&full[st], (uint32_t)max(0, n_pg - p_lo) * 2u * 4096u);
+                        const uint32_t dst = smem_u32(ring + st * PT_TILE_BYTES), bar = smem_u32(&full[st]);
+#pragma unroll
+                        for (int p4 = 0; p4 < 4; p4++) {
+                            if (p4 >= n_pg) break;
+                            if (LINES && p4 < p_lo) continue;
+                            const int y = (pg[p4] * n_kv + it.kvh) * 32;      // first row of the page in the [rows][128] view
+#pragma unroll
+                            for (int h = 0; h < 2; h++)
+                                asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+                                                 dst + h * 16384 + p4 * 4096),
+                                             "l"(map), "r"((LINES && !is_k ? PT_HS : 0) + h * 64), "r"(y), "r"(bar)
+                                             : "memory");
+                        }
+                    }
+                }
+            }
+        } else if (warp >= 12) {
+            // ---------------- queries of the next items, 32 rows of each tile per warp, ahead of the softmax threads ----------------
+            const int wq = warp - 12;
+            uint32_t nq[2] = {0, 0};
+            PtItem it;
+            for (int round = 0; item_at(round, it); round++) {
+#pragma unroll
+                for (int t = 0; t < 2; t++) {
+                    if (it.jb[t] <= it.ja[t]) continue;
+                    if (round > 0) {
+                        pt_load_rows<LINES, 8>(row_of(it, t, wq * 32 + lane), q_s + t * PT_TILE_BYTES, wq * 32, [&] {
+                            if (nq[t] > 0) wait(&q_empty[t], (nq[t] - 1) & 1);        // the tile's last scores have read the queries before
+                        });
+                        mbar_arrive(&q_full[t]);
+                    }
+                    nq[t]++;
+                }
             }
         }
     }
     tc_fence_before();
     __syncthreads();
+    if (gave_up_s) __nanosleep(1000000);                         // copies and MMAs in flight end
     if (warp == 0) {
         tc_fence_after();
         tmem_dealloc(tmem_base, 512);
@@ -635,10 +796,9 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
 }
 
 extern void dl_set_error(const char* fmt, ...);
-static int g_pt_dbg = 0;
-static long long* g_pt_stamps = nullptr;
-extern "C" void dl_debug_set_pt_mode(int m) { g_pt_dbg = m; }
-extern "C" void dl_debug_set_pt_trace(long long* p) { g_pt_stamps = p; }
+extern int dl_device_sm_count();
+
+#define PT_SMEM ((2 + 2 * PT_STAGES) * PT_TILE_BYTES + 8 * 32 * PT_OUT_LD * 4 + 20 * 8)
 
 typedef CUresult (*PtEncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -677,13 +837,11 @@ extern "C" int dl_attention_prefill_tc(const float* q, int M, int n_heads, int n
     a.q = q; a.k_cache = (const __half*)k_cache; a.v_cache = (const __half*)v_cache; a.pos = pos; a.slot = slot;
     a.block_table = block_table; a.meta = meta; a.M = M; a.n_heads = n_heads; a.n_kv_heads = n_kv_heads;
     a.max_pages = max_pages; a.xq_out = xq_out; a.xh_out = xh_out; a.out_mcap = out_mcap; a.y_out = y_out;
-    a.dbg = g_pt_dbg;
-    a.stamps = g_pt_stamps;
     a.tr = dl_trace_next(TR_ATT);
     alignas(64) CUtensorMap kmap, vmap;
     const long long rows = (long long)n_cache_pages * n_kv_heads * 32;
     if (pt_make_map(&kmap, k_cache, rows, PT_HS, false) != 0 || pt_make_map(&vmap, v_cache, rows, PT_HS, false) != 0) return -1;
-    const size_t smem = (1 + 2 * PT_STAGES) * PT_TILE_BYTES + 24 * 8 + 4 * PT_ROWS * 4;
+    const size_t smem = PT_SMEM;
     static bool set = false;
     if (!set) {
         cudaError_t e = cudaFuncSetAttribute(attention_prefill_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -691,7 +849,8 @@ extern "C" int dl_attention_prefill_tc(const float* q, int M, int n_heads, int n
         set = true;
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)((M + PT_ROWS - 1) / PT_ROWS + PT_MAX_SEG), (unsigned)n_heads);      // upper bound of the tiles of all segments
+    const long long most = ((long long)(M + PT_ROWS - 1) / PT_ROWS + PT_MAX_SEG - 1) * n_heads;        // upper bound of the tiles of all segments
+    cfg.gridDim = dim3((unsigned)(most < dl_device_sm_count() ? most : dl_device_sm_count()));
     cfg.blockDim = dim3(PT_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = (cudaStream_t)stream;
@@ -715,13 +874,14 @@ int dl_window_prefill_tc_supported(const DlWindowAttnArgs& a, int rq) {
 }
 
 // The tiles of more than 16 stacked rows; launched behind the kernel that takes the others (programmatic launch: they run side by side).
-int dl_window_prefill_tc(const DlWindowAttnArgs& w, const int* tile_rows, int n_tiles, int rq, cudaStream_t stream) {
+int dl_window_prefill_tc(const DlWindowAttnArgs& w, const int* tile_rows, int n_tiles, int rq, int group, int n_splits, float* partial, cudaStream_t stream) {
     PtLineArgs a;
     a.w = w; a.tile_rows = tile_rows; a.n_tiles = n_tiles; a.rq = rq; a.rep = w.heads / w.kv_heads;
+    a.group = group; a.partial = partial;
     alignas(64) CUtensorMap map;
     // the cache's page count is not known here; every copy reads a page that the block table names
     if (pt_make_map(&map, w.cache, 1ll << 31, 2 * PT_HS, true) != 0) return -1;
-    const size_t smem = (1 + 2 * PT_STAGES) * PT_TILE_BYTES + 24 * 8 + 4 * PT_ROWS * 4;
+    const size_t smem = PT_SMEM;
     static bool set = false;
     if (!set) {
         cudaError_t e = cudaFuncSetAttribute(attention_prefill_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -729,7 +889,7 @@ int dl_window_prefill_tc(const DlWindowAttnArgs& w, const int* tile_rows, int n_
         set = true;
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)n_tiles, (unsigned)w.kv_heads);
+    cfg.gridDim = dim3((unsigned)n_tiles, (unsigned)w.kv_heads, (unsigned)n_splits);
     cfg.blockDim = dim3(PT_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;

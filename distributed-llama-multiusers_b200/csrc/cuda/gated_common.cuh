@@ -1,6 +1,7 @@
 // Pieces shared by the recurrences with data-dependent gates (gated_scan.cu, delta_scan.cu): how a row's query, key and decay are
 // formed, how a sequence is cut into chunks, and the scores inside a chunk under decays per channel.
 #pragma once
+#include "f32_pairs.cuh"
 #include "layer_common.cuh"
 #include "../../../include/dllama_b200.h"
 
@@ -163,15 +164,6 @@ __device__ __forceinline__ void gated_stage_rows(const DlGatedArgs& a, const int
         }
     }
 }
-
-// two f32 in a register pair: one instruction, two multiply-adds, each rounded as fmaf does
-typedef unsigned long long pair_f;
-__device__ __forceinline__ pair_f pair_of(float lo, float hi) { pair_f r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi)); return r; }
-__device__ __forceinline__ float pair_sum(pair_f v) { float lo, hi; asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); return lo + hi; }
-__device__ __forceinline__ pair_f fma2(pair_f x, pair_f y, pair_f z) { pair_f r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(x), "l"(y), "l"(z)); return r; }
-__device__ __forceinline__ pair_f mul2(pair_f x, pair_f y) { pair_f r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(x), "l"(y)); return r; }
-__device__ __forceinline__ pair_f ld_pair(const float* p) { return *reinterpret_cast<const pair_f*>(p); }
-__device__ __forceinline__ void st_pair(float* p, pair_f v) { *reinterpret_cast<pair_f*>(p) = v; }
 
 __device__ __forceinline__ float dot4(float4 x, float4 y, float acc) { return fmaf(x.x, y.x, fmaf(x.y, y.y, fmaf(x.z, y.z, fmaf(x.w, y.w, acc)))); }
 

@@ -547,7 +547,7 @@ __device__ __forceinline__ void window_small_tile(const DlWindowAttnArgs& a, con
 
 template <int DK>
 __global__ void __launch_bounds__(128, 4) window_attention_mma_kernel(DlWindowAttnArgs a, const int* __restrict__ tile_rows, int rq,
-                                                                   int n_splits, float* __restrict__ partial, int only_small, int max_small) {
+                                                                   int n_splits, float* __restrict__ partial, int only_small, int max_small) {      // only_small: 0, or the list tiles that a CTA of the other kernel may take
     constexpr int D = 16 * DK, NV = D / 8;
     extern __shared__ __align__(16) uint8_t smraw[];
     __shared__ int s_row[WM_ROWS];
@@ -577,8 +577,8 @@ __global__ void __launch_bounds__(128, 4) window_attention_mma_kernel(DlWindowAt
         pg_hi = min(pg_hi, pg_lo + per - 1);
     }
     if (n_rows * rep <= 16) {            // decoding: one 16-row tile, the warps share the tokens
-        if (only_small && (tile & 1) && window_tiles_join(a, tile_rows, rq, tile - 1, window_tile_count(tile_rows, gridDim.x, rq, tile - 1), n_rows))
-            return;                      // the end of a prompt: attention_prefill_tc.cu takes it along with the full tile ahead of it
+        if (only_small && (tile & (only_small - 1)) && window_tiles_join(a, tile_rows, rq, tile - 1, window_tile_count(tile_rows, gridDim.x, rq, tile - 1), n_rows))
+            return;                      // the end of a prompt: attention_prefill_tc.cu takes it along with the full tiles ahead of it
         if (pg_lo > pg_hi) {             // a share without pages (of several): the merge leaves it out by its sum
             if (threadIdx.x < n_rows * rep) {
                 float* dst = partial + ((((size_t)tile * a.kv_heads + g) * n_splits + blockIdx.z) * WM_ROWS + threadIdx.x) * (D + 2) + D;
@@ -760,6 +760,7 @@ __global__ void __launch_bounds__(128) window_merge_kernel(DlWindowAttnArgs a, c
     if (m < 0) return;
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const float* base = partial + ((size_t)tile * a.kv_heads + g) * n_splits * WM_ROWS * (D + 2);
+    if (base[(size_t)r * rep * (D + 2) + D + 1] == -2.f) return;              // written already, without shares
     for (int hg = threadIdx.x >> 5; hg < rep; hg += blockDim.x >> 5) {        // a warp per head, a lane per share
         const int k = threadIdx.x & 31;
         const float* p = base + ((size_t)k * WM_ROWS + r * rep + hg) * (D + 2) + D;
@@ -789,7 +790,7 @@ __global__ void __launch_bounds__(128) window_merge_kernel(DlWindowAttnArgs a, c
 
 // attention_prefill_tc.cu
 int dl_window_prefill_tc_supported(const DlWindowAttnArgs& a, int rq);
-int dl_window_prefill_tc(const DlWindowAttnArgs& a, const int* tile_rows, int n_tiles, int rq, cudaStream_t stream);
+int dl_window_prefill_tc(const DlWindowAttnArgs& a, const int* tile_rows, int n_tiles, int rq, int group, int n_splits, float* partial, cudaStream_t stream);
 
 // rows of one sequence per tile: as many positions as fit 64 stacked (position, head) pairs
 extern "C" int dl_window_tc_rows(int heads, int kv_heads) {
@@ -826,8 +827,9 @@ extern "C" int dl_window_attention_tc(const DlWindowAttnArgs* args, const int* t
     if (n_tiles < 1) return 0;
     if (n_splits < 1 || n_splits > WM_MAX_SPLITS || (n_splits > 1 && partial == nullptr)) { dl_set_error("dl_window_attention_tc: n_splits %d without scratch", n_splits); return -1; }
     const size_t smem = ((size_t)2 * WA_PAGE * wm_line_stride(a.dim + (a.vdim > 0 ? a.vdim : a.rope_dims)) + (size_t)WM_ROWS * (a.dim + 8)) * sizeof(__nv_bfloat16);
-    // tiles enough for the chip without sharing pages are prompt portions (or very many users, whose tiles stay here): tcgen05, 128 stacked rows
-    const bool tc5 = n_splits == 1 && dl_window_prefill_tc_supported(a, rq) == 0;
+    // tiles of more than 16 stacked rows are prompt portions: tcgen05, 128 or 256 stacked rows to a CTA
+    const bool tc5 = dl_window_prefill_tc_supported(a, rq) == 0;
+    const int group = (n_tiles + 1) / 2 * a.kv_heads > dl_device_sm_count() ? 4 : 2;
     const int max_small = (3 * dl_device_sm_count() + n_tiles * a.kv_heads - 1) / (n_tiles * a.kv_heads);
     dim3 grid(n_tiles, a.kv_heads, n_splits);
     cudaStream_t st = (cudaStream_t)stream;
@@ -835,7 +837,7 @@ extern "C" int dl_window_attention_tc(const DlWindowAttnArgs* args, const int* t
 #define WM_CASE(DK_)                                                                                                      \
     case DK_:                                                                                                             \
         if (smem > 48 * 1024) cudaFuncSetAttribute(window_attention_mma_kernel<DK_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-        window_attention_mma_kernel<DK_><<<grid, 128, smem, st>>>(a, tile_rows, rq, n_splits, partial, tc5 ? 1 : 0, max_small);                  \
+        window_attention_mma_kernel<DK_><<<grid, 128, smem, st>>>(a, tile_rows, rq, n_splits, partial, tc5 ? group : 0, max_small);                  \
         break;
         WM_CASE(1) WM_CASE(2) WM_CASE(3) WM_CASE(4) WM_CASE(6) WM_CASE(8)
 #undef WM_CASE
@@ -843,7 +845,7 @@ extern "C" int dl_window_attention_tc(const DlWindowAttnArgs* args, const int* t
     }
     if (tc5) {
         LAYER_CHECK_LAUNCH("dl_window_attention_tc");
-        const int rc = dl_window_prefill_tc(a, tile_rows, n_tiles, rq, st);
+        const int rc = dl_window_prefill_tc(a, tile_rows, n_tiles, rq, group, n_splits, partial, st);
         if (rc != 0) return rc;
     }
     if (n_splits > 1) {

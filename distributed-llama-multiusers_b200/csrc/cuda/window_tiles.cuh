@@ -11,8 +11,8 @@ __device__ __forceinline__ int window_tile_count(const int* tile_rows, int n_til
     return n;
 }
 
-// tile e (even, ne rows) is full and tile e + 1 (no rows) continues its sequence: the tcgen05 kernel takes both as one, however few rows
-// the second has
+// tile e (ne rows) is full and tile e + 1 (no rows) continues its sequence: the tcgen05 kernel takes both in one run, however few rows
+// the second has, unless e + 1 starts a group
 __device__ __forceinline__ bool window_tiles_join(const DlWindowAttnArgs& a, const int* tile_rows, int rq, int e, int ne, int no) {
     if (ne != rq || no == 0) return false;
     const int me = tile_rows[(size_t)e * rq], mo = tile_rows[(size_t)(e + 1) * rq];
