@@ -73,8 +73,9 @@ struct PtLineArgs {
     DlWindowAttnArgs w;
     const int* tile_rows;      // [n_tiles][rq], -1 where a tile has fewer rows
     int n_tiles, rq, rep;
-    int group;                 // list tiles that one CTA may take: 2 or 4
-    float* partial;            // [n_tiles][kv_heads][grid.z][64][130] where grid.z > 1: sums, reference maximum, sum of weights
+    int group;                 // list tiles of a CTA: 2 or 4
+    int n_splits;
+    float* partial;            // [n_tiles][kv_heads][n_splits][64][130] where n_splits > 1: sums, reference maximum, sum of weights
 };
 template <bool LINES> struct PtKernelArgs { typedef PtArgs T; };
 template <> struct PtKernelArgs<true> { typedef PtLineArgs T; };
@@ -219,6 +220,45 @@ DL_DEVINL void pt_q80_block(const float (&v)[32], int m, int kblock, int mcap, u
     }
 }
 
+// The eight MMAs of a group (K = 128) by one thread of the converged warp.  What bounds a group of 128 x 128 x 16 MMAs is their issue: inside an
+// `if (elect)` every descriptor passes through registers of its own into the uniform ones, 110 clk an MMA that takes 64; predicated in convergent code
+// they are formed there.
+// D += A B^T, both operands 128-byte-swizzled half tiles 16 KB apart (32 B of a row per MMA)
+DL_DEVINL void pt_mma_ss(uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t desc_hi, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, q, r;\n\t.reg .b32 x, y;\n\t.reg .b64 a, b;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\tsetp.ne.b32 q, %5, 0;\n\tsetp.eq.b32 r, 0, 0;\n\t"
+        "add.u32 x, %1, 0; add.u32 y, %2, 0; mov.b64 a, {x, %3}; mov.b64 b, {y, %3}; @p tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, q;\n\t"
+        "add.u32 x, %1, 2; add.u32 y, %2, 2; mov.b64 a, {x, %3}; mov.b64 b, {y, %3}; @p tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, r;\n\t"
+        "add.u32 x, %1, 4; add.u32 y, %2, 4; mov.b64 a, {x, %3}; mov.b64 b, {y, %3}; @p tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, r;\n\t"
+        "add.u32 x, %1, 6; add.u32 y, %2, 6; mov.b64 a, {x, %3}; mov.b64 b, {y, %3}; @p tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, r;\n\t"
+        "add.u32 x, %1, 1024; add.u32 y, %2, 1024; mov.b64 a, {x, %3}; mov.b64 b, {y, %3}; @p tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, r;\n\t"
+        "add.u32 x, %1, 1026; add.u32 y, %2, 1026; mov.b64 a, {x, %3}; mov.b64 b, {y, %3}; @p tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, r;\n\t"
+        "add.u32 x, %1, 1028; add.u32 y, %2, 1028; mov.b64 a, {x, %3}; mov.b64 b, {y, %3}; @p tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, r;\n\t"
+        "add.u32 x, %1, 1030; add.u32 y, %2, 1030; mov.b64 a, {x, %3}; mov.b64 b, {y, %3}; @p tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, r;\n\t}"
+        ::"r"(d), "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// D += A B, A in tensor memory (8 columns per MMA), B MN-major (two 8-token groups of 1024 B per MMA)
+DL_DEVINL void pt_mma_ts(uint32_t d, uint32_t a, uint32_t b_lo, uint32_t desc_hi, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, q, r;\n\t.reg .b32 x, y;\n\t.reg .b64 a, b;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\tsetp.ne.b32 q, %5, 0;\n\tsetp.eq.b32 r, 0, 0;\n\t"
+        "add.u32 x, %1, 0; add.u32 y, %2, 0; mov.b64 b, {y, %3}; @p tcgen05.mma.cta_group::1.kind::f16 [%0], [x], b, %4, q;\n\t"
+        "add.u32 x, %1, 8; add.u32 y, %2, 128; mov.b64 b, {y, %3}; @p tcgen05.mma.cta_group::1.kind::f16 [%0], [x], b, %4, r;\n\t"
+        "add.u32 x, %1, 16; add.u32 y, %2, 256; mov.b64 b, {y, %3}; @p tcgen05.mma.cta_group::1.kind::f16 [%0], [x], b, %4, r;\n\t"
+        "add.u32 x, %1, 24; add.u32 y, %2, 384; mov.b64 b, {y, %3}; @p tcgen05.mma.cta_group::1.kind::f16 [%0], [x], b, %4, r;\n\t"
+        "add.u32 x, %1, 32; add.u32 y, %2, 512; mov.b64 b, {y, %3}; @p tcgen05.mma.cta_group::1.kind::f16 [%0], [x], b, %4, r;\n\t"
+        "add.u32 x, %1, 40; add.u32 y, %2, 640; mov.b64 b, {y, %3}; @p tcgen05.mma.cta_group::1.kind::f16 [%0], [x], b, %4, r;\n\t"
+        "add.u32 x, %1, 48; add.u32 y, %2, 768; mov.b64 b, {y, %3}; @p tcgen05.mma.cta_group::1.kind::f16 [%0], [x], b, %4, r;\n\t"
+        "add.u32 x, %1, 56; add.u32 y, %2, 896; mov.b64 b, {y, %3}; @p tcgen05.mma.cta_group::1.kind::f16 [%0], [x], b, %4, r;\n\t}"
+        ::"r"(d), "r"(a), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+DL_DEVINL void pt_commit(uint64_t* bar) {
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\t@p tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)) : "memory");
+}
+
 // What a CTA works on: two query tiles of up to 128 (stacked) rows that meet the same keys and values, and the steps that they see.
 struct PtItem {
     int kvh, p0, slot, seq_end;            // key/value head; position of the first row of the segment (or run); tokens of the sequence that exist
@@ -274,49 +314,54 @@ DL_DEVINL bool pt_item(const PtArgs& a, const int (*seg)[4], int n_seg, int idx,
     return false;
 }
 
-// Layer-list models: the run of list tiles that this CTA owns and the share of its steps; false where there is nothing to do.  (By whole warps)
-DL_DEVINL bool pt_run(const PtLineArgs& a, PtItem& it, int& shares) {
+// Layer-list models: the runs of consecutive positions among the CTA's list tiles, [first tile, positions, first position, slot] each.  (By a whole warp)
+DL_DEVINL int pt_runs(const PtLineArgs& a, int (*runs)[4]) {
     const DlWindowAttnArgs& w = a.w;
-    const int t = (int)gridDim.x - 1 - (int)blockIdx.x, lane = threadIdx.x & 31;          // late tiles (long histories) first
-    // the tile ahead, this one and the three behind: rows of each, and where the first one is (a lane per tile)
-    int cnt[5] = {0, 0, 0, 0, 0}, m = 0, mine = 0;
+    const int t0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * a.group, lane = threadIdx.x & 31;          // late tiles (long histories) first
+    int cnt[4] = {0, 0, 0, 0}, m = -1;                           // rows of each tile; the first row of tile `lane`
 #pragma unroll
-    for (int u = 0; u < 5; u++) {
-        const int tu = t - 1 + u;
-        for (int r0 = 0; r0 < a.rq && tu >= 0 && tu < a.n_tiles; r0 += 32) {
-            const int row = r0 + lane < a.rq ? a.tile_rows[(size_t)tu * a.rq + r0 + lane] : -1;
+    for (int u = 0; u < 4; u++) {
+        for (int r0 = 0; r0 < a.rq && u < a.group && t0 + u < a.n_tiles; r0 += 32) {
+            const int row = r0 + lane < a.rq ? a.tile_rows[(size_t)(t0 + u) * a.rq + r0 + lane] : -1;
             cnt[u] += __popc(__ballot_sync(0xffffffffu, row >= 0));
             const int first = __shfl_sync(0xffffffffu, row, 0);
-            if (r0 == 0 && lane == u) { m = first; mine = first >= 0; }
+            if (r0 == 0 && lane == u) m = first;
         }
     }
-    const int pos = mine ? w.pos[m] : 0, slot = mine ? w.slot[m] : 0;
-    bool joined[5];                                              // tile u - 1 is full and u continues its sequence (window_tiles_join)
+    const int pos = m >= 0 ? w.pos[m] : 0, slot = m >= 0 ? w.slot[m] : 0;
+    int n = 0, run = 0, start = 0;
 #pragma unroll
-    for (int u = 1; u < 5; u++) {
-        const bool follows = __shfl_sync(0xffffffffu, pos, u - 1) + a.rq == __shfl_sync(0xffffffffu, pos, u) && __shfl_sync(0xffffffffu, slot, u - 1) == __shfl_sync(0xffffffffu, slot, u);
-        joined[u] = follows && cnt[u - 1] == a.rq && cnt[u] > 0 && ((t - 1 + u) & (a.group - 1)) != 0;
-    }
-    if (cnt[1] == 0 || joined[1]) return false;
-    int run = cnt[1];
-#pragma unroll
-    for (int u = 2; u < 5; u++) {
-        if (!joined[u]) break;
+    for (int u = 0; u < 4; u++) {
+        const int pu = __shfl_sync(0xffffffffu, pos, u), su = __shfl_sync(0xffffffffu, slot, u);
+        if (run == 0) start = u;
         run += cnt[u];
+        // does the next tile go on with this sequence (window_tiles_join)?
+        const bool more = u < 3 && cnt[u] == a.rq && cnt[u < 3 ? u + 1 : 3] > 0 && __shfl_sync(0xffffffffu, pos, u < 3 ? u + 1 : 3) == pu + a.rq && __shfl_sync(0xffffffffu, slot, u < 3 ? u + 1 : 3) == su;
+        const int p_start = __shfl_sync(0xffffffffu, pos, start);
+        if (more) continue;
+        if (run * a.rep > 16) {                                  // (else a decoding tile, which belongs to the other kernel)
+            if (lane == 0) { runs[n][0] = t0 + start; runs[n][1] = run; runs[n][2] = p_start; runs[n][3] = su; }
+            n++;
+        }
+        run = 0;
     }
-    if (run * a.rep <= 16) return false;                         // a decoding tile, which belongs to the other kernel
-    it.begin = t * a.rq;
-    it.rows = run * a.rep;
-    it.p0 = __shfl_sync(0xffffffffu, pos, 1);
-    it.slot = __shfl_sync(0xffffffffu, slot, 1);
-    it.seq_end = it.p0 + run;                                    // what lies behind was not written yet, or is of no use here
+    return n;
+}
+// the item of a run, and into how many shares (grid.z) its steps go: no more than leave each PT_SHARE_STEPS, so that a short run needs no merge
+DL_DEVINL void pt_run_item(const PtLineArgs& a, const int (&run)[4], PtItem& it, int& shares) {
+    const DlWindowAttnArgs& w = a.w;
+    it.begin = run[0] * a.rq;
+    it.rows = run[1] * a.rep;
+    it.p0 = run[2];
+    it.slot = run[3];
+    it.seq_end = it.p0 + run[1];                                 // what lies behind was not written yet, or is of no use here
     it.kvh = blockIdx.y;
     int lo[2], j[2];
 #pragma unroll
     for (int u = 0; u < 2; u++) {
         it.row0[u] = u * PT_ROWS;
         it.head[u] = 0;
-        const int p = it.p0 + u * PT_ROWS / a.rep, last = it.p0 + min((u + 1) * PT_ROWS / a.rep, run) - 1;
+        const int p = it.p0 + u * PT_ROWS / a.rep, last = it.p0 + min((u + 1) * PT_ROWS / a.rep, run[1]) - 1;
         lo[u] = w.window > 0 ? max(0, p - w.window + 1) : 0;
         if (w.chunk > 0) lo[u] = max(lo[u], p / w.chunk * w.chunk);
         j[u] = it.row0[u] < it.rows ? last / PT_KV + 1 : 0;
@@ -324,7 +369,6 @@ DL_DEVINL bool pt_run(const PtLineArgs& a, PtItem& it, int& shares) {
     it.first_page = lo[0] / 32;                                  // (tile 1 starts no earlier)
     it.j0 = lo[0] / PT_KV;
     it.J = max(j[0], j[1]) - it.j0;
-    // shares of the steps by grid.z: no more than leave each PT_SHARE_STEPS, so that a short run is done without a merge
     shares = max(1, min((int)gridDim.z, it.J / PT_SHARE_STEPS));
     const int per = (it.J + shares - 1) / shares, z0 = min(it.J, (int)blockIdx.z * per), z1 = min(it.J, z0 + per);
 #pragma unroll
@@ -335,7 +379,6 @@ DL_DEVINL bool pt_run(const PtLineArgs& a, PtItem& it, int& shares) {
     it.j0 += z0;
     it.J = z1 - z0;
     it.first_page = max(it.first_page, it.j0 * (PT_KV / 32));
-    return (int)blockIdx.z < shares || shares > 1;               // (a share without steps says so in its partial sums)
 }
 
 // Queries of 32 rows into the tile's K-major, swizzled image: lane i holds the address of row r0 + i; N rows are in flight, a row a load
@@ -398,8 +441,6 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
         mbar_init(s_empty, 128);
         mbar_fence_init();
     }
-    int n_seg = 0, shares = 1;
-    PtItem one;                                                  // LINES: a CTA has one item
     if constexpr (!LINES) {
         pdl_wait();                                              // q, this chunk's KV rows and meta come from earlier kernels
         if (warp == 1) {
@@ -418,7 +459,12 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
         // follows this grid must follow that one too, so this grid may not end ahead of it: a CTA with work waits when it is done, and the
         // first CTA waits even without -- one is enough, a grid ends with its last CTA, and all of the idle ones would keep an SM each
         // from those with work)
-        if (!pt_run(a, one, shares)) {
+        if (warp == 1) {
+            const int n = pt_runs(a, seg);
+            if (lane == 0) n_seg_s = n;
+        }
+        __syncthreads();
+        if (n_seg_s == 0) {
             if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) pdl_wait();
             return;
         }
@@ -428,18 +474,19 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
     __syncthreads();
     tc_fence_after();
     const PtWaits wait = {&gave_up_s, globaltimer_ns()};
-    if constexpr (!LINES) n_seg = n_seg_s;
+    const int n_seg = n_seg_s;
+    int shares = 1;                                              // LINES: of the item
     // the items of this CTA, in the same order for every role; rounds run back and forth over the CTAs, so that a long item goes with a short one
     auto item_at = [&](int round, PtItem& it) {
         if constexpr (LINES) {
-            it = one;
-            return round == 0;
+            if (round < n_seg) pt_run_item(a, seg[round], it, shares);
+            return round < n_seg;
         } else {
             const int G = gridDim.x, b = blockIdx.x;
             return pt_item(a, seg, n_seg, round * G + ((round & 1) ? G - 1 - b : b), it);
         }
     };
-    const uint32_t tmem_base = *tmem_holder;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_holder, 0);
     // TMEM columns: outputs at 256 + 128 t.  One buffer of scores at 0, taken in turn, and probabilities at 128 + 64 t; LINES, whose
     // probabilities need 128 columns: scores, then probabilities, at 128 t
     const auto t_s = [&](int t) { return tmem_base + (LINES ? t * 128 : 0); };
@@ -570,15 +617,20 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
             float* out = nullptr;                                // this thread's row; null: none
             bool vec = true;                                     // 16-byte rows
             if constexpr (LINES) {
-                if (row0 >= it.rows) continue;
+                if (row0 >= it.rows || (shares == 1 && blockIdx.z > 0)) continue;
                 out = a.w.out + (size_t)m_row * a.w.ldo + h_row * PT_HS;
                 vec = ((uintptr_t)a.w.out & 15) == 0 && (a.w.ldo & 3) == 0;
-                if (gridDim.z > 1) {                             // a stacked row's slot among the list tile's partial sums
+                if (a.n_splits > 1) {                            // a stacked row's slot among the list tile's partial sums
+                    constexpr int step = PT_ROWS / 2 * (PT_HS + 2);
                     const int u = it.begin / a.rq + r_live / (PT_ROWS / 2);
-                    float* part = a.partial + ((((size_t)u * a.w.kv_heads + it.kvh) * gridDim.z + blockIdx.z) * (PT_ROWS / 2) + r_live % (PT_ROWS / 2)) * (PT_HS + 2);
+                    float* part = a.partial + (((size_t)u * a.w.kv_heads + it.kvh) * a.n_splits + blockIdx.z) * step + r_live % (PT_ROWS / 2) * (PT_HS + 2);
                     if (r_abs < it.rows) {                       // (-2: no merge, -1: nothing in this share)
                         part[PT_HS] = m_used * 0.6931471805599453f;
                         part[PT_HS + 1] = shares == 1 ? -2.f : jb > ja ? l : -1.f;
+                        for (int z = gridDim.z; blockIdx.z == 0 && shares > 1 && z < a.n_splits; z++) {
+                            part[(size_t)z * step + PT_HS] = -INFINITY;
+                            part[(size_t)z * step + PT_HS + 1] = -1.f;
+                        }
                     }
                     if (shares > 1) { out = part; vec = false; }
                 }
@@ -629,61 +681,41 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
         if (warp == 8) {
             // ---------------- MMAs, all by one thread: what it issues runs in that order ----------------
             const uint32_t idesc_s = pt_idesc(PT_ROWS, PT_KV, 0, LINES), idesc_pv = pt_idesc(PT_ROWS, PT_HS, 1, LINES);
+            const uint32_t q_lo = ((smem_u32(q_s) & 0x3FFFFu) >> 4) | (1u << 16), k_lo = ((smem_u32(k_s) & 0x3FFFFu) >> 4) | (1u << 16);
+            const uint32_t v_lo = ((smem_u32(v_s) & 0x3FFFFu) >> 4) | ((16384u >> 4) << 16);
             uint32_t g = 0, n_s = 0, ns[2] = {0, 0}, nq[2] = {0, 0};      // steps, scores, steps of a tile, items of a tile so far
             PtItem it;
             for (int round = 0; item_at(round, it); round++) {
                 auto on = [&](int t, int j) { return j >= it.ja[t] && j < it.jb[t]; };
                 auto scores = [&](int t, int j) {                // S = Q K^T of a step
+                    const int st = (g + j) & 1;
                     if (!on(t, j)) {
-                        if (LINES && t == 1 && j < it.J) {       // (a step that only tile 0 sees)
-                            if (elect_one()) umma_commit(&k_empty[(g + j) & 1]);
-                            __syncwarp();
-                        }
+                        if (LINES && t == 1 && j < it.J) pt_commit(&k_empty[st]);      // (a step that only tile 0 sees)
                         return;
                     }
-                    wait(&k_full[(g + j) & 1], ((g + j) >> 1) & 1);
+                    wait(&k_full[st], ((g + j) >> 1) & 1);
                     if (j == it.ja[t]) wait(&q_full[t], nq[t]++ & 1);
                     if (!LINES && n_s > 0) wait(s_empty, (n_s - 1) & 1);
                     n_s++;
                     tc_fence_after();
-                    if (elect_one()) {
-                        const uint32_t a_lo = ((smem_u32(q_s + t * PT_TILE_BYTES) & 0x3FFFFu) >> 4) | (1u << 16);
-                        const uint32_t b_lo = ((smem_u32(k_s + ((g + j) & 1) * PT_TILE_BYTES) & 0x3FFFFu) >> 4) | (1u << 16);
-#pragma unroll
-                        for (int k = 0; k < 8; k++) {      // K = 16 per MMA: 32 B inside the swizzled row, the second half tile after four
-                            const uint32_t off = (uint32_t)((k >> 2) * (16384 >> 4) + (k & 3) * 2);
-                            uint64_t da, db;
-                            asm("mov.b64 %0, {%1, %2};" : "=l"(da) : "r"(a_lo + off), "r"(desc_hi));
-                            asm("mov.b64 %0, {%1, %2};" : "=l"(db) : "r"(b_lo + off), "r"(desc_hi));
-                            umma_f16_ss(t_s(t), da, db, idesc_s, k > 0 ? 1u : 0u);
-                        }
-                        umma_commit(&s_full[t]);
-                        if (t == 1 || (!LINES && !on(1, j))) umma_commit(&k_empty[(g + j) & 1]);
-                        if (j + 1 == it.jb[t]) umma_commit(&q_empty[t]);
-                    }
                     __syncwarp();
+                    pt_mma_ss(t_s(t), q_lo + t * (PT_TILE_BYTES >> 4), k_lo + st * (PT_TILE_BYTES >> 4), desc_hi, idesc_s, 0);
+                    pt_commit(&s_full[t]);
+                    if (t == 1 || (!LINES && !on(1, j))) pt_commit(&k_empty[st]);
+                    if (j + 1 == it.jb[t]) pt_commit(&q_empty[t]);
                 };
                 auto outputs = [&](int t, int j) {               // O += P V of a step
                     const int st = (g + j) & 1;
                     if (on(t, j)) {
                         wait(&p_full[t], ns[t]++ & 1);
                         tc_fence_after();
+                        __syncwarp();
+                        const uint32_t b_lo = v_lo + st * (PT_TILE_BYTES >> 4), T_O = tmem_base + 256 + t * 128;
+                        pt_mma_ts(T_O, t_p(t), b_lo, desc_hi, idesc_pv, j > it.ja[t] ? 1u : 0u);
+                        if constexpr (LINES) pt_mma_ts(T_O, t_p(t) + 64, b_lo, desc_hi, idesc_pv, 1u);
+                        pt_commit(&o_full[t]);
                     }
-                    if (elect_one()) {
-                        if (on(t, j)) {
-                            const uint32_t b_lo = ((smem_u32(v_s + st * PT_TILE_BYTES) & 0x3FFFFu) >> 4) | ((16384u >> 4) << 16), T_O = tmem_base + 256 + t * 128;
-#pragma unroll
-                            for (int k = 0; k < 8; k++) {      // 16 tokens per MMA: 8 TMEM columns of P, two 8-token groups (2048 B) of V
-                                uint64_t db;
-                                asm("mov.b64 %0, {%1, %2};" : "=l"(db) : "r"(b_lo + k * 128), "r"(desc_hi));
-                                umma_f16_ts(T_O, t_p(t) + k * 8, db, idesc_pv, (j > it.ja[t] || k > 0) ? 1u : 0u);
-                                if constexpr (LINES) umma_f16_ts(T_O, t_p(t) + 64 + k * 8, db, idesc_pv, 1u);
-                            }
-                            umma_commit(&o_full[t]);
-                        }
-                        if (t == 1) umma_commit(&v_empty[st]);
-                    }
-                    __syncwarp();
+                    if (t == 1) pt_commit(&v_empty[st]);
                 };
                 scores(0, 0);
                 scores(1, 0);
@@ -877,7 +909,9 @@ int dl_window_prefill_tc_supported(const DlWindowAttnArgs& a, int rq) {
 int dl_window_prefill_tc(const DlWindowAttnArgs& w, const int* tile_rows, int n_tiles, int rq, int group, int n_splits, float* partial, cudaStream_t stream) {
     PtLineArgs a;
     a.w = w; a.tile_rows = tile_rows; a.n_tiles = n_tiles; a.rq = rq; a.rep = w.heads / w.kv_heads;
-    a.group = group; a.partial = partial;
+    a.group = group; a.n_splits = n_splits; a.partial = partial;
+    // page shares no more than there are SMs for
+    const int groups = (n_tiles + group - 1) / group, spare = dl_device_sm_count() / (groups * w.kv_heads), z = spare < 1 ? 1 : spare < n_splits ? spare : n_splits;
     alignas(64) CUtensorMap map;
     // the cache's page count is not known here; every copy reads a page that the block table names
     if (pt_make_map(&map, w.cache, 1ll << 31, 2 * PT_HS, true) != 0) return -1;
@@ -889,7 +923,7 @@ int dl_window_prefill_tc(const DlWindowAttnArgs& w, const int* tile_rows, int n_
         set = true;
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)n_tiles, (unsigned)w.kv_heads, (unsigned)n_splits);
+    cfg.gridDim = dim3((unsigned)groups, (unsigned)w.kv_heads, (unsigned)z);
     cfg.blockDim = dim3(PT_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;

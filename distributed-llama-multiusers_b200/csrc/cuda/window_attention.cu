@@ -827,9 +827,9 @@ extern "C" int dl_window_attention_tc(const DlWindowAttnArgs* args, const int* t
     if (n_tiles < 1) return 0;
     if (n_splits < 1 || n_splits > WM_MAX_SPLITS || (n_splits > 1 && partial == nullptr)) { dl_set_error("dl_window_attention_tc: n_splits %d without scratch", n_splits); return -1; }
     const size_t smem = ((size_t)2 * WA_PAGE * wm_line_stride(a.dim + (a.vdim > 0 ? a.vdim : a.rope_dims)) + (size_t)WM_ROWS * (a.dim + 8)) * sizeof(__nv_bfloat16);
-    // tiles of more than 16 stacked rows are prompt portions: tcgen05, 128 or 256 stacked rows to a CTA
+    // tiles of more than 16 stacked rows are prompt portions: tcgen05, 128 stacked rows to a CTA, 256 where that fills the SMs
     const bool tc5 = dl_window_prefill_tc_supported(a, rq) == 0;
-    const int group = (n_tiles + 1) / 2 * a.kv_heads > dl_device_sm_count() ? 4 : 2;
+    const int group = (n_tiles + 1) / 2 * a.kv_heads <= dl_device_sm_count() ? 2 : 4;
     const int max_small = (3 * dl_device_sm_count() + n_tiles * a.kv_heads - 1) / (n_tiles * a.kv_heads);
     dim3 grid(n_tiles, a.kv_heads, n_splits);
     cudaStream_t st = (cudaStream_t)stream;
