@@ -310,6 +310,28 @@ DL_DEVINL void umma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                  : "memory");
 }
+// The eight MMAs (K = 16 each) of a 128-wide k-tile, and a commit, by one thread of a CONVERGED warp: predicated, so that the descriptors are
+// formed in uniform registers.  Inside an `if (elect)` each of them passes through a register of its own into the uniform ones first, about
+// 110 clk per MMA: what bounds an issuer of short MMAs.  Operands in shared memory: K-major core matrices 128 B apart (two per MMA).
+DL_DEVINL void umma_f16_ss_x8(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t desc_hi, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, q, r;\n\t.reg .b32 x, y;\n\t.reg .b64 a, b;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\tsetp.ne.b32 q, %5, 0;\n\tsetp.eq.b32 r, 0, 0;\n\t"
+        "add.u32 x, %1, 0; add.u32 y, %2, 0; mov.b64 a, {x, %3}; mov.b64 b, {y, %3}; @p tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, q;\n\t"
+        "add.u32 x, %1, 16; add.u32 y, %2, 16; mov.b64 a, {x, %3}; mov.b64 b, {y, %3}; @p tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, r;\n\t"
+        "add.u32 x, %1, 32; add.u32 y, %2, 32; mov.b64 a, {x, %3}; mov.b64 b, {y, %3}; @p tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, r;\n\t"
+        "add.u32 x, %1, 48; add.u32 y, %2, 48; mov.b64 a, {x, %3}; mov.b64 b, {y, %3}; @p tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, r;\n\t"
+        "add.u32 x, %1, 64; add.u32 y, %2, 64; mov.b64 a, {x, %3}; mov.b64 b, {y, %3}; @p tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, r;\n\t"
+        "add.u32 x, %1, 80; add.u32 y, %2, 80; mov.b64 a, {x, %3}; mov.b64 b, {y, %3}; @p tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, r;\n\t"
+        "add.u32 x, %1, 96; add.u32 y, %2, 96; mov.b64 a, {x, %3}; mov.b64 b, {y, %3}; @p tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, r;\n\t"
+        "add.u32 x, %1, 112; add.u32 y, %2, 112; mov.b64 a, {x, %3}; mov.b64 b, {y, %3}; @p tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, r;\n\t}"
+        ::"r"(tmem_d), "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+DL_DEVINL void umma_commit_elected(uint64_t* bar) {
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\t@p tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar))
+                 : "memory");
+}
 // 32 lanes x 32-bit x 8 consecutive columns -> 8 registers per thread
 DL_DEVINL void tmem_ld_32x32b_x8(uint32_t taddr, uint32_t (&v)[8]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
