@@ -75,6 +75,7 @@ struct PtLineArgs {
     int n_tiles, rq, rep;
     int group;                 // list tiles of a CTA: 2 or 4
     int n_splits;
+    int least;                 // runs of no more stacked rows belong to the other kernel (0: there is none)
     float* partial;            // [n_tiles][kv_heads][n_splits][64][130] where n_splits > 1: sums, reference maximum, sum of weights
 };
 template <bool LINES> struct PtKernelArgs { typedef PtArgs T; };
@@ -339,7 +340,7 @@ DL_DEVINL int pt_runs(const PtLineArgs& a, int (*runs)[4]) {
         const bool more = u < 3 && cnt[u] == a.rq && cnt[u < 3 ? u + 1 : 3] > 0 && __shfl_sync(0xffffffffu, pos, u < 3 ? u + 1 : 3) == pu + a.rq && __shfl_sync(0xffffffffu, slot, u < 3 ? u + 1 : 3) == su;
         const int p_start = __shfl_sync(0xffffffffu, pos, start);
         if (more) continue;
-        if (run * a.rep > 16) {                                  // (else a decoding tile, which belongs to the other kernel)
+        if (run * a.rep > a.least) {
             if (lane == 0) { runs[n][0] = t0 + start; runs[n][1] = run; runs[n][2] = p_start; runs[n][3] = su; }
             n++;
         }
@@ -905,13 +906,22 @@ int dl_window_prefill_tc_supported(const DlWindowAttnArgs& a, int rq) {
                    ((uintptr_t)a.cache & 15) == 0 ? 0 : -1;
 }
 
-// The tiles of more than 16 stacked rows; launched behind the kernel that takes the others (programmatic launch: they run side by side).
-int dl_window_prefill_tc(const DlWindowAttnArgs& w, const int* tile_rows, int n_tiles, int rq, int group, int n_splits, float* partial, cudaStream_t stream) {
+// The most shares that a run's steps go into: none where the SMs are taken, or where no run can be long enough.
+int dl_window_prefill_tc_shares(const DlWindowAttnArgs& w, int n_tiles, int group, int n_splits) {
+    const int ctas = (n_tiles + group - 1) / group * w.kv_heads, spare = dl_device_sm_count() / ctas;
+    const long long seen = w.window > 0 && w.window < w.max_pages * 32ll ? w.window + 2 * PT_ROWS : w.max_pages * 32ll;
+    const long long most = (seen / PT_KV + 2) / PT_SHARE_STEPS, z = spare < most ? spare : most;
+    return z < 1 ? 1 : z < n_splits ? (int)z : n_splits;
+}
+
+// The tiles of more than 16 stacked rows, launched behind the kernel that takes the others (programmatic launch: they run side by side), or
+// (alone) all of them.
+int dl_window_prefill_tc(const DlWindowAttnArgs& w, const int* tile_rows, int n_tiles, int rq, int group, int n_splits, float* partial, bool alone, cudaStream_t stream) {
     PtLineArgs a;
     a.w = w; a.tile_rows = tile_rows; a.n_tiles = n_tiles; a.rq = rq; a.rep = w.heads / w.kv_heads;
     a.group = group; a.n_splits = n_splits; a.partial = partial;
-    // page shares no more than there are SMs for
-    const int groups = (n_tiles + group - 1) / group, spare = dl_device_sm_count() / (groups * w.kv_heads), z = spare < 1 ? 1 : spare < n_splits ? spare : n_splits;
+    a.least = alone ? 0 : 16;
+    const int groups = (n_tiles + group - 1) / group, z = dl_window_prefill_tc_shares(w, n_tiles, group, n_splits);
     alignas(64) CUtensorMap map;
     // the cache's page count is not known here; every copy reads a page that the block table names
     if (pt_make_map(&map, w.cache, 1ll << 31, 2 * PT_HS, true) != 0) return -1;
@@ -931,7 +941,7 @@ int dl_window_prefill_tc(const DlWindowAttnArgs& w, const int* tile_rows, int n_
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = alone ? 0 : 1;
     cudaError_t e = cudaLaunchKernelEx(&cfg, attention_prefill_tc_kernel<true>, a, map, map);
     if (e != cudaSuccess) { dl_set_error("window_prefill_tc launch: %s", cudaGetErrorString(e)); return -(int)e; }
     return 0;

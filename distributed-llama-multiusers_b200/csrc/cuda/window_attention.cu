@@ -369,10 +369,10 @@ __host__ __device__ __forceinline__ int wm_line_stride(int LD) {      // bf16 el
 }
 
 // A decoding tile: all its stacked rows fit ONE 16-row MMA tile, so the four warps share the tokens instead of the rows.  A warp
-// takes every fourth half page (16 tokens) through a buffer of its own -- no barrier between warps until the merge in shared memory;
-// 16 warps per SM keep ~100 KB in flight.  As a quarter-full row tile (one warp of four multiplying, a barrier per page) 32 rows over
+// takes every fourth half page (16 tokens) through two buffers of its own (DEEP; one where the launch has tall tiles, too) -- no barrier between
+// warps until the merge in shared memory; 12 warps per SM keep ~100 KB in flight while they multiply as much.  As a quarter-full row tile (one warp of four multiplying, a barrier per page) 32 rows over
 // 1000 to 2000 positions of 4 key/value heads took 58.5 us with the merge; 40.1 now.
-template <int DK>
+template <int DK, bool DEEP>
 __device__ __forceinline__ void window_small_tile(const DlWindowAttnArgs& a, const int* s_row, int n_rows, int tile, int g, int n_splits, int pg_lo, int pg_hi, int lo,
                                                   int p_first, int slot, __nv_bfloat16* smem, float* __restrict__ partial) {
     constexpr int D = 16 * DK, NV = D / 8, QS = D + 8;
@@ -380,8 +380,9 @@ __device__ __forceinline__ void window_small_tile(const DlWindowAttnArgs& a, con
     const bool own_v = a.vdim > 0, capped = a.softcap > 0.f, biased = a.slope != nullptr;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3, mat = lane >> 3, rr = lane & 7;
     const float c1 = capped ? a.scale * 2.f / a.softcap * WM_LOG2E : a.scale * WM_LOG2E, capK = a.softcap * WM_LOG2E;
-    __nv_bfloat16* kv = smem + (size_t)warp * 16 * LDS;                              // this warp's half page; behind the four: the queries
-    __nv_bfloat16* q_s = smem + (size_t)4 * 16 * LDS;
+    constexpr int NB = DEEP ? 2 : 1;
+    __nv_bfloat16* ring = smem + (size_t)warp * NB * 16 * LDS;                       // this warp's half pages; behind the four warps': the queries
+    __nv_bfloat16* q_s = smem + (size_t)4 * NB * 16 * LDS;
     for (int idx = threadIdx.x; idx < 16 * (D / 4); idx += 128) {
         const int sr = idx / (D / 4), c4 = idx - sr * (D / 4), r = sr / rep;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -410,13 +411,15 @@ __device__ __forceinline__ void window_small_tile(const DlWindowAttnArgs& a, con
 #pragma unroll
     for (int v = 0; v < NV; ++v) { o[v][0] = o[v][1] = o[v][2] = o[v][3] = 0.f; }
     const int p_last = p_first + n_rows - 1, parts = LD / 8, cs_last = a.chunk > 0 ? p_last / a.chunk * a.chunk : 0;
-    for (int hp = 2 * pg_lo + warp; hp <= 2 * pg_hi + 1; hp += 4) {
-        const int first = hp * 16;
-        if (first > p_last) break;
-        if (first + 15 < lo) continue;
-        const int page = a.block_table[(size_t)slot * a.max_pages + (hp >> 1)];
-        const __nv_bfloat16* src = (const __nv_bfloat16*)a.cache + (((size_t)page * a.kv_heads + g) * WA_PAGE + (hp & 1) * 16) * LD;
-        __syncwarp();                                          // every lane is done with the last half page
+    // this warp's half pages: every fourth from the first that reaches a visible position to the last one's; page ids a step ahead of the copies
+    int hp = 2 * pg_lo + warp;
+    while (hp * 16 + 15 < lo) hp += 4;
+    const int hp_end = min(2 * pg_hi + 1, p_last / 16);
+    const int* bt = a.block_table + (size_t)slot * a.max_pages;
+    int page = hp <= hp_end ? bt[hp >> 1] : 0;
+    auto copy = [&](int h, __nv_bfloat16* kv) {
+        const __nv_bfloat16* src = (const __nv_bfloat16*)a.cache + (((size_t)page * a.kv_heads + g) * WA_PAGE + (h & 1) * 16) * LD;
+        page = h + 4 <= hp_end ? bt[(h + 4) >> 1] : 0;
         if (parts == 32) {                                     // key and value of 128: a line per instruction
 #pragma unroll
             for (int j = 0; j < 16; ++j) cp_async16(kv + j * LDS + lane * 8, src + j * 256 + lane * 8);
@@ -426,7 +429,23 @@ __device__ __forceinline__ void window_small_tile(const DlWindowAttnArgs& a, con
                 cp_async16(kv + (size_t)j * LDS + part * 8, src + (size_t)c * 8);
             }
         }
-        cp_async_wait_all();
+    };
+    if (DEEP) {
+        if (hp <= hp_end) copy(hp, ring);
+        cp_async_commit();
+    }
+    for (int n = 0; hp <= hp_end; hp += 4, n ^= 1) {
+        const int first = hp * 16;
+        __nv_bfloat16* kv = ring + (DEEP ? n * 16 * LDS : 0);
+        __syncwarp();                                          // every lane is done with the half page before
+        if (DEEP) {
+            if (hp + 4 <= hp_end) copy(hp + 4, ring + (n ^ 1) * 16 * LDS);
+            cp_async_commit();
+            cp_async_wait_one();
+        } else {
+            copy(hp, kv);
+            cp_async_wait_all();
+        }
         __syncwarp();
         float sc[2][4];
 #pragma unroll
@@ -486,11 +505,15 @@ __device__ __forceinline__ void window_small_tile(const DlWindowAttnArgs& a, con
 #pragma unroll
             for (int v = 0; v < NV; ++v) { o[v][0] *= al[0]; o[v][1] *= al[0]; o[v][2] *= al[1]; o[v][3] *= al[1]; }
         }
-        uint32_t pa[4];
-        pa[0] = pack_bf16(sc[0][0], sc[0][1]);
-        pa[1] = pack_bf16(sc[0][2], sc[0][3]);
-        pa[2] = pack_bf16(sc[1][0], sc[1][1]);
-        pa[3] = pack_bf16(sc[1][2], sc[1][3]);
+        // DEEP: probabilities in two bf16 numbers, the second the first one's remainder, as the tcgen05 kernel takes the prompts of these lines (rounded to
+        // one, the error depends on how often a maximum moves, that is on the number of shares: 2.06e-3 with four, 2.07e-3 with three, 1.66e-3 so)
+        uint32_t pa[4], pb[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float p0 = sc[i >> 1][(i & 1) * 2], p1 = sc[i >> 1][(i & 1) * 2 + 1];
+            pa[i] = pack_bf16(p0, p1);
+            if (DEEP) pb[i] = pack_bf16(p0 - __uint_as_float(pa[i] << 16), p1 - __uint_as_float(pa[i] & 0xffff0000u));
+        }
 #pragma unroll
         for (int vp = 0; vp < NV / 2; ++vp) {
             const int vt = 2 * vp + (mat >> 1);
@@ -499,8 +522,13 @@ __device__ __forceinline__ void window_small_tile(const DlWindowAttnArgs& a, con
             ldmatrix_x4_trans(b, kv + (size_t)((mat & 1) * 8 + rr) * LDS + col);
             mma_bf16(o[2 * vp], pa, b[0], b[1]);
             mma_bf16(o[2 * vp + 1], pa, b[2], b[3]);
+            if (DEEP) {
+                mma_bf16(o[2 * vp], pb, b[0], b[1]);
+                mma_bf16(o[2 * vp + 1], pb, b[2], b[3]);
+            }
         }
     }
+    cp_async_wait_all();
     // the warps' shares meet in the buffers' place: [warp][16][D], maxima and sums behind
     __syncthreads();
     float* acc = reinterpret_cast<float*>(smem);
@@ -545,8 +573,8 @@ __device__ __forceinline__ void window_small_tile(const DlWindowAttnArgs& a, con
     }
 }
 
-template <int DK>
-__global__ void __launch_bounds__(128, 4) window_attention_mma_kernel(DlWindowAttnArgs a, const int* __restrict__ tile_rows, int rq,
+template <int DK, bool DEEP>
+__global__ void __launch_bounds__(128, DEEP ? 3 : 4) window_attention_mma_kernel(DlWindowAttnArgs a, const int* __restrict__ tile_rows, int rq,
                                                                    int n_splits, float* __restrict__ partial, int only_small, int max_small) {      // only_small: 0, or the list tiles that a CTA of the other kernel may take
     constexpr int D = 16 * DK, NV = D / 8;
     extern __shared__ __align__(16) uint8_t smraw[];
@@ -587,7 +615,7 @@ __global__ void __launch_bounds__(128, 4) window_attention_mma_kernel(DlWindowAt
             }
             return;
         }
-        window_small_tile<DK>(a, s_row, n_rows, tile, g, n_splits, pg_lo, pg_hi, lo, p_first, slot, kv_s, partial);
+        window_small_tile<DK, DEEP>(a, s_row, n_rows, tile, g, n_splits, pg_lo, pg_hi, lo, p_first, slot, kv_s, partial);
         return;
     }
     if (only_small) return;              // attention_prefill_tc.cu takes the others
@@ -749,16 +777,19 @@ __global__ void __launch_bounds__(128, 4) window_attention_mma_kernel(DlWindowAt
     }
 }
 
-// merge of the page shares: one CTA per (tile, key/value head, position of the tile).  Every (head, share) weight
+// merge of the page shares: a CTA per (tile, key/value head, position of the tile), in decoding launches no more positions than a tile can have
+// (positions in turn, should one have more).  Every (head, share) weight
 // e^(m_k - m) / l is formed once, by a warp per head, then a thread per (head, column) sums the shares.
 #define WM_MAX_SPLITS 32
 __global__ void __launch_bounds__(128) window_merge_kernel(DlWindowAttnArgs a, const int* __restrict__ tile_rows, int rq, int n_splits,
                                                            const float* __restrict__ partial) {
     __shared__ float w_s[WM_ROWS * WM_MAX_SPLITS];
-    const int tile = blockIdx.x, g = blockIdx.y, r = blockIdx.z, D = a.dim, rep = a.heads / a.kv_heads;
+    const int tile = blockIdx.x, g = blockIdx.y, D = a.dim, rep = a.heads / a.kv_heads;
+  for (int r = blockIdx.z; r < rq; r += gridDim.z) {
     const int m = tile_rows[(size_t)tile * rq + r];                           // not written by the kernel that this launch runs ahead of
     if (m < 0) return;
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    __syncthreads();
     const float* base = partial + ((size_t)tile * a.kv_heads + g) * n_splits * WM_ROWS * (D + 2);
     if (base[(size_t)r * rep * (D + 2) + D + 1] == -2.f) return;              // written already, without shares
     for (int hg = threadIdx.x >> 5; hg < rep; hg += blockDim.x >> 5) {        // a warp per head, a lane per share
@@ -786,11 +817,13 @@ __global__ void __launch_bounds__(128) window_merge_kernel(DlWindowAttnArgs a, c
         }
         a.out[(size_t)m * a.ldo + (size_t)(g * rep + hg) * D + c] = acc;
     }
+  }
 }
 
 // attention_prefill_tc.cu
 int dl_window_prefill_tc_supported(const DlWindowAttnArgs& a, int rq);
-int dl_window_prefill_tc(const DlWindowAttnArgs& a, const int* tile_rows, int n_tiles, int rq, int group, int n_splits, float* partial, cudaStream_t stream);
+int dl_window_prefill_tc(const DlWindowAttnArgs& a, const int* tile_rows, int n_tiles, int rq, int group, int n_splits, float* partial, bool alone, cudaStream_t stream);
+int dl_window_prefill_tc_shares(const DlWindowAttnArgs& a, int n_tiles, int group, int n_splits);
 
 // rows of one sequence per tile: as many positions as fit 64 stacked (position, head) pairs
 extern "C" int dl_window_tc_rows(int heads, int kv_heads) {
@@ -826,31 +859,52 @@ extern "C" int dl_window_attention_tc(const DlWindowAttnArgs* args, const int* t
     }
     if (n_tiles < 1) return 0;
     if (n_splits < 1 || n_splits > WM_MAX_SPLITS || (n_splits > 1 && partial == nullptr)) { dl_set_error("dl_window_attention_tc: n_splits %d without scratch", n_splits); return -1; }
-    const size_t smem = ((size_t)2 * WA_PAGE * wm_line_stride(a.dim + (a.vdim > 0 ? a.vdim : a.rope_dims)) + (size_t)WM_ROWS * (a.dim + 8)) * sizeof(__nv_bfloat16);
     // tiles of more than 16 stacked rows are prompt portions: tcgen05, 128 stacked rows to a CTA, 256 where that fills the SMs
-    const bool tc5 = dl_window_prefill_tc_supported(a, rq) == 0;
+    const bool can_tc5 = dl_window_prefill_tc_supported(a, rq) == 0;
     const int group = (n_tiles + 1) / 2 * a.kv_heads <= dl_device_sm_count() ? 2 : 4;
-    const int max_small = (3 * dl_device_sm_count() + n_tiles * a.kv_heads - 1) / (n_tiles * a.kv_heads);
+    // Which kernel has work, by the number of rows: a row or so per tile is decoding (mma.sync alone, as it takes all tiles then), tiles as good as
+    // full are one prompt (tcgen05 alone, likewise); else both.  A kernel without work costs its launch (us, both and the one: 8 rows under a window of
+    // 256 21.1 and 15.4, a prompt of 32 rows 15.6 and 13.0, of 2000 under 1024 43.2 and 39.6)
+    const int rep = a.heads / a.kv_heads;
+    const bool decode = a.rows > 0 && (((long long)a.rows - n_tiles + 1) * rep <= 16 || (a.rows == n_tiles && n_splits > 1));
+    const bool prompt = can_tc5 && a.rows <= (long long)n_tiles * rq && a.rows > (n_tiles - 1ll) * rq + 16 / rep;
+    const bool tc5 = can_tc5 && !decode;
+    if (prompt) {
+        if (n_splits > 1) n_splits = dl_window_prefill_tc_shares(a, n_tiles, group, n_splits);
+        const int rc = dl_window_prefill_tc(a, tile_rows, n_tiles, rq, group, n_splits, partial, true, (cudaStream_t)stream);
+        if (rc != 0 || n_splits == 1) return rc;
+    }
+    // lines of 128 + 128 without tall tiles: two half pages per warp, three CTAs an SM, and no more shares than are there at once (32 rows over 1000 to 2000
+    // positions of 4 key/value heads 41.2 us with one buffer and four shares on four CTAs an SM, 37.7 now, of 8 61.2 and 57.9)
+    const bool deep = a.dim == 128 && a.vdim == 128 && (tc5 || decode || rq * rep <= 16);
+    const int n_sms = dl_device_sm_count();
+    const int max_small = deep ? (n_tiles * a.kv_heads < 3 * n_sms ? 3 * n_sms / (n_tiles * a.kv_heads) : 1) : (3 * n_sms + n_tiles * a.kv_heads - 1) / (n_tiles * a.kv_heads);
+    const size_t line = wm_line_stride(a.dim + (a.vdim > 0 ? a.vdim : a.rope_dims)) * sizeof(__nv_bfloat16), q_line = (a.dim + 8) * sizeof(__nv_bfloat16);
+    const size_t tall = 2 * WA_PAGE * line + WM_ROWS * q_line, both = 4 * 2 * 16 * line + 16 * q_line, smem = deep && both > tall ? both : tall;
     dim3 grid(n_tiles, a.kv_heads, n_splits);
     cudaStream_t st = (cudaStream_t)stream;
-    switch (a.dim / 16) {
+    auto launch = [&](auto kernel) {
+        if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        kernel<<<grid, 128, smem, st>>>(a, tile_rows, rq, n_splits, partial, tc5 ? group : 0, max_small);
+    };
+    if (deep && !prompt) launch(window_attention_mma_kernel<8, true>);
+    else if (!prompt) switch (a.dim / 16) {
 #define WM_CASE(DK_)                                                                                                      \
     case DK_:                                                                                                             \
-        if (smem > 48 * 1024) cudaFuncSetAttribute(window_attention_mma_kernel<DK_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-        window_attention_mma_kernel<DK_><<<grid, 128, smem, st>>>(a, tile_rows, rq, n_splits, partial, tc5 ? group : 0, max_small);                  \
+        launch(window_attention_mma_kernel<DK_, false>);                                                                  \
         break;
         WM_CASE(1) WM_CASE(2) WM_CASE(3) WM_CASE(4) WM_CASE(6) WM_CASE(8)
 #undef WM_CASE
         default: dl_set_error("dl_window_attention_tc: dim %d", a.dim); return -1;
     }
-    if (tc5) {
+    if (tc5 && !prompt) {
         LAYER_CHECK_LAUNCH("dl_window_attention_tc");
-        const int rc = dl_window_prefill_tc(a, tile_rows, n_tiles, rq, group, n_splits, partial, st);
+        const int rc = dl_window_prefill_tc(a, tile_rows, n_tiles, rq, group, n_splits, partial, false, st);
         if (rc != 0) return rc;
     }
     if (n_splits > 1) {
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(n_tiles, a.kv_heads, rq);
+        cfg.gridDim = dim3(n_tiles, a.kv_heads, decode && a.rows - n_tiles + 1 < rq ? (a.rows - n_tiles + 1 > 0 ? a.rows - n_tiles + 1 : 1) : rq);
         cfg.blockDim = dim3(128);
         cfg.stream = st;
         cudaLaunchAttribute attr[1];

@@ -543,6 +543,7 @@ def _window_args(q, out, heads, kv_heads, dim, rope_dims, scale, softcap, window
     a.cache, a.ctype = cache.data_ptr(), _type(cache)
     a.vdim, a.chunk, a.sink, a.key_heads, a.value_heads = vdim, chunk, _p(sink), key_heads, value_heads
     a.slope, a.gate, a.ld_gate = _p(slope), _p(gate), (gate.stride(0) if gate is not None else 0)
+    a.rows = q.shape[0]
     return a
 
 

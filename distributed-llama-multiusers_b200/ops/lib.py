@@ -314,7 +314,7 @@ class DlWindowAttnArgs(C.Structure):
                 ("pos", C.c_void_p), ("slot", C.c_void_p), ("block_table", C.c_void_p),
                 ("max_pages", C.c_int), ("page_size", C.c_int), ("cache", C.c_void_p), ("ctype", C.c_int),
                 ("vdim", C.c_int), ("chunk", C.c_int), ("sink", C.c_void_p), ("key_heads", C.c_int), ("value_heads", C.c_int),
-                ("slope", C.c_void_p), ("gate", C.c_void_p), ("ld_gate", C.c_longlong)]
+                ("slope", C.c_void_p), ("gate", C.c_void_p), ("ld_gate", C.c_longlong), ("rows", C.c_int)]
 
 
 class DlConvArgs(C.Structure):

@@ -676,6 +676,7 @@ typedef struct {
                                                  after the softmax, see dl_talk_mix).  Not together with key_heads */
     const float* slope;                       /* [heads] or NULL: slope[h] * (pos[m] - j) is taken off the (capped) score of position j */
     const float* gate; long long ld_gate;     /* [M] rows of `heads` numbers or NULL: head h leaves multiplied by sigmoid(gate[m][h]) */
+    int rows;                                 /* rows of the batch, a hint to dl_window_attention_tc which of its kernels have work; 0: not said */
 } DlWindowAttnArgs;
 int dl_window_attention(const DlWindowAttnArgs* args /*host*/, int M, void* stream);
 
