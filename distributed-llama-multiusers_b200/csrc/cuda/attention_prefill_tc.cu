@@ -45,7 +45,7 @@
 #define PT_HS 128
 #define PT_ROWS 128
 #define PT_KV 128                      // tokens per step
-#define PT_THREADS 512
+#define PT_THREADS 384
 #define PT_MAX_SEG 8
 #define PT_TILE_BYTES 32768            // 128 x 128 fp16
 #define PT_STAGES 2                    // K tiles and V tiles in flight
@@ -153,10 +153,9 @@ template <bool LINES> DL_DEVINL pair_f pt_ex2_poly(pair_f x) {
     return pair_of(__int_as_float(__float_as_int(pl) + (__float_as_int(tl) << 23)), __int_as_float(__float_as_int(ph) + (__float_as_int(th) << 23)));
 }
 
-// 32 scores (masked ones are -inf) -> exp2(s * sc - ref) as 16 packed fp16 pairs into TMEM; their sum is added to `sum`.  LINES: as bf16 and, at
-// taddr_lo, the bf16 remainder of each, 17 bits together
-template <bool LINES> DL_DEVINL void pt_probs(const uint32_t (&v)[32], float sc, float ref, uint32_t taddr, uint32_t taddr_lo, pair_f& sum) {
-    uint32_t pk[16], lo[LINES ? 16 : 1];
+// 32 scores (masked ones are -inf) -> exp2(s * sc - ref) as 16 packed fp16 pairs; their sum is added to `sum`.  LINES: as bf16 and, in `lo`, the
+// bf16 remainder of each, 17 bits together
+template <bool LINES> DL_DEVINL void pt_probs(const uint32_t (&v)[32], float sc, float ref, uint32_t (&pk)[16], uint32_t (&lo)[LINES ? 16 : 1], pair_f& sum) {
     const pair_f sc2 = pair_of(sc, sc), ref2 = pair_of(-ref, -ref);
 #pragma unroll
     for (int e = 0; e < 32; e += 2) {
@@ -175,8 +174,6 @@ template <bool LINES> DL_DEVINL void pt_probs(const uint32_t (&v)[32], float sc,
         pk[e >> 1] = pt_pack2<LINES>(pa, pb);
         if constexpr (LINES) lo[e >> 1] = pt_pack2<LINES>(pa - __uint_as_float(pk[e >> 1] << 16), pb - __uint_as_float(pk[e >> 1] & 0xffff0000u));
     }
-    tmem_st_32x32b_x16(taddr, pk);
-    if constexpr (LINES) tmem_st_32x32b_x16(taddr_lo, lo);
 }
 
 // One thread's 32 consecutive outputs of row m (a Q80 block) into the slabs of the next matmul: the block's maximum is in the thread's own
@@ -266,6 +263,7 @@ struct PtItem {
     int first_page, j0, J;                 // pages ahead of first_page are not touched; steps of 128 tokens, the first one at token j0 * 128
     int ja[2], jb[2];                      // steps [ja, jb) of these are tile t's (none: the tile is not there)
     int row0[2], rows, head[2];            // first row of tile t, rows of the segment (or run), the tile's head
+    int shares;                            // LINES: into how many shares (grid.z) the steps of the run go
     int begin;                             // batch row of the segment's first row; LINES: entry of tile_rows where the run starts
 };
 
@@ -348,8 +346,8 @@ DL_DEVINL int pt_runs(const PtLineArgs& a, int (*runs)[4]) {
     }
     return n;
 }
-// the item of a run, and into how many shares (grid.z) its steps go: no more than leave each PT_SHARE_STEPS, so that a short run needs no merge
-DL_DEVINL void pt_run_item(const PtLineArgs& a, const int (&run)[4], PtItem& it, int& shares) {
+// the item of a run: its steps go into no more shares than leave each PT_SHARE_STEPS, so that a short run needs no merge
+DL_DEVINL void pt_run_item(const PtLineArgs& a, const int (&run)[4], PtItem& it) {
     const DlWindowAttnArgs& w = a.w;
     it.begin = run[0] * a.rq;
     it.rows = run[1] * a.rep;
@@ -370,8 +368,8 @@ DL_DEVINL void pt_run_item(const PtLineArgs& a, const int (&run)[4], PtItem& it,
     it.first_page = lo[0] / 32;                                  // (tile 1 starts no earlier)
     it.j0 = lo[0] / PT_KV;
     it.J = max(j[0], j[1]) - it.j0;
-    shares = max(1, min((int)gridDim.z, it.J / PT_SHARE_STEPS));
-    const int per = (it.J + shares - 1) / shares, z0 = min(it.J, (int)blockIdx.z * per), z1 = min(it.J, z0 + per);
+    it.shares = max(1, min((int)gridDim.z, it.J / PT_SHARE_STEPS));
+    const int per = (it.J + it.shares - 1) / it.shares, z0 = min(it.J, (int)blockIdx.z * per), z1 = min(it.J, z0 + per);
 #pragma unroll
     for (int u = 0; u < 2; u++) {
         it.ja[u] = max(lo[u] / PT_KV - it.j0 - z0, 0);
@@ -382,22 +380,18 @@ DL_DEVINL void pt_run_item(const PtLineArgs& a, const int (&run)[4], PtItem& it,
     it.first_page = max(it.first_page, it.j0 * (PT_KV / 32));
 }
 
-// Queries of 32 rows into the tile's K-major, swizzled image: lane i holds the address of row r0 + i; N rows are in flight, a row a load
-template <bool LINES, int N, typename Ready>
+// Queries of 32 rows into the tile's K-major, swizzled image: lane i holds the address of row r0 + i; all in flight, a row a load
+template <bool LINES, typename Ready>
 DL_DEVINL void pt_load_rows(const float* mine, uint8_t* tile, int r0, Ready ready) {
     const int lane = threadIdx.x & 31;
     uint8_t* qd = tile + r0 * 128 + (lane >> 4) * 16384 + (lane & 1) * 8;
-#pragma unroll 1
-    for (int i = 0; i < 32; i += N) {
-        float4 x[N];
+    float4 x[32];
 #pragma unroll
-        for (int u = 0; u < N; u++)
-            x[u] = reinterpret_cast<const float4*>(__shfl_sync(0xffffffffu, (unsigned long long)(uintptr_t)mine, i + u))[lane];
-        if (i == 0) ready();
+    for (int u = 0; u < 32; u++) x[u] = reinterpret_cast<const float4*>(__shfl_sync(0xffffffffu, (unsigned long long)(uintptr_t)mine, u))[lane];
+    ready();
 #pragma unroll
-        for (int u = 0; u < N; u++)              // 16-byte piece c of a half row -> swizzled slot c ^ (row & 7)
-            *reinterpret_cast<uint2*>(qd + (i + u) * 128 + ((((lane >> 1) & 7) ^ (u & 7)) << 4)) = make_uint2(pt_pack2<LINES>(x[u].x, x[u].y), pt_pack2<LINES>(x[u].z, x[u].w));
-    }
+    for (int u = 0; u < 32; u++)                 // 16-byte piece c of a half row -> swizzled slot c ^ (row & 7)
+        *reinterpret_cast<uint2*>(qd + u * 128 + ((((lane >> 1) & 7) ^ (u & 7)) << 4)) = make_uint2(pt_pack2<LINES>(x[u].x, x[u].y), pt_pack2<LINES>(x[u].z, x[u].w));
     fence_proxy_async_smem();
 }
 
@@ -476,11 +470,10 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
     tc_fence_after();
     const PtWaits wait = {&gave_up_s, globaltimer_ns()};
     const int n_seg = n_seg_s;
-    int shares = 1;                                              // LINES: of the item
     // the items of this CTA, in the same order for every role; rounds run back and forth over the CTAs, so that a long item goes with a short one
     auto item_at = [&](int round, PtItem& it) {
         if constexpr (LINES) {
-            if (round < n_seg) pt_run_item(a, seg[round], it, shares);
+            if (round < n_seg) pt_run_item(a, seg[round], it);
             return round < n_seg;
         } else {
             const int G = gridDim.x, b = blockIdx.x;
@@ -488,10 +481,9 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
         }
     };
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_holder, 0);
-    // TMEM columns: outputs at 256 + 128 t.  One buffer of scores at 0, taken in turn, and probabilities at 128 + 64 t; LINES, whose
-    // probabilities need 128 columns: scores, then probabilities, at 128 t
-    const auto t_s = [&](int t) { return tmem_base + (LINES ? t * 128 : 0); };
-    const auto t_p = [&](int t) { return tmem_base + (LINES ? t * 128 : 128 + t * 64); };
+    // TMEM columns: one buffer of scores at 0, which the tiles take in turn; probabilities at 128, of 64 columns for each tile (LINES: of 128, which
+    // the tiles take in turn, too); outputs at 256 + 128 t
+    const auto t_p = [&](int t) { return tmem_base + 128 + (LINES ? 0 : t * 64); };
     auto row_of = [&](const PtItem& it, int t, int row) -> const float* {      // the queries of a tile's row (rows that are not there: of the last one)
         const int r = min((t ? it.row0[1] : it.row0[0]) + row, it.rows - 1);
         if constexpr (LINES) return a.w.q + (size_t)a.tile_rows[it.begin + r / a.rep] * a.w.ldq + (it.kvh * a.rep + r % a.rep) * PT_HS;
@@ -503,20 +495,27 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
     // distance between the two 64-wide halves of N (16 KB), SBO = distance between 8-token groups (1024 B).
     if (warp < 8) {
         // ---------------- softmax: warps 0-3 tile 0, warps 4-7 tile 1; a thread per query row (= TMEM lane) ----------------
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 192;");
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
         const int t = warp >> 2, quarter = warp & 3, row = quarter * 32 + lane;
-        const uint32_t lane_base = (uint32_t)(quarter * 32) << 16, T_S = t_s(t) + lane_base, T_P = t_p(t) + lane_base, T_O = tmem_base + lane_base + 256 + t * 128;
+        const uint32_t lane_base = (uint32_t)(quarter * 32) << 16, T_S = tmem_base + lane_base, T_P = t_p(t) + lane_base, T_O = tmem_base + lane_base + 256 + t * 128;
         float* stage = out_s + (size_t)warp * 32 * PT_OUT_LD;
-        uint32_t ns = 0;                                         // steps of this tile so far
-        PtItem it;
-        for (int round = 0; item_at(round, it); round++) {
+        uint32_t ns = 0, nq = 0, other = 0, seen = 0;            // steps and items of this tile so far; steps of the other tile in earlier items, and those waited for
+        PtItem it, next;
+        // the queries of the tile's next item: all rows in flight at once, ahead of this item's outputs
+        auto load_queries = [&](const PtItem& of) {
+            if (!(t ? of.jb[1] > of.ja[1] : of.jb[0] > of.ja[0])) return;
+            pt_load_rows<LINES>(row_of(of, t, row), q_s + t * PT_TILE_BYTES, quarter * 32, [&] {
+                if (nq > 0) wait(&q_empty[t], (nq - 1) & 1);      // the tile's last scores have read the queries before
+            });
+            nq++;
+            mbar_arrive(&q_full[t]);
+        };
+        bool more = item_at(0, it);
+        if (more) load_queries(it);
+        for (int round = 0; more; round++, it = next) {
             const int ja = t ? it.ja[1] : it.ja[0], jb = t ? it.jb[1] : it.jb[0], row0 = t ? it.row0[1] : it.row0[0], head = t ? it.head[1] : it.head[0];
+            const int ja_o = t ? it.ja[0] : it.ja[1], jb_o = t ? it.jb[0] : it.jb[1];
             const int r_abs = row0 + row, r_live = min(r_abs, it.rows - 1);
-            if (!LINES && jb == 0) continue;
-            if (round == 0 && jb > ja) {                         // the first queries (the others: warps 12-15, ahead of time)
-                pt_load_rows<LINES, 32>(row_of(it, t, row), q_s + t * PT_TILE_BYTES, quarter * 32, [] {});
-                mbar_arrive(&q_full[t]);
-            }
             int pos_r, lb = 0, m_row = 0, h_row = 0;             // last and first visible position of this row; LINES: its batch row and head
             float sc, c1 = 0.f, cap_k = 0.f, slope = 0.f;
             bool shaped = false;                                 // scores leave the accumulator through a cap, a bias or a factor that is not positive
@@ -540,15 +539,13 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
             float m_used = -INFINITY, l = 0.0f;
             for (int j = ja; j < jb; j++, ns++) {
                 uint32_t v[4][32];
-                wait(&s_full[t], ns & 1);                        // LINES: also P V of the step before is complete
+                wait(&s_full[t], ns & 1);
                 tc_fence_after();
 #pragma unroll
                 for (int c = 0; c < 4; c++) tmem_ld_32x32b_x32(T_S + c * 32, v[c]);
                 tmem_ld_wait();
-                if constexpr (!LINES) {                          // the other tile's scores may take the place
-                    tc_fence_before();
-                    mbar_arrive(s_empty);
-                }
+                tc_fence_before();
+                mbar_arrive(s_empty);                            // the next scores may take the place
                 const int tok0 = (it.j0 + j) * PT_KV;
                 const int lim = pos_r - tok0, low = LINES ? lb - tok0 : 0;      // columns low <= e <= lim are visible to this row
                 if constexpr (LINES) {
@@ -567,8 +564,14 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
                 }
                 if (lim < PT_KV - 1 || (LINES && low > 0)) {
 #pragma unroll
-                    for (int e = 0; e < PT_KV; e++)
-                        if (e > lim || (LINES && e < low)) v[e >> 5][e & 31] = 0xff800000u;        // -inf
+                    for (int c = 0; c < 4; c++) {                // a bit per column
+                        const int hi = lim - c * 32, lo = low - c * 32;
+                        uint32_t cols = hi < 0 ? 0u : hi >= 31 ? 0xffffffffu : (2u << hi) - 1;
+                        if (LINES) cols &= lo <= 0 ? 0xffffffffu : lo > 31 ? 0u : 0xffffffffu << lo;
+#pragma unroll
+                        for (int e = 0; e < 32; e++)
+                            if (!(cols & (1u << e))) v[c][e] = 0xff800000u;        // -inf
+                    }
                 }
                 float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
@@ -577,48 +580,65 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
                     for (int c = 0; c < 4; c++) mx4[c] = fmaxf(mx4[c], fmaxf(__uint_as_float(v[c][e]), __uint_as_float(v[c][e + 1])));
                 const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * sc;
                 const bool need = mx > m_used + 8.0f;            // the reference may lag the maximum by 2^8
-                if (!LINES && j > ja) {                          // P V of the step before is done with the probabilities
-                    wait(&o_full[t], (ns - 1) & 1);
-                    tc_fence_after();
-                }
-                if (__any_sync(0xffffffffu, need)) {
+                const bool moved = __any_sync(0xffffffffu, need);
+                float alpha = 1.f;
+                if (moved) {
                     const float m_new = need ? mx : m_used;
-                    const float alpha = need ? pt_ex2(m_used - m_new) : 1.0f;
-                    if (j > ja) {      // the accumulated output moves to the new reference (rare after the first steps)
-                        uint32_t w[32];
-#pragma unroll 1
-                        for (int ch = 0; ch < 4; ch++) {
-                            tmem_ld_32x32b_x32(T_O + ch * 32, w);
-                            tmem_ld_wait();
-#pragma unroll
-                            for (int e = 0; e < 32; e++) w[e] = __float_as_uint(__uint_as_float(w[e]) * alpha);
-                            tmem_st_32x32b_x32(T_O + ch * 32, w);
-                        }
-                    }
+                    if (need) alpha = pt_ex2(m_used - m_new);
                     l *= alpha;
                     m_used = m_new;
                 }
                 const float ref = (m_used == -INFINITY) ? 0.0f : m_used;
                 pair_f sum = 0;
+                uint32_t pk[4][16], lo[4][LINES ? 16 : 1];
+                // LINES: formed ahead of the waits, in the scores' registers, as the place is free only when the other tile's have been multiplied
+                if constexpr (LINES) {
 #pragma unroll
-                for (int c = 0; c < 4; c++) pt_probs<LINES>(v[c], sc, ref, T_P + c * 16, T_P + 64 + c * 16, sum);
+                    for (int c = 0; c < 4; c++) pt_probs<LINES>(v[c], sc, ref, pk[c], lo[c], sum);
+                }
+                if (j > ja) wait(&o_full[t], (ns - 1) & 1);      // this tile's P V before is complete
+                // and the other tile's, whose probabilities lie in this place, up to the one ahead of this in the issuer's order (one by one: a
+                // parity tells one phase from the next, no more)
+                if constexpr (LINES)
+                    for (const uint32_t up_to = other + max(0, min(j + t, jb_o) - ja_o); seen != up_to; seen++) wait(&o_full[t ^ 1], seen & 1);
+                tc_fence_after();
+                if (moved && j > ja) {      // the accumulated output moves to the new reference (rare after the first steps)
+                    uint32_t w[32];
+#pragma unroll 1
+                    for (int ch = 0; ch < 4; ch++) {
+                        tmem_ld_32x32b_x32(T_O + ch * 32, w);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int e = 0; e < 32; e++) w[e] = __float_as_uint(__uint_as_float(w[e]) * alpha);
+                        tmem_st_32x32b_x32(T_O + ch * 32, w);
+                    }
+                }
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    if constexpr (!LINES) pt_probs<LINES>(v[c], sc, ref, pk[c], lo[c], sum);
+                    tmem_st_32x32b_x16(T_P + c * 16, pk[c]);
+                    if constexpr (LINES) tmem_st_32x32b_x16(T_P + 64 + c * 16, lo[c]);
+                }
                 l += pair_sum(sum);
                 tmem_st_wait();
                 tc_fence_before();
                 mbar_arrive(&p_full[t]);
             }
+            other += jb_o - ja_o;
+            more = item_at(round + 1, next);
+            if (more) load_queries(next);
             // ---- finish: O / l -> f32 rows, partial sums, or the Q80 cast into the slabs of the wo matmul ----
             float inv;
             if constexpr (LINES) {
-                if (shares == 1 && a.w.sink) l += pt_ex2(a.w.sink[h_row] * 1.4426950408889634f - m_used);
-                inv = shares > 1 ? 1.f : (a.w.gate ? 1.f / (1.f + expf(-a.w.gate[(size_t)m_row * a.w.ld_gate + h_row])) : 1.f) / l;
+                if (it.shares == 1 && a.w.sink) l += pt_ex2(a.w.sink[h_row] * 1.4426950408889634f - m_used);
+                inv = it.shares > 1 ? 1.f : (a.w.gate ? 1.f / (1.f + expf(-a.w.gate[(size_t)m_row * a.w.ld_gate + h_row])) : 1.f) / l;
             } else {
                 inv = l > 0.0f ? 1.0f / l : 0.0f;
             }
             float* out = nullptr;                                // this thread's row; null: none
             bool vec = true;                                     // 16-byte rows
             if constexpr (LINES) {
-                if (row0 >= it.rows || (shares == 1 && blockIdx.z > 0)) continue;
+                if (row0 >= it.rows || (it.shares == 1 && blockIdx.z > 0)) continue;
                 out = a.w.out + (size_t)m_row * a.w.ldo + h_row * PT_HS;
                 vec = ((uintptr_t)a.w.out & 15) == 0 && (a.w.ldo & 3) == 0;
                 if (a.n_splits > 1) {                            // a stacked row's slot among the list tile's partial sums
@@ -627,17 +647,18 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
                     float* part = a.partial + (((size_t)u * a.w.kv_heads + it.kvh) * a.n_splits + blockIdx.z) * step + r_live % (PT_ROWS / 2) * (PT_HS + 2);
                     if (r_abs < it.rows) {                       // (-2: no merge, -1: nothing in this share)
                         part[PT_HS] = m_used * 0.6931471805599453f;
-                        part[PT_HS + 1] = shares == 1 ? -2.f : jb > ja ? l : -1.f;
-                        for (int z = gridDim.z; blockIdx.z == 0 && shares > 1 && z < a.n_splits; z++) {
+                        part[PT_HS + 1] = it.shares == 1 ? -2.f : jb > ja ? l : -1.f;
+                        for (int z = gridDim.z; blockIdx.z == 0 && it.shares > 1 && z < a.n_splits; z++) {
                             part[(size_t)z * step + PT_HS] = -INFINITY;
                             part[(size_t)z * step + PT_HS + 1] = -1.f;
                         }
                     }
-                    if (shares > 1) { out = part; vec = false; }
+                    if (it.shares > 1) { out = part; vec = false; }
                 }
                 if (jb == ja) continue;
-            } else if (a.y_out != nullptr) {
-                out = a.y_out + (size_t)(it.begin + r_live) * a.n_heads * PT_HS + head * PT_HS;
+            } else {
+                if (jb == ja) continue;
+                if (a.y_out != nullptr) out = a.y_out + (size_t)(it.begin + r_live) * a.n_heads * PT_HS + head * PT_HS;
                 vec = ((uintptr_t)a.y_out & 15) == 0;
             }
             wait(&o_full[t], (ns - 1) & 1);
@@ -677,7 +698,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
             tc_fence_before();                                   // the next item's P V may write the output (behind p_full)
         }
     } else {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
         const uint32_t desc_hi = (1024u >> 4) | (1u << 14) | (2u << 29);
         if (warp == 8) {
             // ---------------- MMAs, all by one thread: what it issues runs in that order ----------------
@@ -690,19 +711,16 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
                 auto on = [&](int t, int j) { return j >= it.ja[t] && j < it.jb[t]; };
                 auto scores = [&](int t, int j) {                // S = Q K^T of a step
                     const int st = (g + j) & 1;
-                    if (!on(t, j)) {
-                        if (LINES && t == 1 && j < it.J) pt_commit(&k_empty[st]);      // (a step that only tile 0 sees)
-                        return;
-                    }
+                    if (!on(t, j)) return;
                     wait(&k_full[st], ((g + j) >> 1) & 1);
                     if (j == it.ja[t]) wait(&q_full[t], nq[t]++ & 1);
-                    if (!LINES && n_s > 0) wait(s_empty, (n_s - 1) & 1);
+                    if (n_s > 0) wait(s_empty, (n_s - 1) & 1);
                     n_s++;
                     tc_fence_after();
                     __syncwarp();
-                    pt_mma_ss(t_s(t), q_lo + t * (PT_TILE_BYTES >> 4), k_lo + st * (PT_TILE_BYTES >> 4), desc_hi, idesc_s, 0);
+                    pt_mma_ss(tmem_base, q_lo + t * (PT_TILE_BYTES >> 4), k_lo + st * (PT_TILE_BYTES >> 4), desc_hi, idesc_s, 0);
                     pt_commit(&s_full[t]);
-                    if (t == 1 || (!LINES && !on(1, j))) pt_commit(&k_empty[st]);
+                    if (t == 1 || !on(1, j)) pt_commit(&k_empty[st]);
                     if (j + 1 == it.jb[t]) pt_commit(&q_empty[t]);
                 };
                 auto outputs = [&](int t, int j) {               // O += P V of a step
@@ -720,7 +738,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
                 };
                 scores(0, 0);
                 scores(1, 0);
-                if (!LINES) scores(0, 1);
+                scores(0, 1);
                 for (int j = 0; j < it.J; j++) {
                     const int st = (g + j) & 1;
                     wait(&v_full[st], ((g + j) >> 1) & 1);
@@ -737,19 +755,18 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
                         fence_proxy_async_smem();
                         __syncwarp();
                     }
-                    // probabilities that take the place of their scores: a tile's next scores behind its P V.  Else the other tile's, or its own
-                    // next but one: they wait in the buffer when the softmax threads come for them
+                    // the scores after next wait in the buffer when the softmax threads come for them
                     outputs(0, j);
-                    scores(LINES ? 0 : 1, j + 1);
+                    scores(1, j + 1);
                     outputs(1, j);
-                    scores(LINES ? 1 : 0, j + (LINES ? 1 : 2));
+                    scores(0, j + 2);
                 }
                 g += it.J;
             }
-        } else if (warp == 10 || warp == 11) {
-            // ---------------- K producer (warp 10) / V producer (warp 11), one lane each ----------------
+        } else if (warp == 9 || warp == 10) {
+            // ---------------- K producer (warp 9) / V producer (warp 10), one lane each ----------------
             if (lane == 0) {
-                const bool is_k = warp == 10;
+                const bool is_k = warp == 9;
                 const uint64_t map = is_k ? reinterpret_cast<uint64_t>(&kmap) : reinterpret_cast<uint64_t>(&vmap);
                 uint64_t* full = is_k ? k_full : v_full;
                 uint64_t* empty = is_k ? k_empty : v_empty;
@@ -795,24 +812,6 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
                                              : "memory");
                         }
                     }
-                }
-            }
-        } else if (warp >= 12) {
-            // ---------------- queries of the next items, 32 rows of each tile per warp, ahead of the softmax threads ----------------
-            const int wq = warp - 12;
-            uint32_t nq[2] = {0, 0};
-            PtItem it;
-            for (int round = 0; item_at(round, it); round++) {
-#pragma unroll
-                for (int t = 0; t < 2; t++) {
-                    if (it.jb[t] <= it.ja[t]) continue;
-                    if (round > 0) {
-                        pt_load_rows<LINES, 8>(row_of(it, t, wq * 32 + lane), q_s + t * PT_TILE_BYTES, wq * 32, [&] {
-                            if (nq[t] > 0) wait(&q_empty[t], (nq[t] - 1) & 1);        // the tile's last scores have read the queries before
-                        });
-                        mbar_arrive(&q_full[t]);
-                    }
-                    nq[t]++;
                 }
             }
         }
