@@ -2,38 +2,34 @@
 // attention_prefill.cu (segments of consecutive positions of one sequence, listed in `meta`), with both products
 // as tcgen05.mma and the score / probability / output tiles in TENSOR MEMORY instead of registers.
 //
-// A CTA owns 128 query rows x one query head and walks the KV history 128 tokens (four pages) at a time:
+// A CTA works on TWO query tiles of 128 rows that meet the same keys and values (two heads of a key/value head, or two row tiles of one head)
+// and walks the KV history 128 tokens (four pages) at a time; one tile's softmax runs beside the other's MMAs:
 //   S = Q K^T     SS-mode MMA, M = 128 rows, N = 128 tokens, K = 128: Q staged once (fp16, K-major, 128-byte swizzle);
 //                 K pages arrive by TMA tensor copies (cp.async.bulk.tensor.2d over this GPU's KV cache, box 64 x 32,
-//                 hardware 128-byte swizzle); S (f32) lands in TMEM, double-buffered
-//   softmax       two threads per query row (= TMEM lane), 64 score columns each, read into registers with tcgen05.ld
-//                 in one pass (the score buffer is handed back at once); the row maximum is exchanged through shared
-//                 memory; exp2 -> fp16 probabilities written back to TMEM with tcgen05.st (every fourth exp2 on the
-//                 FMA pipe: the step is MUFU-bound); running maximum with LAZY rescaling: the reference maximum only
+//                 hardware 128-byte swizzle); S (f32) lands in ONE buffer of TMEM that the tiles take in turn, free again as soon as
+//                 the softmax threads have it in registers, so that the next scores wait for them there
+//   softmax       a thread per query row (= TMEM lane), 128 scores in registers; exp2 -> fp16 probabilities written back to TMEM
+//                 (a quarter of the exp2 on the FMA pipe); running maximum with LAZY rescaling: the reference maximum only
 //                 moves when a row's maximum grew by more than 2^8, so in the steady state the output accumulator is
 //                 never touched by the softmax threads
 //   O += P V      TS-mode MMA: A = P straight from TMEM, B = V pages in shared memory as an MN-major operand (V is
 //                 [token][head dim] in the cache, i.e. N-contiguous: no transpose anywhere), accumulating in TMEM
-// S(j+1) and S(j+2) are issued while the softmax threads are busy with step j, so the tensor core works ahead of them.  Output: O / l -> shared memory -> Q80 cast into the XQ / XH slabs of the wo matmul.
+// CTAs are persistent: each walks its items (pt_item), long ones first and rounds back and forth, and loads the next item's queries ahead of this one's
+// outputs.  What bounds it: the MMAs.  With one tile per CTA scores, softmax and P V of a step followed each other (1950 clk a step for 1024 of MMAs) and
+// every CTA paid 13 us for its start and end: 4001 rows of 32 heads 215 us, 147 here (two steps in 1.75 us; the rest is starts, ends and diagonals).
 //
-// Warp roles (384 threads): warp 0 issues the S MMAs (+ TMEM owner), warp 6 the P V MMAs (an issuing thread spends ~700 clk
-// per group of 8 MMAs, so one thread for both would cap a step at ~1500 clk), warps 1-4 and 8-11 softmax (two threads per
-// row = TMEM lane, 64 columns each; the row maximum is exchanged through shared memory), warp 5
-// K producer and warp 7 V producer (one lane each issues 8 tensor copies of 4 KB per step: 4 pages x 2 halves of the head
-// dimension; K and V have their own 3-stage rings, so a K stage is free again as soon as its scores are complete).
-// (The first version copied K/V with cp.async in 16-byte pieces into un-swizzled core matrices: 4096 LDGSTS per step
-// cost 3500 clk of issue time, three times the MMAs -- scripts/trace_attention_tc.py.)
-// TMEM columns: S0 [0,128) S1 [128,256) P0 [256,320) P1 [320,384) O [384,512).
+// Warp roles (384 threads): warps 0-3 and 4-7 softmax of tile 0 and 1, warp 8 issues all MMAs (one issuer, or the tiles run in step; in convergent code, see
+// pt_mma_ss), warp 9 K producer and warp 10 V producer (one lane each issues 8 tensor copies of 4 KB per step).
 //
 // The second instance (LINES) serves layer-list models: bf16 cache lines [key 128 | value 128], tiles of up to rq consecutive positions
-// of one sequence whose query heads of one key/value head stack on the MMA's rows (row = position * rep + head), so two neighbouring
-// tiles of 64 stacked rows fill the 128 lanes; window or chunk masks (only the steps that a tile sees are walked), soft cap, distance
-// bias, sink, gate; f32 output.  Probabilities are two bf16 numbers each, the second the first one's remainder, and P V two MMAs: rounded to
+// of one sequence whose query heads of one key/value head stack on the MMA's rows (row = position * rep + head), so runs of two or four
+// neighbouring list tiles of 64 stacked rows fill one or two of its tiles; window or chunk masks (only the steps that a run sees are walked, in
+// shares where SMs are idle), soft cap, distance bias, sink, gate; f32 output.  Probabilities are two bf16 numbers each, the second the first one's
+// remainder, and P V two MMAs: rounded to
 // one (2^-9) they are the larger share of the error, and how large depends on how often a row's maximum, whose probability is exact, moves
-// -- every 32 tokens in the mma.sync kernel, every 128 here (2000 tokens under a window of 1024, against 64 bits: 1.929e-3 with one number,
-// 1.926e-3 there, 1.50e-3 with two; 1300 tokens: 2.19e-3, 2.17e-3, 1.64e-3; the time is the same).  The remainders lie in the score buffer that they
-// came from, so S of step j + 2 waits for P V of step j.  mma.sync with its 64-row tiles took 142 us for 2000 rows of 16 heads on 4 under a window of 1024
-// (88 TFLOP/s); 55 us here.
+// (2000 tokens under a window of 1024, against 64 bits: 1.93e-3 with one number, 1.47e-3 with two).  They take 128 columns, so the tiles take one such
+// buffer in turn, too.  2000 rows of 16 heads on 4 under a window of 1024: one run of 128 rows per CTA, in two waves, 54 us; 38 here; 512 rows in
+// page shares on mma.sync 62 us, 19 here.
 //
 // Reference semantics: multiheadAtt_F32 (src/nn/nn-cpu-ops.cpp:749-784), softmax in f32, output cast as OP_CAST
 // (src/llm.cpp:296-301).  KV cache: fp16 pages [page][kv_head][32][128].

@@ -21,7 +21,6 @@ def main():
     ap.add_argument("--layers", type=int, default=32)
     ap.add_argument("--rows", type=int, default=4096)
     ap.add_argument("--wh", default="auto")
-    ap.add_argument("--pt-dbg", type=int, default=0, help="attention_prefill_tc timing experiments (results invalid): 1 no softmax, 2 no KV copies, 4 no MMAs")
     ap.add_argument("--model-dir", default="/dev/shm")
     a = ap.parse_args()
     from dllama_b200.formats import mfile
@@ -32,8 +31,6 @@ def main():
     if not os.path.exists(path):
         mfile.write_random_model(path, a.model, quant.Q40, seed=1, **({} if full else {"n_layers": a.layers}))
     n = a.rows
-    if a.pt_dbg:
-        K.cuda_lib().dl_debug_set_pt_mode(a.pt_dbg)
     eng = LlamaEngine(path, max_rows=n, n_slots=2, max_seq_len=n + 64, use_graphs=False, use_pdl=False, prefill_wh=a.wh)
     prompt = np.random.default_rng(1).integers(1, eng.h.vocab_size, n).tolist()
     slot = eng.alloc_slot()

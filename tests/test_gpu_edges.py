@@ -538,3 +538,39 @@ def test_window_decode_non_finite_values_far_below(value):
     assert torch.isfinite(clean).all() and not torch.isfinite(out[1, :, 3]).any()
     out[1, :, 3] = clean[1, :, 3]
     assert torch.equal(out, clean)
+
+
+@pytest.mark.parametrize("heads,kv,segs", [(40, 40, [(0, 0, 257), (257, 50, 200)]), (32, 8, [(0, 7, 385), (385, 0, 129)]), (33, 11, [(0, 1, 640)])])
+def test_prompt_attention_two_tiles(heads, kv, segs):
+    """More tiles than SMs: two heads of a key/value head side by side, or (heads alone, or three of them) two row tiles of one head, the second one
+    missing or a step longer; several items per CTA."""
+    from test_gpu_kernels import test_attention_prefill_matches_reference as check
+    check(heads, kv, 128, segs, True)
+
+
+@pytest.mark.parametrize("runs,n_splits,rows,ld", [([(1500, 40)], 8, True, 0), ([(1500, 40)], 8, False, 2), ([(900, 64), (40, 3), (1200, 1), (0, 17)], 6, True, 0),
+                                                   ([(700, 1), (5, 1), (1999, 1)], 7, True, 0), ([(0, 16)], 4, True, 0), ([(640, 130), (3, 20)], 16, True, 0)])
+def test_window_shares(runs, n_splits, rows, ld):
+    """Page shares of tall tiles and of decoding ones, alone and in one call, with and without the number of rows said, output rows of 8 bytes: against
+    the per-row kernel (queries and weights rounded to bf16 here: 8e-3)."""
+    heads, kv, dim, pages = 8, 2, 128, 64
+    g = torch.Generator().manual_seed(n_splits)
+    M = sum(n for _, n in runs)
+    cache = torch.randn(len(runs) * pages, kv, 32, 2 * dim, generator=g).bfloat16().cuda()
+    bt = torch.randperm(len(runs) * pages, generator=g).int().view(len(runs), pages).cuda()
+    pos, slot, tiles = [], [], []
+    for s, (p0, n) in enumerate(runs):
+        at = list(range(len(pos), len(pos) + n))
+        pos += list(range(p0, p0 + n))
+        slot += [s] * n
+        tiles += [at[i:i + 16] for i in range(0, n, 16)]
+    tr = torch.tensor([t + [-1] * (16 - len(t)) for t in tiles], dtype=torch.int32, device="cuda")
+    q = torch.randn(M if rows else M + 1000, heads * dim, generator=g).bfloat16().float().cuda()
+    pos, slot = (torch.tensor(v, dtype=torch.int32, device="cuda") for v in (pos, slot))
+    wide = torch.zeros(M, heads * dim + ld, device="cuda")
+    got = wide[:, :heads * dim]
+    want = torch.zeros(M, heads * dim, device="cuda")
+    partial = torch.full((L().window_tc_partial_floats(len(tiles), kv, n_splits, dim),), float("nan"), device="cuda")
+    L().window_attention_tc(q, got, heads, kv, dim, 0, 0.1, 0.0, 0, pos, slot, bt, cache, tr, len(tiles), 16, n_splits, partial, vdim=dim)
+    L().window_attention(q, want, M, heads, kv, dim, 0, 0.1, 0.0, 0, pos, slot, bt, cache, vdim=dim)
+    assert ((got - want).norm(dim=1) <= 8e-3 * want.norm(dim=1)).all()
