@@ -412,7 +412,8 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
     uint64_t* p_full = bars + 14;        // [2] probabilities written
     uint64_t* o_full = bars + 16;        // [2] P V complete
     uint64_t* s_empty = bars + 18;       // the scores have been read into registers (one buffer for both tiles)
-    uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 19);
+    uint64_t* p_turn = bars + 19;        // [2] LINES: the place for probabilities is the tile's, for one step of it
+    uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 21);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     pdl_launch_dependents();
@@ -428,6 +429,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
             mbar_init(&s_full[s], 1);
             mbar_init(&p_full[s], 128);
             mbar_init(&o_full[s], 1);
+            mbar_init(&p_turn[s], 1);
         }
         mbar_init(s_empty, 128);
         mbar_fence_init();
@@ -495,7 +497,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
         const int t = warp >> 2, quarter = warp & 3, row = quarter * 32 + lane;
         const uint32_t lane_base = (uint32_t)(quarter * 32) << 16, T_S = tmem_base + lane_base, T_P = t_p(t) + lane_base, T_O = tmem_base + lane_base + 256 + t * 128;
         float* stage = out_s + (size_t)warp * 32 * PT_OUT_LD;
-        uint32_t ns = 0, nq = 0, other = 0, seen = 0;            // steps and items of this tile so far; steps of the other tile in earlier items, and those waited for
+        uint32_t ns = 0, nq = 0;                                 // steps of this tile so far, items whose queries are loaded
         PtItem it, next;
         // the queries of the tile's next item: all rows in flight at once, ahead of this item's outputs
         auto load_queries = [&](const PtItem& of) {
@@ -510,7 +512,6 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
         if (more) load_queries(it);
         for (int round = 0; more; round++, it = next) {
             const int ja = t ? it.ja[1] : it.ja[0], jb = t ? it.jb[1] : it.jb[0], row0 = t ? it.row0[1] : it.row0[0], head = t ? it.head[1] : it.head[0];
-            const int ja_o = t ? it.ja[0] : it.ja[1], jb_o = t ? it.jb[0] : it.jb[1];
             const int r_abs = row0 + row, r_live = min(r_abs, it.rows - 1);
             int pos_r, lb = 0, m_row = 0, h_row = 0;             // last and first visible position of this row; LINES: its batch row and head
             float sc, c1 = 0.f, cap_k = 0.f, slope = 0.f;
@@ -592,11 +593,11 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
 #pragma unroll
                     for (int c = 0; c < 4; c++) pt_probs<LINES>(v[c], sc, ref, pk[c], lo[c], sum);
                 }
-                if (j > ja) wait(&o_full[t], (ns - 1) & 1);      // this tile's P V before is complete
-                // and the other tile's, whose probabilities lie in this place, up to the one ahead of this in the issuer's order (one by one: a
-                // parity tells one phase from the next, no more)
-                if constexpr (LINES)
-                    for (const uint32_t up_to = other + max(0, min(j + t, jb_o) - ja_o); seen != up_to; seen++) wait(&o_full[t ^ 1], seen & 1);
+                // this tile's P V before is complete; LINES: and the other's, whose probabilities lie in this place.  Neither barrier can be more than the one
+                // phase ahead that a parity tells, as its next phase waits for the probabilities of this step (the phases of the other tile's o_full pass
+                // while this tile has no steps)
+                if constexpr (LINES) wait(&p_turn[t], ns & 1);
+                else if (j > ja) wait(&o_full[t], (ns - 1) & 1);
                 tc_fence_after();
                 if (moved && j > ja) {      // the accumulated output moves to the new reference (rare after the first steps)
                     uint32_t w[32];
@@ -620,7 +621,6 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
                 tc_fence_before();
                 mbar_arrive(&p_full[t]);
             }
-            other += jb_o - ja_o;
             more = item_at(round + 1, next);
             if (more) load_queries(next);
             // ---- finish: O / l -> f32 rows, partial sums, or the Q80 cast into the slabs of the wo matmul ----
@@ -722,6 +722,8 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
                 auto outputs = [&](int t, int j) {               // O += P V of a step
                     const int st = (g + j) & 1;
                     if (on(t, j)) {
+                        // whose P V comes next (between an item's first step and its last one of the tiles has one)
+                        const int next = t == 0 && on(1, j) ? 1 : on(0, j + 1) ? 0 : on(1, j + 1) ? 1 : -1;
                         wait(&p_full[t], ns[t]++ & 1);
                         tc_fence_after();
                         __syncwarp();
@@ -729,9 +731,16 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
                         pt_mma_ts(T_O, t_p(t), b_lo, desc_hi, idesc_pv, j > it.ja[t] ? 1u : 0u);
                         if constexpr (LINES) pt_mma_ts(T_O, t_p(t) + 64, b_lo, desc_hi, idesc_pv, 1u);
                         pt_commit(&o_full[t]);
+                        if (LINES && next >= 0) pt_commit(&p_turn[next]);
                     }
                     if (t == 1) pt_commit(&v_empty[st]);
                 };
+                // LINES: a tile may store probabilities when all that was issued ahead of its turn is complete
+                if (LINES && it.J > 0) {
+                    uint64_t* first = &p_turn[on(0, 0) ? 0 : 1];
+                    if (n_s > 0) pt_commit(first);
+                    else if (lane == 0) mbar_arrive(first);
+                }
                 scores(0, 0);
                 scores(1, 0);
                 scores(0, 1);
@@ -826,7 +835,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
 extern void dl_set_error(const char* fmt, ...);
 extern int dl_device_sm_count();
 
-#define PT_SMEM ((2 + 2 * PT_STAGES) * PT_TILE_BYTES + 8 * 32 * PT_OUT_LD * 4 + 20 * 8)
+#define PT_SMEM ((2 + 2 * PT_STAGES) * PT_TILE_BYTES + 8 * 32 * PT_OUT_LD * 4 + 22 * 8)
 
 typedef CUresult (*PtEncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,

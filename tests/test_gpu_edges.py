@@ -574,3 +574,50 @@ def test_window_shares(runs, n_splits, rows, ld):
     L().window_attention_tc(q, got, heads, kv, dim, 0, 0.1, 0.0, 0, pos, slot, bt, cache, tr, len(tiles), 16, n_splits, partial, vdim=dim)
     L().window_attention(q, want, M, heads, kv, dim, 0, 0.1, 0.0, 0, pos, slot, bt, cache, vdim=dim)
     assert ((got - want).norm(dim=1) <= 8e-3 * want.norm(dim=1)).all()
+
+
+def _window_batch(runs, heads, kv, window=0, softcap=0.0, chunk=0):
+    """Portions (first position, rows) of one sequence each on 128 / 128 bf16 lines, full list tiles, queries that bf16 holds: the tensor-core kernels' output
+    rows (a call of them) and the per-row kernel's."""
+    dim, rq = 128, L().window_tc_rows(heads, kv)
+    pages = max((p0 + n + 31) // 32 for p0, n in runs)
+    g = torch.Generator().manual_seed(len(runs) * 1000 + runs[0][1])
+    M = sum(n for _, n in runs)
+    cache = torch.randn(len(runs) * pages, kv, 32, 2 * dim, generator=g).bfloat16().cuda()
+    bt = torch.randperm(len(runs) * pages, generator=g).int().view(len(runs), pages).cuda()
+    pos, slot, tiles = [], [], []
+    for s, (p0, n) in enumerate(runs):
+        at = list(range(len(pos), len(pos) + n))
+        pos += list(range(p0, p0 + n))
+        slot += [s] * n
+        tiles += [at[i:i + rq] for i in range(0, n, rq)]
+    tr = torch.tensor([t + [-1] * (rq - len(t)) for t in tiles], dtype=torch.int32, device="cuda")
+    q = torch.randn(M, heads * dim, generator=g).bfloat16().float().cuda()
+    pos, slot = (torch.tensor(v, dtype=torch.int32, device="cuda") for v in (pos, slot))
+    want = torch.zeros(M, heads * dim, device="cuda")
+    L().window_attention(q, want, M, heads, kv, dim, 0, 0.1, softcap, window, pos, slot, bt, cache, vdim=dim, chunk=chunk)
+
+    def call():
+        out = torch.full((M, heads * dim), float("nan"), device="cuda")
+        L().window_attention_tc(q, out, heads, kv, dim, 0, 0.1, softcap, window, pos, slot, bt, cache, tr, len(tiles), rq, vdim=dim, chunk=chunk)
+        return out
+    return call, want
+
+
+@pytest.mark.parametrize("runs,heads,kv,opt", [([(0, 272), (0, 400)], 32, 8, {}),                       # one tile of a prompt and three of the next in a CTA
+                                               ([(96, 688), (0, 17)], 32, 8, {}),                      # three and one, the second tile a step longer
+                                               ([(100, 1100)], 32, 8, dict(window=1000)), ([(300, 1100)], 32, 8, dict(window=1024)),
+                                               ([(100, 1100)], 32, 8, dict(window=1024, softcap=50.0)), ([(300, 1200)], 16, 4, dict(window=256, softcap=50.0)),
+                                               ([(100, 1100)], 32, 8, dict(chunk=1024)),               # the border between the tiles' first positions
+                                               ([(300, 500), (0, 200), (1000, 1), (50, 1), (31, 1), (700, 3)], 32, 8, dict(window=512)),
+                                               ([(7 * k, 40 + 9 * k) for k in range(12)], 64, 8, {}), ([(k, 20 + k) for k in range(40)], 32, 8, dict(window=30))])
+def test_window_tiles_of_several_portions(runs, heads, kv, opt):
+    """Groups of four list tiles (more of them than SMs): several runs in a CTA, runs of one tile ahead of two and the reverse, tiles that start and end at
+    different steps; twenty calls give the same bits.  Probabilities in two bf16 numbers (2^-17), a chain of at most 32 steps that truncates by 2^-24 of the
+    running sum each, fast exponentials (2^-22): 2e-4 of a row covers them several times."""
+    assert (sum((n - 1) // (64 * kv // heads) + 1 for _, n in runs) + 1) // 2 * kv > 148
+    call, want = _window_batch(runs, heads, kv, **opt)
+    got = call()
+    assert ((got - want).norm(dim=1) <= 2e-4 * want.norm(dim=1)).all()
+    for _ in range(20):
+        assert torch.equal(call(), got)
