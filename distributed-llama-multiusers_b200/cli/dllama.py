@@ -28,6 +28,7 @@ class RootInference:
         self.engine = ctx.engine
         self.slot = self.engine.alloc_slot()
         self.is_cuda = self.engine.device.type == "cuda"
+        self.waits = getattr(self.engine, "waits", None)
         self.last_ms = 0.0
 
     def forward(self, tokens: List[int], pos: int, want_logits: bool = True):
@@ -45,6 +46,8 @@ class RootInference:
             e1.record()
             out = logits[0].float().cpu().numpy() if want_logits else None
             torch.cuda.synchronize()
+            if self.waits is not None:
+                self.waits.check()
             self.last_ms = e0.elapsed_time(e1)
         else:
             t0 = time.perf_counter()

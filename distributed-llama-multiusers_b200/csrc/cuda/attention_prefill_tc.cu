@@ -34,6 +34,9 @@
 // Reference semantics: multiheadAtt_F32 (src/nn/nn-cpu-ops.cpp:749-784), softmax in f32, output cast as OP_CAST
 // (src/llm.cpp:296-301).  KV cache: fp16 pages [page][kv_head][32][128].
 #include <cuda.h>
+#include <atomic>
+#include <cstring>
+#include <mutex>
 #include "epilogue.cuh"
 #include "f32_pairs.cuh"
 #include "window_tiles.cuh"
@@ -49,6 +52,11 @@
 #define PT_SHARE_STEPS 4
 #define PT_DEADLINE_NS 4000000000ull
 
+struct PtLimit {
+    unsigned long long ns;     // how long a CTA waits (0: not at all)
+    unsigned* status;          // host memory: the device's word of dl_attention_status()
+};
+
 struct PtArgs {
     const float* q;            // [M][n_heads*128]
     const __half* k_cache;     // [pages][n_kv][32][128]
@@ -63,6 +71,7 @@ struct PtArgs {
     int out_mcap;
     float* y_out;
     unsigned long long* tr;
+    PtLimit limit;
 };
 
 struct PtLineArgs {
@@ -73,6 +82,7 @@ struct PtLineArgs {
     int n_splits;
     int least;                 // runs of no more stacked rows belong to the other kernel (0: there is none)
     float* partial;            // [n_tiles][kv_heads][n_splits][64][130] where n_splits > 1: sums, reference maximum, sum of weights
+    PtLimit limit;
 };
 template <bool LINES> struct PtKernelArgs { typedef PtArgs T; };
 template <> struct PtKernelArgs<true> { typedef PtLineArgs T; };
@@ -263,20 +273,22 @@ struct PtItem {
     int begin;                             // batch row of the segment's first row; LINES: entry of tile_rows where the run starts
 };
 
-// A wait that gives up after PT_DEADLINE_NS: the flag ends the other waits, too, and every output of the CTA becomes a NaN
+// A wait that gives up (the CTA has had its time, PT_DEADLINE_NS): the flag ends the other waits, too, every output of the CTA becomes a NaN, and
+// the host learns of it by dl_attention_status()
 struct PtWaits {
     volatile int* gave_up;
-    unsigned long long t0;
+    unsigned long long t0, ns;
     DL_DEVINL void operator()(uint64_t* bar, uint32_t parity) const {
         unsigned n = 0;
         while (!mbar_try_wait(bar, parity)) {
             if ((++n & 0x3FFu) == 0) {
                 if (*gave_up) return;
-                if (globaltimer_ns() - t0 > PT_DEADLINE_NS) { *gave_up = 1; return; }
+                if (globaltimer_ns() - t0 > ns) { *gave_up = 1; return; }
             }
         }
     }
 };
+__device__ unsigned pt_times_given_up;
 
 // Llama path: the items of a batch are (128-row tile of a segment, query head), late tiles (long histories) first: two heads of one key/value head
 // side by side, or two tiles of one head where the heads come alone; single tiles while there are SMs for all of them.  Item `idx` of the
@@ -418,7 +430,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     pdl_launch_dependents();
     if (tid == 0) {
-        gave_up_s = 0;
+        gave_up_s = a.limit.ns == 0;
         for (int s = 0; s < 2; s++) {
             mbar_init(&k_full[s], 1);
             mbar_init(&k_empty[s], 1);
@@ -466,7 +478,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const PtWaits wait = {&gave_up_s, globaltimer_ns()};
+    const PtWaits wait = {&gave_up_s, globaltimer_ns(), a.limit.ns};
     const int n_seg = n_seg_s;
     // the items of this CTA, in the same order for every role; rounds run back and forth over the CTAs, so that a long item goes with a short one
     auto item_at = [&](int round, PtItem& it) {
@@ -823,7 +835,13 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
     }
     tc_fence_before();
     __syncthreads();
-    if (gave_up_s) __nanosleep(1000000);                         // copies and MMAs in flight end
+    if (gave_up_s) {
+        if (tid == 0) {
+            *(volatile unsigned*)a.limit.status = atomicAdd(&pt_times_given_up, 1u) + 1u;
+            __threadfence_system();
+        }
+        __nanosleep(1000000);                                    // copies and MMAs in flight end
+    }
     if (warp == 0) {
         tc_fence_after();
         tmem_dealloc(tmem_base, 512);
@@ -834,6 +852,34 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
 
 extern void dl_set_error(const char* fmt, ...);
 extern int dl_device_sm_count();
+
+// Words in host memory that kernels whose waits gave up write, one per device: the host reads them where it reads results, without a copy of their own.
+static std::atomic<unsigned long long> g_pt_limit{PT_DEADLINE_NS};
+static unsigned* pt_status_word() {
+    constexpr int devices = 64;
+    static std::mutex lock;
+    static unsigned* words = nullptr;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev >= devices) return nullptr;
+    std::lock_guard<std::mutex> guard(lock);
+    if (words == nullptr) {
+        void* p = nullptr;
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;       // the first launch may be a captured one
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        const cudaError_t e = cudaHostAlloc(&p, devices * sizeof(unsigned), cudaHostAllocPortable | cudaHostAllocMapped);
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (e != cudaSuccess) { cudaGetLastError(); return nullptr; }
+        words = (unsigned*)memset(p, 0, devices * sizeof(unsigned));
+    }
+    return words + dev;
+}
+extern "C" const unsigned* dl_attention_status() { return pt_status_word(); }
+extern "C" void dl_debug_set_attention_limit(unsigned long long ns) { g_pt_limit = ns; }
+static int pt_limit(PtLimit* l) {
+    *l = {g_pt_limit, pt_status_word()};
+    if (l->status == nullptr) { dl_set_error("attention_prefill_tc: no host memory for its status"); return -1; }
+    return 0;
+}
 
 #define PT_SMEM ((2 + 2 * PT_STAGES) * PT_TILE_BYTES + 8 * 32 * PT_OUT_LD * 4 + 22 * 8)
 
@@ -874,6 +920,7 @@ extern "C" int dl_attention_prefill_tc(const float* q, int M, int n_heads, int n
     a.q = q; a.k_cache = (const __half*)k_cache; a.v_cache = (const __half*)v_cache; a.pos = pos; a.slot = slot;
     a.block_table = block_table; a.meta = meta; a.M = M; a.n_heads = n_heads; a.n_kv_heads = n_kv_heads;
     a.max_pages = max_pages; a.xq_out = xq_out; a.xh_out = xh_out; a.out_mcap = out_mcap; a.y_out = y_out;
+    if (pt_limit(&a.limit) != 0) return -1;
     a.tr = dl_trace_next(TR_ATT);
     alignas(64) CUtensorMap kmap, vmap;
     const long long rows = (long long)n_cache_pages * n_kv_heads * 32;
@@ -925,6 +972,7 @@ int dl_window_prefill_tc(const DlWindowAttnArgs& w, const int* tile_rows, int n_
     a.w = w; a.tile_rows = tile_rows; a.n_tiles = n_tiles; a.rq = rq; a.rep = w.heads / w.kv_heads;
     a.group = group; a.n_splits = n_splits; a.partial = partial;
     a.least = alone ? 0 : 16;
+    if (pt_limit(&a.limit) != 0) return -1;
     const int groups = (n_tiles + group - 1) / group, z = dl_window_prefill_tc_shares(w, n_tiles, group, n_splits);
     alignas(64) CUtensorMap map;
     // the cache's page count is not known here; every copy reads a page that the block table names

@@ -71,6 +71,7 @@ import numpy as np
 import torch
 
 from ..formats.safetensors import SafetensorsFile
+from ..ops.lib import WaitStatus, layers_lib
 from .memory import graph_capture
 from .paging import PAGE, PageAllocator
 
@@ -1503,6 +1504,7 @@ class LayerListEngine:
         self._graph_launches: Dict[tuple, int] = {}
         self._graph_seen: Dict[tuple, int] = {}
         self._graph_stream = torch.cuda.Stream(device=dev)
+        self.waits = WaitStatus(layers_lib())
         self.layer_probe = None              # a list: forward() appends a copy of the residual stream after every layer
         torch.cuda.synchronize()
 
@@ -1934,6 +1936,7 @@ class LayerListEngine:
         """One forward over a batch of rows: any mix of prompt portions and single decoded tokens; rows of one sequence
         hold consecutive positions in order.  Returns the device logits [n][vocab] of rows logits_from.. (or of
         `logit_rows`, any rows in any order), valid until the next forward."""
+        self.waits.check()
         rows = list(logit_rows) if logit_rows is not None else list(range(logits_from, len(tokens)))
         M = self.set_batch(tokens, positions, slots, rows)
         self._run(M, len(rows), greedy)
@@ -1954,6 +1957,7 @@ class LayerListEngine:
         self.forward(tokens, positions, slots, logits_from, greedy=True)
         self.h_out_tokens.copy_(self.out_tokens, non_blocking=True)
         torch.cuda.current_stream().synchronize()
+        self.waits.check()
         return self.h_out_tokens[:n].tolist()
 
     def decode_greedy_host(self, tokens, positions, slots) -> List[int]:

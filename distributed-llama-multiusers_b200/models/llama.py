@@ -28,7 +28,7 @@ import torch
 from ..formats.mfile import ModelFile, HIDDEN_ACT_SILU
 from ..ops import kernels as K
 from ..ops import quant
-from ..ops.lib import EPI_QKV_ROPE, EPI_SILU_MUL, EPI_STORE
+from ..ops.lib import EPI_QKV_ROPE, EPI_SILU_MUL, EPI_STORE, WaitStatus
 from ..parallel.symm import SymmetricBuffer, validate_tp
 from .memory import graph_capture
 from .oracle import rope_frequencies
@@ -224,6 +224,7 @@ class LlamaEngine:
         self.argmax_scratch = torch.zeros(int(K.cuda_lib().dl_argmax_scratch_bytes(256)), dtype=torch.uint8,
                                           device=dev)
         self._init_mega(kv_dtype)
+        self.waits = WaitStatus(K.cuda_lib())
         self._staging_ev: Optional[torch.cuda.Event] = None
         self._graphs: Dict[Tuple, torch.cuda.CUDAGraph] = {}
         self._graph_launches: Dict[Tuple, int] = {}
@@ -754,6 +755,8 @@ class LlamaEngine:
         """One forward over a batch of rows (any mix of decode rows and prefill-chunk rows; rows of
         the same sequence must be in increasing position order).  Returns the device logits view
         [M - logits_from][vocab] (valid until the next forward)."""
+        if self.world == 1:              # (ranks wait for one another: they look where all of them have run a step)
+            self.waits.check()
         M = self.set_batch(tokens, positions, slots)
         o = self._run_batch(M, logits_from, greedy)
         return self.logits[o:o + M - logits_from]
@@ -775,6 +778,7 @@ class LlamaEngine:
         o = self._run_batch(M, logits_from, True)
         self.h_out_tokens.copy_(self.out_tokens, non_blocking=True)
         torch.cuda.current_stream().synchronize()
+        self.waits.check()
         return self.h_out_tokens[o:o + M - logits_from].tolist()
 
     def decode_greedy_host(self, tokens: List[int], positions: List[int], slots: List[int]) -> List[int]:
@@ -791,6 +795,7 @@ class LlamaEngine:
     def read_history(self, n_steps: int, M: int, first_step: int) -> np.ndarray:
         """Tokens produced by the last device-loop steps: [n_steps][M]."""
         raw = self.history.cpu().numpy()
+        self.waits.check()
         out = np.zeros((n_steps, M), dtype=np.int32)
         for i in range(n_steps):
             idx = (first_step + i) % self.history_cap

@@ -155,6 +155,7 @@ def cuda_lib():
     L = C.CDLL(CUDA_LIB_PATH)
     vp, i32, i64, u32, f32 = C.c_void_p, C.c_int, C.c_longlong, C.c_uint32, C.c_float
     L.dl_last_error.restype = C.c_char_p
+    L.dl_attention_status.restype = vp
     L.dl_device_sm_count.restype = i32
     L.dl_q40t_bytes.restype = i64
     L.dl_q40t_bytes.argtypes = [i32, i32]
@@ -425,6 +426,7 @@ def layers_lib():
             f"{LAYERS_LIB_PATH} is missing: run `python build.py layers` (nvcc, sm_100a) before using GPU ops")
     L = C.CDLL(LAYERS_LIB_PATH)
     vp, i32, i64, u32 = C.c_void_p, C.c_int, C.c_longlong, C.c_uint32
+    L.dl_attention_status.restype = vp
     L.dl_last_error.restype = C.c_char_p
     L.dl_device_sm_count.restype = i32
     L.dl_dense.argtypes = [C.POINTER(DlDenseArgs), vp]
@@ -514,6 +516,23 @@ def check_layers(rc: int, what: str = ""):
     if rc != 0:
         msg = layers_lib().dl_last_error().decode("utf-8", "replace")
         raise NativeLibraryError(f"{what} failed ({rc}): {msg}")
+
+
+class WaitStatus:
+    """Whether a wait inside a prompt attention kernel of `library` gave up on the current device (dl_attention_status): such a launch
+    returned 0 long ago and its outputs are NaN.  An engine looks where it has synchronised with its launches anyway."""
+
+    def __init__(self, library):
+        word = library.dl_attention_status()
+        self._word = C.c_uint.from_address(word) if word else C.c_uint(0)
+        self._seen = self._word.value
+
+    def check(self):
+        """Raises once for each change."""
+        now = self._word.value
+        if now != self._seen:
+            self._seen = now
+            raise NativeLibraryError("a wait inside a prompt attention kernel gave up: outputs of the launches since the last look are not valid")
 
 
 # kernels launched by this process (bench.py reports it as gpu_launches)

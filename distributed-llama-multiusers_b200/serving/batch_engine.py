@@ -61,6 +61,7 @@ class BatchEngine:
     def __init__(self, engine, tokenizer: T.Tokenizer, max_batch: Optional[int] = None,
                  prefill_chunk: Optional[int] = None, control: Optional[ControlChannel] = None):
         self.engine = engine
+        self._waits = getattr(engine, "waits", None)
         self.tok = tokenizer
         self.max_rows = engine.max_rows
         self.sched = T.Scheduler(self.max_rows, engine.n_slots, prefill_chunk or self.max_rows, engine.seq_len)
@@ -159,6 +160,11 @@ class BatchEngine:
                 print(f"🚨 engine step failed: {type(e).__name__}: {e}", flush=True)
                 self._fail_batch(e)
 
+    def _check_waits(self):
+        """Raises if an earlier launch's waits gave up: ahead of what the workers are told to run, and behind every synchronisation."""
+        if self._waits is not None:
+            self._waits.check()
+
     def step(self) -> int:
         """One scheduler step = one forward pass.  Returns the number of rows run."""
         t_a = time.perf_counter()
@@ -173,6 +179,7 @@ class BatchEngine:
         with self._lock:
             rows = [self.reqs.get(i) for i in sampling]
         greedy = all(r is not None and r.temperature == 0.0 for r in rows) and len(rows) > 0
+        self._check_waits()
         if self.control is not None:
             # workers replay exactly the root's launch: a pure prompt step computes the last row's logits only
             for s_, p_ in zip(slots, pos):          # a page shortage must surface before the workers are told to run
@@ -203,12 +210,14 @@ class BatchEngine:
             self._sample_rows(logits[:n_s], self._d_params[0], self._d_params[1], self._d_params[2], self._d_tok)
             self._h_tok.copy_(self._d_tok, non_blocking=True)
             torch.cuda.current_stream().synchronize()
+            self._check_waits()
             sampled = self._h_tok[:n_s].tolist()
         else:
             logits = eng.forward(toks, pos, slots, logits_from=lf)
             self._logits_host[:n_s].copy_(logits[:n_s], non_blocking=True)
             if logits.is_cuda:
                 torch.cuda.current_stream().synchronize()
+                self._check_waits()
             lh = self._logits_host.numpy()
             sampled = [r._sampler.sample(lh[i]) if r is not None else 0 for i, r in enumerate(rows)]
         t_c = time.perf_counter()
@@ -297,6 +306,7 @@ def worker_loop(engine, control: ControlChannel):
     fails on a worker is reported to the root through the mailbox (the root's next send raises) instead of leaving the
     root's kernels spinning on a rank that is gone."""
     torch.cuda.set_device(engine.device)
+    waits = getattr(engine, "waits", None)
     while True:
         pkt = control.recv()
         if pkt is None or pkt["op"] == OP_STOP:
@@ -308,6 +318,8 @@ def worker_loop(engine, control: ControlChannel):
                 engine.warmup_graphs()
                 continue
             if pkt["op"] == OP_FORWARD and pkt["M"] > 0:
+                if waits is not None:
+                    waits.check()
                 M = engine.set_batch(pkt["tokens"], pkt["positions"], pkt["slots"])
                 engine._run_batch(M, pkt["logits_from"], pkt["greedy"])
         except Exception as exc:        # noqa: BLE001 -- whatever it is, the root has to hear about it

@@ -30,6 +30,7 @@ class NativeApiServer:
                  prefill_chunk: Optional[int] = None, host: str = "0.0.0.0", port: int = 9990,
                  max_default_tokens: int = 128, verbose: bool = True):
         self.engine = engine
+        self._waits = getattr(engine, "waits", None)
         self.tok = tokenizer
         self.control = control
         self.host, self.port = host, port
@@ -139,6 +140,11 @@ class NativeApiServer:
                 # (the slots of the failed requests come back through the next dl_srv_next_batch)
                 L.dl_srv_fail_batch(h, f"{type(e).__name__}: {e}".encode("utf-8", "replace"))
 
+    def _check_waits(self):
+        """Raises if an earlier launch's waits gave up: ahead of what the workers are told to run, and behind every synchronisation."""
+        if self._waits is not None:
+            self._waits.check()
+
     def step(self) -> int:
         """One scheduler step = one forward pass.  Returns the number of rows run."""
         L, h, eng, R = self._L, self._h, self.engine, self.max_rows
@@ -154,6 +160,7 @@ class NativeApiServer:
         if n <= 0:
             return 0
         dn = self._desc_np
+        self._check_waits()
         toks, pos, slots = dn[0, :n].tolist(), dn[1, :n].tolist(), dn[2, :n].tolist()
         if self.control is not None:
             # workers replay exactly the root's launch: a pure prompt step computes the last row's logits only
@@ -173,6 +180,7 @@ class NativeApiServer:
             self._sample_rows(logits[:n_s], self._d_params[0], self._d_params[1], self._d_params[2], self._d_tok)
             self._h_tok.copy_(self._d_tok, non_blocking=True)
             torch.cuda.current_stream().synchronize()
+            self._check_waits()
             rc = L.dl_srv_commit(h, n_s, self._h_tok.data_ptr())
         else:
             logits = eng.forward(toks, pos, slots, logits_from=lf)
@@ -180,6 +188,7 @@ class NativeApiServer:
             lh[:n_s].copy_(logits[:n_s], non_blocking=True)
             if logits.is_cuda:
                 torch.cuda.current_stream().synchronize()
+                self._check_waits()
             L.dl_srv_sample_host(h, lh.data_ptr(), lh.stride(0), self._h_tok.data_ptr())
             rc = L.dl_srv_commit(h, n_s, self._h_tok.data_ptr())
         if rc < 0:

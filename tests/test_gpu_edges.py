@@ -1,4 +1,6 @@
 """Edges of the kernels' tiles and of the rules that choose between kernels, against plain 64-bit references."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
@@ -621,3 +623,50 @@ def test_window_tiles_of_several_portions(runs, heads, kv, opt):
     assert ((got - want).norm(dim=1) <= 2e-4 * want.norm(dim=1)).all()
     for _ in range(20):
         assert torch.equal(call(), got)
+
+
+def _give_up(library):
+    """A limit that is over before the kernel starts: its waits for copies end at once, none is left forever."""
+    library.dl_debug_set_attention_limit.argtypes = [C.c_ulonglong]
+    library.dl_debug_set_attention_limit(0)
+    return lambda: library.dl_debug_set_attention_limit(4_000_000_000)
+
+
+def test_a_wait_that_gives_up_reaches_the_caller(tmp_path):
+    """Prompt attention of both kinds: the status word changes once for a launch whose waits gave up and never for others; an engine raises where it
+    reads its tokens, and at the next batch where it does not, once, and goes on."""
+    from dllama_b200.formats import mfile
+    from dllama_b200.models.llama import LlamaEngine
+    from dllama_b200.ops import lib as B
+    call = _prompt(300, 16, 4)
+    status, want = B.WaitStatus(B.layers_lib()), call()
+    restore = _give_up(B.layers_lib())
+    try:
+        out = call()
+        torch.cuda.synchronize()
+    finally:
+        restore()
+    assert out.isnan().any()
+    with pytest.raises(B.NativeLibraryError, match="gave up"):
+        status.check()
+    assert torch.equal(call(), want)
+    status.check()
+
+    path = str(tmp_path / "m.m")
+    mfile.write_random_model(path, dict(mfile.MODEL_SHAPES["tiny"], dim=1024, hidden_dim=2048), exact=True, seed=3)
+    e = LlamaEngine(path, max_rows=256, n_slots=2, max_seq_len=512, use_graphs=False)
+    slot, n = e.alloc_slot(), 200
+    batch = (np.random.default_rng(0).integers(1, 1000, n).tolist(), list(range(n)), [slot] * n)
+    token = e.decode_step_greedy(*batch, logits_from=n - 1)
+    for step in (e.decode_step_greedy, e.forward):
+        restore = _give_up(B.cuda_lib())
+        try:
+            with pytest.raises(B.NativeLibraryError, match="gave up"):
+                step(*batch, logits_from=n - 1)
+                torch.cuda.synchronize()             # forward alone: the next batch raises
+                step(*batch, logits_from=n - 1)
+        finally:
+            restore()
+        torch.cuda.synchronize()
+        assert e.decode_step_greedy(*batch, logits_from=n - 1) == token
+    e.close()

@@ -507,3 +507,23 @@ def test_native_server_sheds_load_when_the_admission_queue_is_full(tok, monkeypa
         assert st["free_slots"] == 1 and st["waiting"] == 0 and st["running"] == 0
     finally:
         srv.close()
+
+
+def test_a_wait_that_gave_up_fails_the_requests_of_that_time(tok):
+    """An engine whose status word changed (a kernel's wait gave up, its outputs are NaN): the running request gets an error and the next one its answer."""
+    from dllama_b200.ops import lib
+    eng = _FakeEngine(max_rows=8, n_slots=2, seq_len=256)
+    eng.waits = lib.WaitStatus(type("NoDevice", (), {"dl_attention_status": lambda self: None})())
+    srv = NativeApiServer(eng, tok, "fake.m", A.InferenceParams(messages=[], temperature=0.0, top_p=0.9, seed=1), host="127.0.0.1", port=0, verbose=False)
+    srv.start()
+    ask = {"messages": [{"role": "user", "content": "hello"}], "max_tokens": 4}
+    try:
+        eng.waits._word.value = 3
+        with pytest.raises(urllib.error.HTTPError) as e:
+            _post(srv.port, ask)
+        assert e.value.code == 500 and "gave up" in json.load(e.value)["error"]["message"]
+        with _post(srv.port, ask) as r:
+            assert json.load(r)["usage"]["completion_tokens"] >= 1
+        assert srv.n_errors == 1
+    finally:
+        srv.close()
