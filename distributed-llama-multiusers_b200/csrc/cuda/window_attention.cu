@@ -844,6 +844,23 @@ extern "C" long long dl_window_tc_partial_floats(int n_tiles, int kv_heads, int 
     return (long long)n_tiles * kv_heads * n_splits * WM_ROWS * (dim + 2);
 }
 
+// Which kernel has work, by the number of rows: a row or so per tile is decoding (mma.sync alone, as it takes all tiles then), tiles as good as
+// full are one prompt (tcgen05 alone, likewise); else, or where the rows are not said, both.  A kernel without work costs its launch (us, both and the one: 8 rows under a
+// window of 256 21.1 and 15.4, a prompt of 32 rows 15.6 and 13.0, of 2000 under 1024 43.2 and 39.6)
+struct WindowRoute { bool mma, tc5, decode; };
+static WindowRoute window_route(const DlWindowAttnArgs& a, int n_tiles, int rq, int n_splits) {
+    const int rep = a.heads / a.kv_heads;
+    const bool can_tc5 = dl_window_prefill_tc_supported(a, rq) == 0;
+    const bool decode = a.rows > 0 && (((long long)a.rows - n_tiles + 1) * rep <= 16 || (a.rows == n_tiles && n_splits > 1));
+    const bool prompt = can_tc5 && a.rows <= (long long)n_tiles * rq && a.rows > (n_tiles - 1ll) * rq + 16 / rep;
+    return {!prompt, prompt || (can_tc5 && !decode), decode};
+}
+// 1: mma.sync, 2: tcgen05, 3: both
+extern "C" int dl_window_attention_tc_route(const DlWindowAttnArgs* args, int n_tiles, int rq, int n_splits) {
+    const WindowRoute r = window_route(*args, n_tiles, rq, n_splits);
+    return (r.mma ? 1 : 0) | (r.tc5 ? 2 : 0);
+}
+
 // n_splits > 1 (few tiles, e.g. decoding): grid.z CTAs share a tile's pages and leave partial sums in `partial`
 // (dl_window_tc_partial_floats() f32) that a merge launch combines.
 extern "C" int dl_window_attention_tc(const DlWindowAttnArgs* args, const int* tile_rows, int n_tiles, int rq, int n_splits,
@@ -860,15 +877,10 @@ extern "C" int dl_window_attention_tc(const DlWindowAttnArgs* args, const int* t
     if (n_tiles < 1) return 0;
     if (n_splits < 1 || n_splits > WM_MAX_SPLITS || (n_splits > 1 && partial == nullptr)) { dl_set_error("dl_window_attention_tc: n_splits %d without scratch", n_splits); return -1; }
     // tiles of more than 16 stacked rows are prompt portions: tcgen05, 128 stacked rows to a CTA, 256 where that fills the SMs
-    const bool can_tc5 = dl_window_prefill_tc_supported(a, rq) == 0;
     const int group = (n_tiles + 1) / 2 * a.kv_heads <= dl_device_sm_count() ? 2 : 4;
-    // Which kernel has work, by the number of rows: a row or so per tile is decoding (mma.sync alone, as it takes all tiles then), tiles as good as
-    // full are one prompt (tcgen05 alone, likewise); else both.  A kernel without work costs its launch (us, both and the one: 8 rows under a window of
-    // 256 21.1 and 15.4, a prompt of 32 rows 15.6 and 13.0, of 2000 under 1024 43.2 and 39.6)
     const int rep = a.heads / a.kv_heads;
-    const bool decode = a.rows > 0 && (((long long)a.rows - n_tiles + 1) * rep <= 16 || (a.rows == n_tiles && n_splits > 1));
-    const bool prompt = can_tc5 && a.rows <= (long long)n_tiles * rq && a.rows > (n_tiles - 1ll) * rq + 16 / rep;
-    const bool tc5 = can_tc5 && !decode;
+    const WindowRoute route = window_route(a, n_tiles, rq, n_splits);
+    const bool tc5 = route.tc5, decode = route.decode, prompt = !route.mma;
     if (prompt) {
         if (n_splits > 1) n_splits = dl_window_prefill_tc_shares(a, n_tiles, group, n_splits);
         const int rc = dl_window_prefill_tc(a, tile_rows, n_tiles, rq, group, n_splits, partial, true, (cudaStream_t)stream);

@@ -651,7 +651,7 @@ class WindowAttentionMixer:
                                     value_heads=opts.get("value_heads", 0), softcap=self.softcap, slope=self.slope, gate=opts["gate"])
             else:
                 L.window_attention_tc(qk, o, H, G, d, rd, self.scale, self.softcap, self.window, e.pos, e.slot, e.block_table,
-                                      self.cache, tile_rows, n_tiles, rq, n_splits, partial, **opts)
+                                      self.cache, tile_rows, n_tiles, rq, n_splits, partial, rows=M, **opts)
         else:
             L.window_attention(q_in, o, M, H, G, d, rd, self.scale, self.softcap, self.window, e.pos, e.slot, e.block_table,
                                self.cache, **opts)

@@ -572,6 +572,12 @@ def window_tc_supported(heads: int, kv_heads: int, dim: int, rope_dims: int, cac
     return layers_lib().dl_window_attention_tc_supported(heads, kv_heads, dim, rope_dims, ctype) == 0
 
 
+def window_tc_route(heads: int, kv_heads: int, dim: int, vdim: int, rows: int, n_tiles: int, rq: int, n_splits: int = 1) -> int:
+    """Kernels that window_attention_tc launches for `rows` rows on a bf16 cache: 1 = mma.sync, 2 = tcgen05, 3 = both."""
+    a = DlWindowAttnArgs(heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, rows=rows, ctype=T_BF16, page_size=PAGE_SIZE)
+    return int(layers_lib().dl_window_attention_tc_route(a, n_tiles, rq, n_splits))
+
+
 def window_tc_partial_floats(n_tiles: int, kv_heads: int, n_splits: int, dim: int) -> int:
     return int(layers_lib().dl_window_tc_partial_floats(n_tiles, kv_heads, n_splits, dim))
 
@@ -580,11 +586,14 @@ def window_attention_tc(q: torch.Tensor, out: torch.Tensor, heads: int, kv_heads
                         softcap: float, window: int, pos, slot, block_table: torch.Tensor, cache: torch.Tensor,
                         tile_rows: torch.Tensor, n_tiles: int, rq: int, n_splits: int = 1, partial: Optional[torch.Tensor] = None,
                         vdim: int = 0, chunk: int = 0, sink: Optional[torch.Tensor] = None, slope: Optional[torch.Tensor] = None,
-                        gate: Optional[torch.Tensor] = None):
+                        gate: Optional[torch.Tensor] = None, rows: Optional[int] = None):
     """The tensor-core kernel over row tiles (tile_rows int32 [n_tiles][rq] on the device, -1 = no row).  n_splits > 1:
-    that many CTAs share each tile's pages (few tiles: decoding) and a merge launch follows; partial: f32 scratch."""
+    that many CTAs share each tile's pages (few tiles: decoding) and a merge launch follows; partial: f32 scratch.  rows: rows of the
+    batch where q has more of them; which kernels are launched goes by it (window_tc_route)."""
     a = _window_args(q, out, heads, kv_heads, dim, rope_dims, scale, softcap, window, pos, slot, block_table, cache, vdim, chunk, sink,
                      slope=slope, gate=gate)
+    if rows is not None:
+        a.rows = rows
     if n_splits > 1:
         assert partial is not None and partial.numel() >= window_tc_partial_floats(n_tiles, kv_heads, n_splits, dim)
     check_layers(layers_lib().dl_window_attention_tc(a, tile_rows.data_ptr(), n_tiles, rq, n_splits, _p(partial), _stream()),

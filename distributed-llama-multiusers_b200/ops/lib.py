@@ -452,6 +452,8 @@ def layers_lib():
     L.dl_window_tc_rows.argtypes = [i32, i32]
     L.dl_window_attention_tc_supported.argtypes = [i32, i32, i32, i32, i32]
     L.dl_window_attention_tc.argtypes = [C.POINTER(DlWindowAttnArgs), vp, i32, i32, i32, vp, vp]
+    L.dl_window_attention_tc_route.argtypes = [C.POINTER(DlWindowAttnArgs), i32, i32, i32]
+    L.dl_window_attention_tc_route.restype = i32
     L.dl_window_tc_partial_floats.argtypes = [i32, i32, i32, i32]
     L.dl_window_tc_partial_floats.restype = i64
     L.dl_talk_attention_tc_supported.argtypes = [i32] * 7

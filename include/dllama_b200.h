@@ -739,6 +739,8 @@ int dl_window_attention_tc_supported(int heads, int kv_heads, int dim, int rope_
 long long dl_window_tc_partial_floats(int n_tiles, int kv_heads, int n_splits, int dim);
 int dl_window_attention_tc(const DlWindowAttnArgs* args /*host*/, const int* tile_rows, int n_tiles, int rq, int n_splits,
                            float* partial, void* stream);
+/* the kernels that it launches for args->rows rows: 1 = mma.sync, 2 = tcgen05, 3 = both (which differ by rounding alone) */
+int dl_window_attention_tc_route(const DlWindowAttnArgs* args, int n_tiles, int rq, int n_splits);
 /* Attention weights mixed across heads AFTER the softmax: with wide[m][g][c * vdim + i] = sum_j p_g(j) v_c,j[i] (every head's
  * weights against the values of all key/value heads), out[m][h * vdim + i] = sum_g talk[h][g] wide[m][g][c(h) * vdim + i],
  * c(h) = h / (heads / kv_heads).  To out (f32) or, with xh, into the tcgen05 GEMM's activation image. */

@@ -328,6 +328,31 @@ def test_window_decode_is_whole_before_what_follows(M, heads, kv, graph):
             assert torch.equal(t, ref)
 
 
+def test_window_routes_of_an_engine(tmp_path, monkeypatch):
+    """An engine says its batch's rows, not its own capacity: a portion of 700 rows of 1024 is tcgen05's alone, decoding mma.sync's, both together both."""
+    from dllama_b200.models import registry
+    from dllama_b200.models.layered import write_random_model
+    layer = {"type": "attention", "mixer": {"heads": 16, "kv_heads": 4, "dim": 128, "vdim": 128, "scale": 0.1, "mask": {"size": 512}},
+             "mlp": {"kind": "dense", "ff": 64}}
+    write_random_model(str(tmp_path), {"architecture": "Venadra", "width": 64, "vocab": 64, "norm": {"eps": 1e-5}, "embedding": {"scale": 1.0},
+                                       "canon": {"taps": 3}, "layers": [layer]}, seed=2)
+    eng = registry.engine_for_dir(str(tmp_path), max_rows=1024, n_slots=4, max_seq_len=1024, dtype="bfloat16")
+    routes, call = [], L().window_attention_tc
+
+    def spy(q, out, heads, kv, dim, rd, *a, **opts):
+        n_tiles, rq, n_splits = a[-4:-1]
+        routes.append(L().window_tc_route(heads, kv, dim, opts["vdim"], opts.get("rows", q.shape[0]), n_tiles, rq, n_splits))
+        call(q, out, heads, kv, dim, rd, *a, **opts)
+    monkeypatch.setattr(L(), "window_attention_tc", spy)
+    tokens = torch.randint(0, 64, (700,), generator=torch.Generator().manual_seed(0)).tolist()
+    slots = [eng.alloc_slot() for _ in range(3)]
+    eng.forward(tokens, range(700), [slots[0]] * 700)
+    eng.forward(tokens[:2], [700, 0], slots[:2])
+    eng.forward(tokens[:200] + [5], list(range(200)) + [701], [slots[2]] * 200 + [slots[0]])
+    assert routes == [2, 1, 3]
+    eng.close()
+
+
 def _prompt(rows, heads, kv, scale=None, keys=None, seed=5, **opt):
     """A prompt of `rows` positions in one sequence on 128 / 128 bf16 lines, no page shares: call() runs it and returns the output rows."""
     dim, pages = 128, (rows + 31) // 32

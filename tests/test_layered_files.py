@@ -345,3 +345,13 @@ def test_silizen_oracle_sink_delta_rule_read_ahead_and_prefix_property():
     o, _ = S.wkv_rows(q, k, v, f, bonus)
     assert torch.allclose(o[0], (q[0] * bonus * k[0]).sum(-1, keepdim=True) * v[0], atol=1e-12)
     assert torch.allclose(o[1], (q[1] * bonus * k[1]).sum(-1, keepdim=True) * v[1] + (q[1] * k[0]).sum(-1, keepdim=True) * v[0], atol=1e-12)
+
+
+def test_window_attention_routes():
+    """Which kernels have work, by the rows said: tiles that are all prompts' (16 of 16 stacked rows at least in each) are tcgen05's, a row or so per tile is
+    mma.sync's, everything else and rows that are not said are both's; lines or tiles that tcgen05 does not take are mma.sync's."""
+    from dllama_b200.ops import layers
+    route = layers.window_tc_route
+    assert [route(32, 8, 128, 128, n, 44, 16) for n in (692, 693, 704, 705, 47, 48)] == [3, 2, 2, 3, 1, 3]
+    assert [route(32, 8, 128, 128, 0, 44, 16), route(32, 8, 128, 128, 32, 32, 16, 4), route(32, 8, 128, 128, 700, 175, 4)] == [3, 1, 1]
+    assert [route(16, 4, 64, 64, 700, 44, 16), route(16, 4, 128, 0, 700, 44, 16), route(16, 16, 128, 128, 700, 11, 64)] == [1, 1, 2]
