@@ -271,8 +271,8 @@ def test_dense_few_rows(M, N, K_, dtype, round_x):
         assert close(half, torch.nn.functional.gelu(z[:, 0::2], approximate="tanh") * z[:, 1::2])
 
 
-def _one_row_tiles(contexts, heads, kv, seed):
-    """Decoding rows of sequences of these lengths on 128 / 128 bf16 lines: call(out) runs the attention, n_splits == 1."""
+def _one_row_tiles(contexts, heads, kv, seed, extra=0):
+    """Decoding rows of sequences of these lengths on 128 / 128 bf16 lines: call(out) runs the attention, n_splits == 1.  extra: rows of q behind them."""
     M, dim = len(contexts), 128
     g = torch.Generator(device="cuda").manual_seed(seed)
     need = [(t + 31) // 32 for t in contexts]
@@ -281,8 +281,9 @@ def _one_row_tiles(contexts, heads, kv, seed):
     for m in range(M):
         bt[m, :need[m]] = perm[sum(need[:m]):sum(need[:m + 1])]
     cache = torch.randn(sum(need), kv, 32, 2 * dim, generator=g, device="cuda").bfloat16()
-    q = torch.randn(M, heads * dim, generator=g, device="cuda")
+    q = torch.randn(M + extra, heads * dim, generator=g, device="cuda")
     rq = L().window_tc_rows(heads, kv)
+    assert L().window_tc_route(heads, kv, dim, dim, M + extra, M, rq) == (3 if extra else 1)
     tiles = torch.full((M, rq), -1, dtype=torch.int32)
     tiles[:, 0] = torch.arange(M, dtype=torch.int32)
     pos, slot = torch.tensor([t - 1 for t in contexts], dtype=torch.int32, device="cuda"), torch.arange(M, dtype=torch.int32, device="cuda")
@@ -291,11 +292,11 @@ def _one_row_tiles(contexts, heads, kv, seed):
 
 
 @pytest.mark.parametrize("M,heads,kv,graph", [(80, 16, 4, False), (40, 32, 8, True)])
-def test_window_decode_is_whole_before_what_follows(M, heads, kv, graph):
+def test_window_decode_is_whole_before_what_follows(M, heads, kv, graph, extra=0):
     """Many decoding rows without page shares, one context much longer than the others, and behind them a programmatically launched product
     that reads the output (a gate on it, then its image): the same bits as with a synchronisation in between."""
     width, N = heads * 128, 256
-    attend = _one_row_tiles([4000] + [1] * (M - 1), heads, kv, M)
+    attend = _one_row_tiles([4000] + [1] * (M - 1), heads, kv, M, extra)
     g = torch.Generator(device="cuda").manual_seed(1)
     w, w2 = (L().make_wh((torch.randn(n, k, generator=g, device="cuda") * k ** -0.5).bfloat16()) for n, k in ((width, N), (N, width)))
     x, ncap = torch.randn(M, N, generator=g, device="cuda"), (M + 7) // 8 * 8
@@ -326,6 +327,12 @@ def test_window_decode_is_whole_before_what_follows(M, heads, kv, graph):
         torch.cuda.synchronize()
         for t, ref in zip((out, gated, y), want):
             assert torch.equal(t, ref)
+
+
+@pytest.mark.parametrize("M,heads,kv,graph", [(80, 16, 4, False), (40, 32, 8, True)])
+def test_window_decode_beside_another_grid_is_whole_before_what_follows(M, heads, kv, graph):
+    """The same with rows enough said for a prompt among them, so that the grid of the tall tiles is launched between, too."""
+    test_window_decode_is_whole_before_what_follows(M, heads, kv, graph, extra=1000)
 
 
 def test_window_routes_of_an_engine(tmp_path, monkeypatch):
