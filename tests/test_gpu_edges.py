@@ -448,6 +448,25 @@ def test_window_prompt_non_finite_keys(value):
         assert bad.all() if value != value else bad.view(-1, 16).any(dim=1).float().mean() > 0.9
 
 
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+@pytest.mark.parametrize("window,at", [(0, 104), (0, 680), (0, 1130), (256, 650), (150, 330), (1000, 40)])
+def test_window_prompt_non_finite_values(value, window, at):
+    """A value that is not finite reaches the tile of 32 positions that holds it and those that see it, or whose first page does: the tile beside one of them in
+    a CTA is as without it."""
+    rows = 1201
+    clean = _prompt(rows, 16, 4, window=window)()
+
+    def spoil(cache):
+        cache[at // 32, :, at % 32, 128:] = value
+    out = _prompt(rows, 16, 4, window=window, keys=spoil)()
+    first = torch.arange(rows, device="cuda") // 32 * 32                       # of a row's tile
+    reached = (first + 31 >= at) & (((first - window + 1).clamp(min=0) // 32 * 32 <= at) if window else torch.ones_like(first, dtype=torch.bool))
+    assert torch.equal(out[~reached], clean[~reached])
+    seen = torch.arange(rows, device="cuda")
+    seen = (seen >= at) & ((seen - at < window) if window else True)
+    assert not torch.isfinite(out[seen]).any()
+
+
 @pytest.mark.parametrize("M,N,K_,batch,dtype", [(1, 40, 2048, 1, "bf16"), (1, 30000, 256, 1, "bf16"), (2, 24, 512, 3, "bf16"), (2, 9000, 128, 2, "f32"), (3, 20000, 264, 1, "bf16"),
                                                 (4, 1000, 256, 24, "bf16"), (4, 64, 4096, 1, "f32"), (8, 3000, 72, 8, "f32"), (32, 64, 64, 1, "f32"), (16, 2000, 64, 16, "f32"),
                                                 (25, 100, 520, 1, "f32")])

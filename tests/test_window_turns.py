@@ -79,13 +79,14 @@ def stall(items, rule, rng):
                     yield "p_full", t, ns[t]
                     ns[t] += 1
                     queue.append(("pv", t))
-                    queue.append(("o_full", t))
                     after = [u for u, k in ((1, j) if t == 0 else (0, j + 1), (0, j + 1), (1, j + 1)) if on(u, k)]
                     if after:
                         turn(after[0])
+                    if rule == "replay" or j + 1 == jb[t]:
+                        queue.append(("o_full", t))
 
     def softmax(t):
-        ns = nq = other = seen = 0
+        ns = nq = no = other = seen = 0
 
         def load(of):
             nonlocal nq
@@ -120,7 +121,8 @@ def stall(items, rule, rng):
             if i + 1 < len(items):
                 yield from load(items[i + 1])
             if jb[t] > ja[t]:
-                yield "o_full", t, ns - 1
+                yield "o_full", t, (no if rule == "turn" else ns - 1)
+                no += 1
 
     roles = [issuer(), softmax(0), softmax(1)]
     weight = [rng.choice([1, 1, 8]) for _ in range(4)]
