@@ -16,7 +16,8 @@
 //                 [token][head dim] in the cache, i.e. N-contiguous: no transpose anywhere), accumulating in TMEM
 // CTAs are persistent: each walks its items (pt_item), long ones first and rounds back and forth, and loads the next item's queries ahead of this one's
 // outputs.  What bounds it: the MMAs.  With one tile per CTA scores, softmax and P V of a step followed each other (1950 clk a step for 1024 of MMAs) and
-// every CTA paid 13 us for its start and end: 4001 rows of 32 heads 215 us, 147 here (two steps in 1.75 us; the rest is starts, ends and diagonals).
+// every CTA paid 13 us for its start and end: 4001 rows of 32 heads 229 us on inputs in turn, 170 here (215 and 147 on the same inputs again and again: two
+// steps in 1.75 us; the rest is starts, ends and diagonals).
 //
 // Warp roles (384 threads): warps 0-3 and 4-7 softmax of tile 0 and 1, warp 8 issues all MMAs (one issuer, or the tiles run in step; in convergent code, see
 // pt_mma_ss), warp 9 K producer and warp 10 V producer (one lane each issues 8 tensor copies of 4 KB per step).
@@ -28,8 +29,9 @@
 // remainder, and P V two MMAs: rounded to
 // one (2^-9) they are the larger share of the error, and how large depends on how often a row's maximum, whose probability is exact, moves
 // (2000 tokens under a window of 1024, against 64 bits: 1.93e-3 with one number, 1.47e-3 with two).  They take 128 columns, so the tiles take one such
-// buffer in turn, too.  2000 rows of 16 heads on 4 under a window of 1024: one run of 128 rows per CTA, in two waves, 54 us; 38 here; 512 rows in
-// page shares on mma.sync 62 us, 19 here.
+// buffer in turn, too.  2000 rows of 16 heads on 4 under a window of 1024: one run of 128 rows per CTA, in two waves, 55.5 us; 41 here; 512 rows in
+// page shares on mma.sync 62 us, 17 to 19 here.  The tiles' values are shared, but each multiplies only the groups of 16 tokens that it sees (the last of them may
+// hold some of the other's, where a portion starts inside a group).
 //
 // Reference semantics: multiheadAtt_F32 (src/nn/nn-cpu-ops.cpp:749-784), softmax in f32, output cast as OP_CAST
 // (src/llm.cpp:296-301).  KV cache: fp16 pages [page][kv_head][32][128].
@@ -224,9 +226,8 @@ DL_DEVINL void pt_q80_block(const float (&v)[32], int m, int kblock, int mcap, u
     }
 }
 
-// The eight MMAs of a group (K = 128) by one thread of the converged warp.  What bounds a group of 128 x 128 x 16 MMAs is their issue: inside an
-// `if (elect)` every descriptor passes through registers of its own into the uniform ones, 110 clk an MMA that takes 64; predicated in convergent code
-// they are formed there.
+// The eight MMAs of a group (K = 128) by one thread of the converged warp, elected by a predicate: with one MMA at a time inside an `if (elect)`
+// 4001 rows of 32 heads took 150 us, 138 so (on the same inputs again and again, with the queries loaded by warps of their own).
 // D += A B^T, both operands 128-byte-swizzled half tiles 16 KB apart (32 B of a row per MMA)
 DL_DEVINL void pt_mma_ss(uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t desc_hi, uint32_t idesc, uint32_t accumulate) {
     asm volatile(

@@ -310,9 +310,8 @@ DL_DEVINL void umma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                  : "memory");
 }
-// The eight MMAs (K = 16 each) of a 128-wide k-tile, and a commit, by one thread of a CONVERGED warp: predicated, so that the descriptors are
-// formed in uniform registers.  Inside an `if (elect)` each of them passes through a register of its own into the uniform ones first, about
-// 110 clk per MMA: what bounds an issuer of short MMAs.  Operands in shared memory: K-major core matrices 128 B apart (two per MMA).
+// The eight MMAs (K = 16 each) of a 128-wide k-tile, and a commit, by one thread of a CONVERGED warp: elected by a predicate, not by a branch.
+// The few-row products (norm, gate|up and down of 4096 x 14336 at 32 rows) took 79.9 us with one MMA at a time inside an `if (elect)`, 78.0 so.  Operands in shared memory: K-major core matrices 128 B apart (two per MMA).
 DL_DEVINL void umma_f16_ss_x8(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t desc_hi, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p, q, r;\n\t.reg .b32 x, y;\n\t.reg .b64 a, b;\n\t"

@@ -1,13 +1,13 @@
 // Persistent decode step: ONE cooperative kernel per token (M <= 4 rows) instead of ~160 launches.
 //
-// Why (measured, profiles/README.md sections 2 and 4): single-stream decode of an 8B model is five
+// Why (measured): single-stream decode of an 8B model is five
 // latency-bound kernels per layer -- each pays launch + dependency release + prologue + pipeline fill
 // while its weights stream for 1-5 us -- and at TP=8 two fence/counter/flag hand-offs on top.  Here the
 // whole forward pass (the reference's 839 op-steps + 66 socket syncs per token, src/nn/nn-executor.cpp:
 // 134-163 over the graph of src/llm.cpp:126-438) is one grid of one CTA per SM:
 //
 //  * a producer warp walks the weight schedule of ALL phases of ALL layers and keeps a 12-stage ring of
-//    bulk async copies (UBLKCP) full; it never waits for a phase boundary, so while the consumers sit in
+//    bulk async copies full; it never waits for a phase boundary, so while the consumers sit in
 //    a grid barrier or wait for a peer GPU the next phase's Q40T rows are already landing in shared memory;
 //  * 16 consumer warps run the phases: [merge-add + RMSNorm + Q80] -> qkv GEMV (+RoPE, paged KV write) ->
 //    split-KV attention -> [split merge + Q80] -> wo GEMV -> [merge-add + RMSNorm + Q80] -> w1|w3 GEMV

@@ -12,10 +12,10 @@
 // expand it in registers and write it with tcgen05.st straight into TENSOR MEMORY, and the MMA takes
 // its A operand from there (`tcgen05.mma [d], [a_tmem], b_desc`).  The first version staged fp16 A
 // tiles in smem: 32 KB written + 32 KB read per 9 KB of weights saturated the 128 B/clk crossbar
-// (per-tile timeline in profiles/: 1450 clk per k-tile, all of it in the MMA queue).
+// (1450 clk per k-tile, all of it in the MMA queue).
 //
 // Warp roles (672 threads):
-//   warp 0       producer: bulk async copies (UBLKCP) of raw 9 KB Q40T tiles (lanes 0-3) and XH slabs (lanes 4-7)
+//   warp 0       producer: bulk async copies of raw 9 KB Q40T tiles (lanes 0-3) and XH slabs (lanes 4-7)
 //   warps 1,18-20 MMA issuers (one elected lane each; tcgen05.mma / tcgen05.commit), k-tiles round-robin,
 //                one accumulator each; warp 1 also allocates TMEM
 //   warps 2-17   dequantisers, 4 groups x 4 warps: group = k-tile % 4 = A stage, warp % 4 = TMEM lane
@@ -161,10 +161,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_q40_tc_kernel(const __grid
     } else if (warp == 1 || warp >= 2 + TC_DEQ_WARPS) {
         // ------------------------------------ MMA issuers ------------------------------------
         // One k-tile costs its issuing thread ~900 clk of mostly fixed latency (two barrier waits, fence,
-        // 8 x ~45 clk UTCHMMA issue, two commits; per-tile timeline in profiles/), far more than the MMAs
+        // eight MMAs issued at ~45 clk each, two commits), far more than the MMAs
         // themselves.  Up to four issuing warps take k-tiles round-robin, each into its OWN accumulator
-        // (summed by the epilogue), so the result stays bit-deterministic.  Warp-uniform control flow (every
-        // lane walks the barriers) with one elected lane issuing keeps the descriptors in uniform registers.
+        // (summed by the epilogue), so the result stays bit-deterministic.  Warp-uniform control flow: every
+        // lane walks the barriers, one elected lane issues.
         const int mw = (warp == 1) ? 0 : warp - (2 + TC_DEQ_WARPS) + 1;
         const uint32_t idesc = umma_idesc_f16_f32(128, NT);
         // K-major no-swizzle descriptor of B: LBO 128 B (K core matrices), SBO 2048 B (8-row groups); only the

@@ -5,9 +5,9 @@
 //      32-block as the XH activation slabs).  fp16((nibble - 8) * d), one rounding: bit-identical to what the
 //      on-the-fly dequantisers of gemm_q40_tc.cu feed the tensor core.  The engine keeps the WH copy resident when
 //      it fits (8B: 15 GB of the 180 GB) or rebuilds it per matrix into a scratch buffer.
-//   2. gemm_wh_tc_kernel is then a plain fp16 SS-mode GEMM: both operands arrive by bulk async copies (UBLKCP) of
+//   2. gemm_wh_tc_kernel is then a plain fp16 SS-mode GEMM: both operands arrive by bulk async copies of
 //      contiguous, pre-tiled 16 KB pieces; nothing is unpacked inside the loop, so the unpack -- the limiter of the
-//      fused kernel (ALU pipe 50 %, tensor pipe 14 % in profiles/ncu_tc_tmemA_w13_m32.txt), which every M tile
+//      fused kernel (ALU pipe 50 %, tensor pipe 14 % at 32 rows of w13), which every M tile
 //      repeated -- is paid once per weight instead of once per 256 activation rows.
 //
 // gemm_wh_tc_kernel<2> pairs two CTAs (cluster of 2 = one TPC) on a 256 weight rows x 256 activation rows tile with

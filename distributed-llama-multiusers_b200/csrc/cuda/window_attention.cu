@@ -371,7 +371,7 @@ __host__ __device__ __forceinline__ int wm_line_stride(int LD) {      // bf16 el
 // A decoding tile: all its stacked rows fit ONE 16-row MMA tile, so the four warps share the tokens instead of the rows.  A warp
 // takes every fourth half page (16 tokens) through two buffers of its own (DEEP; one where the launch has tall tiles, too) -- no barrier between
 // warps until the merge in shared memory; 12 warps per SM keep ~100 KB in flight while they multiply as much.  As a quarter-full row tile (one warp of four multiplying, a barrier per page) 32 rows over
-// 1000 to 2000 positions of 4 key/value heads took 58.5 us with the merge; 40.1 now.
+// 1000 to 2000 positions of 4 key/value heads took 58.5 us with the merge; 40.1 with one buffer, 37.3 with two.
 template <int DK, bool DEEP>
 __device__ __forceinline__ void window_small_tile(const DlWindowAttnArgs& a, const int* s_row, int n_rows, int tile, int g, int n_splits, int pg_lo, int pg_hi, int lo,
                                                   int p_first, int slot, __nv_bfloat16* smem, float* __restrict__ partial) {
@@ -785,39 +785,39 @@ __global__ void __launch_bounds__(128) window_merge_kernel(DlWindowAttnArgs a, c
                                                            const float* __restrict__ partial) {
     __shared__ float w_s[WM_ROWS * WM_MAX_SPLITS];
     const int tile = blockIdx.x, g = blockIdx.y, D = a.dim, rep = a.heads / a.kv_heads;
-  for (int r = blockIdx.z; r < rq; r += gridDim.z) {
-    const int m = tile_rows[(size_t)tile * rq + r];                           // not written by the kernel that this launch runs ahead of
-    if (m < 0) return;
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    __syncthreads();
-    const float* base = partial + ((size_t)tile * a.kv_heads + g) * n_splits * WM_ROWS * (D + 2);
-    if (base[(size_t)r * rep * (D + 2) + D + 1] == -2.f) return;              // written already, without shares
-    for (int hg = threadIdx.x >> 5; hg < rep; hg += blockDim.x >> 5) {        // a warp per head, a lane per share
-        const int k = threadIdx.x & 31;
-        const float* p = base + ((size_t)k * WM_ROWS + r * rep + hg) * (D + 2) + D;
-        const float mk = k < n_splits ? p[0] : -INFINITY, lk = k < n_splits ? p[1] : -1.f;
-        const float sink = a.sink ? a.sink[g * rep + hg] : 0.f, gate = a.gate ? sigmoid_f(a.gate[(size_t)m * a.ld_gate + g * rep + hg]) : 1.f;
-        const float mx = warp_max(mk), e = mk == -INFINITY ? 0.f : expf(mk - mx);
-        float l = warp_sum(lk < 0.f ? 0.f : lk * e);
-        if (a.sink) l += expf(sink - mx);
-        if (k < n_splits) w_s[hg * n_splits + k] = lk < 0.f ? -1.f : e * (gate / l);
-    }
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < rep * D; idx += blockDim.x) {
-        const int hg = idx / D, c = idx - hg * D;
-        const float* p = base + (size_t)(r * rep + hg) * (D + 2) + c;
-        float acc = 0.f;                      // sixteen shares are in flight at once; those without pages (-1) have left nothing to read
-        for (int k0 = 0; k0 < n_splits; k0 += 16) {
-            float v[16];
-#pragma unroll
-            for (int k = 0; k < 16; ++k) v[k] = k0 + k < n_splits ? p[(size_t)(k0 + k) * WM_ROWS * (D + 2)] : 0.f;
-#pragma unroll
-            for (int k = 0; k < 16; ++k)
-                if (k0 + k < n_splits && !(w_s[hg * n_splits + k0 + k] < 0.f)) acc = fmaf(w_s[hg * n_splits + k0 + k], v[k], acc);
+    for (int r = blockIdx.z; r < rq; r += gridDim.z) {
+        const int m = tile_rows[(size_t)tile * rq + r];                           // not written by the kernel that this launch runs ahead of
+        if (m < 0) return;
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        __syncthreads();
+        const float* base = partial + ((size_t)tile * a.kv_heads + g) * n_splits * WM_ROWS * (D + 2);
+        if (base[(size_t)r * rep * (D + 2) + D + 1] == -2.f) return;              // written already, without shares
+        for (int hg = threadIdx.x >> 5; hg < rep; hg += blockDim.x >> 5) {        // a warp per head, a lane per share
+            const int k = threadIdx.x & 31;
+            const float* p = base + ((size_t)k * WM_ROWS + r * rep + hg) * (D + 2) + D;
+            const float mk = k < n_splits ? p[0] : -INFINITY, lk = k < n_splits ? p[1] : -1.f;
+            const float sink = a.sink ? a.sink[g * rep + hg] : 0.f, gate = a.gate ? sigmoid_f(a.gate[(size_t)m * a.ld_gate + g * rep + hg]) : 1.f;
+            const float mx = warp_max(mk), e = mk == -INFINITY ? 0.f : expf(mk - mx);
+            float l = warp_sum(lk < 0.f ? 0.f : lk * e);
+            if (a.sink) l += expf(sink - mx);
+            if (k < n_splits) w_s[hg * n_splits + k] = lk < 0.f ? -1.f : e * (gate / l);
         }
-        a.out[(size_t)m * a.ldo + (size_t)(g * rep + hg) * D + c] = acc;
+        __syncthreads();
+        for (int idx = threadIdx.x; idx < rep * D; idx += blockDim.x) {
+            const int hg = idx / D, c = idx - hg * D;
+            const float* p = base + (size_t)(r * rep + hg) * (D + 2) + c;
+            float acc = 0.f;                      // sixteen shares are in flight at once; those without pages (-1) have left nothing to read
+            for (int k0 = 0; k0 < n_splits; k0 += 16) {
+                float v[16];
+#pragma unroll
+                for (int k = 0; k < 16; ++k) v[k] = k0 + k < n_splits ? p[(size_t)(k0 + k) * WM_ROWS * (D + 2)] : 0.f;
+#pragma unroll
+                for (int k = 0; k < 16; ++k)
+                    if (k0 + k < n_splits && !(w_s[hg * n_splits + k0 + k] < 0.f)) acc = fmaf(w_s[hg * n_splits + k0 + k], v[k], acc);
+            }
+            a.out[(size_t)m * a.ldo + (size_t)(g * rep + hg) * D + c] = acc;
+        }
     }
-  }
 }
 
 // attention_prefill_tc.cu

@@ -99,7 +99,7 @@ class F32Engine:
         self.act_gelu = h.hidden_act != HIDDEN_ACT_SILU
         self.native = self.device.type == "cuda"
         if self.native:
-            from ..ops import kernels as _K          # fails loudly if the CUDA library is missing on a GPU box
+            from ..ops import kernels as _K          # fails loudly if the CUDA library is missing on a machine with a GPU
             _K.cuda_lib()
             self._K = _K
             self._init_native()

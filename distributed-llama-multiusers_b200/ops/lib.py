@@ -1,6 +1,6 @@
 """ctypes binding of libdllama_b200_cuda.so (C ABI declared in include/dllama_b200.h).
 
-The library is built in-tree by ``build.py`` and MUST be present on a GPU box: every op fails
+The library is built in-tree by ``build.py`` and MUST be present on a machine with a GPU: every op fails
 loudly (``NativeLibraryError``) instead of silently falling back to PyTorch.
 """
 from __future__ import annotations

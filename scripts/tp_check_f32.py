@@ -26,7 +26,7 @@ def main():
     if world > 1:
         dist.barrier()
     e = F32Engine(path, rank=rank, world=world, max_rows=16, n_slots=3, max_seq_len=256)
-    assert e.native, "the f32 engine must run its CUDA kernels on a GPU box"
+    assert e.native, "the f32 engine must run its CUDA kernels on a machine with a GPU"
     ok = True
     s = e.alloc_slot()
     prompt = [1, 5, 9, 200, 33, 17, 4]

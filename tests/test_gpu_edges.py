@@ -660,7 +660,8 @@ def _window_batch(runs, heads, kv, window=0, softcap=0.0, chunk=0):
 @pytest.mark.parametrize("runs,heads,kv,opt", [([(0, 272), (0, 400)], 32, 8, {}),                       # one tile of a prompt and three of the next in a CTA
                                                ([(96, 688), (0, 17)], 32, 8, {}),                      # three and one, the second tile a step longer
                                                ([(100, 1100)], 32, 8, dict(window=1000)), ([(300, 1100)], 32, 8, dict(window=1024)),
-                                               ([(100, 1100)], 32, 8, dict(window=1024, softcap=50.0)), ([(300, 1200)], 16, 4, dict(window=256, softcap=50.0)),
+                                               ([(100, 1100)], 32, 8, dict(window=1024, softcap=50.0)), ([(300, 1100)], 32, 8, dict(window=1000, softcap=50.0)),
+                                               ([(300, 1200)], 16, 4, dict(window=256, softcap=50.0)),
                                                ([(100, 1100)], 32, 8, dict(chunk=1024)),               # the border between the tiles' first positions
                                                ([(300, 500), (0, 200), (1000, 1), (50, 1), (31, 1), (700, 3)], 32, 8, dict(window=512)),
                                                ([(7 * k, 40 + 9 * k) for k in range(12)], 64, 8, {}), ([(k, 20 + k) for k in range(40)], 32, 8, dict(window=30))])
