@@ -4,7 +4,7 @@
     python bench.py --gpus N --steps K --warmup W          (N>1: launched under torchrun)
     python bench.py --impl reference ...                   (the unmodified reference, CPU + TCP)
 
-Metric/config are the ones BASELINE.json names.  Weights: random-init `.m` of the named
+Metric and workload: single-stream decoding of Llama-3.1-8B, Q40.  Weights: random-init `.m` of the named
 architecture (no network); prompt: synthetic token ids.  `value` is timed on the device with CUDA
 events (max over ranks) around K decode steps replayed from a CUDA graph in a device-resident
 greedy loop; `e2e.value` is the same K steps through the public API with a pinned-host -> device
@@ -26,7 +26,7 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 if ROOT not in sys.path:
     sys.path.insert(0, ROOT)
 
-BASELINE_PUBLISHED = None       # BASELINE.json "published": {} -> vs_baseline is null
+BASELINE_PUBLISHED = None       # no number was published for this hardware -> vs_baseline is null
 METRIC = "Llama-3.1-8B Q40 single-stream decode tok/s"
 
 

@@ -1,7 +1,6 @@
 // CPU backend: the whole Llama forward pass on host cores, tensor-parallel over TCP.
 //
-// This is the no-GPU configuration of the framework ("root + 1 worker over localhost TCP,
-// q80 buffer, CPU (plumbing, no GPU)") and the native counterpart of the reference's CPU device, op kernels,
+// This is the no-GPU configuration of the framework (root + workers over TCP, q80 buffer) and the native counterpart of the reference's CPU device, op kernels,
 // socket layer, node synchroniser, config broadcast and weight distribution:
 //
 //   reference component                                         here

@@ -1,8 +1,7 @@
 """B2 baseline: the same model run the "library" way -- NCCL all-reduce + Q40 dequantisation +
 cuBLAS matmuls (torch.matmul) + PyTorch elementwise ops.
 
-This is the in-repo baseline BASELINE.json asks the fused kernels to beat ("a path that only calls
-NCCL is the baseline, not the product").  It shares the weight slicing and the Q40T images with
+This is what the fused kernels have to beat: a path that only calls NCCL.  It shares the weight slicing and the Q40T images with
 ``LlamaEngine`` (so both arms stream the same bytes) but:
 
 * every matmul first dequantises its Q40T weight to bf16 (``dl_q40t_dequant`` + cast) and then

@@ -1,7 +1,6 @@
 """CPU engine with the same interface as ``LlamaEngine`` (slots, batched rows with per-row
 positions), built on the PyTorch oracle.  It is what lets the scheduler / batch engine / HTTP API /
-CLI run and be tested on a machine without a GPU, and it is the "plumbing, no GPU" configuration of
-BASELINE.json.  Slow by design; numerics are the reference's (see models/oracle.py).
+CLI run and be tested on a machine without a GPU, and it is the plumbing without a GPU.  Slow by design; numerics are the reference's (see models/oracle.py).
 """
 from __future__ import annotations
 

@@ -3,8 +3,7 @@
 f32 path), and tensor parallelism across ``dllama worker`` processes over TCP.  Workers get their configuration
 and weight slices from the root; they need no model file (reference: README.md:50, src/nn/nn-network.cpp:617-901).
 
-It is what runs when there is no GPU (BASELINE.json's "root + 1 worker over localhost TCP, q80 buffer, CPU"
-configuration).  ``CpuEngine`` (models/cpu_engine.py, pure PyTorch) stays as the numerics oracle.
+It is what runs when there is no GPU (root + 1 worker over localhost TCP, q80 buffer, for instance).  ``CpuEngine`` (models/cpu_engine.py, pure PyTorch) stays as the numerics oracle.
 """
 from __future__ import annotations
 

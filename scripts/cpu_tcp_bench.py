@@ -1,5 +1,5 @@
 #!/usr/bin/env python3
-"""BASELINE.json configuration 1 on a machine without a GPU: Llama-3.2-1B-shaped Q40 random-init `.m`, root +
+"""Tensor parallelism over TCP on a machine without a GPU: Llama-3.2-1B-shaped Q40 random-init `.m`, root +
 (N-1) workers over localhost TCP, q80 buffer, CPU.  Runs this repo's native host backend (`dllama inference` +
 `dllama worker`, separate processes) and the unmodified reference (its own build, same files, same prompt, same
 thread count per node) and prints one JSON line per arm: single-stream decode tok/s from each program's own

@@ -1,5 +1,5 @@
 #!/usr/bin/env python3
-"""HTTP-level load test of `dllama-api` (BASELINE.json config 3): U concurrent users POST streaming
+"""HTTP-level load test of `dllama-api`: U concurrent users POST streaming
 chat completions at a server running in this process (engine thread + threaded HTTP front end);
 reports aggregate generated tok/s over the wall-clock window and the p50 / p95 time to the first
 streamed token as each client sees it.

@@ -126,7 +126,7 @@ def test_dllama_api_executable_serves_http(tiny_model_path, tok_path, backend):
 
 
 def test_root_plus_worker_over_localhost_tcp_on_cpu(tiny_model_path, tok_path):
-    """BASELINE.json configuration 1 (plumbing, no GPU): `dllama worker --port P` + `dllama inference --workers
+    """The plumbing without a GPU: `dllama worker --port P` + `dllama inference --workers
     127.0.0.1:P` as separate processes, q80 buffer; the worker has no model file; the text equals the single-node run."""
     import socket
     import subprocess
