@@ -251,6 +251,141 @@ DL_DEVINL void epilogue_rows(const DlEpilogue& e, const float* out_s, int out_ld
     }
 }
 
+// The same by whole warps that share a tile, four and more consecutive output rows per thread: `warp` of `nw` takes activation rows
+// (SiLU: blocks of 8 rows) in turn, ld(m, r) gives the products r .. r + 3 of activation row m (r a multiple of 4).  Nothing is exchanged
+// between warps, so the caller needs no barrier but the one that makes ld's source complete.  after() is called once by every thread, behind its last ld.
+// U: activation rows in flight per thread.
+//
+// What bounds it: instructions and the latency of each row's chain.  One value per thread and activation row at a time, half the threads idle
+// on paired rows, five shuffles per block and 2-byte image stores (epilogue_rows), the epilogue of a 256 x 256 tile of gate|up took longer than its
+// MMAs (4096 x 14336, 2048 rows: 447 us; without any epilogue work 360); here a block of 32 hidden values is four threads, whose image chunk
+// is one 16-byte store, eight rows of them one line.
+template <int U, class Ld, class After>
+DL_DEVINL void epilogue_vec(const DlEpilogue& e, const Ld& ld, int grow0, int d_real, int M, int m0, int warp, int nw, const After& after) {
+    const int lane = threadIdx.x & 31;
+    if (e.kind == DL_EPI_SILU_MUL) {
+        const int w = lane & 3, ml = lane >> 2, n_task = ((M + 7) >> 3) * 2;
+        const bool gelu = e.act_gelu != 0;
+        const int mcap = e.out_mcap;
+        if (warp >= n_task) after();
+        for (int t = warp; t < n_task; t += nw) {
+            const int blk = t & 1, m = (t >> 1) * 8 + ml, mr = min(m, M - 1);
+            // chunk w of the block's image: hidden values 4 w .. 4 w + 3 and 4 w + 16 .. 4 w + 19 (xh_slot)
+            float4 x[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) x[i] = ld(mr, blk * 64 + (i >> 1) * 32 + 8 * w + (i & 1) * 4);
+            if (t + nw >= n_task) after();
+            float h[8], amax = 0.0f;
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                h[2 * i] = (gelu ? act_gelu(x[i].x) : act_silu(x[i].x)) * x[i].y;
+                h[2 * i + 1] = (gelu ? act_gelu(x[i].z) : act_silu(x[i].z)) * x[i].w;
+                amax = fmaxf(amax, fmaxf(fabsf(h[2 * i]), fabsf(h[2 * i + 1])));
+            }
+            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+            const float d = amax / 127.0f, id = (d != 0.0f) ? (1.0f / d) : 0.0f;
+            const float df = fminf(__half2float(__float2half_rn(d)), 515.0f);      // saturation: q80_block_store
+            __align__(16) __half o[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) o[(i & 4) + ((i & 3) == 1 ? 2 : (i & 3) == 2 ? 1 : (i & 3))] = __float2half_rn((float)__float2int_rn(h[i] * id) * df);
+            if (m < M && grow0 + blk * 64 < d_real) {
+                const int kblock = (grow0 >> 6) + blk;
+                *reinterpret_cast<uint4*>(e.xh_out + ((size_t)(kblock >> 2) * (size_t)(mcap >> 3) + (size_t)((m0 + m) >> 3)) * XH_ROWGROUP_BYTES +
+                                          ((kblock & 3) * 4 + w) * 128 + ((m0 + m) & 7) * 16) = *reinterpret_cast<const uint4*>(o);
+            }
+        }
+        return;
+    }
+    const int r = lane * 4, grow = grow0 + r;
+    const bool live = grow < d_real;                  // d_real is a multiple of 4
+    if (warp >= M) after();
+    if (e.kind == DL_EPI_STORE) {
+        const bool rt = e.q80_roundtrip != 0;
+        const float* res = e.residual;
+        float* d0 = e.dst[0] + e.dst_off;
+        for (int mb = warp; mb < M; mb += U * nw) {
+            float4 v[U], x[U];
+#pragma unroll
+            for (int i = 0; i < U; i++)
+                if (res != nullptr && live && mb + i * nw < M) x[i] = *reinterpret_cast<const float4*>(res + (size_t)(m0 + mb + i * nw) * e.residual_ld + grow);
+#pragma unroll
+            for (int i = 0; i < U; i++) v[i] = ld(min(mb + i * nw, M - 1), r);
+            if (mb + U * nw >= M) after();
+#pragma unroll
+            for (int i = 0; i < U; i++) {
+                if (rt) {                             // eight threads hold a block
+                    float amax = fmaxf(fmaxf(fabsf(v[i].x), fabsf(v[i].y)), fmaxf(fabsf(v[i].z), fabsf(v[i].w)));
+                    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+                    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+                    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
+                    const float d = amax / 127.0f, id = (d != 0.0f) ? (1.0f / d) : 0.0f, df = __half2float(__float2half_rn(d));
+                    v[i].x = (float)__float2int_rn(v[i].x * id) * df; v[i].y = (float)__float2int_rn(v[i].y * id) * df;
+                    v[i].z = (float)__float2int_rn(v[i].z * id) * df; v[i].w = (float)__float2int_rn(v[i].w * id) * df;
+                }
+                if (live && mb + i * nw < M) {
+                    if (res != nullptr) { v[i].x += x[i].x; v[i].y += x[i].y; v[i].z += x[i].z; v[i].w += x[i].w; }
+                    *reinterpret_cast<float4*>(d0 + (size_t)(m0 + mb + i * nw) * e.ld + grow) = v[i];
+                }
+            }
+        }
+    } else {                                          // DL_EPI_QKV_ROPE: two rotated pairs per thread
+        const int region = (grow < e.q_dim) ? 0 : ((grow < e.q_dim + e.kv_dim) ? 1 : 2);
+        const int rrow = (region == 0) ? grow : ((region == 1) ? grow - e.q_dim : grow - e.q_dim - e.kv_dim);
+        const int hd = rrow % e.head_size, kvh = rrow / e.head_size;
+        float2 freq = make_float2(0.0f, 0.0f);
+        if (region < 2 && live) freq = make_float2(e.rope_freqs[hd >> 1], e.rope_freqs[(hd >> 1) + 1]);
+        // lane i: position and page of this warp's i-th row
+        int my_pos = 0, my_page = 0;
+        if (warp + lane * nw < M) {
+            my_pos = e.pos[m0 + warp + lane * nw];
+            if (grow0 + 128 > e.q_dim) my_page = e.block_table[(size_t)e.slot[m0 + warp + lane * nw] * e.max_pages + my_pos / e.page_size];
+        }
+        void* base = (region == 1) ? e.k_cache : e.v_cache;
+        for (int m = warp, i = 0; m < M; m += nw, i++) {
+            float4 v = ld(m, r);
+            if (m + nw >= M) after();
+            const int p = __shfl_sync(0xffffffffu, my_pos, i), page = __shfl_sync(0xffffffffu, my_page, i);
+            if (region < 2) {
+                float sn, cs;
+                sincosf((float)p * freq.x, &sn, &cs);
+                v = make_float4(v.x * cs - v.y * sn, v.x * sn + v.y * cs, v.z, v.w);
+                sincosf((float)p * freq.y, &sn, &cs);
+                v = make_float4(v.x, v.y, v.z * cs - v.w * sn, v.z * sn + v.w * cs);
+            }
+            if (!live) continue;
+            if (region == 0) {
+                *reinterpret_cast<float4*>(e.q_out + (size_t)(m0 + m) * e.q_dim + rrow) = v;
+            } else {
+                const size_t off = (((size_t)page * e.n_kv_heads + kvh) * e.page_size + (p % e.page_size)) * e.head_size + hd;
+                if (e.kv_f32) {
+                    *reinterpret_cast<float4*>(reinterpret_cast<float*>(base) + off) = v;
+                } else {
+                    __half2 lo = __floats2half2_rn(v.x, v.y), hi = __floats2half2_rn(v.z, v.w);
+                    *reinterpret_cast<uint2*>(reinterpret_cast<__half*>(base) + off) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+                }
+            }
+        }
+    }
+}
+// a tile in shared memory, [m][ld]
+struct EpiTile {
+    const float* s;
+    int ld;
+    DL_DEVINL float4 operator()(int m, int r) const { return *reinterpret_cast<const float4*>(s + (size_t)m * ld + r); }
+};
+#define EPI_TILE_LD 132               // row stride of such a tile: 16-byte reads of two rows and four blocks of 8 (SiLU) without bank conflicts
+
+// Does epilogue_vec take this epilogue?  One destination (what goes to peers keeps one word per thread: neighbouring words leave together),
+// whole groups of four rows, 16-byte addresses; an fp16 image alone.
+static inline bool epilogue_vec_ok(const DlEpilogue& e, int d) {
+    const auto al = [](const void* p, long long ld) { return ((uintptr_t)p & 15) == 0 && ld % 4 == 0; };
+    if (e.kind == DL_EPI_SILU_MUL) return e.xh_out != nullptr && e.xq_out == nullptr && ((uintptr_t)e.xh_out & 15) == 0 && d % 64 == 0;
+    if (d % 4 != 0) return false;
+    if (e.kind == DL_EPI_STORE) return e.n_dst == 1 && e.ll == 0 && al(e.dst[0], e.ld) && e.dst_off % 4 == 0 && (e.residual == nullptr || al(e.residual, e.residual_ld));
+    return e.kind == DL_EPI_QKV_ROPE && al(e.q_out, e.q_dim) && al(e.k_cache, e.kv_dim) && al(e.v_cache, e.head_size);
+}
+
 // epilogue_complete: called by ALL threads of every CTA that ran epilogue_rows (uses __syncthreads).
 // DL_EPI_STORE with flags: every CTA fences its (peer) stores, the last one releases the flags.
 DL_DEVINL void epilogue_complete(const DlEpilogue& e, int tid, int n_epi_ctas, int* smem_flag) {

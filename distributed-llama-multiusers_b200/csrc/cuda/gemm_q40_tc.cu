@@ -45,6 +45,7 @@ struct TcArgs {
     int nacc;              // MMA-issuing warps = independent TMEM accumulators (1, 2 or 4; nacc*NT <= 256), summed by the epilogue
     int LA, LB;            // issuing lanes per ring; each divides its stage count so a stage has ONE owner lane
     int n_epi_ctas;
+    int vec;               // epilogue_vec takes the epilogue
     unsigned long long* tr;
     int dbg_mode;          // debug timing experiments (results invalid): 1 = one MMA per k-tile, 2 = no dequant/STTM
     long long* dbg;        // debug: per-tile clock64 stamps of CTA 0 (dl_debug_set_tc_trace), [tile][8]
@@ -308,8 +309,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_q40_tc_kernel(const __grid
         if (tid == 64) TC_DBG(2, 63);
     }
     const int n_chunks = (Mt + TC_EPI_CHUNK - 1) / TC_EPI_CHUNK;
-    // columns [8 eg, 8 eg + 8) of chunk ch of row tile rt + h -> dst[column][128] (with one row tile: the sum over the accumulators)
-    auto drain = [&](int h, int ch, float* dst) {
+    // columns [8 eg, 8 eg + 8) of chunk ch of row tile rt + h -> dst[column][ld] (with one row tile: the sum over the accumulators)
+    auto drain = [&](int h, int ch, float* dst, int ld) {
         const uint32_t taddr = tmem_base + ((uint32_t)(eq * 32) << 16) + (uint32_t)(h * NT + ch * TC_EPI_CHUNK);
         const int ncol = min(TC_EPI_CHUNK, NT - ch * TC_EPI_CHUNK);
         const int c0 = eg * 8;
@@ -327,17 +328,17 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_q40_tc_kernel(const __grid
                 for (int j = 0; j < 8; j++) f[j] += __uint_as_float(v[j]);
             }
 #pragma unroll
-            for (int j = 0; j < 8; j++) dst[(c0 + j) * 128 + etid] = f[j];
+            for (int j = 0; j < 8; j++) dst[(c0 + j) * ld + etid] = f[j];
         }
     };
     if (S > 1) {
         // split-K (of a single row tile: pairs are for more row tiles than SMs): every rank publishes its partial tile in the rings' place, then
         // sums and finishes ITS share of the activation rows over DSMEM, in rank order.  (One rank finishing all rows chunk by chunk took two
         // cluster barriers and S - 1 remote reads of 16 KB per 32 rows.)
-        float* all_s = reinterpret_cast<float*>(smem);               // [NT][128]
+        float* all_s = reinterpret_cast<float*>(smem);               // [NT][EPI_TILE_LD]
         cg::cluster_group cluster = cg::this_cluster();
         if (is_epi)
-            for (int ch = 0; ch < n_chunks; ch++) drain(0, ch, all_s + (size_t)ch * TC_EPI_CHUNK * 128);
+            for (int ch = 0; ch < n_chunks; ch++) drain(0, ch, all_s + (size_t)ch * TC_EPI_CHUNK * EPI_TILE_LD, EPI_TILE_LD);
         tc_fence_before();
         cluster.sync();
         // a rank tells its peers that it has read their shares as soon as it has, ahead of its own epilogue: the barrier at the end then
@@ -347,39 +348,54 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_q40_tc_kernel(const __grid
         if (!is_epi || ms >= me) read_all();
         if (is_epi) {
             pdl_wait();
-            for (int mb = ms; mb < me; mb += TC_EPI_CHUNK) {
-                const int mc = min(TC_EPI_CHUNK, me - mb);
-                for (int idx = tid - 64; idx < mc * 32; idx += TC_DEQ_WARPS * 32) {
-                    float4 x[8];                            // S <= 8: the ranks' shares in flight together, summed in rank order
+            // values r .. r + 3 of activation row m: S <= 8, the ranks' shares in flight together, summed in rank order
+            auto sum_of = [&](int m, int r) {
+                float4 x[8];
 #pragma unroll
-                    for (int c = 0; c < 8; c++)
-                        if (c < S) x[c] = *reinterpret_cast<const float4*>(cluster.map_shared_rank(all_s, c) + (size_t)mb * 128 + idx * 4);
-                    float4 v = x[0];
+                for (int c = 0; c < 8; c++)
+                    if (c < S) x[c] = *reinterpret_cast<const float4*>(cluster.map_shared_rank(all_s, c) + (size_t)m * EPI_TILE_LD + r);
+                float4 v = x[0];
 #pragma unroll
-                    for (int c = 1; c < 8; c++)
-                        if (c < S) { v.x += x[c].x; v.y += x[c].y; v.z += x[c].z; v.w += x[c].w; }
-                    reinterpret_cast<float4*>(out_s)[idx] = v;
+                for (int c = 1; c < 8; c++)
+                    if (c < S) { v.x += x[c].x; v.y += x[c].y; v.z += x[c].z; v.w += x[c].w; }
+                return v;
+            };
+            if (a.vec) {
+                if (ms < me) epilogue_vec<1>(a.epi, [&](int m, int r) { return sum_of(ms + m, r); }, rt * 128, a.d_real, me - ms, m0 + ms, warp - 2, TC_DEQ_WARPS, read_all);
+            } else {
+                for (int mb = ms; mb < me; mb += TC_EPI_CHUNK) {
+                    const int mc = min(TC_EPI_CHUNK, me - mb);
+                    for (int idx = tid - 64; idx < mc * 32; idx += TC_DEQ_WARPS * 32)
+                        reinterpret_cast<float4*>(out_s)[idx] = sum_of(mb + (idx >> 5), (idx & 31) * 4);
+                    asm volatile("bar.sync 1, 512;" ::: "memory");
+                    if (mb + TC_EPI_CHUNK >= me) read_all();
+                    epilogue_rows(a.epi, out_s, 128, 128, rt * 128, a.d_real, mc, m0 + mb, etid, eg, TC_GROUPS);
+                    asm volatile("bar.sync 1, 512;" ::: "memory");      // out_s is rewritten by the next round
                 }
-                asm volatile("bar.sync 1, 512;" ::: "memory");
-                if (mb + TC_EPI_CHUNK >= me) read_all();
-                epilogue_rows(a.epi, out_s, 128, 128, rt * 128, a.d_real, mc, m0 + mb, etid, eg, TC_GROUPS);
-                asm volatile("bar.sync 1, 512;" ::: "memory");      // out_s is rewritten by the next round
             }
         }
         asm volatile("barrier.cluster.wait.acquire;" ::: "memory");     // nobody leaves while a peer may still read its share
+    } else if (is_epi && a.vec) {
+        // every MMA is done, so the rings are free: the whole of both tiles is drained there at once
+        float* all_s = reinterpret_cast<float*>(smem);               // [P][NT][EPI_TILE_LD]
+        for (int h = 0; h < P; h++)
+            for (int ch = 0; ch < n_chunks; ch++) drain(h, ch, all_s + (size_t)(h * NT + ch * TC_EPI_CHUNK) * EPI_TILE_LD, EPI_TILE_LD);
+        if (tid == 64) TC_DBG(4, 63);
+        asm volatile("bar.sync 1, 512;" ::: "memory");
+        pdl_wait();
+        if (tid == 64) TC_DBG(5, 63);
+        for (int h = 0; h < P; h++)
+            epilogue_vec<2>(a.epi, EpiTile{all_s + (size_t)h * NT * EPI_TILE_LD, EPI_TILE_LD}, (rt + h) * 128, a.d_real, Mt, m0, warp - 2, TC_DEQ_WARPS, [] {});
+        if (tid == 64) TC_DBG(6, 63);
     } else if (is_epi) {
         for (int h = 0; h < P; h++)
             for (int ch = 0; ch < n_chunks; ch++) {
                 const int mc = min(TC_EPI_CHUNK, Mt - ch * TC_EPI_CHUNK);
-                drain(h, ch, out_s);
-                if (tid == 64 && ch == 0) TC_DBG(4, 63);
+                drain(h, ch, out_s, 128);
                 asm volatile("bar.sync 1, 512;" ::: "memory");
                 pdl_wait();
-                if (tid == 64 && ch == 0) TC_DBG(5, 63);
                 epilogue_rows(a.epi, out_s, 128, 128, (rt + h) * 128, a.d_real, mc, m0 + ch * TC_EPI_CHUNK, etid, eg, TC_GROUPS);
-                if (tid == 64 && ch == 0) TC_DBG(6, 63);
                 asm volatile("bar.sync 1, 512;" ::: "memory");
-                if (tid == 64 && ch == 0) TC_DBG(7, 63);
             }
     }
     tc_fence_before();
@@ -447,6 +463,7 @@ extern "C" int dl_gemm_q40_tc(const uint8_t* w_q40t, int d, int n, const uint8_t
     const int cta_rows = row_tiles / (a.pair ? 2 : 1);
     a.n_epi_ctas = cta_rows * a.S * ((M + a.NT - 1) / a.NT);
     a.epi = *epi;
+    a.vec = epilogue_vec_ok(*epi, d);
     a.tr = dl_trace_next(TR_TC);
     a.dbg = g_tc_dbg;
     a.dbg_mode = g_tc_dbg_mode;

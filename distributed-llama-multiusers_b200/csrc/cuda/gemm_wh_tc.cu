@@ -31,7 +31,8 @@
 #define WH_TILE_BYTES 32768
 #define WT_NT 256                      // activation rows per tile
 #define WT_THREADS 576
-#define WT_EPI_CHUNK 32
+#define WT_EPI_CHUNK 32                // activation rows per epilogue pass, one row per warp quarter
+#define WT_VEC_CHUNK 64                // the same by whole warps (epilogue_vec): four rows per warp
 
 struct WhArgs {
     const uint8_t* wh;                 // [row_tiles][KT][32 KB]
@@ -42,6 +43,7 @@ struct WhArgs {
     int pf_dist, pf_mask;              // weight tiles are pulled into L2 pf_dist k-steps ahead by the CTAs whose activation tile index & pf_mask == 0
     int dbg;                           // timing experiments (results invalid): 1 = no epilogue work, 2 = no MMAs, 4 = no activation copies
     int bf16;                          // both operand images hold bf16 instead of fp16 (dense-weight models)
+    int vec;                           // epilogue_vec takes the epilogue
     // grouped mode (routed experts): n_groups weight images wh_group_bytes apart; group g multiplies the activation rows
     // [grp[2g], grp[2g] + grp[2g+1]) (device memory; first rows are multiples of 8) and writes those output rows.  The
     // tile list covers m_tiles activation tiles per group; tiles beyond a group's rows are skipped by every role alike.
@@ -139,8 +141,8 @@ __global__ void __launch_bounds__(WT_THREADS, 1) gemm_wh_tc_kernel(const __grid_
     constexpr int STAGE = WH_TILE_BYTES + B_ROWS * 256;   // 96 KB / 64 KB
     trace_begin(a.tr);
     const unsigned long long t0 = globaltimer_ns();
-    float* out_s = reinterpret_cast<float*>(smem + NS * STAGE);          // [32][128]
-    uint64_t* bars = reinterpret_cast<uint64_t*>(out_s + WT_EPI_CHUNK * 128);
+    float* out_s = reinterpret_cast<float*>(smem + NS * STAGE);          // [32][128], or [WT_VEC_CHUNK][EPI_TILE_LD]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(out_s + WT_VEC_CHUNK * EPI_TILE_LD);
     uint64_t* full = bars;               // [NS]  this CTA's copies of a stage have landed
     uint64_t* peer_full = bars + 4;      // [NS]  (leader of a pair) the other CTA's copies have landed
     uint64_t* empty = bars + 8;          // [NS]  the MMAs reading the stage have retired (both CTAs)
@@ -298,23 +300,47 @@ __global__ void __launch_bounds__(WT_THREADS, 1) gemm_wh_tc_kernel(const __grid_
             wt_wait(&acc_full[u], (tcount >> 1) & 1, t0);
             tc_fence_after();
             if (first) { pdl_wait(); first = false; }
+            const uint32_t tq = tmem_base + ((uint32_t)(eq * 32) << 16) + u * WT_NT;
+            auto drained = [&] {      // every warp has read its last columns: the accumulator is free
+                if (tid != 64) return;
+                if (CG == 2 && crank != 0) mbar_arrive_remote(leader_ae + u * 8);
+                else mbar_arrive(&acc_empty[u]);
+            };
+            if (a.vec) {
+                const int n_chunks = (Mt + WT_VEC_CHUNK - 1) / WT_VEC_CHUNK;
+                for (int ch = 0; ch < n_chunks; ch++) {
+                    uint32_t v[2][8];
+#pragma unroll
+                    for (int h = 0; h < 2; h++) tmem_ld_32x32b_x8(tq + (uint32_t)(ch * WT_VEC_CHUNK + eg * 16 + h * 8), v[h]);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int h = 0; h < 2; h++)
+#pragma unroll
+                        for (int j = 0; j < 8; j++) out_s[(eg * 16 + h * 8 + j) * EPI_TILE_LD + etid] = __uint_as_float(v[h][j]);
+                    tc_fence_before();
+                    asm volatile("bar.sync 1, 512;" ::: "memory");
+                    if (ch == n_chunks - 1) drained();
+                    if (!(a.dbg & 1))
+                        epilogue_vec<2>(a.epi, EpiTile{out_s, EPI_TILE_LD}, rt * 128, a.d_real, min(WT_VEC_CHUNK, Mt - ch * WT_VEC_CHUNK),
+                                        w.row0 + m0 + ch * WT_VEC_CHUNK, warp - 2, 16, [] {});
+                    asm volatile("bar.sync 1, 512;" ::: "memory");
+                }
+                tcount++;
+                continue;
+            }
             const int n_chunks = (Mt + WT_EPI_CHUNK - 1) / WT_EPI_CHUNK;
             for (int ch = 0; ch < n_chunks; ch++) {
                 const int mc = min(WT_EPI_CHUNK, Mt - ch * WT_EPI_CHUNK);
-                const uint32_t taddr = tmem_base + ((uint32_t)(eq * 32) << 16) + u * WT_NT + (uint32_t)(ch * WT_EPI_CHUNK) + eg * 8;
                 uint32_t v[8];
-                tmem_ld_32x32b_x8(taddr, v);
+                tmem_ld_32x32b_x8(tq + (uint32_t)(ch * WT_EPI_CHUNK) + eg * 8, v);
                 tmem_ld_wait();
 #pragma unroll
                 for (int j = 0; j < 8; j++) out_s[(eg * 8 + j) * 128 + etid] = __uint_as_float(v[j]);
                 tc_fence_before();
-                asm volatile("bar.sync 1, 512;");
-                if (ch == n_chunks - 1 && tid == 64) {      // every warp has read its last columns: the accumulator is free
-                    if (CG == 2 && crank != 0) mbar_arrive_remote(leader_ae + u * 8);
-                    else mbar_arrive(&acc_empty[u]);
-                }
+                asm volatile("bar.sync 1, 512;" ::: "memory");
+                if (ch == n_chunks - 1) drained();
                 if (!(a.dbg & 1)) epilogue_rows(a.epi, out_s, 128, 128, rt * 128, a.d_real, mc, w.row0 + m0 + ch * WT_EPI_CHUNK, etid, eg, 4);
-                asm volatile("bar.sync 1, 512;");
+                asm volatile("bar.sync 1, 512;" ::: "memory");
             }
             tcount++;
         }
@@ -618,12 +644,13 @@ static int gemm_wh_launch(const uint8_t* wh, int d, int n, const uint8_t* xh, in
     if (grid > a.n_tiles * cg) grid = a.n_tiles * cg;
     a.n_epi_ctas = grid;
     a.epi = *epi;
+    a.vec = epilogue_vec_ok(*epi, d);
     a.dbg = g_wh_dbg;
     a.pf_dist = g_wh_pf_dist < a.KT ? g_wh_pf_dist : 0;
     a.pf_mask = g_wh_pf_mask;
     a.piece = g_wh_piece;
     a.tr = dl_trace_next(TR_TC);
-    const size_t smem = 196608 + WT_EPI_CHUNK * 128 * 4 + 16 * 8 + 16;
+    const size_t smem = 196608 + WT_VEC_CHUNK * EPI_TILE_LD * 4 + 16 * 8 + 16;
     static bool attr_set = false;
     if (!attr_set) {
         cudaError_t e1 = cudaFuncSetAttribute(gemm_wh_tc_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
