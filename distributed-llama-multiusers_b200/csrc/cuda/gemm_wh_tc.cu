@@ -40,7 +40,6 @@ struct WhArgs {
     int d_real, row_tiles, KT, ncap, M, m_tiles, n_tiles;
     int n_epi_ctas;
     int piece;                         // bytes per bulk copy (4096 / 8192 / 16384)
-    int pf_dist, pf_mask;              // weight tiles are pulled into L2 pf_dist k-steps ahead by the CTAs whose activation tile index & pf_mask == 0
     int dbg;                           // timing experiments (results invalid): 1 = no epilogue work, 2 = no MMAs, 4 = no activation copies
     int bf16;                          // both operand images hold bf16 instead of fp16 (dense-weight models)
     int vec;                           // epilogue_vec takes the epilogue
@@ -181,50 +180,40 @@ __global__ void __launch_bounds__(WT_THREADS, 1) gemm_wh_tc_kernel(const __grid_
         // ------------------------------------ producer ------------------------------------
         // the stage is fetched as `piece`-byte bulk copies, one per lane: first the weight tile, then row groups of the
         // activation slab (many requests in flight: one bulk copy streams at only ~16 B/clk)
+        // the whole warp walks the stages together (28672 x 4096 at 2048 rows 359 us, 367 with lanes that wait and issue one by one)
         const int piece = a.piece, npiece = STAGE / piece, na = WH_TILE_BYTES / piece, prow = piece / 256;
-        if (lane < npiece) {
-            pdl_wait();
-            const size_t x_kt_stride = (size_t)(a.ncap >> 3) * XH_ROWGROUP_BYTES;
-            uint32_t it = 0;
-            for (int t = cid; t < a.n_tiles; t += ncl) {
-                WtTile w;
-                if (!wt_tile(a, t, w)) continue;
-                const int rp = w.rp, mt = w.mt;
-                const int rt = rp * CG + (int)crank;
-                const int mrow0 = w.row0 + mt * WT_NT + (int)crank * B_ROWS;
-                const int row_cap = a.grp ? w.row0 + ((w.rows + 7) & ~7) : a.ncap;      // slabs hold 8 rows
-                const int b_rows = max(0, min(B_ROWS, row_cap - mrow0));
-                const uint8_t* src;
-                size_t stride;
-                uint32_t bytes;
-                if (lane < na) {
-                    src = a.wh + (size_t)w.g * (size_t)a.wh_group_bytes + (size_t)rt * KT * WH_TILE_BYTES + lane * piece;
-                    stride = WH_TILE_BYTES;
-                    bytes = piece;
-                } else {
-                    const int r0 = (lane - na) * prow;
-                    src = a.xh + (size_t)((mrow0 + r0) >> 3) * XH_ROWGROUP_BYTES;
-                    stride = x_kt_stride;
-                    bytes = (a.dbg & 4) ? 0u : (uint32_t)max(0, min(prow, b_rows - r0)) * 256u;
-                }
-                const uint32_t total = WH_TILE_BYTES + ((a.dbg & 4) ? 0u : (uint32_t)b_rows * 256u);
-                const bool pf = lane < na && a.pf_dist > 0 && (mt & a.pf_mask) == 0 && a.n_groups == 1;
-                for (int kt = 0; kt < KT; kt++, it++) {
-                    if (pf) {      // optional: pull the weight tile pf_dist k-steps ahead into L2 (measured: no gain, off by default)
-                        int j = kt + a.pf_dist, tt = t;
-                        while (j >= KT) { j -= KT; tt += ncl; }
-                        if (tt < a.n_tiles) {
-                            const int rt2 = (tt / a.m_tiles) * CG + (int)crank;
-                            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a.wh + ((size_t)rt2 * KT + j) * WH_TILE_BYTES + lane * piece),
-                                         "r"(piece)
-                                         : "memory");
-                        }
-                    }
-                    const uint32_t s = it % NS;
-                    if (it >= NS) wt_wait(&empty[s], ((it / NS) & 1) ^ 1, t0);
-                    if (lane == 0) mbar_arrive_expect_tx(&full[s], total);
-                    if (bytes) bulk_g2s(smem + s * STAGE + lane * piece, src + (size_t)kt * stride, bytes, &full[s]);
-                }
+        pdl_wait();
+        const size_t x_kt_stride = (size_t)(a.ncap >> 3) * XH_ROWGROUP_BYTES;
+        uint32_t it = 0;
+        for (int t = cid; t < a.n_tiles; t += ncl) {
+            WtTile w;
+            if (!wt_tile(a, t, w)) continue;
+            const int rp = w.rp, mt = w.mt;
+            const int rt = rp * CG + (int)crank;
+            const int mrow0 = w.row0 + mt * WT_NT + (int)crank * B_ROWS;
+            const int row_cap = a.grp ? w.row0 + ((w.rows + 7) & ~7) : a.ncap;      // slabs hold 8 rows
+            const int b_rows = max(0, min(B_ROWS, row_cap - mrow0));
+            const uint8_t* src = nullptr;
+            size_t stride = 0;
+            uint32_t bytes = 0;
+            if (lane < na) {
+                src = a.wh + (size_t)w.g * (size_t)a.wh_group_bytes + (size_t)rt * KT * WH_TILE_BYTES + lane * piece;
+                stride = WH_TILE_BYTES;
+                bytes = piece;
+            } else if (lane < npiece) {
+                const int r0 = (lane - na) * prow;
+                src = a.xh + (size_t)((mrow0 + r0) >> 3) * XH_ROWGROUP_BYTES;
+                stride = x_kt_stride;
+                bytes = (a.dbg & 4) ? 0u : (uint32_t)max(0, min(prow, b_rows - r0)) * 256u;
+            }
+            const uint32_t total = WH_TILE_BYTES + ((a.dbg & 4) ? 0u : (uint32_t)b_rows * 256u);
+            for (int kt = 0; kt < KT; kt++, it++) {
+                const uint32_t s = it % NS;
+                if (it >= NS) wt_wait(&empty[s], ((it / NS) & 1) ^ 1, t0);
+                __syncwarp();
+                if (lane == 0) mbar_arrive_expect_tx(&full[s], total);
+                if (bytes) bulk_g2s(smem + s * STAGE + lane * piece, src + (size_t)kt * stride, bytes, &full[s]);
+                __syncwarp();
             }
         }
     } else if (warp == 1) {
@@ -267,7 +256,9 @@ __global__ void __launch_bounds__(WT_THREADS, 1) gemm_wh_tc_kernel(const __grid_
                 tcount++;
             }
         } else {
-            // second CTA of a pair: tell the leader when this CTA's half of a stage has landed
+            // second CTA of a pair: tell the leader when this CTA's half of a stage has landed.  What the leader's MMAs read here was written here, by
+            // this SM's copies, which are complete: the arrive carries their order and no data of its own, so its release stays in this CTA.  One at
+            // cluster scope is a memory barrier of ~1.4 us in every stage's round trip (28672 x 4096 at 2048 rows 353 us, 4096 x 14336 205; 313 and 175 so).
             const uint32_t leader_pf = mapa_shared(smem_u32(peer_full), 0);
             uint32_t it = 0;
             for (int t = cid; t < a.n_tiles; t += ncl) {
@@ -276,7 +267,7 @@ __global__ void __launch_bounds__(WT_THREADS, 1) gemm_wh_tc_kernel(const __grid_
                 for (int kt = 0; kt < KT; kt++, it++) {
                     const uint32_t s = it % NS;
                     wt_wait(&full[s], (it / NS) & 1, t0);
-                    if (lane == 0) mbar_arrive_remote(leader_pf + s * 8);
+                    if (lane == 0) asm volatile("mbarrier.arrive.release.cta.shared::cluster.b64 _, [%0];" ::"r"(leader_pf + s * 8) : "memory");
                     __syncwarp();
                 }
             }
@@ -604,10 +595,9 @@ static int gemm_wh_rows_launch(const uint8_t* wh, int d, int n, const uint8_t* x
     return 0;
 }
 
-static int g_wh_dbg = 0, g_wh_pf_dist = 0, g_wh_pf_mask = 0, g_wh_piece = 16384;      // bytes per bulk copy: 16 KB pieces (4 / 8 KB measured: no gain)
+static int g_wh_dbg = 0, g_wh_piece = 16384;      // bytes per bulk copy: 16 KB pieces (4 / 8 KB measured: no gain)
 extern "C" void dl_debug_set_wh_piece(int b) { if (b == 4096 || b == 8192 || b == 16384) g_wh_piece = b; }
 extern "C" void dl_debug_set_wh_mode(int m) { g_wh_dbg = m; }
-extern "C" void dl_debug_set_wh_prefetch(int dist, int mask) { g_wh_pf_dist = dist; g_wh_pf_mask = mask; }
 
 extern "C" long long dl_wh_bytes(int d, int n) { return (long long)((d + 127) / 128) * (n / 128) * WH_TILE_BYTES; }
 
@@ -646,8 +636,6 @@ static int gemm_wh_launch(const uint8_t* wh, int d, int n, const uint8_t* xh, in
     a.epi = *epi;
     a.vec = epilogue_vec_ok(*epi, d);
     a.dbg = g_wh_dbg;
-    a.pf_dist = g_wh_pf_dist < a.KT ? g_wh_pf_dist : 0;
-    a.pf_mask = g_wh_pf_mask;
     a.piece = g_wh_piece;
     a.tr = dl_trace_next(TR_TC);
     const size_t smem = 196608 + WT_VEC_CHUNK * EPI_TILE_LD * 4 + 16 * 8 + 16;
