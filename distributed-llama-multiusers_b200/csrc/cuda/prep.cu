@@ -171,6 +171,8 @@ struct RnqArgs {
 // 8 neighbouring blocks of one row (ROWS = 1: a CTA per row).  The merged row stays in registers between the two passes.
 // What bounds it: bytes (x, partial sums, image) for many rows, latency for few.  With one thread per block, 128 bytes apart, 2048 rows of
 // 4096 took 55.4 us alone, 512 rows 18.3; 25.4 (26.7 with 8 rows per CTA) and 9.3 with this.  32 rows are as fast either way (9 us).
+// With 8 rows per CTA each block's loads waited behind the last one's: 2048 rows of 4096 26.4 us, 8192 53.6; 17.1 and 41.1 with all blocks of a
+// thread in flight and the norm's weights one block ahead.  (One row per CTA: the same there costs registers, spills, and 1 us a launch.)
 template <int ROWS>
 __global__ void __launch_bounds__(RNQ_THREADS) reduce_norm_quant_kernel(const __grid_constant__ RnqArgs a) {
     trace_begin(a.tr);
@@ -196,46 +198,72 @@ __global__ void __launch_bounds__(RNQ_THREADS) reduce_norm_quant_kernel(const __
     const size_t src_rows = (size_t)a.src_stride / a.dim;
     const uint32_t ll_epoch = ll ? ld_volatile_u32(a.step_counter) * a.flag_mul + a.flag_add : 0u;
     const size_t row = (size_t)m * a.dim;
+    auto add_partial = [&](int s, int b, int h, float4& v) {
+        const int e = b * 32 + h * 16 + c * 4;
+        float4 p;
+        if (wire) {
+            const uint8_t* wr = reinterpret_cast<const uint8_t*>(a.partials) + ((size_t)s * src_rows + m) * rowb;
+            const int q4 = *reinterpret_cast<const int*>(wr + e);
+            const float d = __half2float(*reinterpret_cast<const __half*>(wr + a.dim + (b << 1)));
+            p = make_float4((float)(int8_t)(q4 & 0xff) * d, (float)(int8_t)((q4 >> 8) & 0xff) * d,
+                            (float)(int8_t)((q4 >> 16) & 0xff) * d, (float)(q4 >> 24) * d);
+        } else {
+            p = part_load4(a.partials, (size_t)s * a.src_stride + row + e, ll, ll_epoch);
+        }
+        v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w;
+    };
+    auto load = [&](int b, int h) { return *reinterpret_cast<const float4*>(a.x_in + row + b * 32 + h * 16 + c * 4); };
     auto merged = [&](int b, float4 (&v)[2]) {
 #pragma unroll
         for (int h = 0; h < 2; h++) {
-            const int e = b * 32 + h * 16 + c * 4;
-            v[h] = *reinterpret_cast<const float4*>(a.x_in + row + e);
-            for (int s = 0; s < a.n_src; s++) {
-                float4 p;
-                if (wire) {
-                    const uint8_t* wr = reinterpret_cast<const uint8_t*>(a.partials) + ((size_t)s * src_rows + m) * rowb;
-                    const int q4 = *reinterpret_cast<const int*>(wr + e);
-                    const float d = __half2float(*reinterpret_cast<const __half*>(wr + a.dim + (b << 1)));
-                    p = make_float4((float)(int8_t)(q4 & 0xff) * d, (float)(int8_t)((q4 >> 8) & 0xff) * d,
-                                    (float)(int8_t)((q4 >> 16) & 0xff) * d, (float)(q4 >> 24) * d);
-                } else {
-                    p = part_load4(a.partials, (size_t)s * a.src_stride + row + e, ll, ll_epoch);
-                }
-                v[h].x += p.x; v[h].y += p.y; v[h].z += p.z; v[h].w += p.w;
-            }
+            v[h] = load(b, h);
+            for (int s = 0; s < a.n_src; s++) add_partial(s, b, h, v[h]);
         }
     };
     // pass 1: merged residual -> x_out, sum of squares
     float4 keep[KEEP][2];
     float ss = 0.0f;
-    auto first = [&](int b, float4 (&v)[2]) {
-        merged(b, v);
+    auto first = [&](int b, const float4 (&v)[2]) {
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             if (a.x_out != nullptr) *reinterpret_cast<float4*>(a.x_out + row + b * 32 + h * 16 + c * 4) = v[h];
             ss += v[h].x * v[h].x + v[h].y * v[h].y + v[h].z * v[h].z + v[h].w * v[h].w;
         }
     };
+    if (ROWS == 8) {                  // a thread's blocks are in flight together (one row per CTA: a thread has one block of up to 4096 columns)
 #pragma unroll
-    for (int u = 0; u < KEEP; u++)
-        if (live && block_of(u) < nb) first(block_of(u), keep[u]);
+        for (int u = 0; u < KEEP; u++) {
+#pragma unroll
+            for (int h = 0; h < 2; h++) keep[u][h] = live && block_of(u) < nb ? load(block_of(u), h) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        for (int s = 0; s < a.n_src; s++)
+#pragma unroll
+            for (int u = 0; u < KEEP; u++)
+#pragma unroll
+                for (int h = 0; h < 2; h++)
+                    if (live && block_of(u) < nb) add_partial(s, block_of(u), h, keep[u][h]);
+#pragma unroll
+        for (int u = 0; u < KEEP; u++)
+            if (live && block_of(u) < nb) first(block_of(u), keep[u]);
+    } else {
+#pragma unroll
+        for (int u = 0; u < KEEP; u++)
+            if (live && block_of(u) < nb) {
+                merged(block_of(u), keep[u]);
+                first(block_of(u), keep[u]);
+            }
+    }
     for (int u = KEEP; live && block_of(u) < nb; u++) {
         float4 v[2];
+        merged(block_of(u), v);
         first(block_of(u), v);
     }
     float inv = 1.0f;
+    float4 wn[2];
     if (a.norm_w != nullptr) {
+        if (ROWS == 8 && live && block_of(0) < nb)
+#pragma unroll
+            for (int h = 0; h < 2; h++) wn[h] = *reinterpret_cast<const float4*>(a.norm_w + block_of(0) * 32 + h * 16 + c * 4);
         ss += __shfl_xor_sync(0xffffffffu, ss, 1);
         ss += __shfl_xor_sync(0xffffffffu, ss, 2);
         if (c == 0) s_part[warp][lane >> 2] = ss;
@@ -254,12 +282,13 @@ __global__ void __launch_bounds__(RNQ_THREADS) reduce_norm_quant_kernel(const __
         inv = 1.0f / sqrtf(t / (float)a.dim + a.eps);
     }
     // pass 2: norm, Q80
-    auto second = [&](int b, bool on, float4 (&v)[2]) {
+    auto weight = [&](int b, int h) { return *reinterpret_cast<const float4*>(a.norm_w + b * 32 + h * 16 + c * 4); };
+    auto second = [&](int b, bool on, float4 (&v)[2], auto w_of) {
         float amax = 0.0f;
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             if (a.norm_w != nullptr && on) {
-                const float4 w4 = *reinterpret_cast<const float4*>(a.norm_w + b * 32 + h * 16 + c * 4);
+                const float4 w4 = w_of(h);
                 v[h].x = w4.x * (inv * v[h].x); v[h].y = w4.y * (inv * v[h].y);
                 v[h].z = w4.z * (inv * v[h].z); v[h].w = w4.w * (inv * v[h].w);
             }
@@ -313,13 +342,22 @@ __global__ void __launch_bounds__(RNQ_THREADS) reduce_norm_quant_kernel(const __
     for (int u = 0; u < KEEP; u++) {
         const bool on = live && block_of(u) < nb;
         if (!on) keep[u][0] = keep[u][1] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (__any_sync(0xffffffffu, on)) second(block_of(u), on, keep[u]);
+        if (ROWS == 8) {
+            const float4 w[2] = {wn[0], wn[1]};
+            if (a.norm_w != nullptr && u + 1 < KEEP && live && block_of(u + 1) < nb) {      // on their way while this block is cast
+                wn[0] = weight(block_of(u + 1), 0);
+                wn[1] = weight(block_of(u + 1), 1);
+            }
+            if (__any_sync(0xffffffffu, on)) second(block_of(u), on, keep[u], [&](int h) { return w[h]; });
+        } else if (__any_sync(0xffffffffu, on)) {
+            second(block_of(u), on, keep[u], [&](int h) { return weight(block_of(u), h); });
+        }
     }
     for (int u = KEEP; ROWS == 8 ? block_of(u) < nb : (warp + u * NW) * 8 < nb; u++) {
         const bool on = live && block_of(u) < nb;
         float4 v[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
         if (on) merged(block_of(u), v);
-        second(block_of(u), on, v);
+        second(block_of(u), on, v, [&](int h) { return weight(block_of(u), h); });
     }
     trace_end(a.tr);
 }
