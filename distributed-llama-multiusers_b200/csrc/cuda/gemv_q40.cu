@@ -33,6 +33,7 @@
 #define GEMV_CONSUMERS (GEMV_NG * 128)
 #define GEMV_THREADS (GEMV_CONSUMERS + 32)
 #define GEMV_WARPS (GEMV_THREADS / 32)
+#define GEMV_SSQ_ROWS ((GEMV_WARPS + 3) & ~3)      // whole 16-byte pieces ahead of the tiles that peers send
 #define GEMV_MAX_M 8
 
 #define GEMV_TRACE(k)                                                                                      \
@@ -139,14 +140,15 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_q40_kernel(const __grid_
     uint64_t* full = reinterpret_cast<uint64_t*>(smem);                               // barriers first (8-byte aligned)
     uint64_t* empty = full + GEMV_NS;
     uint64_t* act_full = empty + GEMV_NS;
-    uint64_t* red_bar = act_full + 1;                                                // leader: S-1 remote arrivals
-    int* sflag = reinterpret_cast<int*>(red_bar + 1);
+    uint64_t* red_bar = act_full + 1;                                                // leader: the peers' partial tiles
+    uint64_t* ssq_bar = red_bar + 1;                                                 // the ranks' sums of squares
+    int* sflag = reinterpret_cast<int*>(ssq_bar + 1);
     uint8_t* stages = smem + 256;                                                    // [NS][9216]
     uint8_t* act_s = stages + GEMV_NS * Q40T_TILE_BYTES;                             // [nk][M][160]
     float* red = reinterpret_cast<float*>(act_s + (size_t)nk_max * M * XQ_ROW_BYTES);   // [NG*R][MT][rows] (<= NG*MT*128)
     float* out_s = red + GEMV_NG * MT * 128;                                         // [MT][128]
     float* ssq_w = out_s + MT * 128;                                                 // [GEMV_WARPS][MT]
-    float* ssq_all = ssq_w + GEMV_WARPS * MT;                                        // [S][MT] filled by all cluster ranks
+    float* ssq_all = ssq_w + GEMV_SSQ_ROWS * MT;                                     // [S][MT] filled by all cluster ranks
     float* recv = ssq_all + 8 * MT;                                                  // leader: [S-1][MT][128]
 
     const int tid = threadIdx.x;
@@ -193,11 +195,17 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_q40_kernel(const __grid_
             mbar_init(&empty[s], 4);
         }
         mbar_init(act_full, 1);
-        mbar_init(red_bar, S > 1 ? S - 1 : 1);
+        mbar_init(red_bar, 1);
+        mbar_init(ssq_bar, 1);
         mbar_fence_init();
+        if (S > 1) {                                    // what this CTA will be sent
+            mbar_arrive_expect_tx(ssq_bar, (uint32_t)(S * MT * 4));
+            if (crank == 0) mbar_arrive_expect_tx(red_bar, (uint32_t)((S - 1) * M * rows * 4));
+        }
     }
-    // cluster-wide: the leader's red_bar must be initialised before any peer can arrive on it
-    if (S > 1) cg::this_cluster().sync(); else __syncthreads();
+    __syncthreads();
+    // cluster-wide: the barriers must be initialised before any peer's bytes arrive on them (cluster_wait ahead of the first ones)
+    if (S > 1) cluster_arrive_relaxed();
     pdl_launch_dependents();
     GEMV_TRACE(0);
 
@@ -290,22 +298,23 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_q40_kernel(const __grid_
             if (lane == 0) ssq_w[warp * MT + m] = t;
         }
         __syncthreads();
+        if (S > 1) cluster_wait();
         if (warp < MT) {                                  // warp m reduces row m's per-warp partials
             float t = (lane < GEMV_WARPS) ? ssq_w[lane * MT + warp] : 0.0f;
             t = warp_sum(t);
             const int tidm = warp;
             if (lane == 0) {
-            // publish this CTA's share into every cluster rank's table (DSMEM stores): after the
-            // barrier nobody reads remote shared memory, so ranks may exit independently later on
+            // publish this CTA's share into every cluster rank's table; nobody reads remote shared memory, and a rank waits for
+            // all that it is sent, so ranks may exit independently later on
             if (S > 1) {
                 for (int c = 0; c < S; c++)
-                    st_shared_cluster_f32(mapa_shared(smem_u32(ssq_all + crank * MT + tidm), c), t);
+                    st_async_f32(mapa_shared(smem_u32(ssq_all + crank * MT + tidm), c), t, mapa_shared(smem_u32(ssq_bar), c));
             } else {
                 ssq_all[tidm] = t;
             }
             }
         }
-        if (S > 1) cg::this_cluster().sync(); else __syncthreads();
+        if (S > 1) mbar_wait_cluster(ssq_bar, 0); else __syncthreads();
         GEMV_TRACE(4);
         float inv[MT];
 #pragma unroll
@@ -438,24 +447,22 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_q40_kernel(const __grid_
     }
     GEMV_TRACE(3);
     if (S > 1) {
-        // split-K reduction without a second cluster barrier: peers push their partial tile into the
-        // leader's shared memory (DSMEM stores), release-arrive on its mbarrier and exit; the leader
-        // acquires the barrier and sums in rank order (deterministic).
+        // split-K reduction without a second cluster barrier: peers send their partial tile into the leader's shared memory and exit; the
+        // leader waits for the bytes and sums in rank order (deterministic).
         __syncthreads();
+        if (!a.fused) cluster_wait();
         if (crank != 0) {
-            const uint32_t dst = mapa_shared(smem_u32(recv + (size_t)(crank - 1) * MT * 128), 0);
-            for (int idx = tid; idx < MT * rows; idx += GEMV_THREADS) {
-                const int m = idx / rows, r = idx % rows;
-                st_shared_cluster_f32(dst + (uint32_t)(m * 128 + r) * 4u, out_s[m * 128 + r]);
+            const uint32_t dst = mapa_shared(smem_u32(recv + (size_t)(crank - 1) * MT * 128), 0), bar = mapa_shared(smem_u32(red_bar), 0);
+            const int r4 = rows >> 2;
+            for (int idx = tid; idx < M * r4; idx += GEMV_THREADS) {
+                const int at = (idx / r4) * 128 + (idx % r4) * 4;
+                st_async_f32x4(dst + (uint32_t)at * 4u, *reinterpret_cast<const float4*>(out_s + at), bar);
             }
-            fence_acq_rel_cluster();
-            __syncthreads();
-            if (tid == 0) mbar_arrive_remote(mapa_shared(smem_u32(red_bar), 0));
             trace_end(a.tr);
             return;
         }
         mbar_wait_cluster(red_bar, 0);
-        for (int idx = tid; idx < MT * rows; idx += GEMV_THREADS) {
+        for (int idx = tid; idx < M * rows; idx += GEMV_THREADS) {
             const int m = idx / rows, r = idx % rows;
             float vsum = out_s[m * 128 + r];
             for (int c = 0; c < S - 1; c++) vsum += recv[(size_t)c * MT * 128 + m * 128 + r];
@@ -473,7 +480,7 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_q40_kernel(const __grid_
 
 static size_t gemv_smem_bytes(int MT, int nk_max, int M) {
     return 256 + (size_t)GEMV_NS * Q40T_TILE_BYTES + (size_t)nk_max * M * XQ_ROW_BYTES +
-           (size_t)(GEMV_NG * MT * 128 + MT * 128) * 4 + (size_t)(GEMV_WARPS * MT + 8 * MT) * 4 +
+           (size_t)(GEMV_NG * MT * 128 + MT * 128) * 4 + (size_t)(GEMV_SSQ_ROWS * MT + 8 * MT) * 4 +
            (size_t)7 * MT * 128 * 4 + 16;
 }
 
