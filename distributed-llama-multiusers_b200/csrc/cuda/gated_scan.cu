@@ -343,44 +343,68 @@ __global__ void __launch_bounds__(GC_THREADS, RT * NC <= 4 ? 4 : 2) gated_chunk_
     }
 }
 
-// pass 2: over a sequence's chunks in order, scratch <- the state BEFORE the chunk; the slot gets the state after the last
-// one.  One thread per state element (head form: and per element of n).
-template <bool CH>
-__global__ void __launch_bounds__(256) gated_chunk_prefix_kernel(DlMambaBatch b, DlGatedArgs a, GatedScratch sc) {
+// pass 2: over a sequence's chunks in order, scratch <- the state BEFORE the chunk; the slot gets the state after the last one.  A thread owns
+// EV neighbours of a row of the state (four where rows and addresses allow it), head form: or one element of n.
+// What bounds it: the bytes of all chunks' states, in and out, and how many of them a thread has in flight.  One element per thread, eight chunks
+// loaded together behind the last eight's stores: 33.7 us for 32 chunks x 16 heads of 128 x 128 from cold caches; 12.6 with the next chunks' loads ahead
+// of them (2000 rows in all three passes 180.7 and 174.8 us).
+template <bool CH, int EV>
+__global__ void __launch_bounds__(128) gated_chunk_prefix_kernel(DlMambaBatch b, DlGatedArgs a, GatedScratch sc) {
+    constexpr int U = 8;
     const int n = blockIdx.x, h = blockIdx.y;
     const int D = a.dim, V = a.vdim, H = a.n_heads, DV = D * V;
-    const int e = blockIdx.z * blockDim.x + threadIdx.x;
-    if (e >= DV + (CH ? 0 : D)) return;
-    const bool is_n = e >= DV;
+    const int t = blockIdx.z * blockDim.x + threadIdx.x, nv = DV / EV;
+    if (t >= nv + (CH ? 0 : D)) return;
+    const bool is_n = t >= nv;
+    const int e = t * EV;
     const int s0 = b.seq_start[n], nc = (b.seq_start[n + 1] - s0 + GC - 1) / GC;
     const size_t sh = (size_t)b.seq_slot[n] * H + h, ch0 = (size_t)(s0 / GC + n) * H + h;
-    float* Sg = is_n ? a.n_state + sh * D + (e - DV) : a.state + sh * DV + e;
-    float R = b.seq_pos0[n] == 0 ? 0.f : *Sg;
-    float* p0 = is_n ? sc.ns + ch0 * D + (e - DV) : sc.S + ch0 * DV + e;
+    float* Sg = is_n ? a.n_state + sh * D + (t - nv) : a.state + sh * DV + e;
+    float* p0 = is_n ? sc.ns + ch0 * D + (t - nv) : sc.S + ch0 * DV + e;
     const size_t step = is_n ? (size_t)H * D : (size_t)H * DV, dstep = (size_t)H * D;
     const float* t0 = sc.dec + ch0 * D + (CH ? e / V : 0);
-    for (int c0 = 0; c0 < nc; c0 += 8) {          // eight chunks' sums are loaded together, then chained
-        float own[8], dec[8];
+    struct Vec { float v[EV]; };
+    auto get = [&](const float* p) {
+        Vec x = {};
+        if (EV == 4 && !is_n) { const float4 f = *reinterpret_cast<const float4*>(p); x.v[0] = f.x; x.v[1 % EV] = f.y; x.v[2 % EV] = f.z; x.v[3 % EV] = f.w; }
+        else x.v[0] = *p;
+        return x;
+    };
+    auto set = [&](float* p, const Vec& x) {
+        if (EV == 4 && !is_n) *reinterpret_cast<float4*>(p) = make_float4(x.v[0], x.v[1 % EV], x.v[2 % EV], x.v[3 % EV]);
+        else *p = x.v[0];
+    };
+    Vec R = {};
+    if (b.seq_pos0[n] != 0) R = get(Sg);
+    Vec own[U], next[U];
+    float dec[U], dnext[U];
+    auto fetch = [&](int c0, Vec (&o)[U], float (&d)[U]) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            own[i] = c0 + i < nc ? p0[(size_t)(c0 + i) * step] : 0.f;
-            dec[i] = c0 + i < nc ? t0[(size_t)(c0 + i) * dstep] : 0.f;
-        }
+        for (int i = 0; i < U; ++i)
+            if (c0 + i < nc) { o[i] = get(p0 + (size_t)(c0 + i) * step); d[i] = t0[(size_t)(c0 + i) * dstep]; }
+    };
+    fetch(0, own, dec);
+    for (int c0 = 0; c0 < nc; c0 += U) {
+        fetch(c0 + U, next, dnext);
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+        for (int i = 0; i < U; ++i)
             if (c0 + i < nc) {
-                p0[(size_t)(c0 + i) * step] = R;
-                R = fmaf(dec[i], R, own[i]);
+                set(p0 + (size_t)(c0 + i) * step, R);
+#pragma unroll
+                for (int x = 0; x < EV; ++x) R.v[x] = fmaf(dec[i], R.v[x], own[i].v[x]);
             }
+#pragma unroll
+        for (int i = 0; i < U; ++i) { own[i] = next[i]; dec[i] = dnext[i]; }
     }
-    *Sg = R;
+    set(Sg, R);
 }
 
 // Passes 1 and 3 are bound by the instructions that their 16 warps per SM issue (shared memory holds two CTAs of the output kernel): f32
 // multiply-adds throughout, whole running products for the diagonal sub-blocks, and the gates' exponentials, formed in both.  So two
 // neighbours along the contraction are one operand (fma2: two multiply-adds an issue), the diagonal takes two columns and two
 // channels at a time, and a warp's eight rows form their gates side by side: 2000 rows x 16 heads of 128 x 128 240.7 -> 180 us, pass 1
-// 75 -> 63, pass 3 153 -> 103.  Twice the warps at half the registers (a column of the diagonal and half of the tile each): 206,
+// 75 -> 63, pass 3 153 -> 103.  (The products on the tensor cores, each operand in two tf32 parts: pass 1 59, pass 3 104, the state's error 1.35e-7
+// for 1.13e-7: what is left is the gates, the diagonal and the staging, 13 k instructions a warp at half an issue slot.)  Twice the warps at half the registers (a column of the diagonal and half of the tile each): 206,
 // three CTAs of pass 1 on an SM (80 registers, spilled): 205.  Narrow tiles leave shared memory for more CTAs and do with fewer registers:
 // three of pass 3 (80) and four of pass 1 (64), 2000 rows x 32 heads of 64 x 64 136 -> 123 us (head form 156 -> 128; before 175 and 150).
 //
@@ -586,7 +610,11 @@ static int launch_gated_chunked(const DlMambaBatch& b, int n_seq, int max_chunks
     int rc = narrow ? (low ? launch_gated_state<CH, 4, 1>(b, n_seq, max_chunks, a, sc, st) : launch_gated_state<CH, 8, 1>(b, n_seq, max_chunks, a, sc, st))
                     : launch_gated_state<CH, 4, 2>(b, n_seq, max_chunks, a, sc, st);
     if (rc != 0) return rc;
-    gated_chunk_prefix_kernel<CH><<<dim3(n_seq, a.n_heads, (a.dim * (a.vdim + (CH ? 0 : 1)) + 255) / 256), 256, 0, st>>>(b, a, sc);
+    const int per_head = a.dim * a.vdim, extra = CH ? 0 : a.dim;
+    if (a.vdim % 4 == 0 && (((uintptr_t)a.state | (uintptr_t)sc.S) & 15) == 0)
+        gated_chunk_prefix_kernel<CH, 4><<<dim3(n_seq, a.n_heads, (per_head / 4 + extra + 127) / 128), 128, 0, st>>>(b, a, sc);
+    else
+        gated_chunk_prefix_kernel<CH, 1><<<dim3(n_seq, a.n_heads, (per_head + extra + 127) / 128), 128, 0, st>>>(b, a, sc);
     return narrow ? launch_gated_out<MODE, 1>(b, n_seq, max_chunks, a, sc, st) : launch_gated_out<MODE, 2>(b, n_seq, max_chunks, a, sc, st);
 }
 
