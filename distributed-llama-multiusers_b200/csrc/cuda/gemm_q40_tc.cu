@@ -176,9 +176,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_q40_tc_kernel(const __grid
         const bool det = (a.dbg_mode & 4) != 0;      // detail stamps of warp 1 only (slots 0..7)
         const bool stamp = (lane == 0 && mw == 0 && !(a.dbg_mode & 8));
         const int nsb_mask = a.NSB - 1, nsb_log = a.nsb_log;
-        // narrow tiles are dequant-bound: the issuers sleep between probes and leave their sub-partition's issue
-        // slots to the math warps; wide tiles are MMA-bound: the issuers are the critical path and spin
-        const uint32_t mma_sleep = (NT <= 32) ? 64u : 0u;
         const int nstg = a.nstg;
         const uint32_t a_col0 = TC_TMEM_COLS - nstg * TC_A_STAGE_COLS;
         if (mw < nacc) {
@@ -187,9 +184,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_q40_tc_kernel(const __grid
                 const int k = a.pair ? i >> 1 : i;
                 const int sb = k & nsb_mask, pb = (k >> nsb_log) & 1;
                 if (det && stamp) TC_DBG(0, i);
-                mbar_wait_sleep(&fullH[sh], ph, mma_sleep);
+                mbar_wait(&fullH[sh], ph);
                 if (stamp) TC_DBG(det ? 1 : 5, i);
-                mbar_wait_sleep(&fullB[sb], pb, mma_sleep);
+                mbar_wait(&fullB[sb], pb);
                 if (stamp) TC_DBG(det ? 2 : 6, i);
                 tc_fence_after();
                 if (det && stamp) TC_DBG(3, i);
@@ -229,16 +226,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_q40_tc_kernel(const __grid
         const uint32_t sc_off = Q40T_SCALE_OFF + r * 8;
         const int nstg = a.nstg;
         const uint32_t a_taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (TC_TMEM_COLS - nstg * TC_A_STAGE_COLS);
-        const __half2 c1032 = __float2half2_rn(1032.0f);
-        const __half2 c1152 = __float2half2_rn(1152.0f);
-        const __half2 sixteenth = __float2half2_rn(0.0625f);
         const bool stamp = (tid == 64 && !(a.dbg_mode & 12));
         const bool qstamp = (lane == 0 && (a.dbg_mode & 8));      // mode 8: slots 1..4 = arrival time of lane quarter 0..3
         const int nsa = a.NSA;
         int sh = g, ph = 0;      // A stage of k-tile i = i % nstg (g < 4 <= nstg), phase parity = (i / nstg) & 1
         int sa = g, pa = 0;      // raw ring stage i % NSA and its phase parity
         for (int i = g; i < n_it; i += TC_GROUPS) {
-            mbar_wait_sleep(&fullA[sa], pa, 32);
+            mbar_wait(&fullA[sa], pa);
             if (stamp) TC_DBG(1, i);
             const uint8_t* raw = ringA + sa * Q40T_TILE_BYTES;
             uint4 nb[4];
@@ -251,38 +245,23 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_q40_tc_kernel(const __grid
             // complete in order; the refill is >500 ns away (barrier -> producer poll -> HBM fetch).
             __syncwarp();
             if (lane == 0) mbar_arrive(&emptyA[sa]);
-            if (i >= nstg) mbar_wait_sleep(&emptyH[sh], ph ^ 1, 32);      // the MMAs that read this A stage have retired
+            if (i >= nstg) mbar_wait(&emptyH[sh], ph ^ 1);      // the MMAs that read this A stage have retired
             if (stamp) TC_DBG(2, i);
             tc_fence_after();
+            const bool big = __any_sync(0xffffffffu, q40_big(sc.x) || q40_big(sc.y));
+            auto expand = [&](auto is_big) {
 #pragma unroll
-            for (int kb = 0; kb < 4; kb++) {
-                const uint32_t sw = (kb < 2) ? sc.x : sc.y;
-                const uint32_t s16 = (kb & 1) ? (sw >> 16) : (sw & 0xFFFFu);
-                const uint32_t sdup = s16 | (s16 << 16);
-                const __half2 d2 = *reinterpret_cast<const __half2*>(&sdup);
-                const __half2 d2h = __hmul2(d2, sixteenth);      // exact (power of two) unless d is subnormal
-                const uint32_t words[4] = {nb[kb].x, nb[kb].y, nb[kb].z, nb[kb].w};
-                uint32_t v[16];
-#pragma unroll
-                for (int w = 0; w < 4; w++) {
-                    // K-slot order inside the 32-block (XH uses the same): e(4w), e(4w+2), e(4w+1), e(4w+3), then +16
-                    const uint32_t x = words[w];
-                    const uint32_t x8 = x >> 8;
-                    uint32_t l02 = (x & 0x000F000Fu) | 0x64006400u;      // half2(1024+e0, 1024+e2)
-                    uint32_t l13 = (x8 & 0x000F000Fu) | 0x64006400u;     // half2(1024+e1, 1024+e3)
-                    uint32_t h02 = (x & 0x00F000F0u) | 0x64006400u;      // half2(1024+16*e16, 1024+16*e18)
-                    uint32_t h13 = (x8 & 0x00F000F0u) | 0x64006400u;
-                    __half2 v0 = __hmul2(__hsub2(*reinterpret_cast<__half2*>(&l02), c1032), d2);
-                    __half2 v1 = __hmul2(__hsub2(*reinterpret_cast<__half2*>(&l13), c1032), d2);
-                    __half2 v2 = __hmul2(__hsub2(*reinterpret_cast<__half2*>(&h02), c1152), d2h);   // 16(e-8) * d/16
-                    __half2 v3 = __hmul2(__hsub2(*reinterpret_cast<__half2*>(&h13), c1152), d2h);
-                    v[w * 4 + 0] = *reinterpret_cast<uint32_t*>(&v0);
-                    v[w * 4 + 1] = *reinterpret_cast<uint32_t*>(&v1);
-                    v[w * 4 + 2] = *reinterpret_cast<uint32_t*>(&v2);
-                    v[w * 4 + 3] = *reinterpret_cast<uint32_t*>(&v3);
+                for (int kb = 0; kb < 4; kb++) {
+                    const uint32_t sdup = __byte_perm((kb < 2) ? sc.x : sc.y, 0, (kb & 1) ? 0x3232 : 0x1010);
+                    const __half2 d2 = *reinterpret_cast<const __half2*>(&sdup);
+                    uint32_t v[16];
+                    const uint32_t words[4] = {nb[kb].x, nb[kb].y, nb[kb].z, nb[kb].w};
+                    q40_expand<decltype(is_big)::value>(words, d2, v);
+                    if (!(a.dbg_mode & 2)) tmem_st_32x32b_x16(a_taddr + sh * TC_A_STAGE_COLS + kb * 16, v);
                 }
-                if (!(a.dbg_mode & 2)) tmem_st_32x32b_x16(a_taddr + sh * TC_A_STAGE_COLS + kb * 16, v);
-            }
+            };
+            if (big) expand(BoolIs<true>());
+            else expand(BoolIs<false>());
             tmem_st_wait();
             if (stamp) TC_DBG(3, i);
             tc_fence_before();

@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(WT_THREADS, 1) gemm_wh_tc_kernel(const __grid_
 
 // ------------------------------------------------------------------------------------------------
 // Q40T -> WH: one CTA per 128 x 128 tile, thread = (row, 32-block).  Same arithmetic as the dequantisers of
-// gemm_q40_tc.cu: low nibbles ((1024 + e) - 1032) * d, high nibbles ((1024 + 16 e) - 1152) * (d / 16).
+// gemm_q40_tc.cu (q40_expand).
 // ------------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(512) q40t_to_wh_kernel(const uint8_t* __restrict__ q40t, uint8_t* __restrict__ wh) {
     const uint8_t* raw = q40t + (size_t)blockIdx.x * Q40T_TILE_BYTES;
@@ -358,26 +358,13 @@ __global__ void __launch_bounds__(512) q40t_to_wh_kernel(const uint8_t* __restri
     const uint4 nb = *reinterpret_cast<const uint4*>(raw + r * 64 + (((kb + (r >> 1)) & 3) << 4));
     const __half d = *reinterpret_cast<const __half*>(raw + Q40T_SCALE_OFF + r * 8 + kb * 2);
     const __half2 d2 = __half2half2(d);
-    const __half2 d2h = __hmul2(d2, __float2half2_rn(0.0625f));
-    const __half2 c1032 = __float2half2_rn(1032.0f), c1152 = __float2half2_rn(1152.0f);
     const uint32_t words[4] = {nb.x, nb.y, nb.z, nb.w};
+    uint32_t v[16];
+    if (q40_big(*reinterpret_cast<const uint32_t*>(&d2))) q40_expand<true>(words, d2, v);
+    else q40_expand<false>(words, d2, v);
     uint8_t* dst = out + (size_t)(r >> 3) * XH_ROWGROUP_BYTES + (size_t)(kb * 4) * 128 + (size_t)(r & 7) * 16;
 #pragma unroll
-    for (int w = 0; w < 4; w++) {
-        const uint32_t x = words[w], x8 = x >> 8;
-        uint32_t l02 = (x & 0x000F000Fu) | 0x64006400u, l13 = (x8 & 0x000F000Fu) | 0x64006400u;
-        uint32_t h02 = (x & 0x00F000F0u) | 0x64006400u, h13 = (x8 & 0x00F000F0u) | 0x64006400u;
-        __half2 v0 = __hmul2(__hsub2(*reinterpret_cast<__half2*>(&l02), c1032), d2);
-        __half2 v1 = __hmul2(__hsub2(*reinterpret_cast<__half2*>(&l13), c1032), d2);
-        __half2 v2 = __hmul2(__hsub2(*reinterpret_cast<__half2*>(&h02), c1152), d2h);
-        __half2 v3 = __hmul2(__hsub2(*reinterpret_cast<__half2*>(&h13), c1152), d2h);
-        uint4 o;
-        o.x = *reinterpret_cast<uint32_t*>(&v0);
-        o.y = *reinterpret_cast<uint32_t*>(&v1);
-        o.z = *reinterpret_cast<uint32_t*>(&v2);
-        o.w = *reinterpret_cast<uint32_t*>(&v3);
-        *reinterpret_cast<uint4*>(dst + w * 128) = o;
-    }
+    for (int w = 0; w < 4; w++) *reinterpret_cast<uint4*>(dst + w * 128) = make_uint4(v[4 * w], v[4 * w + 1], v[4 * w + 2], v[4 * w + 3]);
 }
 
 extern void dl_set_error(const char* fmt, ...);
