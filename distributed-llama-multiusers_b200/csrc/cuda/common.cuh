@@ -51,8 +51,8 @@ DL_DEVINL void xh_slot(int e, int& w, int& s) {
 }
 
 // The 32 values of a Q40 block, fp16((nibble - 8) d) in one rounding each, from its four words of nibbles; K-slot order of xh_slot(): e(4w), e(4w+2),
-// e(4w+1), e(4w+3), then + 16.  (1024 + e) - 1032, times d; high nibbles stand 4 bits up, where they are the fp16 subnormals e 2^-20: one fma with 2^20 d
-// and -8 d (exact factors) while 2^20 d is finite.  BIG: |d| >= 2^-4 somewhere (q40_big), all by the first form.
+// e(4w+1), e(4w+3), then + 16.  A nibble at bits 4 to 7 of a half is the fp16 subnormal e 2^-20: one fma with 2^20 d and -8 d (exact factors) while 2^20 d
+// is finite.  BIG: |d| >= 2^-4 somewhere (q40_big): (1024 + e) - 1032, times d, two instructions on the fp16 pipe, which takes one every other clock.
 template <bool B> struct BoolIs { static constexpr bool value = B; };
 DL_DEVINL bool q40_big(uint32_t two_scales) { return (((two_scales & 0x7FFF7FFFu) + 0x54005400u) & 0x80008000u) != 0u; }
 template <bool BIG>
@@ -61,15 +61,17 @@ DL_DEVINL void q40_expand(const uint32_t (&words)[4], __half2 d2, uint32_t (&v)[
     const __half2 d20 = __hmul2(__hmul2(d2, k10), k10), m8d = __hmul2(d2, __float2half2_rn(-8.0f));
     auto h2 = [](uint32_t x) { return *reinterpret_cast<const __half2*>(&x); };
     auto u32 = [](__half2 x) { return *reinterpret_cast<const uint32_t*>(&x); };
-    auto low = [&](uint32_t x) { return u32(__hmul2(__hsub2(h2((x & 0x000F000Fu) | 0x64006400u), c1032), d2)); };
-    auto high = [&](uint32_t x) { return BIG ? low(x >> 4) : u32(__hfma2(h2(x & 0x00F000F0u), d20, m8d)); };
+    // the nibbles at bits `at` to `at + 3` of both halves
+    auto value = [&](uint32_t x, int at) {
+        if (BIG) return u32(__hmul2(__hsub2(h2(((x >> at) & 0x000F000Fu) | 0x64006400u), c1032), d2));
+        return u32(__hfma2(h2((at < 4 ? x << 4 : x >> (at - 4)) & 0x00F000F0u), d20, m8d));
+    };
 #pragma unroll
     for (int w = 0; w < 4; w++) {
-        const uint32_t x = words[w], x8 = x >> 8;
-        v[w * 4 + 0] = low(x);
-        v[w * 4 + 1] = low(x8);
-        v[w * 4 + 2] = high(x);
-        v[w * 4 + 3] = high(x8);
+        v[w * 4 + 0] = value(words[w], 0);
+        v[w * 4 + 1] = value(words[w], 8);
+        v[w * 4 + 2] = value(words[w], 4);
+        v[w * 4 + 3] = value(words[w], 12);
     }
 }
 

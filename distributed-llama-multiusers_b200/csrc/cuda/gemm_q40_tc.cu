@@ -14,9 +14,9 @@
 // tiles in smem: 32 KB written + 32 KB read per 9 KB of weights saturated the 128 B/clk crossbar
 // (1450 clk per k-tile, all of it in the MMA queue).
 //
-// Warp roles (672 threads):
+// Warp roles (608 threads):
 //   warp 0       producer: bulk async copies of raw 9 KB Q40T tiles (lanes 0-3) and XH slabs (lanes 4-7)
-//   warps 1,18-20 MMA issuers (one elected lane each; tcgen05.mma / tcgen05.commit), k-tiles round-robin,
+//   warps 1,18   MMA issuers (one elected lane each; tcgen05.mma / tcgen05.commit), k-tiles round-robin,
 //                one accumulator each; warp 1 also allocates TMEM
 //   warps 2-17   dequantisers, 4 groups x 4 warps: group = k-tile % 4 = A stage, warp % 4 = TMEM lane
 //                quarter, thread = weight row: LDS.128 x4 -> packed fp16x2 registers -> tcgen05.st.32x32b.x16
@@ -29,11 +29,13 @@
 #include "epilogue.cuh"
 
 #define TC_DEQ_WARPS 16
-#define TC_THREADS (64 + TC_DEQ_WARPS * 32 + 96)      // producer, MMA warp 0, dequantisers, MMA warps 1-3
+#define TC_THREADS (64 + TC_DEQ_WARPS * 32 + 32)      // producer, MMA warp 0, dequantisers, MMA warp 1
 #define TC_EPI_CHUNK 32           // activation rows per epilogue pass
 #define TC_TMEM_COLS 512
 #define TC_A_STAGE_COLS 64        // 128 K x fp16 = 64 32-bit columns per lane
-#define TC_GROUPS 4               // dequantiser groups (k-tile i -> group i % 4)
+// dequantiser groups (k-tile i -> group i % 4).  Four: a stage of either ring must come back to the group that had it, or to one that has waited behind it
+// (a parity wait cannot see a phase before the last), so the count divides the raw stages; six groups (48 more registers spilled a thread) are slower, 369 us for 359.
+#define TC_GROUPS 4
 
 struct TcArgs {
     const uint8_t* w;
@@ -42,7 +44,7 @@ struct TcArgs {
     int NSA, NSB, nsb_log;
     int nstg;              // A stages in TMEM (64 columns each), at columns [512 - 64*nstg, 512)
     int pair;              // 1: this CTA multiplies row tiles 2c and 2c + 1 side by side (item i = row tile i & 1, k-tile i >> 1; one accumulator each)
-    int nacc;              // MMA-issuing warps = independent TMEM accumulators (1, 2 or 4; nacc*NT <= 256), summed by the epilogue
+    int nacc;              // MMA-issuing warps = independent TMEM accumulators (1 or 2; nacc*NT <= 256), summed by the epilogue
     int LA, LB;            // issuing lanes per ring; each divides its stage count so a stage has ONE owner lane
     int n_epi_ctas;
     int vec;               // epilogue_vec takes the epilogue
@@ -163,7 +165,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_q40_tc_kernel(const __grid
         // ------------------------------------ MMA issuers ------------------------------------
         // One k-tile costs its issuing thread ~900 clk of mostly fixed latency (two barrier waits, fence,
         // eight MMAs issued at ~45 clk each, two commits), far more than the MMAs
-        // themselves.  Up to four issuing warps take k-tiles round-robin, each into its OWN accumulator
+        // themselves.  Up to two issuing warps take k-tiles round-robin, each into its OWN accumulator
         // (summed by the epilogue), so the result stays bit-deterministic.  Warp-uniform control flow: every
         // lane walks the barriers, one elected lane issues.
         const int mw = (warp == 1) ? 0 : warp - (2 + TC_DEQ_WARPS) + 1;
@@ -429,7 +431,7 @@ extern "C" int dl_gemm_q40_tc(const uint8_t* w_q40t, int d, int n, const uint8_t
     // written after a retire that is ordered behind the previous one), so a parity wait can never be lapped
     a.nacc = (a.NT <= 128) ? 2 : 1;                        // (also the two row tiles of a pair)
     a.nstg = (a.NT <= 64) ? 6 : 4;
-    if (a.nacc * a.NT + a.nstg * TC_A_STAGE_COLS > TC_TMEM_COLS || a.nstg < TC_GROUPS || a.nstg > 8 || a.nstg % a.nacc != 0 || (a.nacc != 1 && a.nacc != 2 && a.nacc != 4)) {
+    if (a.nacc * a.NT + a.nstg * TC_A_STAGE_COLS > TC_TMEM_COLS || a.nstg < TC_GROUPS || a.nstg > 8 || a.nstg % a.nacc != 0 || a.nacc < 1 || a.nacc > 2 || a.NSA % TC_GROUPS != 0) {
         dl_set_error("dl_gemm_q40_tc: bad TMEM plan nacc=%d nstg=%d NT=%d", a.nacc, a.nstg, a.NT);
         return -1;
     }
