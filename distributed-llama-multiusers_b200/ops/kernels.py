@@ -354,20 +354,18 @@ def decode_mega_plan(d: int, n: int, align: int, grid: int, cta: int):
 
 
 def choose_tc_split(d: int, n: int, M: int, n_sms: int) -> int:
-    """Cluster split-K factor of the tcgen05 GEMM: a power of two (<= 8) that fills the chip without
+    """Cluster split-K factor of the tcgen05 GEMM: a power of two (<= 4) that fills the chip without
     ever launching more CTAs than SMs (one CTA per SM: a second wave of half-empty CTAs costs more
     than the extra parallelism buys).  The activation tile is 16/32/64/128 rows (256 with a 256-row
     capacity), so wide batches already bring ceil(M / tile) CTAs per row tile."""
     row_tiles = (d + 127) // 128
     nt = 16 if M <= 16 else 32 if M <= 32 else 64 if M <= 64 else 128
     m_tiles = (M + nt - 1) // nt
-    # from 33 rows on a share keeps a long k-loop.  The line was drawn when one rank summed and finished all rows, two cluster barriers per
-    # 32 of them (4096 x 4096 at 64 rows: 18.4 us whole, 15.8 / 20.0 in 2 / 4 shares).  Every rank finishes rows of its own now and shorter
-    # shares would pay too (18.4, 14.4 / 12.8; 6144 x 4096 18.5 and 16.2 in 2), eight of them not (2048 x 2048 12.3 whole, 10.2 in 4, 16.9 in 8),
-    # so the line costs time where it forbids a split, and none where it allows one (4096 x 14336 45.2 whole, 20.6 in 4)
-    min_kt = 1 if M <= 32 else 24
+    # Every rank finishes rows of its own, so short shares pay (us with 1 / 2 / 4 / 8 ranks: 4096 x 4096 at 32 rows 13.2 / 8.9 / 8.1, at 64 rows 13.2 / 10.2
+    # / 8.6, at 128 rows 14.5 / 11.4 / 10.7; 6144 x 4096 at 64 rows 14.3 / 11.3), and eight ranks read too much of each other (2048 x 2048 at 32 rows 8.7 / 8.7
+    # / 8.7 / 9.7, at 128 rows 8.8 / 8.7 / 8.5 / 15.3)
     S = 1
-    while row_tiles * m_tiles * S * 2 <= n_sms and S < 8 and (n // 128) // (S * 2) >= min_kt:
+    while row_tiles * m_tiles * S * 2 <= n_sms and S < 4 and (n // 128) // (S * 2) >= 4:
         S *= 2
     return S
 
