@@ -412,12 +412,22 @@ extern "C" int dl_gemm_q40_tc(const uint8_t* w_q40t, int d, int n, const uint8_t
     a.NT = (M <= 16) ? 16 : (M <= 32) ? 32 : (M <= 64) ? 64 : 128;
     const int row_tiles = (d + 127) / 128, n_sms = dl_device_sm_count();
     const int ks = (k_split == 2 || k_split == 4 || k_split == 8) ? k_split : 1;
-    // 256-wide tiles halve the dequant work per activation row, but only pay when they still leave enough CTAs
-    // to fill the chip (w13: 224 row tiles) ...
-    if (M > 128 && ncap % 256 == 0 && row_tiles * ((M + 255) / 256) * ks >= n_sms / 2) a.NT = 256;
+    // From 129 rows on: tiles of 128 rows, or of up to 256, as many as those need and of equal width (what a tile is short of is multiplied too), which
+    // unpack the weights half as often but go through one accumulator and one issuing warp.  Whichever takes fewer waves of the SMs times clocks of one: a
+    // k-tile 520 clk at 128 rows, 950 or its MMAs' 4 per row above, start and epilogue 13000 + 30 a row (norm and feed-forward, us in 128s / wide, 4096 x 14336 at
+    // 300 rows 156 / 176, 400 rows - / 188 (two tiles of 256: 200), 520 rows - / 255 (three: 275); 2048 x 8192 at 300 rows 65 / 62); wide ones
+    // only where they leave enough CTAs to fill the chip
+    if (M > 128) {
+        const long long m_tiles = (M + 255) / 256, nt = ((M + m_tiles - 1) / m_tiles + 31) / 32 * 32;
+        auto clocks = [&](long long tiles, long long item, long long width) {
+            return (row_tiles * tiles * ks + n_sms - 1) / n_sms * (a.KT / ks * item + 13000 + 30 * width);
+        };
+        if (ncap >= m_tiles * nt && row_tiles * m_tiles * ks >= n_sms / 2 &&
+            clocks(m_tiles, nt * 4 > 950 ? nt * 4 : 950, nt) < clocks((M + 127) / 128, 520, 128)) a.NT = (int)nt;
+    }
     // ... and narrow matrices (qkv / wo: 32-48 row tiles) are better off with narrower tiles that launch more
     // CTAs, even though every CTA then unpacks the weight tile again (the unpack overlaps the MMAs)
-    while (a.NT > 32 && row_tiles * ((M + a.NT - 1) / a.NT) * ks < n_sms / 2) a.NT >>= 1;
+    while (a.NT > 32 && a.NT <= 128 && row_tiles * ((M + a.NT - 1) / a.NT) * ks < n_sms / 2) a.NT >>= 1;
     if (ncap < (M + a.NT - 1) / a.NT * a.NT) { dl_set_error("dl_gemm_q40_tc: ncap=%d too small for M=%d (tile %d)", ncap, M, a.NT); return -1; }
     if (k_split != 1 && k_split != 2 && k_split != 4 && k_split != 8) { dl_set_error("dl_gemm_q40_tc: k_split must be 1,2,4,8"); return -1; }
     if (k_split > a.KT) k_split = 1;
