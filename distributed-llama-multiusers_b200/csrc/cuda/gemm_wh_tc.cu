@@ -29,7 +29,7 @@
 #include "epilogue.cuh"
 
 #define WH_TILE_BYTES 32768
-#define WT_NT 256                      // activation rows per tile
+#define WT_NT 256                      // most activation rows per tile (wh_tile_rows: how many)
 #define WT_THREADS 576
 #define WT_EPI_CHUNK 32                // activation rows per epilogue pass, one row per warp quarter
 #define WT_VEC_CHUNK 64                // the same by whole warps (epilogue_vec): four rows per warp
@@ -38,6 +38,7 @@ struct WhArgs {
     const uint8_t* wh;                 // [row_tiles][KT][32 KB]
     const uint8_t* xh;                 // [KT][ncap/8][2048]
     int d_real, row_tiles, KT, ncap, M, m_tiles, n_tiles;
+    int nt;                            // activation rows per tile: a multiple of 32 (what an MMA of two CTAs takes), at most WT_NT
     int n_epi_ctas;
     int piece;                         // bytes per bulk copy (4096 / 8192 / 16384)
     int dbg;                           // timing experiments (results invalid): 1 = no epilogue work, 2 = no MMAs, 4 = no activation copies
@@ -129,15 +130,15 @@ DL_DEVINL bool wt_tile(const WhArgs& a, int t, WtTile& w) {
         w.row0 = 0;
         w.rows = a.M;
     }
-    return w.mt * WT_NT < w.rows;
+    return w.mt * a.nt < w.rows;
 }
 
 template <int CG>
 __global__ void __launch_bounds__(WT_THREADS, 1) gemm_wh_tc_kernel(const __grid_constant__ WhArgs a) {
     extern __shared__ __align__(1024) uint8_t smem[];
     constexpr int NS = (CG == 1) ? 2 : 3;                 // stages of one 128-wide k step
-    constexpr int B_ROWS = WT_NT / CG;                    // activation rows staged by this CTA
-    constexpr int STAGE = WH_TILE_BYTES + B_ROWS * 256;   // 96 KB / 64 KB
+    constexpr int STAGE = WH_TILE_BYTES + WT_NT / CG * 256;   // 96 KB / 64 KB
+    const int B_ROWS = a.nt / CG;                         // activation rows staged by this CTA
     trace_begin(a.tr);
     const unsigned long long t0 = globaltimer_ns();
     float* out_s = reinterpret_cast<float*>(smem + NS * STAGE);          // [32][128], or [WT_VEC_CHUNK][EPI_TILE_LD]
@@ -190,7 +191,7 @@ __global__ void __launch_bounds__(WT_THREADS, 1) gemm_wh_tc_kernel(const __grid_
             if (!wt_tile(a, t, w)) continue;
             const int rp = w.rp, mt = w.mt;
             const int rt = rp * CG + (int)crank;
-            const int mrow0 = w.row0 + mt * WT_NT + (int)crank * B_ROWS;
+            const int mrow0 = w.row0 + mt * a.nt + (int)crank * B_ROWS;
             const int row_cap = a.grp ? w.row0 + ((w.rows + 7) & ~7) : a.ncap;      // slabs hold 8 rows
             const int b_rows = max(0, min(B_ROWS, row_cap - mrow0));
             const uint8_t* src = nullptr;
@@ -219,7 +220,7 @@ __global__ void __launch_bounds__(WT_THREADS, 1) gemm_wh_tc_kernel(const __grid_
     } else if (warp == 1) {
         if (CG == 1 || crank == 0) {
             // ------------------------------------ MMA issuer ------------------------------------
-            const uint32_t idesc = umma_idesc_f16_f32(128 * CG, WT_NT) | (a.bf16 ? ((1u << 7) | (1u << 10)) : 0u);   // a_format = b_format = BF16
+            const uint32_t idesc = umma_idesc_f16_f32(128 * CG, a.nt) | (a.bf16 ? ((1u << 7) | (1u << 10)) : 0u);   // a_format = b_format = BF16
             const uint32_t desc_hi = (2048u >> 4) | (1u << 14);      // SBO 2048 B (8-row groups), descriptor version 1
             uint32_t it = 0, tcount = 0;
             for (int t = cid; t < a.n_tiles; t += ncl) {
@@ -285,8 +286,8 @@ __global__ void __launch_bounds__(WT_THREADS, 1) gemm_wh_tc_kernel(const __grid_
             WtTile w;
             if (!wt_tile(a, t, w)) continue;
             const int rt = w.rp * CG + (int)crank;
-            const int m0 = w.mt * WT_NT;
-            const int Mt = min(WT_NT, w.rows - m0);
+            const int m0 = w.mt * a.nt;
+            const int Mt = min(a.nt, w.rows - m0);
             const uint32_t u = tcount & 1;
             wt_wait(&acc_full[u], (tcount >> 1) & 1, t0);
             tc_fence_after();
@@ -597,6 +598,19 @@ extern "C" int dl_q40t_to_wh(const uint8_t* q40t, int d, int n, uint8_t* wh, voi
     return 0;
 }
 
+// Rows per tile: the width for which the tiles of the busiest CTA (pair) take least time.  Half of a 256-row tile's time stays whatever its rows are (the
+// weights' copies and each stage's hand-off: 768 rows of 4096 x 14336 in one round of tiles of 256 or 192 are 8 % apart), so rows that are not there
+// are saved, and rounds are not added for narrower ones.
+static int wh_tile_rows(int row_units, int M, int slots) {
+    int best = WT_NT;
+    long long least = -1;
+    for (int nt = WT_NT; nt >= 128; nt -= 32) {
+        const long long rounds = ((long long)row_units * ((M + nt - 1) / nt) + slots - 1) / slots, cost = rounds * (nt + 256);
+        if (least < 0 || cost < least) { least = cost; best = nt; }
+    }
+    return best;
+}
+
 // force_cg: bit 0: 0 = pairs when the row-tile count is even, 1 = single CTAs (for tests and comparisons);
 // bit 1: the images hold bf16 (written by dl_wh_from_dense / dl_xh_from_rows) instead of fp16
 static int gemm_wh_launch(const uint8_t* wh, int d, int n, const uint8_t* xh, int ncap, int M, const DlEpilogue* epi,
@@ -611,12 +625,12 @@ static int gemm_wh_launch(const uint8_t* wh, int d, int n, const uint8_t* xh, in
     a.wh = wh; a.xh = xh; a.d_real = d;
     a.row_tiles = (d + 127) / 128;
     a.KT = n / 128; a.ncap = ncap; a.M = M;
-    a.m_tiles = (M + WT_NT - 1) / WT_NT;
-    const int cg = ((force_cg & 1) || (a.row_tiles & 1)) ? 1 : 2;
+    const int cg = ((force_cg & 1) || (a.row_tiles & 1)) ? 1 : 2, n_sms = dl_device_sm_count();
+    a.nt = grp == nullptr ? wh_tile_rows(a.row_tiles / cg, M, n_sms / cg) : WT_NT;      // (groups: their rows are not known here)
+    a.m_tiles = (M + a.nt - 1) / a.nt;
     a.bf16 = (force_cg & 2) ? 1 : 0;
     a.grp = grp; a.n_groups = n_groups; a.wh_group_bytes = wh_group_bytes;
     a.n_tiles = n_groups * (a.row_tiles / cg) * a.m_tiles;
-    const int n_sms = dl_device_sm_count();
     int grid = (n_sms / cg) * cg;
     if (grid > a.n_tiles * cg) grid = a.n_tiles * cg;
     a.n_epi_ctas = grid;
