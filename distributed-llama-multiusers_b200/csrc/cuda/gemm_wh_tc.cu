@@ -388,7 +388,8 @@ extern "C" int dl_device_sm_count();
 #define WS_MAX_NT 128
 #define WS_THREADS 352
 #define WS_MAX_ROWS 256                // output columns per CTA: two accumulators of 128 lanes
-#define WS_PIECE 4                     // row groups (2 KB each) per bulk copy
+#define WS_PIECE 16                    // row groups (2 KB each) per bulk copy: as few copies as the image's tiles allow (32 rows, 4096 x 14336 32.2 us in fours, 26.2 in eights, 25.8 so)
+#define WS_HINT 2                      // stages that are asked for while the previous kernel ends: more only delay its own (78.4 us for all nine, 73.8 for two)
 #define WS_SMEM (208 * 1024)           // ring + what the last stage's MMA reads behind it
 
 struct WsArgs {
@@ -453,7 +454,7 @@ __global__ void __launch_bounds__(WS_THREADS, 1) gemm_wh_rows_kernel(const __gri
             }
         }
         // the weights' first stages are on their way into L2 while the previous kernel ends (a hint: a kernel that still writes them is waited for)
-        for (int i = 0; is_w && i < min(nk, a.NS); i++)
+        for (int i = 0; is_w && i < min(nk, min(a.NS, WS_HINT)); i++)
             asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src + (size_t)i * step), "r"(bytes) : "memory");
         pdl_wait();
         t0 = globaltimer_ns();
@@ -549,7 +550,9 @@ static int gemm_wh_rows_launch(const uint8_t* wh, int d, int n, const uint8_t* x
     a.NS = (WS_SMEM - over) / a.stage;
     if (a.NS > 16) a.NS = 16;
     // A stage must belong to ONE issuer: with an odd count its uses would alternate between the two, and an issuer that runs ahead
-    // would take the parity of the use before last for its own.  Odd counts are those of wide shares, whose bytes cover one issuer.
+    // would take the parity of the use before last for its own.  Two issuers are worth a stage (32 rows, 4096 x 14336: 32.0 us with nine
+    // stages and one issuer, 27.6 with eight and two) until only three are left, of wide shares whose bytes cover one issuer.
+    if (a.NS > 3) a.NS &= ~1;
     a.nacc = a.NS % 2 == 0 ? 2 : 1;
     a.tmem_cols = 32;
     while (a.tmem_cols < 4 * a.NT) a.tmem_cols *= 2;            // two issuers x two tiles

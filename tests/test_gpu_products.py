@@ -1,0 +1,190 @@
+"""Epilogues by whole warps, Q40 expansion, tile widths and the norm's wide form of the Q40 products, and the walk over the states of a gated scan, at
+the sizes where they can go wrong: remainders of tiles and chunks, addresses that are not 16-byte aligned, scales at the ends of fp16."""
+import numpy as np
+import pytest
+import torch
+
+from dllama_b200.ops import quant
+
+pytestmark = pytest.mark.gpu
+
+
+def K():
+    from dllama_b200.ops import kernels
+    return kernels
+
+
+def L():
+    from dllama_b200.ops import layers
+    return layers
+
+
+def _q40(d, n, seed):
+    rng = np.random.default_rng(seed)
+    raw = quant.quantize_q40((rng.standard_normal((d, n)) * 0.05).astype(np.float32))
+    return torch.from_numpy(raw.reshape(-1)).cuda(), quant.dequantize_q40(raw).reshape(d, n)
+
+
+def _activations(n, M, ncap, seed):
+    x = np.random.default_rng(seed).standard_normal((M, n)).astype(np.float32)
+    xh = K().alloc_xh(n, ncap, "cuda")
+    K().quant_q80(torch.from_numpy(x).cuda(), M, n, ncap, None, xh)
+    return quant.q80_roundtrip(x).astype(np.float64), xh
+
+
+@pytest.mark.parametrize("d,n,M,S", [(300, 512, 5, 1), (132, 512, 16, 2), (512, 1024, 33, 4), (256, 512, 70, 2), (388, 512, 128, 4), (38912, 128, 20, 1),
+                                     (38912, 128, 128, 1), (9600, 256, 150, 1), (9600, 256, 430, 1), (130, 512, 9, 1)])
+@pytest.mark.parametrize("roundtrip", [False, True])
+def test_store_epilogue_aligned_or_not(d, n, M, S, roundtrip):
+    """The same values, bit for bit, whether rows start on 16 bytes (four values per thread) or not (one); tiles alone, in pairs, in shares of K and of
+    every width.  Against f64: operands rounded to fp16, sums of n terms."""
+    k = K()
+    ncap = (M + 255) // 256 * 256 if M > 128 else 16 if M <= 16 else 32 if M <= 32 else 64 if M <= 64 else 128
+    w, wdq = _q40(d, n, d + M)
+    w = k.make_q40t(w, d, n)
+    x, xh = _activations(n, M, ncap, M)
+    res = torch.randn(M, d + 3, device="cuda")
+    out = []
+    for shift, ld in ((0, (d + 3) // 4 * 4), (1, d + 3)):
+        buf = torch.full((M * ld + 8,), float("nan"), device="cuda")
+        r = torch.zeros(M * ld + 8, device="cuda")
+        r[shift:shift + M * ld].view(M, ld)[:, :d] = res[:, :d]
+        k.gemm_q40_tc(w, d, n, xh, ncap, M, k.epi_store([buf.data_ptr() + 4 * shift], ld, 0, roundtrip, residual=r.data_ptr() + 4 * shift, residual_ld=ld), S)
+        y = buf[shift:shift + M * ld].view(M, ld)
+        assert torch.isnan(y[:, d:]).all() and not torch.isnan(y[:, :d]).any()
+        out.append(y[:, :d].clone())
+    assert torch.equal(out[0], out[1])
+    want = x @ wdq.T.astype(np.float64)
+    scale = np.abs(want).max()
+    tol = 2e-3 * scale + (scale / 127 if roundtrip else 0)      # a cast of blocks is good to half a step of the block's largest value
+    assert np.abs(out[0].double().cpu().numpy() - res[:, :d].double().cpu().numpy() - want).max() <= tol
+
+
+@pytest.mark.parametrize("d,n,M,force_cg", [(512, 256, 300, 0), (384, 256, 129, 0), (300, 256, 257, 0), (4096, 256, 768, 0), (132, 128, 40, 1)])
+def test_prompt_product_aligned_or_not(d, n, M, force_cg):
+    """As above for the product on expanded weights, whose tiles have 128 to 256 rows."""
+    k = K()
+    ncap = (M + 7) // 8 * 8
+    w, wdq = _q40(d, n, d + M)
+    wh = k.q40t_to_wh(k.make_q40t(w, d, n), d, n)
+    x, xh = _activations(n, M, ncap, M)
+    out = []
+    for shift, ld in ((0, (d + 3) // 4 * 4), (1, d + 1)):
+        buf = torch.full((M * ld + 8,), float("nan"), device="cuda")
+        k.gemm_wh_tc(wh, d, n, xh, ncap, M, k.epi_store([buf.data_ptr() + 4 * shift], ld, 0, False), force_cg)
+        out.append(buf[shift:shift + M * ld].view(M, ld)[:, :d].clone())
+    assert torch.equal(out[0], out[1])
+    want = x @ wdq.T.astype(np.float64)
+    np.testing.assert_allclose(out[0].cpu().numpy(), want, rtol=0, atol=2e-3 * np.abs(want).max())
+
+
+@pytest.mark.parametrize("scales", [(6e-8, 1e-6, 3e-5, 1e-4), (9e-4, 0.0039, 0.03, 0.0624), (0.0624, 0.0625, 0.07, 1.0), (-0.0624, -0.0625, -3.0, 1e-4), (0.0, 2.0, -1e-5, 500.0)])
+def test_q40_expansion_rounds_once(scales):
+    """Every nibble under scales from fp16's subnormals up, on both sides of the largest that one fma takes: (nibble - 8) d rounded once, in the expanded
+    image and in the fused product, which agree."""
+    k = K()
+    d, n, M = 128, 256, 16
+    rng = np.random.default_rng(1)
+    nib = rng.integers(0, 16, (d, n // 32, 32))
+    nib[:, 0, :16], nib[:, 0, 16:] = np.arange(16), np.arange(16)[::-1]
+    sc = np.asarray(scales, dtype=np.float16)[rng.integers(0, len(scales), (d, n // 32))]
+    raw = np.concatenate([sc[..., None].view(np.uint8), (nib[..., :16] | nib[..., 16:] << 4).astype(np.uint8)], axis=2)
+    w = k.make_q40t(torch.from_numpy(raw.reshape(-1)).cuda(), d, n)
+    want = ((nib - 8) * sc[..., None].astype(np.float64)).astype(np.float16).astype(np.float64).reshape(d, n)
+    # unit activations pick the expanded values out one by one: column c of 16 rows at a time
+    got = np.zeros_like(want)
+    wh = k.q40t_to_wh(w, d, n)
+    for c0 in range(0, n, M):
+        x = np.zeros((M, n), dtype=np.float32)
+        x[np.arange(M), c0 + np.arange(M)] = 127.0
+        xh = k.alloc_xh(n, M, "cuda")
+        k.quant_q80(torch.from_numpy(x).cuda(), M, n, M, None, xh)
+        for run in (lambda e: k.gemm_q40_tc(w, d, n, xh, M, M, e, 1), lambda e: k.gemm_wh_tc(wh, d, n, xh, M, M, e, 1)):
+            y = torch.zeros(M, d, device="cuda")
+            run(k.epi_store([y.data_ptr()], d))
+            assert np.array_equal(y.double().cpu().numpy().T, want[:, c0:c0 + M] * 127.0)
+
+
+@pytest.mark.parametrize("M,dim", [(1184, 4096), (1185, 4128), (1191, 8192), (1200, 544)])
+def test_norm_of_many_rows(M, dim):
+    """Eight rows per CTA (from 1184) against a row per CTA: the merged sums bit for bit, the norm but for the order of its sum of squares, the cast
+    but for one step of a block's values (a block's largest below 8); dims beyond what a thread keeps in registers, rows that end inside a CTA."""
+    k = K()
+    ncap = (M + 127) // 128 * 128
+    x, parts, w = torch.randn(M, dim, device="cuda"), torch.randn(2, M, dim, device="cuda"), torch.rand(dim, device="cuda") + 0.5
+    img = []
+    for step in (M, 592):
+        xh, xo, yo = k.alloc_xh((dim + 127) // 128 * 128, ncap, "cuda"), torch.zeros(M, dim, device="cuda"), torch.zeros(M, dim, device="cuda")
+        for m0 in range(0, M, step):
+            m1 = min(M, m0 + step)
+            k.reduce_norm_quant(x[m0:m1], xo[m0:m1], parts[:, m0:m1].contiguous().data_ptr(), 2, (m1 - m0) * dim, None, None, 0, 0, w, 1e-5, dim, m1 - m0, ncap, None,
+                                xh[m0 // 8 * 2048:], yo[m0:m1])
+        img.append((xh.view(torch.float16).float(), xo, yo))
+    (h0, x0, y0), (h1, x1, y1) = img
+    assert torch.equal(x0, x1) and torch.equal(x0, (x + parts[0]) + parts[1])
+    assert ((y0 - y1).abs() <= 1e-6 * y0.abs()).all() and y0.abs().max() < 8
+    assert (h0 - h1).abs().max() <= 8 / 127 * 1.001 and (h0 != h1).float().mean() < 1e-3 and h0.abs().max() > 1
+
+
+@pytest.mark.parametrize("vdim,rows", [(36, [64 * 8 + 1, 200]), (37, [64 * 9, 130]), (128, [64 * 17 + 5, 129])])
+def test_chunked_scan_walks_every_chunk(vdim, rows):
+    """States in pieces of four (vdim % 4 == 0) and one by one, chunks that do not fill the last eight, a fresh and a continued sequence: as token by token.
+    f32 sums in two orders: 1e-5."""
+    lib, H, dim, S = L(), 2, 32, len(rows)
+    g = torch.Generator(device="cuda").manual_seed(vdim)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    M = sum(rows)
+    starts = np.cumsum([0] + rows).tolist()
+    i32 = lambda t: torch.tensor(t, dtype=torch.int32, device="cuda")
+    pos0 = [0, 900]
+    keep = dict(pos=i32([pos0[s] + t for s in range(S) for t in range(rows[s])]), row_seq=i32([s for s in range(S) for _ in range(rows[s])]), seq_start=i32(starts),
+                seq_rows=i32(list(range(M))), seq_slot=i32([1, 0]), seq_pos0=i32(pos0))
+    q, v, f, key = rnd(M, H * dim), rnd(M, H * vdim), rnd(M, H * dim) + 2, rnd(M, H * dim) * dim ** -0.5
+    state = rnd(S, H, dim, vdim)
+    kw = dict(f=f, f_bias=torch.zeros(H * dim, device="cuda"), k=key, gate=lib.GATE_ROOT_SIGMOID, tau=4.0, q_scale=0.3)
+    got = []
+    for chunked in (False, True):
+        y, st = torch.zeros(M, H * vdim, device="cuda"), state.clone()
+        more = {}
+        if chunked:
+            more = dict(max_chunks=(max(rows) + lib.GATED_CHUNK - 1) // lib.GATED_CHUNK, chunk_slots=M // lib.GATED_CHUNK + S,
+                        scratch=torch.full((lib.gated_chunk_floats(M, S, H, dim, vdim),), float("nan"), device="cuda"))
+        lib.gated_scan(lib.mamba_batch(**keep), S, q, v, y, st, H, dim, vdim, **kw, **more)
+        got.append((y.double(), st.double()))
+    for a, b in zip(*got):
+        assert (a - b).norm() <= 1e-5 * a.norm()
+
+
+@pytest.mark.parametrize("dim,vdim,form", [(128, 128, "lower"), (64, 64, "keys"), (33, 36, "keys"), (96, 132, "lower"), (16, 4, "keys"), (128, 200, "lower")])
+@pytest.mark.parametrize("per", [1, 3])
+def test_whole_states_through_shared_memory(dim, vdim, form, per):
+    """A row per sequence, 160 (sequence, head) units and more: states as whole copies, several per CTA, against 64 bits; fresh sequences, slots in another
+    order, widths that leave threads without a column, states of which only one fits (the other kernel); `rows` understated (three rows each all the same).
+    f32 chains of at most 128 terms: 1e-5."""
+    lib, H, S = L(), 4, 90
+    g = torch.Generator(device="cuda").manual_seed(dim * 1000 + vdim)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    M = S * per
+    q, v, f, fb, key, state = rnd(M, H * dim), rnd(M, H * vdim), rnd(M, H * dim), rnd(H * dim), rnd(M, H * dim) * dim ** -0.5, rnd(S, H, dim, vdim)
+    i32 = lambda t: torch.tensor(t, dtype=torch.int32, device="cuda")
+    start, slots = [0 if s % 3 == 0 else 7 for s in range(S)], list(range(S))[::-1]
+    keep = dict(pos=i32([start[m // per] + m % per for m in range(M)]), row_seq=i32([m // per for m in range(M)]), seq_start=i32([s * per for s in range(S + 1)]),
+                seq_rows=i32(list(range(M))), seq_slot=i32(slots), seq_pos0=i32(start))
+    lower = torch.rand(H * dim, generator=g, device="cuda")
+    kw = dict(f=f, f_bias=fb)
+    kw.update(dict(lower=lower, gate=lib.GATE_LOWER, q_silu=True) if form == "lower" else dict(k=key, gate=lib.GATE_ROOT_SIGMOID, tau=4.0, q_scale=0.5))
+    y, st = torch.zeros(M, H * vdim, device="cuda"), state.clone()
+    lib.gated_scan(lib.mamba_batch(**keep), S, q, v, y, st, H, dim, vdim, rows=S, **kw)
+    z = (f + fb).double().view(S, per, H, dim)
+    lo = lower.double().view(H, dim)
+    gate = lo + (1 - lo) * z.sigmoid() if form == "lower" else z.sigmoid() ** 0.25
+    kk = (1 - lo) * (-z).sigmoid() if form == "lower" else key.double().view(S, per, H, dim)
+    qq = torch.nn.functional.silu(q.double()) if form == "lower" else q.double() * 0.5
+    qq, vv = qq.view(S, per, H, dim), v.double().view(S, per, H, vdim)
+    cur = state.double()[slots] * torch.tensor([p != 0 for p in start], device="cuda").view(S, 1, 1, 1)
+    for t in range(per):
+        cur = gate[:, t, :, :, None] * cur + kk[:, t, :, :, None] * vv[:, t, :, None, :]
+        want = torch.einsum("shd,shdv->shv", qq[:, t], cur)
+        got = y.double().view(S, per, H, vdim)[:, t]
+        assert (got - want).norm() <= 1e-5 * want.norm()
+    assert (st.double()[slots] - cur).norm() <= 1e-5 * cur.norm()
