@@ -153,38 +153,3 @@ def test_chunked_scan_walks_every_chunk(vdim, rows):
         got.append((y.double(), st.double()))
     for a, b in zip(*got):
         assert (a - b).norm() <= 1e-5 * a.norm()
-
-
-@pytest.mark.parametrize("dim,vdim,form", [(128, 128, "lower"), (64, 64, "keys"), (33, 36, "keys"), (96, 132, "lower"), (16, 4, "keys"), (128, 200, "lower")])
-@pytest.mark.parametrize("per", [1, 3])
-def test_whole_states_through_shared_memory(dim, vdim, form, per):
-    """A row per sequence, 160 (sequence, head) units and more: states as whole copies, several per CTA, against 64 bits; fresh sequences, slots in another
-    order, widths that leave threads without a column, states of which only one fits (the other kernel); `rows` understated (three rows each all the same).
-    f32 chains of at most 128 terms: 1e-5."""
-    lib, H, S = L(), 4, 90
-    g = torch.Generator(device="cuda").manual_seed(dim * 1000 + vdim)
-    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
-    M = S * per
-    q, v, f, fb, key, state = rnd(M, H * dim), rnd(M, H * vdim), rnd(M, H * dim), rnd(H * dim), rnd(M, H * dim) * dim ** -0.5, rnd(S, H, dim, vdim)
-    i32 = lambda t: torch.tensor(t, dtype=torch.int32, device="cuda")
-    start, slots = [0 if s % 3 == 0 else 7 for s in range(S)], list(range(S))[::-1]
-    keep = dict(pos=i32([start[m // per] + m % per for m in range(M)]), row_seq=i32([m // per for m in range(M)]), seq_start=i32([s * per for s in range(S + 1)]),
-                seq_rows=i32(list(range(M))), seq_slot=i32(slots), seq_pos0=i32(start))
-    lower = torch.rand(H * dim, generator=g, device="cuda")
-    kw = dict(f=f, f_bias=fb)
-    kw.update(dict(lower=lower, gate=lib.GATE_LOWER, q_silu=True) if form == "lower" else dict(k=key, gate=lib.GATE_ROOT_SIGMOID, tau=4.0, q_scale=0.5))
-    y, st = torch.zeros(M, H * vdim, device="cuda"), state.clone()
-    lib.gated_scan(lib.mamba_batch(**keep), S, q, v, y, st, H, dim, vdim, rows=S, **kw)
-    z = (f + fb).double().view(S, per, H, dim)
-    lo = lower.double().view(H, dim)
-    gate = lo + (1 - lo) * z.sigmoid() if form == "lower" else z.sigmoid() ** 0.25
-    kk = (1 - lo) * (-z).sigmoid() if form == "lower" else key.double().view(S, per, H, dim)
-    qq = torch.nn.functional.silu(q.double()) if form == "lower" else q.double() * 0.5
-    qq, vv = qq.view(S, per, H, dim), v.double().view(S, per, H, vdim)
-    cur = state.double()[slots] * torch.tensor([p != 0 for p in start], device="cuda").view(S, 1, 1, 1)
-    for t in range(per):
-        cur = gate[:, t, :, :, None] * cur + kk[:, t, :, :, None] * vv[:, t, :, None, :]
-        want = torch.einsum("shd,shdv->shv", qq[:, t], cur)
-        got = y.double().view(S, per, H, vdim)[:, t]
-        assert (got - want).norm() <= 1e-5 * want.norm()
-    assert (st.double()[slots] - cur).norm() <= 1e-5 * cur.norm()
