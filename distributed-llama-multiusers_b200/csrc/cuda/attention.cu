@@ -374,11 +374,10 @@ DL_DEVINL void am_split(float v0, float v1, bool lower, uint32_t& top, uint32_t&
     bot = lower ? 0u : h3;
 }
 
-template <int HS>
+template <int HS, int ST>             // ST: ring stages (16 tokens) per warp
 __global__ void __launch_bounds__(ATT_WARPS * 32, 3) attention_mma_kernel(const __grid_constant__ AttArgs a) {
     constexpr int ROWB = HS * 2, CH = ROWB / 16;               // bytes / 16-byte chunks of a token's line
     constexpr int HALF = AM_TOK * ROWB;                        // K (or V) of a half page
-    constexpr int ST = HS == 128 ? 2 : 4;                      // ring stages per warp (16 KB)
     constexpr int KS = HS / 16, NT = HS / 8;
     extern __shared__ __align__(128) uint8_t smem[];
     trace_begin(a.tr);
@@ -700,13 +699,13 @@ static int launch_att(const AttArgs& a, int pdl, cudaStream_t stream) {
     return 0;
 }
 
-template <int HS>
-static int launch_att_mma(const AttArgs& a, int pdl, cudaStream_t stream) {
-    constexpr int smem = ATT_WARPS * 16 * 1024;
+template <int HS, int ST>
+static int launch_att_mma_st(const AttArgs& a, int pdl, cudaStream_t stream) {
+    constexpr int smem = ATT_WARPS * ST * AM_TOK * HS * 4;
     static_assert(ATT_WARPS * 4 * (HS + 2) * 4 + 4 <= smem, "the merge fits the ring");
     static bool attr_set = false;
     if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(attention_mma_kernel<HS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        cudaError_t e = cudaFuncSetAttribute(attention_mma_kernel<HS, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) { dl_set_error("attention smem attr: %s", cudaGetErrorString(e)); return -(int)e; }
         attr_set = true;
     }
@@ -722,9 +721,24 @@ static int launch_att_mma(const AttArgs& a, int pdl, cudaStream_t stream) {
         cfg.attrs = attr;
         cfg.numAttrs = 1;
     }
-    cudaError_t e = cudaLaunchKernelEx(&cfg, attention_mma_kernel<HS>, a);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, attention_mma_kernel<HS, ST>, a);
     if (e != cudaSuccess) { dl_set_error("attention launch: %s", cudaGetErrorString(e)); return -(int)e; }
     return 0;
+}
+
+// Stages by how many CTAs an SM gets, for heads of 128: 64 KB of rings where three share it, 96 for two and 128 for one, so that as much is on its way (us with
+// two stages and so: 16 rows of 1500 to 3000 tokens 38.9 and 35.4, 8 rows 25.1 and 23.9, 32 rows, two CTAs, 55.2 and 55.0; a step of width 4096 and 4 layers
+// behind 200 to 400 tokens, 8 rows 320.6 and 313.0, 32 rows 356 and 352).  With CTAs for half the SMs or fewer a warp has two or three stages in all, and the
+// larger ring only keeps the next kernel's CTAs out (one row 211.4 and 212.9); heads of 64 gain nothing.
+template <int HS>
+static int launch_att_mma(const AttArgs& a, int pdl, cudaStream_t stream) {
+    if constexpr (HS == 128) {
+        const long long ctas = (long long)a.n_splits * a.n_kv_heads * a.M;
+        const int n_sms = dl_device_sm_count();
+        if (ctas > n_sms / 2 && ctas <= n_sms) return launch_att_mma_st<HS, 4>(a, pdl, stream);
+        if (ctas > n_sms && ctas <= 2ll * n_sms) return launch_att_mma_st<HS, 3>(a, pdl, stream);
+    }
+    return launch_att_mma_st<HS, 256 / HS>(a, pdl, stream);
 }
 
 template <int HS, typename KV>

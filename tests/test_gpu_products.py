@@ -153,3 +153,29 @@ def test_chunked_scan_walks_every_chunk(vdim, rows):
         got.append((y.double(), st.double()))
     for a, b in zip(*got):
         assert (a - b).norm() <= 1e-5 * a.norm()
+
+
+@pytest.mark.parametrize("rows,splits", [(1, 1), (5, 2), (9, 1), (18, 1), (19, 1), (37, 1), (38, 1)])
+def test_decode_attention_by_ring_depth(rows, splits):
+    """Heads of 128 with two, three and four stages per warp (CTAs for up to half, one or two of the SMs' worth, more): contexts of 1 to 700 tokens, which end
+    inside a half page and leave warps without one.  Against 64 bits: f32 sums on an fp16 cache, 1e-5."""
+    k, G, H, hs = K(), 8, 32, 128
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    pos = [int(p) for p in np.random.default_rng(rows).integers(0, 700, rows)]
+    pos[0] = 0 if rows > 1 else 333
+    pages = [(p + 32) // 32 for p in pos]
+    bt = torch.zeros(rows, max(pages), dtype=torch.int32, device="cuda")
+    perm, at = torch.randperm(sum(pages), generator=g, device="cuda", dtype=torch.int32), 0
+    for i, n in enumerate(pages):
+        bt[i, :n] = perm[at:at + n]
+        at += n
+    kc, vc = (torch.randn(at, G, 32, hs, generator=g, device="cuda").half() for _ in range(2))
+    q, y = torch.randn(rows, H * hs, generator=g, device="cuda"), torch.zeros(rows, H * hs, device="cuda")
+    scratch = torch.zeros(k.attention_scratch_bytes(rows, H, hs, splits), dtype=torch.uint8, device="cuda")
+    i32 = lambda t: torch.tensor(t, dtype=torch.int32, device="cuda")
+    k.attention(q, rows, H, G, hs, kc, vc, i32(pos), i32(list(range(rows))), bt, bt.shape[1], splits, scratch, None, None, rows, y_out=y)
+    for i, p in enumerate(pos):
+        kk, vv = (c[bt[i, :pages[i]].long()].double().transpose(1, 2).reshape(-1, G, hs)[:p + 1] for c in (kc, vc))
+        s = torch.einsum("ghd,tgd->ght", q[i].double().view(G, H // G, hs), kk) * hs ** -0.5
+        want = torch.einsum("ght,tgd->ghd", s.softmax(dim=-1), vv).reshape(-1)
+        assert (y[i].double() - want).norm() <= 1e-5 * want.norm()
