@@ -155,14 +155,6 @@ DL_DEVINL void mbar_wait(uint64_t* bar, uint32_t parity) {
     }
 }
 
-// wait with a sleep between probes: for roles that share an SM sub-partition with busy math warps, so
-// their polling does not eat the issue slots (costs up to `ns` of wake-up latency)
-DL_DEVINL void mbar_wait_sleep(uint64_t* bar, uint32_t parity, uint32_t ns) {
-    while (!mbar_try_wait(bar, parity)) {
-        if (ns) __nanosleep(ns);
-    }
-}
-
 // ---- cluster-scope variants (DSMEM hand-off between the CTAs of a thread-block cluster) ----
 DL_DEVINL uint32_t mapa_shared(uint32_t cta_smem_addr, uint32_t cta_rank) {
     uint32_t r;
@@ -172,9 +164,6 @@ DL_DEVINL uint32_t mapa_shared(uint32_t cta_smem_addr, uint32_t cta_rank) {
 // arrive (release, cluster scope) on an mbarrier that lives in another CTA of the cluster
 DL_DEVINL void mbar_arrive_remote(uint32_t cluster_smem_addr) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_smem_addr) : "memory");
-}
-DL_DEVINL void st_shared_cluster_f32(uint32_t cluster_smem_addr, float v) {
-    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(cluster_smem_addr), "f"(v) : "memory");
 }
 // "every CTA of the cluster has started and initialised its barriers" (mbar_fence_init), announced early and waited for ahead of the first remote
 // access: all threads call both
@@ -202,7 +191,6 @@ DL_DEVINL void mbar_wait_cluster(uint64_t* bar, uint32_t parity) {
             : "memory");
     } while (!ok);
 }
-DL_DEVINL void fence_acq_rel_cluster() { asm volatile("fence.acq_rel.cluster;" ::: "memory"); }
 
 // generic-proxy smem writes -> visible to the async proxy (bulk copy engine, tcgen05.mma)
 DL_DEVINL void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }

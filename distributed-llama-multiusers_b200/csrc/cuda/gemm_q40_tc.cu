@@ -22,7 +22,9 @@
 //                quarter, thread = weight row: LDS.128 x4 -> packed fp16x2 registers -> tcgen05.st.32x32b.x16
 //   warps 2-17   (again) epilogue: tcgen05.ld TMEM -> registers -> smem tile -> fused epilogue (rows split 4 ways)
 // TMEM columns: nacc f32 accumulators of NT columns from column 0, nstg 64-column A stages at the top
-// (nacc*NT + 64*nstg <= 512: 4 acc + 6 stages for NT <= 32, 2 + 6 for NT = 64, 2 + 4 for 128, 1 + 4 for 256).
+// (nacc*NT + 64*nstg <= 512: 2 accumulators + 6 stages up to NT = 64, 2 + 4 for 128, 1 + 4 above).
+// What bounds narrow tiles: the dequantisers' stores into tensor memory and their instructions (a k-tile 474 clk; 322, HBM's pace for 112 CTAs, without the
+// stores, 395 without the arithmetic).
 // Pipelines: raw ring (producer -> dequant), B ring (producer -> MMA), A stages (dequant -> MMA,
 // released by tcgen05.commit), accumulator barrier (MMA -> epilogue).  K can be split over a
 // thread-block cluster (DSMEM reduction) when there are too few row tiles to fill the chip.

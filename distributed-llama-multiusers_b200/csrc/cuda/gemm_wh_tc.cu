@@ -10,10 +10,11 @@
 //      fused kernel (ALU pipe 50 %, tensor pipe 14 % at 32 rows of w13), which every M tile
 //      repeated -- is paid once per weight instead of once per 256 activation rows.
 //
-// gemm_wh_tc_kernel<2> pairs two CTAs (cluster of 2 = one TPC) on a 256 weight rows x 256 activation rows tile with
+// gemm_wh_tc_kernel<2> pairs two CTAs (cluster of 2 = one TPC) on a 256 weight rows x up to 256 activation rows tile with
 // `tcgen05.mma.cta_group::2`: each CTA stages its own 128 weight rows and HALF of the activation rows (64 KB per
-// 128-wide k step and CTA instead of 96 KB), which is what keeps the L2 -> shared-memory feed (about 43 B/clk per SM)
-// below the tensor pipe's appetite.  gemm_wh_tc_kernel<1> is the single-CTA variant (odd row-tile counts).
+// 128-wide k step and CTA instead of 96 KB).  gemm_wh_tc_kernel<1> is the single-CTA variant (odd row-tile counts).
+// What bounds it: the MMAs under the power limit (28672 x 4096 at 2048 rows 313 us, 301 without its epilogues, 166 without MMAs, whose copies
+// then run at 85 B/clk and SM; cuBLAS 348).
 //
 // Grouped mode: the same kernel runs one product per group of rows against that group's own weights (the experts of a
 // routed feed-forward: rows sorted by expert, segment bounds in device memory), so all experts are ONE launch and the
@@ -23,7 +24,7 @@
 // weight panel in L2); each CTA owns 128 TMEM lanes x 2 accumulators of 256 columns, so the epilogue of tile i
 // (TMEM -> registers -> smem chunk -> the shared fused epilogues of epilogue.cuh) overlaps the MMAs of tile i+1.
 //
-// Warp roles (576 threads): warp 0 producer (4-6 lanes issue one 16 KB bulk copy each per stage), warp 1 MMA issuer + TMEM owner (in the
+// Warp roles (576 threads): warp 0 producer (a converged warp, 4-6 of its lanes a 16 KB bulk copy each per stage), warp 1 MMA issuer + TMEM owner (in the
 // second CTA of a pair: forwards "my half of the stage has landed" to the leader's barrier), warps 2-17 epilogue.
 // Reference semantics: matmul_Q80_Q40_F32 (src/nn/nn-cpu-ops.cpp:352-377), llamafile sgemm (src/nn/llamafile/sgemm.cpp:593-783).
 #include "epilogue.cuh"
@@ -376,7 +377,7 @@ extern "C" int dl_device_sm_count();
 //
 // What bounds it: the weights' bytes.  The 256 x 256 pair tiles above give a 4096-wide output 16 of the 74 pairs, and 28672
 // columns 112 tiles in two waves: norm, gate|up and down of 4096 x 14336 in bf16 at 32 rows took 184 us, 1.9 TB/s
-// (here 86: 47 and 35 us for the products, 5.0 and 3.3 TB/s; 79.5 with the launches chained).  Here the OUTPUT
+// (74 here, the launches chained: 42.4 and 25.3 us for the products alone, 5.5 and 4.6 TB/s).  Here the OUTPUT
 // COLUMNS are dealt to all SMs in groups of 8 (one core-matrix row group of the weight image, 2 KB per k tile), so every SM
 // streams the same number of bytes to within 8 rows; a CTA walks the whole K (or its share of a cluster's) once through a
 // ring of bulk copies, MMA M = 128 with the rows past its share reading whatever lies behind (those accumulator lanes are
@@ -529,7 +530,7 @@ __global__ void __launch_bounds__(WS_THREADS, 1) gemm_wh_rows_kernel(const __gri
 }
 
 // CTAs per cluster that share K: shares of fewer than 5 row groups (40 columns) leave an SM more activations than weights to read and
-// too many k tiles to walk; a pair halves both (32 rows, us with 1 / 2 / 4: 4096 x 14336 45 / 35 / 44, 2048 x 8192 36 / 19 / 29, 128 x 2048
+// too many k tiles to walk; a pair halves both (32 rows, us with 1 / 2 / 4: 4096 x 14336 41 / 25 / 38, 2048 x 8192 24 / 16 / 22, 128 x 2048
 // 11 / 10 / 10; but 6144 x 2048 at 100 rows 21 / 21 / 41, 16384 x 2048 19 / 25 / 41, 28672 x 4096 47 / 60 / 82)
 static int ws_split(int R8, int KT, int n_sms) { return R8 < 5 * n_sms && KT >= 2 ? 2 : 1; }
 
