@@ -19,7 +19,8 @@ PAGE_SIZE = 32
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    # the handle of torch.cuda.current_stream() without the object around it (3.2 us and 0.3, of 9 us that a wrapper took)
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def _p(t: Optional[torch.Tensor]) -> Optional[int]:

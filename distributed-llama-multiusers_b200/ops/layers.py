@@ -10,6 +10,7 @@ from typing import Optional
 import torch
 
 from . import lib
+from .kernels import _stream
 from .lib import (DENSE_GLU_CLAMP, DENSE_GLU_GELU, DENSE_GLU_SILU, DENSE_MUL, DENSE_RELU2, DENSE_ROWGATE_ADD, DENSE_SCALE, DENSE_SIGMOID_MUL, DENSE_SILU, DENSE_SOFTCAP, DENSE_STORE,  # noqa: F401
                   DENSE_XIELU, EPI_DENSE, GATE_EXP_EXP, GATE_LOWER, GATE_ROOT_SIGMOID, GATE_SOFTPLUS, T_BF16, T_F32,
                   DlConvArgs, DlDenseArgs, DlEpilogue, DlGatedArgs, DlHeadNormArgs, DlHyperArgs, DlLatentAttnArgs, DlLightningArgs, DlLatentKvArgs, DlLatentTiles, DlMambaBatch, DlMambaChunks, DlMambaScanArgs, DlMoeArgs,
@@ -17,10 +18,6 @@ from .lib import (DENSE_GLU_CLAMP, DENSE_GLU_GELU, DENSE_GLU_SILU, DENSE_MUL, DE
 
 PAGE_SIZE = 32
 HC_MAX_STREAMS = 16          # DL_HC_MAX_STREAMS of the hyper-connection kernel
-
-
-def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
 
 
 def _p(t: Optional[torch.Tensor]) -> Optional[int]:
