@@ -442,6 +442,185 @@ static void launch_dense_mma(const DlDenseArgs& a, cudaStream_t st, int n_sms) {
     else launch_dense_mma_t<NT, 1>(a, st);
 }
 
+// ------------------------------------------------------------------------------------------------
+// One row (or two) against bf16 weights whose rows lie behind one another, activations rounded to bf16: a CTA per SM streams an equal run of weight rows through a
+// ring of bulk copies.  A warp keeps its inputs in registers for the whole run: all of up to 2048 (stages of four weight rows, a warp takes one, or both of a gated
+// unit, and stores it), or a slice of 2048 of one row (stages of two rows up to 4096 inputs, else of one; the slices meet in shared memory when the run is
+// over).  Groups of warps take stages in turn; no warp waits for another before the end.  A lane's products of a slice are added in the order of the kernels above.
+//
+// What bounds it: the weights' bytes.  The kernels above hold them in registers, two CTAs an SM, and start again every 8 columns.  Cold weights, us, they and
+// this: one row, 16384 x 2048 in pairs 15.1 and 12.7, 8192 x 2048 11.2 and 8.6, 32768 x 2048 27.9 and 23.6, 28672 x 4096 in pairs 40.5 and 37.0 (6.3 TB/s), 4096 x
+// 4096 9.6 and 8.0, 2048 x 8192 8.5 and 8.0, 4096 x 14336 24.7 and 20.7; two rows, 16384 x 2048 in pairs 18.5 and 13.7, 4096 x 4096 17.6 and 11.4.
+// ------------------------------------------------------------------------------------------------
+#define DR_K 2048                      // inputs of a warp
+#define DR_STAGES 24                   // at most
+#define DR_RING (192 * 1024)
+#define DR_PART (16 * 1024)
+#define DR_DEADLINE_NS 4000000000ull
+// rows per stage, warps per row (slices of DR_K inputs), warps per stage, groups of them, stages of the ring
+struct DenseRing { DlDenseArgs a; int rows, slices, group, groups, stages; };
+
+// false after the limit (once one wait has run out, at once)
+__device__ __forceinline__ bool dense_ring_wait(uint64_t* bar, uint32_t parity, volatile int* dead) {
+    unsigned long long t0 = 0, t;
+    for (unsigned n = 0;; ++n) {
+        uint32_t ok;
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"((uint32_t)__cvta_generic_to_shared(bar)), "r"(parity) : "memory");
+        if (ok) return true;
+        if ((n & 0xFFu) == 0xFFu) {
+            asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+            if (t0 == 0) t0 = t;
+            if (*dead || t - t0 > DR_DEADLINE_NS) { *dead = 1; return false; }
+        }
+    }
+}
+// consumers (two rows of activations: their inputs leave registers for eight); one more warp copies
+static __host__ __device__ constexpr int dense_ring_warps(int MT, bool pair, bool sliced) { return MT == 2 ? 8 : pair && !sliced ? 12 : 16; }
+template <int MT, bool PAIR, bool SLICED>
+__global__ void __launch_bounds__((dense_ring_warps(MT, PAIR, SLICED) + 1) * 32, 1) dense_ring_kernel(DenseRing g) {
+    constexpr int WARPS = dense_ring_warps(MT, PAIR, SLICED), RW = PAIR && !SLICED ? 2 : 1;      // RW: rows of a stage per warp
+    const DlDenseArgs& a = g.a;
+    extern __shared__ __align__(128) uint8_t ring[];
+    __shared__ uint64_t full[DR_STAGES], empty[DR_STAGES];
+    __shared__ int dead;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t row_bytes = a.K * 2, stage_bytes = row_bytes * g.rows;
+    // this CTA's stages
+    const int all = (a.N + g.rows - 1) / g.rows, t0 = (int)((long long)all * blockIdx.x / gridDim.x), nt = (int)((long long)all * (blockIdx.x + 1) / gridDim.x) - t0;
+    const __nv_bfloat16* w = (const __nv_bfloat16*)a.W + (size_t)t0 * g.rows * a.K;
+    auto rows_of = [&](int t) { return min(g.rows, a.N - (t0 + t) * g.rows); };
+    if (threadIdx.x == 0) {
+        dead = 0;
+        for (int s = 0; s < g.stages; ++s) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((uint32_t)__cvta_generic_to_shared(&full[s])) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"((uint32_t)__cvta_generic_to_shared(&empty[s])), "r"(g.group) : "memory");
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (warp == WARPS && lane < 2 && lane < nt)      // the first weights are on their way into L2 while the previous kernel ends
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(w + (size_t)lane * g.rows * a.K), "r"(row_bytes * rows_of(lane)) : "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (warp == WARPS) {
+        if (lane == 0)
+            for (int t = 0; t < nt; ++t) {
+                const int s = t % g.stages;
+                if (t >= g.stages && !dense_ring_wait(&empty[s], ((t / g.stages) & 1) ^ 1, &dead)) break;
+                const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&full[s]), bytes = row_bytes * rows_of(t);
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"((uint32_t)__cvta_generic_to_shared(ring + (size_t)s * stage_bytes)), "l"(w + (size_t)t * g.rows * a.K), "r"(bytes), "r"(bar) : "memory");
+            }
+        return;
+    }
+    const int grp = warp / g.group, wi = warp - grp * g.group, slice = SLICED ? wi % g.slices : 0, row = SLICED ? wi / g.slices : wi * RW, k0 = slice * DR_K + lane * 8;
+    float* part = reinterpret_cast<float*>(ring + (size_t)g.stages * stage_bytes);      // SLICED: [this CTA's rows][slices][MT]
+    float x[MT][DR_K / 32];
+#pragma unroll
+    for (int i = 0; i < DR_K / 256; ++i) {
+#pragma unroll
+        for (int m = 0; m < MT; ++m) {
+            WVec<float> v = {};
+            if (k0 + i * 256 < a.K) v.load(a.X + (size_t)m * a.ldx + k0 + i * 256);
+            float f[8];
+            v.get(f);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) x[m][i * 8 + j] = round_bf16(f[j]);
+        }
+    }
+    for (int t = grp; grp < g.groups && t < nt; t += g.groups) {
+        const int s = t % g.stages, n = (t0 + t) * g.rows + row;
+        const bool ok = dense_ring_wait(&full[s], (t / g.stages) & 1, &dead);
+        float acc[MT][RW];
+#pragma unroll
+        for (int m = 0; m < MT; ++m)
+#pragma unroll
+            for (int r = 0; r < RW; ++r) acc[m][r] = ok ? 0.f : __int_as_float(0x7fc00000);
+        if (ok && n + RW <= a.N) {               // (pairs: N is even)
+            const uint8_t* base = ring + (size_t)s * stage_bytes + (size_t)row * row_bytes + k0 * 2;
+#pragma unroll
+            for (int i = 0; i < DR_K / 256; ++i)
+                if (k0 + i * 256 < a.K) {
+#pragma unroll
+                    for (int r = 0; r < RW; ++r) {
+                        WVec<__nv_bfloat16> v;
+                        v.u = *reinterpret_cast<const uint4*>(base + r * row_bytes + i * 512);
+                        float f[8];
+                        v.get(f);
+#pragma unroll
+                        for (int m = 0; m < MT; ++m)
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) acc[m][r] = fmaf(x[m][i * 8 + j], f[j], acc[m][r]);
+                    }
+                }
+        }
+        __syncwarp();
+        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"((uint32_t)__cvta_generic_to_shared(&empty[s])) : "memory");
+#pragma unroll
+        for (int m = 0; m < MT; ++m)
+#pragma unroll
+            for (int r = 0; r < RW; ++r) acc[m][r] = warp_sum(acc[m][r]);
+        if (lane == 0 && n + RW <= a.N) {
+#pragma unroll
+            for (int m = 0; m < MT; ++m) {
+                if (SLICED) part[((t * g.rows + row) * g.slices + slice) * MT + m] = acc[m][0];
+                else if (PAIR) dense_store_pair(a, 0, m, n >> 1, acc[m][0], acc[m][RW - 1]);
+                else dense_store(a, 0, m, n, acc[m][0]);
+            }
+        }
+    }
+    if (!SLICED) return;
+    asm volatile("bar.sync 1, %0;" ::"n"(WARPS * 32) : "memory");
+    const int n0 = t0 * g.rows, rows = min(nt * g.rows, a.N - n0);
+    auto sum = [&](int r, int m) {
+        float v = part[r * g.slices * MT + m];
+        for (int k = 1; k < g.slices; ++k) v += part[(r * g.slices + k) * MT + m];
+        return v;
+    };
+    const int outs = PAIR ? rows / 2 : rows;
+    for (int i = threadIdx.x; i < outs * MT; i += WARPS * 32) {
+        const int m = i / outs, r = i - m * outs;
+        if (PAIR) dense_store_pair(a, 0, m, (n0 >> 1) + r, sum(2 * r, m), sum(2 * r + 1, m));
+        else dense_store(a, 0, m, n0 + r, sum(r, m));
+    }
+}
+// From 1025 inputs and 12 Mi weights on (us, the kernels above and this: 65536 x 1024 30.4 and 32.8, 2048 x 2048 3.4 and 4.8, 2048 x 4096 5.2 and 5.9, 6144 x 2048 7.3 and
+// 7.4, 3072 x 4096 8.9 and 6.9); two rows, whose inputs leave registers for eight warps, where a warp has few bytes to multiply twice (28672 x 4096 in pairs 47.1
+// and 52.6, 2048 x 8192 12.0 and 12.4).
+static bool dense_ring(const DlDenseArgs& a, int n_sms, DenseRing& g) {
+    if (a.M > 2 || a.batch != 1 || a.ldw != a.K || a.K <= DR_K / 2 || a.K > 8 * DR_K || (long long)a.N * a.K < 12ll << 20) return false;
+    if (a.M == 2 && a.K > (a.epi == DL_DENSE_GLU_GELU ? DR_K : 2 * DR_K)) return false;
+    const bool pair = a.epi == DL_DENSE_GLU_GELU;
+    g.a = a;
+    g.slices = (a.K + DR_K - 1) / DR_K;
+    g.rows = g.slices == 1 ? 4 : g.slices == 2 ? 2 : 1;
+    if (pair && g.rows == 1) return false;
+    g.group = g.slices == 1 && pair ? 2 : g.rows * g.slices;
+    g.groups = dense_ring_warps(a.M, pair, g.slices > 1) / g.group;
+    const int fit = (int)(DR_RING / ((long long)a.K * 2 * g.rows)), n_stages = (a.N + g.rows - 1) / g.rows;
+    g.stages = (fit < DR_STAGES ? fit : DR_STAGES) / g.groups * g.groups;          // a stage belongs to one group: a wait cannot see a phase before the last
+    return g.stages >= g.groups && (g.slices == 1 || ((long long)n_stages / n_sms + 1) * g.rows * g.slices * a.M * 4 <= DR_PART);
+}
+template <int MT, bool PAIR, bool SLICED>
+static void launch_dense_ring_t(const DenseRing& g, cudaStream_t st, int n_sms) {
+    static bool set = false;
+    if (!set) {
+        cudaFuncSetAttribute(dense_ring_kernel<MT, PAIR, SLICED>, cudaFuncAttributeMaxDynamicSharedMemorySize, DR_RING + DR_PART);
+        set = true;
+    }
+    launch_after(dense_ring_kernel<MT, PAIR, SLICED>, dim3(n_sms), (dense_ring_warps(MT, PAIR, SLICED) + 1) * 32, st, g, (size_t)g.stages * g.rows * g.a.K * 2 + (SLICED ? DR_PART : 0));
+}
+template <int MT>
+static void launch_dense_ring(const DenseRing& g, cudaStream_t st, int n_sms) {
+    if (g.a.epi == DL_DENSE_GLU_GELU) {
+        if (g.slices == 1) launch_dense_ring_t<MT, true, false>(g, st, n_sms);
+        else launch_dense_ring_t<MT, true, true>(g, st, n_sms);
+    } else {
+        if (g.slices == 1) launch_dense_ring_t<MT, false, false>(g, st, n_sms);
+        else launch_dense_ring_t<MT, false, true>(g, st, n_sms);
+    }
+}
+
 // paired columns (GLU): one warp per value, its gate row and its up row side by side
 template <typename WT, int MT, bool RX>
 __global__ void __launch_bounds__(GV_WARPS * 32) dense_gemv_pair_kernel(DlDenseArgs a) {
@@ -604,6 +783,14 @@ static void launch_dense(const DlDenseArgs& a, cudaStream_t st) {
             if (a.M <= 8) launch_dense_mma<1>(a, st, n_sms);
             else if (a.M <= 16) launch_dense_mma<2>(a, st, n_sms);
             else launch_dense_mma<4>(a, st, n_sms);
+            return;
+        }
+    }
+    if constexpr (sizeof(WT) == 2 && RX) {
+        DenseRing g;
+        if (vec && dense_ring(a, n_sms, g)) {
+            if (a.M == 1) launch_dense_ring<1>(g, st, n_sms);
+            else launch_dense_ring<2>(g, st, n_sms);
             return;
         }
     }

@@ -179,3 +179,25 @@ def test_decode_attention_by_ring_depth(rows, splits):
         s = torch.einsum("ghd,tgd->ght", q[i].double().view(G, H // G, hs), kk) * hs ** -0.5
         want = torch.einsum("ght,tgd->ghd", s.softmax(dim=-1), vv).reshape(-1)
         assert (y[i].double() - want).norm() <= 1e-5 * want.norm()
+
+
+@pytest.mark.parametrize("M,N,K_,epi", [(1, 12290, 1032, "store"), (1, 6147, 2048, "store"), (1, 6146, 2048, "pair"), (1, 12000, 1096, "pair"), (1, 3076, 4096, "pair"), (1, 4099, 3080, "store"),
+                                        (1, 2501, 5040, "store"), (1, 1000, 14336, "store"), (1, 769, 16384, "store"), (1, 2100, 6152, "gate"), (2, 6147, 2048, "store"),
+                                        (2, 6146, 2048, "pair"), (2, 3073, 4096, "store"), (2, 5001, 2600, "gate")])
+def test_rows_through_the_ring(M, N, K_, epi):
+    """One and two rows of enough weights for the ring of bulk copies: rows, pairs and slices that end inside a stage or a warp's share, columns that the SMs do not divide, an
+    output with a stride, epilogues that read.  Against 64 bits: bf16 operands, f32 sums of up to 16384 terms, 1e-6 of the result's norm."""
+    lib = L()
+    g = torch.Generator(device="cuda").manual_seed(N)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    w, x = (rnd(N, K_) * K_ ** -0.5).bfloat16(), rnd(M, K_)
+    cols = N // 2 if epi == "pair" else N
+    buf, aux = torch.full((M, cols + 5), 3.0, device="cuda"), rnd(M, N)
+    y = buf[:, :cols]
+    lib.dense(w, x, y, M, True, **dict(store={}, pair=dict(epi=lib.DENSE_GLU_GELU), gate=dict(epi=lib.DENSE_SIGMOID_MUL, aux=aux))[epi])
+    want = x.bfloat16().double() @ w.double().t()
+    if epi == "pair":
+        want = torch.nn.functional.gelu(want[:, 0::2], approximate="tanh") * want[:, 1::2]
+    if epi == "gate":
+        want = aux.double() * want.sigmoid()
+    assert (y.double() - want).norm() <= 1e-6 * want.norm() and (buf[:, cols:] == 3).all()
