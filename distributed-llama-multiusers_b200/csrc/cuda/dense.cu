@@ -4,7 +4,8 @@
 // (dense_in_rounds), take a shared-memory tiled kernel.  All take a batch dimension
 // (grid.z) with element strides, which is how per-head products (a head's slice of a weight against a head's slice
 // of the activations) run as one launch.  In bf16 mode (`round_x`) the activation operand is rounded to bf16 on
-// load, so products are exact in f32 and only the accumulation differs between the kernels.
+// load, so products are exact in f32 and only the accumulation differs between the kernels; one and two rows of enough weights stream them
+// through a ring in shared memory (dense_ring).
 //
 // Epilogues (what other models of this library fuse into their matmul kernels too): plain store, relu(.)^2,
 // aux * sigmoid(.) (an output gate), cap * tanh(. / cap) (logit soft-capping), . * sigmoid(.) (SiLU), aux * (.) (the second
@@ -283,18 +284,21 @@ __global__ void __launch_bounds__(GV_WARPS * 32) dense_gemv_vec_kernel(DlDenseAr
 //
 // What bounds it: the weights' bytes.  On CUDA cores every row adds 8 FMAs per 16 bytes of weights and lane, and from 9 rows the tiles
 // below (16 K steps of scalar loads) left the weights behind entirely: gate|up + down of 4096 x 14336 took 441 us at 8 rows and
-// 3150 us at 16; 118 and 145 us here.  (Two rows are faster one by one: 2048 x 8192, 39.5 us there, 43.3 here.)
+// 3150 us at 16; 79 and 117 us here.  (Two rows are faster one by one: 2048 x 8192, 12.0 us there, 13.3 here.)
 //
-// Weights go from global memory straight into the A fragments: a lane's 16 bytes are 8 consecutive inputs of row g, and the four pairs
-// fill k slots of two MMAs; the activations' 16 bytes of the same inputs fill the same slots, so no shuffle and no shared memory for the
-// weights.  A CTA owns 16 C columns; its eight warps split K, each staging its own activations (bf16, 128 inputs at a time), and meet in
+// A lane's 16 bytes of weights are 8 consecutive inputs of row g, and the four pairs fill k slots of two MMAs; the activations' 16 bytes of the same
+// inputs fill the same slots, so no shuffle.  A lane copies its weights into places of its own in shared memory (cp.async), one to three halves of a
+// step ahead of the half that it multiplies, so nobody waits for anybody; held in registers, half a step ahead, they took 128 of them, one CTA an SM and
+// 4 TB/s.  Activations of the next step wait in registers, as many rows as leave the CTAs their places.  Registers and now, us, cold weights: 28672 x 4096 in pairs,
+// 3 rows 68 and 47, 8 rows 74 and 50, 16 rows 84 and 76, 24 rows 123 and 114; 4096 x 14336, 3 rows 34.5 and 24.3, 16 rows 56 and 38, 24 rows 84 and 69; 2048 x 8192, 8 rows
+// 20.3 and 14.1, 16 rows 28 and 15.5, 32 rows 44 and 25; 2048 x 2048, 8 rows 6.0 and 4.8; 16384 x 2048 in pairs, 16 rows 22.8 and 22.8.  A CTA owns 16 C columns; its eight warps split K, each staging its own activations (bf16, 128 inputs at a time), and meet in
 // shared memory at the end, summed in warp order.
 //
 // An MMA truncates its sum, so none is chained to another: four are added in pairs, rounded, and the last sum keeps its rounding errors
 // (two-sum).  8 rows against 64 bits, 2^-24 = 6.0e-8 (one column per warp in f32 FMAs / chains of four / now): normal operands, 256 inputs
 // 5.6e-8 / 7.4e-8 / 6.1e-8, 512 inputs 6.3e-8 / 8.3e-8 / 5.8e-8, 2048 7.9e-8 / 9.4e-8 / 6.4e-8, 14336 1.6e-7 / 1.2e-7 / 1.1e-7; operands of one
 // sign, 512 inputs 3.3e-8 / 8.2e-8 / 3.3e-8, 2048 3.2e-8 / 8.5e-8 / 2.9e-8.  No slower: norm, gate|up and down of 4096 x 14336 at 8, 16 and 31 rows
-// 118.1, 153.3 and 244.7 us with the chains, 117.9, 145.2 and 237.8 now.
+// 118.1, 153.3 and 244.7 us with the chains, 117.9, 145.2 and 237.8 without (weights in registers both).
 // ------------------------------------------------------------------------------------------------
 #define DM_STEP 128                    // inputs staged at a time by a warp
 #define DM_LD (DM_STEP + 8)            // row stride of the staged activations (bf16): 16-byte reads of 8 rows without conflicts
@@ -310,8 +314,15 @@ __device__ __forceinline__ void dense_mma_bf16(float (&c)[4], uint32_t a0, uint3
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-template <int NT, int C>               // 8 NT rows, 16 C columns per CTA
-__global__ void __launch_bounds__(256) dense_mma_kernel(DlDenseArgs a) {
+// two: two CTAs an SM (128 registers a thread).  Halves of a step in the ring, and rows of activations on their way a step ahead: as many as fit, but not all of an SM's
+// shared memory, from which loads in flight take their places too (28672 x 4096 in pairs, 16 rows: rings of 3 halves 84 to 94 us, of 2 76; 4096 x 4096, 16
+// rows: 16 rows ahead 17.2 us, on one CTA an SM, 8 13.3 on two)
+static __host__ __device__ constexpr int dense_mma_depth(int NT, int C, bool two) { return NT == 1 ? (C == 1 ? 4 : 3) : C == 1 && !two ? (NT == 4 ? 3 : 4) : NT == 2 && C == 1 ? 4 : 2; }
+static __host__ __device__ constexpr int dense_mma_ahead(int NT, int C, bool two) { return NT == 1 ? 8 : C == 1 && !two ? 16 : two && (NT == 4 || C == 2) ? 4 : 8; }
+static __host__ __device__ constexpr int dense_mma_xs(int NT, int C) { return NT * 8 * 8 * (DM_LD * 2 > 16 * C * 4 ? DM_LD * 2 : 16 * C * 4); }      // activations, then partial sums
+
+template <int NT, int C, bool TWO>     // 8 NT rows, 16 C columns per CTA
+__global__ void __launch_bounds__(256, TWO ? 2 : 1) dense_mma_kernel(DlDenseArgs a) {
     extern __shared__ __align__(16) uint8_t dm_smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int b = blockIdx.z, n0 = blockIdx.x * 16 * C;
@@ -335,41 +346,65 @@ __global__ void __launch_bounds__(256) dense_mma_kernel(DlDenseArgs a) {
     for (int c = 0; c < C; ++c)
 #pragma unroll
         for (int n = 0; n < NT; ++n) acc[c][n][0] = acc[c][n][1] = acc[c][n][2] = acc[c][n][3] = 0.f;
-    const uint4 zero = make_uint4(0, 0, 0, 0);
-    // a lane's weights of half a step: [two 32-input pieces][C][rows g and g + 8]
-    auto fetch = [&](uint4 (&w)[2][C][2], int k0) {
+    // a lane's weights of half a step, [two 32-input pieces][C][rows g and g + 8]: it copies them into places of its own, D - 1 halves ahead
+    constexpr int D = dense_mma_depth(NT, C, TWO), SLOTS = 4 * C;
+    uint4* ring = reinterpret_cast<uint4*>(dm_smem + dense_mma_xs(NT, C)) + (size_t)warp * D * SLOTS * 32 + lane;
+    const int halves = 2 * (s1 - s0);
+    auto fetch = [&](int h) {
+        if (h < halves) {
 #pragma unroll
-        for (int p = 0; p < 2; ++p)
+            for (int p = 0; p < 2; ++p)
 #pragma unroll
-            for (int c = 0; c < C; ++c)
+                for (int c = 0; c < C; ++c)
 #pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    const int k = k0 + p * 32 + t * 8, n = n0 + c * 16 + u * 8 + g;
-                    w[p][c][u] = k < a.K && n < a.N ? *reinterpret_cast<const uint4*>(W + (size_t)n * a.ldw + k) : zero;
-                }
+                    for (int u = 0; u < 2; ++u) {
+                        const int k = s0 * DM_STEP + h * 64 + p * 32 + t * 8, n = n0 + c * 16 + u * 8 + g;
+                        const bool in = k < a.K && n < a.N;
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(ring + ((h % D) * SLOTS + (p * C + c) * 2 + u) * 32)), "l"(in ? W + (size_t)n * a.ldw + k : W), "r"(in ? 16 : 0) : "memory");
+                    }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    uint4 cur[2][C][2], nxt[2][C][2];
-    if (s1 > s0) fetch(cur, s0 * DM_STEP);
+#pragma unroll
+    for (int h = 0; h < D - 1; ++h) fetch(h);
+    // a row's 128 inputs of a step by the whole warp; up to 16 rows are on their way a step ahead
+    constexpr int AHEAD = dense_mma_ahead(NT, C, TWO);
+    float4 xv[AHEAD];
+    auto row_step = [&](int m, int s) {
+        const int k = s * DM_STEP + lane * 4;
+        return m < a.M && k < a.K ? *reinterpret_cast<const float4*>(X + (size_t)m * a.ldx + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    auto row_put = [&](int m, float4 v) {
+        __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+        *reinterpret_cast<uint2*>(xs + m * DM_LD + lane * 4) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+    };
+    if (s1 > s0) {
+#pragma unroll
+        for (int m = 0; m < AHEAD; ++m) xv[m] = row_step(m, s0);
+    }
     for (int s = s0; s < s1; ++s) {
-        const int k0 = s * DM_STEP;
         __syncwarp();
 #pragma unroll 4
-        for (int m = 0; m < NT * 8; ++m) {          // a row's 128 inputs by the whole warp
-            const int k = k0 + lane * 4;
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (m < a.M && k < a.K) v = *reinterpret_cast<const float4*>(X + (size_t)m * a.ldx + k);
-            __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
-            *reinterpret_cast<uint2*>(xs + m * DM_LD + lane * 4) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+        for (int m = AHEAD; m < NT * 8; ++m) row_put(m, row_step(m, s));
+#pragma unroll
+        for (int m = 0; m < AHEAD; ++m) row_put(m, xv[m]);
+        if (s + 1 < s1) {
+#pragma unroll
+            for (int m = 0; m < AHEAD; ++m) xv[m] = row_step(m, s + 1);
         }
         __syncwarp();
 #pragma unroll
         for (int h = 0; h < 2; ++h) {                // halves of 64 inputs: four MMAs, added in pairs
-            if (h == 0 || s + 1 < s1) fetch(nxt, k0 + (h + 1) * 64);
-            uint4 x[2][NT];
+            const int at = (s - s0) * 2 + h;
+            asm volatile("cp.async.wait_group %0;" ::"n"(D - 2) : "memory");
+            uint4 x[2][NT], cur[2][C][2];
 #pragma unroll
             for (int p = 0; p < 2; ++p)
 #pragma unroll
                 for (int n = 0; n < NT; ++n) x[p][n] = *reinterpret_cast<const uint4*>(xs + (n * 8 + g) * DM_LD + h * 64 + p * 32 + t * 8);
+#pragma unroll
+            for (int i = 0; i < SLOTS; ++i) cur[i / (2 * C)][i / 2 % C][i & 1] = ring[((at % D) * SLOTS + i) * 32];
+            fetch(at + D - 1);
 #pragma unroll
             for (int c = 0; c < C; ++c)
 #pragma unroll
@@ -385,10 +420,6 @@ __global__ void __launch_bounds__(256) dense_mma_kernel(DlDenseArgs a) {
 #pragma unroll
                     for (int e = 0; e < 4; ++e) acc[c][n][e] += (d[0][e] + d[1][e]) + (d[2][e] + d[3][e]);
                 }
-#pragma unroll
-            for (int p = 0; p < 2; ++p)
-#pragma unroll
-                for (int c = 0; c < C; ++c) { cur[p][c][0] = nxt[p][c][0]; cur[p][c][1] = nxt[p][c][1]; }
         }
     }
     // [warp][row m][16 C columns], in the activations' place
@@ -423,23 +454,32 @@ __global__ void __launch_bounds__(256) dense_mma_kernel(DlDenseArgs a) {
     }
 }
 
-template <int NT, int C>
-static void launch_dense_mma_t(const DlDenseArgs& a, cudaStream_t st) {
-    constexpr int smem = NT * 8 * 8 * (DM_LD * 2 > 16 * C * 4 ? DM_LD * 2 : 16 * C * 4);
-    static bool set = false;
-    if (!set && smem > 48 * 1024) {
-        cudaFuncSetAttribute(dense_mma_kernel<NT, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        set = true;
-    }
-    launch_after(dense_mma_kernel<NT, C>, dim3((a.N + 16 * C - 1) / (16 * C), 1, a.batch), 256, st, a, smem);
+// once per kernel and device (the other kernels of this file run on any device without being asked)
+template <typename A>
+static void dense_smem(void (*kernel)(A), int bytes, bool (&set)[16]) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 16 && set[dev]) return;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (dev < 16) set[dev] = true;
 }
-// columns per CTA: as many as leave the chip a CTA per SM (they share the staged activations)
+template <int NT, int C, bool TWO>
+static void launch_dense_mma_t(const DlDenseArgs& a, cudaStream_t st) {
+    constexpr int smem = dense_mma_xs(NT, C) + 8 * dense_mma_depth(NT, C, TWO) * 4 * C * 512;
+    static_assert(smem <= 227 * 1024, "shared memory");
+    static bool set[16] = {};
+    dense_smem(dense_mma_kernel<NT, C, TWO>, smem, set);
+    launch_after(dense_mma_kernel<NT, C, TWO>, dim3((a.N + 16 * C - 1) / (16 * C), 1, a.batch), 256, st, a, smem);
+}
+// Columns per CTA (they share the staged activations): 16 until every SM has two CTAs, then 32, and 64 for 9 to 16 rows, whose CTAs of 64 have an SM of their own (us, 32 and
+// 64 columns: 28672 x 4096 in pairs, 8 rows 49.7 and 55.2, 16 rows 77.1 and 75.7, 16384 x 2048 in pairs, 8 rows 16.9 and 18.5, 16 rows 23.3 and 22.8).
 template <int NT>
 static void launch_dense_mma(const DlDenseArgs& a, cudaStream_t st, int n_sms) {
     const long long groups = (long long)(a.N + 15) / 16 * a.batch;
-    if (NT <= 2 && groups >= 4ll * n_sms) launch_dense_mma_t<NT <= 2 ? NT : 1, 4>(a, st);      // (4 x 4 accumulator tiles do not fit the registers)
-    else if (groups >= 2ll * n_sms) launch_dense_mma_t<NT, 2>(a, st);
-    else launch_dense_mma_t<NT, 1>(a, st);
+    if (NT == 2 && groups >= 4ll * n_sms) launch_dense_mma_t<2, NT == 2 ? 4 : 1, false>(a, st);
+    else if (groups >= 2ll * n_sms) launch_dense_mma_t<NT, 2, NT <= 2>(a, st);
+    else if (groups > n_sms) launch_dense_mma_t<NT, 1, true>(a, st);
+    else launch_dense_mma_t<NT, 1, false>(a, st);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -603,11 +643,8 @@ static bool dense_ring(const DlDenseArgs& a, int n_sms, DenseRing& g) {
 }
 template <int MT, bool PAIR, bool SLICED>
 static void launch_dense_ring_t(const DenseRing& g, cudaStream_t st, int n_sms) {
-    static bool set = false;
-    if (!set) {
-        cudaFuncSetAttribute(dense_ring_kernel<MT, PAIR, SLICED>, cudaFuncAttributeMaxDynamicSharedMemorySize, DR_RING + DR_PART);
-        set = true;
-    }
+    static bool set[16] = {};
+    dense_smem(dense_ring_kernel<MT, PAIR, SLICED>, DR_RING + DR_PART, set);
     launch_after(dense_ring_kernel<MT, PAIR, SLICED>, dim3(n_sms), (dense_ring_warps(MT, PAIR, SLICED) + 1) * 32, st, g, (size_t)g.stages * g.rows * g.a.K * 2 + (SLICED ? DR_PART : 0));
 }
 template <int MT>

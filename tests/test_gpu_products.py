@@ -201,3 +201,17 @@ def test_rows_through_the_ring(M, N, K_, epi):
     if epi == "gate":
         want = aux.double() * want.sigmoid()
     assert (y.double() - want).norm() <= 1e-6 * want.norm() and (buf[:, cols:] == 3).all()
+
+
+@pytest.mark.parametrize("M", [3, 8, 9, 16, 17, 32])
+@pytest.mark.parametrize("N,K_", [(40, 8), (2047, 1032), (2370, 136), (4700, 264), (4790, 1096), (9500, 200)])
+def test_few_rows_by_columns_per_cta(M, N, K_):
+    """3 to 32 rows by every width of a CTA, with rows, columns and inputs left over, warps without a step of inputs and rings longer than a warp's steps.  Against 64 bits: bf16 operands,
+    f32 sums, 1e-6 of the result's norm."""
+    lib = L()
+    g = torch.Generator(device="cuda").manual_seed(N + M)
+    w, x = (torch.randn(N, K_, generator=g, device="cuda") * K_ ** -0.5).bfloat16(), torch.randn(M, K_, generator=g, device="cuda")
+    buf = torch.full((M, N + 3), 3.0, device="cuda")
+    lib.dense(w, x, buf[:, :N], M, True)
+    want = x.bfloat16().double() @ w.double().t()
+    assert (buf[:, :N].double() - want).norm() <= 1e-6 * want.norm() and (buf[:, N:] == 3).all()
