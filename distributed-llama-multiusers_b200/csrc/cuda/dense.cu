@@ -279,12 +279,12 @@ __global__ void __launch_bounds__(GV_WARPS * 32) dense_gemv_vec_kernel(DlDenseAr
 }
 
 // ------------------------------------------------------------------------------------------------
-// 3 to 32 rows, bf16 weights, activations rounded to bf16 (K % 8 == 0, aligned rows): mma.sync with the weights as the 16-row operand, so
+// 3 to 32 rows (two of many inputs), bf16 weights, activations rounded to bf16 (K % 8 == 0, aligned rows): mma.sync with the weights as the 16-row operand, so
 // the products of 8 activation rows cost one instruction per 16 x 16 weights.
 //
 // What bounds it: the weights' bytes.  On CUDA cores every row adds 8 FMAs per 16 bytes of weights and lane, and from 9 rows the tiles
 // below (16 K steps of scalar loads) left the weights behind entirely: gate|up + down of 4096 x 14336 took 441 us at 8 rows and
-// 3150 us at 16; 79 and 117 us here.  (Two rows are faster one by one: 2048 x 8192, 12.0 us there, 13.3 here.)
+// 3150 us at 16; 79 and 117 us here.  (Two rows: launch_dense.)
 //
 // A lane's 16 bytes of weights are 8 consecutive inputs of row g, and the four pairs fill k slots of two MMAs; the activations' 16 bytes of the same
 // inputs fill the same slots, so no shuffle.  A lane copies its weights into places of its own in shared memory (cp.async), one to three halves of a
@@ -483,14 +483,14 @@ static void launch_dense_mma(const DlDenseArgs& a, cudaStream_t st, int n_sms) {
 }
 
 // ------------------------------------------------------------------------------------------------
-// One row (or two) against bf16 weights whose rows lie behind one another, activations rounded to bf16: a CTA per SM streams an equal run of weight rows through a
+// One row (or two of up to 2048 inputs) against bf16 weights whose rows lie behind one another, activations rounded to bf16: a CTA per SM streams an equal run of weight rows through a
 // ring of bulk copies.  A warp keeps its inputs in registers for the whole run: all of up to 2048 (stages of four weight rows, a warp takes one, or both of a gated
 // unit, and stores it), or a slice of 2048 of one row (stages of two rows up to 4096 inputs, else of one; the slices meet in shared memory when the run is
 // over).  Groups of warps take stages in turn; no warp waits for another before the end.  A lane's products of a slice are added in the order of the kernels above.
 //
 // What bounds it: the weights' bytes.  The kernels above hold them in registers, two CTAs an SM, and start again every 8 columns.  Cold weights, us, they and
 // this: one row, 16384 x 2048 in pairs 15.1 and 12.7, 8192 x 2048 11.2 and 8.6, 32768 x 2048 27.9 and 23.6, 28672 x 4096 in pairs 40.5 and 37.0 (6.3 TB/s), 4096 x
-// 4096 9.6 and 8.0, 2048 x 8192 8.5 and 8.0, 4096 x 14336 24.7 and 20.7; two rows, 16384 x 2048 in pairs 18.5 and 13.7, 4096 x 4096 17.6 and 11.4.
+// 4096 9.6 and 8.0, 2048 x 8192 8.5 and 8.0, 4096 x 14336 24.7 and 20.7; two rows, 16384 x 2048 in pairs 18.5 and 13.7, 8192 x 2048 in pairs 11.3 and 9.0.
 // ------------------------------------------------------------------------------------------------
 #define DR_K 2048                      // inputs of a warp
 #define DR_STAGES 24                   // at most
@@ -625,11 +625,11 @@ __global__ void __launch_bounds__((dense_ring_warps(MT, PAIR, SLICED) + 1) * 32,
     }
 }
 // From 1025 inputs and 12 Mi weights on (us, the kernels above and this: 65536 x 1024 30.4 and 32.8, 2048 x 2048 3.4 and 4.8, 2048 x 4096 5.2 and 5.9, 6144 x 2048 7.3 and
-// 7.4, 3072 x 4096 8.9 and 6.9); two rows, whose inputs leave registers for eight warps, where a warp has few bytes to multiply twice (28672 x 4096 in pairs 47.1
-// and 52.6, 2048 x 8192 12.0 and 12.4).
+// 7.4, 3072 x 4096 8.9 and 6.9); two rows, whose inputs leave registers for eight warps, where a warp holds
+// them all (in slices 28672 x 4096 in pairs 52.6, by one MMA for both 46.2).
 static bool dense_ring(const DlDenseArgs& a, int n_sms, DenseRing& g) {
     if (a.M > 2 || a.batch != 1 || a.ldw != a.K || a.K <= DR_K / 2 || a.K > 8 * DR_K || (long long)a.N * a.K < 12ll << 20) return false;
-    if (a.M == 2 && a.K > (a.epi == DL_DENSE_GLU_GELU ? DR_K : 2 * DR_K)) return false;
+    if (a.M == 2 && a.K > DR_K) return false;
     const bool pair = a.epi == DL_DENSE_GLU_GELU;
     g.a = a;
     g.slices = (a.K + DR_K - 1) / DR_K;
@@ -649,12 +649,13 @@ static void launch_dense_ring_t(const DenseRing& g, cudaStream_t st, int n_sms) 
 }
 template <int MT>
 static void launch_dense_ring(const DenseRing& g, cudaStream_t st, int n_sms) {
+    constexpr bool SLICED = MT == 1;                 // (two rows of more inputs are no work of this kernel)
     if (g.a.epi == DL_DENSE_GLU_GELU) {
         if (g.slices == 1) launch_dense_ring_t<MT, true, false>(g, st, n_sms);
-        else launch_dense_ring_t<MT, true, true>(g, st, n_sms);
+        else launch_dense_ring_t<MT, true, SLICED>(g, st, n_sms);
     } else {
         if (g.slices == 1) launch_dense_ring_t<MT, false, false>(g, st, n_sms);
-        else launch_dense_ring_t<MT, false, true>(g, st, n_sms);
+        else launch_dense_ring_t<MT, false, SLICED>(g, st, n_sms);
     }
 }
 
@@ -813,10 +814,14 @@ static void launch_dense(const DlDenseArgs& a, cudaStream_t st) {
                      ((uintptr_t)a.W & 15) == 0 && ((uintptr_t)a.X & 15) == 0;
     const int n_sms = dl_device_sm_count();
     if constexpr (sizeof(WT) == 2 && RX) {
-        // with few steps of K most warps of an mma CTA idle: of very many columns, 3 and 4 rows go direct (us, direct and mma: 16 x 8192 x 256,
-        // 3 rows 51 and 75, 4 rows 60 and 75, 8 rows 115 and 78; 16 x 2048 x 512, 3 rows 21.9 and 21.5; 8192 x 256, 3 rows 5.7 and 3.8)
-        const bool direct = a.M <= 4 && a.K <= (a.M == 3 ? 512 : 256) && (long long)a.N * a.batch >= 128ll * n_sms;
-        if (vec && a.M >= 3 && a.M <= 32 && !direct) {
+        // With few steps of K most warps of an mma CTA idle, and of few products its sum is the less exact one (from 64 bits, f32 FMAs and mma: 264 inputs 5.5e-8 and
+        // 5.7e-8, 320 5.8e-8 and 5.6e-8): of very many columns, 3 and 4 rows of few inputs go direct (us, direct and mma: 16 x 8192 x 256, 3 rows 51.3 and
+        // 52.2, 4 rows 60.7 and 52.3; 16 x 2048 x 512, 3 rows 22.1 and 15.9).
+        const bool direct = a.M <= 4 && a.K <= (a.M == 3 ? 312 : 256) && (long long)a.N * a.batch >= 128ll * n_sms;
+        // Two rows whose inputs a warp cannot hold, of weights enough for two CTAs an SM (us, one by one and here: 4096 x 4096 17.6 and 8.8, 4096 x
+        // 14336 37.3 and 23.9, 2400 x 8192 20.1 and 13.7, 32768 x 4096 60.5 and 54.2, 28672 x 4096 in pairs 47.1 and 46.2; 2048 x 8192 12.0 and 13.3).
+        const bool two = a.M == 2 && a.K > DR_K && a.N > 16 * n_sms && (long long)a.N * a.K * a.batch >= 12ll << 20;
+        if (vec && (two || (a.M >= 3 && a.M <= 32 && !direct))) {
             if (a.M <= 8) launch_dense_mma<1>(a, st, n_sms);
             else if (a.M <= 16) launch_dense_mma<2>(a, st, n_sms);
             else launch_dense_mma<4>(a, st, n_sms);
