@@ -216,3 +216,18 @@ def test_every_environment_variable_is_documented():
     seen |= set(re.findall(r"DLLAMA_[A-Z0-9_]+", open(os.path.join(root, "bench.py")).read()))
     missing = sorted(v for v in seen if v not in ENV_VARS)
     assert not missing, f"undocumented environment variables: {missing}"
+
+
+def test_scripts_call_functions_that_exist():
+    """Every `dl_...` function that a Python file of the repository takes from a native library is defined in the native sources."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    pkg = os.path.join(root, "distributed-llama-multiusers_b200")
+
+    def files(top, *ends):
+        return [os.path.join(d, f) for d, _, fs in os.walk(top) for f in fs if f.endswith(ends)]
+    defined = set()
+    for f in files(os.path.join(pkg, "csrc"), ".cu", ".cuh", ".cpp", ".hpp"):
+        defined.update(re.findall(r"\b(dl_[a-z0-9_]+)\s*\(", open(f).read()))
+    for f in files(os.path.join(root, "scripts"), ".py") + files(pkg, ".py") + [os.path.join(root, "bench.py")]:
+        called = set(re.findall(r"\.(dl_[a-z0-9_]+)\b", open(f).read()))
+        assert called <= defined, (f, called - defined)
