@@ -35,12 +35,12 @@
 //
 // Reference semantics: multiheadAtt_F32 (src/nn/nn-cpu-ops.cpp:749-784), softmax in f32, output cast as OP_CAST
 // (src/llm.cpp:296-301).  KV cache: fp16 pages [page][kv_head][32][128].
-#include <cuda.h>
 #include <atomic>
 #include <cstring>
 #include <mutex>
 #include "epilogue.cuh"
 #include "f32_pairs.cuh"
+#include "tensor_map.cuh"
 #include "window_tiles.cuh"
 
 #define PT_HS 128
@@ -916,30 +916,13 @@ static int pt_limit(PtLimit* l) {
 
 #define PT_SMEM ((2 + 2 * PT_STAGES) * PT_TILE_BYTES + 8 * 32 * PT_OUT_LD * 4 + 22 * 8)
 
-typedef CUresult (*PtEncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
 // [rows][width] fp16 or bf16 view of a KV cache on THIS GPU (rows = pages x kv heads x 32), box = 64 columns x 32 rows (one page of
 // one head, half of the head dimension), 128-byte swizzle: the image tcgen05.mma reads as a swizzled K- or MN-major tile
 static int pt_make_map(CUtensorMap* m, const void* base, long long rows, int width, bool bf16) {
-    static PtEncodeTiled enc = nullptr;
-    if (enc == nullptr) {
-        void* fn = nullptr;
-        cudaDriverEntryPointQueryResult qr;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qr) != cudaSuccess || fn == nullptr) {
-            dl_set_error("attention_prefill_tc: cuTensorMapEncodeTiled not available");
-            return -1;
-        }
-        enc = (PtEncodeTiled)fn;
-    }
     const cuuint64_t dims[2] = {(cuuint64_t)width, (cuuint64_t)rows};
     const cuuint64_t strides[1] = {(cuuint64_t)width * 2};
-    const cuuint32_t box[2] = {64, 32}, es[2] = {1, 1};
-    const CUresult r = enc(m, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) { dl_set_error("attention_prefill_tc: cuTensorMapEncodeTiled failed (%d)", (int)r); return -1; }
-    return 0;
+    const cuuint32_t box[2] = {64, 32};
+    return dl_tensor_map("attention_prefill_tc", m, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
 extern "C" int dl_attention_prefill_tc(const float* q, int M, int n_heads, int n_kv_heads, int head_size, const void* k_cache,

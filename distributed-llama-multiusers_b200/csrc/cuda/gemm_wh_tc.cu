@@ -24,10 +24,11 @@
 // weight panel in L2); each CTA owns 128 TMEM lanes x 2 accumulators of 256 columns, so the epilogue of tile i
 // (TMEM -> registers -> smem chunk -> the shared fused epilogues of epilogue.cuh) overlaps the MMAs of tile i+1.
 //
-// Warp roles (576 threads): warp 0 producer (a converged warp, 4-6 of its lanes a 16 KB bulk copy each per stage), warp 1 MMA issuer + TMEM owner (in the
-// second CTA of a pair: forwards "my half of the stage has landed" to the leader's barrier), warps 2-17 epilogue.
+// Warp roles (576 threads): warp 0 producer (a converged warp, 4-6 of its lanes a copy each per stage), warp 1 MMA issuer (in the first CTA of a pair) + TMEM
+// owner, warps 2-17 epilogue.
 // Reference semantics: matmul_Q80_Q40_F32 (src/nn/nn-cpu-ops.cpp:352-377), llamafile sgemm (src/nn/llamafile/sgemm.cpp:593-783).
 #include "epilogue.cuh"
+#include "tensor_map.cuh"
 
 #define WH_TILE_BYTES 32768
 #define WT_NT 256                      // most activation rows per tile (wh_tile_rows: how many)
@@ -92,6 +93,13 @@ DL_DEVINL void wt_cluster_sync() {
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+// box (256 doublewords, a row group; rows; one slab) at {0, c1, c2} into this CTA, counted by a barrier of either CTA of the pair
+DL_DEVINL void wt_copy_pair(uint32_t dst, const CUtensorMap* map, int c1, int c2, uint32_t cluster_bar) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
+                 "l"(map), "r"(0), "r"(c1), "r"(c2), "r"(cluster_bar)
+                 : "memory");
+}
+
 // Bounded waits: a protocol bug must end in a trap (an error the host sees), never in a hung GPU.
 #define WT_DEADLINE_NS 4000000000ull
 DL_DEVINL void wt_wait(uint64_t* bar, uint32_t parity, unsigned long long t0) {
@@ -135,7 +143,8 @@ DL_DEVINL bool wt_tile(const WhArgs& a, int t, WtTile& w) {
 }
 
 template <int CG>
-__global__ void __launch_bounds__(WT_THREADS, 1) gemm_wh_tc_kernel(const __grid_constant__ WhArgs a) {
+__global__ void __launch_bounds__(WT_THREADS, 1) gemm_wh_tc_kernel(const __grid_constant__ WhArgs a, const __grid_constant__ CUtensorMap wmap,
+                                                                   const __grid_constant__ CUtensorMap xmap) {
     extern __shared__ __align__(1024) uint8_t smem[];
     constexpr int NS = (CG == 1) ? 2 : 3;                 // stages of one 128-wide k step
     constexpr int STAGE = WH_TILE_BYTES + WT_NT / CG * 256;   // 96 KB / 64 KB
@@ -144,8 +153,7 @@ __global__ void __launch_bounds__(WT_THREADS, 1) gemm_wh_tc_kernel(const __grid_
     const unsigned long long t0 = globaltimer_ns();
     float* out_s = reinterpret_cast<float*>(smem + NS * STAGE);          // [32][128], or [WT_VEC_CHUNK][EPI_TILE_LD]
     uint64_t* bars = reinterpret_cast<uint64_t*>(out_s + WT_VEC_CHUNK * EPI_TILE_LD);
-    uint64_t* full = bars;               // [NS]  this CTA's copies of a stage have landed
-    uint64_t* peer_full = bars + 4;      // [NS]  (leader of a pair) the other CTA's copies have landed
+    uint64_t* full = bars;               // [NS]  the copies of a stage have landed (a pair's, of both CTAs: in the first one alone)
     uint64_t* empty = bars + 8;          // [NS]  the MMAs reading the stage have retired (both CTAs)
     uint64_t* acc_full = bars + 12;      // [2]   accumulator complete
     uint64_t* acc_empty = bars + 14;     // [2]   accumulator drained by the epilogue(s)
@@ -161,7 +169,6 @@ __global__ void __launch_bounds__(WT_THREADS, 1) gemm_wh_tc_kernel(const __grid_
     if (tid == 0) {
         for (int s = 0; s < NS; s++) {
             mbar_init(&full[s], 1);
-            mbar_init(&peer_full[s], 1);
             mbar_init(&empty[s], 1);
         }
         for (int u = 0; u < 2; u++) {
@@ -180,42 +187,74 @@ __global__ void __launch_bounds__(WT_THREADS, 1) gemm_wh_tc_kernel(const __grid_
 
     if (warp == 0) {
         // ------------------------------------ producer ------------------------------------
-        // the stage is fetched as `piece`-byte bulk copies, one per lane: first the weight tile, then row groups of the
-        // activation slab (many requests in flight: one bulk copy streams at only ~16 B/clk)
         // the whole warp walks the stages together (28672 x 4096 at 2048 rows 359 us, 367 with lanes that wait and issue one by one)
-        const int piece = a.piece, npiece = STAGE / piece, na = WH_TILE_BYTES / piece, prow = piece / 256;
-        pdl_wait();
-        const size_t x_kt_stride = (size_t)(a.ncap >> 3) * XH_ROWGROUP_BYTES;
-        uint32_t it = 0;
-        for (int t = cid; t < a.n_tiles; t += ncl) {
-            WtTile w;
-            if (!wt_tile(a, t, w)) continue;
-            const int rp = w.rp, mt = w.mt;
-            const int rt = rp * CG + (int)crank;
-            const int mrow0 = w.row0 + mt * a.nt + (int)crank * B_ROWS;
-            const int row_cap = a.grp ? w.row0 + ((w.rows + 7) & ~7) : a.ncap;      // slabs hold 8 rows
-            const int b_rows = max(0, min(B_ROWS, row_cap - mrow0));
-            const uint8_t* src = nullptr;
-            size_t stride = 0;
-            uint32_t bytes = 0;
-            if (lane < na) {
-                src = a.wh + (size_t)w.g * (size_t)a.wh_group_bytes + (size_t)rt * KT * WH_TILE_BYTES + lane * piece;
-                stride = WH_TILE_BYTES;
-                bytes = piece;
-            } else if (lane < npiece) {
-                const int r0 = (lane - na) * prow;
-                src = a.xh + (size_t)((mrow0 + r0) >> 3) * XH_ROWGROUP_BYTES;
-                stride = x_kt_stride;
-                bytes = (a.dbg & 4) ? 0u : (uint32_t)max(0, min(prow, b_rows - r0)) * 256u;
+        if (CG == 2) {
+            // A stage is two tensor copies of 16 KB of weights and two of half of this CTA's activation rows each, both CTAs' counted by the FIRST one's
+            // barrier, so that its MMAs wait for what they read in either CTA by one barrier.  The alternative, bulk copies counted in their own CTA and an
+            // arrive by the second one on a barrier of the first, costs a memory barrier of ~1.4 us a stage at cluster scope (28672 x 4096 at 2048 rows 353
+            // us, 4096 x 14336 205), and with less the memory model orders nothing between the CTAs.  So: 324 and 182, on a card where the same
+            // without epilogues takes 312 (301 above).
+            const int bg = a.nt >> 5, i = lane >> 1, half = lane & 1;      // row groups of an activation copy; lane: i = 0 weights, 1 activations
+            const CUtensorMap* map = i == 0 ? &wmap : &xmap;
+            const uint32_t leader_full = mapa_shared(smem_u32(full), 0);
+            const uint32_t dst = i == 0 ? half * 16384 : WH_TILE_BYTES + half * bg * XH_ROWGROUP_BYTES;
+            pdl_wait();
+            uint32_t it = 0;
+            for (int t = cid; t < a.n_tiles; t += ncl) {
+                WtTile w;
+                if (!wt_tile(a, t, w)) continue;
+                const int row0 = w.row0 + w.mt * a.nt;
+                auto live = [&](int c, int h) { return !(a.dbg & 4) && row0 + c * B_ROWS + h * bg * 8 < w.row0 + w.rows; };      // the copy has rows of the product
+                const uint32_t total = 2 * WH_TILE_BYTES + (live(0, 0) + live(0, 1) + live(1, 0) + live(1, 1)) * bg * XH_ROWGROUP_BYTES;
+                const bool on = i == 0 || (i == 1 && live(crank, half));
+                const int c1 = i == 0 ? half * 8 : ((row0 + (int)crank * B_ROWS) >> 3) + half * bg;
+                const int c2 = i == 0 ? w.g * (int)(a.wh_group_bytes / WH_TILE_BYTES) + (w.rp * CG + (int)crank) * KT : 0;
+                for (int kt = 0; kt < KT; kt++, it++) {
+                    const uint32_t s = it % NS;
+                    if (it >= NS) wt_wait(&empty[s], ((it / NS) & 1) ^ 1, t0);
+                    __syncwarp();
+                    if (crank == 0 && lane == 0) mbar_arrive_expect_tx(&full[s], total);
+                    if (on) wt_copy_pair(smem_u32(smem + s * STAGE) + dst, map, c1, c2 + kt, leader_full + s * 8);
+                    __syncwarp();
+                }
             }
-            const uint32_t total = WH_TILE_BYTES + ((a.dbg & 4) ? 0u : (uint32_t)b_rows * 256u);
-            for (int kt = 0; kt < KT; kt++, it++) {
-                const uint32_t s = it % NS;
-                if (it >= NS) wt_wait(&empty[s], ((it / NS) & 1) ^ 1, t0);
-                __syncwarp();
-                if (lane == 0) mbar_arrive_expect_tx(&full[s], total);
-                if (bytes) bulk_g2s(smem + s * STAGE + lane * piece, src + (size_t)kt * stride, bytes, &full[s]);
-                __syncwarp();
+        } else {
+            // the stage is fetched as `piece`-byte bulk copies, one per lane: first the weight tile, then row groups of the
+            // activation slab (many requests in flight: one bulk copy streams at only ~16 B/clk)
+            const int piece = a.piece, npiece = STAGE / piece, na = WH_TILE_BYTES / piece, prow = piece / 256;
+            pdl_wait();
+            const size_t x_kt_stride = (size_t)(a.ncap >> 3) * XH_ROWGROUP_BYTES;
+            uint32_t it = 0;
+            for (int t = cid; t < a.n_tiles; t += ncl) {
+                WtTile w;
+                if (!wt_tile(a, t, w)) continue;
+                const int rp = w.rp, mt = w.mt;
+                const int rt = rp * CG + (int)crank;
+                const int mrow0 = w.row0 + mt * a.nt + (int)crank * B_ROWS;
+                const int row_cap = a.grp ? w.row0 + ((w.rows + 7) & ~7) : a.ncap;      // slabs hold 8 rows
+                const int b_rows = max(0, min(B_ROWS, row_cap - mrow0));
+                const uint8_t* src = nullptr;
+                size_t stride = 0;
+                uint32_t bytes = 0;
+                if (lane < na) {
+                    src = a.wh + (size_t)w.g * (size_t)a.wh_group_bytes + (size_t)rt * KT * WH_TILE_BYTES + lane * piece;
+                    stride = WH_TILE_BYTES;
+                    bytes = piece;
+                } else if (lane < npiece) {
+                    const int r0 = (lane - na) * prow;
+                    src = a.xh + (size_t)((mrow0 + r0) >> 3) * XH_ROWGROUP_BYTES;
+                    stride = x_kt_stride;
+                    bytes = (a.dbg & 4) ? 0u : (uint32_t)max(0, min(prow, b_rows - r0)) * 256u;
+                }
+                const uint32_t total = WH_TILE_BYTES + ((a.dbg & 4) ? 0u : (uint32_t)b_rows * 256u);
+                for (int kt = 0; kt < KT; kt++, it++) {
+                    const uint32_t s = it % NS;
+                    if (it >= NS) wt_wait(&empty[s], ((it / NS) & 1) ^ 1, t0);
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_expect_tx(&full[s], total);
+                    if (bytes) bulk_g2s(smem + s * STAGE + lane * piece, src + (size_t)kt * stride, bytes, &full[s]);
+                    __syncwarp();
+                }
             }
         }
     } else if (warp == 1) {
@@ -235,8 +274,8 @@ __global__ void __launch_bounds__(WT_THREADS, 1) gemm_wh_tc_kernel(const __grid_
                 tc_fence_after();
                 for (int kt = 0; kt < KT; kt++, it++) {
                     const uint32_t s = it % NS, ph = (it / NS) & 1;
-                    wt_wait(&full[s], ph, t0);
-                    if (CG == 2) wt_wait_cluster(&peer_full[s], ph, t0);
+                    if (CG == 2) wt_wait_cluster(&full[s], ph, t0);
+                    else wt_wait(&full[s], ph, t0);
                     tc_fence_after();
                     if (elect_one()) {
                         const uint32_t sa = smem_u32(smem + s * STAGE);
@@ -256,22 +295,6 @@ __global__ void __launch_bounds__(WT_THREADS, 1) gemm_wh_tc_kernel(const __grid_
                     __syncwarp();
                 }
                 tcount++;
-            }
-        } else {
-            // second CTA of a pair: tell the leader when this CTA's half of a stage has landed.  What the leader's MMAs read here was written here, by
-            // this SM's copies, which are complete: the arrive carries their order and no data of its own, so its release stays in this CTA.  One at
-            // cluster scope is a memory barrier of ~1.4 us in every stage's round trip (28672 x 4096 at 2048 rows 353 us, 4096 x 14336 205; 313 and 175 so).
-            const uint32_t leader_pf = mapa_shared(smem_u32(peer_full), 0);
-            uint32_t it = 0;
-            for (int t = cid; t < a.n_tiles; t += ncl) {
-                WtTile w;
-                if (!wt_tile(a, t, w)) continue;
-                for (int kt = 0; kt < KT; kt++, it++) {
-                    const uint32_t s = it % NS;
-                    wt_wait(&full[s], (it / NS) & 1, t0);
-                    if (lane == 0) asm volatile("mbarrier.arrive.release.cta.shared::cluster.b64 _, [%0];" ::"r"(leader_pf + s * 8) : "memory");
-                    __syncwarp();
-                }
             }
         }
     } else {
@@ -615,6 +638,16 @@ static int wh_tile_rows(int row_units, int M, int slots) {
     return best;
 }
 
+// the operands of a pair's copies as [slab][row group][2 KB]: of the activations, no row group behind the last that has a row
+static int wh_pair_maps(const WhArgs& a, CUtensorMap* wmap, CUtensorMap* xmap) {
+    const cuuint64_t tiles = (a.n_groups - 1) * (a.wh_group_bytes / WH_TILE_BYTES) + (cuuint64_t)a.row_tiles * a.KT, x_groups = (a.grp ? a.ncap : a.M + 7) / 8;
+    const cuuint64_t wd[3] = {256, 16, tiles}, ws[2] = {XH_ROWGROUP_BYTES, WH_TILE_BYTES}, xd[3] = {256, x_groups, (cuuint64_t)a.KT};
+    const cuuint64_t xs[2] = {XH_ROWGROUP_BYTES, (cuuint64_t)a.ncap / 8 * XH_ROWGROUP_BYTES};
+    const cuuint32_t wb[3] = {256, 8, 1}, xb[3] = {256, (cuuint32_t)a.nt / 32, 1};
+    if (dl_tensor_map("dl_gemm_wh_tc", wmap, CU_TENSOR_MAP_DATA_TYPE_INT64, 3, a.wh, wd, ws, wb, CU_TENSOR_MAP_SWIZZLE_NONE) != 0) return -1;
+    return dl_tensor_map("dl_gemm_wh_tc", xmap, CU_TENSOR_MAP_DATA_TYPE_INT64, 3, a.xh, xd, xs, xb, CU_TENSOR_MAP_SWIZZLE_NONE);
+}
+
 // force_cg: bit 0: 0 = pairs when the row-tile count is even, 1 = single CTAs (for tests and comparisons);
 // bit 1: the images hold bf16 (written by dl_wh_from_dense / dl_xh_from_rows) instead of fp16
 static int gemm_wh_launch(const uint8_t* wh, int d, int n, const uint8_t* xh, int ncap, int M, const DlEpilogue* epi,
@@ -629,7 +662,7 @@ static int gemm_wh_launch(const uint8_t* wh, int d, int n, const uint8_t* xh, in
     a.wh = wh; a.xh = xh; a.d_real = d;
     a.row_tiles = (d + 127) / 128;
     a.KT = n / 128; a.ncap = ncap; a.M = M;
-    const int cg = ((force_cg & 1) || (a.row_tiles & 1)) ? 1 : 2, n_sms = dl_device_sm_count();
+    const int cg = ((force_cg & 1) || (a.row_tiles & 1) || wh_group_bytes % WH_TILE_BYTES != 0) ? 1 : 2, n_sms = dl_device_sm_count();
     a.nt = grp == nullptr ? wh_tile_rows(a.row_tiles / cg, M, n_sms / cg) : WT_NT;      // (groups: their rows are not known here)
     a.m_tiles = (M + a.nt - 1) / a.nt;
     a.bf16 = (force_cg & 2) ? 1 : 0;
@@ -672,7 +705,9 @@ static int gemm_wh_launch(const uint8_t* wh, int d, int n, const uint8_t* xh, in
     }
     cfg.attrs = attrs;
     cfg.numAttrs = na;
-    cudaError_t e = (cg == 2) ? cudaLaunchKernelEx(&cfg, gemm_wh_tc_kernel<2>, a) : cudaLaunchKernelEx(&cfg, gemm_wh_tc_kernel<1>, a);
+    alignas(64) CUtensorMap wmap = {}, xmap = {};
+    if (cg == 2 && wh_pair_maps(a, &wmap, &xmap) != 0) return -1;
+    cudaError_t e = (cg == 2) ? cudaLaunchKernelEx(&cfg, gemm_wh_tc_kernel<2>, a, wmap, xmap) : cudaLaunchKernelEx(&cfg, gemm_wh_tc_kernel<1>, a, wmap, xmap);
     if (e != cudaSuccess) { dl_set_error("gemm wh launch: %s", cudaGetErrorString(e)); return -(int)e; }
     return 0;
 }

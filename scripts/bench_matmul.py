@@ -40,7 +40,7 @@ def main():
     ap.add_argument("--wh-m", default="", help="rows for the two-phase prompt GEMM (gemm_wh_tc), e.g. 256,512,1024,2048,4096")
     ap.add_argument("--wh-cg", type=int, default=0, help="1 = force single CTAs (no cta_group::2 pairs)")
     ap.add_argument("--wh-dbg", type=int, default=0, help="timing experiments of gemm_wh_tc (results invalid): 1 no epilogue, 2 no MMAs, 4 no activation copies")
-    ap.add_argument("--wh-piece", type=int, default=0, help="gemm_wh_tc bytes per bulk copy (4096, 8192, 16384)")
+    ap.add_argument("--wh-piece", type=int, default=0, help="gemm_wh_tc bytes per bulk copy of single CTAs (4096, 8192, 16384)")
     ap.add_argument("--out", default="")
     ap.add_argument("--shapes", default="qkv,wo,w13,w2,wcls")
     a = ap.parse_args()

@@ -78,6 +78,23 @@ def test_prompt_product_aligned_or_not(d, n, M, force_cg):
     np.testing.assert_allclose(out[0].cpu().numpy(), want, rtol=0, atol=2e-3 * np.abs(want).max())
 
 
+@pytest.mark.parametrize("d,n,M", [(4096, 4096, 768), (4096, 4096, 2001), (9728, 4096, 1100), (512, 8192, 300), (2048, 4096, 150), (1280, 5120, 40)])
+def test_prompt_product_pairs_and_single_ctas(d, n, M):
+    """Pairs of CTAs, whose ring of three stages wraps many times in a tile and across tiles with one CTA ahead of the other, give the bits that single CTAs
+    give (both add the same products in the same order), call for call."""
+    k = K()
+    ncap = (M + 7) // 8 * 8 + 8
+    w, _ = _q40(d, n, d + M)
+    wh = k.q40t_to_wh(k.make_q40t(w, d, n), d, n)
+    _, xh = _activations(n, M, ncap, M)
+    out = []
+    for force_cg in [1] + [0] * 10:
+        y = torch.zeros(M, d, device="cuda")
+        k.gemm_wh_tc(wh, d, n, xh, ncap, M, k.epi_store([y.data_ptr()], d, 0, False), force_cg)
+        out.append(y)
+    assert out[0].abs().max() > 0 and all(torch.equal(y, out[0]) for y in out[1:])
+
+
 @pytest.mark.parametrize("scales", [(6e-8, 1e-6, 3e-5, 1e-4), (9e-4, 0.0039, 0.03, 0.0624), (0.0624, 0.0625, 0.07, 1.0), (-0.0624, -0.0625, -3.0, 1e-4), (0.0, 2.0, -1e-5, 500.0)])
 def test_q40_expansion_rounds_once(scales):
     """Every nibble under scales from fp16's subnormals up, on both sides of the largest that one fma takes: (nibble - 8) d rounded once, in the expanded
