@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(WT_THREADS, 1) gemm_wh_tc_kernel(const __grid_
                 const int rp = w.rp, mt = w.mt;
                 const int rt = rp * CG + (int)crank;
                 const int mrow0 = w.row0 + mt * a.nt + (int)crank * B_ROWS;
-                const int row_cap = a.grp ? w.row0 + ((w.rows + 7) & ~7) : a.ncap;      // slabs hold 8 rows
+                const int row_cap = w.row0 + ((w.rows + 7) & ~7);      // slabs hold 8 rows; the image may be a part of a larger one and end there
                 const int b_rows = max(0, min(B_ROWS, row_cap - mrow0));
                 const uint8_t* src = nullptr;
                 size_t stride = 0;

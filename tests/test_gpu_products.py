@@ -95,6 +95,25 @@ def test_prompt_product_pairs_and_single_ctas(d, n, M):
     assert out[0].abs().max() > 0 and all(torch.equal(y, out[0]) for y in out[1:])
 
 
+@pytest.mark.parametrize("force_cg", [0, 1])
+def test_prompt_product_of_an_images_last_part(force_cg):
+    """Activations that are the last part of a larger image, which ends behind their last row (a tile has more): the same bits as from an image of their own."""
+    k = K()
+    d, n, M, parts = 512, 512, 136, 5
+    w, _ = _q40(d, n, 3)
+    wh = k.q40t_to_wh(k.make_q40t(w, d, n), d, n)
+    _, xh = _activations(n, M, M, 5)
+    image = torch.zeros(n // 128, parts, M // 8 * 2048, dtype=torch.uint8, device="cuda")
+    image[:, -1] = xh.view(n // 128, -1)
+    part = image.view(-1)[(parts - 1) * (M // 8) * 2048:]
+    out = []
+    for x, ncap in ((xh, M), (part, parts * M)):
+        y = torch.zeros(M, d, device="cuda")
+        k.gemm_wh_tc(wh, d, n, x, ncap, M, k.epi_store([y.data_ptr()], d, 0, False), force_cg)
+        out.append(y)
+    assert out[0].abs().max() > 0 and torch.equal(*out)
+
+
 @pytest.mark.parametrize("scales", [(6e-8, 1e-6, 3e-5, 1e-4), (9e-4, 0.0039, 0.03, 0.0624), (0.0624, 0.0625, 0.07, 1.0), (-0.0624, -0.0625, -3.0, 1e-4), (0.0, 2.0, -1e-5, 500.0)])
 def test_q40_expansion_rounds_once(scales):
     """Every nibble under scales from fp16's subnormals up, on both sides of the largest that one fma takes: (nibble - 8) d rounded once, in the expanded
