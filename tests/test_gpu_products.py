@@ -144,8 +144,10 @@ def test_q40_expansion_rounds_once(scales):
 @pytest.mark.parametrize("M,dim", [(1184, 4096), (1185, 4128), (1191, 8192), (1200, 544)])
 def test_norm_of_many_rows(M, dim):
     """Eight rows per CTA (from 1184) against a row per CTA: the merged sums bit for bit, the norm but for the order of its sum of squares, the cast
-    but for one step of a block's values (a block's largest below 8); dims beyond what a thread keeps in registers, rows that end inside a CTA."""
+    but for one step of a block's values (the 127th part of its largest, no more than the largest of all); dims beyond what a thread keeps in registers, rows
+    that end inside a CTA."""
     k = K()
+    torch.manual_seed(M)
     ncap = (M + 127) // 128 * 128
     x, parts, w = torch.randn(M, dim, device="cuda"), torch.randn(2, M, dim, device="cuda"), torch.rand(dim, device="cuda") + 0.5
     img = []
@@ -158,8 +160,8 @@ def test_norm_of_many_rows(M, dim):
         img.append((xh.view(torch.float16).float(), xo, yo))
     (h0, x0, y0), (h1, x1, y1) = img
     assert torch.equal(x0, x1) and torch.equal(x0, (x + parts[0]) + parts[1])
-    assert ((y0 - y1).abs() <= 1e-6 * y0.abs()).all() and y0.abs().max() < 8
-    assert (h0 - h1).abs().max() <= 8 / 127 * 1.001 and (h0 != h1).float().mean() < 1e-3 and h0.abs().max() > 1
+    assert ((y0 - y1).abs() <= 1e-6 * y0.abs()).all()
+    assert (h0 - h1).abs().max() <= y0.abs().max() / 127 * 1.001 and (h0 != h1).float().mean() < 1e-3 and h0.abs().max() > 1
 
 
 @pytest.mark.parametrize("vdim,rows", [(36, [64 * 8 + 1, 200]), (37, [64 * 9, 130]), (128, [64 * 17 + 5, 129])])
