@@ -400,6 +400,57 @@ static int g_tc_dbg_mode = 0;
 extern "C" void dl_debug_set_tc_mode(int m) { g_tc_dbg_mode = m; }
 extern "C" void dl_debug_set_tc_trace(long long* p) { g_tc_dbg = p; }
 
+// Activation rows per tile.  Narrow batches: the next power of two from 16 on.  From 129 rows on: tiles of 128 rows, or of up to 256, as many as those need and
+// of equal width (what a tile is short of is multiplied too), which unpack the weights half as often but go through one accumulator and one issuing warp.
+// Whichever takes fewer waves of the SMs times clocks of one: a k-tile 520 clk at 128 rows, 950 or its MMAs' 4 per row above, start and epilogue 13000 +
+// 30 a row (norm and feed-forward, us in 128s / wide, 4096 x 14336 at 300 rows 156 / 176, 400 rows - / 188 (two tiles of 256: 200), 520 rows - / 255
+// (three: 275); 2048 x 8192 at 300 rows 65 / 62); wide ones only where they leave enough CTAs to fill the chip.
+static int tc_tile(int d, int n, int M, int ncap, int ks, int n_sms) {
+    const int row_tiles = (d + 127) / 128, KT = n / Q40T_TILE_K;
+    int nt = (M <= 16) ? 16 : (M <= 32) ? 32 : (M <= 64) ? 64 : 128;
+    if (M > 128) {
+        const long long m_tiles = (M + 255) / 256, wide = ((M + m_tiles - 1) / m_tiles + 31) / 32 * 32;
+        auto clocks = [&](long long tiles, long long item, long long width) {
+            return (row_tiles * tiles * ks + n_sms - 1) / n_sms * (KT / ks * item + 13000 + 30 * width);
+        };
+        if (ncap >= m_tiles * wide && row_tiles * m_tiles * ks >= n_sms / 2 &&
+            clocks(m_tiles, wide * 4 > 950 ? wide * 4 : 950, wide) < clocks((M + 127) / 128, 520, 128)) nt = (int)wide;
+    }
+    // narrow matrices (qkv / wo: 32-48 row tiles) are better off with narrower tiles that launch more
+    // CTAs, even though every CTA then unpacks the weight tile again (the unpack overlaps the MMAs)
+    while (nt > 32 && nt <= 128 && row_tiles * ((M + nt - 1) / nt) * ks < n_sms / 2) nt >>= 1;
+    return nt;
+}
+
+// Ranks that share K: the count for which a launch takes least time, as fitted to 472 products of 512 to 8192 columns, 256 to 14336 inputs and 4 to 512 rows
+// (whole models of width 2048, 4096 and 8192 and a rank's part of them in 2, 4 and 8; cold weights): us a k-tile by the tile's rows, a start that grows with
+// the CTAs, and the ranks' exchange, which grows with both.  Clusters have to find room at once: 36 of four ranks do not (1536 x 4096 at 384 rows, two and four
+// ranks 11.3 and 18.3), 12 of eight are late (1536 x 4096 at 8 rows, four and eight ranks 4.9 and 5.6; ten, 1280 x 8192, 7.4 and 6.2).  Us
+// with 1 / 2 / 4 / 8 ranks: 4096 x 4096 at 32 rows 12.2 / 8.1 / 7.8, 128 rows 13.9 / 11.0 / 10.7; 768 x 4096 at 32 rows 12.0 / 7.7 / 5.3 / 4.5;
+// 4096 x 1024 at 8 rows 4.2 / 3.9 / 5.3, 64 rows 4.6 / 5.9 / 6.5; 8192 x 1024 at 8 rows 4.3 / 5.6; 4096 x 512 at 8 rows 3.2 / 3.5 / 5.1.
+extern "C" int dl_gemm_q40_tc_split(int d, int n, int M, int n_sms) {
+    const int row_tiles = (d + 127) / 128, KT = n / Q40T_TILE_K;
+    int best = 1;
+    double least = 0;
+    for (int S = 1; S <= 8 && S <= KT; S *= 2) {
+        const int nt = tc_tile(d, n, M, 1 << 30, S, n_sms), m_tiles = (M + nt - 1) / nt, ctas = row_tiles * m_tiles * S;
+        if ((S == 4 && ctas > 128) || (S == 8 && ctas > 80) || (S > 1 && ctas > n_sms)) continue;
+        auto ramp = [&](int from, int over) { return ctas <= from ? 0.0 : ctas >= from + over ? 1.0 : (double)(ctas - from) / over; };
+        const double item = nt <= 32 ? 0.31 : nt == 64 ? 0.33 : nt == 128 ? 0.44 : 0.00085 * (4 * nt > 950 ? 4 * nt : 950);
+        const double rows = (nt <= 32 ? 0.0 : nt == 64 ? 1.0 : 2.2 + 0.025 * (nt - 128)) * M / ((double)m_tiles * nt);
+        const double start = S == 1 ? 1.9 + 1.9 * ramp(45, 88) : S == 2 ? 2.9 + 1.7 * ramp(64, 47) : S == 4 ? 3.0 + 2.1 * ramp(64, 47) : ctas <= 48 ? 2.9 : 3.9;
+        const double us = (KT + S - 1) / S * item + rows + start;
+        if (S == 1 || us < least) { best = S; least = us; }
+    }
+    return best;
+}
+
+// the tile that dl_gemm_q40_tc takes on this device, or that one of 148 SMs takes where there is none
+extern "C" int dl_gemm_q40_tc_tile(int d, int n, int M, int ncap, int k_split) {
+    const int n_sms = dl_device_sm_count();
+    return tc_tile(d, n, M, ncap, k_split, n_sms > 0 ? n_sms : 148);
+}
+
 extern "C" int dl_gemm_q40_tc(const uint8_t* w_q40t, int d, int n, const uint8_t* xh, int ncap, int M, int k_split,
                               const DlEpilogue* epi, int pdl, void* stream) {
     if (n % Q40T_TILE_K != 0) { dl_set_error("dl_gemm_q40_tc: n=%d not a multiple of 128", n); return -1; }
@@ -411,25 +462,8 @@ extern "C" int dl_gemm_q40_tc(const uint8_t* w_q40t, int d, int n, const uint8_t
     a.d_pad = (d + 127) / 128 * 128;
     a.KT = n / Q40T_TILE_K;
     a.ncap = ncap; a.M = M;
-    a.NT = (M <= 16) ? 16 : (M <= 32) ? 32 : (M <= 64) ? 64 : 128;
     const int row_tiles = (d + 127) / 128, n_sms = dl_device_sm_count();
-    const int ks = (k_split == 2 || k_split == 4 || k_split == 8) ? k_split : 1;
-    // From 129 rows on: tiles of 128 rows, or of up to 256, as many as those need and of equal width (what a tile is short of is multiplied too), which
-    // unpack the weights half as often but go through one accumulator and one issuing warp.  Whichever takes fewer waves of the SMs times clocks of one: a
-    // k-tile 520 clk at 128 rows, 950 or its MMAs' 4 per row above, start and epilogue 13000 + 30 a row (norm and feed-forward, us in 128s / wide, 4096 x 14336 at
-    // 300 rows 156 / 176, 400 rows - / 188 (two tiles of 256: 200), 520 rows - / 255 (three: 275); 2048 x 8192 at 300 rows 65 / 62); wide ones
-    // only where they leave enough CTAs to fill the chip
-    if (M > 128) {
-        const long long m_tiles = (M + 255) / 256, nt = ((M + m_tiles - 1) / m_tiles + 31) / 32 * 32;
-        auto clocks = [&](long long tiles, long long item, long long width) {
-            return (row_tiles * tiles * ks + n_sms - 1) / n_sms * (a.KT / ks * item + 13000 + 30 * width);
-        };
-        if (ncap >= m_tiles * nt && row_tiles * m_tiles * ks >= n_sms / 2 &&
-            clocks(m_tiles, nt * 4 > 950 ? nt * 4 : 950, nt) < clocks((M + 127) / 128, 520, 128)) a.NT = (int)nt;
-    }
-    // ... and narrow matrices (qkv / wo: 32-48 row tiles) are better off with narrower tiles that launch more
-    // CTAs, even though every CTA then unpacks the weight tile again (the unpack overlaps the MMAs)
-    while (a.NT > 32 && a.NT <= 128 && row_tiles * ((M + a.NT - 1) / a.NT) * ks < n_sms / 2) a.NT >>= 1;
+    a.NT = tc_tile(d, n, M, ncap, (k_split == 2 || k_split == 4 || k_split == 8) ? k_split : 1, n_sms);
     if (ncap < (M + a.NT - 1) / a.NT * a.NT) { dl_set_error("dl_gemm_q40_tc: ncap=%d too small for M=%d (tile %d)", ncap, M, a.NT); return -1; }
     if (k_split != 1 && k_split != 2 && k_split != 4 && k_split != 8) { dl_set_error("dl_gemm_q40_tc: k_split must be 1,2,4,8"); return -1; }
     if (k_split > a.KT) k_split = 1;

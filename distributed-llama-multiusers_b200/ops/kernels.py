@@ -355,20 +355,13 @@ def decode_mega_plan(d: int, n: int, align: int, grid: int, cta: int):
 
 
 def choose_tc_split(d: int, n: int, M: int, n_sms: int) -> int:
-    """Cluster split-K factor of the tcgen05 GEMM: a power of two (<= 4) that fills the chip without
-    ever launching more CTAs than SMs (one CTA per SM: a second wave of half-empty CTAs costs more
-    than the extra parallelism buys).  The activation tile is 16/32/64/128 rows (256 with a 256-row
-    capacity), so wide batches already bring ceil(M / tile) CTAs per row tile."""
-    row_tiles = (d + 127) // 128
-    nt = 16 if M <= 16 else 32 if M <= 32 else 64 if M <= 64 else 128
-    m_tiles = (M + nt - 1) // nt
-    # Every rank finishes rows of its own, so short shares pay (us with 1 / 2 / 4 / 8 ranks: 4096 x 4096 at 32 rows 13.2 / 8.9 / 8.1, at 64 rows 13.2 / 10.2
-    # / 8.6, at 128 rows 14.5 / 11.4 / 10.7; 6144 x 4096 at 64 rows 14.3 / 11.3), and eight ranks read too much of each other (2048 x 2048 at 32 rows 8.7 / 8.7
-    # / 8.7 / 9.7, at 128 rows 8.8 / 8.7 / 8.5 / 15.3)
-    S = 1
-    while row_tiles * m_tiles * S * 2 <= n_sms and S < 4 and (n // 128) // (S * 2) >= 4:
-        S *= 2
-    return S
+    """How many CTAs of a cluster share K in the tcgen05 GEMM (1, 2, 4 or 8): what takes least time for these sizes (gemm_q40_tc.cu)."""
+    return cuda_lib().dl_gemm_q40_tc_split(d, n, M, n_sms)
+
+
+def tc_tile(d: int, n: int, M: int, ncap: int, k_split: int) -> int:
+    """Activation rows per tile that the tcgen05 GEMM takes for these sizes."""
+    return cuda_lib().dl_gemm_q40_tc_tile(d, n, M, ncap, k_split)
 
 
 def choose_splits(d: int, n: int, epi_kind: int, n_sms: int = 148, M: int = 1):

@@ -201,8 +201,10 @@ def cuda_lib():
     L.dl_decode_mega.restype = i32
     L.dl_decode_mega_plan.argtypes = [i32, i32, i32, i32, i32, C.POINTER(i32), C.POINTER(i32), C.POINTER(i32)]
     L.dl_decode_mega_plan.restype = i32
+    L.dl_gemm_q40_tc_split.argtypes = [i32] * 4
+    L.dl_gemm_q40_tc_tile.argtypes = [i32] * 5
     for name in ("dl_q40_repack", "dl_q40t_dequant", "dl_reduce_norm_quant", "dl_quant_q80", "dl_embedding",
-                 "dl_sample_rows", "dl_gemm_f32", "dl_gemv_q40", "dl_gemm_q40_tc", "dl_q40t_to_wh", "dl_gemm_wh_tc", "dl_attention", "dl_attention_prefill", "dl_attention_prefill_tc", "dl_argmax", "dl_ipc_alloc", "dl_ipc_open",
+                 "dl_sample_rows", "dl_gemm_f32", "dl_gemv_q40", "dl_gemm_q40_tc", "dl_gemm_q40_tc_split", "dl_gemm_q40_tc_tile", "dl_q40t_to_wh", "dl_gemm_wh_tc", "dl_attention", "dl_attention_prefill", "dl_attention_prefill_tc", "dl_argmax", "dl_ipc_alloc", "dl_ipc_open",
                  "dl_ipc_close", "dl_ipc_free", "dl_peer_barrier", "dl_wait_flags"):
         getattr(L, name).restype = i32
     _cuda = L

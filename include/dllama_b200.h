@@ -166,6 +166,9 @@ long long dl_gemv_q40_smem_bytes(int n, int M, int k_split);
  * TMEM accumulators (reference: llamafile_sgemm Q40xQ80, src/nn/llamafile/sgemm.cpp:593-783) */
 int dl_gemm_q40_tc(const uint8_t* w_q40t, int d, int n, const uint8_t* xh, int ncap, int M, int k_split,
                    const DlEpilogue* epi /*host*/, int pdl, void* stream);
+/* host helpers: the k_split that takes least time for these sizes, and the activation rows per tile that dl_gemm_q40_tc takes with one */
+int dl_gemm_q40_tc_split(int d, int n, int M, int n_sms);
+int dl_gemm_q40_tc_tile(int d, int n, int M, int ncap, int k_split);
 /* prompt-sized batches, two phases: the Q40T image is expanded once into WH (fp16 tiles of 128 x 128 in the UMMA
  * K-major core-matrix image, dl_wh_bytes(d, n) bytes), then a persistent SS-mode tcgen05 GEMM with CTA pairs
  * (cta_group::2, 256 x 256 tiles, double-buffered TMEM accumulators) runs on it; same epilogues as above.

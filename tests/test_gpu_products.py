@@ -33,7 +33,7 @@ def _activations(n, M, ncap, seed):
 
 
 @pytest.mark.parametrize("d,n,M,S", [(300, 512, 5, 1), (132, 512, 16, 2), (512, 1024, 33, 4), (256, 512, 70, 2), (388, 512, 128, 4), (38912, 128, 20, 1),
-                                     (38912, 128, 128, 1), (9600, 256, 150, 1), (9600, 256, 430, 1), (130, 512, 9, 1)])
+                                     (38912, 128, 128, 1), (9600, 256, 150, 1), (9600, 256, 430, 1), (130, 512, 9, 1), (768, 4096, 20, 8), (1280, 2048, 40, 8), (384, 1024, 3, 8)])
 @pytest.mark.parametrize("roundtrip", [False, True])
 def test_store_epilogue_aligned_or_not(d, n, M, S, roundtrip):
     """The same values, bit for bit, whether rows start on 16 bytes (four values per thread) or not (one); tiles alone, in pairs, in shares of K and of
