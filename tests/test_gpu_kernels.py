@@ -244,40 +244,27 @@ def test_gemm_wh_tc_matches_reference(d, n, M, ncap, force_cg):
     np.testing.assert_allclose(got, ref, rtol=2e-3, atol=2e-3 * scale)
 
 
-def _tc_tile(d, M, S, ncap, n_sms=148):
-    """The activation tile width dl_gemm_q40_tc picks (mirror of gemm_q40_tc.cu:388-396), so the wide-tile tests
-    below fail loudly if a change of the heuristic stops exercising the plans they are meant to cover."""
-    row_tiles = (d + 127) // 128
-    nt = 16 if M <= 16 else 32 if M <= 32 else 64 if M <= 64 else 128
-    if M > 128 and ncap % 256 == 0 and row_tiles * ((M + 255) // 256) * S >= n_sms // 2:
-        nt = 256
-    while nt > 32 and row_tiles * ((M + nt - 1) // nt) * S < n_sms // 2:
-        nt >>= 1
-    return nt
-
-
 @pytest.mark.parametrize("d,n,M,S,ncap,want_nt", [
     (9600, 1024, 64, 1, 64, 64), (9600, 1024, 50, 1, 64, 64), (9600, 1024, 128, 1, 128, 128), (9600, 1024, 100, 2, 128, 128),
-    (9600, 1024, 256, 1, 256, 256), (9600, 1024, 300, 1, 512, 256), (4864, 1024, 256, 2, 256, 256), (9600, 512, 200, 1, 256, 256),
+    (9600, 1024, 256, 1, 256, 256), (9600, 1024, 300, 1, 512, 128), (9600, 1024, 500, 1, 512, 256), (9600, 512, 700, 1, 768, 256), (4864, 1024, 256, 2, 256, 256),
+    (9600, 512, 150, 1, 256, 160), (9600, 512, 180, 1, 256, 192), (9600, 512, 200, 1, 256, 224), (9600, 512, 520, 1, 768, 192), (9600, 512, 370, 2, 512, 192),
 ])
 def test_gemm_q40_tc_wide_tiles(d, n, M, S, ncap, want_nt):
-    """The prefill configurations: 64-, 128- and 256-wide activation tiles (different stage counts, accumulator
-    counts, TMEM column maps and the chunked 256-wide epilogue) at shapes that really select them."""
-    sms = torch.cuda.get_device_properties(0).multi_processor_count
-    assert _tc_tile(d, M, S, ncap, sms) == want_nt, "the tile heuristic changed: pick shapes that select this tile again"
+    """The prefill configurations: 64-, 128- and up to 256-wide activation tiles (different stage counts, accumulator
+    counts, TMEM column maps and epilogues), several of them and a last one that is not full, at shapes that really select them."""
+    assert K().tc_tile(d, n, M, ncap, S) == want_nt, "the tile rule changed: pick shapes that select this tile again"
     got, ref = _gemm_case(d, n, M, S, seed=d + n + M, ncap_override=ncap)
     assert not np.isnan(got).any()
     scale = np.abs(ref).max()
     np.testing.assert_allclose(got, ref, rtol=2e-3, atol=2e-3 * scale)
 
 
-@pytest.mark.parametrize("M,ncap,want_nt", [(64, 64, 64), (128, 128, 128), (256, 256, 256)])
+@pytest.mark.parametrize("M,ncap,want_nt", [(64, 64, 64), (128, 128, 128), (150, 256, 160), (180, 256, 192), (200, 256, 224), (256, 256, 256)])
 def test_wide_tile_epilogues(M, ncap, want_nt):
     """SiLU*mul -> Q80 slabs and RoPE + q / paged-KV write through the wide tensor-core tiles (the TTFT path)."""
     k = K()
     from dllama_b200.formats.mfile import LlmHeader
     from dllama_b200.models.oracle import apply_rope, rope_frequencies
-    sms = torch.cuda.get_device_properties(0).multi_processor_count
     dim = 512
     rng = np.random.default_rng(100 + M)
     x = rng.standard_normal((M, dim), dtype=np.float32) * 2
@@ -286,7 +273,7 @@ def test_wide_tile_epilogues(M, ncap, want_nt):
     k.quant_q80(torch.from_numpy(x).cuda(), M, dim, ncap, None, xh)
     # ---- SiLU * mul: 2 * hid rows interleaved (gate, up) ----
     hid = 4864                                       # 2 * hid = 76 row tiles; a multiple of 128 (XH slabs are per k-tile)
-    assert _tc_tile(2 * hid, M, 1, ncap, sms) == want_nt
+    assert k.tc_tile(2 * hid, dim, M, ncap, 1) == want_nt
     raw1, w1 = _rand_q40(hid, dim, 31)
     raw3, w3 = _rand_q40(hid, dim, 32)
     w = torch.zeros(k.q40t_bytes(2 * hid, dim), dtype=torch.uint8, device="cuda")
@@ -304,7 +291,7 @@ def test_wide_tile_epilogues(M, ncap, want_nt):
     hs, n_heads, n_kv = 128, 59, 8                  # q_dim 7552 + 2 * 1024 = 9600 rows: 75 row tiles
     q_dim, kv_dim = n_heads * hs, n_kv * hs
     d = q_dim + 2 * kv_dim
-    assert _tc_tile(d, M, 1, ncap, sms) == want_nt
+    assert k.tc_tile(d, dim, M, ncap, 1) == want_nt
     h = LlmHeader(dim=q_dim, n_heads=n_heads, n_kv_heads=n_kv, rope_theta=500000.0, rope_type=2, rope_scaling_factor=8.0,
                   rope_scaling_low_freq_factor=1.0, rope_scaling_high_freq_factor=4.0, rope_scaling_orig_max_seq_len=8192)
     freqs = rope_frequencies(h)
