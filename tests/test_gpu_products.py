@@ -1,4 +1,4 @@
-"""Epilogues by whole warps, Q40 expansion, tile widths and the norm's wide form of the Q40 products, and the walk over the states of a gated scan, at
+"""Epilogues by whole warps (plain, SiLU and rotary), Q40 expansion, tile widths and the norm's wide form of the Q40 products, and the walk over the states of a gated scan, at
 the sizes where they can go wrong: remainders of tiles and chunks, addresses that are not 16-byte aligned, scales at the ends of fp16."""
 import numpy as np
 import pytest
@@ -112,6 +112,91 @@ def test_prompt_product_of_an_images_last_part(force_cg):
         k.gemm_wh_tc(wh, d, n, x, ncap, M, k.epi_store([y.data_ptr()], d, 0, False), force_cg)
         out.append(y)
     assert out[0].abs().max() > 0 and torch.equal(*out)
+
+
+def _product(kernel, w, d, n, xh, ncap, M, S, epi):
+    k = K()
+    if kernel == "q40":
+        k.gemm_q40_tc(w, d, n, xh, ncap, M, epi, S)
+    else:
+        k.gemm_wh_tc(k.q40t_to_wh(w, d, n), d, n, xh, ncap, M, epi)
+
+
+# rows that end inside a group of 8, ranks whose rows start inside one, ranks with a row or none, several tiles, chunks of 64 rows
+CASES = [("q40", M, S) for M in (1, 3, 13, 33, 70) for S in (1, 2, 4)] + [("q40", 9, 8), ("q40", 150, 1), ("q40", 256, 2), ("wh", 1, 1), ("wh", 129, 1), ("wh", 300, 1)]
+
+
+@pytest.mark.parametrize("kernel,M,S", CASES)
+@pytest.mark.parametrize("hid,gelu", [(384, False), (160, True)])
+def test_silu_epilogue_by_warps_or_by_values(kernel, M, S, hid, gelu):
+    """The image of act(gate) * up is the same bit for bit whether whole warps write it or (with a second image asked for) one value per thread does, and the
+    rows behind the last stay as they were.  Against f64: half a step of the cast and fp16 operands."""
+    k = K()
+    d, n = 2 * hid, 1024
+    ncap = 16 if M <= 16 else 32 if M <= 32 else 64 if M <= 64 else (M + 255) // 256 * 256
+    w, wdq = _q40(d, n, d)
+    w = k.make_q40t(w, d, n)
+    x, xh = _activations(n, M, ncap, M)
+    wide, out = (hid + 127) // 128 * 128, []
+    for xq in (None, k.alloc_xq(wide, ncap, "cuda")):
+        image = torch.full((k.xh_bytes(wide, ncap),), 0x3A, dtype=torch.uint8, device="cuda")
+        _product(kernel, w, d, n, xh, ncap, M, S, k.epi_silu_mul(xq, image, ncap, gelu))
+        out.append(image)
+    assert torch.equal(*out)
+    rows = out[0].view(wide // 128, ncap // 8, 16, 8, 16).permute(1, 3, 0, 2, 4).reshape(ncap, -1)       # a row's 16-byte pieces
+    assert (rows[M:] == 0x3A).all()
+    y = x @ wdq.T.astype(np.float64)
+    g, u = y[:, 0::2], y[:, 1::2]
+    want = (0.5 * g * (1 + np.tanh(0.797884560802865 * (g + 0.044715 * g ** 3))) if gelu else g / (1 + np.exp(-g))) * u
+    # K-slot order inside a block of 32 (xh_slot): value 16 hi + 4 w + r at piece w, place 4 hi + (0, 2, 1, 3)[r]
+    got = rows[:M].contiguous().view(torch.float16).view(M, -1, 4, 8).double().cpu().numpy()             # [row][block][piece][place]
+    e = np.arange(32)
+    got = got[:, :, (e & 15) >> 2, (e >> 4) * 4 + np.array([0, 2, 1, 3])[e & 3]].reshape(M, -1)[:, :hid]
+    scale = np.abs(want).max()
+    assert np.abs(got - want).max() <= scale / 127 * 0.51 + 5e-3 * scale
+
+
+@pytest.mark.parametrize("kernel,M,S", CASES)
+@pytest.mark.parametrize("heads,kv_heads,hs,dtype", [(3, 1, 64, torch.float16), (5, 3, 64, torch.float32), (3, 2, 128, torch.float16), (1, 1, 128, torch.float32)])
+def test_rope_epilogue_by_warps_or_by_values(kernel, M, S, heads, kv_heads, hs, dtype):
+    """Rotated queries and keys, and values, of heads whose regions begin and end inside a tile, into caches of both types: the same bit for bit whether rows start
+    on 16 bytes (two pairs per thread) or not (one value).  Against f64: fp16 operands and, in the caches, results; angles in f32."""
+    k = K()
+    q_dim, kv_dim, n, pages = heads * hs, kv_heads * hs, 1024, 12
+    d = q_dim + 2 * kv_dim
+    ncap = 16 if M <= 16 else 32 if M <= 32 else 64 if M <= 64 else (M + 255) // 256 * 256
+    w, wdq = _q40(d, n, d)
+    w = k.make_q40t(w, d, n)
+    x, xh = _activations(n, M, ncap, M)
+    freqs = 10000.0 ** (-torch.arange(hs // 2, dtype=torch.float64) / (hs // 2))
+    freqs = freqs.float().cuda()
+    rng = np.random.default_rng(M)
+    slots = rng.integers(0, 2, M)                                    # two sequences, their rows mixed
+    pos = np.array([5 + 7 * s + int((slots[:i] == s).sum()) for i, s in enumerate(slots)])
+    table = rng.permutation(2 * pages).reshape(2, pages).astype(np.int32)
+    i32 = lambda t: torch.tensor(np.asarray(t), dtype=torch.int32, device="cuda")
+    out = []
+    for shift in (0, 1):
+        q = torch.full((M * q_dim + 8,), 7.0, device="cuda")
+        kc, vc = (torch.full((2 * pages, kv_heads, 32, hs), 7.0, dtype=dtype, device="cuda") for _ in range(2))
+        keep = (i32(pos), i32(slots), i32(table))
+        _product(kernel, w, d, n, xh, ncap, M, S, k.epi_qkv_rope(q[shift:], q_dim, kv_dim, hs, freqs, *keep, pages, kv_heads, kc, vc))
+        torch.cuda.synchronize()
+        assert (q[shift + M * q_dim:] == 7).all()
+        out.append((q[shift:shift + M * q_dim].view(M, q_dim), kc, vc))
+    assert all(torch.equal(a, b) for a, b in zip(*out))
+    y = x @ wdq.T.astype(np.float64)
+    ang = pos[:, None].astype(np.float64) * freqs.double().cpu().numpy()
+    rot = lambda t: np.stack([t[..., 0::2] * np.cos(ang)[:, None] - t[..., 1::2] * np.sin(ang)[:, None],
+                              t[..., 0::2] * np.sin(ang)[:, None] + t[..., 1::2] * np.cos(ang)[:, None]], axis=-1).reshape(t.shape)
+    parts = [rot(y[:, :q_dim].reshape(M, -1, hs)), rot(y[:, q_dim:q_dim + kv_dim].reshape(M, -1, hs)), y[:, q_dim + kv_dim:].reshape(M, -1, hs)]
+    q, kc, vc = (t.double().cpu().numpy() for t in out[0])
+    tol = 3e-3 * np.abs(y).max()
+    assert np.abs(q.reshape(M, -1, hs) - parts[0]).max() <= tol
+    at = table[slots, pos // 32], slice(None), pos % 32
+    assert np.abs(kc[at] - parts[1]).max() <= tol and np.abs(vc[at] - parts[2]).max() <= tol
+    kc[at] = vc[at] = 7
+    assert (kc == 7).all() and (vc == 7).all()
 
 
 @pytest.mark.parametrize("scales", [(6e-8, 1e-6, 3e-5, 1e-4), (9e-4, 0.0039, 0.03, 0.0624), (0.0624, 0.0625, 0.07, 1.0), (-0.0624, -0.0625, -3.0, 1e-4), (0.0, 2.0, -1e-5, 500.0)])
