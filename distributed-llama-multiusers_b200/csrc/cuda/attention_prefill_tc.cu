@@ -36,11 +36,10 @@
 // Reference semantics: multiheadAtt_F32 (src/nn/nn-cpu-ops.cpp:749-784), softmax in f32, output cast as OP_CAST
 // (src/llm.cpp:296-301).  KV cache: fp16 pages [page][kv_head][32][128].
 #include <atomic>
-#include <cstring>
-#include <mutex>
 #include "epilogue.cuh"
 #include "f32_pairs.cuh"
 #include "tensor_map.cuh"
+#include "waits.cuh"
 #include "window_tiles.cuh"
 
 #define PT_HS 128
@@ -52,12 +51,6 @@
 #define PT_STAGES 2                    // K tiles and V tiles in flight
 #define PT_OUT_LD 20
 #define PT_SHARE_STEPS 4
-#define PT_DEADLINE_NS 4000000000ull
-
-struct PtLimit {
-    unsigned long long ns;     // how long a CTA waits (0: not at all)
-    unsigned* status;          // host memory: the device's word of dl_attention_status()
-};
 
 struct PtArgs {
     const float* q;            // [M][n_heads*128]
@@ -73,7 +66,7 @@ struct PtArgs {
     int out_mcap;
     float* y_out;
     unsigned long long* tr;
-    PtLimit limit;
+    WaitLimit limit;
 };
 
 struct PtLineArgs {
@@ -84,7 +77,7 @@ struct PtLineArgs {
     int n_splits;
     int least;                 // runs of no more stacked rows belong to the other kernel (0: there is none)
     float* partial;            // [n_tiles][kv_heads][n_splits][64][130] where n_splits > 1: sums, reference maximum, sum of weights
-    PtLimit limit;
+    WaitLimit limit;
 };
 template <bool LINES> struct PtKernelArgs { typedef PtArgs T; };
 template <> struct PtKernelArgs<true> { typedef PtLineArgs T; };
@@ -292,7 +285,7 @@ struct PtItem {
     int begin;                             // batch row of the segment's first row; LINES: entry of tile_rows where the run starts
 };
 
-// A wait that gives up (the CTA has had its time, PT_DEADLINE_NS): the flag ends the other waits, too, every output of the CTA becomes a NaN, and
+// A wait that gives up (the CTA has had its time, WAIT_DEADLINE_NS): the flag ends the other waits, too, every output of the CTA becomes a NaN, and
 // the host learns of it by dl_attention_status()
 struct PtWaits {
     volatile int* gave_up;
@@ -307,7 +300,6 @@ struct PtWaits {
         }
     }
 };
-__device__ unsigned pt_times_given_up;
 
 // Llama path: the items of a batch are (128-row tile of a segment, query head), late tiles (long histories) first: two heads of one key/value head
 // side by side, or two tiles of one head where the heads come alone; single tiles while there are SMs for all of them.  Item `idx` of the
@@ -869,11 +861,8 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
     tc_fence_before();
     __syncthreads();
     if (gave_up_s) {
-        if (tid == 0) {
-            *(volatile unsigned*)a.limit.status = atomicAdd(&pt_times_given_up, 1u) + 1u;
-            __threadfence_system();
-        }
-        __nanosleep(1000000);                                    // copies and MMAs in flight end
+        if (tid == 0) wait_report(a.limit);
+        wait_settle();
     }
     if (warp == 0) {
         tc_fence_after();
@@ -886,31 +875,11 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attention_prefill_tc_kernel(con
 extern void dl_set_error(const char* fmt, ...);
 extern int dl_device_sm_count();
 
-// Words in host memory that kernels whose waits gave up write, one per device: the host reads them where it reads results, without a copy of their own.
-static std::atomic<unsigned long long> g_pt_limit{PT_DEADLINE_NS};
-static unsigned* pt_status_word() {
-    constexpr int devices = 64;
-    static std::mutex lock;
-    static unsigned* words = nullptr;
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev >= devices) return nullptr;
-    std::lock_guard<std::mutex> guard(lock);
-    if (words == nullptr) {
-        void* p = nullptr;
-        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;       // the first launch may be a captured one
-        cudaThreadExchangeStreamCaptureMode(&mode);
-        const cudaError_t e = cudaHostAlloc(&p, devices * sizeof(unsigned), cudaHostAllocPortable | cudaHostAllocMapped);
-        cudaThreadExchangeStreamCaptureMode(&mode);
-        if (e != cudaSuccess) { cudaGetLastError(); return nullptr; }
-        words = (unsigned*)memset(p, 0, devices * sizeof(unsigned));
-    }
-    return words + dev;
-}
-extern "C" const unsigned* dl_attention_status() { return pt_status_word(); }
+static std::atomic<unsigned long long> g_pt_limit{WAIT_DEADLINE_NS};
 extern "C" void dl_debug_set_attention_limit(unsigned long long ns) { g_pt_limit = ns; }
-static int pt_limit(PtLimit* l) {
-    *l = {g_pt_limit, pt_status_word()};
-    if (l->status == nullptr) { dl_set_error("attention_prefill_tc: no host memory for its status"); return -1; }
+static int pt_limit(WaitLimit* l) {
+    if (dl_wait_limit("attention_prefill_tc", l) != 0) return -1;
+    l->ns = g_pt_limit;
     return 0;
 }
 

@@ -11,7 +11,9 @@
 // aux * sigmoid(.) (an output gate), cap * tanh(. / cap) (logit soft-capping), . * sigmoid(.) (SiLU), aux * (.) (the second
 // half of a gated unit), xIELU (a quadratic for z > 0, an exponential for z <= 0, two constants), a constant factor, and a sum
 // into Y behind one sigmoid gate per row.  A bias per output column, where given, is added first.
+#define WAIT_UNIT 1u
 #include "layer_common.cuh"
+#include "waits.cuh"
 #include "../../../include/dllama_b200.h"
 
 __device__ __forceinline__ float dense_epi(float acc, int epi, float aux, float param, float param2) {
@@ -496,24 +498,9 @@ static void launch_dense_mma(const DlDenseArgs& a, cudaStream_t st, int n_sms) {
 #define DR_STAGES 24                   // at most
 #define DR_RING (192 * 1024)
 #define DR_PART (16 * 1024)
-#define DR_DEADLINE_NS 4000000000ull
 // rows per stage, warps per row (slices of DR_K inputs), warps per stage, groups of them, stages of the ring
-struct DenseRing { DlDenseArgs a; int rows, slices, group, groups, stages; };
+struct DenseRing { DlDenseArgs a; int rows, slices, group, groups, stages; WaitLimit limit; };
 
-// false after the limit (once one wait has run out, at once)
-__device__ __forceinline__ bool dense_ring_wait(uint64_t* bar, uint32_t parity, volatile int* dead) {
-    unsigned long long t0 = 0, t;
-    for (unsigned n = 0;; ++n) {
-        uint32_t ok;
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"((uint32_t)__cvta_generic_to_shared(bar)), "r"(parity) : "memory");
-        if (ok) return true;
-        if ((n & 0xFFu) == 0xFFu) {
-            asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-            if (t0 == 0) t0 = t;
-            if (*dead || t - t0 > DR_DEADLINE_NS) { *dead = 1; return false; }
-        }
-    }
-}
 // consumers (two rows of activations: their inputs leave registers for eight); one more warp copies
 static __host__ __device__ constexpr int dense_ring_warps(int MT, bool pair, bool sliced) { return MT == 2 ? 8 : pair && !sliced ? 12 : 16; }
 template <int MT, bool PAIR, bool SLICED>
@@ -522,7 +509,7 @@ __global__ void __launch_bounds__((dense_ring_warps(MT, PAIR, SLICED) + 1) * 32,
     const DlDenseArgs& a = g.a;
     extern __shared__ __align__(128) uint8_t ring[];
     __shared__ uint64_t full[DR_STAGES], empty[DR_STAGES];
-    __shared__ int dead;
+    __shared__ WaitState ws;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t row_bytes = a.K * 2, stage_bytes = row_bytes * g.rows;
     // this CTA's stages
@@ -530,7 +517,7 @@ __global__ void __launch_bounds__((dense_ring_warps(MT, PAIR, SLICED) + 1) * 32,
     const __nv_bfloat16* w = (const __nv_bfloat16*)a.W + (size_t)t0 * g.rows * a.K;
     auto rows_of = [&](int t) { return min(g.rows, a.N - (t0 + t) * g.rows); };
     if (threadIdx.x == 0) {
-        dead = 0;
+        wait_init(ws, g.limit);
         for (int s = 0; s < g.stages; ++s) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((uint32_t)__cvta_generic_to_shared(&full[s])) : "memory");
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"((uint32_t)__cvta_generic_to_shared(&empty[s])), "r"(g.group) : "memory");
@@ -546,11 +533,12 @@ __global__ void __launch_bounds__((dense_ring_warps(MT, PAIR, SLICED) + 1) * 32,
         if (lane == 0)
             for (int t = 0; t < nt; ++t) {
                 const int s = t % g.stages;
-                if (t >= g.stages && !dense_ring_wait(&empty[s], ((t / g.stages) & 1) ^ 1, &dead)) break;
+                if (wait_gave_up(ws) || (t >= g.stages && !wait_phase(&empty[s], ((t / g.stages) & 1) ^ 1, ws, g.limit))) break;
                 const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&full[s]), bytes = row_bytes * rows_of(t);
                 asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
                 asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"((uint32_t)__cvta_generic_to_shared(ring + (size_t)s * stage_bytes)), "l"(w + (size_t)t * g.rows * a.K), "r"(bytes), "r"(bar) : "memory");
             }
+        if (wait_gave_up(ws)) wait_settle();
         return;
     }
     const int grp = warp / g.group, wi = warp - grp * g.group, slice = SLICED ? wi % g.slices : 0, row = SLICED ? wi / g.slices : wi * RW, k0 = slice * DR_K + lane * 8;
@@ -570,7 +558,7 @@ __global__ void __launch_bounds__((dense_ring_warps(MT, PAIR, SLICED) + 1) * 32,
     }
     for (int t = grp; grp < g.groups && t < nt; t += g.groups) {
         const int s = t % g.stages, n = (t0 + t) * g.rows + row;
-        const bool ok = dense_ring_wait(&full[s], (t / g.stages) & 1, &dead);
+        const bool ok = wait_phase(&full[s], (t / g.stages) & 1, ws, g.limit) && !wait_gave_up(ws);      // (a stage behind one given up shows the parity of the use before)
         float acc[MT][RW];
 #pragma unroll
         for (int m = 0; m < MT; ++m)
@@ -609,6 +597,7 @@ __global__ void __launch_bounds__((dense_ring_warps(MT, PAIR, SLICED) + 1) * 32,
             }
         }
     }
+    if (wait_gave_up(ws)) wait_settle();
     if (!SLICED) return;
     asm volatile("bar.sync 1, %0;" ::"n"(WARPS * 32) : "memory");
     const int n0 = t0 * g.rows, rows = min(nt * g.rows, a.N - n0);
@@ -830,7 +819,7 @@ static void launch_dense(const DlDenseArgs& a, cudaStream_t st) {
     }
     if constexpr (sizeof(WT) == 2 && RX) {
         DenseRing g;
-        if (vec && dense_ring(a, n_sms, g)) {
+        if (vec && dense_ring(a, n_sms, g) && dl_wait_limit("dl_dense", &g.limit) == 0) {
             if (a.M == 1) launch_dense_ring<1>(g, st, n_sms);
             else launch_dense_ring<2>(g, st, n_sms);
             return;

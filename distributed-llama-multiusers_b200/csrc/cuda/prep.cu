@@ -2,7 +2,11 @@
 // error plumbing.
 #include <stdarg.h>
 #include <stdio.h>
+#include <atomic>
+#include <cstring>
+#include <mutex>
 #include "epilogue.cuh"
+#include "waits.cuh"
 
 static thread_local char g_err[512] = "";
 void dl_set_error(const char* fmt, ...) {
@@ -12,6 +16,35 @@ void dl_set_error(const char* fmt, ...) {
     va_end(ap);
 }
 extern "C" const char* dl_last_error(void) { return g_err; }
+
+// ---- limits of waits -----------------------------------------------------------------
+// Words in host memory that kernels whose waits gave up write, one per device: the host reads them where it reads results, without a copy of their own.
+static std::atomic<unsigned long long> g_wait_limit{WAIT_DEADLINE_NS};
+static unsigned* wait_status_word() {
+    constexpr int devices = 64;
+    static std::mutex lock;
+    static unsigned* words = nullptr;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev >= devices) return nullptr;
+    std::lock_guard<std::mutex> guard(lock);
+    if (words == nullptr) {
+        void* p = nullptr;
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;       // the first launch may be a captured one
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        const cudaError_t e = cudaHostAlloc(&p, devices * sizeof(unsigned), cudaHostAllocPortable | cudaHostAllocMapped);
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (e != cudaSuccess) { cudaGetLastError(); return nullptr; }
+        words = (unsigned*)memset(p, 0, devices * sizeof(unsigned));
+    }
+    return words + dev;
+}
+extern "C" const unsigned* dl_attention_status() { return wait_status_word(); }
+extern "C" void dl_debug_set_wait_limit(unsigned long long ns) { g_wait_limit = ns; }
+int dl_wait_limit(const char* who, WaitLimit* l) {
+    *l = {g_wait_limit, wait_status_word()};
+    if (l->status == nullptr) { dl_set_error("%s: no host memory for its status", who); return -1; }
+    return 0;
+}
 
 // ---- optional launch timeline -----------------------------------------------------------------
 static unsigned long long* g_trace_base = nullptr;

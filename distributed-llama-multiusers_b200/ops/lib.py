@@ -523,8 +523,8 @@ def check_layers(rc: int, what: str = ""):
 
 
 class WaitStatus:
-    """Whether a wait inside a prompt attention kernel of `library` gave up on the current device (dl_attention_status): such a launch
-    returned 0 long ago and its outputs are NaN.  An engine looks where it has synchronised with its launches anyway."""
+    """Whether a wait inside a kernel of `library` gave up on the current device (dl_attention_status): such a launch returned 0 long ago and its
+    outputs are not valid.  An engine looks where it has synchronised with its launches anyway."""
 
     def __init__(self, library):
         word = library.dl_attention_status()
@@ -536,7 +536,7 @@ class WaitStatus:
         now = self._word.value
         if now != self._seen:
             self._seen = now
-            raise NativeLibraryError("a wait inside a prompt attention kernel gave up: outputs of the launches since the last look are not valid")
+            raise NativeLibraryError("a wait inside a kernel gave up: outputs of the launches since the last look are not valid")
 
 
 # kernels launched by this process (bench.py reports it as gpu_launches)

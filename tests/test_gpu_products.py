@@ -326,6 +326,35 @@ def test_rows_through_the_ring(M, N, K_, epi):
     assert (y.double() - want).norm() <= 1e-6 * want.norm() and (buf[:, cols:] == 3).all()
 
 
+@pytest.mark.parametrize("M,N,K_,epi", [(1, 6146, 2048, "store"), (2, 6146, 2048, "pair"), (1, 1000, 14336, "store"), (1, 3076, 4096, "pair")])
+def test_a_ring_that_gives_up_reaches_the_caller(M, N, K_, epi):
+    """A limit that is over before the kernel starts: no copy is issued, so its waits run out.  The status word changes once for that launch, whose outputs
+    are NaN, and not for the next one, which is right."""
+    import ctypes
+    from dllama_b200.ops import lib as B
+    lib, library = L(), B.layers_lib()
+    g = torch.Generator(device="cuda").manual_seed(N)
+    w, x = (torch.randn(N, K_, generator=g, device="cuda") * K_ ** -0.5).bfloat16(), torch.randn(M, K_, generator=g, device="cuda")
+    y = [torch.zeros(M, N // 2 if epi == "pair" else N, device="cuda") for _ in range(3)]
+    run = lambda out: lib.dense(w, x, out, M, True, **(dict(epi=lib.DENSE_GLU_GELU) if epi == "pair" else {}))
+    run(y[0])
+    status = B.WaitStatus(library)
+    library.dl_debug_set_wait_limit.argtypes = [ctypes.c_ulonglong]
+    library.dl_debug_set_wait_limit(0)
+    try:
+        run(y[1])
+        torch.cuda.synchronize()
+    finally:
+        library.dl_debug_set_wait_limit(4_000_000_000)
+    assert y[1].isnan().all()
+    with pytest.raises(B.NativeLibraryError, match="gave up"):
+        status.check()
+    run(y[2])
+    torch.cuda.synchronize()
+    status.check()
+    assert torch.equal(y[0], y[2]) and not y[0].isnan().any()
+
+
 @pytest.mark.parametrize("M", [3, 8, 9, 16, 17, 32])
 @pytest.mark.parametrize("N,K_", [(40, 8), (2047, 1032), (2370, 136), (4700, 264), (4790, 1096), (9500, 200)])
 def test_few_rows_by_columns_per_cta(M, N, K_):
