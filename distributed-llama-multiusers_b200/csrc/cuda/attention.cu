@@ -14,7 +14,9 @@
 //  * the output is cast to Q80 and written directly in the XQ / XH slab layout the wo matmul
 //    consumes (OP_CAST y->yq_slice, src/llm.cpp:296-301).
 #include <math.h>
+#define WAIT_UNIT 4u
 #include "epilogue.cuh"
+#include "waits.cuh"
 
 #define ATT_PAGE 32            // tokens per KV page (fixed)
 #define ATT_STAGES 4
@@ -40,6 +42,7 @@ struct AttArgs {
     int out_mcap;
     float* y_out;              // [M][n_heads*HS] or NULL
     unsigned long long* tr;
+    WaitLimit limit;           // (attention_kernel)
 };
 
 // 32 values per lane -> lane i ends with the warp-wide sum of value i (31 shuffles)
@@ -108,6 +111,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attention_kernel(const __grid_
     const int np = max(0, pg1 - pg0);
     const int* bt = a.block_table + (size_t)a.slot[m] * a.max_pages;
 
+    bool alive = true;                                         // no wait was given up
     if (warp == ATT_WARPS) {
         // producer warp: the 32 lanes fetch 32 block-table entries at once (one load latency instead of one per
         // page in front of every copy), lane 0 issues the bulk copies
@@ -119,11 +123,13 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attention_kernel(const __grid_
                 if (lane == 0) {
                     const int i = i0 + j;
                     const int s = i % ATT_STAGES;
-                    if (i >= ATT_STAGES) mbar_wait(&empty[s], ((i / ATT_STAGES) & 1) ^ 1);
+                    if (i >= ATT_STAGES) alive = alive && wait_phase(&empty[s], ((i / ATT_STAGES) & 1) ^ 1, a.limit, true) && a.limit.ns != 0;      // (no time: tests)
                     const size_t poff = ((size_t)page * a.n_kv_heads + kvh) * (size_t)PAGE_BYTES;
-                    mbar_arrive_expect_tx(&full[s], 2 * PAGE_BYTES);
-                    bulk_g2s(ring + (s * 2 + 0) * PAGE_BYTES, reinterpret_cast<const uint8_t*>(a.k_cache) + poff, PAGE_BYTES, &full[s]);
-                    bulk_g2s(ring + (s * 2 + 1) * PAGE_BYTES, reinterpret_cast<const uint8_t*>(a.v_cache) + poff, PAGE_BYTES, &full[s]);
+                    if (alive) {
+                        mbar_arrive_expect_tx(&full[s], 2 * PAGE_BYTES);
+                        bulk_g2s(ring + (s * 2 + 0) * PAGE_BYTES, reinterpret_cast<const uint8_t*>(a.k_cache) + poff, PAGE_BYTES, &full[s]);
+                        bulk_g2s(ring + (s * 2 + 1) * PAGE_BYTES, reinterpret_cast<const uint8_t*>(a.v_cache) + poff, PAGE_BYTES, &full[s]);
+                    }
                 }
                 __syncwarp();
             }
@@ -152,7 +158,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attention_kernel(const __grid_
 
         for (int i = 0; i < np; i++) {
             const int s = i % ATT_STAGES;
-            mbar_wait(&full[s], (i / ATT_STAGES) & 1);
+            alive = alive && wait_phase(&full[s], (i / ATT_STAGES) & 1, a.limit, true);
             const KV* Kp = reinterpret_cast<const KV*>(ring + (s * 2 + 0) * PAGE_BYTES);
             const KV* Vp = reinterpret_cast<const KV*>(ring + (s * 2 + 1) * PAGE_BYTES);
             const int ntok = min(ATT_PAGE, T - (pg0 + i) * ATT_PAGE);   // valid tokens in this page
@@ -216,11 +222,19 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attention_kernel(const __grid_
                 }
             }
             __syncwarp();
-            if (lane == 0) mbar_arrive(&empty[s]);
+            if (lane == 0 && alive) mbar_arrive(&empty[s]);
         }
         // per-warp partials -> smem
 #pragma unroll
         for (int c = 0; c < NCH; c++) {
+            if (!alive) {
+                run_m[c] = 0.0f;
+                run_l[c] = 1.0f;
+#pragma unroll
+                for (int h = 0; h < 4; h++)
+#pragma unroll
+                    for (int d = 0; d < DPL; d++) acc[c][h][d] = __int_as_float(0x7fffffff);
+            }
 #pragma unroll
             for (int h = 0; h < 4; h++)
 #pragma unroll
@@ -231,6 +245,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attention_kernel(const __grid_
             }
         }
     }
+    if (!alive) wait_settle();
     __syncthreads();
 
     // CTA-level merge of the 4 warps: thread d < HS owns head dim d
@@ -774,6 +789,7 @@ extern "C" int dl_attention(const float* q, int M, int n_heads, int n_kv_heads, 
     a.part_ml = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(scratch) + ATT_COUNTER_BYTES + o);
     a.xq_out = xq_out; a.xh_out = xh_out; a.out_mcap = out_mcap; a.y_out = y_out;
     a.tr = dl_trace_next(TR_ATT);
+    if (dl_wait_limit("dl_attention", &a.limit) != 0) return -1;
     const int G = n_heads / n_kv_heads;
     cudaStream_t st = (cudaStream_t)stream;
     if (kv_f32) {

@@ -498,9 +498,31 @@ static void launch_dense_mma(const DlDenseArgs& a, cudaStream_t st, int n_sms) {
 #define DR_STAGES 24                   // at most
 #define DR_RING (192 * 1024)
 #define DR_PART (16 * 1024)
-// rows per stage, warps per row (slices of DR_K inputs), warps per stage, groups of them, stages of the ring
-struct DenseRing { DlDenseArgs a; int rows, slices, group, groups, stages; WaitLimit limit; };
+// rows per stage, warps per row (slices of DR_K inputs), warps per stage, groups of them, stages of the ring, stages that are copied at most
+struct DenseRing { DlDenseArgs a; int rows, slices, group, groups, stages, most; WaitLimit limit; };
 
+// false: given up (once one wait of the CTA has been, all its later ones).  In line and with the CTA's state in shared memory: a call costs this kernel registers
+// (2048 x 8192 7.7 us so, 9.8 by the waits of waits.cuh)
+struct DenseRingState { unsigned long long t0; int gave_up; };
+__device__ __forceinline__ bool dense_ring_gave_up(const DenseRingState& w) { return *(const volatile int*)&w.gave_up != 0; }
+__device__ __forceinline__ bool dense_ring_wait(uint64_t* bar, uint32_t parity, DenseRingState& w, const WaitLimit& l) {
+    const uint32_t at = (uint32_t)__cvta_generic_to_shared(bar);
+    for (unsigned n = 1; !wait_try(at, parity); ++n) {
+        if ((n & 0x3Fu) != 0) continue;
+        if (dense_ring_gave_up(w)) return false;
+        if ((n & 0x3FFu) != 0) continue;
+        unsigned long long now;
+        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
+        const unsigned long long t0 = atomicCAS(&w.t0, 0ull, now);
+        if (l.ns != 0 && (t0 == 0 || (long long)(now - t0) <= (long long)l.ns)) continue;
+        if (atomicExch(&w.gave_up, 1) == 0) {
+            *(volatile unsigned*)l.status = (WAIT_UNIT << 24) + ((atomicAdd(&g_times_given_up, 1u) + 1u) & 0xFFFFFFu);
+            __threadfence_system();
+        }
+        return false;
+    }
+    return true;
+}
 // consumers (two rows of activations: their inputs leave registers for eight); one more warp copies
 static __host__ __device__ constexpr int dense_ring_warps(int MT, bool pair, bool sliced) { return MT == 2 ? 8 : pair && !sliced ? 12 : 16; }
 template <int MT, bool PAIR, bool SLICED>
@@ -509,7 +531,7 @@ __global__ void __launch_bounds__((dense_ring_warps(MT, PAIR, SLICED) + 1) * 32,
     const DlDenseArgs& a = g.a;
     extern __shared__ __align__(128) uint8_t ring[];
     __shared__ uint64_t full[DR_STAGES], empty[DR_STAGES];
-    __shared__ WaitState ws;
+    __shared__ DenseRingState ws;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t row_bytes = a.K * 2, stage_bytes = row_bytes * g.rows;
     // this CTA's stages
@@ -517,7 +539,8 @@ __global__ void __launch_bounds__((dense_ring_warps(MT, PAIR, SLICED) + 1) * 32,
     const __nv_bfloat16* w = (const __nv_bfloat16*)a.W + (size_t)t0 * g.rows * a.K;
     auto rows_of = [&](int t) { return min(g.rows, a.N - (t0 + t) * g.rows); };
     if (threadIdx.x == 0) {
-        wait_init(ws, g.limit);
+        ws.t0 = 0;
+        ws.gave_up = 0;
         for (int s = 0; s < g.stages; ++s) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((uint32_t)__cvta_generic_to_shared(&full[s])) : "memory");
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"((uint32_t)__cvta_generic_to_shared(&empty[s])), "r"(g.group) : "memory");
@@ -531,14 +554,14 @@ __global__ void __launch_bounds__((dense_ring_warps(MT, PAIR, SLICED) + 1) * 32,
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (warp == WARPS) {
         if (lane == 0)
-            for (int t = 0; t < nt; ++t) {
+            for (int t = 0; t < min(nt, g.most); ++t) {
                 const int s = t % g.stages;
-                if (wait_gave_up(ws) || (t >= g.stages && !wait_phase(&empty[s], ((t / g.stages) & 1) ^ 1, ws, g.limit))) break;
+                if (t >= g.stages && !dense_ring_wait(&empty[s], ((t / g.stages) & 1) ^ 1, ws, g.limit)) break;
                 const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&full[s]), bytes = row_bytes * rows_of(t);
                 asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
                 asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"((uint32_t)__cvta_generic_to_shared(ring + (size_t)s * stage_bytes)), "l"(w + (size_t)t * g.rows * a.K), "r"(bytes), "r"(bar) : "memory");
             }
-        if (wait_gave_up(ws)) wait_settle();
+        if (dense_ring_gave_up(ws)) __nanosleep(1000000);      // copies in flight land
         return;
     }
     const int grp = warp / g.group, wi = warp - grp * g.group, slice = SLICED ? wi % g.slices : 0, row = SLICED ? wi / g.slices : wi * RW, k0 = slice * DR_K + lane * 8;
@@ -558,7 +581,7 @@ __global__ void __launch_bounds__((dense_ring_warps(MT, PAIR, SLICED) + 1) * 32,
     }
     for (int t = grp; grp < g.groups && t < nt; t += g.groups) {
         const int s = t % g.stages, n = (t0 + t) * g.rows + row;
-        const bool ok = wait_phase(&full[s], (t / g.stages) & 1, ws, g.limit) && !wait_gave_up(ws);      // (a stage behind one given up shows the parity of the use before)
+        const bool ok = dense_ring_wait(&full[s], (t / g.stages) & 1, ws, g.limit) && !dense_ring_gave_up(ws);      // (a stage behind one given up shows the parity of the use before)
         float acc[MT][RW];
 #pragma unroll
         for (int m = 0; m < MT; ++m)
@@ -583,7 +606,7 @@ __global__ void __launch_bounds__((dense_ring_warps(MT, PAIR, SLICED) + 1) * 32,
                 }
         }
         __syncwarp();
-        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"((uint32_t)__cvta_generic_to_shared(&empty[s])) : "memory");
+        if (lane == 0 && ok) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"((uint32_t)__cvta_generic_to_shared(&empty[s])) : "memory");
 #pragma unroll
         for (int m = 0; m < MT; ++m)
 #pragma unroll
@@ -597,7 +620,7 @@ __global__ void __launch_bounds__((dense_ring_warps(MT, PAIR, SLICED) + 1) * 32,
             }
         }
     }
-    if (wait_gave_up(ws)) wait_settle();
+    if (dense_ring_gave_up(ws)) __nanosleep(1000000);      // copies in flight land
     if (!SLICED) return;
     asm volatile("bar.sync 1, %0;" ::"n"(WARPS * 32) : "memory");
     const int n0 = t0 * g.rows, rows = min(nt * g.rows, a.N - n0);
@@ -820,6 +843,7 @@ static void launch_dense(const DlDenseArgs& a, cudaStream_t st) {
     if constexpr (sizeof(WT) == 2 && RX) {
         DenseRing g;
         if (vec && dense_ring(a, n_sms, g) && dl_wait_limit("dl_dense", &g.limit) == 0) {
+            g.most = g.limit.ns == 0 ? 2 : 1 << 30;                                        // (no time: tests)
             if (a.M == 1) launch_dense_ring<1>(g, st, n_sms);
             else launch_dense_ring<2>(g, st, n_sms);
             return;

@@ -28,7 +28,9 @@
 // Pipelines: raw ring (producer -> dequant), B ring (producer -> MMA), A stages (dequant -> MMA,
 // released by tcgen05.commit), accumulator barrier (MMA -> epilogue).  K can be split over a
 // thread-block cluster (DSMEM reduction) when there are too few row tiles to fill the chip.
+#define WAIT_UNIT 2u
 #include "epilogue.cuh"
+#include "waits.cuh"
 
 #define TC_DEQ_WARPS 16
 #define TC_THREADS (64 + TC_DEQ_WARPS * 32 + 32)      // producer, MMA warp 0, dequantisers, MMA warp 1
@@ -51,12 +53,31 @@ struct TcArgs {
     int n_epi_ctas;
     int vec;               // epilogue_vec takes the epilogue
     unsigned long long* tr;
-    int dbg_mode;          // debug timing experiments (results invalid): 1 = one MMA per k-tile, 2 = no dequant/STTM
+    int dbg_mode;          // debug timing experiments (results invalid): 1 = one MMA per k-tile, 2 = no dequant/STTM; 16 = no weights behind the first ringful (a limit of no time: tests)
     long long* dbg;        // debug: per-tile clock64 stamps of CTA 0 (dl_debug_set_tc_trace), [tile][8]
     DlEpilogue epi;
+    WaitLimit limit;
 };
 
 #define TC_DBG(slot, i) do { if (a.dbg && blockIdx.x == 0 && blockIdx.y == 0 && (i) < 64) a.dbg[(i) * 8 + (slot)] = clock64(); } while (0)
+
+// The waits of the dequantisers, the issuers and the epilogue have no limit of their own (with one in each a step of 32 rows of width 4096 and 4 layers
+// took 353 to 359 us for 350): the producer, which has nothing else to do by then, ends them.  It gives up where it can issue nothing, or has
+// issued all and sees no end, for longer than the limit; then, its copies having landed, it says of every stage that it is full and free until the
+// accumulators are through.  What the launch stores then is not valid.
+static __device__ __noinline__ void tc_end_waits(uint64_t* fullA, uint64_t* fullB, uint64_t* fullH, uint64_t* emptyH, uint64_t* accum_full) {
+    wait_settle();
+    for (int n = 0; n < (1 << 20) && !mbar_test_wait(accum_full, 0); n++) {
+        for (int s = 0; s < 16; s++) {
+            mbar_arrive(&fullA[s]);
+            if (s >= 8) continue;
+            mbar_arrive(&fullB[s]);
+            mbar_arrive(&emptyH[s]);
+            for (int j = 0; j < 4; j++) mbar_arrive(&fullH[s]);
+        }
+        __nanosleep(500);
+    }
+}
 
 __global__ void __launch_bounds__(TC_THREADS, 1) gemm_q40_tc_kernel(const __grid_constant__ TcArgs a) {
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -139,12 +160,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_q40_tc_kernel(const __grid
         }
         __syncwarp();
         pdl_wait();
+        unsigned idle = 0;
         while (__any_sync(0xffffffffu, i < n_role)) {
             bool issued = false;
             if (i < n_role) {
                 if (role_a) {
                     const int sa = i % a.NSA;
-                    if (mbar_test_wait(&emptyA[sa], ((i / a.NSA) & 1) ^ 1)) {      // i >= NSA here
+                    if (mbar_test_wait(&emptyA[sa], ((i / a.NSA) & 1) ^ 1) && !(a.dbg_mode & 16)) {      // i >= NSA here
                         if (!(a.dbg_mode & 4)) TC_DBG(0, i);
                         mbar_arrive_expect_tx(&fullA[sa], Q40T_TILE_BYTES);
                         bulk_g2s_hint(ringA + sa * Q40T_TILE_BYTES, tile_of(i), Q40T_TILE_BYTES, &fullA[sa], pol);
@@ -161,8 +183,17 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_q40_tc_kernel(const __grid
                     }
                 }
             }
-            if (!__any_sync(0xffffffffu, issued)) __nanosleep(40);      // leave the issue slots to the dequantisers
+            if (!__any_sync(0xffffffffu, issued)) {
+                __nanosleep(40);      // leave the issue slots to the dequantisers
+                if ((++idle & 0xFFFu) == 0 && (unsigned long long)idle * 40 >= a.limit.ns) break;      // about 40 ns and more each time
+            }
         }
+        const bool stuck = __any_sync(0xffffffffu, i < n_role);
+        if (lane == 0) {
+            if (stuck) wait_report(a.limit);
+            if (stuck || !wait_phase(accum_full, 0, a.limit, true)) tc_end_waits(fullA, fullB, fullH, emptyH, accum_full);
+        }
+        __syncwarp();
     } else if (warp == 1 || warp >= 2 + TC_DEQ_WARPS) {
         // ------------------------------------ MMA issuers ------------------------------------
         // One k-tile costs its issuing thread ~900 clk of mostly fixed latency (two barrier waits, fence,
@@ -493,7 +524,8 @@ extern "C" int dl_gemm_q40_tc(const uint8_t* w_q40t, int d, int n, const uint8_t
     a.vec = epilogue_vec_ok(*epi, d);
     a.tr = dl_trace_next(TR_TC);
     a.dbg = g_tc_dbg;
-    a.dbg_mode = g_tc_dbg_mode;
+    if (dl_wait_limit("dl_gemm_q40_tc", &a.limit) != 0) return -1;
+    a.dbg_mode = g_tc_dbg_mode | (a.limit.ns == 0 ? 16 : 0);
     const size_t smem = (size_t)a.NSB * a.NT * 256 + (size_t)a.NSA * Q40T_TILE_BYTES +
                         (size_t)TC_EPI_CHUNK * 128 * 4 + (2 * 16 + 4 * 8) * 8 + 8 + 16;
     static size_t max_set = 0;

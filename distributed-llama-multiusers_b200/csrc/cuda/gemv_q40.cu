@@ -25,7 +25,9 @@
 //    launch the first stages stream while the previous kernel (or a peer GPU) still runs.
 //  * the epilogue (epilogue.cuh) fuses RoPE + KV-cache write, SiLU*mul + Q80 cast, or the
 //    Q80-cast partial-sum push to every peer GPU with release flags.
+#define WAIT_UNIT 3u
 #include "epilogue.cuh"
+#include "waits.cuh"
 
 #define GEMV_NS 12                      // pipeline stages
 #define GEMV_NG 4                       // consumer groups of 128 threads
@@ -52,6 +54,7 @@ struct GemvArgs {
     unsigned long long* tr;
     DlNormProlog norm;
     DlEpilogue epi;
+    WaitLimit limit;
 };
 
 DL_DEVINL void consumer_bar() { asm volatile("bar.sync 1, %0;" ::"n"(GEMV_CONSUMERS) : "memory"); }
@@ -305,7 +308,7 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_q40_kernel(const __grid_
             const int tidm = warp;
             if (lane == 0) {
             // publish this CTA's share into every cluster rank's table; nobody reads remote shared memory, and a rank waits for
-            // all that it is sent, so ranks may exit independently later on
+            // all that it is sent, so ranks may exit independently later on (without a limit: every rank's own waits end, and then it sends)
             if (S > 1) {
                 for (int c = 0; c < S; c++)
                     st_async_f32(mapa_shared(smem_u32(ssq_all + crank * MT + tidm), c), t, mapa_shared(smem_u32(ssq_bar), c));
@@ -366,12 +369,14 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_q40_kernel(const __grid_
             }
         }
         if (is_prod_lane) {
-            for (; p_it < n_it; p_it += GEMV_NPROD, p_i += GEMV_NPROD) {
+            bool alive = a.limit.ns != 0;        // (no time: tests)
+            for (; alive && p_it < n_it; p_it += GEMV_NPROD, p_i += GEMV_NPROD) {
                 p_norm();
                 const int s = p_it % GEMV_NS;
-                mbar_wait(&empty[s], ((p_it / GEMV_NS) & 1) ^ 1);
+                if (!wait_phase(&empty[s], ((p_it / GEMV_NS) & 1) ^ 1, a.limit, true)) { alive = false; break; }
                 issue(p_u, p_i, s);
             }
+            if (!alive) wait_settle();
         }
     } else {
         // ------------------------------ consumers ------------------------------
@@ -379,7 +384,8 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_q40_kernel(const __grid_
         const int t = tid & 127;
         const int row = t % rows;            // local row
         const int kq = t / rows;             // handles blocks kb with (kb % R) == kq
-        if (!a.fused) mbar_wait(act_full, 0);
+        bool alive = true;                   // no wait was given up
+        if (!a.fused) alive = wait_phase(act_full, 0, a.limit, true);
         pdl_wait();                          // already satisfied (producer / prologue waited); orders the epilogue's reads
         if (tid == 0) { GEMV_TRACE(1); }
 
@@ -393,7 +399,7 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_q40_kernel(const __grid_
             for (int i = g; i < nk; i += GEMV_NG) {
                 const int it = u * nk + i;
                 const int s = it % GEMV_NS;
-                mbar_wait(&full[s], (it / GEMV_NS) & 1);
+                if (!wait_phase(&full[s], (it / GEMV_NS) & 1, a.limit, alive)) alive = false;
                 const uint8_t* st = stages + s * Q40T_TILE_BYTES;
                 const uint8_t* act = act_s + (size_t)i * M * XQ_ROW_BYTES;
                 if (R == 1) gemv_tile_row<MT>(st, act, row, rtile >> 1, M, acc);
@@ -426,12 +432,12 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_q40_kernel(const __grid_
                     }
                 }
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&empty[s]);
+                if (lane == 0 && alive) mbar_arrive(&empty[s]);
             }
             if (tid == 0 && u == n_my - 1) { GEMV_TRACE(2); }
             // partial sums of the NG*R (group, kq) owners of each row -> out_s
 #pragma unroll
-            for (int m = 0; m < MT; m++) red[((g * R + kq) * MT + m) * rows + row] = acc[m];
+            for (int m = 0; m < MT; m++) red[((g * R + kq) * MT + m) * rows + row] = alive ? acc[m] : __int_as_float(0x7fffffff);
             consumer_bar();
             for (int idx = tid; idx < MT * rows; idx += GEMV_CONSUMERS) {
                 const int m = idx / rows, r = idx % rows;
@@ -444,6 +450,7 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_q40_kernel(const __grid_
             epilogue_rows(a.epi, out_s, 128, rows, rt * Q40T_TILE_ROWS + rs * rows, a.d_real, M, 0, tid);
             if (u + 1 < n_my) consumer_bar();   // out_s / red are reused by the next unit
         }
+        if (!alive) wait_settle();
     }
     GEMV_TRACE(3);
     if (S > 1) {
@@ -567,6 +574,7 @@ extern "C" int dl_gemv_q40(const uint8_t* w_q40t, int d, int n, const uint8_t* x
     a.epi = *epi;
     a.trace = g_gemv_trace;
     a.tr = dl_trace_next(TR_GEMV);
+    if (dl_wait_limit("dl_gemv_q40", &a.limit) != 0) return -1;
     const int grid = owners * a.S;
     cudaStream_t st = (cudaStream_t)stream;
     switch (mt_of(M)) {

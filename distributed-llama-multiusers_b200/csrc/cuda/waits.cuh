@@ -1,18 +1,18 @@
-// Waits on mbarriers that end: a CTA whose wait has run out of time gives up all its waits, goes on without what it waited for (its outputs are not
-// valid) and leaves a word in host memory, which dl_attention_status() tells of.  Loops around waits are finite, so the kernel ends.
+// Waits on mbarriers that end: a thread whose wait has run out of time goes on without what it waited for, hardly waits any more, frees and fills no stage, and
+// leaves a word in host memory, which dl_attention_status() tells of: the outputs are not valid.  Loops around waits are finite, so the kernel ends.
+//
+// There is no state but the thread's own, and the limit is the LAST field of a kernel's arguments, read on the slow path alone: what a launch here pays for are
+// cold reads and shared stores ahead of its first copies, and registers (a step of one row, width 4096, 4 layers 211.0 us without limits, 216 to 219 with
+// the limit among the other arguments and two words of shared memory for a CTA's state, 211.5 so).  The kernel's parameter has to be a
+// __grid_constant__: a reference to it copies all of it to the stack otherwise.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 // argument of a kernel that waits (dl_wait_limit)
 struct WaitLimit {
-    unsigned long long ns;       // from the first wait of a CTA that has failed for some time and behind the kernels ahead of it; 0: no waiting at all
+    unsigned long long ns;       // how long (attention_prefill_tc.cu: a CTA in all)
     unsigned* status;            // host memory: the device's word of dl_attention_status()
-};
-// of a CTA, in shared memory
-struct WaitState {
-    unsigned long long t0;
-    int gave_up;
 };
 // 0, or -1 where there is no host memory for the status (dl_last_error)
 int dl_wait_limit(const char* who, WaitLimit* limit);
@@ -23,41 +23,42 @@ int dl_wait_limit(const char* who, WaitLimit* limit);
 #endif
 static __device__ unsigned g_times_given_up;
 
-__device__ __forceinline__ void wait_report(const WaitLimit& l) {
+static __device__ __noinline__ void wait_report(const WaitLimit& l) {
     *(volatile unsigned*)l.status = (WAIT_UNIT << 24) + ((atomicAdd(&g_times_given_up, 1u) + 1u) & 0xFFFFFFu);
     __threadfence_system();
 }
-// by one thread, ahead of a barrier of the CTA
-__device__ __forceinline__ void wait_init(WaitState& w, const WaitLimit& l) {
-    w.t0 = 0;
-    w.gave_up = l.ns == 0;
-    if (l.ns == 0) wait_report(l);
+__device__ __forceinline__ bool wait_try(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
 }
-__device__ __forceinline__ bool wait_gave_up(const WaitState& w) { return *(const volatile int*)&w.gave_up != 0; }
-// asked now and then by a wait that fails: is the CTA's time over?
-__device__ __forceinline__ bool wait_over(WaitState& w, const WaitLimit& l) {
-    if (wait_gave_up(w)) return true;
-    unsigned long long now;
+// of a wait that has failed for some time: the time counts from here on, and from the end of the kernels ahead (which this one may have started under);
+// a thread that has given up a wait before has none left
+static __device__ __noinline__ bool wait_slow(uint32_t bar, uint32_t parity, const WaitLimit& l, bool alive) {
+    unsigned long long t0, now;
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
-    const unsigned long long t0 = atomicCAS(&w.t0, 0ull, now);
-    if (t0 == 0 || (long long)(now - t0) <= (long long)l.ns) return false;
-    if (atomicExch(&w.gave_up, 1) == 0) wait_report(l);
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
+    do {
+        for (int n = 0; n < 256; n++)
+            if (wait_try(bar, parity)) return true;
+        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
+    } while (alive && now - t0 < l.ns);
+    if (alive) wait_report(l);
+    return false;
+}
+// false: given up.  alive: the thread has given up no wait before
+__device__ __forceinline__ bool wait_phase(uint64_t* bar, uint32_t parity, const WaitLimit& l, bool alive) {
+    const uint32_t at = (uint32_t)__cvta_generic_to_shared(bar);
+    for (unsigned n = 0; !wait_try(at, parity);)
+        if (++n == 1024) return wait_slow(at, parity, l, alive);
     return true;
 }
-// CLUSTER: what other CTAs of the cluster did ahead of the phase's end is seen too.  false: given up
-template <bool CLUSTER = false>
-__device__ __forceinline__ bool wait_phase(uint64_t* bar, uint32_t parity, WaitState& w, const WaitLimit& l) {
-    const uint32_t at = (uint32_t)__cvta_generic_to_shared(bar);
-    for (unsigned n = 1;; n++) {
-        uint32_t ok;
-        if (CLUSTER)
-            asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(at), "r"(parity) : "memory");
-        else
-            asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(at), "r"(parity) : "memory");
-        if (ok) return true;
-        if ((n & 0x3Fu) == 0 && (wait_gave_up(w) || ((n & 0x3FFu) == 0 && wait_over(w, l)))) return false;
-    }
+// ahead of the end of a thread that gave up: copies in flight land
+static __device__ __noinline__ void wait_settle() {
+    unsigned long long t0, now;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
+    do {
+        __nanosleep(100000);
+        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
+    } while (now - t0 < 1000000);
 }
-// ahead of the end of a CTA that gave up: its copies and MMAs in flight end
-__device__ __forceinline__ void wait_settle() { __nanosleep(1000000); }
