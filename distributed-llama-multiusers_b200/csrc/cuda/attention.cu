@@ -16,6 +16,7 @@
 #include <math.h>
 #define WAIT_UNIT 4u
 #include "epilogue.cuh"
+#include "smem_limit.cuh"
 #include "waits.cuh"
 
 #define ATT_PAGE 32            // tokens per KV page (fixed)
@@ -690,13 +691,9 @@ static size_t att_smem_bytes(int HS, int NCH, int esize) {
 
 template <int HS, int NCH, typename KV>
 static int launch_att(const AttArgs& a, int pdl, cudaStream_t stream) {
-    static bool attr_set = false;
     const size_t smem = att_smem_bytes(HS, NCH, (int)sizeof(KV));
-    if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(attention_kernel<HS, NCH, KV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) { dl_set_error("attention smem attr: %s", cudaGetErrorString(e)); return -(int)e; }
-        attr_set = true;
-    }
+    static SmemLimit given;
+    if (const int rc = dl_smem_limit("attention", attention_kernel<HS, NCH, KV>, smem, given)) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(a.n_splits, a.n_kv_heads, a.M);
     cfg.blockDim = dim3(ATT_THREADS);
@@ -718,12 +715,8 @@ template <int HS, int ST>
 static int launch_att_mma_st(const AttArgs& a, int pdl, cudaStream_t stream) {
     constexpr int smem = ATT_WARPS * ST * AM_TOK * HS * 4;
     static_assert(ATT_WARPS * 4 * (HS + 2) * 4 + 4 <= smem, "the merge fits the ring");
-    static bool attr_set = false;
-    if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(attention_mma_kernel<HS, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) { dl_set_error("attention smem attr: %s", cudaGetErrorString(e)); return -(int)e; }
-        attr_set = true;
-    }
+    static SmemLimit given;
+    if (const int rc = dl_smem_limit("attention", attention_mma_kernel<HS, ST>, smem, given)) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(a.n_splits, a.n_kv_heads, a.M);
     cfg.blockDim = dim3(ATT_WARPS * 32);

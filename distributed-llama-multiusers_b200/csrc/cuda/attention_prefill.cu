@@ -14,6 +14,7 @@
 #include <math.h>
 #include <mma.h>
 #include "epilogue.cuh"
+#include "smem_limit.cuh"
 
 #define PF_QTILE 64
 #define PF_WARPS 4
@@ -271,12 +272,8 @@ static int launch_pf(const PfArgs& a, int pdl, cudaStream_t stream) {
     const size_t ring = (size_t)PF_STAGES * 2 * PF_PAGE * (HS + 8) * sizeof(__half);
     const size_t outb = (size_t)PF_QTILE * HS * sizeof(float);
     const size_t smem = ring > outb ? ring : outb;
-    static bool set = false;
-    if (!set) {
-        cudaError_t e = cudaFuncSetAttribute(attention_prefill_kernel<HS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) { dl_set_error("attention_prefill smem attr: %s", cudaGetErrorString(e)); return -(int)e; }
-        set = true;
-    }
+    static SmemLimit given;
+    if (const int rc = dl_smem_limit("attention_prefill", attention_prefill_kernel<HS>, smem, given)) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)((a.M + PF_QTILE - 1) / PF_QTILE + PF_MAX_SEG), (unsigned)a.n_heads);      // upper bound of the tiles of all segments
     cfg.blockDim = dim3(PF_THREADS);

@@ -38,6 +38,7 @@
 #include <atomic>
 #include "epilogue.cuh"
 #include "f32_pairs.cuh"
+#include "smem_limit.cuh"
 #include "tensor_map.cuh"
 #include "waits.cuh"
 #include "window_tiles.cuh"
@@ -911,12 +912,8 @@ extern "C" int dl_attention_prefill_tc(const float* q, int M, int n_heads, int n
     const long long rows = (long long)n_cache_pages * n_kv_heads * 32;
     if (pt_make_map(&kmap, k_cache, rows, PT_HS, false) != 0 || pt_make_map(&vmap, v_cache, rows, PT_HS, false) != 0) return -1;
     const size_t smem = PT_SMEM;
-    static bool set = false;
-    if (!set) {
-        cudaError_t e = cudaFuncSetAttribute(attention_prefill_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) { dl_set_error("attention_prefill_tc smem attr: %s", cudaGetErrorString(e)); return -(int)e; }
-        set = true;
-    }
+    static SmemLimit given;
+    if (const int rc = dl_smem_limit("attention_prefill_tc", attention_prefill_tc_kernel<false>, smem, given)) return rc;
     cudaLaunchConfig_t cfg = {};
     const long long most = ((long long)(M + PT_ROWS - 1) / PT_ROWS + PT_MAX_SEG - 1) * n_heads;        // upper bound of the tiles of all segments
     cfg.gridDim = dim3((unsigned)(most < dl_device_sm_count() ? most : dl_device_sm_count()));
@@ -963,12 +960,8 @@ int dl_window_prefill_tc(const DlWindowAttnArgs& w, const int* tile_rows, int n_
     // the cache's page count is not known here; every copy reads a page that the block table names
     if (pt_make_map(&map, w.cache, 1ll << 31, 2 * PT_HS, true) != 0) return -1;
     const size_t smem = PT_SMEM;
-    static bool set = false;
-    if (!set) {
-        cudaError_t e = cudaFuncSetAttribute(attention_prefill_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) { dl_set_error("window_prefill_tc smem attr: %s", cudaGetErrorString(e)); return -(int)e; }
-        set = true;
-    }
+    static SmemLimit given;
+    if (const int rc = dl_smem_limit("window_prefill_tc", attention_prefill_tc_kernel<true>, smem, given)) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)groups, (unsigned)w.kv_heads, (unsigned)z);
     cfg.blockDim = dim3(PT_THREADS);

@@ -26,6 +26,7 @@
 #include <math.h>
 #include "epilogue.cuh"
 #include "mega_sched.h"
+#include "smem_limit.cuh"
 
 #define MG_NS 12                          // weight ring stages (9216 B each)
 #define MG_CONS 512                       // consumer threads (16 warps, 4 groups of 128)
@@ -1449,12 +1450,8 @@ extern "C" int dl_decode_mega_supported(const DlDecodeArgs* a, int grid) {
 
 template <int MT>
 static int launch_mega(const DlDecodeArgs& a, int grid, cudaStream_t stream) {
-    static bool attr_set = false;
-    if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(decode_mega_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, SM_TOTAL);
-        if (e != cudaSuccess) { dl_set_error("decode_mega smem attr: %s", cudaGetErrorString(e)); return -(int)e; }
-        attr_set = true;
-    }
+    static SmemLimit given;
+    if (const int rc = dl_smem_limit("decode_mega", decode_mega_kernel<MT>, SM_TOTAL, given)) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(MG_THREADS);

@@ -13,6 +13,7 @@
 // into Y behind one sigmoid gate per row.  A bias per output column, where given, is added first.
 #define WAIT_UNIT 1u
 #include "layer_common.cuh"
+#include "smem_limit.cuh"
 #include "waits.cuh"
 #include "../../../include/dllama_b200.h"
 
@@ -456,21 +457,12 @@ __global__ void __launch_bounds__(256, TWO ? 2 : 1) dense_mma_kernel(DlDenseArgs
     }
 }
 
-// once per kernel and device (the other kernels of this file run on any device without being asked)
-template <typename A>
-static void dense_smem(void (*kernel)(A), int bytes, bool (&set)[16]) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 16 && set[dev]) return;
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (dev < 16) set[dev] = true;
-}
 template <int NT, int C, bool TWO>
 static void launch_dense_mma_t(const DlDenseArgs& a, cudaStream_t st) {
     constexpr int smem = dense_mma_xs(NT, C) + 8 * dense_mma_depth(NT, C, TWO) * 4 * C * 512;
     static_assert(smem <= 227 * 1024, "shared memory");
-    static bool set[16] = {};
-    dense_smem(dense_mma_kernel<NT, C, TWO>, smem, set);
+    static SmemLimit given;
+    if (dl_smem_limit("dl_dense", dense_mma_kernel<NT, C, TWO>, smem, given) != 0) return;      // (the caller looks at CUDA's last error)
     launch_after(dense_mma_kernel<NT, C, TWO>, dim3((a.N + 16 * C - 1) / (16 * C), 1, a.batch), 256, st, a, smem);
 }
 // Columns per CTA (they share the staged activations): 16 until every SM has two CTAs, then 32, and 64 for 9 to 16 rows, whose CTAs of 64 have an SM of their own (us, 32 and
@@ -655,8 +647,8 @@ static bool dense_ring(const DlDenseArgs& a, int n_sms, DenseRing& g) {
 }
 template <int MT, bool PAIR, bool SLICED>
 static void launch_dense_ring_t(const DenseRing& g, cudaStream_t st, int n_sms) {
-    static bool set[16] = {};
-    dense_smem(dense_ring_kernel<MT, PAIR, SLICED>, DR_RING + DR_PART, set);
+    static SmemLimit given;
+    if (dl_smem_limit("dl_dense", dense_ring_kernel<MT, PAIR, SLICED>, DR_RING + DR_PART, given) != 0) return;
     launch_after(dense_ring_kernel<MT, PAIR, SLICED>, dim3(n_sms), (dense_ring_warps(MT, PAIR, SLICED) + 1) * 32, st, g, (size_t)g.stages * g.rows * g.a.K * 2 + (SLICED ? DR_PART : 0));
 }
 template <int MT>

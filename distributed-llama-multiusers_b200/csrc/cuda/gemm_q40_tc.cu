@@ -30,6 +30,7 @@
 // thread-block cluster (DSMEM reduction) when there are too few row tiles to fill the chip.
 #define WAIT_UNIT 2u
 #include "epilogue.cuh"
+#include "smem_limit.cuh"
 #include "waits.cuh"
 
 #define TC_DEQ_WARPS 16
@@ -528,12 +529,8 @@ extern "C" int dl_gemm_q40_tc(const uint8_t* w_q40t, int d, int n, const uint8_t
     a.dbg_mode = g_tc_dbg_mode | (a.limit.ns == 0 ? 16 : 0);
     const size_t smem = (size_t)a.NSB * a.NT * 256 + (size_t)a.NSA * Q40T_TILE_BYTES +
                         (size_t)TC_EPI_CHUNK * 128 * 4 + (2 * 16 + 4 * 8) * 8 + 8 + 16;
-    static size_t max_set = 0;
-    if (smem > max_set) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_q40_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) { dl_set_error("gemm tc smem attr: %s", cudaGetErrorString(e)); return -(int)e; }
-        max_set = smem;
-    }
+    static SmemLimit given;
+    if (const int rc = dl_smem_limit("gemm tc", gemm_q40_tc_kernel, smem, given)) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(cta_rows * a.S), (unsigned)((M + a.NT - 1) / a.NT));
     cfg.blockDim = dim3(TC_THREADS);

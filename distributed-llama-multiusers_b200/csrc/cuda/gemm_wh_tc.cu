@@ -28,6 +28,7 @@
 // owner, warps 2-17 epilogue.
 // Reference semantics: matmul_Q80_Q40_F32 (src/nn/nn-cpu-ops.cpp:352-377), llamafile sgemm (src/nn/llamafile/sgemm.cpp:593-783).
 #include "epilogue.cuh"
+#include "smem_limit.cuh"
 #include "tensor_map.cuh"
 
 #define WH_TILE_BYTES 32768
@@ -580,12 +581,8 @@ static int gemm_wh_rows_launch(const uint8_t* wh, int d, int n, const uint8_t* x
     a.nacc = a.NS % 2 == 0 ? 2 : 1;
     a.tmem_cols = 32;
     while (a.tmem_cols < 4 * a.NT) a.tmem_cols *= 2;            // two issuers x two tiles
-    static bool attr_set = false;
-    if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_wh_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, WS_SMEM);
-        if (e != cudaSuccess) { dl_set_error("gemm wh rows smem attr: %s", cudaGetErrorString(e)); return -(int)e; }
-        attr_set = true;
-    }
+    static SmemLimit given;
+    if (const int rc = dl_smem_limit("gemm wh rows", gemm_wh_rows_kernel, WS_SMEM, given)) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(clusters * a.S));
     cfg.blockDim = dim3(WS_THREADS);
@@ -677,13 +674,8 @@ static int gemm_wh_launch(const uint8_t* wh, int d, int n, const uint8_t* xh, in
     a.piece = g_wh_piece;
     a.tr = dl_trace_next(TR_TC);
     const size_t smem = 196608 + WT_VEC_CHUNK * EPI_TILE_LD * 4 + 16 * 8 + 16;
-    static bool attr_set = false;
-    if (!attr_set) {
-        cudaError_t e1 = cudaFuncSetAttribute(gemm_wh_tc_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        cudaError_t e2 = cudaFuncSetAttribute(gemm_wh_tc_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e1 != cudaSuccess || e2 != cudaSuccess) { dl_set_error("gemm wh smem attr: %s", cudaGetErrorString(e1 != cudaSuccess ? e1 : e2)); return -1; }
-        attr_set = true;
-    }
+    static SmemLimit given[2];
+    if (const int rc = cg == 2 ? dl_smem_limit("gemm wh", gemm_wh_tc_kernel<2>, smem, given[1]) : dl_smem_limit("gemm wh", gemm_wh_tc_kernel<1>, smem, given[0])) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(WT_THREADS);

@@ -27,6 +27,7 @@
 //    Q80-cast partial-sum push to every peer GPU with release flags.
 #define WAIT_UNIT 3u
 #include "epilogue.cuh"
+#include "smem_limit.cuh"
 #include "waits.cuh"
 
 #define GEMV_NS 12                      // pipeline stages
@@ -506,14 +507,10 @@ extern "C" void dl_debug_set_gemv_trace(unsigned long long* p) { g_gemv_trace = 
 
 template <int MT>
 static int launch_gemv(const GemvArgs& a, int grid, int pdl, cudaStream_t stream) {
-    static size_t attr_max = 0;
     const size_t smem = gemv_smem_bytes(MT, (a.KT + a.S - 1) / a.S, a.M);
     if (smem > 227 * 1024) { dl_set_error("dl_gemv_q40: %zu B of shared memory needed (n=%d, M=%d, k_split=%d): raise k_split", smem, a.n, a.M, a.S); return -1; }
-    if (smem > attr_max) {
-        cudaError_t e = cudaFuncSetAttribute(gemv_q40_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) { dl_set_error("gemv smem attr: %s", cudaGetErrorString(e)); return -(int)e; }
-        attr_max = smem;
-    }
+    static SmemLimit given;
+    if (const int rc = dl_smem_limit("gemv", gemv_q40_kernel<MT>, smem, given)) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(GEMV_THREADS);
