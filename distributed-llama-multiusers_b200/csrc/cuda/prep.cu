@@ -23,20 +23,22 @@ static std::atomic<unsigned long long> g_wait_limit{WAIT_DEADLINE_NS};
 static unsigned* wait_status_word() {
     constexpr int devices = 64;
     static std::mutex lock;
-    static unsigned* words = nullptr;
+    static std::atomic<unsigned*> words{nullptr};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev >= devices) return nullptr;
+    unsigned* w = words.load(std::memory_order_acquire);
+    if (w != nullptr) return w + dev;
     std::lock_guard<std::mutex> guard(lock);
-    if (words == nullptr) {
+    if ((w = words.load()) == nullptr) {
         void* p = nullptr;
         cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;       // the first launch may be a captured one
         cudaThreadExchangeStreamCaptureMode(&mode);
         const cudaError_t e = cudaHostAlloc(&p, devices * sizeof(unsigned), cudaHostAllocPortable | cudaHostAllocMapped);
         cudaThreadExchangeStreamCaptureMode(&mode);
         if (e != cudaSuccess) { cudaGetLastError(); return nullptr; }
-        words = (unsigned*)memset(p, 0, devices * sizeof(unsigned));
+        words.store(w = (unsigned*)memset(p, 0, devices * sizeof(unsigned)), std::memory_order_release);
     }
-    return words + dev;
+    return w + dev;
 }
 extern "C" const unsigned* dl_attention_status() { return wait_status_word(); }
 extern "C" void dl_debug_set_wait_limit(unsigned long long ns) { g_wait_limit = ns; }
@@ -70,9 +72,12 @@ extern "C" int dl_trace_kind(int i) { return (i >= 0 && i < g_trace_n) ? g_trace
     } while (0)
 
 extern "C" int dl_device_sm_count(void) {
+    static std::atomic<int> counts[64];
     int dev = 0, n = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return -1;
+    if (dev < 64 && (n = counts[dev].load(std::memory_order_relaxed)) > 0) return n;
     if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return -1;
+    if (dev < 64) counts[dev].store(n, std::memory_order_relaxed);
     return n;
 }
 
