@@ -454,23 +454,24 @@ static int tc_tile(int d, int n, int M, int ncap, int ks, int n_sms) {
     return nt;
 }
 
-// Ranks that share K: the count for which a launch takes least time, as fitted to 472 products of 512 to 8192 columns, 256 to 14336 inputs and 4 to 512 rows
-// (whole models of width 2048, 4096 and 8192 and a rank's part of them in 2, 4 and 8; cold weights): us a k-tile by the tile's rows, a start that grows with
-// the CTAs, and the ranks' exchange, which grows with both.  Clusters have to find room at once: 36 of four ranks do not (1536 x 4096 at 384 rows, two and four
-// ranks 11.3 and 18.3), 12 of eight are late (1536 x 4096 at 8 rows, four and eight ranks 4.9 and 5.6; ten, 1280 x 8192, 7.4 and 6.2).  Us
-// with 1 / 2 / 4 / 8 ranks: 4096 x 4096 at 32 rows 12.2 / 8.1 / 7.8, 128 rows 13.9 / 11.0 / 10.7; 768 x 4096 at 32 rows 12.0 / 7.7 / 5.3 / 4.5;
-// 4096 x 1024 at 8 rows 4.2 / 3.9 / 5.3, 64 rows 4.6 / 5.9 / 6.5; 8192 x 1024 at 8 rows 4.3 / 5.6; 4096 x 512 at 8 rows 3.2 / 3.5 / 5.1.
+// Ranks that share K: the count for which a launch takes least time, as fitted to 330 products of 512 to 8192 columns, 256 to 14336 inputs and 4 to 512 rows, each
+// behind the norm that makes its activations (whole models of width 2048, 4096 and 8192 and a rank's part of them in 2, 4 and 8; cold weights; one behind
+// the other alone they flatter few CTAs, whose successors start on the idle SMs): us a k-tile by the tile's rows, a start that grows with the CTAs, and
+// the ranks' exchange, which grows with both.  Clusters have to find room at once: 36 of four ranks do not, nor 16 of eight.  Us with 1 / 2 / 4 / 8 ranks, the
+// norm included: 4096 x 4096 at 8 rows 15.0 / 11.3 / 9.2, 64 rows 16.1 / 13.7 / 12.4; 4096 x 2048 at 8 rows 9.8 / 8.5 / 7.5, 64 rows 10.7 / 10.6 / 10.4;
+// 1536 x 4096 at 8 rows 15.0 / 10.9 / 8.6 / 7.7; 1024 x 2048 at 8 rows 9.7 / 8.3 / 7.3 / 6.8; 4096 x 1024 at 8 rows 7.4 / 7.3 / 6.9; 2048 x 2048 at 8 rows 9.9 / 8.2 /
+// 7.3 / 11.9; 2048 x 512 at 8 rows 6.5 / 6.8 / 7.0; 4096 x 1792 at 64 rows 10.1 / 10.2 / 10.3.
 extern "C" int dl_gemm_q40_tc_split(int d, int n, int M, int n_sms) {
     const int row_tiles = (d + 127) / 128, KT = n / Q40T_TILE_K;
     int best = 1;
     double least = 0;
     for (int S = 1; S <= 8 && S <= KT; S *= 2) {
         const int nt = tc_tile(d, n, M, 1 << 30, S, n_sms), m_tiles = (M + nt - 1) / nt, ctas = row_tiles * m_tiles * S;
-        if ((S == 4 && ctas > 128) || (S == 8 && ctas > 80) || (S > 1 && ctas > n_sms)) continue;
+        if ((S == 4 && ctas > 128) || (S == 8 && ctas > 96) || (S > 1 && ctas > n_sms)) continue;
         auto ramp = [&](int from, int over) { return ctas <= from ? 0.0 : ctas >= from + over ? 1.0 : (double)(ctas - from) / over; };
-        const double item = nt <= 32 ? 0.31 : nt == 64 ? 0.33 : nt == 128 ? 0.44 : 0.00085 * (4 * nt > 950 ? 4 * nt : 950);
-        const double rows = (nt <= 32 ? 0.0 : nt == 64 ? 1.0 : 2.2 + 0.025 * (nt - 128)) * M / ((double)m_tiles * nt);
-        const double start = S == 1 ? 1.9 + 1.9 * ramp(45, 88) : S == 2 ? 2.9 + 1.7 * ramp(64, 47) : S == 4 ? 3.0 + 2.1 * ramp(64, 47) : ctas <= 48 ? 2.9 : 3.9;
+        const double item = (nt <= 32 ? 0.41 : nt == 64 ? 0.42 : nt == 128 ? 0.465 : 0.00085 * (4 * nt > 950 ? 4 * nt : 950)) * (S == 1 ? 1.03 : 1.0);
+        const double rows = (nt <= 32 ? 0.0 : nt == 64 ? 0.95 : 3.8 + 0.025 * (nt - 128)) * M / ((double)m_tiles * nt);
+        const double start = S == 1 ? 1.8 + 1.45 * ramp(47, 90) : S == 2 ? 3.3 + (M <= 32 ? 0.0 : 1.45 * ramp(68, 50)) : S == 4 ? 3.1 + 1.8 * ramp(100, 50) : 2.75 + 0.8 * ramp(55, 32);
         const double us = (KT + S - 1) / S * item + rows + start;
         if (S == 1 || us < least) { best = S; least = us; }
     }

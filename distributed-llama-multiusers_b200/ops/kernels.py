@@ -6,6 +6,7 @@ capture; nothing here allocates except where stated.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 from typing import List, Optional, Sequence
 
 import torch
@@ -354,6 +355,7 @@ def decode_mega_plan(d: int, n: int, align: int, grid: int, cta: int):
     return r0.value, r1.value, nc.value
 
 
+@functools.lru_cache(maxsize=4096)
 def choose_tc_split(d: int, n: int, M: int, n_sms: int) -> int:
     """How many CTAs of a cluster share K in the tcgen05 GEMM (1, 2, 4 or 8): what takes least time for these sizes (gemm_q40_tc.cu)."""
     return cuda_lib().dl_gemm_q40_tc_split(d, n, M, n_sms)
