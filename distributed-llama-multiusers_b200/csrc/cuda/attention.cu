@@ -43,7 +43,6 @@ struct AttArgs {
     int out_mcap;
     float* y_out;              // [M][n_heads*HS] or NULL
     unsigned long long* tr;
-    WaitLimit limit;           // (attention_kernel)
 };
 
 // 32 values per lane -> lane i ends with the warp-wide sum of value i (31 shuffles)
@@ -66,7 +65,7 @@ template <> DL_DEVINL float kv_to_float<float>(float v) { return v; }
 template <> DL_DEVINL float kv_to_float<__half>(__half v) { return __half2float(v); }
 
 template <int HS, int NCH, typename KV>
-__global__ void __launch_bounds__(ATT_THREADS, 1) attention_kernel(const __grid_constant__ AttArgs a) {
+__global__ void __launch_bounds__(ATT_THREADS, 1) attention_kernel(const __grid_constant__ AttArgs a, const __grid_constant__ WaitLimit limit) {
     constexpr int DPL = HS / 32;                       // head dims per lane
     constexpr int PAGE_BYTES = ATT_PAGE * HS * (int)sizeof(KV);
     constexpr int GMAX = NCH * 4;
@@ -124,7 +123,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attention_kernel(const __grid_
                 if (lane == 0) {
                     const int i = i0 + j;
                     const int s = i % ATT_STAGES;
-                    if (i >= ATT_STAGES) alive = alive && wait_phase(&empty[s], ((i / ATT_STAGES) & 1) ^ 1, a.limit, true) && a.limit.ns != 0;      // (no time: tests)
+                    if (i >= ATT_STAGES) alive = alive && wait_phase(&empty[s], ((i / ATT_STAGES) & 1) ^ 1, limit, true) && limit.ns != 0;      // (no time: tests)
                     const size_t poff = ((size_t)page * a.n_kv_heads + kvh) * (size_t)PAGE_BYTES;
                     if (alive) {
                         mbar_arrive_expect_tx(&full[s], 2 * PAGE_BYTES);
@@ -159,7 +158,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attention_kernel(const __grid_
 
         for (int i = 0; i < np; i++) {
             const int s = i % ATT_STAGES;
-            alive = alive && wait_phase(&full[s], (i / ATT_STAGES) & 1, a.limit, true);
+            alive = alive && wait_phase(&full[s], (i / ATT_STAGES) & 1, limit, true);
             const KV* Kp = reinterpret_cast<const KV*>(ring + (s * 2 + 0) * PAGE_BYTES);
             const KV* Vp = reinterpret_cast<const KV*>(ring + (s * 2 + 1) * PAGE_BYTES);
             const int ntok = min(ATT_PAGE, T - (pg0 + i) * ATT_PAGE);   // valid tokens in this page
@@ -691,6 +690,8 @@ static size_t att_smem_bytes(int HS, int NCH, int esize) {
 
 template <int HS, int NCH, typename KV>
 static int launch_att(const AttArgs& a, int pdl, cudaStream_t stream) {
+    WaitLimit limit;
+    if (dl_wait_limit("dl_attention", &limit) != 0) return -1;
     const size_t smem = att_smem_bytes(HS, NCH, (int)sizeof(KV));
     static SmemLimit given;
     if (const int rc = dl_smem_limit("attention", attention_kernel<HS, NCH, KV>, smem, given)) return rc;
@@ -706,7 +707,7 @@ static int launch_att(const AttArgs& a, int pdl, cudaStream_t stream) {
         cfg.attrs = attr;
         cfg.numAttrs = 1;
     }
-    cudaError_t e = cudaLaunchKernelEx(&cfg, attention_kernel<HS, NCH, KV>, a);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, attention_kernel<HS, NCH, KV>, a, limit);
     if (e != cudaSuccess) { dl_set_error("attention launch: %s", cudaGetErrorString(e)); return -(int)e; }
     return 0;
 }
@@ -782,7 +783,6 @@ extern "C" int dl_attention(const float* q, int M, int n_heads, int n_kv_heads, 
     a.part_ml = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(scratch) + ATT_COUNTER_BYTES + o);
     a.xq_out = xq_out; a.xh_out = xh_out; a.out_mcap = out_mcap; a.y_out = y_out;
     a.tr = dl_trace_next(TR_ATT);
-    if (dl_wait_limit("dl_attention", &a.limit) != 0) return -1;
     const int G = n_heads / n_kv_heads;
     cudaStream_t st = (cudaStream_t)stream;
     if (kv_f32) {

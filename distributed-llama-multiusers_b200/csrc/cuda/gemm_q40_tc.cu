@@ -64,10 +64,11 @@ struct TcArgs {
 
 // The waits of the dequantisers, the issuers and the epilogue have no limit of their own (with one in each a step of 32 rows of width 4096 and 4 layers
 // took 353 to 359 us for 350): the producer, which has nothing else to do by then, ends them.  It gives up where it can issue nothing, or has
-// issued all and sees no end, for longer than the limit; then, its copies having landed, it says of every stage that it is full and free until the
-// accumulators are through.  What the launch stores then is not valid.
-static __device__ __noinline__ void tc_end_waits(uint64_t* fullA, uint64_t* fullB, uint64_t* fullH, uint64_t* emptyH, uint64_t* accum_full) {
+// issued all and sees no end, for longer than the limit; then, its copies having landed, it fills the weights' ring with scales that are NaN and says of every
+// stage that it is full and free until the accumulators are through (a stage may be multiplied as it was, so most of what is stored then is NaN, not all).
+static __device__ __noinline__ void tc_end_waits(uint8_t* ringA, int bytes, uint64_t* fullA, uint64_t* fullB, uint64_t* fullH, uint64_t* emptyH, uint64_t* accum_full) {
     wait_settle();
+    for (int i = 0; i < bytes / 4; i++) reinterpret_cast<volatile uint32_t*>(ringA)[i] = 0xFFFFFFFFu;
     for (int n = 0; n < (1 << 20) && !mbar_test_wait(accum_full, 0); n++) {
         for (int s = 0; s < 16; s++) {
             mbar_arrive(&fullA[s]);
@@ -192,7 +193,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_q40_tc_kernel(const __grid
         const bool stuck = __any_sync(0xffffffffu, i < n_role);
         if (lane == 0) {
             if (stuck) wait_report(a.limit);
-            if (stuck || !wait_phase(accum_full, 0, a.limit, true)) tc_end_waits(fullA, fullB, fullH, emptyH, accum_full);
+            // ranks of a cluster meet right behind their accumulators: there the last stage that is filled is looked at instead
+            const int last = (n_it - 1) % a.nstg, turn = ((n_it - 1) / a.nstg) & 1;
+            if (stuck || !wait_phase(S > 1 ? &fullH[last] : accum_full, S > 1 ? turn : 0, a.limit, true)) tc_end_waits(ringA, a.NSA * Q40T_TILE_BYTES, fullA, fullB, fullH, emptyH, accum_full);
         }
         __syncwarp();
     } else if (warp == 1 || warp >= 2 + TC_DEQ_WARPS) {
@@ -426,6 +429,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_q40_tc_kernel(const __grid
 
 extern void dl_set_error(const char* fmt, ...);
 extern "C" int dl_device_sm_count();
+int dl_sm_count(int dev);
 
 static long long* g_tc_dbg = nullptr;
 static int g_tc_dbg_mode = 0;
@@ -495,7 +499,9 @@ extern "C" int dl_gemm_q40_tc(const uint8_t* w_q40t, int d, int n, const uint8_t
     a.d_pad = (d + 127) / 128 * 128;
     a.KT = n / Q40T_TILE_K;
     a.ncap = ncap; a.M = M;
-    const int row_tiles = (d + 127) / 128, n_sms = dl_device_sm_count();
+    int dev = 0;
+    if (const cudaError_t e = cudaGetDevice(&dev)) { dl_set_error("dl_gemm_q40_tc: %s", cudaGetErrorString(e)); return -(int)e; }
+    const int row_tiles = (d + 127) / 128, n_sms = dl_sm_count(dev);
     a.NT = tc_tile(d, n, M, ncap, (k_split == 2 || k_split == 4 || k_split == 8) ? k_split : 1, n_sms);
     if (ncap < (M + a.NT - 1) / a.NT * a.NT) { dl_set_error("dl_gemm_q40_tc: ncap=%d too small for M=%d (tile %d)", ncap, M, a.NT); return -1; }
     if (k_split != 1 && k_split != 2 && k_split != 4 && k_split != 8) { dl_set_error("dl_gemm_q40_tc: k_split must be 1,2,4,8"); return -1; }
@@ -526,12 +532,12 @@ extern "C" int dl_gemm_q40_tc(const uint8_t* w_q40t, int d, int n, const uint8_t
     a.vec = epilogue_vec_ok(*epi, d);
     a.tr = dl_trace_next(TR_TC);
     a.dbg = g_tc_dbg;
-    if (dl_wait_limit("dl_gemm_q40_tc", &a.limit) != 0) return -1;
+    if (dl_wait_limit("dl_gemm_q40_tc", &a.limit, dev) != 0) return -1;
     a.dbg_mode = g_tc_dbg_mode | (a.limit.ns == 0 ? 16 : 0);
     const size_t smem = (size_t)a.NSB * a.NT * 256 + (size_t)a.NSA * Q40T_TILE_BYTES +
                         (size_t)TC_EPI_CHUNK * 128 * 4 + (2 * 16 + 4 * 8) * 8 + 8 + 16;
     static SmemLimit given;
-    if (const int rc = dl_smem_limit("gemm tc", gemm_q40_tc_kernel, smem, given)) return rc;
+    if (const int rc = dl_smem_limit("gemm tc", gemm_q40_tc_kernel, smem, given, dev)) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(cta_rows * a.S), (unsigned)((M + a.NT - 1) / a.NT));
     cfg.blockDim = dim3(TC_THREADS);

@@ -135,6 +135,21 @@ DL_DEVINL void gemv_tile_row(const uint8_t* st, const uint8_t* act, int row, int
     }
 }
 
+// The consumers' waits have no limit of their own (with one, steps of one to three rows took 0.3 to 3 % longer, and 0.5 to 1 % with the producer lanes watching
+// the last stages too): a producer lane whose stage is not freed for longer than the limit ends them.  (With all copies issued there is nothing left
+// to wait for but these.)  Copies in flight having landed, the ring is filled with scales that are NaN, and its stages and the activations are said to
+// have come, over and over for longer than any consumer needs.
+static __device__ __noinline__ void gemv_end_waits(uint64_t* full, uint64_t* act_full, uint8_t* stages, const WaitLimit& l) {
+    if (l.ns == 0) wait_report(l);
+    wait_settle();
+    for (int i = 0; i < GEMV_NS * Q40T_TILE_BYTES / 4; i++) reinterpret_cast<volatile uint32_t*>(stages)[i] = 0xFFFFFFFFu;
+    for (int n = 0; n < (1 << 14); n++) {
+        mbar_arrive(act_full);
+        for (int s = 0; s < GEMV_NS; s++) mbar_arrive(&full[s]);
+        __nanosleep(500);
+    }
+}
+
 template <int MT>
 __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_q40_kernel(const __grid_constant__ GemvArgs a) {
     extern __shared__ __align__(128) uint8_t smem[];
@@ -361,6 +376,7 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_q40_kernel(const __grid_
 
     if (warp == GEMV_CONSUMERS / 32) {
         // ------------------------------ producer warp ------------------------------
+        bool alive = true;
         if (is_producer) {
             if (!a.fused) {
                 pdl_wait();
@@ -370,23 +386,22 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_q40_kernel(const __grid_
             }
         }
         if (is_prod_lane) {
-            bool alive = a.limit.ns != 0;        // (no time: tests)
+            alive = a.limit.ns != 0;             // (no time: tests)
             for (; alive && p_it < n_it; p_it += GEMV_NPROD, p_i += GEMV_NPROD) {
                 p_norm();
                 const int s = p_it % GEMV_NS;
                 if (!wait_phase(&empty[s], ((p_it / GEMV_NS) & 1) ^ 1, a.limit, true)) { alive = false; break; }
                 issue(p_u, p_i, s);
             }
-            if (!alive) wait_settle();
         }
+        if (__any_sync(0xffffffffu, !alive) && lane == 0) gemv_end_waits(full, act_full, stages, a.limit);
     } else {
         // ------------------------------ consumers ------------------------------
         const int g = tid >> 7;              // consumer group: k-tile i of a unit goes to group i % NG
         const int t = tid & 127;
         const int row = t % rows;            // local row
         const int kq = t / rows;             // handles blocks kb with (kb % R) == kq
-        bool alive = true;                   // no wait was given up
-        if (!a.fused) alive = wait_phase(act_full, 0, a.limit, true);
+        if (!a.fused) mbar_wait(act_full, 0);
         pdl_wait();                          // already satisfied (producer / prologue waited); orders the epilogue's reads
         if (tid == 0) { GEMV_TRACE(1); }
 
@@ -400,7 +415,7 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_q40_kernel(const __grid_
             for (int i = g; i < nk; i += GEMV_NG) {
                 const int it = u * nk + i;
                 const int s = it % GEMV_NS;
-                if (!wait_phase(&full[s], (it / GEMV_NS) & 1, a.limit, alive)) alive = false;
+                mbar_wait(&full[s], (it / GEMV_NS) & 1);
                 const uint8_t* st = stages + s * Q40T_TILE_BYTES;
                 const uint8_t* act = act_s + (size_t)i * M * XQ_ROW_BYTES;
                 if (R == 1) gemv_tile_row<MT>(st, act, row, rtile >> 1, M, acc);
@@ -433,12 +448,12 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_q40_kernel(const __grid_
                     }
                 }
                 __syncwarp();
-                if (lane == 0 && alive) mbar_arrive(&empty[s]);
+                if (lane == 0) mbar_arrive(&empty[s]);
             }
             if (tid == 0 && u == n_my - 1) { GEMV_TRACE(2); }
             // partial sums of the NG*R (group, kq) owners of each row -> out_s
 #pragma unroll
-            for (int m = 0; m < MT; m++) red[((g * R + kq) * MT + m) * rows + row] = alive ? acc[m] : __int_as_float(0x7fffffff);
+            for (int m = 0; m < MT; m++) red[((g * R + kq) * MT + m) * rows + row] = acc[m];
             consumer_bar();
             for (int idx = tid; idx < MT * rows; idx += GEMV_CONSUMERS) {
                 const int m = idx / rows, r = idx % rows;
@@ -451,7 +466,6 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_q40_kernel(const __grid_
             epilogue_rows(a.epi, out_s, 128, rows, rt * Q40T_TILE_ROWS + rs * rows, a.d_real, M, 0, tid);
             if (u + 1 < n_my) consumer_bar();   // out_s / red are reused by the next unit
         }
-        if (!alive) wait_settle();
     }
     GEMV_TRACE(3);
     if (S > 1) {
@@ -506,11 +520,11 @@ static unsigned long long* g_gemv_trace = nullptr;
 extern "C" void dl_debug_set_gemv_trace(unsigned long long* p) { g_gemv_trace = p; }
 
 template <int MT>
-static int launch_gemv(const GemvArgs& a, int grid, int pdl, cudaStream_t stream) {
+static int launch_gemv(const GemvArgs& a, int grid, int pdl, int dev, cudaStream_t stream) {
     const size_t smem = gemv_smem_bytes(MT, (a.KT + a.S - 1) / a.S, a.M);
     if (smem > 227 * 1024) { dl_set_error("dl_gemv_q40: %zu B of shared memory needed (n=%d, M=%d, k_split=%d): raise k_split", smem, a.n, a.M, a.S); return -1; }
     static SmemLimit given;
-    if (const int rc = dl_smem_limit("gemv", gemv_q40_kernel<MT>, smem, given)) return rc;
+    if (const int rc = dl_smem_limit("gemv", gemv_q40_kernel<MT>, smem, given, dev)) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(GEMV_THREADS);
@@ -571,13 +585,15 @@ extern "C" int dl_gemv_q40(const uint8_t* w_q40t, int d, int n, const uint8_t* x
     a.epi = *epi;
     a.trace = g_gemv_trace;
     a.tr = dl_trace_next(TR_GEMV);
-    if (dl_wait_limit("dl_gemv_q40", &a.limit) != 0) return -1;
+    int dev = 0;
+    if (const cudaError_t e = cudaGetDevice(&dev)) { dl_set_error("dl_gemv_q40: %s", cudaGetErrorString(e)); return -(int)e; }
+    if (dl_wait_limit("dl_gemv_q40", &a.limit, dev) != 0) return -1;
     const int grid = owners * a.S;
     cudaStream_t st = (cudaStream_t)stream;
     switch (mt_of(M)) {
-        case 1: return launch_gemv<1>(a, grid, pdl, st);
-        case 2: return launch_gemv<2>(a, grid, pdl, st);
-        case 4: return launch_gemv<4>(a, grid, pdl, st);
-        default: return launch_gemv<8>(a, grid, pdl, st);
+        case 1: return launch_gemv<1>(a, grid, pdl, dev, st);
+        case 2: return launch_gemv<2>(a, grid, pdl, dev, st);
+        case 4: return launch_gemv<4>(a, grid, pdl, dev, st);
+        default: return launch_gemv<8>(a, grid, pdl, dev, st);
     }
 }

@@ -20,12 +20,11 @@ extern "C" const char* dl_last_error(void) { return g_err; }
 // ---- limits of waits -----------------------------------------------------------------
 // Words in host memory that kernels whose waits gave up write, one per device: the host reads them where it reads results, without a copy of their own.
 static std::atomic<unsigned long long> g_wait_limit{WAIT_DEADLINE_NS};
-static unsigned* wait_status_word() {
+static unsigned* wait_status_word(int dev = -1) {
     constexpr int devices = 64;
     static std::mutex lock;
     static std::atomic<unsigned*> words{nullptr};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev >= devices) return nullptr;
+    if ((dev < 0 && cudaGetDevice(&dev) != cudaSuccess) || dev >= devices) return nullptr;
     unsigned* w = words.load(std::memory_order_acquire);
     if (w != nullptr) return w + dev;
     std::lock_guard<std::mutex> guard(lock);
@@ -42,8 +41,8 @@ static unsigned* wait_status_word() {
 }
 extern "C" const unsigned* dl_attention_status() { return wait_status_word(); }
 extern "C" void dl_debug_set_wait_limit(unsigned long long ns) { g_wait_limit = ns; }
-int dl_wait_limit(const char* who, WaitLimit* l) {
-    *l = {g_wait_limit, wait_status_word()};
+int dl_wait_limit(const char* who, WaitLimit* l, int dev) {
+    *l = {g_wait_limit, wait_status_word(dev)};
     if (l->status == nullptr) { dl_set_error("%s: no host memory for its status", who); return -1; }
     return 0;
 }
@@ -71,14 +70,17 @@ extern "C" int dl_trace_kind(int i) { return (i >= 0 && i < g_trace_n) ? g_trace
         }                                                                               \
     } while (0)
 
-extern "C" int dl_device_sm_count(void) {
+int dl_sm_count(int dev) {
     static std::atomic<int> counts[64];
-    int dev = 0, n = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return -1;
+    int n = 0;
     if (dev < 64 && (n = counts[dev].load(std::memory_order_relaxed)) > 0) return n;
     if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return -1;
     if (dev < 64) counts[dev].store(n, std::memory_order_relaxed);
     return n;
+}
+extern "C" int dl_device_sm_count(void) {
+    int dev = 0;
+    return cudaGetDevice(&dev) == cudaSuccess ? dl_sm_count(dev) : -1;
 }
 
 // ------------------------------------------------------------------------------------------------

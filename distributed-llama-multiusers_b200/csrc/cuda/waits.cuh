@@ -1,10 +1,10 @@
 // Waits on mbarriers that end: a thread whose wait has run out of time goes on without what it waited for, hardly waits any more, frees and fills no stage, and
 // leaves a word in host memory, which dl_attention_status() tells of: the outputs are not valid.  Loops around waits are finite, so the kernel ends.
 //
-// There is no state but the thread's own, and the limit is the LAST field of a kernel's arguments, read on the slow path alone: what a launch here pays for are
-// cold reads and shared stores ahead of its first copies, and registers (a step of one row, width 4096, 4 layers 211.0 us without limits, 216 to 219 with
-// the limit among the other arguments and two words of shared memory for a CTA's state, 211.5 so).  The kernel's parameter has to be a
-// __grid_constant__: a reference to it copies all of it to the stack otherwise.
+// There is no state but the thread's own, and the limit comes last among a kernel's arguments and is read on the slow path alone: what a launch here pays for are
+// cold reads and shared stores ahead of its first copies, registers, and arguments themselves (decode attention of 8 rows, launched alone, 7.6 us, 8.2 with 16
+// bytes more).  The kernel's parameter has to be a __grid_constant__: a reference to it copies all of it to the stack otherwise.  Kernels that
+// stream weights let a warp that only issues copies watch over the other roles' waits (gemv_q40.cu, gemm_q40_tc.cu).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -14,8 +14,8 @@ struct WaitLimit {
     unsigned long long ns;       // how long (attention_prefill_tc.cu: a CTA in all)
     unsigned* status;            // host memory: the device's word of dl_attention_status()
 };
-// 0, or -1 where there is no host memory for the status (dl_last_error)
-int dl_wait_limit(const char* who, WaitLimit* limit);
+// 0, or -1 where there is no host memory for the status (dl_last_error); dev: the current device where the caller knows it
+int dl_wait_limit(const char* who, WaitLimit* limit, int dev = -1);
 
 #define WAIT_DEADLINE_NS 4000000000ull
 #ifndef WAIT_UNIT

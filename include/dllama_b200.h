@@ -207,8 +207,8 @@ int dl_attention_prefill_tc(const float* q, int M, int n_heads, int n_kv_heads, 
                             int pdl, void* stream);
 
 /* Kernels that wait on copies inside a CTA (dl_attention_prefill_tc, dl_window_attention_tc's prompts, dl_attention on a ring of pages, dl_gemv_q40, dl_gemm_q40_tc,
- * dl_dense's ring for one and two rows) wait for some seconds at most.  Where one gives up, the outputs of that launch are not valid (NaN, but
- * dl_gemm_q40_tc's) and this word (in host memory; each device has its own, this is the current one's) changes: read it behind a synchronisation
+ * dl_dense's ring for one and two rows) wait for some seconds at most.  Where one gives up, the outputs of that launch are not valid (NaN, of
+ * dl_gemm_q40_tc most) and this word (in host memory; each device has its own, this is the current one's) changes: read it behind a synchronisation
  * with the launch.  NULL: no device, or no memory for it. */
 const unsigned* dl_attention_status(void);
 

@@ -391,7 +391,8 @@ def _given_up(call):
 @pytest.mark.parametrize("kernel,d,n,M,S", [("tc", 300, 4096, 20, 1), ("tc", 300, 8192, 20, 4), ("tc", 38912, 1024, 40, 1), ("tc", 9600, 2048, 200, 1), ("row", 300, 4096, 2, 1),
                                             ("row", 512, 8192, 8, 4), ("row", 128, 2048, 1, 1), ("norm", 512, 8192, 3, 4), ("norm", 9600, 2048, 1, 1)])
 def test_a_product_that_gives_up_reaches_the_caller(kernel, d, n, M, S):
-    """Waits that run out: the kernel ends, row by row all outputs are NaN, the status word changes once for that launch and not for the next one, which is right."""
+    """Waits that run out: the kernel ends, its outputs are NaN (of the tensor cores' most: a stage may be multiplied as it was), the status word changes once for
+    that launch and not for the next one, which is right."""
     k = K()
     ncap = (M + 255) // 256 * 256
     w, _ = _q40(d, n, 1)
@@ -412,7 +413,7 @@ def test_a_product_that_gives_up_reaches_the_caller(kernel, d, n, M, S):
             k.gemv_q40(w, d, n, None, M, epi, 1, S, norm=k.norm_prolog(x, None, None, 0, 0, None, None, 0, 0, norm, 1e-5))
     run(y[0])
     status = _given_up(lambda: run(y[1]))
-    assert kernel == "tc" or y[1].isnan().all()
+    assert y[1].isnan().float().mean() > 0.5 if kernel == "tc" else y[1].isnan().all()
     run(y[2])
     torch.cuda.synchronize()
     status.check()
