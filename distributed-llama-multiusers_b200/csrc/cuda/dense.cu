@@ -485,6 +485,9 @@ static void launch_dense_mma(const DlDenseArgs& a, cudaStream_t st, int n_sms) {
 // What bounds it: the weights' bytes.  The kernels above hold them in registers, two CTAs an SM, and start again every 8 columns.  Cold weights, us, they and
 // this: one row, 16384 x 2048 in pairs 15.1 and 12.7, 8192 x 2048 11.2 and 8.6, 32768 x 2048 27.9 and 23.6, 28672 x 4096 in pairs 40.5 and 37.0 (6.3 TB/s), 4096 x
 // 4096 9.6 and 8.0, 2048 x 8192 8.5 and 8.0, 4096 x 14336 24.7 and 20.7; two rows, 16384 x 2048 in pairs 18.5 and 13.7, 8192 x 2048 in pairs 11.3 and 9.0.
+//
+// The price: up to 208 KB of every SM's shared memory.  A kernel behind this one that needs more than 20 KB starts its prologue on an SM when the ring has left it, and
+// kernels of other streams wait for one too (norm, gate|up and down of 2048 x 8192 take 24.7 us with that).
 // ------------------------------------------------------------------------------------------------
 #define DR_K 2048                      // inputs of a warp
 #define DR_STAGES 24                   // at most

@@ -5,16 +5,16 @@
 //      32-block as the XH activation slabs).  fp16((nibble - 8) * d), one rounding: bit-identical to what the
 //      on-the-fly dequantisers of gemm_q40_tc.cu feed the tensor core.  The engine keeps the WH copy resident when
 //      it fits (8B: 15 GB of the 180 GB) or rebuilds it per matrix into a scratch buffer.
-//   2. gemm_wh_tc_kernel is then a plain fp16 SS-mode GEMM: both operands arrive by bulk async copies of
-//      contiguous, pre-tiled 16 KB pieces; nothing is unpacked inside the loop, so the unpack -- the limiter of the
+//   2. gemm_wh_tc_kernel is then a plain fp16 SS-mode GEMM: both operands arrive by bulk or tensor copies of
+//      contiguous, pre-tiled pieces of up to 16 KB; nothing is unpacked inside the loop, so the unpack -- the limiter of the
 //      fused kernel (ALU pipe 50 %, tensor pipe 14 % at 32 rows of w13), which every M tile
 //      repeated -- is paid once per weight instead of once per 256 activation rows.
 //
 // gemm_wh_tc_kernel<2> pairs two CTAs (cluster of 2 = one TPC) on a 256 weight rows x up to 256 activation rows tile with
 // `tcgen05.mma.cta_group::2`: each CTA stages its own 128 weight rows and HALF of the activation rows (64 KB per
 // 128-wide k step and CTA instead of 96 KB).  gemm_wh_tc_kernel<1> is the single-CTA variant (odd row-tile counts).
-// What bounds it: the MMAs under the power limit (28672 x 4096 at 2048 rows 313 us, 301 without its epilogues, 166 without MMAs, whose copies
-// then run at 85 B/clk and SM; cuBLAS 348).
+// What bounds it: the MMAs under the power limit (28672 x 4096 at 2048 rows 324 us, 312 without its epilogues; on a faster card 301 without them, 166 without MMAs,
+// whose copies then run at 85 B/clk and SM, and cuBLAS 348).
 //
 // Grouped mode: the same kernel runs one product per group of rows against that group's own weights (the experts of a
 // routed feed-forward: rows sorted by expert, segment bounds in device memory), so all experts are ONE launch and the
